@@ -138,6 +138,7 @@ PACKED_ARGTYPES = [ctypes.POINTER(TVMValue), ctypes.POINTER(ctypes.c_int), ctype
                    ctypes.POINTER(TVMValue), ctypes.POINTER(ctypes.c_int), ctypes.c_void_p]
 
 _lib = None
+_pycall = None
 
 
 class LibraryError(RuntimeError):
@@ -170,6 +171,26 @@ def load() -> ctypes.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def pycall():
+    """The extension module that packs torch tensors and makes the calls; raises LibraryError
+    when it has not been built."""
+    global _pycall
+    if _pycall is None:
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        try:
+            from . import _pycall as module
+        except ImportError as e:
+            raise LibraryError(f"{os.path.join(_PKG, '_pycall.so')} cannot be loaded ({e}): build it with "
+                               "`python -m sparsetir_b200.build`") from e
+        _pycall = module
+    return _pycall
+
+
+def entry_address(fn) -> int:
+    """Address of an exported function of the loaded library."""
+    return ctypes.cast(fn, ctypes.c_void_p).value
 
 
 def last_error() -> str:

@@ -2,7 +2,8 @@
 
 Usage: ``python -m sparsetir_b200.build [--force] [--verbose]``.
 Objects go to ``build/`` at the repository root; the shared library is written next to this
-file so that it travels with the source tree.
+file so that it travels with the source tree, and so is ``_pycall.so``, the Python extension
+that packs torch tensors for it.
 """
 from __future__ import annotations
 
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG_DIR)
@@ -19,6 +21,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 OBJ_DIR = os.path.join(ROOT, "build", "obj")
 LIB_PATH = os.path.join(PKG_DIR, "libsparsetir_b200.so")
+
+PYCALL_PATH = os.path.join(PKG_DIR, "_pycall.so")
 
 SOURCES = [
     "runtime.cc", "abi.cc", "format.cc", "validate.cu",
@@ -65,11 +69,37 @@ def _compile(src: str, force: bool, verbose: bool, hdr_mtime: float) -> str:
     return obj
 
 
+def build_pycall(force: bool = False) -> str:
+    """The extension module against this Python's and this torch's headers (g++)."""
+    import torch
+
+    src = os.path.join(CSRC, "pycall.cc")
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(INCLUDE, "sparsetir_b200.h")))
+    if not force and os.path.exists(PYCALL_PATH) and os.path.getmtime(PYCALL_PATH) > newest:
+        return PYCALL_PATH
+    torch_dir = os.path.dirname(os.path.abspath(torch.__file__))
+    lib_dir = os.path.join(torch_dir, "lib")
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
+           "-isystem", sysconfig.get_path("include"), "-isystem", os.path.join(torch_dir, "include"),
+           "-isystem", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           "-isystem", cuda_include, src, "-o", PYCALL_PATH, "-L", lib_dir, f"-Wl,-rpath,{lib_dir}",
+           "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(f"$ {' '.join(cmd)}\n{res.stdout}{res.stderr}")
+        raise RuntimeError("g++ failed on pycall.cc")
+    return PYCALL_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ_DIR, exist_ok=True)
     hdr = _newest_header()
     with cf.ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as pool:
+        pycall = pool.submit(build_pycall, force)
         objs = list(pool.map(lambda s: _compile(s, force, verbose, hdr), SOURCES))
+        pycall.result()
     if (force or not os.path.exists(LIB_PATH)
             or os.path.getmtime(LIB_PATH) < max(os.path.getmtime(o) for o in objs)):
         cmd = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode",

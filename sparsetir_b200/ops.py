@@ -19,6 +19,8 @@ import torch
 
 from . import _lib as L
 
+_addr = L.entry_address
+
 
 class SparseTIRError(RuntimeError):
     """Raised when an entry point returns -1 (the counterpart of tvm.TVMError)."""
@@ -68,25 +70,19 @@ def use_current_stream(device: Optional[torch.device] = None) -> None:
 class PreparedCall:
     """One packed call with its argument arrays already built (see PackedFunc.prepare)."""
 
-    __slots__ = ("_fn", "_values", "_codes", "_n", "_keep", "_dev_index", "_ret", "_ret_code",
-                 "_set_stream")
+    __slots__ = ("_args", "_keep", "_invoke")
 
     def __init__(self, fn, values, codes, n, keep, device):
-        self._fn, self._values, self._codes, self._n, self._keep = fn, values, codes, n, keep
-        self._dev_index = None
+        index = -1
         if device is not None:
-            self._dev_index = device.index if device.index is not None else torch.cuda.current_device()
-        self._ret = L.TVMValue()
-        self._ret_code = ctypes.c_int(0)
-        self._set_stream = L.load().sparsetir_set_stream
+            index = device.index if device.index is not None else torch.cuda.current_device()
+        self._keep = (fn, values, codes, keep)
+        self._args = (_addr(fn), _addr(L.load().sparsetir_set_stream), ctypes.addressof(values),
+                      ctypes.addressof(codes), n, index)
+        self._invoke = L.pycall().invoke_packed
 
     def __call__(self) -> None:
-        if self._dev_index is not None:
-            self._set_stream(self._dev_index,
-                             ctypes.c_void_p(torch.cuda.current_stream(self._dev_index).cuda_stream))
-        rc = self._fn(self._values, self._codes, self._n, ctypes.byref(self._ret),
-                      ctypes.byref(self._ret_code), None)
-        if rc != 0:
+        if self._invoke(*self._args) != 0:
             raise SparseTIRError(L.last_error())
 
 
@@ -96,6 +92,7 @@ class PackedFunc:
     def __init__(self, symbol: str):
         self.symbol = symbol
         self._fn = None
+        self._entry = None
 
     @property
     def entry_name(self) -> str:
@@ -104,10 +101,18 @@ class PackedFunc:
     def _resolve(self):
         if self._fn is None:
             self._fn = getattr(L.load(), self.symbol)
+            self._entry = (L.pycall().invoke, _addr(self._fn), _addr(L.load().sparsetir_set_stream))
         return self._fn
 
     def __call__(self, *args) -> None:
-        self.prepare(*args)()
+        if self._entry is None:
+            self._resolve()
+        invoke, fn, set_stream = self._entry
+        rc = invoke(fn, set_stream, args)
+        if rc is None:  # an argument that only prepare() takes, or refuses with its message
+            self.prepare(*args)()
+        elif rc != 0:
+            raise SparseTIRError(L.last_error())
 
     def prepare(self, *args) -> "PreparedCall":
         """Packs the arguments once; the returned object repeats the call without rebuilding
@@ -189,9 +194,10 @@ def hyb_args(x: torch.Tensor, y: torch.Tensor, buckets: Sequence[Sequence[torch.
     (examples/spmm/bench_spmm.py:207-222): ``[b, c] + [w, rows, cols] per bucket`` followed by
     the scalars this library needs because it is not specialised at build time.  With ``peer_c``
     (addresses of the peers' copies of ``y``) the list is that of ``hyb_spmm_peers``."""
-    args = [x.reshape(-1), y.reshape(-1)]
+    args = [x, y]
     for w, rows, cols in buckets:
-        args += [w.reshape(-1), rows.reshape(-1), cols.reshape(-1)]
+        args += (w, rows, cols)
+    L.pycall().flatten(args)
     args.append(int(feat_size))
     if flags or peer_c is not None:
         args.append(int(flags))
@@ -205,10 +211,11 @@ def rgms_ell3d_args(w: torch.Tensor, x: torch.Tensor, y: torch.Tensor,
     """Argument list of ``rgms_ell3d`` in the reference's layout
     (examples/rgms/rgcn/bench_rgcn_composable.py:196-208): ``[w, x, y]``, then ``a, rows, cols`` per
     bucket, then ``mid`` per bucket, then ``feat_size``.  ``buckets`` holds ``(a, rows, cols, mid)``."""
-    args = [w.reshape(-1), x.reshape(-1), y.reshape(-1)]
+    args = [w, x, y]
     for a, rows, cols, _ in buckets:
-        args += [a.reshape(-1), rows.reshape(-1), cols.reshape(-1)]
-    args += [mid.reshape(-1) for _, _, _, mid in buckets]
+        args += (a, rows, cols)
+    args += [mid for _, _, _, mid in buckets]
+    L.pycall().flatten(args)
     args.append(int(feat_size))
     return args
 
@@ -219,9 +226,10 @@ def rgms_ell3d_f16_args(w: torch.Tensor, x: torch.Tensor, y: torch.Tensor,
     (examples/rgms/rgcn/bench_rgcn_tensorcore.py:842-852): ``[w, x, y]``, then ``a, rows, cols`` per
     bucket, then ``mid`` per bucket, then the two feature sizes.  ``buckets`` holds
     ``(a, rows, cols, mid)`` with ``a`` in float16."""
-    args = [w.reshape(-1), x.reshape(-1), y.reshape(-1)]
+    args = [w, x, y]
     for a, rows, cols, _ in buckets:
-        args += [a.reshape(-1), rows.reshape(-1), cols.reshape(-1)]
-    args += [mid.reshape(-1) for _, _, _, mid in buckets]
+        args += (a, rows, cols)
+    args += [mid for _, _, _, mid in buckets]
+    L.pycall().flatten(args)
     args += [int(feat_in), int(feat_out)]
     return args
