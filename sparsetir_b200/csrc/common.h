@@ -37,6 +37,10 @@ void* workspace(int device_id, cudaStream_t stream, size_t bytes);
 // before it ends, so steady-state calls neither allocate nor clear.
 void* zeroed_workspace(int device_id, cudaStream_t stream, size_t bytes);
 
+// Whether both buffers of (device, stream) already hold that much, so that asking for them neither
+// allocates nor synchronises (neither is possible while the stream is being captured).
+bool workspace_fits(int device_id, cudaStream_t stream, size_t bytes, size_t zeroed_bytes);
+
 // Deep checks of index arrays before a launch (validate.cu): enabled by SPARSETIR_VALIDATE=1 or
 // sparsetir_set_validate(1).  Each returns 0, or -1 after recording which array is wrong where;
 // they synchronise `st`.  nnz < 0 skips the check of the last row pointer.

@@ -1,0 +1,384 @@
+// CSR SpMM, fp32, split by stored entries:  C[i,:] = sum_{p in row i} A[p] * B[indices[p],:]
+//
+// A block owns a contiguous range of stored entries (SUBS sub-warps of LPR lanes, `span` entries
+// each), so a hub row of thousands of entries is spread over many sub-warps and a run of short
+// rows costs what its entries cost: one launch, whatever the row lengths.  It replaces a row-wise
+// kernel with two more launches for the rows of more than 32 entries (169 k-node power-law graph,
+// F = 32 / 512: 71 / 357 us against 25 / 220 us) and a row-wise kernel for the feature counts
+// that are not whole tiles, where one sub-warp walked a hub row alone (100 k-node power-law
+// graph, F = 100: 2302 us against 28 us).
+//
+// Rows are found without a plan: a 32-ary search of `indptr` for the first entry of a sub-warp,
+// then a register window of row ends (row_walk.cuh).  Every output row has one writer and one
+// order of summation, so results repeat bit by bit:
+//  - a row inside one sub-warp is written by it;
+//  - the pieces of a row that crosses sub-warps meet in shared memory and are added in order by
+//    the sub-warp in which the row (or the block's part of it) starts;
+//  - the pieces of a row that crosses blocks meet in a scratch buffer; the block that counts in
+//    last adds them in order.  Nobody waits: counters are back at zero when the launch ends.
+// Rows without entries are cleared by the block that owns that share of the rows.
+//
+// Bound: latency of the dependent chain (search, ids, rows of B) on small matrices, the L2-to-SM
+// gather rate (about 17 TB/s) on large ones.
+#include <algorithm>
+
+#include "common.h"
+#include "row_walk.cuh"
+
+namespace sptir {
+namespace {
+
+constexpr int kThreads = 256;
+
+struct SplitArgs {
+  const float* a;
+  const float* b;
+  float* c;
+  const int32_t* indptr;
+  const int32_t* indices;
+  float* part;         // two scratch rows per block: the piece of a row that began before it, and
+                       // of a row that goes on behind it
+  unsigned* counters;  // [blocks][feature tiles], zero before and after every launch
+  int m, nnz, feat, span;
+  float rows_per_entry;
+};
+
+template <int LPR>
+__device__ __forceinline__ unsigned group_ballot(unsigned mask, bool pred) {
+  const unsigned all = __ballot_sync(mask, pred);
+  if constexpr (LPR == 32) {
+    return all;
+  } else {
+    return (all >> ((threadIdx.x & 31) / LPR * LPR)) & ((1u << LPR) - 1u);
+  }
+}
+
+// A lane owns VPL vectors of W floats of the feature tile (VPL * LPR * W floats), LPR * W apart: one
+// 16-byte vector where rows allow it, several 4- or 8-byte ones where their length or alignment
+// does not (odd feature counts: tiles of up to 160 floats instead of 32, so that ids are read that
+// much less often: 30 k rows, F = 299, 104 us with one vector, 66 with four, 59 with five).
+template <int LPR, int W, int VPL>
+__global__ void __launch_bounds__(kThreads, 4)
+csr_split_kernel(const SplitArgs s) {
+  using LV = LaneVec<W>;
+  using V = typename LV::type;
+  constexpr int SUBS = kThreads / LPR;
+  constexpr int NW = 32 / LPR;                       // sub-warps of a warp
+  constexpr int kU = W == 4 ? 8 : VPL <= 4 ? 16 / VPL : 4;  // more rows spill registers
+  constexpr int U = kU < LPR ? kU : LPR;             // gathered rows in flight per lane
+  constexpr int TILE = LPR * W * VPL;
+  __shared__ __align__(16) float s_lead[SUBS][TILE];  // piece of a row that began before the sub-warp
+  __shared__ __align__(16) float s_tail[SUBS][TILE];  // piece of a row that goes on behind it
+  __shared__ int s_state[SUBS];                          // kLead, kOpen, kTail
+  constexpr int kLead = 1, kOpen = 2, kTail = 4;         // kOpen: the lead piece is the whole span
+
+  const int wlane = threadIdx.x & 31;
+  const int lane = threadIdx.x % LPR;
+  const int sub = threadIdx.x / LPR;
+  const unsigned mask = group_mask<LPR>();
+  const long long block_entries = static_cast<long long>(SUBS) * s.span;
+  const long long blk0 = blockIdx.x * block_entries;
+  const unsigned row_bytes = static_cast<unsigned>(s.feat) * 4u;
+  const long long p0l = blk0 + static_cast<long long>(sub) * s.span;
+  const int p0 = static_cast<int>(min(p0l, static_cast<long long>(s.nnz)));
+  const int count = static_cast<int>(min(p0l + s.span, static_cast<long long>(s.nnz))) - p0;
+  int cid = 0;
+  float av = 0.f;
+  auto first_ids = [&]() {
+    if (lane < count) {
+      cid = __ldg(s.indices + p0 + lane);
+      av = __ldg(s.a + p0 + lane);
+    }
+  };
+  first_ids();  // on their way while the row is searched
+
+  const long long w0 = blk0 + static_cast<long long>((threadIdx.x / 32) * NW) * s.span;  // first entry of the warp
+  int first_row = 0;
+  bool first_lead = false;  // the first row of the sub-warp began before it
+  if (w0 < s.nnz) {
+    int pos[NW], row[NW];
+#pragma unroll
+    for (int i = 0; i < NW; ++i)
+      pos[i] = static_cast<int>(min(w0 + static_cast<long long>(i) * s.span, static_cast<long long>(s.nnz) - 1));
+    warp_rows_of<NW>(s.indptr, s.m, pos, s.rows_per_entry, wlane, row);
+    first_row = row[0];
+#pragma unroll
+    for (int i = 1; i < NW; ++i)
+      if (wlane / LPR == i) first_row = row[i];
+    first_lead = count > 0 && __ldg(s.indptr + first_row) < p0;
+  }
+
+  const int tiles = (s.feat + TILE - 1) / TILE;
+  for (int tile = blockIdx.y; tile < tiles; tile += gridDim.y) {
+    const int f0 = tile * TILE + lane * W;
+    // vectors past the row read the tile's first vector once more and store nothing
+    bool inside[VPL];
+    unsigned at[VPL];
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      inside[v] = f0 + v * (LPR * W) < s.feat;
+      at[v] = (inside[v] ? f0 + v * (LPR * W) : tile * TILE) * 4u;
+    }
+    const char* bl = reinterpret_cast<const char*>(s.b);
+    char* cl = reinterpret_cast<char*>(s.c);
+    auto c_row = [&](int r) -> char* {
+      return cl + static_cast<unsigned long long>(static_cast<unsigned>(r)) * row_bytes;
+    };
+    if (tile > static_cast<int>(blockIdx.y)) {
+      first_ids();
+      __syncthreads();  // the pieces of the tile before have been collected
+    }
+    int r = first_row, state = 0;
+    if (w0 < s.nnz) {  // the whole warp, its sub-warps in step
+      int wend = row_window<LPR>(s.indptr, s.m, r, lane);
+      bool lead = first_lead;
+      if (lead) state = kLead;
+      bool pending = false;  // entries of an unfinished row in acc
+      V acc[VPL];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) acc[v] = LV::zero();
+      const int steps = static_cast<int>(min(static_cast<long long>(s.span), s.nnz - w0));
+      for (int s0 = 0; s0 < steps; s0 += LPR) {
+        int cidn = 0;
+        float avn = 0.f;
+        if (s0 + LPR + lane < count) {  // ids and values of the next batch
+          cidn = __ldg(s.indices + p0 + s0 + LPR + lane);
+          avn = __ldg(s.a + p0 + s0 + LPR + lane);
+        }
+        const int cnt = max(0, min(LPR, count - s0));
+        // Most batches of a matrix of long rows lie inside one row for every sub-warp of the warp.
+        unsigned ends = 0, any_ends = 0;
+        int to = 0;
+        if (!__all_sync(0xffffffffu, lane != 0 || (cnt == LPR && wend - (p0 + s0) > LPR))) {
+          const int e = p0 + min(s0 + lane, count - 1);  // lanes past the last entry repeat it
+          int row_end;
+          const int row = row_in_window<LPR>(s.indptr, s.m, r, wend, e, row_end);
+          ends = group_ballot<LPR>(0xffffffffu, lane < cnt && row_end == e + 1);
+          any_ends = NW == 1 ? ends : __reduce_or_sync(0xffffffffu, ends);
+          r = __shfl_sync(0xffffffffu, row, LPR - 1, LPR);
+          if (cnt > 0) pending = ((ends >> (cnt - 1)) & 1u) == 0u;
+          if (!pending && cnt > 0) r = min(r + 1, s.m - 1);
+          // where the sum up to this entry goes if a row ends here; -1: the lead piece
+          to = lead && (ends & ((1u << lane) - 1u)) == 0u ? -1 : row;
+          if (ends != 0u) lead = false;
+          wend = row_window<LPR>(s.indptr, s.m, r, lane);
+        } else {
+          pending = true;
+        }
+#pragma unroll
+        for (int k0 = 0; k0 < LPR; k0 += U) {
+          if (k0 < steps - s0) {
+            V x[U][VPL];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {  // entries past the end have column 0 and are not added
+              const unsigned col = static_cast<unsigned>(__shfl_sync(0xffffffffu, cid, k0 + u, LPR));
+              const char* src = bl + static_cast<unsigned long long>(col) * row_bytes;
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) x[u][v] = LV::ldg(src + at[v]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
+              if (k0 + u < cnt) {
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
+              }
+              if ((any_ends >> (k0 + u)) & 1u) {  // a row ends here in some sub-warp of the warp
+                const int rk = __shfl_sync(0xffffffffu, to, k0 + u, LPR);
+                const bool end = (ends >> (k0 + u)) & 1u;
+                // one store instruction for both destinations: no branch among the sub-warps
+                char* dst = rk < 0 ? reinterpret_cast<char*>(&s_lead[sub][0]) - tile * (TILE * 4) : c_row(rk);
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) {
+                  if (end && inside[v]) LV::st(dst + at[v], acc[v]);
+                  LV::zero_if(acc[v], end);
+                }
+              }
+            }
+          }
+        }
+        cid = cidn;
+        av = avn;
+      }
+      if (pending) {
+        float* piece = lead ? s_lead[sub] : s_tail[sub];
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) LV::sts(piece + v * (LPR * W) + lane * W, acc[v]);
+        state |= lead ? kOpen : kTail;
+      }
+    }
+    if (lane == 0) s_state[sub] = state;
+    __syncthreads();
+
+    // ---- rows that cross sub-warps
+    auto finish = [&](V (&sum)[VPL], int row, bool from_before, bool goes_on) {
+      if (from_before || goes_on) {
+        const int begin = __ldg(s.indptr + row), end = __ldg(s.indptr + row + 1);
+        const int b0 = static_cast<int>(begin / block_entries), b1 = static_cast<int>((end - 1) / block_entries);
+        char* pl = reinterpret_cast<char*>(s.part);
+        auto piece = [&](int b) -> char* {
+          return pl + (2ull * static_cast<unsigned>(b) + (b == b0 ? 1u : 0u)) * row_bytes;
+        };
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+          if (inside[v]) LV::stcg(piece(blockIdx.x) + at[v], sum[v]);
+        __threadfence();
+        __syncwarp(mask);
+        unsigned* counter = s.counters + static_cast<size_t>(b0) * tiles + tile;
+        unsigned seen = 0;
+        if (lane == 0) seen = atomicAdd(counter, 1u);
+        seen = __shfl_sync(mask, seen, 0, LPR);
+        if (seen != static_cast<unsigned>(b1 - b0)) return;
+        if (lane == 0) *counter = 0u;  // last piece to arrive: all of them are visible
+        __threadfence();
+        constexpr int G = VPL < 5 ? 8 / VPL : 2;
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) sum[v] = LV::zero();
+        for (int b = b0; b <= b1; b += G) {
+          V x[G][VPL];
+#pragma unroll
+          for (int u = 0; u < G; ++u)
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) x[u][v] = LV::ldcg(piece(min(b + u, b1)) + at[v]);
+#pragma unroll
+          for (int u = 0; u < G; ++u)
+            if (b + u <= b1) {
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) LV::add(sum[v], x[u][v]);
+            }
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+        if (inside[v]) LV::stcs(c_row(row) + at[v], sum[v]);  // written once: keep B rows in L2
+    };
+    // adds the lead pieces of sub-warps k, k + 1, ... until the row ends; true if it leaves the block
+    auto collect = [&](V (&sum)[VPL], int k) -> bool {
+      for (; k < SUBS; ++k) {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) LV::add(sum[v], LV::lds(&s_lead[k][v * (LPR * W) + lane * W]));
+        if ((s_state[k] & kOpen) == 0) return false;
+      }
+      return true;
+    };
+    const bool more_blocks = blk0 + block_entries < s.nnz;
+    if (sub == 0 && (state & kLead)) {
+      V sum[VPL];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) sum[v] = LV::zero();
+      const bool goes_on = collect(sum, 0);
+      finish(sum, first_row, true, goes_on && more_blocks);
+    }
+    if (state & kTail) {
+      V sum[VPL];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) sum[v] = LV::lds(&s_tail[sub][v * (LPR * W) + lane * W]);
+      const bool goes_on = collect(sum, sub + 1);
+      finish(sum, r, false, goes_on && more_blocks);
+    }
+  }  // feature tiles
+
+  // ---- rows without entries: this block's share of the rows
+  if (blockIdx.y == 0) {
+    const int per = static_cast<int>((static_cast<long long>(s.m) + gridDim.x - 1) / gridDim.x);
+    const long long ra = static_cast<long long>(blockIdx.x) * per;
+    const long long rb = min(static_cast<long long>(s.m), ra + per);
+    for (long long r0 = ra + threadIdx.x - wlane; r0 < rb; r0 += kThreads) {
+      const long long rr = r0 + wlane;
+      const bool empty = rr < rb && __ldg(s.indptr + rr) == __ldg(s.indptr + rr + 1);
+      unsigned todo = __ballot_sync(0xffffffffu, empty);
+      while (todo != 0u) {
+        const int k = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        char* dst = reinterpret_cast<char*>(s.c) + static_cast<unsigned long long>(r0 + k) * row_bytes;
+        for (unsigned at = wlane * (W * 4u); at < row_bytes; at += 32u * W * 4u) LV::stcs(dst + at, LV::zero());
+      }
+    }
+  }
+}
+
+template <int LPR, int W, int VPL>
+int launch_split(SplitArgs s, int device_id, cudaStream_t st) {
+  constexpr int SUBS = kThreads / LPR;
+  const int tiles = ceil_div(s.feat, LPR * W * VPL);
+  s.rows_per_entry = static_cast<float>(s.m) / static_cast<float>(s.nnz);
+  // One wave of resident blocks with equal shares of the entries: a block's fixed cost (search,
+  // meeting of the pieces) is paid once, 4.5 M entries, F = 64: 94 us against 109 with four waves.
+  // A block walks the feature tiles one after the other, all blocks roughly in step, which keeps
+  // the slice of B that they gather from in L2; matrices too small to give every resident block
+  // a batch of entries deal the tiles to more blocks (60 k entries, F = 512: 25 against 37 us).
+  const long long resident = 4ll * kNumSMs, batch = static_cast<long long>(SUBS) * LPR;
+  const long long fewest = (s.nnz + batch - 1) / batch;
+  const int gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident / fewest)));
+  const long long want = resident / gy * SUBS;
+  s.span = static_cast<int>((s.nnz + want - 1) / want + LPR - 1) / LPR * LPR;
+  const long long per_block = static_cast<long long>(SUBS) * s.span;
+  const int blocks = static_cast<int>(std::max((s.nnz + per_block - 1) / per_block,
+                                               (static_cast<long long>(s.m) + 8 * kThreads - 1) / (8 * kThreads)));
+  const size_t part_bytes = 2 * static_cast<size_t>(blocks) * s.feat * sizeof(float);
+  const size_t counter_bytes = static_cast<size_t>(blocks) * tiles * sizeof(unsigned);
+  if (!workspace_fits(device_id, st, part_bytes, counter_bytes)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+      // the first call on this stream is being captured into a graph, where the library's buffers
+      // cannot grow: this call gets memory that the graph owns
+      char* own = nullptr;
+      const size_t at = (part_bytes + 255) & ~static_cast<size_t>(255);
+      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + counter_bytes, st));
+      SPTIR_CUDA_OK(cudaMemsetAsync(own + at, 0, counter_bytes, st));
+      s.part = reinterpret_cast<float*>(own);
+      s.counters = reinterpret_cast<unsigned*>(own + at);
+      csr_split_kernel<LPR, W, VPL><<<dim3(blocks, gy), kThreads, 0, st>>>(s);
+      SPTIR_LAUNCH_OK("csr_split_kernel");
+      SPTIR_CUDA_OK(cudaFreeAsync(own, st));
+      return 0;
+    }
+  }
+  s.part = static_cast<float*>(workspace(device_id, st, part_bytes));
+  s.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
+  if (s.part == nullptr || s.counters == nullptr) return -1;
+  csr_split_kernel<LPR, W, VPL><<<dim3(blocks, gy), kThreads, 0, st>>>(s);
+  SPTIR_LAUNCH_OK("csr_split_kernel");
+  return 0;
+}
+
+}  // namespace
+
+int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
+                  int m, int n, int feat, int nnz, int device_id, cudaStream_t st) {
+  if (nnz == 0) {
+    SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(m) * feat * sizeof(float), st));
+    return 0;
+  }
+  const SplitArgs s{a, b, c, indptr, indices, nullptr, nullptr, m, nnz, feat, 0, 0.f};
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+  if (feat % 4 == 0 && bits % 16 == 0) {
+    // The narrowest group that covers a row, a warp at most: several sub-warps per warp keep more
+    // rows in flight (4.5 M entries, F = 64: 16 lanes 93, 32 lanes 160, 8 lanes 107 us), a second
+    // pass over the entries costs more than it brings (169 k-node power-law graph, F = 128: 32
+    // lanes 56, 16 lanes 68 us) unless every row of B is gathered so often that a slice of B that
+    // stays in L2 pays for it.
+    int lanes = feat <= 32 ? 8 : (feat <= 64 ? 16 : 32);
+    while (lanes > 8 && n > 0 && nnz / n >= 64 &&
+           static_cast<size_t>(n) * std::min(lanes * 16, feat * 4) > (size_t{48} << 20))
+      lanes /= 2;
+    if (lanes == 8) return launch_split<8, 4, 1>(s, device_id, st);
+    if (lanes == 16) return launch_split<16, 4, 1>(s, device_id, st);
+    return launch_split<32, 4, 1>(s, device_id, st);
+  }
+  if (feat % 2 == 0 && bits % 8 == 0) {
+    if (feat <= 16) return launch_split<8, 2, 1>(s, device_id, st);
+    if (feat <= 32) return launch_split<16, 2, 1>(s, device_id, st);
+    if (feat <= 64) return launch_split<32, 2, 1>(s, device_id, st);
+    return launch_split<32, 2, 2>(s, device_id, st);
+  }
+  if (feat <= 8) return launch_split<8, 1, 1>(s, device_id, st);
+  if (feat <= 16) return launch_split<16, 1, 1>(s, device_id, st);
+  if (feat <= 32) return launch_split<32, 1, 1>(s, device_id, st);
+  if (feat <= 64) return launch_split<32, 1, 2>(s, device_id, st);
+  if (feat <= 128) return launch_split<32, 1, 4>(s, device_id, st);
+  return launch_split<32, 1, 5>(s, device_id, st);
+}
+
+}  // namespace sptir

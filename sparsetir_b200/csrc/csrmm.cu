@@ -3,14 +3,14 @@
 // like the reference's scheduled GPU kernel (examples/spmm/bench_spmm_naive.py:102-119) rows
 // without entries are written as zeros.
 //
-// Mapping: a group of LPR lanes owns 1, 2 or 4 consecutive rows and streams their stored
-// entries as one contiguous slot stream (see spmm_core.cuh); each lane keeps VPL 16-byte
-// pieces of the output row in registers and stores them when the row's last entry has been
-// consumed.  One writer per output row: no atomics, deterministic summation in CSR order.
+// Two kernels.  Matrices of a few thousand rows, and callers that promise short rows (the
+// aggregation launch of RGMS), take the row-wise kernel below: row pointer -> ids -> rows of B is
+// the shortest chain of memory round trips there is.  All others take the kernel that splits the
+// matrix by stored entries (csr_split.cu).
 #include <cstdlib>
 
 #include "common.h"
-#include "spmm_core.cuh"
+#include "vec.cuh"
 
 namespace sptir {
 namespace {
@@ -27,11 +27,17 @@ constexpr int kThreads = 256;
 // entries are one contiguous slot stream whose ids/values are read a batch of LPR ahead, and the
 // dense rows are gathered 8 at a time.  One writer per output row, CSR summation order, rows
 // without entries written as zeros.
-template <int LPR, int W>  // W floats per lane: 4 (16-byte vectors) or 8 (32-byte vectors)
+//
+// HUBS: a row of more than kLongRow entries, which one sub-warp would walk alone (a 2,000-entry row
+// of an 8,000-row graph: 100 us beside 5 us for all the others), is left to the end of the block
+// and then shared by all its sub-warps; their partial sums are added in order.
+constexpr int kLongRow = 64;
+
+template <int LPR, int W, bool HUBS>  // W floats per lane: 4 (16-byte vectors) or 8 (32-byte vectors)
 __global__ void __launch_bounds__(kThreads, 4)
 csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
                   const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int m,
-                  int feat, int rpi, int long_row) {
+                  int feat, int rpi) {
   using LV = LaneVec<W>;
   using V = typename LV::type;
   constexpr int SUBS = kThreads / LPR;
@@ -40,27 +46,31 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const unsigned mask = group_mask<LPR>();
   const long long item = static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR;
   const long long r0l = item * rpi;
-  if (r0l >= m) return;
-  const int r0 = static_cast<int>(r0l);
-  const int nr = min(rpi, m - r0);
+  if (!HUBS && r0l >= m) return;
+  const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m)));
+  const int nr = min(rpi, m - r0);  // 0 past the last row
+  __shared__ int s_long[HUBS ? SUBS * (LPR - 1) : 1];  // long rows of the block, by (sub-warp, row)
+  __shared__ int s_longs;
+  if (HUBS) {
+    if (threadIdx.x == 0) s_longs = 0;
+    __syncthreads();
+  }
   const int ptr = __ldg(indptr + r0 + min(lane, nr));  // lane j: start of row r0+j (j <= nr)
-  const int p0 = __shfl_sync(mask, ptr, 0, LPR);
-  const int nslots = __shfl_sync(mask, ptr, nr, LPR) - p0;
   const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
   const unsigned off = (blockIdx.y * LPR + lane) * (W * 4u);
   const char* bl = reinterpret_cast<const char*>(b) + off;
   char* cl = reinterpret_cast<char*>(c) + off +
              static_cast<unsigned long long>(static_cast<unsigned>(r0)) * row_bytes;
 
-  // Rows longer than long_row (hub rows) belong to the long-row launch that follows (it was
-  // given their list, and their output rows cleared, by the planning kernel).  An item that
-  // contains such rows streams the runs of ordinary rows between them, one run at a time; an
-  // item without them (the usual case) is one run.
+  // An item that contains long rows streams the runs of ordinary rows between them, one run at a
+  // time; an item without them (the usual case) is one run.
   unsigned long_rows_mask = 0;
-  if (long_row > 0) {
+  if (HUBS) {
     const int len = __shfl_down_sync(mask, ptr, 1, LPR) - ptr;
+    const bool is_long = lane < nr && len > kLongRow;
     const int shift = (threadIdx.x & 31) / LPR * LPR;
-    long_rows_mask = __ballot_sync(mask, lane < nr && len > long_row) >> shift;
+    long_rows_mask = __ballot_sync(mask, is_long) >> shift;
+    if (is_long) s_long[atomicAdd(&s_longs, 1)] = r0 + lane;
   }
   int jb = 0;
   while (jb < nr) {
@@ -132,169 +142,59 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
     }
     jb = je;
   }
-}
 
-// ---------------------------------------------------------------------------------------------
-// Hub rows.  A row of thousands of entries walked by one sub-warp would set the launch time
-// (1.5 ms for the 13,000-entry row of a 170 k-row power-law graph against 60 us for everything
-// else), and an item of a dozen 200-entry rows is a smaller tail of the same kind.  So rows of
-// more than 32 entries (measured best of 32..256 on that graph: 78 / 113 / 362 us at F = 32 / 128 /
-// 512 against 111 / 155 / 436 us at 256) are cut into chunks of kLongChunk (128) entries: a
-// planning kernel lists the chunks and clears those output rows, the main kernel leaves the rows
-// alone, and a third launch (one sub-warp per listed chunk, upper-bound grid, blocks past the
-// list end at once) adds the partial sums atomically.  Rows of up to 128 entries still have one
-// writer and CSR summation order; the order in which the chunks of a longer row are added is
-// not fixed.  Matrices below 8192 rows and 65536 entries keep the single launch.
-constexpr int kLongChunk = 128;
-
-__global__ void __launch_bounds__(kThreads)
-csr_plan_long_rows_kernel(const int32_t* __restrict__ indptr, int m, int feat, float* __restrict__ c,
-                          int* __restrict__ count, int2* __restrict__ list, int max_entries,
-                          int long_row) {
-  const int row = blockIdx.x * kThreads + threadIdx.x;
-  int len = 0;
-  if (row < m) len = __ldg(indptr + row + 1) - __ldg(indptr + row);
-  const bool is_long = len > long_row;
-  if (is_long) {
-    const int nch = (len + kLongChunk - 1) / kLongChunk;
-    const int base = atomicAdd(count, nch);
-    for (int k = 0; k < nch; ++k)
-      if (base + k < max_entries) list[base + k] = make_int2(row, k);
-  }
-  unsigned todo = __ballot_sync(0xffffffffu, is_long);
-  const int lane = threadIdx.x & 31;
-  while (todo != 0) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const int r = __shfl_sync(0xffffffffu, row, src);
-    float* dst = c + static_cast<size_t>(r) * feat;
-    for (int f = lane; f < feat; f += 32) dst[f] = 0.f;
-  }
-}
-
-template <int LPR>  // 16-byte lanes; blockIdx.y = feature tile of 4 * LPR floats
-__global__ void __launch_bounds__(kThreads, 4)
-csr_long_rows_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
-                     const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int feat,
-                     const int* __restrict__ count, const int2* __restrict__ list, int max_entries) {
-  constexpr int SUBS = kThreads / LPR;
-  constexpr int U = 8;
-  const int lane = threadIdx.x % LPR;
-  const unsigned mask = group_mask<LPR>();
-  const long long e = static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR;
-  if (e >= min(__ldg(count), max_entries)) return;
-  const int2 work = list[e];
-  const int row_begin = __ldg(indptr + work.x);
-  const int p0 = row_begin + work.y * kLongChunk;
-  const int nslots = min(kLongChunk, __ldg(indptr + work.x + 1) - p0);
-  const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
-  const unsigned off = (blockIdx.y * LPR + lane) * 16u;
-  const char* bl = reinterpret_cast<const char*>(b) + off;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < nslots; s0 += LPR) {
-    int cid = 0;
-    float av = 0.f;
-    if (s0 + lane < nslots) {
-      cid = __ldg(indices + p0 + s0 + lane);
-      av = __ldg(a + p0 + s0 + lane);
-    }
-    const int cnt = min(LPR, nslots - s0);
+  if (HUBS) {
+    __shared__ __align__(32) float s_part[SUBS][LPR * W];
+    __syncthreads();
+    const int longs = s_longs;
+    const int sub = threadIdx.x / LPR;
+    for (int k = 0; k < longs; ++k) {  // which order the rows come in changes nothing
+      const int row = s_long[k];
+      const int begin = __ldg(indptr + row), end = __ldg(indptr + row + 1);
+      V acc = LV::zero();
+      for (int e0 = begin + sub * LPR; e0 < end; e0 += SUBS * LPR) {
+        const bool live = lane < end - e0;
+        const int cid = live ? __ldg(indices + e0 + lane) : 0;
+        const float av = live ? __ldg(a + e0 + lane) : 0.f;
+        const int cnt = min(LPR, end - e0);
 #pragma unroll
-    for (int k0 = 0; k0 < LPR; k0 += U) {
-      if (k0 < cnt) {
-        float4 x[U];
+        for (int k0 = 0; k0 < LPR; k0 += U) {
+          if (k0 < cnt) {
+            V x[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const unsigned col = static_cast<unsigned>(__shfl_sync(mask, cid, k0 + u, LPR));
-          x[u] = __ldg(reinterpret_cast<const float4*>(bl + static_cast<unsigned long long>(col) * row_bytes));
-        }
+            for (int u = 0; u < U; ++u) {
+              const unsigned col = static_cast<unsigned>(__shfl_sync(mask, cid, k0 + u, LPR));
+              x[u] = LV::ldg(bl + static_cast<unsigned long long>(col) * row_bytes);
+            }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const float ak = __shfl_sync(mask, av, k0 + u, LPR);  // slots past the end carry 0
-          if (k0 + u < cnt) Vec<4>::fma(acc, ak, x[u]);
+            for (int u = 0; u < U; ++u) {
+              const float ak = __shfl_sync(mask, av, k0 + u, LPR);
+              if (k0 + u < cnt) LV::fma(acc, ak, x[u]);
+            }
+          }
         }
       }
+      LV::sts(&s_part[sub][lane * W], acc);
+      __syncthreads();
+      if (sub == 0) {
+        for (int j = 1; j < SUBS; ++j) LV::add(acc, LV::lds(&s_part[j][lane * W]));
+        LV::stcs(reinterpret_cast<char*>(c) + off + static_cast<unsigned long long>(static_cast<unsigned>(row)) * row_bytes, acc);
+      }
+      __syncthreads();
     }
   }
-  atomicAdd(reinterpret_cast<float4*>(reinterpret_cast<char*>(c) + static_cast<size_t>(work.x) * row_bytes + off), acc);
-}
-
-template <int LPR, int VPL, int VEC>
-__global__ void __launch_bounds__(kThreads)
-csrmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
-             const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int m,
-             int feat, int rows_per_item) {
-  using V = typename Vec<VEC>::type;
-  constexpr int SUBS = kThreads / LPR;
-  const int lane = threadIdx.x % LPR;
-  const unsigned mask = group_mask<LPR>();
-  const long long item = static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR;
-  const long long r0l = item * rows_per_item;
-  if (r0l >= m) return;
-  const int r0 = static_cast<int>(r0l);
-  const int r1 = min(m, r0 + rows_per_item);
-  const FeatLane<LPR, VPL, VEC> fl(feat, blockIdx.y, lane);
-  V* cv = reinterpret_cast<V*>(c);
-
-  int row = r0;
-  int row_end = __ldg(indptr + r0 + 1);
-  const int p0 = __ldg(indptr + r0);
-  const int p1 = __ldg(indptr + r1);
-  int p = p0;  // next slot to be consumed
-
-  V acc[VPL];
-#pragma unroll
-  for (int v = 0; v < VPL; ++v) acc[v] = Vec<VEC>::zero();
-
-  auto flush_finished_rows = [&]() {
-    // store every row whose last entry has been consumed (also rows without entries)
-    while (row < r1 && p >= row_end) {
-      V* dst = cv + static_cast<size_t>(row) * fl.row_vecs;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        if (fl.valid[v]) __stcs(dst + fl.off[v], acc[v]);  // written once: keep B rows in L2
-        acc[v] = Vec<VEC>::zero();
-      }
-      ++row;
-      if (row < r1) row_end = __ldg(indptr + row + 1);
-    }
-  };
-
-  flush_finished_rows();  // leading empty rows
-  auto on_done = [&](V(&)[VPL], int n) {
-    p += n;
-    flush_finished_rows();
-  };
-  const V* bv = reinterpret_cast<const V*>(b);
-  if (feat % (LPR * VPL * VEC) == 0)
-    stream_slots<LPR, VPL, VEC, true, true>(indices + p0, a + p0, p1 - p0, bv, fl, lane, mask, acc, on_done);
-  else
-    stream_slots<LPR, VPL, VEC, true, false>(indices + p0, a + p0, p1 - p0, bv, fl, lane, mask, acc, on_done);
-}
-
-template <int LPR, int VPL, int VEC>
-int launch(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-           int m, int feat, cudaStream_t stream) {
-  constexpr int SUBS = kThreads / LPR;
-  const int tile_feat = LPR * VPL * VEC;
-  // Several consecutive rows per sub-warp amortise the pipeline start-up, but only once there
-  // are enough rows to fill the machine a few times over; small matrices get one row each.
-  const long long resident_subs = static_cast<long long>(kNumSMs) * 8 * SUBS;
-  const int rows_per_item = m >= 4 * resident_subs ? 4 : (m >= 2 * resident_subs ? 2 : 1);
-  dim3 grid(ceil_div(ceil_div(m, rows_per_item), SUBS), ceil_div(feat, tile_feat));
-  csrmm_kernel<LPR, VPL, VEC><<<grid, kThreads, 0, stream>>>(a, b, c, indptr, indices, m, feat,
-                                                              rows_per_item);
-  SPTIR_LAUNCH_OK("csrmm_kernel");
-  return 0;
 }
 
 }  // namespace
 }  // namespace sptir
 
 namespace sptir {
-// The launcher behind sparsetir_csrmm_raw.  hub_rows = false: never uses the hub-row launches
-// (and so never touches the per-stream workspace) — for callers that know their rows are short
-// or that hold the workspace themselves.
+int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
+                  int m, int n, int feat, int nnz, int device_id, cudaStream_t st);
+
+// The launcher behind sparsetir_csrmm_raw.  hub_rows = false: the caller knows that its rows are
+// short, and that b and c are 16-byte aligned with feat = 64; such a call never touches the
+// per-stream workspace (the caller may hold it).
 // lane_floats: 0 = the library's default lane width, 8 = 32-byte lanes where the operands allow.
 int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
               int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats) {
@@ -306,8 +206,12 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (validate_enabled() && validate_csr("sparsetir_csrmm", indptr, m, indices, nnz, n, st) != 0) return -1;
   const bool vec4 = (feat % 4 == 0) && aligned16(b) && aligned16(c);
-  if (vec4 && static_cast<long long>(feat) * 4 < (1ll << 32) &&
-      static_cast<long long>(m) * feat * 4 < (1ll << 32) * 1024) {
+  // The row-wise kernel needs whole feature tiles.  Its share ends where the split by entries is
+  // the faster one although it has to search for its rows: 4,096 rows of 10 entries, F = 64, 4.8
+  // against 7.1 us; 16,886 power-law rows, F = 32, 23.4 (with the two launches for hub rows that
+  // it needed there) against 9.6 us.
+  const bool small = m < 8192 && nnz < 65536;
+  if (vec4 && (small || !hub_rows)) {
     // lanes per row: one per 32-byte vector when the operands allow it, else one per 16-byte
     // vector; narrowed until the n x tile slice of B that a pass over the rows gathers from fits
     // the resident part of L2 (see hyb_spmm.cu)
@@ -327,75 +231,28 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
       const long long want_items = 4ll * kNumSMs * 4 * subs;
       while (rpi > 1 && (m + rpi - 1) / rpi < want_items) rpi /= 2;
       dim3 grid(ceil_div(ceil_div(m, rpi), subs), feat / (w * lanes));
-      // hub rows get their own launches once the matrix is large enough for one of them to
-      // matter next to the cost of two more (small) launches
-      // rows longer than this go to the hub-row launches (SPARSETIR_CSR_LONG_ROW overrides)
-      static const int long_row_len = [] {
-        const char* e = std::getenv("SPARSETIR_CSR_LONG_ROW");
-        const int v = e ? std::atoi(e) : 0;
-        return v >= 32 ? v : 32;
-      }();
-      const bool long_rows = hub_rows && w == 4 && nnz > long_row_len && (m >= 8192 || nnz >= 65536);
-      int* count = nullptr;
-      int2* list = nullptr;
-      int max_entries = 0;
-      if (long_rows) {
-        max_entries = nnz / kLongChunk + nnz / long_row_len + 1;
-        char* ws = static_cast<char*>(workspace(device_id, st, 16 + static_cast<size_t>(max_entries) * sizeof(int2)));
-        if (!ws) return -1;
-        count = reinterpret_cast<int*>(ws);
-        list = reinterpret_cast<int2*>(ws + 16);
-        SPTIR_CUDA_OK(cudaMemsetAsync(count, 0, sizeof(int), st));
-        csr_plan_long_rows_kernel<<<ceil_div(m, kThreads), kThreads, 0, st>>>(indptr, m, feat, c, count, list,
-                                                                             max_entries, long_row_len);
-        SPTIR_LAUNCH_OK("csr_plan_long_rows_kernel");
-      }
-      const int long_row = long_rows ? long_row_len : 0;
-#define SPTIR_CSR_LEAN(L, WW) \
-  csrmm_lean_kernel<L, WW><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi, long_row)
+#define SPTIR_CSR_LEAN(L, WW)                                                                                   \
+  if (hub_rows)                                                                                                 \
+    csrmm_lean_kernel<L, WW, true><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi);           \
+  else                                                                                                          \
+    csrmm_lean_kernel<L, WW, false><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi)
       if (w == 8) {
-        if (lanes == 4) SPTIR_CSR_LEAN(4, 8);
-        else if (lanes == 8) SPTIR_CSR_LEAN(8, 8);
-        else if (lanes == 16) SPTIR_CSR_LEAN(16, 8);
-        else SPTIR_CSR_LEAN(32, 8);
+        if (lanes == 4) { SPTIR_CSR_LEAN(4, 8); }
+        else if (lanes == 8) { SPTIR_CSR_LEAN(8, 8); }
+        else if (lanes == 16) { SPTIR_CSR_LEAN(16, 8); }
+        else { SPTIR_CSR_LEAN(32, 8); }
       } else {
-        if (lanes == 8) SPTIR_CSR_LEAN(8, 4);
-        else if (lanes == 16) SPTIR_CSR_LEAN(16, 4);
-        else SPTIR_CSR_LEAN(32, 4);
+        if (lanes == 8) { SPTIR_CSR_LEAN(8, 4); }
+        else if (lanes == 16) { SPTIR_CSR_LEAN(16, 4); }
+        else { SPTIR_CSR_LEAN(32, 4); }
       }
 #undef SPTIR_CSR_LEAN
       SPTIR_LAUNCH_OK("csrmm_lean_kernel");
-      if (long_rows) {
-        dim3 lgrid(ceil_div(max_entries, subs), feat / (4 * lanes));
-        if (lanes == 8)
-          csr_long_rows_kernel<8><<<lgrid, kThreads, 0, st>>>(a, b, c, indptr, indices, feat, count, list, max_entries);
-        else if (lanes == 16)
-          csr_long_rows_kernel<16><<<lgrid, kThreads, 0, st>>>(a, b, c, indptr, indices, feat, count, list, max_entries);
-        else
-          csr_long_rows_kernel<32><<<lgrid, kThreads, 0, st>>>(a, b, c, indptr, indices, feat, count, list, max_entries);
-        SPTIR_LAUNCH_OK("csr_long_rows_kernel");
-      }
       return 0;
     }
   }
-  if (vec4) {
-    const int nv = feat / 4;
-    if (nv <= 8) return launch<8, 1, 4>(a, b, c, indptr, indices, m, feat, st);
-    if (nv <= 16) return launch<16, 1, 4>(a, b, c, indptr, indices, m, feat, st);
-    if (nv <= 32) return launch<32, 1, 4>(a, b, c, indptr, indices, m, feat, st);
-    // Wider rows go feature tile by feature tile (blockIdx.y, the slowest grid dimension), the
-    // tile chosen so that the n x tile slice of B a pass gathers from stays resident in L2.
-    const size_t l2_budget = 56u << 20;  // what stays resident of data that every SM reads
-    const size_t slice_128 = static_cast<size_t>(n) * 128 * sizeof(float);
-    if (nv > 64 && 4 * slice_128 <= l2_budget)
-      return launch<32, 4, 4>(a, b, c, indptr, indices, m, feat, st);
-    if (2 * slice_128 <= l2_budget) return launch<32, 2, 4>(a, b, c, indptr, indices, m, feat, st);
-    return launch<32, 1, 4>(a, b, c, indptr, indices, m, feat, st);
-  }
-  if (feat <= 8) return launch<8, 1, 1>(a, b, c, indptr, indices, m, feat, st);
-  if (feat <= 16) return launch<16, 1, 1>(a, b, c, indptr, indices, m, feat, st);
-  if (feat <= 32) return launch<32, 1, 1>(a, b, c, indptr, indices, m, feat, st);
-  return launch<32, 4, 1>(a, b, c, indptr, indices, m, feat, st);  // tiles of 128 features
+  if (!hub_rows) return fail("sparsetir_csrmm: short-row call with operands that are not whole tiles");
+  return csr_split_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, st);
 }
 
 int csrmm_impl(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,

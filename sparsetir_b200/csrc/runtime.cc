@@ -103,6 +103,13 @@ int peer_table(const char* fn, const void* own, int n_peers, void* const* peers,
   return 0;
 }
 
+bool workspace_fits(int device_id, cudaStream_t stream, size_t bytes, size_t zeroed_bytes) {
+  std::lock_guard<std::mutex> lock(g_ws_mutex);
+  const std::pair<int, cudaStream_t> key{device_id, stream};
+  const auto a = g_ws[0].find(key), b = g_ws[1].find(key);
+  return a != g_ws[0].end() && a->second.bytes >= bytes && b != g_ws[1].end() && b->second.bytes >= zeroed_bytes;
+}
+
 void* workspace(int device_id, cudaStream_t stream, size_t bytes) {
   return grow(0, device_id, stream, bytes);
 }

@@ -98,7 +98,46 @@ __device__ __forceinline__ float dot8(const Pack4& x, const Pack4& y) {
 }
 
 // A lane's piece of a dense row: 4 floats (one 16-byte vector) or 8 floats (one 32-byte vector).
+// 1 or 2 floats where the row length or the alignment of the operands allows no more.
 template <int W> struct LaneVec;
+template <> struct LaneVec<1> {
+  using type = float;
+  static __device__ __forceinline__ float zero() { return 0.f; }
+  static __device__ __forceinline__ float ldg(const void* p) { return __ldg(reinterpret_cast<const float*>(p)); }
+  static __device__ __forceinline__ void stcs(void* p, float v) { __stcs(reinterpret_cast<float*>(p), v); }
+  static __device__ __forceinline__ void fma(float& acc, float w, float x) { acc = fmaf(w, x, acc); }
+  static __device__ __forceinline__ void atomic_add(void* p, float v) { atomicAdd(reinterpret_cast<float*>(p), v); }
+  static __device__ __forceinline__ float ldcg(const void* p) { return __ldcg(reinterpret_cast<const float*>(p)); }
+  static __device__ __forceinline__ void stcg(void* p, float v) { __stcg(reinterpret_cast<float*>(p), v); }
+  static __device__ __forceinline__ void add(float& acc, float x) { acc += x; }
+  static __device__ __forceinline__ void sts(float* p, float v) { *p = v; }
+  static __device__ __forceinline__ float lds(const float* p) { return *p; }
+  static __device__ __forceinline__ void st(void* p, const float& v) { *reinterpret_cast<float*>(p) = v; }
+  // selects instead of a branch, for accumulators of sub-warps that run in step
+  static __device__ __forceinline__ void zero_if(float& acc, bool z) {
+    acc = z ? 0.f : acc;
+  }
+};
+template <> struct LaneVec<2> {
+  using type = float2;
+  static __device__ __forceinline__ float2 zero() { return make_float2(0.f, 0.f); }
+  static __device__ __forceinline__ float2 ldg(const void* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+  static __device__ __forceinline__ void stcs(void* p, const float2& v) { __stcs(reinterpret_cast<float2*>(p), v); }
+  static __device__ __forceinline__ void fma(float2& acc, float w, const float2& x) {
+    acc.x = fmaf(w, x.x, acc.x); acc.y = fmaf(w, x.y, acc.y);
+  }
+  static __device__ __forceinline__ void atomic_add(void* p, const float2& v) { atomicAdd(reinterpret_cast<float2*>(p), v); }
+  static __device__ __forceinline__ float2 ldcg(const void* p) { return __ldcg(reinterpret_cast<const float2*>(p)); }
+  static __device__ __forceinline__ void stcg(void* p, const float2& v) { __stcg(reinterpret_cast<float2*>(p), v); }
+  static __device__ __forceinline__ void add(float2& acc, const float2& x) { acc.x += x.x; acc.y += x.y; }
+  static __device__ __forceinline__ void sts(float* p, const float2& v) { *reinterpret_cast<float2*>(p) = v; }
+  static __device__ __forceinline__ float2 lds(const float* p) { return *reinterpret_cast<const float2*>(p); }
+  static __device__ __forceinline__ void st(void* p, const float2& v) { *reinterpret_cast<float2*>(p) = v; }
+  // selects instead of a branch, for accumulators of sub-warps that run in step
+  static __device__ __forceinline__ void zero_if(float2& acc, bool z) {
+    acc.x = z ? 0.f : acc.x; acc.y = z ? 0.f : acc.y;
+  }
+};
 template <> struct LaneVec<4> {
   using type = float4;
   static __device__ __forceinline__ float4 zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
@@ -115,6 +154,11 @@ template <> struct LaneVec<4> {
   // shared memory (16-byte aligned)
   static __device__ __forceinline__ void sts(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
   static __device__ __forceinline__ float4 lds(const float* p) { return *reinterpret_cast<const float4*>(p); }
+  static __device__ __forceinline__ void st(void* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+  // selects instead of a branch, for accumulators of sub-warps that run in step
+  static __device__ __forceinline__ void zero_if(float4& acc, bool z) {
+    acc.x = z ? 0.f : acc.x; acc.y = z ? 0.f : acc.y; acc.z = z ? 0.f : acc.z; acc.w = z ? 0.f : acc.w;
+  }
 };
 template <> struct LaneVec<8> {
   using type = Pack4;
@@ -157,6 +201,15 @@ template <> struct LaneVec<8> {
     Pack4 r;
     r.q[0] = d[0].x; r.q[1] = d[0].y; r.q[2] = d[1].x; r.q[3] = d[1].y;
     return r;
+  }
+  // shared or global memory: in two halves, because 32-byte accesses exist for global memory only
+  static __device__ __forceinline__ void st(void* p, const Pack4& v) {
+    reinterpret_cast<ulonglong2*>(p)[0] = make_ulonglong2(v.q[0], v.q[1]);
+    reinterpret_cast<ulonglong2*>(p)[1] = make_ulonglong2(v.q[2], v.q[3]);
+  }
+  static __device__ __forceinline__ void zero_if(Pack4& acc, bool z) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc.q[i] = z ? 0ull : acc.q[i];
   }
 };
 

@@ -1,0 +1,68 @@
+"""CSR SpMM split by stored entries: rows that cross sub-warps, blocks and feature tiles, runs of
+rows without entries, and every vector width, against a float64 product."""
+import numpy as np
+import pytest
+import torch
+
+from sparsetir_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# degree sequences; all but the first have 8,192 rows or 65,536 entries, where the split begins
+SHAPES = {
+    "hubs_in_a_small_matrix": [0, 3, 1500, 65, 64, 0, 2, 900] + [5] * 700 + [700],
+    "one_row_of_everything": [0] * 40 + [70_001] + [0] * 9000,
+    "rows_longer_than_a_block": [9000, 1, 0, 17_000, 2] * 4,
+    "empty_runs": ([0] * 5000 + [1] * 40) * 5 + [0] * 3000,
+    "single_entries": [1] * 70_003,
+    "mixed": [0, 1, 2, 300, 7, 0, 0, 33, 32, 31] * 1700,
+}
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+@pytest.mark.parametrize("feat,offset", [(32, 0), (64, 0), (100, 0), (300, 0), (41, 0), (46, 0), (299, 0), (130, 0), (1, 0),
+                                         (64, 1), (128, 2)])
+def test_rows_meet_across_sub_warps_and_blocks(cuda_device, shape, feat, offset):
+    deg = np.asarray(SHAPES[shape], np.int64)
+    m, n, nnz = len(deg), 4001, int(deg.sum())
+    rng = np.random.default_rng(feat)
+    indptr = np.zeros(m + 1, np.int32)
+    indptr[1:] = np.cumsum(deg)
+    dev = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    cols = dev(rng.integers(0, n, nnz).astype(np.int32))
+    vals = dev(rng.uniform(-1, 1, nnz).astype(np.float32))
+    x = dev(rng.uniform(-1, 1, n * feat + offset).astype(np.float32))[offset:]  # offset: other alignments
+    y = torch.full((m * feat + offset,), float("nan"), device=cuda_device)[offset:]
+    ptr = dev(indptr)
+    ops.csrmm(vals, x, y, ptr, cols)
+    rows = torch.repeat_interleave(torch.arange(m, device=cuda_device), dev(deg))
+    want = torch.zeros(m, feat, dtype=torch.float64, device=cuda_device)
+    mag = torch.zeros(m, feat, dtype=torch.float64, device=cuda_device)
+    for p in range(0, nnz, 20_000):
+        part = vals[p:p + 20_000, None].double() * x.view(n, feat)[cols[p:p + 20_000].long()].double()
+        want.index_add_(0, rows[p:p + 20_000], part)
+        mag.index_add_(0, rows[p:p + 20_000], part.abs())
+    # an fp32 sum of d products in any order: at most d half-ulps of the sum of magnitudes
+    bound = mag * (dev(deg)[:, None].double() + 1) * 2.0 ** -24
+    assert bool(((y.view(m, feat).double() - want).abs() <= bound).all())
+    again = y.clone()
+    ops.csrmm(vals, x, y, ptr, cols)
+    assert torch.equal(again, y)  # one writer and one order: the same bits
+
+
+def test_first_call_on_a_stream_can_be_captured(cuda_device):
+    m, feat = 9000, 41
+    ptr = torch.arange(0, 8 * m + 1, 8, dtype=torch.int32, device=cuda_device)
+    cols = torch.randint(0, m, (8 * m,), dtype=torch.int32, device=cuda_device)
+    vals, x = torch.rand(8 * m, device=cuda_device), torch.rand(m * feat, device=cuda_device)
+    want, got = torch.empty(m * feat, device=cuda_device), torch.empty(m * feat, device=cuda_device)
+    ops.csrmm(vals, x, want, ptr, cols)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        ops.csrmm(vals, x, got, ptr, cols)
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
