@@ -172,8 +172,11 @@ hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* __restrict__ b
 }
 
 // ---------------------------------------------------------------------------------------------
-// Lean kernel: the fast path for 16-byte aligned operands, whole feature tiles and ELL widths
-// of 1, 2, 4 or a multiple of 8 (every power-of-two bucket list).  Written for instruction
+// Lean kernel: ELL widths of 1, 2, 4 or a multiple of 8 (every power-of-two bucket list), any
+// feature count and alignment.  Feature counts that are not whole tiles and rows that are not whole
+// 16-byte vectors run it with predicated or narrower vectors instead of the kernels below (F = 100
+// on a 100 k-node power-law graph 58 -> 35 us, F = 41 on 60 k nodes 50 -> 16 us, F = 184 on 194 k
+// nodes with 36 entries per row in two column partitions 1065 -> 566 us).  Written for instruction
 // economy — the gathers come from L2 at well over 10 TB/s if, and only if, the warp spends its
 // issue slots on loads: per stored slot the loop executes one shuffle + one address + one
 // 16-byte load, then one shuffle + four FMAs; row ends sit at compile-time positions of the
@@ -196,23 +199,24 @@ constexpr int kFlagAtomic = static_cast<int>(0x80000000u);  // add atomically in
 
 // row_flag(g): flag word of ELL row g (called by the lane that will hold it)
 // row_end(acc, flag word): all lanes of the sub-warp, after the last slot of an ELL row
-template <int LPR, int WM, int W, class RowFlag, class RowEnd>  // WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
+template <int LPR, int WM, int W, int VPL, bool WHOLE, class RowFlag, class RowEnd>  // WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
 __device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
                                           const float* __restrict__ wts, int r0, int nr, int nslots,
                                           int per_row, const char* __restrict__ bl,
-                                          unsigned row_bytes, int lane, unsigned mask,
-                                          RowFlag&& row_flag, RowEnd&& row_end) {
-  using LV = LaneVec<W>;
-  using V = typename LV::type;
-  constexpr int U = (32 / W) < LPR ? (32 / W) : LPR;  // gathered rows in flight: 32 registers
-  // address of this lane's vector in dense row `col`: one 32x32->64 multiply-add
+                                          unsigned row_bytes, const LaneTile<LPR, W, VPL, WHOLE>& lt, int lane,
+                                          unsigned mask, RowFlag&& row_flag, RowEnd&& row_end) {
+  using LT = LaneTile<LPR, W, VPL, WHOLE>;
+  using V = typename LT::Piece;
+  constexpr int kU = W == 8 ? 4 : W == 4 ? 8 : VPL == 1 ? 16 : VPL == 2 ? 8 : 4;  // gathered rows in flight
+  constexpr int U = WM == 8 && kU > 8 ? 8 : (kU < LPR ? kU : LPR);
+  // address of dense row `col`: one 32x32->64 multiply-add
   auto vec_of = [&](const char* base, int col) -> const char* {
     return base + static_cast<unsigned long long>(static_cast<unsigned>(col)) * row_bytes;
   };
   static_assert(LPR % U == 0, "a batch is a whole number of chunks");
   constexpr int RPB = WM < 8 ? LPR / WM : 0;  // ELL rows that end inside one batch (narrow rows)
 
-  V acc = LV::zero();
+  V acc = LT::zero();
   int c = 0, rf = 0;
   float a = 0.f;
   if (lane < nslots) {
@@ -241,10 +245,10 @@ __device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
         V x[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          x[u] = LV::ldg(vec_of(bl, __shfl_sync(mask, c, k0 + u, LPR)));
+          x[u] = lt.ldg(vec_of(bl, __shfl_sync(mask, c, k0 + u, LPR)));
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          LV::fma(acc, __shfl_sync(mask, a, k0 + u, LPR), x[u]);
+          LT::fma(acc, __shfl_sync(mask, a, k0 + u, LPR), x[u]);
           if (WM < 8 && (k0 + u + 1) % WM == 0)
             row_end(acc, __shfl_sync(mask, rf, (k0 + u) / WM, LPR));
         }
@@ -264,13 +268,13 @@ __device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
           V x[U];
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            x[u] = LV::ldg(vec_of(bl, __shfl_sync(mask, c, k0 + u, LPR)));  // dead slots: column 0
+            x[u] = lt.ldg(vec_of(bl, __shfl_sync(mask, c, k0 + u, LPR)));  // dead slots: column 0
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const float ak = __shfl_sync(mask, a, k0 + u, LPR);
             const int rfe = (WM < 8) ? __shfl_sync(mask, rf, (k0 + u) / WM, LPR) : 0;
             if (k0 + u < cnt) {
-              LV::fma(acc, ak, x[u]);
+              LT::fma(acc, ak, x[u]);
               if (WM < 8 && (k0 + u + 1) % WM == 0) row_end(acc, rfe);
             }
           }
@@ -304,11 +308,12 @@ struct LeanArgs {
 
 // The one store of a finished piece of an output row: into this GPU's C and, when the call has
 // peers, into every peer's copy (plain stores over NVLink; nothing waits on them).
-template <int W>
-__device__ __forceinline__ void store_out(char* p, const typename LaneVec<W>::type& v, const PeerOut* po) {
-  LaneVec<W>::stcs(p, v);
+template <int LPR, int W, int VPL, bool WHOLE>
+__device__ __forceinline__ void store_out(const LaneTile<LPR, W, VPL, WHOLE>& lt, char* row, const LanePiece<W, VPL>& v,
+                                          const PeerOut* po) {
+  lt.stcs(row, v);
   if (po != nullptr)
-    for (int k = 0; k < po->n; ++k) LaneVec<W>::stcg(p + po->delta[k], v);
+    for (int k = 0; k < po->n; ++k) lt.stcg(row + po->delta[k], v);
 }
 
 // Bits of `pred` over the LPR lanes of this thread's sub-warp, lane 0 of the sub-warp in bit 0.
@@ -326,41 +331,41 @@ __device__ __forceinline__ unsigned sub_ballot(unsigned mask, bool pred) {
 // sub-warp.  A piece is the part of a run of equal row ids that lies inside one work item
 // (items hold `rpi` consecutive ELL rows; rpi = 1 for wide buckets).  Pieces are numbered in
 // ELL-row order; piece k keeps its partial sum in the scratch row of its first ELL row.
-template <int LPR, int W>
-__device__ __noinline__ void finish_split_row(typename LaneVec<W>::type acc,
+template <int LPR, int W, int VPL, bool WHOLE>
+__device__ __noinline__ void finish_split_row(const LaneTile<LPR, W, VPL, WHOLE> lt, LanePiece<W, VPL> acc,
                                               const int32_t* __restrict__ rows, int nrows, int g,
-                                              int rpi, int rid, int part_base, char* pl, char* cl,
+                                              int rpi, int rid, int part_base, char* part, char* c,
                                               unsigned* counters, unsigned row_bytes, int lane,
                                               unsigned mask, const PeerOut* po) {
-  using LV = LaneVec<W>;
+  using LT = LaneTile<LPR, W, VPL, WHOLE>;
   constexpr unsigned kFull = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u);
   int first = g, last = g;
   while (true) {  // LPR ELL rows per step, backwards then forwards
     const int idx = first - 1 - lane;
-    const unsigned bits = sub_ballot<LPR>(mask, idx >= 0 && __ldg(rows + idx) == rid);
+    const unsigned bits = sub_ballot<LPR>(mask, idx >= 0 && __ldg(rows + max(idx, 0)) == rid);
     const int n = bits == kFull ? LPR : __ffs(~bits) - 1;
     first -= n;
     if (n < LPR) break;
   }
   while (true) {
     const int idx = last + 1 + lane;
-    const unsigned bits = sub_ballot<LPR>(mask, idx < nrows && __ldg(rows + idx) == rid);
+    const unsigned bits = sub_ballot<LPR>(mask, idx < nrows && __ldg(rows + min(idx, nrows - 1)) == rid);
     const int n = bits == kFull ? LPR : __ffs(~bits) - 1;
     last += n;
     if (n < LPR) break;
   }
   const int item0 = first / rpi;
   const int npieces = last / rpi - item0 + 1;
-  char* dst = cl + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes;
+  char* dst = c + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes;
   if (npieces == 1) {  // the whole run lies inside this item
-    store_out<W>(dst, acc, po);
+    store_out(lt, dst, acc, po);
     return;
   }
   const int mine = max(first, g / rpi * rpi);
   auto part_of = [&](int ell_row) -> char* {
-    return pl + static_cast<unsigned long long>(static_cast<unsigned>(part_base + ell_row)) * row_bytes;
+    return part + static_cast<unsigned long long>(static_cast<unsigned>(part_base + ell_row)) * row_bytes;
   };
-  LV::stcg(part_of(mine), acc);
+  lt.stcg(part_of(mine), acc);
   __threadfence();
   __syncwarp(mask);
   unsigned* counter = counters + static_cast<size_t>(part_base + first) * gridDim.y + blockIdx.y;
@@ -371,49 +376,118 @@ __device__ __noinline__ void finish_split_row(typename LaneVec<W>::type acc,
   // last piece to arrive: every other piece's partial sum is visible
   if (lane == 0) *counter = 0u;
   __threadfence();
-  typename LV::type sum = LV::ldcg(part_of(first));
-  for (int k = 1; k < npieces; ++k) LV::add(sum, LV::ldcg(part_of((item0 + k) * rpi)));
-  store_out<W>(dst, sum, po);
+  typename LT::Piece sum = lt.ldcg(part_of(first));
+  for (int k = 1; k < npieces; ++k) LT::add(sum, lt.ldcg(part_of((item0 + k) * rpi)));
+  store_out(lt, dst, sum, po);
+}
+
+// The same for an ELL row wide enough to be shared by all the sub-warps of this warp (one ELL row
+// per piece): the whole warp takes part.  `before` and `behind` are the row ids of the 32 ELL rows
+// on either side, requested before the row was gathered, so that the run of equal ids is known
+// without another trip to memory; the partial sums of the run are read by all sub-warps at once.
+// On the 169 k-node power-law graph at F = 32 the two serial walks (over the ids, over the 26
+// pieces of the largest row) were the last 8 us of a 21 us launch.
+template <int LPR, int W, int VPL, bool WHOLE>
+__device__ __noinline__ void finish_split_row_warp(const LaneTile<LPR, W, VPL, WHOLE> lt, LanePiece<W, VPL> acc,
+                                                   const int32_t* __restrict__ rows, int nrows, int g,
+                                                   int rid, int before, int behind, int part_base,
+                                                   char* part, char* c, unsigned* counters,
+                                                   unsigned row_bytes, const PeerOut* po) {
+  using LT = LaneTile<LPR, W, VPL, WHOLE>;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int NW = 32 / LPR;
+  const int wlane = threadIdx.x & 31, lane = wlane % LPR, sub = wlane / LPR;
+  int first = g, last = g;
+  while (true) {
+    const unsigned bits = __ballot_sync(kAll, first - 1 - wlane >= 0 && before == rid);
+    const int n = bits == kAll ? 32 : __ffs(~bits) - 1;
+    first -= n;
+    if (n < 32) break;
+    before = __ldg(rows + max(first - 1 - wlane, 0));
+  }
+  while (true) {
+    const unsigned bits = __ballot_sync(kAll, last + 1 + wlane < nrows && behind == rid);
+    const int n = bits == kAll ? 32 : __ffs(~bits) - 1;
+    last += n;
+    if (n < 32) break;
+    behind = __ldg(rows + min(last + 1 + wlane, nrows - 1));
+  }
+  char* dst = c + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes;
+  if (first == last) {  // not split after all
+    if (sub == 0) store_out(lt, dst, acc, po);
+    return;
+  }
+  auto part_of = [&](int ell_row) -> char* {
+    return part + static_cast<unsigned long long>(static_cast<unsigned>(part_base + ell_row)) * row_bytes;
+  };
+  if (sub == 0) lt.stcg(part_of(g), acc);
+  __threadfence();
+  __syncwarp();
+  unsigned* counter = counters + static_cast<size_t>(part_base + first) * gridDim.y + blockIdx.y;
+  unsigned seen = 0;
+  if (wlane == 0) seen = atomicAdd(counter, 1u);
+  seen = __shfl_sync(kAll, seen, 0);
+  if (seen != static_cast<unsigned>(last - first)) return;
+  // last piece to arrive: every other piece's partial sum is visible
+  if (wlane == 0) *counter = 0u;
+  __threadfence();
+  typename LT::Piece sum = LT::zero();
+  constexpr int G = VPL * W >= 8 ? 4 : 8;
+  for (int k0 = first + sub; k0 <= last; k0 += NW * G) {
+    typename LT::Piece x[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) x[u] = lt.ldcg(part_of(min(k0 + u * NW, last)));
+#pragma unroll
+    for (int u = 0; u < G; ++u)
+      if (k0 + u * NW <= last) LT::add(sum, x[u]);
+  }
+#pragma unroll
+  for (int o = LPR; o < 32; o *= 2)
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) LaneVec<W>::add_xor(sum.v[v], o);
+  if (sub == 0) store_out(lt, dst, sum, po);
 }
 
 // A narrow item of the widest bucket that holds ELL rows of a split row (rare: only bucket lists
 // whose last width is small put split rows into a narrow bucket).  Plain loop, one ELL row at a
 // time; consecutive ELL rows of the same output row inside the item are added up first.
-template <int LPR, int W>
-__device__ __noinline__ void split_item(const int32_t* __restrict__ cols, const float* __restrict__ wts,
-                                        const int32_t* __restrict__ rows, int nrows, int r0, int nr,
-                                        int width, int rpi, int part_base, const char* __restrict__ bl,
-                                        char* pl, char* cl, unsigned* counters, unsigned row_bytes,
-                                        int lane, unsigned mask, const PeerOut* po) {
-  using LV = LaneVec<W>;
-  typename LV::type acc = LV::zero();
+template <int LPR, int W, int VPL, bool WHOLE>
+__device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, const int32_t* __restrict__ cols,
+                                        const float* __restrict__ wts, const int32_t* __restrict__ rows,
+                                        int nrows, int r0, int nr, int width, int rpi, int part_base,
+                                        const char* __restrict__ b, char* part, char* c,
+                                        unsigned* counters, unsigned row_bytes, int lane, unsigned mask,
+                                        const PeerOut* po) {
+  using LT = LaneTile<LPR, W, VPL, WHOLE>;
+  typename LT::Piece acc = LT::zero();
   for (int j = 0; j < nr; ++j) {
     const int g = r0 + j;
     for (int s = 0; s < width; ++s) {
       const int col = __ldg(cols + j * width + s);
       const float a = __ldg(wts + j * width + s);
-      LV::fma(acc, a, LV::ldg(bl + static_cast<unsigned long long>(static_cast<unsigned>(col)) * row_bytes));
+      LT::fma(acc, a, lt.ldg(b + static_cast<unsigned long long>(static_cast<unsigned>(col)) * row_bytes));
     }
     const int rid = __ldg(rows + g);
     const bool next_same = g + 1 < nrows && __ldg(rows + g + 1) == rid;
     if (next_same && j + 1 < nr) continue;  // the next ELL row of this item continues the row
     if (next_same || (g > 0 && __ldg(rows + g - 1) == rid))
-      finish_split_row<LPR, W>(acc, rows, nrows, g, rpi, rid, part_base, pl, cl, counters, row_bytes, lane, mask,
-                               po);
+      finish_split_row(lt, acc, rows, nrows, g, rpi, rid, part_base, part, c, counters, row_bytes, lane, mask, po);
     else
-      store_out<W>(cl + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes, acc, po);
-    acc = LV::zero();
+      store_out(lt, c + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes, acc, po);
+    acc = LT::zero();
   }
 }
 
-template <int LPR, int W, bool PEERS>
+// blockIdx.y = feature tile of LPR * W * VPL floats; the last one may be partly filled
+template <int LPR, int W, int VPL, bool WHOLE, bool PEERS>
 __global__ void __launch_bounds__(kThreads, 8)
 hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant__ LeanArgs la) {
-  using LV = LaneVec<W>;
-  using V = typename LV::type;
+  using LT = LaneTile<LPR, W, VPL, WHOLE>;
+  using V = typename LT::Piece;
   const PeerOut* po = PEERS ? &la.peers : nullptr;
   constexpr int SUBS = kThreads / LPR;
-  __shared__ __align__(32) float s_part[SUBS][LPR * W];  // wide rows: partial sums of the spans
+  constexpr int NW = 32 / LPR;
+  __shared__ __align__(32) float s_part[SUBS][LT::kFloats];  // wide rows: partial sums of the spans
   const int lane = threadIdx.x % LPR;
   const int sub = threadIdx.x / LPR;
   const unsigned mask = group_mask<LPR>();
@@ -422,10 +496,10 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   const int rpi = tb.rows_per_item[q], spr = tb.chunks_per_row[q];
   const int part_base = tb.part_base[q];
   const unsigned stride = static_cast<unsigned>(la.feat) * 4u;  // bytes per dense row
-  const unsigned off = (blockIdx.y * LPR + lane) * (W * 4u);  // this lane's piece of the tile
-  const char* bl = reinterpret_cast<const char*>(la.b) + off;
-  char* cl = reinterpret_cast<char*>(la.c) + off;
-  char* pl = reinterpret_cast<char*>(la.part) + off;
+  const LT lt(la.feat, blockIdx.y, lane);
+  const char* bl = reinterpret_cast<const char*>(la.b);
+  char* cl = reinterpret_cast<char*>(la.c);
+  char* pl = reinterpret_cast<char*>(la.part);
   const int32_t* rows = tb.rows[q];
   if (rows == nullptr) cl += static_cast<size_t>(tb.row_base[q]) * stride;
   const bool all_atomic = la.all_atomic != 0;
@@ -446,8 +520,8 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
       bool any = false;
       for (int j = lane; j < nr; j += LPR) any = any || is_split_row(rows, r0 + j, nrows, __ldg(rows + r0 + j));
       if (sub_ballot<LPR>(mask, any) != 0u) {
-        split_item<LPR, W>(tb.cols[q] + first, tb.w[q] + first, rows, nrows, r0, nr, width, rpi, part_base,
-                           bl, pl, cl, la.counters, stride, lane, mask, po);
+        split_item(lt, tb.cols[q] + first, tb.w[q] + first, rows, nrows, r0, nr, width, rpi, part_base,
+                   bl, pl, cl, la.counters, stride, lane, mask, po);
         return;
       }
     }
@@ -456,17 +530,17 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
       return row_id(rows, g, 0) | (all_atomic ? kFlagAtomic : 0);
     };
     auto row_end = [&](V& acc, int rf) {
-      if (rf < 0) LV::atomic_add(y_of(rf & 0x7fffffff), acc);
-      else store_out<W>(y_of(rf), acc, po);  // written once: do not displace B rows in L2
-      acc = LV::zero();
+      if (rf < 0) lt.atomic_add(y_of(rf & 0x7fffffff), acc);
+      else store_out(lt, y_of(rf), acc, po);  // written once: do not displace B rows in L2
+      acc = LT::zero();
     };
     const int32_t* cols = tb.cols[q] + first;
     const float* wts = tb.w[q] + first;
     const int nslots = nr * width;
-    if (width == 1) lean_item<LPR, 1, W>(cols, wts, r0, nr, nslots, width, bl, stride, lane, mask, row_flag, row_end);
-    else if (width == 2) lean_item<LPR, 2, W>(cols, wts, r0, nr, nslots, width, bl, stride, lane, mask, row_flag, row_end);
-    else if (width == 4) lean_item<LPR, 4, W>(cols, wts, r0, nr, nslots, width, bl, stride, lane, mask, row_flag, row_end);
-    else lean_item<LPR, 8, W>(cols, wts, r0, nr, nslots, width, bl, stride, lane, mask, row_flag, row_end);
+    if (width == 1) lean_item<LPR, 1, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
+    else if (width == 2) lean_item<LPR, 2, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
+    else if (width == 4) lean_item<LPR, 4, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
+    else lean_item<LPR, 8, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
     return;
   }
 
@@ -477,28 +551,39 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   const bool live = rl < nrows;
   const int r = live ? static_cast<int>(rl) : 0;
   const int span = ((width + spr - 1) / spr + 7) & ~7;  // slots per span, a multiple of 8
-  V total = LV::zero();
+  // all sub-warps of the first warp of an ELL row belong to it: that warp finishes the row
+  const bool by_warp = spr >= NW && !all_atomic && part_base >= 0;
+  int rid = 0, before = 0, behind = 0;
+  if (live && part < NW) {
+    rid = row_id(rows, r, 0);
+    if (by_warp) {
+      before = __ldg(rows + max(r - 1 - static_cast<int>(threadIdx.x & 31), 0));
+      behind = __ldg(rows + min(r + 1 + static_cast<int>(threadIdx.x & 31), nrows - 1));
+    }
+  }
+  V total = LT::zero();
   if (live && part * span < width) {
     const int s0 = part * span;
     const int nslots = min(span, width - s0);
     const size_t first = static_cast<size_t>(r) * width + s0;
     auto no_flag = [](int) -> int { return 0; };
     auto keep = [&](V& acc, int) { total = acc; };
-    lean_item<LPR, 8, W>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lane, mask,
-                         no_flag, keep);
+    lean_item<LPR, 8, W, VPL, WHOLE>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lt, lane, mask,
+                              no_flag, keep);
   }
-  if (part != 0) LV::sts(&s_part[sub][lane * W], total);
+  if (part != 0) LT::sts(s_part[sub], lane, total);
   __syncthreads();
-  if (!live || part != 0) return;
-  for (int k = 1; k < spr; ++k) LV::add(total, LV::lds(&s_part[sub + k][lane * W]));
-  const int rid = row_id(rows, r, 0);
-  if (all_atomic) {
-    LV::atomic_add(y_of(rid), total);
+  if (!live || part >= NW || (part != 0 && !by_warp)) return;
+  if (part == 0)
+    for (int k = 1; k < spr; ++k) LT::add(total, LT::lds(s_part[sub + k], lane));
+  if (by_warp) {
+    finish_split_row_warp(lt, total, rows, nrows, r, rid, before, behind, part_base, pl, cl, la.counters, stride, po);
+  } else if (all_atomic) {
+    lt.atomic_add(y_of(rid), total);
   } else if (part_base >= 0 && is_split_row(rows, r, nrows, rid)) {
-    finish_split_row<LPR, W>(total, rows, nrows, r, 1, rid, part_base, pl, cl, la.counters, stride, lane, mask,
-                             po);
+    finish_split_row(lt, total, rows, nrows, r, 1, rid, part_base, pl, cl, la.counters, stride, lane, mask, po);
   } else {
-    store_out<W>(y_of(rid), total, po);
+    store_out(lt, y_of(rid), total, po);
   }
 }
 
@@ -683,7 +768,7 @@ long long plan_blocks_lean(HybTable& tb, int subs) {
 // reads (measured: about half of the 126 MB), because re-reading the index arrays once per tile
 // costs little next to re-fetching B rows from HBM.
 int lanes_per_row_impl(int feat, bool vec4, int n, int lane_w) {
-  const int units = vec4 ? feat / lane_w : feat;
+  const int units = vec4 ? ceil_div(feat, lane_w) : feat;
   const int min_lanes = lane_w == 8 ? 4 : 8;
   int lanes = units <= min_lanes ? min_lanes : (units <= 8 ? 8 : (units <= 16 ? 16 : 32));
   if (vec4) {
@@ -703,8 +788,9 @@ int lanes_per_row_impl(int feat, bool vec4, int n, int lane_w) {
       const int v = e ? std::atoi(e) : -1;
       return v >= 0 ? v : 4;
     }();
-    if (lanes > min_lanes && feat % (min_lanes * lane_w) == 0 && feat / (min_lanes * lane_w) <= narrow_passes)
-      lanes = min_lanes;
+    if (lanes > min_lanes && ceil_div(feat, min_lanes * lane_w) <= narrow_passes) lanes = min_lanes;
+    // narrower too where a quarter of the lanes would lie past the end of the row
+    while (lanes > min_lanes && ceil_div(units, lanes) * lanes * 4 > units * 5) lanes /= 2;
   }
   return lanes;
 }
@@ -724,36 +810,60 @@ long long plan_blocks(HybTable& tb, int subs) {
   return blocks;
 }
 
-template <int LPR, int W>
-int launch_lean(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
+template <int LPR, int W, int VPL, bool WHOLE>
+int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
+  const int tiles = ceil_div(la.feat, W * LPR * VPL);
   long long slots = 0;
   for (int q = 0; q < tb.nb; ++q) slots += static_cast<long long>(tb.nrows[q]) * tb.width[q];
-  plan_items_lean(tb, lean_item_slots(LPR, W, la.feat / (W * LPR), slots), kThreads / LPR);
+  plan_items_lean(tb, lean_item_slots(LPR, W, tiles, slots), kThreads / LPR);
   const long long blocks = plan_blocks_lean(tb, kThreads / LPR);
   if (blocks < 0) return fail("sparsetir_hyb_spmm: too many thread blocks");
-  dim3 grid(static_cast<unsigned>(blocks), la.feat / (W * LPR));
+  dim3 grid(static_cast<unsigned>(blocks), tiles);
   if (la.peers.n > 0) {
-    if constexpr (W == 4)
-      hyb_spmm_lean_kernel<LPR, W, true><<<grid, kThreads, 0, stream>>>(tb, la);
+    if constexpr (W == 4 && WHOLE)
+      hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true><<<grid, kThreads, 0, stream>>>(tb, la);
     else
-      return fail("sparsetir_hyb_spmm_peers: no 32-byte-lane form");  // the dispatcher picks 16-byte lanes
+      return fail("sparsetir_hyb_spmm_peers: whole tiles of 16-byte lanes only");  // the dispatcher picks them
   } else {
-    hyb_spmm_lean_kernel<LPR, W, false><<<grid, kThreads, 0, stream>>>(tb, la);
+    hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, false><<<grid, kThreads, 0, stream>>>(tb, la);
   }
   SPTIR_LAUNCH_OK("hyb_spmm_lean_kernel");
   return 0;
 }
 
+// Whole tiles get a kernel of their own: with predicated vectors F = 512 takes 195 us on the
+// 169 k-node graph instead of 186.
+template <int LPR, int W, int VPL>
+int launch_lean(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
+  if constexpr (W >= 4)
+    if (la.feat % (LPR * W * VPL) == 0) return launch_lean_as<LPR, W, VPL, true>(tb, la, stream);
+  return launch_lean_as<LPR, W, VPL, false>(tb, la, stream);
+}
+
+// lane_w = 1 or 2 (rows that are not whole 16-byte vectors): a warp per row, up to 128 floats of it
+// per pass over the ids
+inline int lean_tile_floats(int feat, int lanes, int lane_w) {
+  if (lane_w >= 4) return lanes * lane_w;
+  return feat <= 32 * lane_w ? 32 * lane_w : (feat <= 64 ? 64 : 128);
+}
+
 int dispatch_lean(HybTable& tb, const LeanArgs& la, int lanes, int lane_w, cudaStream_t st) {
   if (lane_w == 8) {
-    if (lanes == 4) return launch_lean<4, 8>(tb, la, st);
-    if (lanes == 8) return launch_lean<8, 8>(tb, la, st);
-    if (lanes == 16) return launch_lean<16, 8>(tb, la, st);
-    return launch_lean<32, 8>(tb, la, st);
+    if (lanes == 4) return launch_lean<4, 8, 1>(tb, la, st);
+    if (lanes == 8) return launch_lean<8, 8, 1>(tb, la, st);
+    if (lanes == 16) return launch_lean<16, 8, 1>(tb, la, st);
+    return launch_lean<32, 8, 1>(tb, la, st);
   }
-  if (lanes == 8) return launch_lean<8, 4>(tb, la, st);
-  if (lanes == 16) return launch_lean<16, 4>(tb, la, st);
-  return launch_lean<32, 4>(tb, la, st);
+  if (lane_w == 4) {
+    if (lanes == 8) return launch_lean<8, 4, 1>(tb, la, st);
+    if (lanes == 16) return launch_lean<16, 4, 1>(tb, la, st);
+    return launch_lean<32, 4, 1>(tb, la, st);
+  }
+  const int tile = lean_tile_floats(la.feat, 32, lane_w);
+  if (lane_w == 2) return tile == 64 ? launch_lean<32, 2, 1>(tb, la, st) : launch_lean<32, 2, 2>(tb, la, st);
+  if (tile == 32) return launch_lean<32, 1, 1>(tb, la, st);
+  if (tile == 64) return launch_lean<32, 1, 2>(tb, la, st);
+  return launch_lean<32, 1, 4>(tb, la, st);
 }
 
 template <int LPR>
@@ -840,9 +950,10 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
     }
   }
   const bool vec4 = (feat % 4 == 0) && aligned16(b) && aligned16(c);
-  // the lean kernel takes whole feature tiles and ELL widths of 1, 2, 4 or a multiple of 8; with
-  // 32-byte aligned operands and a multiple of 32 features its lanes own 8 floats, else 4
-  bool lean = vec4 && static_cast<long long>(feat) * 4 < (1ll << 32);
+  // the lean kernel takes ELL widths of 1, 2, 4 or a multiple of 8; its lanes own 16-byte vectors
+  // (32-byte ones on request, for 32-byte aligned operands and a multiple of 32 features), or 8- and
+  // 4-byte ones where the row length or the alignment allows no more
+  bool lean = static_cast<long long>(feat) * 4 < (1ll << 32);
   for (int q = 0; q < tb.nb; ++q) {
     const int w = tb.width[q];
     lean = lean && (w == 1 || w == 2 || w == 4 || w % 8 == 0);
@@ -855,9 +966,12 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
     lane_w = 4;
     lanes = lanes_per_row_impl(feat, vec4, n, lane_w);
   }
-  lean = lean && feat % (lane_w * lanes) == 0;
+  if (!vec4) {
+    lane_w = feat % 2 == 0 && (reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 8 == 0 ? 2 : 1;
+    if (lean) lanes = 32;
+  }
   const size_t c_bytes = static_cast<size_t>(m) * feat * sizeof(float);
-  if (to_peers && (!lean || all_atomic || (flags & SPARSETIR_HYB_ZERO_C)))
+  if (to_peers && (!lean || !vec4 || feat % (lane_w * lanes) != 0 || all_atomic || (flags & SPARSETIR_HYB_ZERO_C)))
     return fail("sparsetir_hyb_spmm_peers: needs the one-writer kernel (feat_size a multiple of its tile, "
                 "16-byte aligned b and c, bucket widths 1, 2, 4 or multiples of 8, no ALL_ATOMIC or ZERO_C "
                 "flag); run sparsetir_hyb_spmm and sparsetir_peer_scatter instead");
@@ -883,7 +997,7 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
           tb.part_base[q] = static_cast<int32_t>(part_rows);
           part_rows += tb.nrows[q];
         }
-      const int tiles = feat / (lane_w * lanes);
+      const int tiles = ceil_div(feat, lean_tile_floats(feat, lanes, lane_w));
       const size_t part_bytes = static_cast<size_t>(part_rows) * feat * sizeof(float);
       const size_t counter_bytes = static_cast<size_t>(part_rows) * tiles * sizeof(unsigned);
       if (part_rows > INT32_MAX || part_bytes > hyb_scratch_limit()) {

@@ -117,6 +117,9 @@ template <> struct LaneVec<1> {
   static __device__ __forceinline__ void zero_if(float& acc, bool z) {
     acc = z ? 0.f : acc;
   }
+  static __device__ __forceinline__ void add_xor(float& v, int mask) {  // full warps only
+    v += __shfl_xor_sync(0xffffffffu, v, mask);
+  }
 };
 template <> struct LaneVec<2> {
   using type = float2;
@@ -136,6 +139,9 @@ template <> struct LaneVec<2> {
   // selects instead of a branch, for accumulators of sub-warps that run in step
   static __device__ __forceinline__ void zero_if(float2& acc, bool z) {
     acc.x = z ? 0.f : acc.x; acc.y = z ? 0.f : acc.y;
+  }
+  static __device__ __forceinline__ void add_xor(float2& v, int mask) {  // full warps only
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, mask); v.y += __shfl_xor_sync(0xffffffffu, v.y, mask);
   }
 };
 template <> struct LaneVec<4> {
@@ -158,6 +164,9 @@ template <> struct LaneVec<4> {
   // selects instead of a branch, for accumulators of sub-warps that run in step
   static __device__ __forceinline__ void zero_if(float4& acc, bool z) {
     acc.x = z ? 0.f : acc.x; acc.y = z ? 0.f : acc.y; acc.z = z ? 0.f : acc.z; acc.w = z ? 0.f : acc.w;
+  }
+  static __device__ __forceinline__ void add_xor(float4& v, int mask) {  // full warps only
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, mask); v.y += __shfl_xor_sync(0xffffffffu, v.y, mask); v.z += __shfl_xor_sync(0xffffffffu, v.z, mask); v.w += __shfl_xor_sync(0xffffffffu, v.w, mask);
   }
 };
 template <> struct LaneVec<8> {
@@ -210,6 +219,90 @@ template <> struct LaneVec<8> {
   static __device__ __forceinline__ void zero_if(Pack4& acc, bool z) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc.q[i] = z ? 0ull : acc.q[i];
+  }
+  static __device__ __forceinline__ void add_xor(Pack4& v, int mask) {  // full warps only
+    Pack4 o;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o.q[i] = __shfl_xor_sync(0xffffffffu, v.q[i], mask);
+    add(v, o);
+  }
+};
+
+// What a group of LPR lanes holds of a feature tile of LPR * W * VPL floats: VPL vectors of W floats
+// per lane, LPR * W floats apart.  Vectors past the end of the row are loaded from the tile's first
+// vector instead (an address another lane loads anyway) and never stored.
+template <int W, int VPL>
+struct LanePiece {
+  typename LaneVec<W>::type v[VPL];
+};
+// WHOLE promises that rows are whole tiles (feat a multiple of LPR * W * VPL): no predicates.
+template <int LPR, int W, int VPL, bool WHOLE>
+struct LaneTile {
+  using LV = LaneVec<W>;
+  using Piece = LanePiece<W, VPL>;
+  static constexpr int kFloats = LPR * W * VPL;
+  unsigned at[VPL];   // byte offset of the v-th vector inside a dense row
+  bool inside[VPL];
+  __device__ __forceinline__ LaneTile(int feat, int tile, int lane) {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const int f = tile * kFloats + v * (LPR * W) + lane * W;
+      inside[v] = WHOLE || f < feat;
+      at[v] = static_cast<unsigned>(inside[v] ? f : tile * kFloats) * 4u;
+    }
+  }
+  static __device__ __forceinline__ Piece zero() {
+    Piece p;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) p.v[v] = LV::zero();
+    return p;
+  }
+  static __device__ __forceinline__ void fma(Piece& acc, float w, const Piece& x) {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) LV::fma(acc.v[v], w, x.v[v]);
+  }
+  static __device__ __forceinline__ void add(Piece& acc, const Piece& x) {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) LV::add(acc.v[v], x.v[v]);
+  }
+  __device__ __forceinline__ Piece ldg(const char* row) const {
+    Piece p;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) p.v[v] = LV::ldg(row + at[v]);
+    return p;
+  }
+  // L2-coherent, for data that another block wrote during this launch
+  __device__ __forceinline__ Piece ldcg(const char* row) const {
+    Piece p;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) p.v[v] = LV::ldcg(row + at[v]);
+    return p;
+  }
+  __device__ __forceinline__ void stcs(char* row, const Piece& p) const {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (inside[v]) LV::stcs(row + at[v], p.v[v]);
+  }
+  __device__ __forceinline__ void stcg(char* row, const Piece& p) const {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (inside[v]) LV::stcg(row + at[v], p.v[v]);
+  }
+  __device__ __forceinline__ void atomic_add(char* row, const Piece& p) const {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (inside[v]) LV::atomic_add(row + at[v], p.v[v]);
+  }
+  // a tile in shared memory
+  static __device__ __forceinline__ void sts(float* tile, int lane, const Piece& p) {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) LV::sts(tile + v * (LPR * W) + lane * W, p.v[v]);
+  }
+  static __device__ __forceinline__ Piece lds(const float* tile, int lane) {
+    Piece p;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) p.v[v] = LV::lds(tile + v * (LPR * W) + lane * W);
+    return p;
   }
 };
 
