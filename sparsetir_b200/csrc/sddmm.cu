@@ -3,192 +3,124 @@
 // :510-569 (fused_sddmm with the edge->row binary search) of the reference; generated kernel
 // being replaced: examples/sddmm/bench_sddmm.py:97-167.
 //
-// Mapping.  The reference runs a separate preprocess kernel that stores row(p) for every
-// stored position and then gives every (ty, group) slot one edge with the dot product split
-// over tx lanes and reduced across threads.  Here one kernel does both:
-//  - a warp owns a contiguous range of stored positions and walks it 32 positions at a time;
-//    lane l reads indices[base+l] (coalesced) and finds row(base+l) by advancing from the
-//    warp's current row through indptr (the positions are sorted by row, so this is a short
-//    walk, with a binary search as the fallback for long runs of empty rows);
-//  - the 32 positions are split over the warp's sub-warps of LPR lanes, LPR positions each;
-//    a sub-warp loads the B row of one position at a time (every lane VPL 16-byte pieces,
-//    several positions in flight), keeps the A row in registers while the row id stays the
-//    same, and accumulates one partial sum per position in its own registers;
-//  - the LPR partial sums held by each of the LPR lanes are then reduced with a transposing
-//    butterfly: LPR-1 shuffles leave lane l with the finished dot product of position l,
-//    instead of log2(LPR) shuffles per position; the warp stores 32 consecutive results with
-//    one coalesced store.
+// The reference runs a separate preprocess kernel that stores row(p) for every stored position and
+// then gives every (ty, group) slot one edge with the dot product split over tx lanes and reduced
+// across threads.  Here one kernel does both: a warp owns a contiguous range of stored positions and
+// finds their rows itself, a sub-warp loads the B row of one position at a time (several positions
+// in flight) and keeps one partial sum per position, and the partial sums of several positions are
+// reduced together by a transposing butterfly, so that the warp stores 32 consecutive results with
+// one coalesced store.
 #include <cstdint>
 #include <cstdlib>
 
 #include <algorithm>
 
 #include "common.h"
-#include "vec.cuh"
+#include "row_walk.cuh"
 
 namespace sptir {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kEdgesPerWarp = 256;
 
-// row(p) = upper_bound(indptr[0..m], p) - 1, the search of
-// tests/python/sparsetir/sparse_tir_lowered_buffer_scripts.py:530-549
-__device__ __forceinline__ int edge_row_search(const int32_t* __restrict__ indptr, int lo_row,
-                                               int m, int p) {
-  int low = lo_row, high = m + 1;
-  while (low < high) {
-    int mid = low + (high - low) / 2;
-    if (__ldg(indptr + mid) > p) high = mid; else low = mid + 1;
-  }
-  return low - 1;
-}
-
-template <int LPR, int VPL, int VEC>
-__global__ void __launch_bounds__(kThreads)
+// General kernel: any feature count and alignment, rows of any length.
+//
+// A warp owns `chunk` consecutive positions and takes them 32 at a time; their rows come out of a
+// register window of row ends (row_walk.cuh).  Its sub-warps of LPR lanes take LPR positions each,
+// eight at a time: the rows of B of U positions and, where the row changes, their rows of A are
+// requested together, so that a matrix of short rows does not wait for A once per row (169 k-node
+// power-law graph, 5 entries per row, F = 64: 66 us when it did).  The feature tiles are walked
+// inside the kernel, the eight sums staying in registers; seven shuffles transpose and add them
+// over eight lanes, one more per doubling of the group adds the rest.
+template <int LPR, int W, int VPL, bool PEERS>
+__global__ void __launch_bounds__(kThreads, 4)
 sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
              const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-             const float* __restrict__ scale, int m, int feat, int nnz) {
-  using V = typename Vec<VEC>::type;
-  constexpr int U = (8 / VPL) < LPR ? (8 / VPL) : LPR;  // positions whose B rows are in flight
+             const float* __restrict__ scale, int m, int feat, int nnz, int chunk, float rows_per_entry,
+             const __grid_constant__ PeerOut po) {
+  using LT = LaneTile<LPR, W, VPL, false>;
+  using V = typename LT::Piece;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int U = VPL * W >= 4 ? 4 : 8;  // positions in flight
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const int sub = wlane / LPR;
-  const unsigned mask = group_mask<LPR>();
   const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
-  const long long e_begin = warp * kEdgesPerWarp;
-  if (e_begin >= nnz) return;
-  const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + kEdgesPerWarp));
-  const int row_vecs = feat / VEC;
-  const V* av = reinterpret_cast<const V*>(a);
-  const V* bv = reinterpret_cast<const V*>(b);
+  const long long begin = warp * chunk;
+  if (begin >= nnz) return;
+  const int e0 = static_cast<int>(begin);
+  const int count = static_cast<int>(min(static_cast<long long>(chunk), nnz - begin));
+  const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
+  const char* ab = reinterpret_cast<const char*>(a);
+  const char* bb = reinterpret_cast<const char*>(b);
+  const int tiles = (feat + LT::kFloats - 1) / LT::kFloats;
 
-  int off[VPL];
-  bool valid[VPL];
+  int col = wlane < count ? __ldg(indices + e0 + wlane) : 0;
+  int r = warp_row_of(indptr, m, e0, rows_per_entry, wlane);
+  int wend = row_window<32>(indptr, m, r, wlane);
+  for (int s0 = 0; s0 < count; s0 += 32) {
+    const bool live = wlane < count - s0;
+    const int e = e0 + min(s0 + wlane, count - 1);  // lanes past the last position repeat its row
+    int col_next = 0;
+    if (s0 + 32 + wlane < count) col_next = __ldg(indices + e0 + s0 + 32 + wlane);
+    const float mul = live && scale != nullptr ? __ldg(scale + e) : 1.f;
+    int row_end;
+    const int row = row_in_window<32>(indptr, m, r, wend, e, row_end);
+    r = __shfl_sync(kAll, row, 31);
+    wend = row_window<32>(indptr, m, r, wlane);
+    // bit k: position k of this sub-warp is in another row than position k - 1
+    const int row_before = __shfl_up_sync(kAll, row, 1, LPR);
+    const unsigned changes = __ballot_sync(kAll, lane == 0 || row != row_before) >> (sub * LPR);
+    float out = 0.f;
 #pragma unroll
-  for (int v = 0; v < VPL; ++v) {
-    off[v] = v * LPR + lane;
-    valid[v] = off[v] < row_vecs;
-  }
-
-  int warp_row = max(0, min(m - 1, edge_row_search(indptr, 0, m, static_cast<int>(e_begin))));
-  int cur_row = -1;
-  V arow[VPL];
+    for (int g = 0; g < LPR / 8; ++g) {
+      float part[8];
 #pragma unroll
-  for (int v = 0; v < VPL; ++v) arow[v] = Vec<VEC>::zero();
-
-  int warp_end = __ldg(indptr + warp_row + 1);  // first position past the warp's current row
-  for (int base = static_cast<int>(e_begin); base < e_end; base += 32) {
-    if (base + 32 <= min(warp_end, e_end)) {
-      // Fast path: all 32 positions belong to the warp's current row (the common case when rows
-      // are longer than a batch) — no row lookup, no per-position row bookkeeping.
-      const int col = __ldg(indices + base + wlane);
-      if (cur_row != warp_row) {
-        cur_row = warp_row;
-        const V* src = av + static_cast<size_t>(cur_row) * row_vecs;
+      for (int k = 0; k < 8; ++k) part[k] = 0.f;
+      for (int t = 0; t < tiles; ++t) {
+        const LT lt(feat, t, lane);
+        V arow = LT::zero();
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) arow[v] = valid[v] ? __ldg(src + off[v]) : Vec<VEC>::zero();
-      }
-      float part[LPR];
+        for (int h = 0; h < 8; h += U) {
+          V x[U], ar[U];
 #pragma unroll
-      for (int k0 = 0; k0 < LPR; k0 += U) {
-        V x[U][VPL];
+          for (int u = 0; u < U; ++u) {
+            const int k = g * 8 + h + u;
+            const unsigned ck = static_cast<unsigned>(__shfl_sync(kAll, col, k, LPR));
+            const unsigned rk = static_cast<unsigned>(__shfl_sync(kAll, row, k, LPR));
+            x[u] = lt.ldg(bb + static_cast<unsigned long long>(ck) * row_bytes);
+            if (h + u == 0 || ((changes >> k) & 1u)) ar[u] = lt.ldg(ab + static_cast<unsigned long long>(rk) * row_bytes);
+          }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const V* src = bv + static_cast<size_t>(__shfl_sync(mask, col, k0 + u, LPR)) * row_vecs;
-#pragma unroll
-          for (int v = 0; v < VPL; ++v) x[u][v] = valid[v] ? __ldg(src + off[v]) : Vec<VEC>::zero();
+          for (int u = 0; u < U; ++u) {
+            const int k = g * 8 + h + u;
+            if (h + u == 0 || ((changes >> k) & 1u)) arow = ar[u];
+            part[h + u] += lt.dot(arow, x[u]);
+          }
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          float s = 0.f;
-#pragma unroll
-          for (int v = 0; v < VPL; ++v) s = Vec<VEC>::dot(arow[v], x[u][v], s);
-          part[k0 + u] = s;
-        }
       }
 #pragma unroll
-      for (int offl = LPR / 2, n = LPR; offl >= 1; offl >>= 1, n >>= 1) {
-        const bool upper = (lane & offl) != 0;
+      for (int off = 4, n = 8; off >= 1; off >>= 1, n >>= 1) {  // afterwards part[0] is position lane % 8
+        const bool upper = (lane & off) != 0;
 #pragma unroll
         for (int i = 0; i < n / 2; ++i) {
-          float send = upper ? part[i] : part[i + n / 2];
-          float keep = upper ? part[i + n / 2] : part[i];
-          part[i] = keep + __shfl_xor_sync(mask, send, offl, LPR);
+          const float send = upper ? part[i] : part[i + n / 2];
+          const float keep = upper ? part[i + n / 2] : part[i];
+          part[i] = keep + __shfl_xor_sync(kAll, send, off);
         }
       }
-      float r = part[0];
-      if (scale != nullptr) r *= __ldg(scale + base + wlane);
-      c[base + wlane] = r;
-      continue;
-    }
-    const int e = base + wlane;
-    const bool live = e < e_end;
-    int col = 0, row = warp_row;
-    if (live) {
-      col = __ldg(indices + e);
-      int steps = 0;
-      // row < m - 1 keeps every read inside indptr even if nnz disagrees with indptr[m]
-      while (row < m - 1 && __ldg(indptr + row + 1) <= e) {
-        ++row;
-        if (++steps == 8) {  // long run of empty rows: finish with a search
-          row = min(m - 1, edge_row_search(indptr, row, m, e));
-          break;
-        }
-      }
-    }
-    // the next batch starts from the row of this batch's last live position
-    warp_row = __shfl_sync(0xffffffffu, row, min(31, e_end - 1 - base));
-    warp_end = __ldg(indptr + warp_row + 1);
-
-    const int cnt = min(LPR, e_end - (base + sub * LPR));  // live positions of this sub-warp (may be <= 0)
-    float part[LPR];
 #pragma unroll
-    for (int k = 0; k < LPR; ++k) part[k] = 0.f;
-#pragma unroll
-    for (int k0 = 0; k0 < LPR; k0 += U) {
-      if (k0 < cnt) {  // uniform inside the sub-warp
-        V x[U][VPL];
-        int rk[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          int ck = __shfl_sync(mask, col, k0 + u, LPR);  // dead positions carry column 0
-          rk[u] = __shfl_sync(mask, row, k0 + u, LPR);
-          const V* src = bv + static_cast<size_t>(ck) * row_vecs;
-#pragma unroll
-          for (int v = 0; v < VPL; ++v) x[u][v] = valid[v] ? __ldg(src + off[v]) : Vec<VEC>::zero();
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (rk[u] != cur_row) {  // uniform inside the sub-warp
-            cur_row = rk[u];
-            const V* src = av + static_cast<size_t>(cur_row) * row_vecs;
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) arow[v] = valid[v] ? __ldg(src + off[v]) : Vec<VEC>::zero();
-          }
-          float s = 0.f;
-#pragma unroll
-          for (int v = 0; v < VPL; ++v) s = Vec<VEC>::dot(arow[v], x[u][v], s);
-          part[k0 + u] = s;
-        }
-      }
-    }
-    // transposing butterfly: afterwards part[0] of lane l is the dot product of position l
-#pragma unroll
-    for (int offl = LPR / 2, n = LPR; offl >= 1; offl >>= 1, n >>= 1) {
-      const bool upper = (lane & offl) != 0;
-#pragma unroll
-      for (int i = 0; i < n / 2; ++i) {
-        float send = upper ? part[i] : part[i + n / 2];
-        float keep = upper ? part[i + n / 2] : part[i];
-        part[i] = keep + __shfl_xor_sync(mask, send, offl, LPR);
-      }
+      for (int off = 8; off < LPR; off <<= 1) part[0] += __shfl_xor_sync(kAll, part[0], off);
+      if (lane / 8 == g) out = part[0];
     }
     if (live) {
-      float r = part[0];
-      if (scale != nullptr) r *= __ldg(scale + e);
-      c[e] = r;
+      const float v = out * mul;
+      c[e] = v;
+      if constexpr (PEERS)
+        for (int k = 0; k < po.n; ++k)
+          *reinterpret_cast<float*>(reinterpret_cast<char*>(c + e) + po.delta[k]) = v;
     }
+    col = col_next;
   }
 }
 
@@ -330,44 +262,32 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   }
 }
 
-// Fallback for feature sizes beyond the register-resident variants: a full warp per position,
-// looping over the feature dimension.
-__global__ void __launch_bounds__(kThreads)
-sddmm_generic_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                     float* __restrict__ c, const int32_t* __restrict__ indptr,
-                     const int32_t* __restrict__ indices, const float* __restrict__ scale, int m,
-                     int feat, int nnz) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
-  const long long e_begin = warp * 32;
-  if (e_begin >= nnz) return;
-  const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + 32));
-  int row = max(0, min(m - 1, edge_row_search(indptr, 0, m, static_cast<int>(e_begin))));
-  for (int e = static_cast<int>(e_begin); e < e_end; ++e) {
-    while (row < m - 1 && __ldg(indptr + row + 1) <= e) ++row;
-    const float* ar = a + static_cast<size_t>(row) * feat;
-    const float* br = b + static_cast<size_t>(__ldg(indices + e)) * feat;
-    float s = 0.f;
-    for (int k = lane; k < feat; k += 32) s = fmaf(__ldg(ar + k), __ldg(br + k), s);
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) c[e] = scale ? s * __ldg(scale + e) : s;
-  }
-}
-
 __global__ void __launch_bounds__(kThreads)
 edge_to_row_kernel(const int32_t* __restrict__ indptr, int32_t* __restrict__ mid, int m, int nnz) {
   const long long p = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
   if (p < nnz) mid[p] = edge_row_search(indptr, 0, m, static_cast<int>(p));
 }
 
-template <int LPR, int VPL, int VEC>
+template <int LPR, int W, int VPL>
 int launch(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-           const float* scale, int m, int feat, int nnz, cudaStream_t stream) {
-  const int warps = ceil_div(nnz, kEdgesPerWarp);
-  const int blocks = ceil_div(warps, kThreads / 32);
-  sddmm_kernel<LPR, VPL, VEC><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m,
-                                                              feat, nnz);
+           const float* scale, int m, int feat, int nnz, const PeerOut& po, cudaStream_t stream) {
+  // one wave of resident blocks; two for the narrow vectors, whose positions take longer (50 k-node
+  // power-law graph, F = 299: 88 against 97 us)
+  const long long warps = static_cast<long long>(kNumSMs) * 4 * (kThreads / 32) * (W < 4 ? 2 : 1);
+  int chunk = static_cast<int>((nnz + warps - 1) / warps);
+  chunk = (chunk + 31) & ~31;
+  const int blocks = ceil_div(ceil_div(nnz, chunk), kThreads / 32);
+  const float rows_per_entry = static_cast<float>(m) / static_cast<float>(nnz);
+  if constexpr (W == 4) {
+    if (po.n > 0) {
+      sddmm_kernel<LPR, W, VPL, true><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, feat, nnz,
+                                                                       chunk, rows_per_entry, po);
+      SPTIR_LAUNCH_OK("sddmm_kernel");
+      return 0;
+    }
+  }
+  sddmm_kernel<LPR, W, VPL, false><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, feat, nnz,
+                                                                    chunk, rows_per_entry, po);
   SPTIR_LAUNCH_OK("sddmm_kernel");
   return 0;
 }
@@ -392,20 +312,15 @@ template <int LPR>
 int launch_lean_tile(const float* a, const float* b, float* c, const int32_t* indptr,
                      const int32_t* indices, const float* scale, int m, int feat, int nnz, int foff,
                      int last_tile, const PeerOut& po, cudaStream_t stream) {
-  // long chunks amortise the row search; short ones keep small inputs spread over the SMs
-  int chunk = nnz >= (1 << 22) ? 1024 : 256;
+  // About 1024 positions per warp amortise the row search, in whole waves of resident blocks: a
+  // launch of a few waves ends with a partly filled one otherwise (3.02 waves cost as much as 4;
+  // 1.7 M positions, F = 64: 59 us in 1.4 waves of 256 positions per warp).
   const int wpb = kThreads / 32;
-  int blocks = ceil_div(ceil_div(nnz, chunk), wpb);
-  // A launch of only a few waves of blocks ends with a partly filled wave (3.02 waves cost as
-  // much as 4): then the chunk is resized so that the blocks fill a whole number of waves.
-  const long long resident = static_cast<long long>(kNumSMs) * lean_blocks_per_sm<LPR>();
-  if (nnz >= (1 << 22) && blocks > resident / 2 && blocks < 8 * resident) {
-    const long long waves = std::max<long long>(1, (blocks + resident / 2) / resident);
-    const long long want_warps = waves * resident * wpb;
-    chunk = static_cast<int>((nnz + want_warps - 1) / want_warps);
-    chunk = (chunk + 31) & ~31;
-    blocks = ceil_div(ceil_div(nnz, chunk), wpb);
-  }
+  const long long resident = static_cast<long long>(kNumSMs) * lean_blocks_per_sm<LPR>() * wpb;
+  const long long waves = std::max<long long>(1, (nnz / 1024 + resident / 2) / resident);
+  int chunk = 1024;
+  if (waves < 8) chunk = static_cast<int>((nnz + waves * resident - 1) / (waves * resident) + 31) & ~31;
+  const int blocks = ceil_div(ceil_div(nnz, chunk), wpb);
   if (po.n > 0)
     sddmm_lean_kernel<LPR, true><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, nnz, feat,
                                                                   foff, foff != 0, chunk, last_tile, po);
@@ -476,26 +391,27 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(nnz) * sizeof(float), st));
     return 0;
   }
-  if (lean) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
-  const bool vec4 = (feat % 4 == 0) && aligned16(a) && aligned16(b);
-  if (vec4) {
-    const int nv = feat / 4;
-    if (nv <= 8) return launch<8, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (nv <= 16) return launch<16, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (nv <= 32) return launch<32, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (nv <= 64) return launch<32, 2, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (nv <= 128) return launch<32, 4, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-  } else {
-    if (feat <= 8) return launch<8, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (feat <= 16) return launch<16, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (feat <= 32) return launch<32, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (feat <= 64) return launch<32, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
-    if (feat <= 128) return launch<32, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, st);
+  // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one
+  // (60 k rows, F = 64: 12 entries per row 25.5 against 27.9 us, 28 entries 49 against 54; the
+  // power-law graph of 5 entries per row 54 against 46 us).
+  if (lean && nnz / m >= 10) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
+  if (feat % 4 == 0 && bits % 16 == 0) {
+    if (feat <= 32) return launch<8, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    if (feat <= 64) return launch<16, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<32, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   }
-  const int blocks = ceil_div(ceil_div(nnz, 32), kThreads / 32);
-  sddmm_generic_kernel<<<blocks, kThreads, 0, st>>>(a, b, c, indptr, indices, scale, m, feat, nnz);
-  SPTIR_LAUNCH_OK("sddmm_generic_kernel");
-  return 0;
+  if (feat % 2 == 0 && bits % 8 == 0) {
+    if (feat <= 16) return launch<8, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    if (feat <= 32) return launch<16, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    if (feat <= 64) return launch<32, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<32, 2, 2>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  }
+  if (feat <= 8) return launch<8, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  if (feat <= 16) return launch<16, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  if (feat <= 32) return launch<32, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  if (feat <= 64) return launch<32, 1, 2>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  return launch<32, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
 }
 }  // namespace
 }  // namespace sptir

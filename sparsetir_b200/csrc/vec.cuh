@@ -120,6 +120,7 @@ template <> struct LaneVec<1> {
   static __device__ __forceinline__ void add_xor(float& v, int mask) {  // full warps only
     v += __shfl_xor_sync(0xffffffffu, v, mask);
   }
+  static __device__ __forceinline__ float dot(const float& a, const float& b) { return a * b; }
 };
 template <> struct LaneVec<2> {
   using type = float2;
@@ -143,6 +144,7 @@ template <> struct LaneVec<2> {
   static __device__ __forceinline__ void add_xor(float2& v, int mask) {  // full warps only
     v.x += __shfl_xor_sync(0xffffffffu, v.x, mask); v.y += __shfl_xor_sync(0xffffffffu, v.y, mask);
   }
+  static __device__ __forceinline__ float dot(const float2& a, const float2& b) { return fmaf(a.y, b.y, a.x * b.x); }
 };
 template <> struct LaneVec<4> {
   using type = float4;
@@ -168,6 +170,7 @@ template <> struct LaneVec<4> {
   static __device__ __forceinline__ void add_xor(float4& v, int mask) {  // full warps only
     v.x += __shfl_xor_sync(0xffffffffu, v.x, mask); v.y += __shfl_xor_sync(0xffffffffu, v.y, mask); v.z += __shfl_xor_sync(0xffffffffu, v.z, mask); v.w += __shfl_xor_sync(0xffffffffu, v.w, mask);
   }
+  static __device__ __forceinline__ float dot(const float4& a, const float4& b) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x))); }
 };
 template <> struct LaneVec<8> {
   using type = Pack4;
@@ -264,6 +267,16 @@ struct LaneTile {
   static __device__ __forceinline__ void add(Piece& acc, const Piece& x) {
 #pragma unroll
     for (int v = 0; v < VPL; ++v) LV::add(acc.v[v], x.v[v]);
+  }
+  // a vector past the end of the row counts for nothing
+  __device__ __forceinline__ float dot(const Piece& a, const Piece& b) const {
+    float s = 0.f;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const float d = LV::dot(a.v[v], b.v[v]);
+      s += inside[v] ? d : 0.f;
+    }
+    return s;
   }
   __device__ __forceinline__ Piece ldg(const char* row) const {
     Piece p;

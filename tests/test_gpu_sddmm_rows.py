@@ -1,0 +1,42 @@
+"""SDDMM on short, long and empty rows, with every vector width and alignment, against float64 dot
+products."""
+import numpy as np
+import pytest
+import torch
+
+from sparsetir_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    "one_position": [0, 0, 1],
+    "singles": [1] * 5001,
+    "empty_runs": ([0] * 400 + [1, 2, 3] + [0] * 33 + [5]) * 20,
+    "hubs_among_short_rows": [3, 0, 1, 900, 2, 2, 31, 32, 33, 0, 1] * 30,
+    "long_rows": [700, 0, 1500, 64, 65],
+}
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+@pytest.mark.parametrize("feat,offset", [(1, 0), (8, 0), (23, 0), (31, 0), (33, 0), (46, 0), (56, 0), (64, 0), (100, 0),
+                                         (130, 0), (264, 0), (299, 0), (512, 0), (64, 1), (64, 2), (96, 4)])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_rows_and_alignments(cuda_device, shape, feat, offset, scaled):
+    deg = np.asarray(SHAPES[shape], np.int64)
+    m, n, nnz = len(deg), 777, int(deg.sum())
+    rng = np.random.default_rng(feat)
+    dev = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    indptr = np.zeros(m + 1, np.int32)
+    indptr[1:] = np.cumsum(deg)
+    cols = dev(rng.integers(0, n, nnz).astype(np.int32))
+    a = dev(rng.uniform(-1, 1, m * feat + offset).astype(np.float32))[offset:]
+    b = dev(rng.uniform(-1, 1, n * feat + offset).astype(np.float32))[offset:]
+    scale = dev(rng.uniform(0, 1, nnz).astype(np.float32))
+    out = torch.full((nnz,), float("nan"), device=cuda_device)
+    ops.sddmm(a, b, out, dev(indptr), cols, *([scale] if scaled else []))
+    rows = torch.repeat_interleave(torch.arange(m, device=cuda_device), dev(deg))
+    prod = a.view(m, feat)[rows].double() * b.view(n, feat)[cols.long()].double()
+    s = scale.double() if scaled else 1.0
+    want, mag = prod.sum(1) * s, prod.abs().sum(1) * s
+    # an fp32 sum of feat products in any order and one more product: feat + 1 half-ulps of the magnitudes
+    assert bool(((out.double() - want).abs() <= mag * (feat + 2) * 2.0 ** -24).all())
