@@ -303,6 +303,16 @@ SPARSETIR_API int sparsetir_rgms_ell3d(SPARSETIR_PACKED_ARGS);
  * accumulated in fp32; accumulates into the caller's zero-filled y. */
 SPARSETIR_API int sparsetir_rgms_ell3d_f16(SPARSETIR_PACKED_ARGS);
 
+/* (w, x, y, map, m, num_rels, feat_in, feat_out, add): a sparse convolution whose (offset, output)
+ * pairs never repeat, with its neighbour map laid out in advance: y[d, :] = (add ? y[d, :] : 0) + sum
+ * over offsets r with map entry s >= 0 of x[s, :] * w[r, :, :].  map holds
+ * ceil(m / 128) * num_rels * 128 entries, map[(d / 128 * num_rels + r) * 128 + d % 128] = s, or -1
+ * where output d has no pair of offset r or d >= m.  w, x float16; y float16 or float32 (written, not
+ * accumulated, unless add is 1); feat_in a multiple of 16, feat_out a multiple of 32 up to 256, 16-byte
+ * aligned operands.  The same result as sparsetir_rgms_ell3d_f16 on the layer's ELL3D buckets
+ * (examples/rgms/sparse_conv/sparse_conv.py:93-125), which takes every other shape. */
+SPARSETIR_API int sparsetir_sparse_conv_f16(SPARSETIR_PACKED_ARGS);
+
 /* ---- operators, plain-pointer form (device pointers; stream is a cudaStream_t) -------- */
 SPARSETIR_API int sparsetir_csrmm_raw(const float* a, const float* b, float* c,
                                       const int32_t* indptr, const int32_t* indices, int m, int n,
@@ -408,6 +418,10 @@ SPARSETIR_API int sparsetir_rgms_ell3d_f16_raw(const void* w, const void* x, voi
                                                const SparsetirEll3dBucketH* buckets, int num_buckets,
                                                int m, int n, int num_rels, int feat_in, int feat_out,
                                                int device_id, void* stream);
+SPARSETIR_API int sparsetir_sparse_conv_f16_raw(const void* w, const void* x, void* y, int y_is_f16,
+                                                const int32_t* map, int m, int n, int num_rels,
+                                                int feat_in, int feat_out, int add, int device_id,
+                                                void* stream);
 
 /* RGMS that never allocates device memory.  No counterpart in the reference: it exists for
  * hosts that may not call the CUDA allocator when they need the operator (loops that forbid

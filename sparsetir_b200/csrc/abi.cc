@@ -518,6 +518,38 @@ int sparsetir_rgms_ell3d_f16(SPARSETIR_PACKED_ARGS) {
                                       sptir::stream_for(p.device_id));
 }
 
+int sparsetir_sparse_conv_f16(SPARSETIR_PACKED_ARGS) {
+  (void)resource_handle;
+  Packed p{"sparsetir_sparse_conv_f16", args, type_codes, num_args};
+  if (num_args != 9) return fail("sparsetir_sparse_conv_f16: num_args should be 9, got %d", num_args);
+  void *w = nullptr, *x = nullptr, *y = nullptr, *map = nullptr;
+  int64_t lw = 0, lx = 0, ly = 0, lmap = 0, m = 0, rels = 0, fin = 0, fout = 0, add = 0;
+  TRY(p.tensor(0, "w", kDLFloat, 16, &w, &lw));
+  TRY(p.tensor(1, "x", kDLFloat, 16, &x, &lx));
+  int y_is_f16 = 1;
+  if (p.is_tensor(2) && args[2].v_handle != nullptr && static_cast<const DLTensor*>(args[2].v_handle)->dtype.bits == 32)
+    y_is_f16 = 0;
+  TRY(p.tensor(2, "y", kDLFloat, y_is_f16 ? 16 : 32, &y, &ly));
+  TRY(p.tensor(3, "map", kDLInt, 32, &map, &lmap));
+  TRY(p.integer(4, "m", &m));
+  TRY(p.integer(5, "num_rels", &rels));
+  TRY(p.integer(6, "feat_in", &fin));
+  TRY(p.integer(7, "feat_out", &fout));
+  TRY(p.integer(8, "add", &add));
+  TRY(fits_i32(p.fn, "m", m)); TRY(fits_i32(p.fn, "num_rels", rels));
+  TRY(fits_i32(p.fn, "feat_in", fin)); TRY(fits_i32(p.fn, "feat_out", fout));
+  if (fin == 0 || fout == 0) return fail("sparsetir_sparse_conv_f16: feat_in and feat_out must be positive");
+  if (lx % fin != 0) return fail("sparsetir_sparse_conv_f16: len(x) is not a multiple of feat_in");
+  TRY(fits_i32(p.fn, "n", lx / fin));
+  TRY(check_len(p.fn, "w", lw, rels * fin * fout));
+  TRY(check_len(p.fn, "y", ly, m * fout));
+  TRY(check_len(p.fn, "map", lmap, (m + 127) / 128 * rels * 128));
+  set_void_return(out_ret_value, out_ret_tcode);
+  return sparsetir_sparse_conv_f16_raw(w, x, y, y_is_f16, static_cast<const int32_t*>(map), (int)m, (int)(lx / fin),
+                                       (int)rels, (int)fin, (int)fout, add != 0, p.device_id,
+                                       sptir::stream_for(p.device_id));
+}
+
 int sparsetir_tcspmm(SPARSETIR_PACKED_ARGS) {
   (void)resource_handle;
   Packed p{"sparsetir_tcspmm", args, type_codes, num_args};

@@ -40,6 +40,7 @@ int rgms_tc_timeouts(unsigned int* count);  // the same counter of rgms_tc.cu
 int tcspmm_timeouts(unsigned int* count);   // ... and of tcspmm.cu
 int rgms_f16_timeouts(unsigned int* count);  // ... and of rgms_f16.cu
 int rgms_fused_timeouts(unsigned int* count);  // ... and of rgms_fused.cu
+int conv_timeouts(unsigned int* count);        // ... and of sparse_conv.cu
 
 namespace {
 
@@ -597,6 +598,8 @@ extern "C" int sparsetir_tc_timeouts(int device_id, unsigned int* count) {
   if (rgms_f16_timeouts(&rh) != 0) return -1;
   unsigned int rf = 0;
   if (rgms_fused_timeouts(&rf) != 0) return -1;
-  *count = bsr + rgms + tcs + rh + rf;
+  unsigned int cv = 0;
+  if (conv_timeouts(&cv) != 0) return -1;
+  *count = bsr + rgms + tcs + rh + rf + cv;
   return 0;
 }

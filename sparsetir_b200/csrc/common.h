@@ -48,7 +48,7 @@ bool validate_enabled();
 int validate_indptr(const char* op, const char* what, const int32_t* indptr, long long rows,
                     long long nnz, cudaStream_t st);
 int validate_range(const char* op, const char* what, const int32_t* ids, long long count,
-                   long long bound, cudaStream_t st);
+                   long long bound, cudaStream_t st, long long lowest = 0);
 int validate_csr(const char* op, const int32_t* indptr, long long rows, const int32_t* indices,
                  long long nnz, long long cols, cudaStream_t st);
 

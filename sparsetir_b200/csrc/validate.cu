@@ -39,11 +39,11 @@ __global__ void check_indptr_kernel(const int32_t* __restrict__ indptr, long lon
   }
 }
 
-__global__ void check_range_kernel(const int32_t* __restrict__ ids, long long count, long long bound) {
+__global__ void check_range_kernel(const int32_t* __restrict__ ids, long long count, long long lowest, long long bound) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
     const int32_t v = ids[i];
-    if (v < 0 || v >= bound) report(kOutOfRange, i, v);
+    if (v < lowest || v >= bound) report(kOutOfRange, i, v);
   }
 }
 
@@ -97,10 +97,10 @@ int validate_indptr(const char* op, const char* what, const int32_t* indptr, lon
 }
 
 int validate_range(const char* op, const char* what, const int32_t* ids, long long count,
-                   long long bound, cudaStream_t st) {
+                   long long bound, cudaStream_t st, long long lowest) {
   if (count <= 0 || ids == nullptr) return 0;
   if (begin_check(st) != 0) return -1;
-  check_range_kernel<<<grid_for(count), 256, 0, st>>>(ids, count, bound);
+  check_range_kernel<<<grid_for(count), 256, 0, st>>>(ids, count, lowest, bound);
   SPTIR_LAUNCH_OK("check_range_kernel");
   return end_check(op, what, st);
 }

@@ -180,6 +180,7 @@ bsrmm = PackedFunc("sparsetir_bsrmm")
 rgms = PackedFunc("sparsetir_rgms")
 rgms_ell3d = PackedFunc("sparsetir_rgms_ell3d")
 rgms_ell3d_f16 = PackedFunc("sparsetir_rgms_ell3d_f16")
+sparse_conv_f16 = PackedFunc("sparsetir_sparse_conv_f16")
 tcspmm = PackedFunc("sparsetir_tcspmm")
 csr_reduce = PackedFunc("sparsetir_csr_reduce")
 sparse_softmax = PackedFunc("sparsetir_sparse_softmax")

@@ -99,8 +99,27 @@ def ell3d_from_maps(nbmaps, nbsizes, transposed: bool, num_inputs: int,
     return out, m, int(sum(len(s) for s, _ in rels))
 
 
+def neighbour_map(nbmaps, nbsizes, transposed: bool, num_outputs: int, device: torch.device) -> Optional[torch.Tensor]:
+    """The layer's pairs as ``sparsetir_sparse_conv_f16`` takes them, on ``device``: tiles of 128 outputs,
+    ``map[(tile * K + k) * 128 + t]`` = input point of output ``tile * 128 + t`` at kernel offset ``k``,
+    or -1; None when an (offset, output) pair repeats."""
+    maps = torch.as_tensor(nbmaps).to(device, torch.int64)
+    sizes = torch.as_tensor([int(s) for s in (nbsizes.tolist() if hasattr(nbsizes, "tolist") else nbsizes)],
+                            dtype=torch.int64).to(device)
+    offsets, pairs = len(sizes), int(sizes.sum())
+    src, dst = (maps[:pairs, 1], maps[:pairs, 0]) if transposed else (maps[:pairs, 0], maps[:pairs, 1])
+    rel = torch.repeat_interleave(torch.arange(offsets, device=device), sizes, output_size=pairs)
+    out = torch.full((-(-num_outputs // 128) * offsets * 128,), -1, dtype=torch.int32, device=device)
+    out[(dst // 128 * offsets + rel) * 128 + dst % 128] = src.int()
+    return out if int((out >= 0).sum()) == pairs else None
+
+
 class SparseConvPlan:
     """The structure of one layer, converted once (host side) and kept on the device.
+
+    A layer whose (offset, output) pairs never repeat is kept as a neighbour map too: such a call is
+    one launch of ``sparsetir_sparse_conv_f16``, which writes its result, for every channel count
+    that this operator takes; all others run ``sparsetir_rgms_ell3d_f16`` on the ELL3D buckets.
 
     ``plan(inputs, weights)`` then runs the operator; the maps of a layer do not change between
     calls, so the host conversion is not part of the steady state (the reference also converts
@@ -116,6 +135,7 @@ class SparseConvPlan:
         self.device = device if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.buckets = [tuple(torch.from_numpy(np.ascontiguousarray(a)).to(self.device) for a in bk)
                         for bk in host]
+        self._map = neighbour_map(nbmaps, nbsizes, bool(transposed), self.num_outputs, self.device)
 
     def __call__(self, inputs: torch.Tensor, weights: torch.Tensor,
                  out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float16) -> torch.Tensor:
@@ -128,10 +148,19 @@ class SparseConvPlan:
             raise ValueError("inputs and weights disagree on feat_in")
         x = inputs.to(self.device, torch.float16).contiguous()
         w = weights.to(self.device, torch.float16).contiguous()
+        mapped = (self._map is not None and feat_in % 16 == 0 and feat_out % 32 == 0 and 0 < feat_in and 0 < feat_out <= 256
+                  and out_dtype in (torch.float16, torch.float32)
+                  and (x.data_ptr() | w.data_ptr() | (0 if out is None else out.data_ptr())) % 16 == 0)
+        add = out is not None
         if out is None:
-            out = torch.zeros(self.num_outputs, feat_out, dtype=out_dtype, device=self.device)
+            make = torch.empty if mapped else torch.zeros
+            out = make(self.num_outputs, feat_out, dtype=out_dtype, device=self.device)
         elif tuple(out.shape) != (self.num_outputs, feat_out) or not out.is_contiguous():
             raise ValueError("out must be a contiguous [num_outputs, feat_out] tensor (it is added to)")
+        if mapped:
+            ops.sparse_conv_f16(w.view(-1), x.view(-1), out.view(-1), self._map, self.num_outputs, self.num_offsets, feat_in,
+                                feat_out, int(add))
+            return out
         ops.rgms_ell3d_f16(*ops.rgms_ell3d_f16_args(w, x, out, self.buckets, feat_in, feat_out))
         return out
 

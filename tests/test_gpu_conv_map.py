@@ -1,0 +1,67 @@
+"""The sparse convolution with its neighbour map laid out in advance: channel counts around the
+slices and boxes of the kernel, ragged tiles, offsets without pairs, and addition into an output."""
+import numpy as np
+import pytest
+import torch
+
+from sparsetir_b200 import _lib as L
+from sparsetir_b200 import ops
+from sparsetir_b200.sparse_conv import SparseConvPlan, neighbour_map
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("feat_in", [16, 32, 48, 64, 96, 128, 256])
+@pytest.mark.parametrize("feat_out", [32, 64, 96, 160, 256])
+@pytest.mark.parametrize("n_out,offsets,fill", [(1, 1, 1.0), (127, 3, 0.5), (129, 27, 0.3), (20_001, 8, 0.6)])
+def test_matches_a_float64_product(cuda_device, feat_in, feat_out, n_out, offsets, fill):
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(feat_in + feat_out + n_out)
+    n_in = max(2, n_out // 2)
+    maps, sizes = [], []
+    for k in range(offsets):
+        outs = torch.nonzero(torch.rand(n_out, device=cuda_device, generator=g) < (0.0 if k == 1 else fill))[:, 0]
+        ins = torch.randint(0, n_in, (len(outs),), device=cuda_device, generator=g)
+        maps.append(torch.stack([ins, outs], 1))
+        sizes.append(len(outs))
+    pairs = torch.cat(maps)
+    x = torch.rand(n_in, feat_in, device=cuda_device, generator=g).half() - 0.5
+    w = (torch.randn(offsets, feat_in, feat_out, device=cuda_device, generator=g) / np.sqrt(feat_in)).half()
+    table = neighbour_map(pairs, np.asarray(sizes), False, n_out, cuda_device)
+    want = torch.zeros(n_out, feat_out, dtype=torch.float64, device=cuda_device)
+    mag = torch.zeros_like(want)
+    for k, mp in enumerate(maps):
+        want[mp[:, 1]] += x[mp[:, 0]].double() @ w[k].double()
+        mag[mp[:, 1]] += x[mp[:, 0]].double().abs() @ w[k].double().abs()
+    # fp32 sums of exact fp16 products (the tensor core may cut below the last bit of the largest
+    # term of every 16-term step: one ulp a step); the start value and a float16 result round once more
+    bound = mag * (offsets * feat_in / 16 + 2) * 2.0 ** -22
+    for dtype, add in ((torch.float32, 0), (torch.float32, 1), (torch.float16, 0), (torch.float16, 1)):
+        y = torch.full((n_out * feat_out,), 3.0, dtype=dtype, device=cuda_device)
+        ops.sparse_conv_f16(w.view(-1), x.view(-1), y, table, n_out, offsets, feat_in, feat_out, add)
+        ref = want + 3.0 * add
+        extra = ref.abs() * 2.0 ** -22 if dtype == torch.float32 else (ref.abs() + want.abs()) * 2.0 ** -10 + 2.0 ** -20
+        assert bool(((y.view(n_out, feat_out).double() - ref).abs() <= bound + extra).all()), (dtype, add)
+    count = L.ctypes.c_uint(0)
+    assert L.load().sparsetir_tc_timeouts(cuda_device.index or 0, L.ctypes.byref(count)) == 0 and count.value == 0
+
+
+def test_repeated_pairs_keep_the_buckets(cuda_device):
+    pairs = torch.tensor([[0, 1], [2, 1], [1, 0]])
+    assert neighbour_map(pairs, [2, 1], False, 3, cuda_device) is None
+    x, w = torch.rand(3, 64, device=cuda_device).half(), torch.rand(2, 64, 64, device=cuda_device).half()
+    y = SparseConvPlan(pairs, [2, 1], False, 3, 3, device=cuda_device)(x, w, out_dtype=torch.float32)
+    want = torch.zeros(3, 64, device=cuda_device)
+    want[1] = (x[0].float() + x[2].float()) @ w[0].float()
+    want[0] = x[1].float() @ w[1].float()
+    torch.testing.assert_close(y, want, rtol=1e-2, atol=1e-2)
+
+
+def test_shapes_it_does_not_take_are_refused(cuda_device):
+    h = lambda n: torch.zeros(n, dtype=torch.float16, device=cuda_device)  # noqa: E731
+    table = torch.full((128,), -1, dtype=torch.int32, device=cuda_device)
+    for fi, fo in ((8, 32), (16, 16), (16, 288)):
+        with pytest.raises(ops.SparseTIRError, match="multiple of 16"):
+            ops.sparse_conv_f16(h(fi * fo), h(fi), h(fo), table, 1, 1, fi, fo, 0)
+    with pytest.raises(ops.SparseTIRError, match="map"):
+        ops.sparse_conv_f16(h(32 * 32), h(32), h(32), table[:64], 1, 1, 32, 32, 0)
