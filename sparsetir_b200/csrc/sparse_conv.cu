@@ -7,16 +7,18 @@
 // The product is one GEMM per tile with K = R * feat_in: row t of the left operand is the
 // concatenation of the X rows of its pairs (zeros where there is none), the right operand is W as
 // it lies in memory.  A persistent block per SM walks the tiles; per 64-wide slice of K
-//  - six groups of four warps fetch the left operand, 16 bytes per thread and load, eight loads in
-//    flight per thread, and write it into the swizzled stage (a slice may straddle offsets, so
-//    channel counts that are not multiples of 64 waste nothing);
+//  - six groups of four warps fetch the left operand with 16-byte asynchronous copies into the
+//    swizzled stage (a slice may straddle offsets, so channel counts that are not multiples of 64
+//    waste nothing; a missing pair is a copy of no bytes, which fills in zeros);
 //  - one thread brings the slice of W with TMA, one issues the MMAs into one of two accumulators;
 //  - four warps take finished tiles out of TMEM and write (or add to) Y, each row once.
 //
-// Register loads and not asynchronous copies: 16-byte cp.async reaches about 16 bytes per clock and
-// SM, which bounded the same product at 85 us (100,000 points, 27 offsets, 64 -> 128 channels).
-// The map replaces one built, checked and cleared on every call: together with the cleared Y that
-// took 37 us of 122.
+// Bound by the instructions and round trips of the ring, not by a unit (100,000 points, 27 offsets,
+// 64 -> 128: tensor pipe 34 %, L1 data pipe 61 %, L2 22 %): the time goes with the steps and hardly
+// depends on the share of pairs or on feat_out.  What the steps cost is therefore what was cut: no
+// divisions in the loops and MMAs from an elected thread 97 -> 64 us, asynchronous copies instead of
+// loads and stores 64 -> 61 us.  Gathering by TMA (four rows per copy) took 215 us.  The map replaces one
+// built, checked and cleared on every call: together with the cleared Y that took 37 us of 122.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -97,11 +99,30 @@ __device__ __forceinline__ void write32(__half* y, const unsigned char* wbase, i
   }
 }
 
+// One row's 32 outputs from its pairs alone, lane = output.  A row without a pair of some offset takes
+// part in that offset's product with zeros, and 0 * W is NaN where W is not finite: rows that came
+// out with a NaN are formed again here, from the terms of the sum and no others.
+__device__ __noinline__ float row_by_pairs(const __half* __restrict__ x, const __half* __restrict__ w,
+                                           const int32_t* __restrict__ entries, int num_rels, int feat_in,
+                                           int feat_out, int col) {
+  float sum = 0.f;
+  for (int rel = 0; rel < num_rels; ++rel) {
+    const int e = __ldg(entries + static_cast<size_t>(rel) * kTM);
+    if (e < 0) continue;
+    const __half* xr = x + static_cast<size_t>(e) * feat_in;
+    const __half* wr = w + static_cast<size_t>(rel) * feat_in * feat_out + col;
+#pragma unroll 8
+    for (int fi = 0; fi < feat_in; ++fi)
+      sum = fmaf(__half2float(__ldg(xr + fi)), __half2float(__ldg(wr + static_cast<size_t>(fi) * feat_out)), sum);
+  }
+  return sum;
+}
+
 template <typename OutT>
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ y, const __half* __restrict__ x,
-                   const int32_t* __restrict__ map, int m, int num_rels, int feat_in, int feat_out, int tmem_cols,
-                   int acc_cols, int nstages, int groups, int add) {
+                   const __half* __restrict__ w, const int32_t* __restrict__ map, int m, int num_rels, int feat_in,
+                   int feat_out, int tmem_cols, int acc_cols, int nstages, int groups, int add) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];   // both operands of the stage are there
   __shared__ __align__(8) uint64_t bar_empty[kMaxStages];  // the tensor core has read the stage
@@ -143,42 +164,48 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
 
   if (warp == 0) {
     // ---- W: rows [64 s, 64 s + 64) of the (R * feat_in) x feat_out array; past its end zeros
-    if (lane == 0) {
-      int it = 0;
+    if (tc05::elect_one()) {
+      int s = 0;
+      uint32_t phase = 0;
+      unsigned char* st = base + kZBytes;
       for (int k = 0; k < my_tiles && ok; ++k) {
-        for (int sidx = 0; sidx < steps; ++sidx, ++it) {
-          const int s = it % nstages, use = it / nstages;
-          if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
-          unsigned char* st = base + s * stride;
+        for (int sidx = 0; sidx < steps; ++sidx) {
+          if (!tc05::mbar_wait(&bar_empty[s], phase ^ 1u)) { ok = false; break; }
           tc05::mbar_arrive_expect_tx(&bar_full[s], nwb * kWBox);
-          for (int j = 0; j < nwb; ++j)
-            tc05::tma_load_2d(st + kZBytes + j * kWBox, &tm_w, j * 64, sidx * kKC, &bar_full[s]);
-          armed = it + 1;
+          for (int j = 0; j < nwb; ++j) tc05::tma_load_2d(st + j * kWBox, &tm_w, j * 64, sidx * kKC, &bar_full[s]);
+          ++armed;
+          st += stride;
+          if (++s == nstages) { s = 0; phase ^= 1u; st = base + kZBytes; }
         }
       }
     }
   } else if (warp == 1) {
     // ---- MMAs: M = 128 outputs, N = feat_out, K = 16 per instruction
-    if (lane == 0) {
+    if (tc05::elect_one()) {
       const uint32_t idesc = tc05::instr_desc(tc05::kFmtF16, kTM, feat_out, /*a_mn=*/0, /*b_mn=*/1);
       const uint64_t dz0 = tc05::smem_desc_swizzled(tc05::smem_u32(base), 0, 1024, tc05::kSwizzle128B);
       const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base) + kZBytes, kWBox, 1024, tc05::kSwizzle128B);
-      int it = 0;
+      const int last = (ktotal - (steps - 1) * kKC) / 16;  // instructions of the last slice
+      int s = 0;
+      uint32_t phase = 0;
+      uint64_t dz = dz0, dw = dw0;
       for (int k = 0; k < my_tiles && ok; ++k) {
         const int buf = k & 1, buse = k >> 1;
-        if (buse > 0 && !tc05::mbar_wait(&bar_acc_empty[buf], (buse - 1) & 1)) { ok = false; break; }
+        if (!tc05::mbar_wait(&bar_acc_empty[buf], (buse & 1) ^ 1)) { ok = false; break; }
         const uint32_t acc = tmem + buf * acc_cols;
-        for (int sidx = 0; sidx < steps; ++sidx, ++it) {
-          const int s = it % nstages, use = it / nstages;
-          if (!tc05::mbar_wait(&bar_full[s], use & 1)) { ok = false; break; }
+        for (int sidx = 0; sidx < steps; ++sidx) {
+          if (!tc05::mbar_wait(&bar_full[s], phase)) { ok = false; break; }
           tc05::fence_after_sync();
-          const uint64_t dz = tc05::desc_advance(dz0, s * stride);
-          const uint64_t dw = tc05::desc_advance(dw0, s * stride);
-          const int ksteps = min(kKC, ktotal - sidx * kKC) / 16;  // the last slice may be short
-          for (int ks = 0; ks < ksteps; ++ks)
-            tc05::mma_f16(acc, tc05::desc_advance(dz, ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
-                          (sidx > 0 || ks > 0) ? 1u : 0u);
+          const int ksteps = sidx + 1 < steps ? kKC / 16 : last;
+#pragma unroll
+          for (int ks = 0; ks < kKC / 16; ++ks)
+            if (ks < ksteps)
+              tc05::mma_f16(acc, tc05::desc_advance(dz, ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
+                            (sidx > 0 || ks > 0) ? 1u : 0u);
           tc05::mma_commit(&bar_empty[s]);
+          dz = tc05::desc_advance(dz, stride);
+          dw = tc05::desc_advance(dw, stride);
+          if (++s == nstages) { s = 0; phase ^= 1u; dz = dz0; dw = dw0; }
         }
         if (!ok) break;
         tc05::mma_commit(&bar_acc_full[buf]);
@@ -188,47 +215,71 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     // ---- gather: group g fills the left operand of steps g, g + groups, ...; warp gw of it rows
     // gw * 32 .. gw * 32 + 31, eight lanes per row.  No more groups than stages: a group that has
     // written step n knows that the tensor core is past step n - nstages, and may wait for the stage
-    // of step n + groups only if that puts it at most one phase of the stage's barrier behind.  The map entries of a group's next step are
-    // requested before this step's rows are written.
+    // of step n + groups only if that puts it at most one phase of the stage's barrier behind.  The map
+    // entries of a group's next step are requested before this step's rows are written.
+    //
+    // (offset, piece) of the lane move by whole rows of the ring: quotients and remainders are formed once.
     const int g = (warp - kFirstGather) >> 2, gw = (warp - kFirstGather) & 3;
-    const int total = my_tiles * steps, cpr = feat_in / 8;  // 16-byte pieces per X row
+    const int cpr = feat_in / 8;  // 16-byte pieces per X row
     const int chunk = lane & 7;
-    int entry[8], off = 0;
-    auto entries_of = [&](int n) {
-      const int k = n / steps, sidx = n - k * steps;
-      const int kc = sidx * 8 + chunk;
-      const int rel = kc / cpr;
-      off = kc - rel * cpr;
-      const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
-      const bool in = rel < num_rels;
-      const int32_t* mp = map + (static_cast<size_t>(tile) * num_rels + (in ? rel : 0)) * kTM + gw * 32 + (lane >> 3);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int e = __ldg(mp + 4 * i);
-        entry[i] = in ? e : -1;
+    const int step_rel = groups * 8 / cpr, step_off = groups * 8 - step_rel * cpr;
+    const int tile_rel = steps * 8 / cpr, tile_off = steps * 8 - tile_rel * cpr;
+    int sidx = g, rel = (g * 8 + chunk) / cpr, off = g * 8 + chunk - rel * cpr;
+    int left = my_tiles;  // tiles from the one of this step on
+    const size_t tile_map = static_cast<size_t>(num_rels) * kTM;
+    const int32_t* mp = map + static_cast<size_t>(blockIdx.x) * tile_map + gw * 32 + (lane >> 3);
+    auto into_tile = [&]() {  // steps past the end of a tile belong to the block's next ones
+      while (left > 0 && sidx >= steps) {
+        sidx -= steps;
+        --left;
+        mp += tile_map * gridDim.x;
+        rel -= tile_rel;
+        off -= tile_off;
+        if (off < 0) { off += cpr; --rel; }
       }
     };
-    if (g < groups && g < total) entries_of(g);
-    for (int n = g; g < groups && n < total; n += groups) {
-      uint4 v[8];
+    int entry[8];
+    auto entries_of_step = [&]() {
+      const bool in = rel < num_rels;
+      const int32_t* e = mp + static_cast<size_t>(in ? rel : 0) * kTM;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        v[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (entry[i] >= 0)
-          v[i] = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(entry[i]) * feat_in) + off);
+        const int v = __ldg(e + 4 * i);
+        entry[i] = in ? v : -1;
       }
-      if (n + groups < total) entries_of(n + groups);
-      const int s = n % nstages, use = n / nstages;
-      if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
-      unsigned char* st = base + s * stride;
+    };
+    int s = g;
+    uint32_t phase = 0;
+    if (g < groups) into_tile();
+    if (g < groups && left > 0) entries_of_step();
+    while (g < groups && left > 0) {
+      const int piece = off;
+      int from[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) from[i] = entry[i];
+      sidx += groups;
+      rel += step_rel;
+      off += step_off;
+      if (off >= cpr) { off -= cpr; ++rel; }
+      into_tile();
+      if (left > 0) entries_of_step();
+      if (!tc05::mbar_wait(&bar_empty[s], phase ^ 1u)) { ok = false; break; }
+      const uint32_t st = tc05::smem_u32(base + s * stride);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = gw * 32 + 4 * i + (lane >> 3);
-        *reinterpret_cast<uint4*>(st + (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4)) = v[i];
+        const uint32_t dst = st + (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
+        const __half* src = x + static_cast<size_t>(max(from[i], 0)) * feat_in + piece * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(from[i] >= 0 ? 16u : 0u)
+                     : "memory");
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
       tc05::fence_async_smem();
       __syncwarp();
       if (lane == 0) arrive(&bar_full[s]);
+      s += groups;
+      if (s >= nstages) { s -= nstages; phase ^= 1u; }
     }
   } else if (warp >= 4) {
     // ---- epilogue: thread = tile row = TMEM lane, 32 columns at a time
@@ -255,15 +306,26 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<uint4*>(my_row + q * 16) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
         __syncwarp();
+        bool nan = false;
+#pragma unroll
+        for (int q = 0; q < 32; ++q) nan |= __uint_as_float(r[q]) != __uint_as_float(r[q]);
+        for (unsigned todo = __ballot_sync(0xffffffffu, nan && lane < nrows); todo != 0u; todo &= todo - 1u) {
+          const int lr = __ffs(todo) - 1;
+          const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
+          const int32_t* entries = map + static_cast<size_t>(tile) * num_rels * kTM + (warp & 3) * 32 + lr;
+          *reinterpret_cast<float*>(buf0 + ((warp & 3) * 32 + lr) * kOutStride + lane * 4) =
+              row_by_pairs(x, w, entries, num_rels, feat_in, feat_out, c0 + lane);
+          __syncwarp();
+        }
         write32(y, wbase, row_base, nrows, feat_out, c0, lane, add != 0);
       }
     }
   }
 
   const bool all_ok = !__syncthreads_or(!ok);
-  if (!all_ok && tid == 0) {
-    atomicAdd(&g_conv_timeouts, 1u);
-    // gave up: let the loads already issued land (bounded) before the block's memory is released
+  if (!all_ok) {
+    if (tid == 0) atomicAdd(&g_conv_timeouts, 1u);
+    // gave up: the loading thread lets the loads it has issued land (bounded) before the block's memory is released
     for (int it = max(0, armed - nstages); it < armed; ++it)
       tc05::mbar_wait(&bar_full[it % nstages], (it / nstages) & 1);
   }
@@ -273,7 +335,7 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
 }
 
 template <typename OutT>
-int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const int32_t* map, int m, int num_rels, int feat_in,
+int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const __half* w, const int32_t* map, int m, int num_rels, int feat_in,
            int feat_out, int add, cudaStream_t st) {
   static thread_local int configured_device = -1;
   int dev = 0;
@@ -289,7 +351,7 @@ int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const int32_t* map
   int tmem_cols = 32;
   while (tmem_cols < 2 * acc_cols) tmem_cols *= 2;
   const int grid = std::min(ceil_div(m, kTM), kNumSMs);
-  sparse_conv_kernel<OutT><<<grid, kThreads, smem, st>>>(tm_w, y, x, map, m, num_rels, feat_in, feat_out, tmem_cols,
+  sparse_conv_kernel<OutT><<<grid, kThreads, smem, st>>>(tm_w, y, x, w, map, m, num_rels, feat_in, feat_out, tmem_cols,
                                                         acc_cols, nstages, std::min(kGroups, nstages), add);
   SPTIR_LAUNCH_OK("sparse_conv_kernel");
   return 0;
@@ -334,6 +396,8 @@ extern "C" int sparsetir_sparse_conv_f16_raw(const void* w, const void* x, void*
                    CU_TENSOR_MAP_SWIZZLE_128B) != 0)
     return -1;
   if (y_is_f16)
-    return launch(tm_w, static_cast<__half*>(y), static_cast<const __half*>(x), map, m, num_rels, feat_in, feat_out, add, st);
-  return launch(tm_w, static_cast<float*>(y), static_cast<const __half*>(x), map, m, num_rels, feat_in, feat_out, add, st);
+    return launch(tm_w, static_cast<__half*>(y), static_cast<const __half*>(x), static_cast<const __half*>(w), map, m,
+                  num_rels, feat_in, feat_out, add, st);
+  return launch(tm_w, static_cast<float*>(y), static_cast<const __half*>(x), static_cast<const __half*>(w), map, m,
+                num_rels, feat_in, feat_out, add, st);
 }

@@ -74,6 +74,19 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, int m, int n, ui
          (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// True for one thread of a converged warp.  Unlike `lane == 0` it tells the compiler that a single
+// thread runs what follows, so the operands of an MMA need no handling per thread (the sparse
+// convolution with one or the other and no other change: 98 / 81 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

@@ -103,7 +103,8 @@ def neighbour_map(nbmaps, nbsizes, transposed: bool, num_outputs: int, device: t
     """The layer's pairs as ``sparsetir_sparse_conv_f16`` takes them, on ``device``: tiles of 128 outputs,
     ``map[(tile * K + k) * 128 + t]`` = input point of output ``tile * 128 + t`` at kernel offset ``k``,
     or -1; None when an (offset, output) pair repeats."""
-    maps = torch.as_tensor(nbmaps).to(device, torch.int64)
+    maps = nbmaps if isinstance(nbmaps, torch.Tensor) else torch.from_numpy(np.array(nbmaps, dtype=np.int64))
+    maps = maps.to(device, torch.int64)
     sizes = torch.as_tensor([int(s) for s in (nbsizes.tolist() if hasattr(nbsizes, "tolist") else nbsizes)],
                             dtype=torch.int64).to(device)
     offsets, pairs = len(sizes), int(sizes.sum())
@@ -114,12 +115,32 @@ def neighbour_map(nbmaps, nbsizes, transposed: bool, num_outputs: int, device: t
     return out if int((out >= 0).sum()) == pairs else None
 
 
+def map_pays(num_outputs: int, offsets: int, pairs: int, feat_in: int, feat_out: int) -> bool:
+    """Whether the kernel over the neighbour map is the faster one for these sizes.
+
+    It multiplies the full ``128 x (offsets * feat_in)`` operand of every tile whatever the share of
+    pairs; the buckets' tensor-core kernel pays per pair, but takes only multiples of 64 channels and
+    builds a map of its own on every call when ``feat_out >= 2 * feat_in``.  Measured on 5,000 to
+    100,000 points, 8 and 27 offsets, 10 to 60 % of the pairs (float16 result, us, map / buckets):
+    100,000 x 27, 64 -> 64 channels 56 / 43 at 20 %, 57 / 56 at 30 %, 57 / 85 at 60 %; 256 -> 256
+    270 / 184 at 30 %, 275 / 322 at 60 %; 5,000 x 8 13 / 25; 64 -> 96 and other channel counts
+    47 / 900 at 40 % of 8 offsets.  The two estimates follow these within about 15 %."""
+    if feat_in % 16 != 0 or feat_out % 32 != 0 or not 0 < feat_out <= 256 or feat_in <= 0:
+        return False
+    if feat_in % 64 != 0 or feat_out % 64 != 0 or feat_out >= 2 * feat_in:
+        return True
+    waves = -(-num_outputs // (128 * 148))  # tiles of 128 outputs on 148 SMs
+    by_map = 8.0 + waves * offsets * feat_in / 64 * (0.42 if feat_out > 128 else 0.33)
+    by_pairs = max(24.0, 18.0 + pairs * 1e-6 * (0.42 * feat_in + 0.38 * feat_out - 15.0))
+    return by_map <= by_pairs
+
+
 class SparseConvPlan:
     """The structure of one layer, converted once (host side) and kept on the device.
 
-    A layer whose (offset, output) pairs never repeat is kept as a neighbour map too: such a call is
-    one launch of ``sparsetir_sparse_conv_f16``, which writes its result, for every channel count
-    that this operator takes; all others run ``sparsetir_rgms_ell3d_f16`` on the ELL3D buckets.
+    A layer whose (offset, output) pairs never repeat is kept as a neighbour map too: where
+    ``map_pays`` says so a call is one launch of ``sparsetir_sparse_conv_f16``, which writes its
+    result; all others run ``sparsetir_rgms_ell3d_f16`` on the ELL3D buckets.
 
     ``plan(inputs, weights)`` then runs the operator; the maps of a layer do not change between
     calls, so the host conversion is not part of the steady state (the reference also converts
@@ -135,7 +156,10 @@ class SparseConvPlan:
         self.device = device if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.buckets = [tuple(torch.from_numpy(np.ascontiguousarray(a)).to(self.device) for a in bk)
                         for bk in host]
-        self._map = neighbour_map(nbmaps, nbsizes, bool(transposed), self.num_outputs, self.device)
+        # at most 1 GB: layers beyond that, and layers with repeated pairs, keep the buckets alone
+        self._map = None
+        if self.num_pairs > 0 and self.num_offsets * self.num_outputs <= 1 << 28:
+            self._map = neighbour_map(nbmaps, nbsizes, bool(transposed), self.num_outputs, self.device)
 
     def __call__(self, inputs: torch.Tensor, weights: torch.Tensor,
                  out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float16) -> torch.Tensor:
@@ -148,8 +172,9 @@ class SparseConvPlan:
             raise ValueError("inputs and weights disagree on feat_in")
         x = inputs.to(self.device, torch.float16).contiguous()
         w = weights.to(self.device, torch.float16).contiguous()
-        mapped = (self._map is not None and feat_in % 16 == 0 and feat_out % 32 == 0 and 0 < feat_in and 0 < feat_out <= 256
-                  and out_dtype in (torch.float16, torch.float32)
+        mapped = (self._map is not None
+                  and map_pays(self.num_outputs, self.num_offsets, self.num_pairs, feat_in, feat_out)
+                  and (out_dtype if out is None else out.dtype) in (torch.float16, torch.float32)
                   and (x.data_ptr() | w.data_ptr() | (0 if out is None else out.data_ptr())) % 16 == 0)
         add = out is not None
         if out is None:

@@ -46,6 +46,20 @@ def test_matches_a_float64_product(cuda_device, feat_in, feat_out, n_out, offset
     assert L.load().sparsetir_tc_timeouts(cuda_device.index or 0, L.ctypes.byref(count)) == 0 and count.value == 0
 
 
+def test_weights_that_are_not_finite_reach_their_own_pairs_only(cuda_device):
+    n, pairs = 300, torch.tensor([[5, 7], [9, 7], [2, 299]])
+    x = torch.full((n, 32), 0.5, device=cuda_device).half()
+    w = torch.full((2, 32, 64), 0.25, device=cuda_device).half()
+    w[1, 3, 40] = float("inf")
+    want = torch.zeros(n, 64, device=cuda_device)
+    want[7], want[299] = 8.0, 4.0
+    want[7, 40] = want[299, 40] = float("inf")
+    table = neighbour_map(pairs, [1, 2], False, n, cuda_device)
+    y = torch.empty(n * 64, device=cuda_device)
+    ops.sparse_conv_f16(w.view(-1), x.view(-1), y, table, n, 2, 32, 64, 0)
+    assert torch.equal(y.view(n, 64), want)
+
+
 def test_repeated_pairs_keep_the_buckets(cuda_device):
     pairs = torch.tensor([[0, 1], [2, 1], [1, 0]])
     assert neighbour_map(pairs, [2, 1], False, 3, cuda_device) is None
@@ -55,6 +69,21 @@ def test_repeated_pairs_keep_the_buckets(cuda_device):
     want[1] = (x[0].float() + x[2].float()) @ w[0].float()
     want[0] = x[1].float() @ w[1].float()
     torch.testing.assert_close(y, want, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("nbmaps,sizes", [(np.zeros((0, 2), np.int64), []), (np.zeros((0, 2), np.int64), [0, 0]),
+                                          (np.array([[0, 1], [2, 1], [1, 0]])[:, ::-1], [2, 1])])
+@pytest.mark.parametrize("feat_in,feat_out", [(64, 128), (256, 64), (32, 48)])
+def test_plans_of_few_pairs(cuda_device, nbmaps, sizes, feat_in, feat_out):
+    x = torch.rand(3, feat_in, device=cuda_device).half()
+    w = torch.rand(len(sizes), feat_in, feat_out, device=cuda_device).half() / 16
+    y = SparseConvPlan(nbmaps, sizes, True, 3, 3, device=cuda_device)(x, w, out_dtype=torch.float32)
+    want, at = torch.zeros(3, feat_out, dtype=torch.float64, device=cuda_device), 0
+    for k, size in enumerate(sizes):
+        for o, i in nbmaps[at:at + size].tolist():
+            want[o] += x[i].double() @ w[k].double()
+        at += size
+    torch.testing.assert_close(y.double(), want, rtol=1e-5, atol=1e-5)
 
 
 def test_shapes_it_does_not_take_are_refused(cuda_device):
