@@ -418,7 +418,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (lane == 0) ok = tc05::mbar_wait(&bar_full[stage], use & 1);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        if (lane == 0) {
+        if (tc05::elect_one()) {
           tc05::fence_after_sync();
           const uint64_t db_s = tc05::desc_advance(db0, stage * kPStageBytes);
 #pragma unroll

@@ -380,7 +380,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     }
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
+    if (tc05::elect_one()) {
       const uint32_t idesc = tc05::instr_desc(tc05::kFmtF16, kTM, feat_out, /*a_mn=*/0, /*b_mn=*/1);
       // Z box, K-major: rows of 128 bytes, groups of 8 rows 1024 bytes apart; 16 columns = 32 bytes per step
       const uint64_t dz0 = tc05::smem_desc_swizzled(tc05::smem_u32(base), 0, 1024, tc05::kSwizzle128B);
@@ -647,7 +647,7 @@ rgms_f16_os_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     }
   } else if (warp == 1) {
     // ---- MMA issuer: one accumulator per tile, summed over all relations and slices
-    if (lane == 0) {
+    if (tc05::elect_one()) {
       const uint32_t idesc = tc05::instr_desc(tc05::kFmtF16, kTM, feat_out, /*a_mn=*/0, /*b_mn=*/1);
       const uint64_t dz0 = tc05::smem_desc_swizzled(tc05::smem_u32(base), 0, 1024, tc05::kSwizzle128B);
       const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base) + kZBoxB, kWBoxB, 1024, tc05::kSwizzle128B);

@@ -221,7 +221,7 @@ rgms_fused_kernel(const float* __restrict__ a, const float* __restrict__ w,
 
   if (warp == 0) {
     // ---- MMA issuer
-    if (lane == 0) {
+    if (tc05::elect_one()) {
       // Two instructions per K-step: z * [W; Wlo]^T (N = 128: columns 0..63 receive z*W, columns
       // 64..127 z*Wlo) and zlo * W^T (N = 64, added to columns 0..63); the epilogue adds the halves.
       constexpr uint32_t idesc128 = tc05::instr_desc(tc05::kFmtTF32, kTM, 2 * kF, /*a_mn=*/0, /*b_mn=*/0);

@@ -325,7 +325,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
     }
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
+    if (tc05::elect_one()) {
       // Two instructions per K-step instead of three: z * [W; Wlo]^T (N = 128: columns 0..63
       // receive z*W, columns 64..127 z*Wlo) and zlo * W^T (N = 64, added to columns 0..63); the
       // epilogue adds the two column halves.  An MMA of this size costs about the same whatever
