@@ -37,7 +37,6 @@ namespace sptir {
 
 __device__ unsigned int g_tc_timeouts = 0;  // bounded waits that ran out, since module load
 int rgms_tc_timeouts(unsigned int* count);  // the same counter of rgms_tc.cu
-int tcspmm_timeouts(unsigned int* count);   // ... and of tcspmm.cu
 int rgms_f16_timeouts(unsigned int* count);  // ... and of rgms_f16.cu
 int rgms_fused_timeouts(unsigned int* count);  // ... and of rgms_fused.cu
 int conv_timeouts(unsigned int* count);        // ... and of sparse_conv.cu
@@ -592,14 +591,12 @@ extern "C" int sparsetir_tc_timeouts(int device_id, unsigned int* count) {
   unsigned int bsr = 0, rgms = 0;
   SPTIR_CUDA_OK(cudaMemcpyFromSymbol(&bsr, g_tc_timeouts, sizeof(unsigned int)));
   if (rgms_tc_timeouts(&rgms) != 0) return -1;
-  unsigned int tcs = 0;
-  if (tcspmm_timeouts(&tcs) != 0) return -1;
   unsigned int rh = 0;
   if (rgms_f16_timeouts(&rh) != 0) return -1;
   unsigned int rf = 0;
   if (rgms_fused_timeouts(&rf) != 0) return -1;
   unsigned int cv = 0;
   if (conv_timeouts(&cv) != 0) return -1;
-  *count = bsr + rgms + tcs + rh + rf + cv;
+  *count = bsr + rgms + rh + rf + cv;
   return 0;
 }

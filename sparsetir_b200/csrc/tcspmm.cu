@@ -5,223 +5,303 @@
 // (src/sparse/format.cc:353-429): every t-row tile keeps the sorted distinct columns it touches,
 // g at a time; A holds the t x g values (mask) of a group, `indices` its g source rows.
 //
-// Tensor-core mapping (g = 16, t = 8, 16 or 32, feat a multiple of 128).  A group is a
-// (t x 16) x (16 x F) product — far too short for M, so, as in the BSR kernel, it is computed
-// transposed: one thread block owns (row tile io, 128 features),
-//   D^T[f, ii] (128 x T, fp32 in TMEM)  +=  Bg^T[f, ji] (128 x 16)  *  A_jo[ii, ji]^T (16 x T)
-// one tcgen05.mma.kind::f16 (M = 128 features, N = T tile rows, K = 16 slots) per group; T is t
-// padded to 16 (the rows 8..15 of the A operand stay zero for t = 8).  The 16 gathered rows of B
-// are the MN-major operand (features contiguous), the group's A block the K-major one.
-// Operands travel global -> registers -> shared memory in the un-swizzled core-matrix layout
-// (whole 128-byte lines per load, conflict-free 16-byte stores: see bsrmm_tc.cu); a thread
-// keeps two groups in registers, three shared-memory stages, bounded mbarrier waits.
-// Row tiles with many groups (hub rows) are cut into chunks of 32 groups handled by different
-// thread blocks: a small planning kernel lists the extra chunks (and clears the output rows of
-// those tiles), the main launch has one block per tile plus one per possible extra chunk, and
-// the chunks of a cut tile add their partial results atomically.
+// Tensor-core form (g = 16, t = 8, 16 or 32, feat a multiple of 8).  Of a group's work the gather of
+// 16 rows of B is what costs: 2 KB per 64 features against 8 instructions of m16n8k16.  So the
+// operands never touch shared memory: a warp owns 64 features of a row tile and loads both
+// operands straight into the registers that the instruction reads.
+//  - Which slot of the group plays which k of the instruction is free as long as A and B agree: the four
+//    k's of a lane are four neighbouring slots, so a lane reads its part of a row of A as 8 bytes and
+//    its four source rows as 16 bytes of `indices`.
+//  - Which feature plays which column is free too: lane group n reads 16 bytes (8 features) of each
+//    of its rows, instruction j takes the j-th feature of every piece.  Whole 128-byte lines per row,
+//    and a lane ends with 8 consecutive features of a result row per 16-byte store.
+// Two groups are in flight per warp.  Row tiles of up to kLight groups are one warp's work; longer
+// ones (hub rows) are cut at multiples of kWindow groups of the whole matrix: a block owns a window,
+// its four warps share the part of each long tile that lies in it and meet in shared memory; parts
+// of a tile in several windows meet in a scratch buffer, where the block that counts in last adds them in
+// order.  One launch, no plan, every output written once, the same bits on every call.
+//
+// It replaces a tcgen05 kernel (one block per tile and 128 features, operands through shared memory,
+// atomics for hub tiles) whose steps waited for one another: PLACEHOLDER
+// Bound: the L2-to-SM gather of B and the latency of indptr -> indices -> B on small matrices.
 // Other shapes run on CUDA cores.
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "common.h"
-#include "tc05.cuh"
+#include "row_walk.cuh"
 #include "vec.cuh"
 
 namespace sptir {
-
-__device__ unsigned int g_tcspmm_timeouts = 0;
-
 namespace {
 
 constexpr int kThreads = 128;
 constexpr int kG = 16;
-constexpr int kTileF = 128;
-constexpr int kStages = 3;
-constexpr int kSets = 2;
-constexpr int kBBytes = kG * kTileF * 2;   // gathered rows of one group: 16 x 128 fp16 = 4 KB
-constexpr int kAMax = 32 * kG * 2;         // A block, T <= 32 rows: 1 KB
-constexpr int kStageBytes = kBBytes + kAMax;
-constexpr int kChunk = 32;                 // groups per thread block
-constexpr int kIdxCache = kChunk * kG;     // source rows of the block's groups
-// B operand (MN-major): core matrix (kc = ji/8, fc = f/8) at (kc*16 + fc)*128, slot ji%8 at
-// 16-byte stride inside it, 8 features contiguous
-constexpr uint32_t kB_SBO = 128, kB_LBO = 16 * 128;
+constexpr int kSlab = 64;     // features per warp
+constexpr int kLight = 16;    // longest tile of a single warp, in groups
+constexpr int kWindow = 128;  // groups per block of the long tiles
 
 template <typename OutT> __device__ __forceinline__ OutT to_out(float v);
 template <> __device__ __forceinline__ float to_out<float>(float v) { return v; }
 template <> __device__ __forceinline__ __half to_out<__half>(float v) { return __float2half_rn(v); }
 
-__device__ __forceinline__ void add_out(float* p, float v) { atomicAdd(p, v); }
-__device__ __forceinline__ void add_out(__half* p, float v) { atomicAdd(p, __float2half_rn(v)); }
+struct TcArgs {
+  const __half* a;
+  const __half* b;
+  void* c;
+  const int32_t* indptr;
+  const int32_t* indices;
+  float* part;         // two pieces per window and slab: of a tile that began before it, of one that goes on behind it
+  unsigned* counters;  // [windows][slabs], zero before and after every launch
+  int mb, nnzb, t, feat, slabs, windows;
+  float tiles_per_group;
+  bool vec_indices;    // `indices` is 16-byte aligned
+  bool vec_out;        // rows of C are made of whole 16-byte pieces
+};
 
-// Lists the chunks 1, 2, ... of every row tile with more than kChunk groups as (tile, chunk)
-// pairs and clears the output rows of those tiles (their chunks accumulate atomically).
-template <typename OutT>
-__global__ void __launch_bounds__(256)
-tcspmm_plan_kernel(const int32_t* __restrict__ indptr, int mb, int t, int feat, OutT* __restrict__ c,
-                   int* __restrict__ count, int2* __restrict__ list, int max_extra) {
-  const int io = blockIdx.x * 256 + threadIdx.x;
-  int ngrp = 0;
-  if (io < mb) ngrp = __ldg(indptr + io + 1) - __ldg(indptr + io);
-  const bool heavy = ngrp > kChunk;
-  if (heavy) {
-    const int extra = (ngrp + kChunk - 1) / kChunk - 1;
-    const int base = atomicAdd(count, extra);
-    for (int k = 0; k < extra; ++k)
-      if (base + k < max_extra) list[base + k] = make_int2(io, k + 1);
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// 8 consecutive results of row `ii` (inside the tile) from feature f on
+__device__ __forceinline__ void store8(const TcArgs& s, float* c, int io, int ii, int f, const float (&v)[8]) {
+  float* dst = c + (static_cast<size_t>(io) * s.t + ii) * s.feat + f;
+  if (s.vec_out) {
+    __stcs(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
+    __stcs(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dst[j] = v[j];
   }
-  unsigned todo = __ballot_sync(0xffffffffu, heavy);
-  const int lane = threadIdx.x & 31;
-  while (todo != 0) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const int tile = __shfl_sync(0xffffffffu, io, src);
-    OutT* dst = c + static_cast<size_t>(tile) * t * feat;
-    for (int e = lane; e < t * feat; e += 32) dst[e] = to_out<OutT>(0.f);
+}
+__device__ __forceinline__ void store8(const TcArgs& s, __half* c, int io, int ii, int f, const float (&v)[8]) {
+  __half* dst = c + (static_cast<size_t>(io) * s.t + ii) * s.feat + f;
+  if (s.vec_out) {
+    uint4 o;
+    __half2* h = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+    __stcs(reinterpret_cast<uint4*>(dst), o);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dst[j] = __float2half_rn(v[j]);
   }
 }
 
-template <int T, typename OutT>  // T = tile rows padded to a multiple of 16
-__global__ void __launch_bounds__(kThreads)
-tcspmm_tc_kernel(const __half* __restrict__ a, const __half* __restrict__ b, OutT* __restrict__ c,
-                 const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int t,
-                 int feat, int mb, const int* __restrict__ count, const int2* __restrict__ list,
-                 int max_extra) {
-  __shared__ __align__(128) unsigned char smem[kStages * kStageBytes];
-  __shared__ __align__(8) uint64_t bar_free[kStages];
-  __shared__ __align__(8) uint64_t bar_done;
-  __shared__ uint32_t s_tmem;
-  __shared__ int32_t s_idx[kIdxCache];
-  // blocks 0..mb-1: chunk 0 of tile blockIdx.x; the others: an entry of the list of extra chunks
-  int io = blockIdx.x, chunk = 0;
-  if (io >= mb) {
-    const int e = io - mb;
-    if (e >= min(__ldg(count), max_extra)) return;
-    const int2 w = list[e];
-    io = w.x;
-    chunk = w.y;
-  }
-  const int f0 = blockIdx.y * kTileF;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile_g0 = __ldg(indptr + io), tile_ngrp = __ldg(indptr + io + 1) - tile_g0;
-  const bool accumulate = tile_ngrp > kChunk;  // the tile is cut: partial results are added
-  const int g0 = tile_g0 + chunk * kChunk;
-  const int ngrp = min(kChunk, tile_ngrp - chunk * kChunk);
+// A slot that a row does not use has a zero in A, and 0 * B is NaN where B is not finite.  Results that
+// came out as NaN are formed again from the slots that the row does use: 8 features of one row.
+__device__ __noinline__ void by_slots(const TcArgs& s, int g0, int g1, int ii, int f, float* out) {
+  for (int j = 0; j < 8; ++j) out[j] = 0.f;
+  for (int g = g0; g < g1; ++g)
+    for (int ji = 0; ji < kG; ++ji) {
+      const float av = __half2float(s.a[(static_cast<size_t>(g) * s.t + ii) * kG + ji]);
+      if (av == 0.f) continue;
+      const __half* br = s.b + static_cast<size_t>(s.indices[static_cast<size_t>(g) * kG + ji]) * s.feat + f;
+      for (int j = 0; j < 8; ++j) out[j] = fmaf(av, __half2float(br[j]), out[j]);
+    }
+}
 
-  OutT* crow = c + (static_cast<size_t>(io) * t) * feat + f0 + warp * 32 + lane;
-  if (ngrp <= 0) {  // empty tile: zeros, no tensor-core work
-    for (int ii = 0; ii < t; ++ii) crow[static_cast<size_t>(ii) * feat] = to_out<OutT>(0.f);
+// MT = tiles of 16 rows.  acc[mt][j][c]: instruction j = feature j of every 8-feature piece; c = 0, 1:
+// row lane/4, pieces 2(lane%4) and the next; c = 2, 3: row lane/4 + 8.
+template <int MT>
+__device__ __forceinline__ void accumulate(const TcArgs& s, int g0, int g1, int f0, int lane, float (&acc)[MT][8][4]) {
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[mt][j][c] = 0.f;
+  const int q = lane & 3, r = lane >> 2;
+  const bool in = f0 + r * 8 < s.feat;
+  const __half* bl = s.b + (in ? f0 + r * 8 : 0);
+  auto ids_of = [&](int g) {
+    const int32_t* p = s.indices + static_cast<size_t>(g) * kG + q * 4;
+    if (s.vec_indices) return __ldg(reinterpret_cast<const int4*>(p));
+    return make_int4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  };
+  auto rows_of = [&](const int4& id, uint4 (&v)[4]) {
+    const int row[4] = {id.x, id.y, id.z, id.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (in) v[k] = __ldg(reinterpret_cast<const uint4*>(bl + static_cast<size_t>(row[k]) * s.feat));
+    }
+  };
+  auto values_of = [&](int g, uint32_t (&av)[MT][4]) {
+    const __half* p = s.a + (static_cast<size_t>(g) * s.t + r) * kG + q * 4;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const uint2 lo = __ldg(reinterpret_cast<const uint2*>(p + mt * 16 * kG));
+      uint2 hi = make_uint2(0u, 0u);
+      if (s.t >= 16) hi = __ldg(reinterpret_cast<const uint2*>(p + (mt * 16 + 8) * kG));
+      av[mt][0] = lo.x; av[mt][1] = hi.x; av[mt][2] = lo.y; av[mt][3] = hi.y;
+    }
+  };
+  auto multiply = [&](const uint4 (&v)[4], const uint32_t (&av)[MT][4]) {
+    auto one = [&](int j, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+      const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+      const uint32_t b0 = __byte_perm(w0, w1, sel), b1 = __byte_perm(w2, w3, sel);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) mma16816(acc[mt][j], av[mt], b0, b1);
+    };
+    one(0, v[0].x, v[1].x, v[2].x, v[3].x); one(1, v[0].x, v[1].x, v[2].x, v[3].x);
+    one(2, v[0].y, v[1].y, v[2].y, v[3].y); one(3, v[0].y, v[1].y, v[2].y, v[3].y);
+    one(4, v[0].z, v[1].z, v[2].z, v[3].z); one(5, v[0].z, v[1].z, v[2].z, v[3].z);
+    one(6, v[0].w, v[1].w, v[2].w, v[3].w); one(7, v[0].w, v[1].w, v[2].w, v[3].w);
+  };
+  int4 id0 = make_int4(0, 0, 0, 0), id1 = id0;
+  if (g0 < g1) id0 = ids_of(g0);
+  if (g0 + 1 < g1) id1 = ids_of(g0 + 1);
+  for (int g = g0; g < g1; g += 2) {
+    const bool two = g + 1 < g1;
+    uint4 v0[4], v1[4];
+    uint32_t a0[MT][4], a1[MT][4];
+    rows_of(id0, v0);
+    if (two) rows_of(id1, v1);
+    values_of(g, a0);
+    if (two) values_of(g + 1, a1);
+    if (g + 2 < g1) id0 = ids_of(g + 2);
+    if (g + 3 < g1) id1 = ids_of(g + 3);
+    multiply(v0, a0);
+    if (two) multiply(v1, a1);
+  }
+  bool nan = false;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) nan |= acc[mt][j][c] != acc[mt][j][c];
+  if (nan) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int ii = mt * 16 + r + (c >> 1) * 8, f = f0 + (2 * q + (c & 1)) * 8;
+        float out[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (ii < s.t && f < s.feat) by_slots(s, g0, g1, ii, f, out);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[mt][j][c] = out[j];
+      }
+  }
+}
+
+template <int MT, typename OutT>
+__global__ void __launch_bounds__(kThreads)
+tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
+  __shared__ float s_sum[4][MT][4][8][32];  // [warp][row tile][c][j][lane]
+  __shared__ unsigned s_seen;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slab = static_cast<int>(blockIdx.x) % s.slabs, unit = static_cast<int>(blockIdx.x) / s.slabs;
+  const int f0 = slab * kSlab;
+  const int q = lane & 3, r = lane >> 2;
+  OutT* c = static_cast<OutT*>(s.c);
+  float acc[MT][8][4];
+
+  if (unit >= s.windows) {  // ---- a short tile per warp
+    const int io = (unit - s.windows) * 4 + warp;
+    if (io >= s.mb) return;
+    const int g0 = __ldg(s.indptr + io), g1 = __ldg(s.indptr + io + 1);
+    if (g1 - g0 > kLight) return;
+    accumulate<MT>(s, g0, g1, f0, lane, acc);
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int ii = mt * 16 + r + (k >> 1) * 8, f = f0 + (2 * q + (k & 1)) * 8;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = acc[mt][j][k];
+        if (ii < s.t && f < s.feat) store8(s, c, io, ii, f, v);
+      }
     return;
   }
-  if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) tc05::mbar_init(&bar_free[s], 1);
-    tc05::mbar_init(&bar_done, 1);
-    tc05::fence_mbar_init();
-  }
-  if (warp == 0) tc05::tmem_alloc(&s_tmem, 32);
-  for (int i = tid; i < min(ngrp * kG, kIdxCache); i += kThreads)
-    s_idx[i] = __ldg(indices + static_cast<size_t>(g0) * kG + i);
-  // rows t..T-1 of the A operand are never loaded: they must read as zero
-  if (T != 0) {
-    for (int i = tid; i < kStages * kAMax / 16; i += kThreads) {
-      const int s = i / (kAMax / 16), r = i % (kAMax / 16);
-      *reinterpret_cast<uint4*>(smem + s * kStageBytes + kBBytes + r * 16) = make_uint4(0, 0, 0, 0);
-    }
-  }
-  tc05::fence_async_smem();
-  tc05::fence_before_sync();
-  __syncthreads();
-  tc05::fence_after_sync();
-  const uint32_t tmem = s_tmem;
 
-  // B: a load instruction k (k = 0, 1) covers rows 4k..4k+3 (+8 for warps 2, 3) x 8 chunks of 16
-  // bytes; store j writes the piece loaded by instruction j ^ (lane & 1) (see bsrmm_tc.cu)
-  const int b_fc = (warp & 1) * 8 + (lane & 7);
-  const int b_row0 = (warp >> 1) * 8 + (lane >> 3);
-  const bool b_odd = (lane & 1) != 0;
-  // A: piece p < 2t = (row ii = p / 2, 8-slot chunk kc = p % 2), 16 bytes
-  const int a_ii = tid >> 1, a_kc = tid & 1;
-  const bool a_mine = tid < 2 * t;
-  struct Pieces {
-    uint4 b[2];
-    uint4 a;
-  };
-  auto load_group = [&](int it, Pieces& x) {
+  // ---- a window: the long tiles that reach into it, one after the other
+  const int w0 = unit * kWindow, w1 = min(w0 + kWindow, s.nnzb);
+  int cur = warp_row_of(s.indptr, s.mb, w0, s.tiles_per_group, lane);
+  while (cur < s.mb) {
+    const int start = __ldg(s.indptr + min(cur + lane, s.mb)), end = __ldg(s.indptr + min(cur + lane + 1, s.mb));
+    unsigned todo = __ballot_sync(0xffffffffu, end - start > kLight && start < w1 && end > w0);
+    while (todo != 0u) {  // the same in all four warps
+      const int k = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const int io = cur + k;
+      const int g0 = __shfl_sync(0xffffffffu, start, k), g1 = __shfl_sync(0xffffffffu, end, k);
+      const int p0 = max(g0, w0), p1 = min(g1, w1), per = (p1 - p0 + 3) / 4;
+      accumulate<MT>(s, min(p1, p0 + warp * per), min(p1, p0 + (warp + 1) * per), f0, lane, acc);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int slot = it * kG + b_row0 + k * 4;
-      const int src = s_idx[slot];
-      x.b[k] = __ldg(reinterpret_cast<const uint4*>(b + static_cast<size_t>(src) * feat + f0 + b_fc * 8));
-    }
-    if (a_mine)
-      x.a = __ldg(reinterpret_cast<const uint4*>(a + (static_cast<size_t>(g0 + it) * t + a_ii) * kG + a_kc * 8));
-  };
-  auto store_group = [&](int stage, const Pieces& x) {
-    unsigned char* st = smem + stage * kStageBytes;
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const uint4 v = b_odd ? x.b[j ^ 1] : x.b[j];
-      const int row = b_row0 + (b_odd ? (j ^ 1) : j) * 4;  // slot ji of the piece
-      *reinterpret_cast<uint4*>(st + ((row >> 3) * 16 + b_fc) * 128 + (row & 7) * 16) = v;
-    }
-    // A operand (K-major): core matrix (kc, ng = ii/8) at (kc*(T/8) + ng)*128, row ii%8 at 16 bytes
-    if (a_mine)
-      *reinterpret_cast<uint4*>(st + kBBytes + (a_kc * (T / 8) + (a_ii >> 3)) * 128 + (a_ii & 7) * 16) = x.a;
-  };
-
-  constexpr uint32_t idesc = tc05::instr_desc(tc05::kFmtF16, kTileF, T, /*a_mn=*/1, /*b_mn=*/0);
-  const uint64_t da0 = tc05::smem_desc(tc05::smem_u32(smem), kB_LBO, kB_SBO);
-  const uint64_t db0 = tc05::smem_desc(tc05::smem_u32(smem) + kBBytes, (T / 8) * 128, 128);
-  bool ok = true;
-  auto step = [&](int it, Pieces& x) -> bool {
-    const int stage = it % kStages;
-    if (it >= kStages) {  // the MMA of group it-kStages was the previous reader of this stage
-      if (!tc05::mbar_wait(&bar_free[stage], ((it - kStages) / kStages) & 1)) ok = false;
-    }
-    if (ok) store_group(stage, x);
-    if (it + kSets < ngrp) load_group(it + kSets, x);
-    tc05::fence_async_smem();
-    if (__syncthreads_or(!ok)) return false;
-    if (warp == 0 && lane == 0) {
-      tc05::fence_after_sync();
-      tc05::mma_f16(tmem, tc05::desc_advance(da0, stage * kStageBytes),
-                    tc05::desc_advance(db0, stage * kStageBytes), idesc, it > 0 ? 1u : 0u);
-      tc05::mma_commit(&bar_free[stage]);
-      if (it == ngrp - 1) tc05::mma_commit(&bar_done);
-    }
-    return true;
-  };
-
-  Pieces x[kSets];
+        for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-  for (int k = 0; k < kSets; ++k) {
-    x[k].a = make_uint4(0, 0, 0, 0);
-    if (k < ngrp) load_group(k, x[k]);
-  }
-  for (int it = 0; it < ngrp && ok; it += kSets) {
+          for (int j = 0; j < 8; ++j) s_sum[warp][mt][cc][j][lane] = acc[mt][j][cc];
+      __syncthreads();
+      // warp w finishes the pieces c = w: row (lane/4 + 8 (w/2)), 8 features
+      const int e0 = g0 / kWindow, e1 = (g1 - 1) / kWindow;
+      float v[MT][8];
 #pragma unroll
-    for (int k = 0; k < kSets; ++k)
-      if (ok && it + k < ngrp && !step(it + k, x[k])) ok = false;  // uniform: ends in a barrier vote
-  }
-
-  if (ok && !tc05::mbar_wait(&bar_done, 0)) ok = false;
-  ok = !__syncthreads_or(!ok);
-  tc05::fence_after_sync();
-  if (ok) {
-    uint32_t r[32];
-    tc05::tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16), r);  // columns >= T: unused
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-    for (int ii = 0; ii < T; ++ii) {
-      if (ii < t) {
-        if (accumulate) add_out(crow + static_cast<size_t>(ii) * feat, __uint_as_float(r[ii]));
-        else crow[static_cast<size_t>(ii) * feat] = to_out<OutT>(__uint_as_float(r[ii]));
+        for (int j = 0; j < 8; ++j)
+          v[mt][j] = (s_sum[0][mt][warp][j][lane] + s_sum[1][mt][warp][j][lane]) +
+                     (s_sum[2][mt][warp][j][lane] + s_sum[3][mt][warp][j][lane]);
+      bool mine = true;
+      if (e0 != e1) {
+        // a piece: 8 floats per (row tile, warp, lane), the layout of v
+        auto piece = [&](int e, int mt) {
+          const size_t slot = (static_cast<size_t>(2 * e + (e == e0 ? 1 : 0)) * s.slabs + slab) * MT + mt;
+          return reinterpret_cast<float4*>(s.part) + (slot * kThreads + threadIdx.x) * 2;
+        };
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          __stcg(piece(unit, mt), make_float4(v[mt][0], v[mt][1], v[mt][2], v[mt][3]));
+          __stcg(piece(unit, mt) + 1, make_float4(v[mt][4], v[mt][5], v[mt][6], v[mt][7]));
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          unsigned* counter = s.counters + static_cast<size_t>(e0) * s.slabs + slab;
+          s_seen = atomicAdd(counter, 1u);
+          if (s_seen == static_cast<unsigned>(e1 - e0)) *counter = 0u;  // last piece to arrive
+        }
+        __syncthreads();
+        mine = s_seen == static_cast<unsigned>(e1 - e0);
+        if (mine) {
+          __threadfence();
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[mt][j] = 0.f;
+#pragma unroll 4
+            for (int e = e0; e <= e1; ++e) {
+              const float4 x = __ldcg(piece(e, mt)), y = __ldcg(piece(e, mt) + 1);
+              v[mt][0] += x.x; v[mt][1] += x.y; v[mt][2] += x.z; v[mt][3] += x.w;
+              v[mt][4] += y.x; v[mt][5] += y.y; v[mt][6] += y.z; v[mt][7] += y.w;
+            }
+          }
+        }
       }
+      if (mine) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int ii = mt * 16 + r + (warp >> 1) * 8, f = f0 + (2 * q + (warp & 1)) * 8;
+          if (ii < s.t && f < s.feat) store8(s, c, io, ii, f, v[mt]);
+        }
+      }
+      __syncthreads();  // the meeting place is free for the next tile
     }
-  } else if (tid == 0) {
-    atomicAdd(&g_tcspmm_timeouts, 1u);
+    const int last = __shfl_sync(0xffffffffu, end, 31);
+    if (last >= w1) break;
+    // 32 tiles on; over a run of empty tiles with a search
+    const bool empty = last == __shfl_sync(0xffffffffu, start, 0);
+    const int next = empty ? warp_row_of(s.indptr, s.mb, last, s.tiles_per_group, lane) : 0;
+    cur = max(cur + 32, next);
   }
-  tc05::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tc05::tmem_dealloc(tmem, 32);
 }
 
 // CUDA-core form for every other shape: a block per row tile; a thread owns output elements
@@ -248,29 +328,46 @@ tcspmm_simt_kernel(const __half* __restrict__ a, const __half* __restrict__ b, O
   }
 }
 
+template <int MT, typename OutT>
+int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
+  s.slabs = ceil_div(s.feat, kSlab);
+  s.windows = ceil_div(s.nnzb, kWindow);
+  s.tiles_per_group = s.nnzb > 0 ? static_cast<float>(s.mb) / static_cast<float>(s.nnzb) : 0.f;
+  const long long blocks = (static_cast<long long>(s.windows) + ceil_div(s.mb, 4)) * s.slabs;
+  if (blocks > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
+  const size_t part_bytes = 2 * static_cast<size_t>(s.windows) * s.slabs * MT * kThreads * 8 * sizeof(float);
+  const size_t counter_bytes = static_cast<size_t>(s.windows) * s.slabs * sizeof(unsigned);
+  char* own = nullptr;
+  if (!workspace_fits(device_id, st, part_bytes, counter_bytes)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+      // the library's buffers cannot grow inside a capture: this call gets memory that the graph owns
+      const size_t at = (part_bytes + 255) & ~static_cast<size_t>(255);
+      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + std::max<size_t>(counter_bytes, 4), st));
+      SPTIR_CUDA_OK(cudaMemsetAsync(own + at, 0, counter_bytes, st));
+      s.part = reinterpret_cast<float*>(own);
+      s.counters = reinterpret_cast<unsigned*>(own + at);
+    }
+  }
+  if (own == nullptr) {
+    s.part = static_cast<float*>(workspace(device_id, st, part_bytes));
+    s.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
+    if (s.part == nullptr || s.counters == nullptr) return -1;
+  }
+  tcspmm_mma_kernel<MT, OutT><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(s);
+  SPTIR_LAUNCH_OK("tcspmm_mma_kernel");
+  if (own != nullptr) SPTIR_CUDA_OK(cudaFreeAsync(own, st));
+  return 0;
+}
+
 template <typename OutT>
 int launch_all(const __half* a, const __half* b, OutT* c, const int32_t* indptr, const int32_t* indices,
                int mb, int nnzb, int t, int g, int feat, int device_id, cudaStream_t st) {
-  const bool tc = g == kG && (t == 8 || t == 16 || t == 32) && feat % kTileF == 0 &&
-                  feat / kTileF <= 65535 && aligned16(a) && aligned16(b);
-  if (tc) {
-    // work list of the extra chunks of cut tiles: at most nnzb / kChunk entries
-    const int max_extra = nnzb / kChunk + 1;
-    char* ws = static_cast<char*>(workspace(device_id, st, 16 + static_cast<size_t>(max_extra) * sizeof(int2)));
-    if (!ws) return -1;
-    int* count = reinterpret_cast<int*>(ws);
-    int2* list = reinterpret_cast<int2*>(ws + 16);
-    SPTIR_CUDA_OK(cudaMemsetAsync(count, 0, sizeof(int), st));
-    tcspmm_plan_kernel<OutT><<<ceil_div(mb, 256), 256, 0, st>>>(indptr, mb, t, feat, c, count, list, max_extra);
-    SPTIR_LAUNCH_OK("tcspmm_plan_kernel");
-    if (static_cast<long long>(mb) + max_extra > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
-    dim3 grid(mb + max_extra, feat / kTileF);
-    if (t <= 16)
-      tcspmm_tc_kernel<16, OutT><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, t, feat, mb, count, list, max_extra);
-    else
-      tcspmm_tc_kernel<32, OutT><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, t, feat, mb, count, list, max_extra);
-    SPTIR_LAUNCH_OK("tcspmm_tc_kernel");
-    return 0;
+  if (g == kG && (t == 8 || t == 16 || t == 32) && feat % 8 == 0 && aligned16(a) && aligned16(b)) {
+    const TcArgs s{a, b, c, indptr, indices, nullptr, nullptr, mb, nnzb, t, feat, 0, 0, 0.f, aligned16(indices), aligned16(c)};
+    if (t == 32) return launch_mma<2, OutT>(s, device_id, st);
+    return launch_mma<1, OutT>(s, device_id, st);
   }
   tcspmm_simt_kernel<OutT><<<mb, 256, 0, st>>>(a, b, c, indptr, indices, t, g, feat);
   SPTIR_LAUNCH_OK("tcspmm_simt_kernel");
@@ -278,12 +375,6 @@ int launch_all(const __half* a, const __half* b, OutT* c, const int32_t* indptr,
 }
 
 }  // namespace
-
-int tcspmm_timeouts(unsigned int* count) {
-  SPTIR_CUDA_OK(cudaMemcpyFromSymbol(count, g_tcspmm_timeouts, sizeof(unsigned int)));
-  return 0;
-}
-
 }  // namespace sptir
 
 extern "C" int sparsetir_tcspmm_raw(const void* a_f16, const void* b_f16, void* c, int c_is_f16,
