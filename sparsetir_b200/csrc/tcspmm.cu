@@ -16,14 +16,18 @@
 //    of its rows, instruction j takes the j-th feature of every piece.  Whole 128-byte lines per row,
 //    and a lane ends with 8 consecutive features of a result row per 16-byte store.
 // Two groups are in flight per warp.  Row tiles of up to kLight groups are one warp's work; longer
-// ones (hub rows) are cut at multiples of kWindow groups of the whole matrix: a block owns a window,
+// ones (hub rows) are cut at multiples of a window of groups of the whole matrix: a block owns a window,
 // its four warps share the part of each long tile that lies in it and meet in shared memory; parts
 // of a tile in several windows meet in a scratch buffer, where the block that counts in last adds them in
 // order.  One launch, no plan, every output written once, the same bits on every call.
 //
 // It replaces a tcgen05 kernel (one block per tile and 128 features, operands through shared memory,
-// atomics for hub tiles) whose steps waited for one another: PLACEHOLDER
-// Bound: the L2-to-SM gather of B and the latency of indptr -> indices -> B on small matrices.
+// atomics for hub tiles) whose steps waited for one another, and CUDA-core code for the feature counts
+// that are not multiples of 128.  Power-law graphs, float16 result, us, before / now: 169 k rows (57,508
+// groups) F = 64 6010 / 32, F = 128 137 / 61, F = 512 422 / 222; 20 k rows F = 128 52 / 14; 3 k rows 39 / 9.
+// Bound: the round trips indptr -> indices -> B of a short tile, with 20 warps of two groups per SM in
+// flight; 4.5 TB/s of gathered operands at F = 128.  Slower: neighbouring short tiles as one stream per
+// warp (72 us at F = 128), 16 or 24 warps per SM (66, 111), windows of 32 groups at this size (68).
 // Other shapes run on CUDA cores.
 #include <cuda_fp16.h>
 
@@ -40,7 +44,6 @@ constexpr int kThreads = 128;
 constexpr int kG = 16;
 constexpr int kSlab = 64;     // features per warp
 constexpr int kLight = 16;    // longest tile of a single warp, in groups
-constexpr int kWindow = 128;  // groups per block of the long tiles
 
 template <typename OutT> __device__ __forceinline__ OutT to_out(float v);
 template <> __device__ __forceinline__ float to_out<float>(float v) { return v; }
@@ -55,6 +58,7 @@ struct TcArgs {
   float* part;         // two pieces per window and slab: of a tile that began before it, of one that goes on behind it
   unsigned* counters;  // [windows][slabs], zero before and after every launch
   int mb, nnzb, t, feat, slabs, windows;
+  int window_log;      // groups per block of the long tiles: 2^window_log
   float tiles_per_group;
   bool vec_indices;    // `indices` is 16-byte aligned
   bool vec_out;        // rows of C are made of whole 16-byte pieces
@@ -93,22 +97,30 @@ __device__ __forceinline__ void store8(const TcArgs& s, __half* c, int io, int i
 }
 
 // A slot that a row does not use has a zero in A, and 0 * B is NaN where B is not finite.  Results that
-// came out as NaN are formed again from the slots that the row does use: 8 features of one row.
-__device__ __noinline__ void by_slots(const TcArgs& s, int g0, int g1, int ii, int f, float* out) {
-  for (int j = 0; j < 8; ++j) out[j] = 0.f;
+// came out as NaN are formed again from the slots that the row does use: out[j * stride] = the sum over
+// the groups [g0, g1) for feature f + j of row ii.  Apart from the main loop, so that it costs no
+// registers there.
+template <typename OutT>
+__device__ __noinline__ void by_slots(const TcArgs& s, int g0, int g1, int ii, int f, OutT* out, int stride) {
+  float sum[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sum[j] = 0.f;
   for (int g = g0; g < g1; ++g)
     for (int ji = 0; ji < kG; ++ji) {
       const float av = __half2float(s.a[(static_cast<size_t>(g) * s.t + ii) * kG + ji]);
       if (av == 0.f) continue;
       const __half* br = s.b + static_cast<size_t>(s.indices[static_cast<size_t>(g) * kG + ji]) * s.feat + f;
-      for (int j = 0; j < 8; ++j) out[j] = fmaf(av, __half2float(br[j]), out[j]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[j] = fmaf(av, __half2float(br[j]), sum[j]);
     }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) out[j * stride] = to_out<OutT>(sum[j]);
 }
 
-// MT = tiles of 16 rows.  acc[mt][j][c]: instruction j = feature j of every 8-feature piece; c = 0, 1:
+// True if a result of this lane is a NaN.  MT = tiles of 16 rows.  acc[mt][j][c]: instruction j = feature j of every 8-feature piece; c = 0, 1:
 // row lane/4, pieces 2(lane%4) and the next; c = 2, 3: row lane/4 + 8.
 template <int MT>
-__device__ __forceinline__ void accumulate(const TcArgs& s, int g0, int g1, int f0, int lane, float (&acc)[MT][8][4]) {
+__device__ __forceinline__ bool accumulate(const TcArgs& s, int g0, int g1, int f0, int lane, float (&acc)[MT][8][4]) {
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -176,22 +188,11 @@ __device__ __forceinline__ void accumulate(const TcArgs& s, int g0, int g1, int 
     for (int j = 0; j < 8; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) nan |= acc[mt][j][c] != acc[mt][j][c];
-  if (nan) {
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int ii = mt * 16 + r + (c >> 1) * 8, f = f0 + (2 * q + (c & 1)) * 8;
-        float out[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (ii < s.t && f < s.feat) by_slots(s, g0, g1, ii, f, out);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[mt][j][c] = out[j];
-      }
-  }
+  return nan;
 }
 
 template <int MT, typename OutT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, MT == 1 ? 5 : 2)
 tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   __shared__ float s_sum[4][MT][4][8][32];  // [warp][row tile][c][j][lane]
   __shared__ unsigned s_seen;
@@ -207,7 +208,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
     if (io >= s.mb) return;
     const int g0 = __ldg(s.indptr + io), g1 = __ldg(s.indptr + io + 1);
     if (g1 - g0 > kLight) return;
-    accumulate<MT>(s, g0, g1, f0, lane, acc);
+    const bool nan = accumulate<MT>(s, g0, g1, f0, lane, acc);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -218,11 +219,17 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
         for (int j = 0; j < 8; ++j) v[j] = acc[mt][j][k];
         if (ii < s.t && f < s.feat) store8(s, c, io, ii, f, v);
       }
+    if (nan) {
+      for (int k = 0; k < 4 * MT; ++k) {
+        const int ii = (k >> 2) * 16 + r + (k >> 1 & 1) * 8, f = f0 + (2 * q + (k & 1)) * 8;
+        if (ii < s.t && f < s.feat) by_slots(s, g0, g1, ii, f, c + (static_cast<size_t>(io) * s.t + ii) * s.feat + f, 1);
+      }
+    }
     return;
   }
 
   // ---- a window: the long tiles that reach into it, one after the other
-  const int w0 = unit * kWindow, w1 = min(w0 + kWindow, s.nnzb);
+  const int w0 = unit << s.window_log, w1 = w0 + min(1 << s.window_log, s.nnzb - w0);
   int cur = warp_row_of(s.indptr, s.mb, w0, s.tiles_per_group, lane);
   while (cur < s.mb) {
     const int start = __ldg(s.indptr + min(cur + lane, s.mb)), end = __ldg(s.indptr + min(cur + lane + 1, s.mb));
@@ -233,16 +240,23 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
       const int io = cur + k;
       const int g0 = __shfl_sync(0xffffffffu, start, k), g1 = __shfl_sync(0xffffffffu, end, k);
       const int p0 = max(g0, w0), p1 = min(g1, w1), per = (p1 - p0 + 3) / 4;
-      accumulate<MT>(s, min(p1, p0 + warp * per), min(p1, p0 + (warp + 1) * per), f0, lane, acc);
+      const int q0 = min(p1, p0 + warp * per), q1 = min(p1, q0 + per);
+      const bool nan = accumulate<MT>(s, q0, q1, f0, lane, acc);
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
           for (int j = 0; j < 8; ++j) s_sum[warp][mt][cc][j][lane] = acc[mt][j][cc];
+      if (nan) {
+        for (int k = 0; k < 4 * MT; ++k) {
+          const int ii = (k >> 2) * 16 + r + (k >> 1 & 1) * 8, f = f0 + (2 * q + (k & 1)) * 8;
+          if (ii < s.t && f < s.feat) by_slots(s, q0, q1, ii, f, &s_sum[warp][k >> 2][k & 3][0][lane], 32);
+        }
+      }
       __syncthreads();
       // warp w finishes the pieces c = w: row (lane/4 + 8 (w/2)), 8 features
-      const int e0 = g0 / kWindow, e1 = (g1 - 1) / kWindow;
+      const int e0 = g0 >> s.window_log, e1 = (g1 - 1) >> s.window_log;
       float v[MT][8];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
@@ -331,7 +345,11 @@ tcspmm_simt_kernel(const __half* __restrict__ a, const __half* __restrict__ b, O
 template <int MT, typename OutT>
 int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
   s.slabs = ceil_div(s.feat, kSlab);
-  s.windows = ceil_div(s.nnzb, kWindow);
+  // Windows of 128 groups keep the scratch small; down to 32 where there would not be enough blocks
+  // (20 k rows, 6,118 groups, F = 64: 12.4 against 18.9 us).
+  s.window_log = 5;
+  while (s.window_log < 7 && (static_cast<long long>(s.nnzb) * s.slabs >> s.window_log) > 4 * kNumSMs) ++s.window_log;
+  s.windows = ceil_div(s.nnzb, 1 << s.window_log);
   s.tiles_per_group = s.nnzb > 0 ? static_cast<float>(s.mb) / static_cast<float>(s.nnzb) : 0.f;
   const long long blocks = (static_cast<long long>(s.windows) + ceil_div(s.mb, 4)) * s.slabs;
   if (blocks > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
@@ -365,7 +383,7 @@ template <typename OutT>
 int launch_all(const __half* a, const __half* b, OutT* c, const int32_t* indptr, const int32_t* indices,
                int mb, int nnzb, int t, int g, int feat, int device_id, cudaStream_t st) {
   if (g == kG && (t == 8 || t == 16 || t == 32) && feat % 8 == 0 && aligned16(a) && aligned16(b)) {
-    const TcArgs s{a, b, c, indptr, indices, nullptr, nullptr, mb, nnzb, t, feat, 0, 0, 0.f, aligned16(indices), aligned16(c)};
+    const TcArgs s{a, b, c, indptr, indices, nullptr, nullptr, mb, nnzb, t, feat, 0, 0, 0, 0.f, aligned16(indices), aligned16(c)};
     if (t == 32) return launch_mma<2, OutT>(s, device_id, st);
     return launch_mma<1, OutT>(s, device_id, st);
   }
