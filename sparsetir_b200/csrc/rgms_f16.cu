@@ -23,8 +23,8 @@
 //       of four warps take the even / odd tiles out of TMEM and add them to Y.
 // A single one-column bucket whose (relation, destination) pairs never repeat and whose values
 // are 0 / 1 can also be computed destination-stationary, without reductions (rgms_f16_os_kernel).
-// Shapes the tensor-core launch does not take (feat_in or feat_out not a multiple of 64, feat_out
-// above 256, unaligned operands) go through a CUDA-core transform with the same Z.
+// Shapes the tensor-core launch does not take (feat_in not a multiple of 16, feat_out not a multiple of
+// 32 or above 256, unaligned operands) go through a CUDA-core transform with the same Z.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -62,6 +62,23 @@ __device__ __forceinline__ int bucket_of(const BucketTable& tb, int q) {
   return b;
 }
 
+// ranges[b * R + r] = first Z row of relation r inside bucket b, ranges[nb * R] = total rows: one block
+__device__ __forceinline__ void write_ranges(const BucketTable& tb, int num_rels, int32_t* __restrict__ ranges) {
+  for (int e = threadIdx.x; e <= tb.nb * num_rels; e += kThreads) {
+    if (e == tb.nb * num_rels) {
+      ranges[e] = tb.z_base[tb.nb];
+      continue;
+    }
+    const int b = e / num_rels, r = e % num_rels;
+    int lo = 0, hi = tb.num_groups[b];  // first group of the bucket with mid >= r
+    while (lo < hi) {
+      const int m = lo + (hi - lo) / 2;
+      if (__ldg(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
+    }
+    ranges[e] = tb.z_base[b] + lo * tb.rows_per_group[b];
+  }
+}
+
 // ---- launch (1).  A thread owns VEC consecutive features of one Z row; consecutive threads own
 // consecutive pieces of the same row.  The last block computes the (bucket, relation) ranges:
 // ranges[b * R + r] = first Z row of relation r inside bucket b, ranges[nb * R] = total rows.
@@ -71,19 +88,7 @@ gather_rows_f16_kernel(const __grid_constant__ BucketTable tb, const __half* __r
                        __half* __restrict__ z, int32_t* __restrict__ all_rows,
                        int32_t* __restrict__ ranges, int num_rels, int feat_in) {
   if (blockIdx.x == gridDim.x - 1) {
-    for (int e = threadIdx.x; e <= tb.nb * num_rels; e += kThreads) {
-      if (e == tb.nb * num_rels) {
-        ranges[e] = tb.z_base[tb.nb];
-        continue;
-      }
-      const int b = e / num_rels, r = e % num_rels;
-      int lo = 0, hi = tb.num_groups[b];  // first group of the bucket with mid >= r
-      while (lo < hi) {
-        const int m = lo + (hi - lo) / 2;
-        if (__ldg(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
-      }
-      ranges[e] = tb.z_base[b] + lo * tb.rows_per_group[b];
-    }
+    write_ranges(tb, num_rels, ranges);
     return;
   }
   // a block walks tiles of kThreads / chunks consecutive rows; 32-bit index arithmetic only
@@ -139,6 +144,112 @@ gather_rows_f16_kernel(const __grid_constant__ BucketTable tb, const __half* __r
   }
 }
 
+// ---- launch (1) for rows of whole 16-byte pieces: the same outputs as gather_rows_f16_kernel<8>, with
+// the same order of addition, and several X rows in flight per thread.  A tile of the grid is
+// kThreads / chunks lanes of rows x R rows of ONE bucket, so its width is uniform and the loads of
+// R rows x W slots (8 of them, or 8 slots at a time of a wider row) are issued together; with one row
+// after the other the chain ids -> X row was waited for once per row (1.5 M edges, 1.2 M rows of 64
+// features: the call 122 -> 105 us).  Bound: the L2 gather of X and the write of Z.
+struct GatherTiles {
+  int32_t first[kMaxBuckets + 1];  // first tile of every bucket
+};
+__host__ __device__ __forceinline__ int rows_in_flight(int width) { return width == 1 || width == 2 ? 4 : (width <= 4 ? 2 : 1); }
+
+__device__ __forceinline__ void add_piece(float (&acc)[8], float av, const uint4& raw) {
+  const __half2* h = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const float2 f = __half22float2(h[v]);
+    acc[2 * v] = fmaf(av, f.x, acc[2 * v]);
+    acc[2 * v + 1] = fmaf(av, f.y, acc[2 * v + 1]);
+  }
+}
+__device__ __forceinline__ uint4 pack_piece(const float (&acc)[8]) {
+  uint4 out;
+  __half2* h = reinterpret_cast<__half2*>(&out);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) h[v] = __floats2half2_rn(acc[2 * v], acc[2 * v + 1]);
+  return out;
+}
+
+// R rows (step apart, from e on) of W >= width slots each; slots past the width are not read
+template <int W, int R>
+__device__ __forceinline__ void gather_few(const __half* __restrict__ a, const int32_t* __restrict__ cols,
+                                           const uint4* __restrict__ x, uint4* __restrict__ z, unsigned e, unsigned step,
+                                           unsigned rows, int width, int chunks) {
+  float av[R][W];
+  int col[R][W];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      const unsigned row = e + r * step;
+      const bool in = row < rows && j < width;
+      const size_t at = in ? static_cast<size_t>(row) * width + j : 0;
+      av[r][j] = __half2float(__ldg(a + at));
+      col[r][j] = __ldg(cols + at);
+    }
+  uint4 raw[R][W];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < W; ++j) raw[r][j] = __ldg(x + static_cast<size_t>(col[r][j]) * chunks);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned row = e + r * step;
+    if (row >= rows) continue;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (j < width) add_piece(acc, av[r][j], raw[r][j]);
+    z[static_cast<size_t>(row) * chunks] = pack_piece(acc);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
+                        const __half* __restrict__ x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
+                        int32_t* __restrict__ ranges, int num_rels, int chunks) {
+  if (blockIdx.x == gridDim.x - 1) {
+    write_ranges(tb, num_rels, ranges);
+    return;
+  }
+  const int lanes = kThreads / chunks;  // rows side by side
+  const int rl = static_cast<int>(threadIdx.x) / chunks, ch = static_cast<int>(threadIdx.x) % chunks;
+  int b = 0;
+  while (b + 1 < tb.nb && static_cast<int>(blockIdx.x) >= gt.first[b + 1]) ++b;
+  const int width = tb.width[b], rows = tb.z_base[b + 1] - tb.z_base[b];
+  const int R = rows_in_flight(width);
+  const int e0 = (static_cast<int>(blockIdx.x) - gt.first[b]) * (lanes * R);
+  for (int i = threadIdx.x; i < lanes * R && i < rows - e0; i += kThreads)
+    all_rows[tb.z_base[b] + e0 + i] = __ldg(tb.rows[b] + e0 + i);
+  const unsigned e = static_cast<unsigned>(e0) + rl;
+  if (rl >= lanes || e >= static_cast<unsigned>(rows)) return;
+  const uint4* xv = reinterpret_cast<const uint4*>(x) + ch;
+  uint4* zv = reinterpret_cast<uint4*>(z) + static_cast<size_t>(tb.z_base[b]) * chunks + ch;
+  if (width == 1) return gather_few<1, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+  if (width == 2) return gather_few<2, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+  if (width <= 4) return gather_few<4, 2>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+  const __half* ap = tb.a[b] + static_cast<size_t>(e) * width;
+  const int32_t* cp = tb.cols[b] + static_cast<size_t>(e) * width;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  int j = 0;
+  for (; j + 8 <= width; j += 8) {
+    float av[8];
+    uint4 raw[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      av[u] = __half2float(__ldg(ap + j + u));
+      raw[u] = __ldg(xv + static_cast<size_t>(__ldg(cp + j + u)) * chunks);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) add_piece(acc, av[u], raw[u]);
+  }
+  for (; j < width; ++j)
+    add_piece(acc, __half2float(__ldg(ap + j)), __ldg(xv + static_cast<size_t>(__ldg(cp + j)) * chunks));
+  zv[static_cast<size_t>(e) * chunks] = pack_piece(acc);
+}
+
 // ---- launch (1) when every bucket has one column per row (the sparse-convolution shape): the Z
 // row is the X row times one value.  A thread owns one 16-byte piece of R rows that lie
 // kThreads / chunks rows apart and keeps the R chains (value, column id -> X row) in flight
@@ -149,19 +260,7 @@ scale_rows_f16_kernel(const __grid_constant__ BucketTable tb, const __half* __re
                       __half* __restrict__ z, int32_t* __restrict__ all_rows,
                       int32_t* __restrict__ ranges, int num_rels, int feat_in) {
   if (blockIdx.x == gridDim.x - 1) {
-    for (int e = threadIdx.x; e <= tb.nb * num_rels; e += kThreads) {
-      if (e == tb.nb * num_rels) {
-        ranges[e] = tb.z_base[tb.nb];
-        continue;
-      }
-      const int b = e / num_rels, r = e % num_rels;
-      int lo = 0, hi = tb.num_groups[b];
-      while (lo < hi) {
-        const int m = lo + (hi - lo) / 2;
-        if (__ldg(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
-      }
-      ranges[e] = tb.z_base[b] + lo * tb.rows_per_group[b];
-    }
+    write_ranges(tb, num_rels, ranges);
     return;
   }
   const int chunks = feat_in / 8;                     // <= kThreads (checked by the caller)
@@ -324,7 +423,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
   __shared__ int s_tile[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* base = smem_raw + ((1024u - (tc05::smem_u32(smem_raw) & 1023u)) & 1023u);
-  const int nkc = feat_in / kKC, nwb = feat_out / 64;
+  const int nkc = (feat_in + kKC - 1) / kKC, nwb = (feat_out + 63) / 64;
 
   if (warp == 0) {
     int rel, row0, row1;
@@ -398,9 +497,10 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
           tc05::fence_after_sync();
           const uint64_t dz = tc05::desc_advance(dz0, s * kStageB);
           const uint64_t dw = tc05::desc_advance(dw0, s * kStageB);
+          const int ksteps = min(kKC, feat_in - c * kKC) / 16;  // the last slice may be short
 #pragma unroll
           for (int ks = 0; ks < kKC / 16; ++ks)
-            tc05::mma_f16(acc, tc05::desc_advance(dz, ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
+            if (ks < ksteps) tc05::mma_f16(acc, tc05::desc_advance(dz, ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
                           (c > 0 || ks > 0) ? 1u : 0u);
           tc05::mma_commit(&bar_empty[s]);
         }
@@ -761,19 +861,7 @@ namespace {
 // ranges[b * R + r] for every bucket (what the last block of the gather launches computes)
 __global__ void __launch_bounds__(kThreads)
 bucket_ranges_kernel(const __grid_constant__ BucketTable tb, int num_rels, int32_t* __restrict__ ranges) {
-  for (int e = threadIdx.x; e <= tb.nb * num_rels; e += kThreads) {
-    if (e == tb.nb * num_rels) {
-      ranges[e] = tb.z_base[tb.nb];
-      continue;
-    }
-    const int b = e / num_rels, r = e % num_rels;
-    int lo = 0, hi = tb.num_groups[b];
-    while (lo < hi) {
-      const int m = lo + (hi - lo) / 2;
-      if (__ldg(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
-    }
-    ranges[e] = tb.z_base[b] + lo * tb.rows_per_group[b];
-  }
+  write_ranges(tb, num_rels, ranges);
 }
 
 // 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error.
@@ -920,13 +1008,26 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
     const int rows_per_block = (kThreads / (feat_in / 8)) * kCopyR;
     const int nblk = static_cast<int>(std::min<long long>(ceil_div(total, rows_per_block), 64ll * kNumSMs));
     scale_rows_f16_kernel<<<nblk + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
+  } else if (vec && feat_in / 8 <= kThreads) {
+    GatherTiles gt{};
+    const int lanes = kThreads / (feat_in / 8);
+    long long tiles = 0;
+    for (int b = 0; b < tb.nb; ++b) {
+      gt.first[b] = static_cast<int32_t>(tiles);
+      tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
+    }
+    gather_tiles_f16_kernel<<<static_cast<unsigned>(tiles + 1), kThreads, 0, st>>>(tb, gt, x, z, all_rows, ranges,
+                                                                                  num_rels, feat_in / 8);
   } else if (vec)
     gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
   else
     gather_rows_f16_kernel<1><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
   SPTIR_LAUNCH_OK("gather_rows_f16_kernel");
 
-  if (tc_shape) {
+  // Slices and boxes may reach past the last feature: what they bring from there is zeros, or the next
+  // relation's weights, and is not multiplied.  100 k nodes, 1.5 M edges, 46 relations, 32 -> 32: the
+  // CUDA-core transform 268 us in all, this 64 us.
+  if (path != 2 && feat_in % 16 == 0 && feat_out % 32 == 0 && feat_out <= kMaxOut && aligned16(w) && aligned16(y)) {
     const int rc = launch_tc<OutT, false>(z, w, y, ranges, all_rows, static_cast<int>(num_ranges), num_rels, total,
                                           feat_in, feat_out, st);
     if (rc <= 0) return rc;
