@@ -4,8 +4,9 @@
 // reference; generated kernel being replaced: examples/blocksparse/bsr_spmm.py:359-425 (wmma,
 // fp16 accumulate).  Block-rows without blocks are written as zeros (T.init of the reference).
 //
-// This file holds the CUDA-core kernel that works for every block size; bsrmm_tc.cu holds the
-// tensor-core kernel for the block sizes it supports and is tried first.
+// This file holds the CUDA-core kernel that works for every block size; bsrmm_tc.cu (block size 32,
+// features in steps of 128) and bsrmm_mma.cu (block sizes in steps of 16, features in steps of 8) hold
+// the tensor-core kernels and are tried first, in this order.
 #include <cuda_fp16.h>
 
 #include "common.h"
@@ -16,6 +17,9 @@ namespace sptir {
 int bsrmm_tc_launch(const __half* a, const __half* b, float* c, const int32_t* indptr,
                     const int32_t* indices, int nb, int mb, int nnzb, int blk, int feat,
                     cudaStream_t stream);
+// defined in bsrmm_mma.cu
+int bsrmm_mma_launch(const __half* a, const __half* b, float* c, const int32_t* indptr, const int32_t* indices,
+                     int nb, int blk, int feat, cudaStream_t st);
 
 namespace {
 
@@ -80,6 +84,8 @@ extern "C" int sparsetir_bsrmm_raw(const void* a_f16, const void* b_f16, float* 
   const __half* a = static_cast<const __half*>(a_f16);
   const __half* b = static_cast<const __half*>(b_f16);
   int rc = bsrmm_tc_launch(a, b, c, indptr, indices, nb, mb, nnzb, blk, feat, st);
+  if (rc <= 0) return rc;
+  rc = bsrmm_mma_launch(a, b, c, indptr, indices, nb, blk, feat, st);
   if (rc <= 0) return rc;
   dim3 grid(nb, ceil_div(feat, kThreads), ceil_div(blk, kBi));
   if (grid.y > 65535 || grid.z > 65535) return fail("sparsetir_bsrmm: shape exceeds the grid limits");

@@ -8,13 +8,8 @@
 // Tensor-core form (g = 16, t = 8, 16 or 32, feat a multiple of 8).  Of a group's work the gather of
 // 16 rows of B is what costs: 2 KB per 64 features against 8 instructions of m16n8k16.  So the
 // operands never touch shared memory: a warp owns 64 features of a row tile and loads both
-// operands straight into the registers that the instruction reads.
-//  - Which slot of the group plays which k of the instruction is free as long as A and B agree: the four
-//    k's of a lane are four neighbouring slots, so a lane reads its part of a row of A as 8 bytes and
-//    its four source rows as 16 bytes of `indices`.
-//  - Which feature plays which column is free too: lane group n reads 16 bytes (8 features) of each
-//    of its rows, instruction j takes the j-th feature of every piece.  Whole 128-byte lines per row,
-//    and a lane ends with 8 consecutive features of a result row per 16-byte store.
+// operands straight into the registers that the instruction reads (mma16.cuh); its four source rows are
+// 16 bytes of `indices`.
 // Two groups are in flight per warp.  Row tiles of up to kLight groups are one warp's work; longer
 // ones (hub rows) are cut at multiples of a window of groups of the whole matrix: a block owns a window,
 // its four warps share the part of each long tile that lies in it and meet in shared memory; parts
@@ -34,6 +29,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "mma16.cuh"
 #include "row_walk.cuh"
 #include "vec.cuh"
 
@@ -42,7 +38,6 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kG = 16;
-constexpr int kSlab = 64;     // features per warp
 constexpr int kLight = 16;    // longest tile of a single warp, in groups
 
 template <typename OutT> __device__ __forceinline__ OutT to_out(float v);
@@ -63,13 +58,6 @@ struct TcArgs {
   bool vec_indices;    // `indices` is 16-byte aligned
   bool vec_out;        // rows of C are made of whole 16-byte pieces
 };
-
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // 8 consecutive results of row `ii` (inside the tile) from feature f on
 __device__ __forceinline__ void store8(const TcArgs& s, float* c, int io, int ii, int f, const float (&v)[8]) {
@@ -117,16 +105,11 @@ __device__ __noinline__ void by_slots(const TcArgs& s, int g0, int g1, int ii, i
   for (int j = 0; j < 8; ++j) out[j * stride] = to_out<OutT>(sum[j]);
 }
 
-// True if a result of this lane is a NaN.  MT = tiles of 16 rows.  acc[mt][j][c]: instruction j = feature j of every 8-feature piece; c = 0, 1:
-// row lane/4, pieces 2(lane%4) and the next; c = 2, 3: row lane/4 + 8.
+// acc = the groups [g0, g1) of a tile (MT = tiles of 16 rows; layout of acc: mma16.cuh).  True if a
+// result of this lane is a NaN.
 template <int MT>
 __device__ __forceinline__ bool accumulate(const TcArgs& s, int g0, int g1, int f0, int lane, float (&acc)[MT][8][4]) {
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[mt][j][c] = 0.f;
+  mma16::clear(acc);
   const int q = lane & 3, r = lane >> 2;
   const bool in = f0 + r * 8 < s.feat;
   const __half* bl = s.b + (in ? f0 + r * 8 : 0);
@@ -153,18 +136,6 @@ __device__ __forceinline__ bool accumulate(const TcArgs& s, int g0, int g1, int 
       av[mt][0] = lo.x; av[mt][1] = hi.x; av[mt][2] = lo.y; av[mt][3] = hi.y;
     }
   };
-  auto multiply = [&](const uint4 (&v)[4], const uint32_t (&av)[MT][4]) {
-    auto one = [&](int j, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
-      const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
-      const uint32_t b0 = __byte_perm(w0, w1, sel), b1 = __byte_perm(w2, w3, sel);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) mma16816(acc[mt][j], av[mt], b0, b1);
-    };
-    one(0, v[0].x, v[1].x, v[2].x, v[3].x); one(1, v[0].x, v[1].x, v[2].x, v[3].x);
-    one(2, v[0].y, v[1].y, v[2].y, v[3].y); one(3, v[0].y, v[1].y, v[2].y, v[3].y);
-    one(4, v[0].z, v[1].z, v[2].z, v[3].z); one(5, v[0].z, v[1].z, v[2].z, v[3].z);
-    one(6, v[0].w, v[1].w, v[2].w, v[3].w); one(7, v[0].w, v[1].w, v[2].w, v[3].w);
-  };
   int4 id0 = make_int4(0, 0, 0, 0), id1 = id0;
   if (g0 < g1) id0 = ids_of(g0);
   if (g0 + 1 < g1) id1 = ids_of(g0 + 1);
@@ -178,8 +149,8 @@ __device__ __forceinline__ bool accumulate(const TcArgs& s, int g0, int g1, int 
     if (two) values_of(g + 1, a1);
     if (g + 2 < g1) id0 = ids_of(g + 2);
     if (g + 3 < g1) id1 = ids_of(g + 3);
-    multiply(v0, a0);
-    if (two) multiply(v1, a1);
+    mma16::multiply(acc, v0, a0);
+    if (two) mma16::multiply(acc, v1, a1);
   }
   bool nan = false;
 #pragma unroll
@@ -198,7 +169,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   __shared__ unsigned s_seen;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slab = static_cast<int>(blockIdx.x) % s.slabs, unit = static_cast<int>(blockIdx.x) / s.slabs;
-  const int f0 = slab * kSlab;
+  const int f0 = slab * mma16::kSlab;
   const int q = lane & 3, r = lane >> 2;
   OutT* c = static_cast<OutT*>(s.c);
   float acc[MT][8][4];
@@ -344,7 +315,7 @@ tcspmm_simt_kernel(const __half* __restrict__ a, const __half* __restrict__ b, O
 
 template <int MT, typename OutT>
 int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
-  s.slabs = ceil_div(s.feat, kSlab);
+  s.slabs = ceil_div(s.feat, mma16::kSlab);
   // Windows of 128 groups keep the scratch small; down to 32 where there would not be enough blocks
   // (20 k rows, 6,118 groups, F = 64: 12.4 against 18.9 us).
   s.window_log = 5;
