@@ -65,8 +65,12 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
   };
   int pb = pa, kb = ka;
   next(pb, kb);
-  auto id_of = [&](int p) { return p < p1 ? __ldg(indices + p) : 0; };
-  int ca = id_of(pa), cb = id_of(pb);
+  auto id_of = [&](int p) { return __ldg(indices + min(p, p1 - 1)); };  // past the last block: not used
+  int ca = 0, cb = 0;
+  if (p0 < p1) {
+    ca = id_of(pa);
+    cb = id_of(pb);
+  }
   for (long long g = g0; g < g1; g += 2) {
     const bool two = g + 1 < g1;
     uint4 va[4], vb[4];

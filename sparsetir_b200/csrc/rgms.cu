@@ -41,6 +41,8 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
                    const int32_t* indptr_i, const int32_t* indices_i, const int32_t* indptr_j,
                    const int32_t* indices_j, int num_rels, int feat, int nnz_i,
                    const float* z, cudaStream_t stream);
+int rgms_wide_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i, const float* z,
+                     int num_rels, int nnz_i, int feat, cudaStream_t stream);
 
 namespace {
 
@@ -182,7 +184,7 @@ int launch_tile(const float* a, const float* w, const float* x, float* y, const 
 extern "C" int sparsetir_rgms_workspace(int feat, int nnz_i, size_t* scratch_bytes) {
   if (!scratch_bytes || feat < 0 || nnz_i < 0) return sptir::fail("sparsetir_rgms_workspace: bad argument");
   // the two-launch form keeps one aggregated feature row per (relation, destination) pair
-  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * 64 * sizeof(float) : 0;
+  *scratch_bytes = feat == 64 || feat == 128 || feat == 256 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : 0;
   return 0;
 }
 
@@ -239,6 +241,19 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
       int rc = rgms_tc_launch(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, feat,
                               nnz_i, z, st);
       if (rc <= 0) return rc;
+    }
+    if (feat == 128 || feat == 256) {
+      // The same two steps with the transform of rgms_wide.cu.  A call that is being captured before
+      // its stream has the scratch, or that finds no memory for Z, keeps the kernels without scratch.
+      const size_t zb = static_cast<size_t>(nnz_i) * feat * sizeof(float);
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      if (!workspace_fits(device_id, st, zb, 0)) SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+      float* z = capture == cudaStreamCaptureStatusNone ? static_cast<float*>(workspace(device_id, st, zb)) : nullptr;
+      if (z != nullptr) {
+        if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, feat, nnz_j, device_id, stream) != 0)
+          return -1;
+        return rgms_wide_launch(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat, st);
+      }
     }
     if (feat == 32)
       return launch_tile<32>(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, st);

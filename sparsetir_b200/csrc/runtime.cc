@@ -107,7 +107,8 @@ bool workspace_fits(int device_id, cudaStream_t stream, size_t bytes, size_t zer
   std::lock_guard<std::mutex> lock(g_ws_mutex);
   const std::pair<int, cudaStream_t> key{device_id, stream};
   const auto a = g_ws[0].find(key), b = g_ws[1].find(key);
-  return a != g_ws[0].end() && a->second.bytes >= bytes && b != g_ws[1].end() && b->second.bytes >= zeroed_bytes;
+  return a != g_ws[0].end() && a->second.bytes >= bytes &&
+         (zeroed_bytes == 0 || (b != g_ws[1].end() && b->second.bytes >= zeroed_bytes));
 }
 
 void* workspace(int device_id, cudaStream_t stream, size_t bytes) {

@@ -325,7 +325,7 @@ int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
   const long long blocks = (static_cast<long long>(s.windows) + ceil_div(s.mb, 4)) * s.slabs;
   if (blocks > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
   const size_t part_bytes = 2 * static_cast<size_t>(s.windows) * s.slabs * MT * kThreads * 8 * sizeof(float);
-  const size_t counter_bytes = static_cast<size_t>(s.windows) * s.slabs * sizeof(unsigned);
+  const size_t counter_bytes = static_cast<size_t>(std::max(s.windows, 1)) * s.slabs * sizeof(unsigned);
   char* own = nullptr;
   if (!workspace_fits(device_id, st, part_bytes, counter_bytes)) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -333,7 +333,7 @@ int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
     if (capture != cudaStreamCaptureStatusNone) {
       // the library's buffers cannot grow inside a capture: this call gets memory that the graph owns
       const size_t at = (part_bytes + 255) & ~static_cast<size_t>(255);
-      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + std::max<size_t>(counter_bytes, 4), st));
+      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + counter_bytes, st));
       SPTIR_CUDA_OK(cudaMemsetAsync(own + at, 0, counter_bytes, st));
       s.part = reinterpret_cast<float*>(own);
       s.counters = reinterpret_cast<unsigned*>(own + at);
