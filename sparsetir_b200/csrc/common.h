@@ -41,6 +41,19 @@ void* zeroed_workspace(int device_id, cudaStream_t stream, size_t bytes);
 // allocates nor synchronises (neither is possible while the stream is being captured).
 bool workspace_fits(int device_id, cudaStream_t stream, size_t bytes, size_t zeroed_bytes);
 
+// Scratch and zeroed counters of one operator call: the buffers above, or, while the stream is being
+// captured, memory that belongs to the graph.  A captured launch must not keep the addresses of the
+// library's buffers: a later call that needs more frees them, and a replay on another stream would
+// share them with the calls of this one.
+struct CallScratch {
+  char* scratch = nullptr;
+  unsigned* counters = nullptr;
+  void* owned = nullptr;  // allocated by the graph
+};
+int take_scratch(int device_id, cudaStream_t stream, size_t bytes, size_t counter_bytes, CallScratch* out);
+// After the last launch that uses it.
+int return_scratch(const CallScratch& cs, cudaStream_t stream);
+
 // Deep checks of index arrays before a launch (validate.cu): enabled by SPARSETIR_VALIDATE=1 or
 // sparsetir_set_validate(1).  Each returns 0, or -1 after recording which array is wrong where;
 // they synchronise `st`.  nnz < 0 skips the check of the last row pointer.

@@ -317,30 +317,13 @@ int launch_split(SplitArgs s, int device_id, cudaStream_t st) {
                                                (static_cast<long long>(s.m) + 8 * kThreads - 1) / (8 * kThreads)));
   const size_t part_bytes = 2 * static_cast<size_t>(blocks) * s.feat * sizeof(float);
   const size_t counter_bytes = static_cast<size_t>(blocks) * tiles * sizeof(unsigned);
-  if (!workspace_fits(device_id, st, part_bytes, counter_bytes)) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
-    if (capture != cudaStreamCaptureStatusNone) {
-      // the first call on this stream is being captured into a graph, where the library's buffers
-      // cannot grow: this call gets memory that the graph owns
-      char* own = nullptr;
-      const size_t at = (part_bytes + 255) & ~static_cast<size_t>(255);
-      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + counter_bytes, st));
-      SPTIR_CUDA_OK(cudaMemsetAsync(own + at, 0, counter_bytes, st));
-      s.part = reinterpret_cast<float*>(own);
-      s.counters = reinterpret_cast<unsigned*>(own + at);
-      csr_split_kernel<LPR, W, VPL><<<dim3(blocks, gy), kThreads, 0, st>>>(s);
-      SPTIR_LAUNCH_OK("csr_split_kernel");
-      SPTIR_CUDA_OK(cudaFreeAsync(own, st));
-      return 0;
-    }
-  }
-  s.part = static_cast<float*>(workspace(device_id, st, part_bytes));
-  s.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
-  if (s.part == nullptr || s.counters == nullptr) return -1;
+  CallScratch cs;
+  if (take_scratch(device_id, st, part_bytes, counter_bytes, &cs) != 0) return -1;
+  s.part = reinterpret_cast<float*>(cs.scratch);
+  s.counters = cs.counters;
   csr_split_kernel<LPR, W, VPL><<<dim3(blocks, gy), kThreads, 0, st>>>(s);
   SPTIR_LAUNCH_OK("csr_split_kernel");
-  return 0;
+  return return_scratch(cs, st);
 }
 
 }  // namespace

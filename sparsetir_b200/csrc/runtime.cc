@@ -119,6 +119,33 @@ void* zeroed_workspace(int device_id, cudaStream_t stream, size_t bytes) {
   return grow(1, device_id, stream, bytes);
 }
 
+int take_scratch(int device_id, cudaStream_t stream, size_t bytes, size_t counter_bytes, CallScratch* out) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SPTIR_CUDA_OK(cudaStreamIsCapturing(stream, &capture));
+  if (capture == cudaStreamCaptureStatusNone) {
+    out->scratch = static_cast<char*>(workspace(device_id, stream, bytes));
+    if (out->scratch == nullptr) return -1;
+    if (counter_bytes > 0) {
+      out->counters = static_cast<unsigned*>(zeroed_workspace(device_id, stream, counter_bytes));
+      if (out->counters == nullptr) return -1;
+    }
+    return 0;
+  }
+  const size_t at = (bytes + 255) & ~static_cast<size_t>(255);
+  SPTIR_CUDA_OK(cudaMallocAsync(&out->owned, std::max<size_t>(at + counter_bytes, 1), stream));
+  out->scratch = static_cast<char*>(out->owned);
+  if (counter_bytes > 0) {
+    out->counters = reinterpret_cast<unsigned*>(out->scratch + at);
+    SPTIR_CUDA_OK(cudaMemsetAsync(out->counters, 0, counter_bytes, stream));
+  }
+  return 0;
+}
+
+int return_scratch(const CallScratch& cs, cudaStream_t stream) {
+  if (cs.owned != nullptr) SPTIR_CUDA_OK(cudaFreeAsync(cs.owned, stream));
+  return 0;
+}
+
 }  // namespace sptir
 
 extern "C" {

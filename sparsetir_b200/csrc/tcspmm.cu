@@ -326,28 +326,13 @@ int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
   if (blocks > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
   const size_t part_bytes = 2 * static_cast<size_t>(s.windows) * s.slabs * MT * kThreads * 8 * sizeof(float);
   const size_t counter_bytes = static_cast<size_t>(std::max(s.windows, 1)) * s.slabs * sizeof(unsigned);
-  char* own = nullptr;
-  if (!workspace_fits(device_id, st, part_bytes, counter_bytes)) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
-    if (capture != cudaStreamCaptureStatusNone) {
-      // the library's buffers cannot grow inside a capture: this call gets memory that the graph owns
-      const size_t at = (part_bytes + 255) & ~static_cast<size_t>(255);
-      SPTIR_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&own), at + counter_bytes, st));
-      SPTIR_CUDA_OK(cudaMemsetAsync(own + at, 0, counter_bytes, st));
-      s.part = reinterpret_cast<float*>(own);
-      s.counters = reinterpret_cast<unsigned*>(own + at);
-    }
-  }
-  if (own == nullptr) {
-    s.part = static_cast<float*>(workspace(device_id, st, part_bytes));
-    s.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
-    if (s.part == nullptr || s.counters == nullptr) return -1;
-  }
+  CallScratch cs;
+  if (take_scratch(device_id, st, part_bytes, counter_bytes, &cs) != 0) return -1;
+  s.part = reinterpret_cast<float*>(cs.scratch);
+  s.counters = cs.counters;
   tcspmm_mma_kernel<MT, OutT><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(s);
   SPTIR_LAUNCH_OK("tcspmm_mma_kernel");
-  if (own != nullptr) SPTIR_CUDA_OK(cudaFreeAsync(own, st));
-  return 0;
+  return return_scratch(cs, st);
 }
 
 template <typename OutT>
