@@ -297,45 +297,12 @@ csr_split_kernel(const SplitArgs s) {
   }
 }
 
-template <int LPR, int W, int VPL>
-int launch_split(SplitArgs s, int device_id, cudaStream_t st) {
-  constexpr int SUBS = kThreads / LPR;
-  const int tiles = ceil_div(s.feat, LPR * W * VPL);
-  s.rows_per_entry = static_cast<float>(s.m) / static_cast<float>(s.nnz);
-  // One wave of resident blocks with equal shares of the entries: a block's fixed cost (search,
-  // meeting of the pieces) is paid once, 4.5 M entries, F = 64: 94 us against 109 with four waves.
-  // A block walks the feature tiles one after the other, all blocks roughly in step, which keeps
-  // the slice of B that they gather from in L2; matrices too small to give every resident block
-  // a batch of entries deal the tiles to more blocks (60 k entries, F = 512: 25 against 37 us).
-  const long long resident = 4ll * kNumSMs, batch = static_cast<long long>(SUBS) * LPR;
-  const long long fewest = (s.nnz + batch - 1) / batch;
-  const int gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident / fewest)));
-  const long long want = resident / gy * SUBS;
-  s.span = static_cast<int>((s.nnz + want - 1) / want + LPR - 1) / LPR * LPR;
-  const long long per_block = static_cast<long long>(SUBS) * s.span;
-  const int blocks = static_cast<int>(std::max((s.nnz + per_block - 1) / per_block,
-                                               (static_cast<long long>(s.m) + 8 * kThreads - 1) / (8 * kThreads)));
-  const size_t part_bytes = 2 * static_cast<size_t>(blocks) * s.feat * sizeof(float);
-  const size_t counter_bytes = static_cast<size_t>(blocks) * tiles * sizeof(unsigned);
-  CallScratch cs;
-  if (take_scratch(device_id, st, part_bytes, counter_bytes, &cs) != 0) return -1;
-  s.part = reinterpret_cast<float*>(cs.scratch);
-  s.counters = cs.counters;
-  csr_split_kernel<LPR, W, VPL><<<dim3(blocks, gy), kThreads, 0, st>>>(s);
-  SPTIR_LAUNCH_OK("csr_split_kernel");
-  return return_scratch(cs, st);
-}
+// Lanes per row, floats per vector, vectors per lane.
+struct SplitShape {
+  int lanes, w, vpl;
+};
 
-}  // namespace
-
-int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-                  int m, int n, int feat, int nnz, int device_id, cudaStream_t st) {
-  if (nnz == 0) {
-    SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(m) * feat * sizeof(float), st));
-    return 0;
-  }
-  const SplitArgs s{a, b, c, indptr, indices, nullptr, nullptr, m, nnz, feat, 0, 0.f};
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+SplitShape split_shape(uintptr_t bits, int n, int feat, int nnz) {
   if (feat % 4 == 0 && bits % 16 == 0) {
     // The narrowest group that covers a row, a warp at most: several sub-warps per warp keep more
     // rows in flight (4.5 M entries, F = 64: 16 lanes 93, 32 lanes 160, 8 lanes 107 us), a second
@@ -346,22 +313,101 @@ int csr_split_run(const float* a, const float* b, float* c, const int32_t* indpt
     while (lanes > 8 && n > 0 && nnz / n >= 64 &&
            static_cast<size_t>(n) * std::min(lanes * 16, feat * 4) > (size_t{48} << 20))
       lanes /= 2;
-    if (lanes == 8) return launch_split<8, 4, 1>(s, device_id, st);
-    if (lanes == 16) return launch_split<16, 4, 1>(s, device_id, st);
-    return launch_split<32, 4, 1>(s, device_id, st);
+    return {lanes, 4, 1};
   }
-  if (feat % 2 == 0 && bits % 8 == 0) {
-    if (feat <= 16) return launch_split<8, 2, 1>(s, device_id, st);
-    if (feat <= 32) return launch_split<16, 2, 1>(s, device_id, st);
-    if (feat <= 64) return launch_split<32, 2, 1>(s, device_id, st);
-    return launch_split<32, 2, 2>(s, device_id, st);
+  if (feat % 2 == 0 && bits % 8 == 0) return {feat <= 16 ? 8 : (feat <= 32 ? 16 : 32), 2, feat <= 64 ? 1 : 2};
+  if (feat <= 32) return {feat <= 8 ? 8 : (feat <= 16 ? 16 : 32), 1, 1};
+  return {32, 1, feat <= 64 ? 2 : (feat <= 128 ? 4 : 5)};
+}
+
+struct SplitPlan {
+  int gy, span, blocks;
+  size_t part_bytes, counter_bytes;
+};
+
+SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
+  const int subs = kThreads / sh.lanes;
+  const int tiles = ceil_div(feat, sh.lanes * sh.w * sh.vpl);
+  // One wave of resident blocks with equal shares of the entries: a block's fixed cost (search,
+  // meeting of the pieces) is paid once, 4.5 M entries, F = 64: 94 us against 109 with four waves.
+  // A block walks the feature tiles one after the other, all blocks roughly in step, which keeps
+  // the slice of B that they gather from in L2; matrices too small to give every resident block
+  // a batch of entries deal the tiles to more blocks (60 k entries, F = 512: 25 against 37 us).
+  const long long resident = 4ll * kNumSMs, batch = static_cast<long long>(subs) * sh.lanes;
+  const long long fewest = (nnz + batch - 1) / batch;
+  SplitPlan p;
+  p.gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident / fewest)));
+  const long long want = resident / p.gy * subs;
+  p.span = static_cast<int>((nnz + want - 1) / want + sh.lanes - 1) / sh.lanes * sh.lanes;
+  const long long per_block = static_cast<long long>(subs) * p.span;
+  p.blocks = static_cast<int>(std::max((nnz + per_block - 1) / per_block,
+                                       (static_cast<long long>(m) + 8 * kThreads - 1) / (8 * kThreads)));
+  p.part_bytes = 2 * static_cast<size_t>(p.blocks) * feat * sizeof(float);
+  p.counter_bytes = static_cast<size_t>(p.blocks) * tiles * sizeof(unsigned);
+  return p;
+}
+
+template <int LPR, int W, int VPL>
+int launch_split(const SplitArgs& s, const SplitPlan& p, cudaStream_t st) {
+  csr_split_kernel<LPR, W, VPL><<<dim3(p.blocks, p.gy), kThreads, 0, st>>>(s);
+  SPTIR_LAUNCH_OK("csr_split_kernel");
+  return 0;
+}
+
+int dispatch_split(const SplitArgs& s, const SplitShape& sh, const SplitPlan& p, cudaStream_t st) {
+  if (sh.w == 4) {
+    if (sh.lanes == 8) return launch_split<8, 4, 1>(s, p, st);
+    if (sh.lanes == 16) return launch_split<16, 4, 1>(s, p, st);
+    return launch_split<32, 4, 1>(s, p, st);
   }
-  if (feat <= 8) return launch_split<8, 1, 1>(s, device_id, st);
-  if (feat <= 16) return launch_split<16, 1, 1>(s, device_id, st);
-  if (feat <= 32) return launch_split<32, 1, 1>(s, device_id, st);
-  if (feat <= 64) return launch_split<32, 1, 2>(s, device_id, st);
-  if (feat <= 128) return launch_split<32, 1, 4>(s, device_id, st);
-  return launch_split<32, 1, 5>(s, device_id, st);
+  if (sh.w == 2) {
+    if (sh.lanes == 8) return launch_split<8, 2, 1>(s, p, st);
+    if (sh.lanes == 16) return launch_split<16, 2, 1>(s, p, st);
+    if (sh.vpl == 1) return launch_split<32, 2, 1>(s, p, st);
+    return launch_split<32, 2, 2>(s, p, st);
+  }
+  if (sh.lanes == 8) return launch_split<8, 1, 1>(s, p, st);
+  if (sh.lanes == 16) return launch_split<16, 1, 1>(s, p, st);
+  if (sh.vpl == 1) return launch_split<32, 1, 1>(s, p, st);
+  if (sh.vpl == 2) return launch_split<32, 1, 2>(s, p, st);
+  if (sh.vpl == 4) return launch_split<32, 1, 4>(s, p, st);
+  return launch_split<32, 1, 5>(s, p, st);
+}
+
+inline uintptr_t low_bits(const float* b, const float* c) {
+  return reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+}
+
+}  // namespace
+
+// Bytes of scratch that the pieces of a call need.
+size_t csr_split_scratch(const float* b, const float* c, int m, int n, int feat, int nnz) {
+  if (nnz == 0) return 0;
+  return split_plan(split_shape(low_bits(b, c), n, feat, nnz), m, feat, nnz).part_bytes;
+}
+
+// pieces: that many bytes, 16-byte aligned, from a caller that holds the stream's scratch buffer; null:
+// the call takes its scratch itself.
+int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
+                  int m, int n, int feat, int nnz, void* pieces, int device_id, cudaStream_t st) {
+  if (nnz == 0) {
+    SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(m) * feat * sizeof(float), st));
+    return 0;
+  }
+  const SplitShape sh = split_shape(low_bits(b, c), n, feat, nnz);
+  const SplitPlan p = split_plan(sh, m, feat, nnz);
+  CallScratch cs;
+  if (pieces != nullptr) {
+    cs.scratch = static_cast<char*>(pieces);
+    cs.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, p.counter_bytes));
+    if (cs.counters == nullptr) return -1;
+  } else if (take_scratch(device_id, st, p.part_bytes, p.counter_bytes, &cs) != 0) {
+    return -1;
+  }
+  const SplitArgs s{a, b, c, indptr, indices, reinterpret_cast<float*>(cs.scratch), cs.counters, m, nnz, feat, p.span,
+                    static_cast<float>(m) / static_cast<float>(nnz)};
+  if (dispatch_split(s, sh, p, st) != 0) return -1;
+  return return_scratch(cs, st);
 }
 
 }  // namespace sptir

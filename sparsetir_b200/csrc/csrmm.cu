@@ -190,14 +190,50 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
 
 namespace sptir {
 int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-                  int m, int n, int feat, int nnz, int device_id, cudaStream_t st);
+                  int m, int n, int feat, int nnz, void* pieces, int device_id, cudaStream_t st);
+size_t csr_split_scratch(const float* b, const float* c, int m, int n, int feat, int nnz);
+
+namespace {
+// Whether a call takes the row-wise kernel, and with which lanes.
+bool row_wise(const float* b, const float* c, int m, int n, int feat, int nnz, bool hub_rows, int lane_floats,
+              int* lane_w, int* lanes_per_row) {
+  const bool vec4 = (feat % 4 == 0) && aligned16(b) && aligned16(c);
+  // The row-wise kernel needs whole feature tiles.  Its share ends where the split by entries is
+  // the faster one although it has to search for its rows: 4,096 rows of 10 entries, F = 64, 4.8
+  // against 7.1 us; 16,886 power-law rows, F = 32, 23.4 (with the two launches for hub rows that
+  // it needed there) against 9.6 us.
+  const bool small = m < 8192 && nnz < 65536;
+  if (!vec4 || (!small && hub_rows)) return false;
+  // lanes per row: one per 32-byte vector when the operands allow it, else one per 16-byte
+  // vector; narrowed until the n x tile slice of B that a pass over the rows gathers from fits
+  // the resident part of L2 (see hyb_spmm.cu)
+  const int w = (feat % 32 == 0 && aligned32(b) && aligned32(c)) ? (lane_floats == 8 ? 8 : max_lane_floats()) : 4;
+  const int nv = feat / w;
+  int lanes = nv <= 4 ? 4 : (nv <= 8 ? 8 : (nv <= 16 ? 16 : 32));
+  if (w == 4 && lanes < 8) lanes = 8;
+  const size_t l2_budget = 48u << 20;
+  const int min_lanes = w == 8 ? 4 : 8;
+  while (lanes > min_lanes && static_cast<size_t>(n) * lanes * w * 4 > l2_budget) lanes /= 2;
+  *lane_w = w;
+  *lanes_per_row = lanes;
+  return feat % (w * lanes) == 0;
+}
+}  // namespace
+
+// Scratch that a csrmm call over these operands needs (0: none), for callers that hold the stream's buffer.
+size_t csrmm_scratch(const float* b, const float* c, int m, int n, int feat, int nnz) {
+  int w = 0, lanes = 0;
+  return row_wise(b, c, m, n, feat, nnz, true, 0, &w, &lanes) ? 0 : csr_split_scratch(b, c, m, n, feat, nnz);
+}
 
 // The launcher behind sparsetir_csrmm_raw.  hub_rows = false: the caller knows that its rows are
-// short, and that b and c are 16-byte aligned with feat = 64; such a call never touches the
-// per-stream workspace (the caller may hold it).
+// short, and that b and c are 16-byte aligned with feat a multiple of 64 that makes whole tiles; such a
+// call never touches the per-stream workspace (the caller may hold it).
 // lane_floats: 0 = the library's default lane width, 8 = 32-byte lanes where the operands allow.
+// pieces: csrmm_scratch() bytes from a caller that holds the stream's scratch buffer, null from others.
 int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-              int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats) {
+              int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats,
+              void* pieces) {
   if (m < 0 || feat < 0 || nnz < 0) return fail("sparsetir_csrmm: negative size");
   if (m == 0 || feat == 0) return 0;
   if (!b || !c || !indptr || (nnz > 0 && (!a || !indices)))
@@ -205,59 +241,42 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
   if (use_device(device_id) != 0) return -1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (validate_enabled() && validate_csr("sparsetir_csrmm", indptr, m, indices, nnz, n, st) != 0) return -1;
-  const bool vec4 = (feat % 4 == 0) && aligned16(b) && aligned16(c);
-  // The row-wise kernel needs whole feature tiles.  Its share ends where the split by entries is
-  // the faster one although it has to search for its rows: 4,096 rows of 10 entries, F = 64, 4.8
-  // against 7.1 us; 16,886 power-law rows, F = 32, 23.4 (with the two launches for hub rows that
-  // it needed there) against 9.6 us.
-  const bool small = m < 8192 && nnz < 65536;
-  if (vec4 && (small || !hub_rows)) {
-    // lanes per row: one per 32-byte vector when the operands allow it, else one per 16-byte
-    // vector; narrowed until the n x tile slice of B that a pass over the rows gathers from fits
-    // the resident part of L2 (see hyb_spmm.cu)
-    const int w = (feat % 32 == 0 && aligned32(b) && aligned32(c)) ? (lane_floats == 8 ? 8 : max_lane_floats()) : 4;
-    const int nv = feat / w;
-    int lanes = nv <= 4 ? 4 : (nv <= 8 ? 8 : (nv <= 16 ? 16 : 32));
-    if (w == 4 && lanes < 8) lanes = 8;
-    const size_t l2_budget = 48u << 20;
-    const int min_lanes = w == 8 ? 4 : 8;
-    while (lanes > min_lanes && static_cast<size_t>(n) * lanes * w * 4 > l2_budget) lanes /= 2;
-    if (feat % (w * lanes) == 0) {
-      const int subs = kThreads / lanes;
-      // about four id batches per item, but never so few items that SMs sit idle
-      const double avg = m > 0 ? static_cast<double>(nnz) / m : 0.0;
-      int rpi = static_cast<int>(4.0 * lanes / (avg > 1.0 ? avg : 1.0));
-      rpi = rpi < 1 ? 1 : (rpi > lanes - 1 ? lanes - 1 : rpi);
-      const long long want_items = 4ll * kNumSMs * 4 * subs;
-      while (rpi > 1 && (m + rpi - 1) / rpi < want_items) rpi /= 2;
-      dim3 grid(ceil_div(ceil_div(m, rpi), subs), feat / (w * lanes));
+  int w = 0, lanes = 0;
+  if (row_wise(b, c, m, n, feat, nnz, hub_rows, lane_floats, &w, &lanes)) {
+    const int subs = kThreads / lanes;
+    // about four id batches per item, but never so few items that SMs sit idle
+    const double avg = m > 0 ? static_cast<double>(nnz) / m : 0.0;
+    int rpi = static_cast<int>(4.0 * lanes / (avg > 1.0 ? avg : 1.0));
+    rpi = rpi < 1 ? 1 : (rpi > lanes - 1 ? lanes - 1 : rpi);
+    const long long want_items = 4ll * kNumSMs * 4 * subs;
+    while (rpi > 1 && (m + rpi - 1) / rpi < want_items) rpi /= 2;
+    dim3 grid(ceil_div(ceil_div(m, rpi), subs), feat / (w * lanes));
 #define SPTIR_CSR_LEAN(L, WW)                                                                                   \
   if (hub_rows)                                                                                                 \
     csrmm_lean_kernel<L, WW, true><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi);           \
   else                                                                                                          \
     csrmm_lean_kernel<L, WW, false><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi)
-      if (w == 8) {
-        if (lanes == 4) { SPTIR_CSR_LEAN(4, 8); }
-        else if (lanes == 8) { SPTIR_CSR_LEAN(8, 8); }
-        else if (lanes == 16) { SPTIR_CSR_LEAN(16, 8); }
-        else { SPTIR_CSR_LEAN(32, 8); }
-      } else {
-        if (lanes == 8) { SPTIR_CSR_LEAN(8, 4); }
-        else if (lanes == 16) { SPTIR_CSR_LEAN(16, 4); }
-        else { SPTIR_CSR_LEAN(32, 4); }
-      }
-#undef SPTIR_CSR_LEAN
-      SPTIR_LAUNCH_OK("csrmm_lean_kernel");
-      return 0;
+    if (w == 8) {
+      if (lanes == 4) { SPTIR_CSR_LEAN(4, 8); }
+      else if (lanes == 8) { SPTIR_CSR_LEAN(8, 8); }
+      else if (lanes == 16) { SPTIR_CSR_LEAN(16, 8); }
+      else { SPTIR_CSR_LEAN(32, 8); }
+    } else {
+      if (lanes == 8) { SPTIR_CSR_LEAN(8, 4); }
+      else if (lanes == 16) { SPTIR_CSR_LEAN(16, 4); }
+      else { SPTIR_CSR_LEAN(32, 4); }
     }
+#undef SPTIR_CSR_LEAN
+    SPTIR_LAUNCH_OK("csrmm_lean_kernel");
+    return 0;
   }
   if (!hub_rows) return fail("sparsetir_csrmm: short-row call with operands that are not whole tiles");
-  return csr_split_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, st);
+  return csr_split_run(a, b, c, indptr, indices, m, n, feat, nnz, pieces, device_id, st);
 }
 
 int csrmm_impl(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
                int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows) {
-  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, hub_rows, 0);
+  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, hub_rows, 0, nullptr);
 }
 
 // For matrices of very short rows (the aggregation launch of RGMS: 2.2 entries per row), where the
@@ -268,7 +287,8 @@ int csrmm_impl(const float* a, const float* b, float* c, const int32_t* indptr, 
 int csrmm_short_rows_impl(const float* a, const float* b, float* c, const int32_t* indptr,
                           const int32_t* indices, int m, int n, int feat, int nnz, int device_id,
                           void* stream) {
-  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, false, m >= (1 << 19) ? 8 : 0);
+  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, false, m >= (1 << 19) ? 8 : 0,
+                   nullptr);
 }
 }  // namespace sptir
 

@@ -161,9 +161,12 @@ extern "C" int sparsetir_sddmm_raw(const float* a, const float* b, float* c, con
                                    int nnz, int device_id, void* stream);
 extern "C" int sparsetir_sparse_softmax_raw(const float* a, float* b, const int32_t* indptr, int n, int nnz,
                                             int device_id, void* stream);
-extern "C" int sparsetir_csrmm_raw(const float* a, const float* b, float* c, const int32_t* indptr,
-                                   const int32_t* indices, int m, int n, int feat, int nnz, int device_id,
-                                   void* stream);
+namespace sptir {
+// defined in csrmm.cu
+size_t csrmm_scratch(const float* b, const float* c, int m, int n, int feat, int nnz);
+int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices, int m, int n,
+              int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats, void* pieces);
+}  // namespace sptir
 
 extern "C" int sparsetir_fusedmm_raw(const float* q, const float* k, const float* v, float* o,
                                      const int32_t* indptr, const int32_t* indices, int m, int n, int nnz,
@@ -196,16 +199,25 @@ extern "C" int sparsetir_fusedmm_raw(const float* q, const float* k, const float
       default: break;
     }
   }
-  // other feature sizes: the three operators one after the other, the per-position scores and
-  // probabilities in the per-stream workspace (scores first: the SpMM's own use of the workspace
-  // for its hub-row list falls into that half, which is dead by then)
   if (nnz == 0) {
     SPTIR_CUDA_OK(cudaMemsetAsync(o, 0, static_cast<size_t>(m) * feat * sizeof(float), st));
     return 0;
   }
-  float* ws = static_cast<float*>(workspace(device_id, st, 2 * static_cast<size_t>(nnz) * sizeof(float)));
+  // One request for all that the three hold at the same time: scores, probabilities, and the pieces of
+  // rows that the SpMM splits.  A second request would get the same buffer again, or a larger one in
+  // its place.  While the stream is being captured the SpMM takes its pieces from the graph.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+  const bool eager = capture == cudaStreamCaptureStatusNone;
+  const size_t at = (2 * static_cast<size_t>(nnz) * sizeof(float) + 255) & ~static_cast<size_t>(255);
+  const size_t piece_bytes = eager ? csrmm_scratch(v, o, m, n, feat, nnz) : 0;
+  char* ws = static_cast<char*>(workspace(device_id, st, piece_bytes > 0 ? at + piece_bytes
+                                                                         : 2 * static_cast<size_t>(nnz) * sizeof(float)));
   if (!ws) return -1;
-  if (sparsetir_sddmm_raw(q, k, ws, indptr, indices, nullptr, m, n, feat, nnz, device_id, stream) != 0) return -1;
-  if (sparsetir_sparse_softmax_raw(ws, ws + nnz, indptr, m, nnz, device_id, stream) != 0) return -1;
-  return sparsetir_csrmm_raw(ws + nnz, v, o, indptr, indices, m, n, feat, nnz, device_id, stream);
+  float* scores = reinterpret_cast<float*>(ws);
+  float* probs = scores + nnz;
+  if (sparsetir_sddmm_raw(q, k, scores, indptr, indices, nullptr, m, n, feat, nnz, device_id, stream) != 0) return -1;
+  if (sparsetir_sparse_softmax_raw(scores, probs, indptr, m, nnz, device_id, stream) != 0) return -1;
+  return csrmm_run(probs, v, o, indptr, indices, m, n, feat, nnz, device_id, stream, /*hub_rows=*/true, 0,
+                   piece_bytes > 0 ? ws + at : nullptr);
 }

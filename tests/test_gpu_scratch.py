@@ -97,3 +97,55 @@ def test_calls_on_two_streams_at_once(cuda_device, op, captured):
     torch.cuda.synchronize()
     for (y, _), w in zip(pairs, want):
         assert torch.equal(y, w)
+
+
+def attention_float64(q, k, v, ptr, cols):
+    """(result, bound of the error of fp32 stages in any order).  The numerator is not shifted by the row maximum:
+    exp(s) / sum exp(s - max), as in the reference (tests/refimpl.py)."""
+    (m, feat), n = q.shape, k.shape[0]
+    deg = (ptr[1:] - ptr[:-1]).long()
+    rows = torch.repeat_interleave(torch.arange(m, device=q.device), deg)
+    s, mag = (torch.cat([(x[rows[p:p + 50_000]] * y[cols[p:p + 50_000].long()]).sum(1) for p in range(0, len(cols), 50_000)])
+              for x, y in ((q.double(), k.double()), (q.abs().double(), k.abs().double())))
+    top = torch.full((m,), -float("inf"), dtype=torch.float64, device=q.device).scatter_reduce(0, rows, s, "amax")
+    total = torch.zeros(m, dtype=torch.float64, device=q.device).index_add_(0, rows, torch.exp(s - top[rows]))
+    prob = torch.exp(s) / total[rows]
+    out, size = (torch.zeros(m, feat, dtype=torch.float64, device=q.device) for _ in range(2))
+    for p in range(0, len(cols), 50_000):
+        part = prob[p:p + 50_000, None] * v[cols[p:p + 50_000].long()].double()
+        out.index_add_(0, rows[p:p + 50_000], part)
+        size.index_add_(0, rows[p:p + 50_000], part.abs())
+    # a score is off by feat half-ulps of its terms, which becomes a relative error of its exponential (two
+    # scores: its own and the maximum); __expf(x) adds 2 + 1.2 |x| ulps with |x| up to twice the largest
+    # score; row sum, quotient and weighted sum add (entries of the row + a few) half-ulps
+    score = 2 * float(mag.max()) * (feat + 2) * 2.0 ** -24 + (6 + 2.4 * float(s.abs().max())) * 2.0 ** -23
+    return out, size * (2 * score + (2 * deg[:, None].double() + 16) * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("feat", [128, 256, 300, 500, 512])
+@pytest.mark.parametrize("m,mean", [(19_717, 4), (50_000, 6), (2_000, 50)])
+def test_attention_keeps_its_probabilities_beside_the_pieces(cuda_device, feat, m, mean):
+    # the SpMM stage splits rows over blocks and needs scratch while the scratch of the stage before is its operand
+    ptr, cols = csr(cuda_device, m, m, mean, seed=feat)
+    q, k, v = (torch.rand(m, feat, device=cuda_device) * 2 - 1 for _ in range(3))
+    q *= 2.0 / feat ** 0.5
+    want, bound = attention_float64(q, k, v, ptr, cols)
+    o = torch.full((m * feat,), float("nan"), device=cuda_device)
+    call = lambda: ops.fusedmm(q.view(-1), k.view(-1), v.view(-1), o, ptr, cols)  # noqa: E731
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()  # a stream without buffers: they come out as small as asked for
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    assert bool(((o.view(m, feat).double() - want).abs() <= bound).all())
+    first = o.clone()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    assert torch.equal(first, o)
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    o.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(first, o)
