@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <vector>
@@ -35,6 +36,12 @@ bool dl_type(at::ScalarType t, DLDataType* out) {
   }
 }
 
+// Without the GIL, taken again whichever way the scope is left.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // Runs the call without the GIL on torch's current stream of `device` (-1: no device argument).
 int run(PackedFn fn, SetStreamFn set_stream, TVMValue* values, int* codes, int n, int device) {
   TVMValue ret;
@@ -44,16 +51,18 @@ int run(PackedFn fn, SetStreamFn set_stream, TVMValue* values, int* codes, int n
     void* st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
     if (set_stream(device, st) != 0) return -1;
   }
-  int rc = 0;
-  Py_BEGIN_ALLOW_THREADS
-  rc = fn(values, codes, n, &ret, &ret_code, nullptr);
-  Py_END_ALLOW_THREADS
-  return rc;
+  const NoGil no_gil;
+  return fn(values, codes, n, &ret, &ret_code, nullptr);
 }
+
+// C++ exceptions end at the functions below: a tensor without storage (inside torch.vmap, torch.func.jvp or
+// FakeTensorMode) throws from data_ptr(), and an exception that reached the interpreter's C frames would
+// end the process.
 
 // invoke(fn, set_stream, args) -> return code, or None when an argument is of a kind that only the
 // general packing on the Python side takes (or refuses with its message).
 PyObject* invoke(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
+  HANDLE_TH_ERRORS
   if (argc != 3 || !PyTuple_Check(argv[2])) {
     PyErr_SetString(PyExc_TypeError, "invoke(fn, set_stream, args)");
     return nullptr;
@@ -120,11 +129,13 @@ PyObject* invoke(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
     }
   }
   return PyLong_FromLong(run(fn, set_stream, values, codes, n, device));
+  END_HANDLE_TH_ERRORS
 }
 
 // invoke_packed(fn, set_stream, values, codes, n, device): the call of argument arrays packed before
 // (addresses of the arrays; device -1: no device argument).
 PyObject* invoke_packed(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
+  HANDLE_TH_ERRORS
   if (argc != 6) {
     PyErr_SetString(PyExc_TypeError, "invoke_packed(fn, set_stream, values, codes, n, device)");
     return nullptr;
@@ -141,11 +152,13 @@ PyObject* invoke_packed(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
     return nullptr;
   }
   return PyLong_FromLong(run(fn, set_stream, values, codes, static_cast<int>(n), static_cast<int>(device)));
+  END_HANDLE_TH_ERRORS
 }
 
 // flatten(list): replaces every tensor of the list that is not one-dimensional by its flat view
 // (or copy, as Tensor.reshape(-1) decides), in place; returns the list.
 PyObject* flatten(PyObject*, PyObject* list) {
+  HANDLE_TH_ERRORS
   if (!PyList_Check(list)) {
     PyErr_SetString(PyExc_TypeError, "flatten(list)");
     return nullptr;
@@ -159,6 +172,7 @@ PyObject* flatten(PyObject*, PyObject* list) {
   }
   Py_INCREF(list);
   return list;
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {

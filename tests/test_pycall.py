@@ -1,6 +1,9 @@
 """The extension that packs torch tensors for the packed calls: what a callee sees of every kind of
 argument, including more arguments than fit its stack arrays."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -63,3 +66,27 @@ def test_argument_lists_hold_flat_tensors():
     args = ops.hyb_args(x, y, [(w, rows, cols)], 8, 4)
     assert [a.dim() for a in args[:5]] == [1] * 5 and args[5:] == [8, 4]
     assert args[0].data_ptr() == x.data_ptr() and args[1] is y
+
+
+WITHOUT_STORAGE = {
+    "vmap": "torch.vmap(call)(torch.zeros(3, 4))",
+    "jvp": "torch.func.jvp(call, (torch.zeros(4),), (torch.ones(4),))",
+    "fake": """
+from torch._subclasses.fake_tensor import FakeTensorMode
+with FakeTensorMode():
+    call(torch.zeros(4))
+""",
+}
+
+
+@pytest.mark.parametrize("where", sorted(WITHOUT_STORAGE))
+def test_a_tensor_without_storage_is_a_python_error(where):
+    # in a process of its own: the fault to be seen here ends the process
+    calls = ["ops.csrmm(t, t, t, t, t)", "ops.csrmm(*[t] * 60)", "ops.hyb_spmm(*ops.hyb_args(t.view(1, -1), t, [(t, t, t)], 4))"]
+    code = "import torch\nfrom sparsetir_b200 import ops\n"
+    for op in calls:
+        body = "".join(f"    {line}\n" for line in WITHOUT_STORAGE[where].strip().splitlines())
+        code += f"def call(t):\n    {op}\n    return t\ntry:\n{body}except RuntimeError:\n    print('RuntimeError')\n"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert (r.returncode, r.stdout.split()) == (0, ["RuntimeError"] * 3), r.stderr[-2000:]
