@@ -70,6 +70,7 @@ csr_split_kernel(const SplitArgs s) {
   __shared__ __align__(16) float s_lead[SUBS][TILE];  // piece of a row that began before the sub-warp
   __shared__ __align__(16) float s_tail[SUBS][TILE];  // piece of a row that goes on behind it
   __shared__ int s_state[SUBS];                          // kLead, kOpen, kTail
+  __shared__ int s_bounds[2];                            // first stored entry, end of the last
   constexpr int kLead = 1, kOpen = 2, kTail = 4;         // kOpen: the lead piece is the whole span
 
   const int wlane = threadIdx.x & 31;
@@ -77,35 +78,53 @@ csr_split_kernel(const SplitArgs s) {
   const int sub = threadIdx.x / LPR;
   const unsigned mask = group_mask<LPR>();
   const long long block_entries = static_cast<long long>(SUBS) * s.span;
-  const long long blk0 = blockIdx.x * block_entries;
   const unsigned row_bytes = static_cast<unsigned>(s.feat) * 4u;
-  const long long p0l = blk0 + static_cast<long long>(sub) * s.span;
-  const int p0 = static_cast<int>(min(p0l, static_cast<long long>(s.nnz)));
-  const int count = static_cast<int>(min(p0l + s.span, static_cast<long long>(s.nnz))) - p0;
-  int cid = 0;
+  const long long warp_at = blockIdx.x * block_entries + static_cast<long long>((threadIdx.x / 32) * NW) * s.span;
+  // The stored entries are those between the first and the last row pointer: of a slice of a larger
+  // matrix, or of arrays with room behind, not all nnz.  The two pointers are not waited for: ids and
+  // row of the first entry are requested as if they were 0 and nnz, and once more where they are not.
+  int lo = 0, hi = s.nnz;
+  const int ptr_first = __ldg(s.indptr), ptr_last = __ldg(s.indptr + s.m);
+  int p0 = 0, count = 0, steps = 0, cid = 0;  // of the sub-warp: first entry, entries; entries of the warp's first sub-warp
   float av = 0.f;
   auto first_ids = [&]() {
+    cid = 0;
+    av = 0.f;
     if (lane < count) {
       cid = __ldg(s.indices + p0 + lane);
       av = __ldg(s.a + p0 + lane);
     }
   };
-  first_ids();  // on their way while the row is searched
-
-  const long long w0 = blk0 + static_cast<long long>((threadIdx.x / 32) * NW) * s.span;  // first entry of the warp
   int first_row = 0;
   bool first_lead = false;  // the first row of the sub-warp began before it
-  if (w0 < s.nnz) {
-    int pos[NW], row[NW];
+#pragma unroll 1
+  while (true) {
+    const long long w0 = lo + warp_at;  // first entry of the warp
+    const long long p0l = w0 + static_cast<long long>(wlane / LPR) * s.span;
+    p0 = static_cast<int>(min(p0l, static_cast<long long>(hi)));
+    count = static_cast<int>(min(p0l + s.span, static_cast<long long>(hi))) - p0;
+    first_ids();  // on their way while the row is searched
+    steps = static_cast<int>(max(0ll, min(static_cast<long long>(s.span), hi - w0)));
+    if (steps > 0) {
+      int pos[NW], row[NW];
 #pragma unroll
-    for (int i = 0; i < NW; ++i)
-      pos[i] = static_cast<int>(min(w0 + static_cast<long long>(i) * s.span, static_cast<long long>(s.nnz) - 1));
-    warp_rows_of<NW>(s.indptr, s.m, pos, s.rows_per_entry, wlane, row);
-    first_row = row[0];
+      for (int i = 0; i < NW; ++i)
+        pos[i] = static_cast<int>(min(w0 + static_cast<long long>(i) * s.span, static_cast<long long>(hi) - 1));
+      warp_rows_of<NW>(s.indptr, s.m, pos, s.rows_per_entry, wlane, row);
+      first_row = row[0];
 #pragma unroll
-    for (int i = 1; i < NW; ++i)
-      if (wlane / LPR == i) first_row = row[i];
-    first_lead = count > 0 && __ldg(s.indptr + first_row) < p0;
+      for (int i = 1; i < NW; ++i)
+        if (wlane / LPR == i) first_row = row[i];
+      first_lead = count > 0 && __ldg(s.indptr + first_row) < p0;
+    }
+    const int lo_now = max(0, min(ptr_first, s.nnz)), hi_now = max(lo_now, min(ptr_last, s.nnz));
+    if (lo == lo_now && hi == hi_now) break;
+    lo = lo_now;
+    hi = hi_now;
+  }
+  if (threadIdx.x == 0) {  // read behind a barrier: they need no registers in the loops
+    s_bounds[0] = lo;
+    s_bounds[1] = hi;
   }
 
   const int tiles = (s.feat + TILE - 1) / TILE;
@@ -129,7 +148,7 @@ csr_split_kernel(const SplitArgs s) {
       __syncthreads();  // the pieces of the tile before have been collected
     }
     int r = first_row, state = 0;
-    if (w0 < s.nnz) {  // the whole warp, its sub-warps in step
+    if (steps > 0) {  // the whole warp, its sub-warps in step
       int wend = row_window<LPR>(s.indptr, s.m, r, lane);
       bool lead = first_lead;
       if (lead) state = kLead;
@@ -137,7 +156,6 @@ csr_split_kernel(const SplitArgs s) {
       V acc[VPL];
 #pragma unroll
       for (int v = 0; v < VPL; ++v) acc[v] = LV::zero();
-      const int steps = static_cast<int>(min(static_cast<long long>(s.span), s.nnz - w0));
       for (int s0 = 0; s0 < steps; s0 += LPR) {
         int cidn = 0;
         float avn = 0.f;
@@ -213,7 +231,8 @@ csr_split_kernel(const SplitArgs s) {
     // ---- rows that cross sub-warps
     auto finish = [&](V (&sum)[VPL], int row, bool from_before, bool goes_on) {
       if (from_before || goes_on) {
-        const int begin = __ldg(s.indptr + row), end = __ldg(s.indptr + row + 1);
+        const int begin = __ldg(s.indptr + row) - s_bounds[0];
+        const int end = min(__ldg(s.indptr + row + 1), s_bounds[1]) - s_bounds[0];
         const int b0 = static_cast<int>(begin / block_entries), b1 = static_cast<int>((end - 1) / block_entries);
         char* pl = reinterpret_cast<char*>(s.part);
         auto piece = [&](int b) -> char* {
@@ -261,7 +280,7 @@ csr_split_kernel(const SplitArgs s) {
       }
       return true;
     };
-    const bool more_blocks = blk0 + block_entries < s.nnz;
+    const bool more_blocks = s_bounds[0] + (blockIdx.x + 1) * block_entries < s_bounds[1];
     if (sub == 0 && (state & kLead)) {
       V sum[VPL];
 #pragma unroll

@@ -66,3 +66,28 @@ def test_first_call_on_a_stream_can_be_captured(cuda_device):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("feat", [64, 41, 100, 512])
+@pytest.mark.parametrize("front,behind", [(0, 700), (1000, 0), (12_345, 30_000), (40_000, 1)])
+def test_entries_outside_the_row_pointers_count_for_nothing(cuda_device, feat, front, behind):
+    # row pointers of a row slice that start behind 0, and arrays with room behind the last row
+    rng = np.random.default_rng(feat)
+    m, n = 9000, 3000
+    deg = rng.poisson(7, m)
+    deg[[0, 1, 4000, 8998, 8999]] = [0, 3000, 5000, 700, 0]
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    nnz = int(indptr[-1])
+    dev = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    cols = dev(rng.integers(0, n, front + nnz + behind).astype(np.int32))
+    vals = torch.full((front + nnz + behind,), float("nan"), device=cuda_device)
+    vals[front:front + nnz] = torch.rand(nnz, device=cuda_device)
+    x = torch.rand(n * feat, device=cuda_device)
+    want, got, after = (torch.empty(m * feat, device=cuda_device) for _ in range(3))
+    ptr = dev(indptr)
+    ops.csrmm(vals[front:front + nnz].clone(), x, want, ptr, cols[front:front + nnz].clone())
+    ops.csrmm(vals, x, got, ptr + front, cols)
+    # blocks of other entries each: the same sums, the pieces of a row cut elsewhere
+    torch.testing.assert_close(got, want, rtol=5000 * 2.0 ** -24, atol=0)  # of up to 5,000 terms that are not negative
+    ops.csrmm(vals[front:front + nnz].clone(), x, after, ptr, cols[front:front + nnz].clone())
+    assert torch.equal(after, want)  # the call before left the counters at zero
