@@ -985,6 +985,7 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
     LeanArgs la{b, c, nullptr, nullptr, feat, all_atomic, PeerOut{}};
     if (to_peers) la.peers = *peers;
     bool clear = (flags & SPARSETIR_HYB_ZERO_C) || (all_atomic && (flags & SPARSETIR_HYB_REARM));
+    CallScratch cs;
     for (int q = 0; q < tb.nb; ++q) tb.part_base[q] = -1;
     if (!all_atomic) {
       // split rows live in the widest bucket(s) that carry row ids: one scratch row per ELL row
@@ -1010,16 +1011,25 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
         la.all_atomic = 1;
         clear = true;
       } else if (part_rows > 0) {
-        la.part = static_cast<float*>(workspace(device_id, st, part_bytes));
-        la.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
-        if (la.part == nullptr || la.counters == nullptr) return -1;
+        // Whole tiles are captured with the stream's own buffers where these have been reserved; everything
+        // else that is being captured gets memory of the graph (ragged feature counts and unaligned
+        // operands need no reservation: the kernels that they took before this one had no scratch).
+        if (vec4 && feat % (lane_w * lanes) == 0 && workspace_fits(device_id, st, part_bytes, counter_bytes)) {
+          cs.scratch = static_cast<char*>(workspace(device_id, st, part_bytes));
+          cs.counters = static_cast<unsigned*>(zeroed_workspace(device_id, st, counter_bytes));
+        } else if (take_scratch(device_id, st, part_bytes, counter_bytes, &cs) != 0) {
+          return -1;
+        }
+        la.part = reinterpret_cast<float*>(cs.scratch);
+        la.counters = cs.counters;
       }
     }
     if (clear) SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, c_bytes, st));
-    return dispatch_lean(tb, la, lanes, lane_w, st);
+    if (dispatch_lean(tb, la, lanes, lane_w, st) != 0) return -1;
+    return return_scratch(cs, st);
   }
 
-  // ---- fallback kernels for odd widths, feature counts or alignments
+  // ---- fallback kernels for ELL widths other than 1, 2, 4 and multiples of 8
   plan_items(tb, item_slots(lanes));
   if (flags & SPARSETIR_HYB_ZERO_C) {
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, c_bytes, st));

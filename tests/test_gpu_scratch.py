@@ -43,6 +43,16 @@ def tcspmm_call(device, feat):
     return y, lambda: ops.tcspmm(a, x, y, gp, ids, 375, 375, len(tiles), feat, 16, 16)
 
 
+def hyb_call(device, feat):
+    ptr, cols = (t.cpu().numpy() for t in csr(device, 3000, 4000, 5))
+    r, c, _, v, _ = fmt.column_part_hyb(3000, 4000, ptr, cols, 1, [1, 2, 4, 8, 16, 32],
+                                        data=np.random.default_rng(0).random(len(cols), np.float32))
+    up = lambda t: torch.from_numpy(np.ascontiguousarray(t).reshape(-1)).to(device)  # noqa: E731
+    buckets = [(up(v[0][b]), up(r[0][b]), up(c[0][b])) for b in range(6) if len(r[0][b])]
+    x, y = torch.rand(4000 * feat, device=device), torch.zeros(3000 * feat, device=device)
+    return y, lambda: ops.hyb_spmm(*ops.hyb_args(x, y, buckets, feat))
+
+
 CALLS = {"csrmm": csrmm_call, "tcspmm": tcspmm_call}
 
 
@@ -97,6 +107,22 @@ def test_calls_on_two_streams_at_once(cuda_device, op, captured):
     torch.cuda.synchronize()
     for (y, _), w in zip(pairs, want):
         assert torch.equal(y, w)
+
+
+@pytest.mark.parametrize("feat", [41, 100, 130])
+def test_the_first_hyb_call_on_a_stream_can_be_captured(cuda_device, feat):
+    y, call = hyb_call(cuda_device, feat)
+    call()
+    want, graph, stream = y.clone(), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    grow_buffers(stream)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
 
 
 def attention_float64(q, k, v, ptr, cols):
