@@ -687,12 +687,12 @@ hyb_spmm_async_kernel(const __grid_constant__ HybTable tb, const float* __restri
                                           valid, ring, acc, on_done);
 }
 
-// Fallback kernels only: zeroes the output rows that they accumulate into atomically (chunked wide
-// rows and split rows), so that repeated calls on the same C stay correct without a full memset.
-// One thread inspects one ELL row (coalesced reads of the row ids); the rows that need clearing
-// are rare, and each is then cleared by the whole warp.
+// Zeroes the output rows that are accumulated into atomically, so that repeated calls on the same C stay
+// correct without a full memset and rows that no bucket names stay as they are: with `all` every row of the
+// buckets, else what the fallback kernels add to (chunked wide rows and split rows).  One thread inspects
+// one ELL row (coalesced reads of the row ids); each row to be cleared is then cleared by the whole warp.
 __global__ void __launch_bounds__(kThreads)
-hyb_rearm_kernel(const __grid_constant__ HybTable tb, float* __restrict__ c, int feat) {
+hyb_rearm_kernel(const __grid_constant__ HybTable tb, float* __restrict__ c, int feat, bool all) {
   const int q = find_bucket(tb, blockIdx.x);
   const int nrows = tb.nrows[q];
   const int32_t* __restrict__ rows = tb.rows[q];
@@ -701,7 +701,7 @@ hyb_rearm_kernel(const __grid_constant__ HybTable tb, float* __restrict__ c, int
   bool clear = false;
   if (r < nrows) {
     row = row_id(rows, static_cast<int>(r), tb.row_base[q]);
-    clear = tb.chunks_per_row[q] > 1 || is_split_row(rows, static_cast<int>(r), nrows, row);
+    clear = all || tb.chunks_per_row[q] > 1 || is_split_row(rows, static_cast<int>(r), nrows, row);
     // of a run of equal ids only the first ELL row clears
     if (clear && r > 0 && rows != nullptr && __ldg(rows + r - 1) == row) clear = false;
   }
@@ -980,6 +980,19 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
     return 0;
   }
 
+  auto clear_rows = [&](bool all) -> int {
+    long long blocks = 0;
+    for (int q = 0; q < tb.nb; ++q) {
+      tb.block_start[q] = static_cast<int32_t>(blocks);
+      blocks += ceil_div(tb.nrows[q], kThreads);
+    }
+    tb.block_start[tb.nb] = static_cast<int32_t>(blocks);
+    if (blocks > INT32_MAX) return fail("sparsetir_hyb_spmm: too many thread blocks");
+    hyb_rearm_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(tb, c, feat, all);
+    SPTIR_LAUNCH_OK("hyb_rearm_kernel");
+    return 0;
+  };
+
   if (lean) {
     // ---- one writer per output row (or everything atomic when the caller asks for it)
     LeanArgs la{b, c, nullptr, nullptr, feat, all_atomic, PeerOut{}};
@@ -1002,14 +1015,14 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
       const size_t part_bytes = static_cast<size_t>(part_rows) * feat * sizeof(float);
       const size_t counter_bytes = static_cast<size_t>(part_rows) * tiles * sizeof(unsigned);
       if (part_rows > INT32_MAX || part_bytes > hyb_scratch_limit()) {
-        // a bucket list whose widest bucket holds most of the matrix: adding atomically into a
-        // cleared C costs less memory than a scratch copy of that size
+        // a bucket list whose widest bucket holds most of the matrix: adding atomically into
+        // cleared rows of C costs less memory than a scratch copy of that size
         if (to_peers)
           return fail("sparsetir_hyb_spmm_peers: the split rows need %zu bytes of scratch, beyond the limit; "
                       "run sparsetir_hyb_spmm and sparsetir_peer_scatter instead", part_bytes);
         for (int q = 0; q < tb.nb; ++q) tb.part_base[q] = -1;
         la.all_atomic = 1;
-        clear = true;
+        if (!clear && clear_rows(true) != 0) return -1;
       } else if (part_rows > 0) {
         // Whole tiles are captured with the stream's own buffers where these have been reserved; everything
         // else that is being captured gets memory of the graph (ragged feature counts and unaligned
@@ -1037,15 +1050,7 @@ int hyb_spmm_run(const float* b, float* c, const SparsetirEllBucket* buckets, co
     if (all_atomic) {
       SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, c_bytes, st));
     } else {
-      long long blocks = 0;
-      for (int q = 0; q < tb.nb; ++q) {
-        tb.block_start[q] = static_cast<int32_t>(blocks);
-        blocks += ceil_div(tb.nrows[q], kThreads);
-      }
-      tb.block_start[tb.nb] = static_cast<int32_t>(blocks);
-      if (blocks > INT32_MAX) return fail("sparsetir_hyb_spmm: too many thread blocks");
-      hyb_rearm_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(tb, c, feat);
-      SPTIR_LAUNCH_OK("hyb_rearm_kernel");
+      if (clear_rows(false) != 0) return -1;
     }
   }
 

@@ -1,5 +1,9 @@
 """hyb SpMM on feature counts that are not whole tiles and operands of every alignment, with rows
 that are split over several ELL rows, against a float64 product."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -28,8 +32,11 @@ def test_ragged_features_and_alignments(cuda_device, buckets, parts, feat, offse
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)  # noqa: E731
     bk = [(dev(v[p][b]), dev(r[p][b]), dev(c[p][b])) for p in range(parts) for b in range(len(buckets)) if len(r[p][b])]
     x = dev(rng.uniform(-1, 1, n * feat + offset).astype(np.float32))[offset:]
+    named = dev((deg > 0)[:, None].repeat(feat, 1).reshape(-1))
+    flags = L.HYB_ALL_ATOMIC | L.HYB_ZERO_C if parts > 1 else 0
     y = torch.zeros(m * feat + offset, device=cuda_device)[offset:]
-    flags = L.HYB_ZERO_C | (L.HYB_ALL_ATOMIC if parts > 1 else 0)
+    if parts == 1:  # no row needs clearing, and rows that occur in no bucket stay as they are
+        y[named] = float("nan")
     for _ in range(2):
         ops.hyb_spmm(*ops.hyb_args(x, y, bk, feat, flags))
     a = torch.zeros(m, n, dtype=torch.float64, device=cuda_device)
@@ -38,3 +45,36 @@ def test_ragged_features_and_alignments(cuda_device, buckets, parts, feat, offse
     # an fp32 sum of d products in any order: at most d half-ulps of the sum of magnitudes
     bound = mag * (dev(deg)[:, None].double() + 1) * 2.0 ** -24
     assert bool(((y.view(m, feat).double() - want).abs() <= bound).all())
+
+
+BEYOND_THE_LIMIT = """
+import numpy as np, torch
+from sparsetir_b200 import format as fmt, ops
+rng = np.random.default_rng(0)
+deg = np.concatenate([[2900, 0, 520, 0], rng.integers(0, 9, 900)])
+ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+cols = np.concatenate([np.sort(rng.choice(3000, d, replace=False)) for d in deg]).astype(np.int32)
+vals = rng.uniform(0.5, 1, len(cols)).astype(np.float32)
+r, c, _, v, _ = fmt.column_part_hyb(len(deg), 3000, ptr, cols, 1, [1, 4, 8], data=vals)
+up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+buckets = [(up(v[0][b]), up(r[0][b]), up(c[0][b])) for b in range(3)]
+a = torch.zeros(len(deg), 3000, dtype=torch.float64, device="cuda")
+a[up(np.repeat(np.arange(len(deg)), deg)), up(cols).long()] = up(vals).double()
+for feat in (64, 41, 100, 130):
+    x, y = torch.rand(3000, feat, device="cuda"), torch.full((len(deg), feat), 3.0, device="cuda")
+    for _ in range(2):
+        ops.hyb_spmm(*ops.hyb_args(x, y, buckets, feat))
+    want = a @ x.double()
+    want[up(deg == 0)] = 3.0
+    # up to 2,900 terms that are not negative, in any order
+    torch.testing.assert_close(y.double(), want, rtol=2901 * 2.0 ** -24, atol=0)
+print("done")
+"""
+
+
+def test_without_scratch_rows_of_no_bucket_stay_and_calls_repeat(cuda_device):
+    # SPARSETIR_HYB_SCRATCH_MB=0 (read once per process): split rows are added atomically into cleared rows
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", BEYOND_THE_LIMIT], env=dict(os.environ, SPARSETIR_HYB_SCRATCH_MB="0"), cwd=root,
+                       capture_output=True, text=True, timeout=600)
+    assert (r.returncode, r.stdout.split()) == (0, ["done"]), r.stderr[-2000:]
