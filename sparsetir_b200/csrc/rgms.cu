@@ -178,13 +178,18 @@ int launch_tile(const float* a, const float* w, const float* x, float* y, const 
   return 0;
 }
 
+// Bytes of Z at 128 and 256 features; 0 at other sizes.
+size_t wide_scratch(int feat, int nnz_i) {
+  return feat == 128 || feat == 256 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : 0;
+}
+
 }  // namespace
 }  // namespace sptir
 
 extern "C" int sparsetir_rgms_workspace(int feat, int nnz_i, size_t* scratch_bytes) {
   if (!scratch_bytes || feat < 0 || nnz_i < 0) return sptir::fail("sparsetir_rgms_workspace: bad argument");
   // the two-launch form keeps one aggregated feature row per (relation, destination) pair
-  *scratch_bytes = feat == 64 || feat == 128 || feat == 256 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : 0;
+  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : sptir::wide_scratch(feat, nnz_i);
   return 0;
 }
 
@@ -242,18 +247,22 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
                               nnz_i, z, st);
       if (rc <= 0) return rc;
     }
-    if (feat == 128 || feat == 256) {
-      // The same two steps with the transform of rgms_wide.cu.  A call that is being captured before
-      // its stream has the scratch, or that finds no memory for Z, keeps the kernels without scratch.
-      const size_t zb = static_cast<size_t>(nnz_i) * feat * sizeof(float);
+    if (wide_scratch(feat, nnz_i) > 0) {
+      // The same two steps with the transform of rgms_wide.cu.  Z is the stream's scratch, or, while the
+      // stream is being captured, memory of the graph.  An eager call that finds no memory for Z keeps the
+      // kernels without scratch.
+      CallScratch cs;
       cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-      if (!workspace_fits(device_id, st, zb, 0)) SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
-      float* z = capture == cudaStreamCaptureStatusNone ? static_cast<float*>(workspace(device_id, st, zb)) : nullptr;
-      if (z != nullptr) {
+      SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+      const int rc = take_scratch(device_id, st, wide_scratch(feat, nnz_i), 0, &cs);
+      if (rc == 0) {
+        float* z = reinterpret_cast<float*>(cs.scratch);
         if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, feat, nnz_j, device_id, stream) != 0)
           return -1;
-        return rgms_wide_launch(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat, st);
+        if (rgms_wide_launch(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat, st) != 0) return -1;
+        return return_scratch(cs, st);
       }
+      if (capture != cudaStreamCaptureStatusNone) return -1;
     }
     if (feat == 32)
       return launch_tile<32>(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, st);

@@ -125,6 +125,35 @@ def test_the_first_hyb_call_on_a_stream_can_be_captured(cuda_device, feat):
         assert torch.equal(y, want)
 
 
+def test_captured_rgms_outlives_the_buffers_of_its_stream(cuda_device):
+    n, rels, per, feat = 600, 4, 900, 128
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(0)
+    pair = torch.sort(torch.stack([torch.randperm(n, device=cuda_device, generator=g)[:300] for _ in range(rels)]), 1)[0]
+    ptr_i = torch.arange(0, rels * 300 + 1, 300, dtype=torch.int32, device=cuda_device)
+    ptr_j = torch.arange(0, rels * per + 1, per // 300, dtype=torch.int32, device=cuda_device)
+    src = torch.randint(0, n, (rels * per,), dtype=torch.int32, device=cuda_device, generator=g)
+    a, w, x = (torch.rand(k, device=cuda_device, generator=g) for k in (rels * per, rels * feat * feat, n * feat))
+    y = torch.zeros(n * feat, device=cuda_device)
+    rows = pair.reshape(-1).int()
+    call = lambda: ops.rgms(a, w, x, y, ptr_i, rows, ptr_j, src)  # noqa: E731
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    want = y.clone()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    grow_buffers(stream)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        # fp32 sums of at most 4 rows of terms that are not negative, added in any order
+        torch.testing.assert_close(y, want, rtol=8 * 2.0 ** -24, atol=0)
+
+
 def attention_float64(q, k, v, ptr, cols):
     """(result, bound of the error of fp32 stages in any order).  The numerator is not shifted by the row maximum:
     exp(s) / sum exp(s - max), as in the reference (tests/refimpl.py)."""
