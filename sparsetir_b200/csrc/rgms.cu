@@ -178,9 +178,12 @@ int launch_tile(const float* a, const float* w, const float* x, float* y, const 
   return 0;
 }
 
-// Bytes of Z at 128 and 256 features; 0 at other sizes.
+// Bytes of Z at 128 and 256 features; 0 where the kernels without scratch are taken: at other sizes, and
+// beyond 1 GiB (a layer of a million pairs at 256 features), so that a stream is not left with a buffer of
+// any size for layers that the kernels without scratch can do.
 size_t wide_scratch(int feat, int nnz_i) {
-  return feat == 128 || feat == 256 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : 0;
+  const size_t bytes = feat == 128 || feat == 256 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : 0;
+  return bytes <= (size_t{1} << 30) ? bytes : 0;
 }
 
 }  // namespace

@@ -201,3 +201,16 @@ def test_later_operators_validation_messages():
         ops.csr2bsr(f32(5), f32(4), i32(10), i32(5), i32(2), i32(1), 2)
     with pytest.raises(ops.SparseTIRError, match="indices.shape"):
         ops.ellmm(f32(2 * 3 * 16), f32(5 * 4 * 8), f32(2 * 4 * 8), i32(5), 2, 5, 8, 3, 4)
+
+
+def _query(name, *sizes, outs):
+    got = [ctypes.c_size_t(0) for _ in range(outs)]
+    assert getattr(L.load(), name)(*sizes, *(ctypes.byref(g) for g in got)) == 0, L.last_error()
+    return [g.value for g in got]
+
+
+def test_rgms_scratch_is_bounded():
+    assert _query("sparsetir_rgms_workspace", 64, 5000, outs=1) == [5000 * 64 * 4]
+    assert _query("sparsetir_rgms_workspace", 256, 1_000_000, outs=1) == [1_000_000 * 256 * 4]
+    for feat, pairs in ((128, 1 << 22), (256, 1 << 21), (32, 5000)):  # the kernels without scratch
+        assert _query("sparsetir_rgms_workspace", feat, pairs, outs=1) == [0]
