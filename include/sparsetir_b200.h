@@ -106,7 +106,11 @@ SPARSETIR_API void* sparsetir_get_stream(int device_id);
  * fail while the stream is being captured into a CUDA graph.  A caller that wants neither reserves
  * the buffers up front: after sparsetir_reserve_workspace(device, stream, s, c) no call on that
  * stream that needs at most s scratch bytes and c counter bytes allocates, synchronises or frees.
- * The *_workspace queries give the sizes an operator call needs (upper bounds). */
+ * The *_workspace queries give the sizes an operator call needs (upper bounds).
+ * Inside a capture csrmm, tcspmm, rgms at 128 and 256 features, the SpMM stage of fusedmm, and hyb_spmm on
+ * ragged or unaligned operands take memory of the graph instead.  The others keep the addresses of the
+ * stream's buffers in the graph: reserve the largest size that the stream will need before the capture, and do
+ * not replay such graphs beside calls of the same stream. */
 SPARSETIR_API int sparsetir_reserve_workspace(int device_id, void* stream, size_t scratch_bytes,
                                               size_t counter_bytes);
 
@@ -338,6 +342,14 @@ SPARSETIR_API int sparsetir_hyb_spmm_peers_raw(const float* b, float* c,
 SPARSETIR_API int sparsetir_hyb_spmm_workspace(const SparsetirEllBucket* buckets, int num_buckets,
                                                int feat, size_t* scratch_bytes,
                                                size_t* counter_bytes);
+/* The same for sparsetir_csrmm(_raw), sparsetir_fusedmm(_raw) and sparsetir_tcspmm(_raw), whatever the
+ * alignment of the operands. */
+SPARSETIR_API int sparsetir_csrmm_workspace(int m, int n, int feat, int nnz, size_t* scratch_bytes,
+                                            size_t* counter_bytes);
+SPARSETIR_API int sparsetir_fusedmm_workspace(int m, int n, int nnz, int feat, size_t* scratch_bytes,
+                                              size_t* counter_bytes);
+SPARSETIR_API int sparsetir_tcspmm_workspace(int nnzb, int feat, int tile_size, int group_size,
+                                             size_t* scratch_bytes, size_t* counter_bytes);
 /* The feature tile the main hyb kernel uses for 16/32-byte aligned operands with n rows of b:
  * `lanes` lanes of `lane_floats` floats each (the kernel is hyb_spmm_lean_kernel<lanes, lane_floats>,
  * launched with feat / (lanes * lane_floats) tiles in grid.y).  For tools that match a launch with

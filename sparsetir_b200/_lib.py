@@ -98,6 +98,9 @@ PLAIN_SYMBOLS = {
     "sparsetir_hyb_spmm_tile": (_i, [_i, _i, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "sparsetir_hyb_spmm_workspace": (_i, [ctypes.POINTER(EllBucket), _i, _i,
                                           ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)]),
+    "sparsetir_csrmm_workspace": (_i, [_i] * 4 + [ctypes.POINTER(ctypes.c_size_t)] * 2),
+    "sparsetir_fusedmm_workspace": (_i, [_i] * 4 + [ctypes.POINTER(ctypes.c_size_t)] * 2),
+    "sparsetir_tcspmm_workspace": (_i, [_i] * 4 + [ctypes.POINTER(ctypes.c_size_t)] * 2),
     "sparsetir_set_validate": (_i, [_i]),
     "sparsetir_peer_scatter": (_i, [_i, _vp, _vp, ctypes.c_size_t, _i, ctypes.POINTER(ctypes.c_void_p)]),
     "sparsetir_version": (_i, []),

@@ -399,13 +399,24 @@ inline uintptr_t low_bits(const float* b, const float* c) {
 
 }  // namespace
 
-// Bytes of scratch that the pieces of a call need.
+// Bytes of scratch that the pieces of this call need.
 size_t csr_split_scratch(const float* b, const float* c, int m, int n, int feat, int nnz) {
   if (nnz == 0) return 0;
   return split_plan(split_shape(low_bits(b, c), n, feat, nnz), m, feat, nnz).part_bytes;
 }
 
-// pieces: that many bytes, 16-byte aligned, from a caller that holds the stream's scratch buffer; null:
+// The most that a call of these sizes needs, whatever its operands' alignment.
+void csr_split_scratch_bound(int m, int n, int feat, int nnz, size_t* part_bytes, size_t* counter_bytes) {
+  *part_bytes = *counter_bytes = 0;
+  if (m == 0 || feat == 0 || nnz == 0) return;
+  for (const uintptr_t bits : {16, 8, 4}) {
+    const SplitPlan p = split_plan(split_shape(bits, n, feat, nnz), m, feat, nnz);
+    *part_bytes = std::max(*part_bytes, p.part_bytes);
+    *counter_bytes = std::max(*counter_bytes, p.counter_bytes);
+  }
+}
+
+// pieces: csr_split_scratch() bytes, 16-byte aligned, from a caller that holds the stream's scratch buffer; null:
 // the call takes its scratch itself.
 int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
                   int m, int n, int feat, int nnz, void* pieces, int device_id, cudaStream_t st) {

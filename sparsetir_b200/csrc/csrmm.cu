@@ -192,6 +192,7 @@ namespace sptir {
 int csr_split_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
                   int m, int n, int feat, int nnz, void* pieces, int device_id, cudaStream_t st);
 size_t csr_split_scratch(const float* b, const float* c, int m, int n, int feat, int nnz);
+void csr_split_scratch_bound(int m, int n, int feat, int nnz, size_t* part_bytes, size_t* counter_bytes);
 
 namespace {
 // Whether a call takes the row-wise kernel, and with which lanes.
@@ -291,6 +292,13 @@ int csrmm_short_rows_impl(const float* a, const float* b, float* c, const int32_
                    nullptr);
 }
 }  // namespace sptir
+
+extern "C" int sparsetir_csrmm_workspace(int m, int n, int feat, int nnz, size_t* scratch_bytes, size_t* counter_bytes) {
+  if (m < 0 || n < 0 || feat < 0 || nnz < 0 || !scratch_bytes || !counter_bytes)
+    return sptir::fail("sparsetir_csrmm_workspace: bad argument");
+  sptir::csr_split_scratch_bound(m, n, feat, nnz, scratch_bytes, counter_bytes);
+  return 0;
+}
 
 extern "C" int sparsetir_csrmm_raw(const float* a, const float* b, float* c, const int32_t* indptr,
                                    const int32_t* indices, int m, int n, int feat, int nnz,

@@ -313,21 +313,36 @@ tcspmm_simt_kernel(const __half* __restrict__ a, const __half* __restrict__ b, O
   }
 }
 
-template <int MT, typename OutT>
-int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
-  s.slabs = ceil_div(s.feat, mma16::kSlab);
+struct TcPlan {
+  int slabs, window_log, windows;
+  size_t part_bytes, counter_bytes;
+};
+
+TcPlan tc_plan(int nnzb, int t, int feat) {
+  TcPlan p;
+  p.slabs = ceil_div(feat, mma16::kSlab);
   // Windows of 128 groups keep the scratch small; down to 32 where there would not be enough blocks
   // (20 k rows, 6,118 groups, F = 64: 12.4 against 18.9 us).
-  s.window_log = 5;
-  while (s.window_log < 7 && (static_cast<long long>(s.nnzb) * s.slabs >> s.window_log) > 4 * kNumSMs) ++s.window_log;
-  s.windows = ceil_div(s.nnzb, 1 << s.window_log);
+  p.window_log = 5;
+  while (p.window_log < 7 && (static_cast<long long>(nnzb) * p.slabs >> p.window_log) > 4 * kNumSMs) ++p.window_log;
+  p.windows = ceil_div(nnzb, 1 << p.window_log);
+  const int row_tiles = t > 16 ? 2 : 1;
+  p.part_bytes = 2 * static_cast<size_t>(p.windows) * p.slabs * row_tiles * kThreads * 8 * sizeof(float);
+  p.counter_bytes = static_cast<size_t>(std::max(p.windows, 1)) * p.slabs * sizeof(unsigned);
+  return p;
+}
+
+template <int MT, typename OutT>
+int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
+  const TcPlan p = tc_plan(s.nnzb, s.t, s.feat);
+  s.slabs = p.slabs;
+  s.window_log = p.window_log;
+  s.windows = p.windows;
   s.tiles_per_group = s.nnzb > 0 ? static_cast<float>(s.mb) / static_cast<float>(s.nnzb) : 0.f;
   const long long blocks = (static_cast<long long>(s.windows) + ceil_div(s.mb, 4)) * s.slabs;
   if (blocks > INT32_MAX) return fail("sparsetir_tcspmm: too many thread blocks");
-  const size_t part_bytes = 2 * static_cast<size_t>(s.windows) * s.slabs * MT * kThreads * 8 * sizeof(float);
-  const size_t counter_bytes = static_cast<size_t>(std::max(s.windows, 1)) * s.slabs * sizeof(unsigned);
   CallScratch cs;
-  if (take_scratch(device_id, st, part_bytes, counter_bytes, &cs) != 0) return -1;
+  if (take_scratch(device_id, st, p.part_bytes, p.counter_bytes, &cs) != 0) return -1;
   s.part = reinterpret_cast<float*>(cs.scratch);
   s.counters = cs.counters;
   tcspmm_mma_kernel<MT, OutT><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(s);
@@ -335,10 +350,13 @@ int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
   return return_scratch(cs, st);
 }
 
+// Whether the operands' shape, alignment aside, is one that the matrix instruction takes.
+inline bool mma_shape(int t, int g, int feat) { return g == kG && (t == 8 || t == 16 || t == 32) && feat % 8 == 0; }
+
 template <typename OutT>
 int launch_all(const __half* a, const __half* b, OutT* c, const int32_t* indptr, const int32_t* indices,
                int mb, int nnzb, int t, int g, int feat, int device_id, cudaStream_t st) {
-  if (g == kG && (t == 8 || t == 16 || t == 32) && feat % 8 == 0 && aligned16(a) && aligned16(b)) {
+  if (mma_shape(t, g, feat) && aligned16(a) && aligned16(b)) {
     const TcArgs s{a, b, c, indptr, indices, nullptr, nullptr, mb, nnzb, t, feat, 0, 0, 0, 0.f, aligned16(indices), aligned16(c)};
     if (t == 32) return launch_mma<2, OutT>(s, device_id, st);
     return launch_mma<1, OutT>(s, device_id, st);
@@ -350,6 +368,19 @@ int launch_all(const __half* a, const __half* b, OutT* c, const int32_t* indptr,
 
 }  // namespace
 }  // namespace sptir
+
+extern "C" int sparsetir_tcspmm_workspace(int nnzb, int feat, int tile_size, int group_size, size_t* scratch_bytes,
+                                          size_t* counter_bytes) {
+  using namespace sptir;
+  if (nnzb < 0 || feat < 0 || tile_size < 1 || group_size < 1 || !scratch_bytes || !counter_bytes)
+    return fail("sparsetir_tcspmm_workspace: bad argument");
+  *scratch_bytes = *counter_bytes = 0;
+  if (feat == 0 || !mma_shape(tile_size, group_size, feat)) return 0;
+  const TcPlan p = tc_plan(nnzb, tile_size, feat);
+  *scratch_bytes = p.part_bytes;
+  *counter_bytes = p.counter_bytes;
+  return 0;
+}
 
 extern "C" int sparsetir_tcspmm_raw(const void* a_f16, const void* b_f16, void* c, int c_is_f16,
                                     const int32_t* indptr, const int32_t* indices, int mb, int nb,

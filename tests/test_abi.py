@@ -214,3 +214,15 @@ def test_rgms_scratch_is_bounded():
     assert _query("sparsetir_rgms_workspace", 256, 1_000_000, outs=1) == [1_000_000 * 256 * 4]
     for feat, pairs in ((128, 1 << 22), (256, 1 << 21), (32, 5000)):  # the kernels without scratch
         assert _query("sparsetir_rgms_workspace", feat, pairs, outs=1) == [0]
+
+
+def test_scratch_queries_refuse_bad_arguments():
+    out = [ctypes.byref(ctypes.c_size_t(0)) for _ in range(2)]
+    for name in ("sparsetir_csrmm_workspace", "sparsetir_fusedmm_workspace", "sparsetir_tcspmm_workspace"):
+        assert getattr(L.load(), name)(-1, 8, 8, 8, *out) == -1 and "bad argument" in L.last_error()
+        assert getattr(L.load(), name)(8, 8, 8, 8, None, None) == -1 and "bad argument" in L.last_error()
+        assert _query(name, 0, 8, 16, 16, outs=2)[0] == 0
+    # scores, probabilities and the SpMM's pieces
+    csrmm, both = (_query(f"sparsetir_{op}_workspace", *sizes, outs=2)
+                   for op, sizes in (("csrmm", (9000, 9000, 100, 80_000)), ("fusedmm", (9000, 9000, 80_000, 100))))
+    assert both == [csrmm[0] + 2 * 80_000 * 4, csrmm[1]] and csrmm[0] > 0 and csrmm[1] > 0

@@ -56,6 +56,11 @@ def hyb_call(device, feat):
 CALLS = {"csrmm": csrmm_call, "tcspmm": tcspmm_call}
 
 
+def fresh_stream():
+    """A stream without buffers: of the high-priority pool, which hands out 32 before it repeats."""
+    return torch.cuda.Stream(priority=-1)
+
+
 def grow_buffers(stream):
     """Makes the library give up the buffers that the stream has for larger ones."""
     assert L.load().sparsetir_reserve_workspace(0, ctypes.c_void_p(stream.cuda_stream), 48 << 20, 4 << 20) == 0
@@ -113,7 +118,7 @@ def test_calls_on_two_streams_at_once(cuda_device, op, captured):
 def test_the_first_hyb_call_on_a_stream_can_be_captured(cuda_device, feat):
     y, call = hyb_call(cuda_device, feat)
     call()
-    want, graph, stream = y.clone(), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    want, graph, stream = y.clone(), torch.cuda.CUDAGraph(), fresh_stream()
     torch.cuda.synchronize()
     with torch.cuda.graph(graph, stream=stream):
         call()
@@ -187,7 +192,7 @@ def test_attention_keeps_its_probabilities_beside_the_pieces(cuda_device, feat, 
     want, bound = attention_float64(q, k, v, ptr, cols)
     o = torch.full((m * feat,), float("nan"), device=cuda_device)
     call = lambda: ops.fusedmm(q.view(-1), k.view(-1), v.view(-1), o, ptr, cols)  # noqa: E731
-    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()  # a stream without buffers: they come out as small as asked for
+    stream, graph = fresh_stream(), torch.cuda.CUDAGraph()  # its buffers come out as small as asked for
     torch.cuda.synchronize()
     with torch.cuda.stream(stream):
         call()
@@ -204,3 +209,30 @@ def test_attention_keeps_its_probabilities_beside_the_pieces(cuda_device, feat, 
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(first, o)
+
+
+@pytest.mark.parametrize("feat", [100, 256, 41])
+def test_calls_on_a_reserved_stream_allocate_nothing(cuda_device, feat):
+    lib, stream = L.load(), fresh_stream()
+    m = n = 20_000
+    ptr, cols = csr(cuda_device, m, n, 12)
+    nnz = len(cols)
+    vals, q, k, v, o = (torch.rand(size, device=cuda_device) for size in (nnz, m * feat, n * feat, n * feat, m * feat))
+    calls = [(("sparsetir_csrmm_workspace", m, n, feat, nnz), lambda: ops.csrmm(vals, v, o, ptr, cols)),
+             (("sparsetir_fusedmm_workspace", m, n, nnz, feat), lambda: ops.fusedmm(q, k, v, o, ptr, cols))]
+    groups, t = 3000, 16
+    a = torch.ones(groups * t * 16, device=cuda_device, dtype=torch.float16)
+    gp = torch.tensor([0, 2900, 2900, groups], dtype=torch.int32, device=cuda_device)
+    ids = torch.arange(groups * 16, device=cuda_device).remainder(n).int()
+    b, c = torch.rand(n * 64, device=cuda_device).half(), torch.empty(3 * t * 64, device=cuda_device)
+    calls.append((("sparsetir_tcspmm_workspace", groups, 64, t, 16), lambda: ops.tcspmm(a, b, c, gp, ids, 3, n // 16, groups, 64, t, 16)))
+    for (query, *sizes), call in calls:
+        need = [ctypes.c_size_t(0) for _ in range(2)]
+        assert getattr(lib, query)(*sizes, *(ctypes.byref(x) for x in need)) == 0
+        assert lib.sparsetir_reserve_workspace(0, ctypes.c_void_p(stream.cuda_stream), *need) == 0
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        with torch.cuda.stream(stream):
+            call()
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == free
