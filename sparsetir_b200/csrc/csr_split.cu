@@ -36,9 +36,9 @@ struct SplitArgs {
   float* c;
   const int32_t* indptr;
   const int32_t* indices;
-  float* part;         // two scratch rows per block: the piece of a row that began before it, and
+  float* part;         // two scratch rows per block with entries: the piece of a row that began before it, and
                        // of a row that goes on behind it
-  unsigned* counters;  // [blocks][feature tiles], zero before and after every launch
+  unsigned* counters;  // [blocks with entries][feature tiles], zero before and after every launch
   int m, nnz, feat, span;
   float rows_per_entry;
 };
@@ -359,10 +359,10 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
   const long long want = resident / p.gy * subs;
   p.span = static_cast<int>((nnz + want - 1) / want + sh.lanes - 1) / sh.lanes * sh.lanes;
   const long long per_block = static_cast<long long>(subs) * p.span;
-  p.blocks = static_cast<int>(std::max((nnz + per_block - 1) / per_block,
-                                       (static_cast<long long>(m) + 8 * kThreads - 1) / (8 * kThreads)));
-  p.part_bytes = 2 * static_cast<size_t>(p.blocks) * feat * sizeof(float);
-  p.counter_bytes = static_cast<size_t>(p.blocks) * tiles * sizeof(unsigned);
+  const long long with_entries = (nnz + per_block - 1) / per_block;  // the first blocks; the others clear rows
+  p.blocks = static_cast<int>(std::max(with_entries, (static_cast<long long>(m) + 8 * kThreads - 1) / (8 * kThreads)));
+  p.part_bytes = 2 * static_cast<size_t>(with_entries) * feat * sizeof(float);
+  p.counter_bytes = static_cast<size_t>(with_entries) * tiles * sizeof(unsigned);
   return p;
 }
 

@@ -226,3 +226,12 @@ def test_scratch_queries_refuse_bad_arguments():
     csrmm, both = (_query(f"sparsetir_{op}_workspace", *sizes, outs=2)
                    for op, sizes in (("csrmm", (9000, 9000, 100, 80_000)), ("fusedmm", (9000, 9000, 80_000, 100))))
     assert both == [csrmm[0] + 2 * 80_000 * 4, csrmm[1]] and csrmm[0] > 0 and csrmm[1] > 0
+
+
+def test_csrmm_scratch_goes_with_the_blocks_that_hold_entries():
+    few, many = (_query("sparsetir_csrmm_workspace", m, 1000, 512, 70_000, outs=2) for m in (9000, 2_000_000_000))
+    assert few == many and few[0] <= 4 << 20
+    # one wave of blocks at most, however many entries
+    for feat in (1, 41, 100, 512, 4096):
+        scratch, counters = _query("sparsetir_csrmm_workspace", 1_000_000, 1_000_000, feat, 2_000_000_000, outs=2)
+        assert scratch <= 2 * 4 * 148 * feat * 4 and counters <= 4 * 148 * (feat // 32 + 1) * 4
