@@ -326,8 +326,11 @@ TcPlan tc_plan(int nnzb, int t, int feat) {
   p.window_log = 5;
   while (p.window_log < 7 && (static_cast<long long>(nnzb) * p.slabs >> p.window_log) > 4 * kNumSMs) ++p.window_log;
   p.windows = ceil_div(nnzb, 1 << p.window_log);
-  const int row_tiles = t > 16 ? 2 : 1;
-  p.part_bytes = 2 * static_cast<size_t>(p.windows) * p.slabs * row_tiles * kThreads * 8 * sizeof(float);
+  // Longer windows where the pieces would take more than 64 MB (there are thousands of blocks by then): with
+  // windows of 128 groups they grow with the matrix, at 512 features to the size of its values.
+  const size_t window_bytes = 2 * static_cast<size_t>(p.slabs) * (t > 16 ? 2 : 1) * kThreads * 8 * sizeof(float);
+  while (p.windows > 1 && p.windows * window_bytes > (size_t{64} << 20)) p.windows = ceil_div(nnzb, 1 << ++p.window_log);
+  p.part_bytes = p.windows * window_bytes;
   p.counter_bytes = static_cast<size_t>(std::max(p.windows, 1)) * p.slabs * sizeof(unsigned);
   return p;
 }

@@ -235,3 +235,11 @@ def test_csrmm_scratch_goes_with_the_blocks_that_hold_entries():
     for feat in (1, 41, 100, 512, 4096):
         scratch, counters = _query("sparsetir_csrmm_workspace", 1_000_000, 1_000_000, feat, 2_000_000_000, outs=2)
         assert scratch <= 2 * 4 * 148 * feat * 4 and counters <= 4 * 148 * (feat // 32 + 1) * 4
+
+
+def test_tcspmm_scratch_is_bounded():
+    for feat in (8, 128, 512, 4096):
+        for groups in (0, 1, 57_508, 3_000_000, 130_000_000, 2 ** 31 - 1):
+            scratch, counters = _query("sparsetir_tcspmm_workspace", groups, feat, 32, 16, outs=2)
+            assert scratch <= 64 << 20 and counters <= 1 << 20
+    assert _query("sparsetir_tcspmm_workspace", 3000, 64, 16, 8, outs=2) == [0, 0]  # a shape for CUDA cores

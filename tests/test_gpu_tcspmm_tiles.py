@@ -1,9 +1,12 @@
 """The condensed SpMM with row tiles of every length: empty runs, tiles at the border between one warp and a
 window, hub tiles over several windows, feature counts that are not whole slabs."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
+from sparsetir_b200 import _lib as L
 from sparsetir_b200 import format as fmt
 from sparsetir_b200 import ops
 
@@ -97,3 +100,27 @@ def test_unaligned_operands(cuda_device):
         ops.tcspmm(up(mask).half(), b, c, up(gp), ids, 32, 32, len(tiles), 72, 16, 16)
         outs.append(c.clone())
     assert torch.equal(outs[0], outs[1])
+
+
+def test_long_windows_of_large_products(cuda_device):
+    # 4,096 features: windows of 128 groups would need more scratch than the operator takes
+    feat, t, n = 4096, 16, 6400
+    lengths = [400, 0, 3, 130, 399, 16, 17] + [350] * 60  # groups per row tile
+    gp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    groups = int(gp[-1])
+    need = [ctypes.c_size_t(0) for _ in range(2)]
+    assert L.load().sparsetir_tcspmm_workspace(groups, feat, t, 16, *(ctypes.byref(x) for x in need)) == 0
+    assert need[0].value < groups * (feat // 64) * 64  # what windows of 128 groups need: the case is beyond the limit
+    rng = np.random.default_rng(0)
+    ids = np.concatenate([np.sort(rng.choice(n, g * 16, replace=False)) for g in lengths]).astype(np.int32)
+    up = lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(cuda_device)  # noqa: E731
+    a = torch.rand(groups * t * 16, device=cuda_device).half()
+    b = torch.rand(n, feat, device=cuda_device).half()
+    c = torch.full((len(lengths) * t * feat,), 3.0, device=cuda_device)
+    for _ in range(2):
+        ops.tcspmm(a, b.view(-1), c, up(gp), up(ids), len(lengths), n // 16, groups, feat, t, 16)
+    for io, g in enumerate(lengths):
+        block = a.view(groups, t, 16)[gp[io]:gp[io + 1]].permute(1, 0, 2).reshape(t, -1).double()
+        want = block @ b[up(ids[gp[io] * 16:gp[io + 1] * 16]).long()].double()
+        # fp32 sums of exact products that are not negative
+        assert bool(((c.view(-1, t, feat)[io].double() - want).abs() <= want * (g * 16 + 4) * 2.0 ** -23).all())
