@@ -146,6 +146,8 @@ class SparseConvPlan:
     calls, so the host conversion is not part of the steady state (the reference also converts
     before it times, rgms.py:677-710 against :861-864)."""
 
+    _map: Optional[torch.Tensor] = None  # also of a plan that was saved when plans had no map
+
     def __init__(self, nbmaps, nbsizes, transposed: bool, num_inputs: int,
                  num_outputs: Optional[int] = None, device: Optional[torch.device] = None,
                  group_size: int = 128, buckets: Sequence[int] = (1,)):
@@ -157,7 +159,6 @@ class SparseConvPlan:
         self.buckets = [tuple(torch.from_numpy(np.ascontiguousarray(a)).to(self.device) for a in bk)
                         for bk in host]
         # at most 1 GB: layers beyond that, and layers with repeated pairs, keep the buckets alone
-        self._map = None
         if self.num_pairs > 0 and self.num_offsets * self.num_outputs <= 1 << 28:
             self._map = neighbour_map(nbmaps, nbsizes, bool(transposed), self.num_outputs, self.device)
 

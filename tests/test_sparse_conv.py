@@ -2,11 +2,14 @@
 examples/rgms/sparse_conv/sparse_conv.py:93-125): neighbour maps -> one relation per kernel offset
 -> CSF -> ELL3D with buckets = [1] -> the half-precision RGMS operator, against the plain
 gather-matmul-scatter  y[o] += x[i] @ W[offset]  that a sparse convolution stands for."""
+import pickle
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import oracle as orc
+from sparsetir_b200 import ops
 from sparsetir_b200 import sparse_conv as sc
 
 
@@ -73,6 +76,19 @@ def test_maps_are_validated():
         sc.ell3d_from_maps(maps, [len(maps), 1, 0], False, 20, 20)
     with pytest.raises(ValueError, match=r"\[pairs, 2\]"):
         sc.ell3d_from_maps(maps.reshape(-1), sizes, False, 20, 20)
+
+
+def test_a_plan_saved_without_a_map_still_reaches_the_operator():
+    # plans of the time before the neighbour map hold the buckets alone
+    maps, sizes, x, w = layer(2, 3, 20, 20, 16, 16, False, repeats=False)
+    plan = sc.SparseConvPlan(maps, sizes, False, 20, 20, device=torch.device("cpu"))
+    assert plan._map is not None
+    saved = {name: value for name, value in plan.__dict__.items() if name != "_map"}
+    old = pickle.loads(pickle.dumps(plan))
+    old.__dict__.clear()
+    old.__dict__.update(saved)
+    with pytest.raises(ops.SparseTIRError, match="no CPU path"):
+        old(torch.from_numpy(x), torch.from_numpy(w))
 
 
 @pytest.mark.gpu
