@@ -183,12 +183,15 @@ def pycall():
     when it has not been built."""
     global _pycall
     if _pycall is None:
-        import torch  # noqa: F401  (its libraries must be loaded first)
+        import torch  # its libraries must be loaded first
         try:
             from . import _pycall as module
         except ImportError as e:
             raise LibraryError(f"{os.path.join(_PKG, '_pycall.so')} cannot be loaded ({e}): build it with "
                                "`python -m sparsetir_b200.build`") from e
+        if module.torch_version != torch.__version__:
+            raise LibraryError(f"{os.path.join(_PKG, '_pycall.so')} was built for torch {module.torch_version}, this is "
+                               f"torch {torch.__version__}: build it with `python -m sparsetir_b200.build`")
         _pycall = module
     return _pycall
 

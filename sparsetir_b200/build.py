@@ -69,28 +69,45 @@ def _compile(src: str, force: bool, verbose: bool, hdr_mtime: float) -> str:
     return obj
 
 
-def build_pycall(force: bool = False) -> str:
-    """The extension module against this Python's and this torch's headers (g++)."""
-    import torch
+def build_pycall(force: bool = False, cuda: bool | None = None, out: str = PYCALL_PATH) -> str | None:
+    """The extension module against this Python's and this torch's headers (g++).  Without torch there
+    is nothing to pack and nothing is built; a torch without CUDA (``cuda=False``) has no streams to ask for."""
+    try:
+        import torch
+    except ImportError:
+        print("torch is not installed: building the library alone, without _pycall.so", file=sys.stderr)
+        return None
 
     src = os.path.join(CSRC, "pycall.cc")
-    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(INCLUDE, "sparsetir_b200.h")))
-    if not force and os.path.exists(PYCALL_PATH) and os.path.getmtime(PYCALL_PATH) > newest:
-        return PYCALL_PATH
     torch_dir = os.path.dirname(os.path.abspath(torch.__file__))
     lib_dir = os.path.join(torch_dir, "lib")
-    cuda_include = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    if cuda is None:
+        cuda = torch.version.cuda is not None
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DSPTIR_TORCH_VERSION="{torch.__version__}"',
+           f"-DSPTIR_TORCH_CUDA={int(cuda)}", "-I", INCLUDE,
            "-isystem", sysconfig.get_path("include"), "-isystem", os.path.join(torch_dir, "include"),
-           "-isystem", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
-           "-isystem", cuda_include, src, "-o", PYCALL_PATH, "-L", lib_dir, f"-Wl,-rpath,{lib_dir}",
-           "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+           "-isystem", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include")]
+    if cuda:
+        cmd += ["-isystem", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    cmd += [src, "-o", out, "-L", lib_dir, f"-Wl,-rpath,{lib_dir}", "-ltorch_python", "-ltorch_cpu",
+            *(["-lc10_cuda"] if cuda else []), "-lc10"]
+    # the command names torch's version and folder and Python's headers: another one of them builds anew
+    made_by = os.path.join(OBJ_DIR, "pycall.cmd") if out == PYCALL_PATH else out + ".cmd"
+    key = "\n".join(cmd).replace(ROOT, "")  # wherever this tree lies
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(INCLUDE, "sparsetir_b200.h")))
+    if not force and os.path.exists(out) and os.path.exists(made_by) and os.path.getmtime(out) > newest:
+        with open(made_by) as f:
+            if f.read() == key:
+                return out
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(f"$ {' '.join(cmd)}\n{res.stdout}{res.stderr}")
         raise RuntimeError("g++ failed on pycall.cc")
-    return PYCALL_PATH
+    os.makedirs(os.path.dirname(made_by), exist_ok=True)
+    with open(made_by, "w") as f:
+        f.write(key)
+    return out
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -10,7 +10,9 @@
 // the entry points it resolved, so that another build of the library can be loaded.
 #include <Python.h>
 
+#if SPTIR_TORCH_CUDA
 #include <c10/cuda/CUDAStream.h>
+#endif
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -47,10 +49,15 @@ int run(PackedFn fn, SetStreamFn set_stream, TVMValue* values, int* codes, int n
   TVMValue ret;
   int ret_code = 0;
   ret.v_int64 = 0;
+#if SPTIR_TORCH_CUDA  // without it torch has no CUDA tensors
   if (device >= 0) {
     void* st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
     if (set_stream(device, st) != 0) return -1;
   }
+#else
+  (void)set_stream;
+  (void)device;
+#endif
   const NoGil no_gil;
   return fn(values, codes, n, &ret, &ret_code, nullptr);
 }
@@ -186,4 +193,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pycall", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__pycall() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__pycall() {
+  PyObject* m = PyModule_Create(&module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", SPTIR_TORCH_VERSION) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from sparsetir_b200 import _lib as L
+from sparsetir_b200 import build
 from sparsetir_b200 import ops
 
 
@@ -90,3 +91,34 @@ def test_a_tensor_without_storage_is_a_python_error(where):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert (r.returncode, r.stdout.split()) == (0, ["RuntimeError"] * 3), r.stderr[-2000:]
+
+
+def test_another_torch_builds_the_extension_anew(monkeypatch):
+    build.build_pycall()
+    ran = []
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **_: ran.append(cmd) or subprocess.CompletedProcess(cmd, 1, "", ""))
+    assert build.build_pycall() == build.PYCALL_PATH and not ran
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.raises(RuntimeError, match="g\\+\\+ failed"):
+        build.build_pycall()
+    assert len(ran) == 1 and '-DSPTIR_TORCH_VERSION="0.0.1"' in ran[0]
+    monkeypatch.setattr(L, "_pycall", None)
+    with pytest.raises(L.LibraryError, match="this is torch 0.0.1"):
+        L.pycall()
+
+
+def test_the_library_builds_without_torch(monkeypatch):
+    monkeypatch.setitem(sys.modules, "torch", None)  # import torch raises ImportError
+    assert build.build_pycall(force=True) is None
+
+
+def test_the_extension_builds_without_cuda(tmp_path):
+    out = build.build_pycall(cuda=False, out=str(tmp_path / "_pycall.so"))
+    code = ("import importlib.util, torch\n"
+            f"spec = importlib.util.spec_from_file_location('_pycall', {out!r})\n"
+            "module = importlib.util.module_from_spec(spec)\nspec.loader.exec_module(module)\n"
+            "t = torch.zeros(3, 4)\nprint(module.flatten([t])[0].shape == (12,), module.invoke(8, 8, ('text',)))\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == ["True", "None"], r.stderr[-2000:]
+    needed = subprocess.run(["readelf", "-d", out], capture_output=True, text=True).stdout
+    assert "libc10.so" in needed and "cuda" not in needed.replace("torch_cuda", "")
