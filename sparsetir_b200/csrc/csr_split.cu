@@ -164,52 +164,65 @@ csr_split_kernel(const SplitArgs s) {
           avn = __ldg(s.a + p0 + s0 + LPR + lane);
         }
         const int cnt = max(0, min(LPR, count - s0));
-        // Most batches of a matrix of long rows lie inside one row for every sub-warp of the warp.
-        unsigned ends = 0, any_ends = 0;
-        int to = 0;
-        if (!__all_sync(0xffffffffu, lane != 0 || (cnt == LPR && wend - (p0 + s0) > LPR))) {
+        auto rows_of_b = [&](int k0, V (&x)[U][VPL]) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) {  // entries past the end have column 0 and are not added
+            const unsigned col = static_cast<unsigned>(__shfl_sync(0xffffffffu, cid, k0 + u, LPR));
+            const char* src = bl + static_cast<unsigned long long>(col) * row_bytes;
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) x[u][v] = LV::ldg(src + at[v]);
+          }
+        };
+        // Most batches of a matrix of long rows lie inside one row for every sub-warp of the warp: a loop of
+        // their own without tests per entry (10 M entries in rows of 500 on average, F = 128: 322 -> 277 us).
+        if (__all_sync(0xffffffffu, lane != 0 || (cnt == LPR && wend - (p0 + s0) > LPR))) {
+          pending = true;
+#pragma unroll
+          for (int k0 = 0; k0 < LPR; k0 += U) {
+            V x[U][VPL];
+            rows_of_b(k0, x);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
+            }
+          }
+        } else {
           const int e = p0 + min(s0 + lane, count - 1);  // lanes past the last entry repeat it
           int row_end;
           const int row = row_in_window<LPR>(s.indptr, s.m, r, wend, e, row_end);
-          ends = group_ballot<LPR>(0xffffffffu, lane < cnt && row_end == e + 1);
-          any_ends = NW == 1 ? ends : __reduce_or_sync(0xffffffffu, ends);
+          const unsigned ends = group_ballot<LPR>(0xffffffffu, lane < cnt && row_end == e + 1);
+          const unsigned any_ends = NW == 1 ? ends : __reduce_or_sync(0xffffffffu, ends);
           r = __shfl_sync(0xffffffffu, row, LPR - 1, LPR);
           if (cnt > 0) pending = ((ends >> (cnt - 1)) & 1u) == 0u;
           if (!pending && cnt > 0) r = min(r + 1, s.m - 1);
           // where the sum up to this entry goes if a row ends here; -1: the lead piece
-          to = lead && (ends & ((1u << lane) - 1u)) == 0u ? -1 : row;
+          const int to = lead && (ends & ((1u << lane) - 1u)) == 0u ? -1 : row;
           if (ends != 0u) lead = false;
           wend = row_window<LPR>(s.indptr, s.m, r, lane);
-        } else {
-          pending = true;
-        }
 #pragma unroll
-        for (int k0 = 0; k0 < LPR; k0 += U) {
-          if (k0 < steps - s0) {
-            V x[U][VPL];
+          for (int k0 = 0; k0 < LPR; k0 += U) {
+            if (k0 < steps - s0) {
+              V x[U][VPL];
+              rows_of_b(k0, x);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {  // entries past the end have column 0 and are not added
-              const unsigned col = static_cast<unsigned>(__shfl_sync(0xffffffffu, cid, k0 + u, LPR));
-              const char* src = bl + static_cast<unsigned long long>(col) * row_bytes;
+              for (int u = 0; u < U; ++u) {
+                const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
+                if (k0 + u < cnt) {
 #pragma unroll
-              for (int v = 0; v < VPL; ++v) x[u][v] = LV::ldg(src + at[v]);
-            }
+                  for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
+                }
+                if ((any_ends >> (k0 + u)) & 1u) {  // a row ends here in some sub-warp of the warp
+                  const int rk = __shfl_sync(0xffffffffu, to, k0 + u, LPR);
+                  const bool end = (ends >> (k0 + u)) & 1u;
+                  // one store instruction for both destinations: no branch among the sub-warps
+                  char* dst = rk < 0 ? reinterpret_cast<char*>(&s_lead[sub][0]) - tile * (TILE * 4) : c_row(rk);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
-              if (k0 + u < cnt) {
-#pragma unroll
-                for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
-              }
-              if ((any_ends >> (k0 + u)) & 1u) {  // a row ends here in some sub-warp of the warp
-                const int rk = __shfl_sync(0xffffffffu, to, k0 + u, LPR);
-                const bool end = (ends >> (k0 + u)) & 1u;
-                // one store instruction for both destinations: no branch among the sub-warps
-                char* dst = rk < 0 ? reinterpret_cast<char*>(&s_lead[sub][0]) - tile * (TILE * 4) : c_row(rk);
-#pragma unroll
-                for (int v = 0; v < VPL; ++v) {
-                  if (end && inside[v]) LV::st(dst + at[v], acc[v]);
-                  LV::zero_if(acc[v], end);
+                  for (int v = 0; v < VPL; ++v) {
+                    if (end && inside[v]) LV::st(dst + at[v], acc[v]);
+                    LV::zero_if(acc[v], end);
+                  }
                 }
               }
             }
