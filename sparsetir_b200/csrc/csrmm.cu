@@ -7,6 +7,7 @@
 // aggregation launch of RGMS), take the row-wise kernel below: row pointer -> ids -> rows of B is
 // the shortest chain of memory round trips there is.  All others take the kernel that splits the
 // matrix by stored entries (csr_split.cu).
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.h"
@@ -28,16 +29,100 @@ constexpr int kThreads = 256;
 // dense rows are gathered 8 at a time.  One writer per output row, CSR summation order, rows
 // without entries written as zeros.
 //
-// HUBS: a row of more than kLongRow entries, which one sub-warp would walk alone (a 2,000-entry row
-// of an 8,000-row graph: 100 us beside 5 us for all the others), is left to the end of the block
-// and then shared by all its sub-warps; their partial sums are added in order.
+// HUBS: a row of more than `long_row` entries, which one sub-warp would walk alone (a 2,000-entry row
+// of an 8,000-row graph: 100 us beside 5 us for all the others), is left to the end of its block
+// and then shared by all sub-warps; their partial sums are added in order.  long_row is 64, or four
+// times the average row where that is more: rows that are all about as long are spread over the sub-warps
+// as they are (1,000 rows of 60 entries, F = 64: 13 us, taken one after the other by the block 18).  Blocks
+// without long rows pay for one barrier behind the row pointers; what the others need inline, or the barrier
+// at the end, cost up to a tenth (8,191 rows of 3 entries, F = 512: 16.4 against 18.0 us).
 constexpr int kLongRow = 64;
+
+// acc += the entries [p0, p1) of a row, taken LPR at a time, `stride` apart
+template <int LPR, int W>
+__device__ __forceinline__ void add_entries(const float* __restrict__ a, const int32_t* __restrict__ indices,
+                                            const char* __restrict__ bl, unsigned row_bytes, int p0, int p1, int stride,
+                                            int lane, unsigned mask, typename LaneVec<W>::type& acc) {
+  using LV = LaneVec<W>;
+  constexpr int U = (32 / W) < LPR ? (32 / W) : LPR;
+  for (int e0 = p0; e0 < p1; e0 += stride) {
+    const bool live = lane < p1 - e0;
+    const int cid = live ? __ldg(indices + e0 + lane) : 0;
+    const float av = live ? __ldg(a + e0 + lane) : 0.f;
+    const int cnt = min(LPR, p1 - e0);
+#pragma unroll
+    for (int k0 = 0; k0 < LPR; k0 += U) {
+      if (k0 < cnt) {
+        typename LV::type x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned col = static_cast<unsigned>(__shfl_sync(mask, cid, k0 + u, LPR));
+          x[u] = LV::ldg(bl + static_cast<unsigned long long>(col) * row_bytes);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const float ak = __shfl_sync(mask, av, k0 + u, LPR);
+          if (k0 + u < cnt) LV::fma(acc, ak, x[u]);
+        }
+      }
+    }
+  }
+}
+
+// All of a block whose items hold long rows: the other rows one after the other by their sub-warps, then
+// the long ones by all sub-warps.  It starts from the kernel's arguments: nothing is kept for it elsewhere.
+template <int LPR, int W>
+__device__ __noinline__ void block_with_long_rows(const float* a, const float* b, float* c, const int32_t* indptr,
+                                                  const int32_t* indices, int m, int feat, int rpi, int long_row) {
+  using LV = LaneVec<W>;
+  constexpr int SUBS = kThreads / LPR;
+  __shared__ unsigned s_long[SUBS];  // the long rows of every sub-warp's item, a bit each
+  __shared__ __align__(32) float s_part[SUBS][LPR * W];
+  const int lane = threadIdx.x % LPR, sub = threadIdx.x / LPR;
+  const unsigned mask = group_mask<LPR>();
+  const long long item0 = static_cast<long long>(blockIdx.x) * SUBS;
+  const int r0 = static_cast<int>(min((item0 + sub) * rpi, static_cast<long long>(m)));
+  const int nr = min(rpi, m - r0);
+  const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
+  const unsigned off = (blockIdx.y * LPR + lane) * (W * 4u);
+  const char* bl = reinterpret_cast<const char*>(b) + off;
+  char* cl = reinterpret_cast<char*>(c) + off;
+  auto c_row = [&](int r) -> char* { return cl + static_cast<unsigned long long>(static_cast<unsigned>(r)) * row_bytes; };
+  unsigned long_rows = 0;
+  for (int j = 0; j < nr; ++j) {
+    const int begin = __ldg(indptr + r0 + j), end = __ldg(indptr + r0 + j + 1);
+    if (end - begin > long_row) {
+      long_rows |= 1u << j;
+      continue;
+    }
+    typename LV::type acc = LV::zero();
+    add_entries<LPR, W>(a, indices, bl, row_bytes, begin, end, LPR, lane, mask, acc);
+    LV::stcs(c_row(r0 + j), acc);
+  }
+  if (lane == 0) s_long[sub] = long_rows;
+  __syncthreads();
+  for (int owner = 0; owner < SUBS; ++owner) {
+    for (unsigned todo = s_long[owner]; todo != 0u; todo &= todo - 1u) {
+      const int row = static_cast<int>((item0 + owner) * rpi) + __ffs(todo) - 1;
+      const int begin = __ldg(indptr + row), end = __ldg(indptr + row + 1);
+      typename LV::type acc = LV::zero();
+      add_entries<LPR, W>(a, indices, bl, row_bytes, begin + sub * LPR, end, SUBS * LPR, lane, mask, acc);
+      LV::sts(&s_part[sub][lane * W], acc);
+      __syncthreads();
+      if (sub == 0) {
+        for (int j = 1; j < SUBS; ++j) LV::add(acc, LV::lds(&s_part[j][lane * W]));
+        LV::stcs(c_row(row), acc);
+      }
+      __syncthreads();
+    }
+  }
+}
 
 template <int LPR, int W, bool HUBS>  // W floats per lane: 4 (16-byte vectors) or 8 (32-byte vectors)
 __global__ void __launch_bounds__(kThreads, 4)
 csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
                   const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int m,
-                  int feat, int rpi) {
+                  int feat, int rpi, int long_row) {
   using LV = LaneVec<W>;
   using V = typename LV::type;
   constexpr int SUBS = kThreads / LPR;
@@ -49,12 +134,6 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   if (!HUBS && r0l >= m) return;
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m)));
   const int nr = min(rpi, m - r0);  // 0 past the last row
-  __shared__ int s_long[HUBS ? SUBS * (LPR - 1) : 1];  // long rows of the block, by (sub-warp, row)
-  __shared__ int s_longs;
-  if (HUBS) {
-    if (threadIdx.x == 0) s_longs = 0;
-    __syncthreads();
-  }
   const int ptr = __ldg(indptr + r0 + min(lane, nr));  // lane j: start of row r0+j (j <= nr)
   const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
   const unsigned off = (blockIdx.y * LPR + lane) * (W * 4u);
@@ -62,43 +141,30 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   char* cl = reinterpret_cast<char*>(c) + off +
              static_cast<unsigned long long>(static_cast<unsigned>(r0)) * row_bytes;
 
-  // An item that contains long rows streams the runs of ordinary rows between them, one run at a
-  // time; an item without them (the usual case) is one run.
-  unsigned long_rows_mask = 0;
   if (HUBS) {
     const int len = __shfl_down_sync(mask, ptr, 1, LPR) - ptr;
-    const bool is_long = lane < nr && len > kLongRow;
-    const int shift = (threadIdx.x & 31) / LPR * LPR;
-    long_rows_mask = __ballot_sync(mask, is_long) >> shift;
-    if (is_long) s_long[atomicAdd(&s_longs, 1)] = r0 + lane;
-  }
-  int jb = 0;
-  while (jb < nr) {
-    int je = nr;
-    if (long_rows_mask != 0) {
-      const unsigned ordinary = ~long_rows_mask & ((nr < 32 ? (1u << nr) : 0u) - 1u) & (~0u << jb);
-      if (ordinary == 0) break;
-      jb = __ffs(ordinary) - 1;
-      const unsigned longer = long_rows_mask & (~0u << jb);
-      je = longer != 0 ? __ffs(longer) - 1 : nr;
+    if (__syncthreads_or(lane < nr && len > long_row)) {
+      block_with_long_rows<LPR, W>(a, b, c, indptr, indices, m, feat, rpi, long_row);
+      return;
     }
-    // ---- rows [jb, je) of the item: one contiguous slot stream
-    const int p0s = __shfl_sync(mask, ptr, jb, LPR);
-    const int nslots_s = __shfl_sync(mask, ptr, je, LPR) - p0s;
-    char* cls = cl + static_cast<unsigned>(jb) * row_bytes;
+  }
+  if (nr > 0) {
+    // ---- the rows of the item: one contiguous slot stream
+    const int p0s = __shfl_sync(mask, ptr, 0, LPR);
+    const int nslots_s = __shfl_sync(mask, ptr, nr, LPR) - p0s;
     const int32_t* cols_s = indices + p0s;
     const float* wts_s = a + p0s;
     V acc = LV::zero();
-    int j = jb;                                             // row being accumulated
-    int row_end = __shfl_sync(mask, ptr, jb + 1, LPR) - p0s;  // its end, as a slot number
+    int j = 0;                                             // row being accumulated
+    int row_end = __shfl_sync(mask, ptr, 1, LPR) - p0s;  // its end, as a slot number
     int s = 0;                                              // slots consumed so far
     auto finish_rows = [&]() {  // store every row whose last entry has been consumed
-      while (j < je && s >= row_end) {
-        LV::stcs(cls, acc);  // written once: keep B rows in L2
+      while (j < nr && s >= row_end) {
+        LV::stcs(cl, acc);  // written once: keep B rows in L2
         acc = LV::zero();
-        cls += row_bytes;
+        cl += row_bytes;
         ++j;
-        row_end = __shfl_sync(mask, ptr, min(j + 1, je), LPR) - p0s;
+        row_end = __shfl_sync(mask, ptr, min(j + 1, nr), LPR) - p0s;
       }
     };
     finish_rows();  // rows without entries at the front
@@ -139,48 +205,6 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
       }
       cid = cidn;
       av = avn;
-    }
-    jb = je;
-  }
-
-  if (HUBS) {
-    __shared__ __align__(32) float s_part[SUBS][LPR * W];
-    __syncthreads();
-    const int longs = s_longs;
-    const int sub = threadIdx.x / LPR;
-    for (int k = 0; k < longs; ++k) {  // which order the rows come in changes nothing
-      const int row = s_long[k];
-      const int begin = __ldg(indptr + row), end = __ldg(indptr + row + 1);
-      V acc = LV::zero();
-      for (int e0 = begin + sub * LPR; e0 < end; e0 += SUBS * LPR) {
-        const bool live = lane < end - e0;
-        const int cid = live ? __ldg(indices + e0 + lane) : 0;
-        const float av = live ? __ldg(a + e0 + lane) : 0.f;
-        const int cnt = min(LPR, end - e0);
-#pragma unroll
-        for (int k0 = 0; k0 < LPR; k0 += U) {
-          if (k0 < cnt) {
-            V x[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const unsigned col = static_cast<unsigned>(__shfl_sync(mask, cid, k0 + u, LPR));
-              x[u] = LV::ldg(bl + static_cast<unsigned long long>(col) * row_bytes);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const float ak = __shfl_sync(mask, av, k0 + u, LPR);
-              if (k0 + u < cnt) LV::fma(acc, ak, x[u]);
-            }
-          }
-        }
-      }
-      LV::sts(&s_part[sub][lane * W], acc);
-      __syncthreads();
-      if (sub == 0) {
-        for (int j = 1; j < SUBS; ++j) LV::add(acc, LV::lds(&s_part[j][lane * W]));
-        LV::stcs(reinterpret_cast<char*>(c) + off + static_cast<unsigned long long>(static_cast<unsigned>(row)) * row_bytes, acc);
-      }
-      __syncthreads();
     }
   }
 }
@@ -251,12 +275,13 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     rpi = rpi < 1 ? 1 : (rpi > lanes - 1 ? lanes - 1 : rpi);
     const long long want_items = 4ll * kNumSMs * 4 * subs;
     while (rpi > 1 && (m + rpi - 1) / rpi < want_items) rpi /= 2;
+    const int long_row = std::max(kLongRow, static_cast<int>(4.0 * avg));
     dim3 grid(ceil_div(ceil_div(m, rpi), subs), feat / (w * lanes));
 #define SPTIR_CSR_LEAN(L, WW)                                                                                   \
   if (hub_rows)                                                                                                 \
-    csrmm_lean_kernel<L, WW, true><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi);           \
+    csrmm_lean_kernel<L, WW, true><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi, long_row); \
   else                                                                                                          \
-    csrmm_lean_kernel<L, WW, false><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi)
+    csrmm_lean_kernel<L, WW, false><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi, 0)
     if (w == 8) {
       if (lanes == 4) { SPTIR_CSR_LEAN(4, 8); }
       else if (lanes == 8) { SPTIR_CSR_LEAN(8, 8); }

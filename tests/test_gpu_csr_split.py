@@ -11,6 +11,8 @@ pytestmark = pytest.mark.gpu
 # degree sequences; all but the first have 8,192 rows or 65,536 entries, where the split begins
 SHAPES = {
     "hubs_in_a_small_matrix": [0, 3, 1500, 65, 64, 0, 2, 900] + [5] * 700 + [700],
+    # four times the average row is 169: rows up to that stay with their sub-warp
+    "hubs_among_long_rows": [40] * 300 + [0, 165, 169, 170, 900, 171] + [40] * 300 + [170],
     "one_row_of_everything": [0] * 40 + [70_001] + [0] * 9000,
     "rows_longer_than_a_block": [9000, 1, 0, 17_000, 2] * 4,
     "empty_runs": ([0] * 5000 + [1] * 40) * 5 + [0] * 3000,
