@@ -53,12 +53,17 @@ __device__ __forceinline__ unsigned group_ballot(unsigned mask, bool pred) {
   }
 }
 
+// Resident blocks.  The widest pieces per lane spill at 64 registers: three blocks of 80 hold them (50 k-node
+// power-law graph, F = 299: 80 against 77.6 us; 100 k nodes, F = 222: 76 against 70; 30 k rows of 38 entries,
+// F = 151: 104 against 99; two single floats per lane: F = 41, 49 against 53).
+__host__ __device__ constexpr int blocks_per_sm(int w, int vpl) { return vpl > 1 && vpl * w > 2 ? 3 : 4; }
+
 // A lane owns VPL vectors of W floats of the feature tile (VPL * LPR * W floats), LPR * W apart: one
 // 16-byte vector where rows allow it, several 4- or 8-byte ones where their length or alignment
 // does not (odd feature counts: tiles of up to 160 floats instead of 32, so that ids are read that
 // much less often: 30 k rows, F = 299, 104 us with one vector, 66 with four, 59 with five).
 template <int LPR, int W, int VPL>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, blocks_per_sm(W, VPL))
 csr_split_kernel(const SplitArgs s) {
   using LV = LaneVec<W>;
   using V = typename LV::type;
@@ -365,7 +370,7 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
   // A block walks the feature tiles one after the other, all blocks roughly in step, which keeps
   // the slice of B that they gather from in L2; matrices too small to give every resident block
   // a batch of entries deal the tiles to more blocks (60 k entries, F = 512: 25 against 37 us).
-  const long long resident = 4ll * kNumSMs, batch = static_cast<long long>(subs) * sh.lanes;
+  const long long resident = static_cast<long long>(blocks_per_sm(sh.w, sh.vpl)) * kNumSMs, batch = static_cast<long long>(subs) * sh.lanes;
   const long long fewest = (nnz + batch - 1) / batch;
   SplitPlan p;
   p.gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident / fewest)));
