@@ -6,7 +6,7 @@
 // kernel with two more launches for the rows of more than 32 entries (169 k-node power-law graph,
 // F = 32 / 512: 71 / 357 us against 25 / 220 us) and a row-wise kernel for the feature counts
 // that are not whole tiles, where one sub-warp walked a hub row alone (100 k-node power-law
-// graph, F = 100: 2302 us against 28 us).
+// graph, F = 100: 2302 us against 33.5 us).
 //
 // Rows are found without a plan: a 32-ary search of `indptr` for the first entry of a sub-warp,
 // then a register window of row ends (row_walk.cuh).  Every output row has one writer and one

@@ -30,7 +30,7 @@
 
 namespace sptir {
 
-// defined in csrmm.cu: the CSR SpMM launcher with 32-byte lanes, never the hub-row launches
+// defined in csrmm.cu: the row-wise CSR SpMM, which needs no scratch, with 32-byte lanes on large matrices
 int csrmm_short_rows_impl(const float* a, const float* b, float* c, const int32_t* indptr,
                           const int32_t* indices, int m, int n, int feat, int nnz, int device_id,
                           void* stream);
