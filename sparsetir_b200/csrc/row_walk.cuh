@@ -19,9 +19,28 @@ __device__ __forceinline__ int edge_row_search(const int32_t* __restrict__ indpt
   return low - 1;
 }
 
+// First index of [lo, hi) whose pointer lies behind p, or hi, found by a whole warp: 32-ary steps, every
+// level is one load per lane (4 dependent reads instead of 18 at 2^18 rows).  Reads stay in [lo, hi).
+__device__ __forceinline__ int warp_upper_bound(const int32_t* __restrict__ indptr, int lo, int hi, int p, int wlane) {
+  while (hi - lo >= 32) {
+    const int step = (hi - lo + 31) / 32;
+    const long long probe = static_cast<long long>(lo) + static_cast<long long>(wlane + 1) * step;
+    const bool in = probe < hi;
+    const bool gt = !in || __ldg(indptr + (in ? probe : 0)) > p;
+    const int first = __ffs(__ballot_sync(0xffffffffu, gt)) - 1;  // lane 31 probes >= hi: always set
+    const int q = lo + (first + 1) * step;
+    if (first > 0) lo = q - step + 1;
+    hi = min(hi, q);
+  }
+  const int idx = lo + wlane;
+  const bool in = idx < hi;
+  const bool gt = !in || __ldg(indptr + (in ? idx : 0)) > p;  // lane hi - lo (< 32) has idx == hi
+  return lo + __ffs(__ballot_sync(0xffffffffu, gt)) - 1;
+}
+
 // Row of position p, clamped into [0, m - 1], found by a whole warp: 32 probes around a first
 // guess (position x rows / entries), at distances that double, then 32-ary steps inside the
-// bracket — every level is one load per lane.  Two or three memory round trips where the rows are
+// bracket.  Two or three memory round trips where the rows are
 // roughly equally long in the large, four or five for any other matrix of 2^18 rows (a binary
 // search: 18).  Every read stays inside indptr whatever p says.
 __device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ indptr, int m, int p,
@@ -40,20 +59,7 @@ __device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ indptr, i
     if (first < 32) hi = above;
     if (first > 0) lo = below + 1;
   }
-  while (hi - lo >= 32) {
-    const int step = (hi - lo + 31) / 32;
-    const long long probe = static_cast<long long>(lo) + static_cast<long long>(wlane + 1) * step;
-    const bool in = probe < hi;
-    const bool gt = !in || __ldg(indptr + (in ? probe : 0)) > p;
-    const int first = __ffs(__ballot_sync(0xffffffffu, gt)) - 1;  // lane 31 probes >= hi: always set
-    const int q = lo + (first + 1) * step;
-    if (first > 0) lo = q - step + 1;
-    hi = min(hi, q);
-  }
-  const int idx = lo + wlane;
-  const bool in = idx < hi;
-  const bool gt = !in || __ldg(indptr + (in ? idx : 0)) > p;  // lane hi - lo (< 32) has idx == hi
-  return max(0, min(m - 1, lo + __ffs(__ballot_sync(0xffffffffu, gt)) - 2));
+  return max(0, min(m - 1, warp_upper_bound(indptr, lo, hi, p, wlane) - 1));
 }
 
 // Rows of N ascending positions, found by a whole warp: the first by the search, the others by

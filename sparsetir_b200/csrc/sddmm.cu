@@ -132,27 +132,10 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
 // adding to it, and picks the tile so that the slice of B a launch gathers from stays in L2.
 // A lane owns 8 consecutive features: one 256-bit load per gathered row, the dot product as
 // packed two-wide fp32 FMAs.  A warp owns `chunk` consecutive positions, finds the row of its
-// first position with a 32-ary search done by the whole warp (4 dependent reads instead of 18
-// at 2^18 rows), and loads the column ids of the next batch before it gathers for this one.
-// first index idx in [0, m+1] with idx == m+1 or indptr[idx] > p, found by the whole warp;
-// row(p) is that index minus one (the search of sparse_tir_lowered_buffer_scripts.py:530-549)
-__device__ __forceinline__ int warp_row_search(const int32_t* __restrict__ indptr, int m, int p,
-                                               int wlane) {
-  int lo = 0, hi = m + 1;
-  while (hi - lo >= 32) {
-    const int step = (hi - lo + 31) / 32;
-    const long long probe = static_cast<long long>(lo) + static_cast<long long>(wlane + 1) * step;
-    const bool gt = probe >= hi || __ldg(indptr + probe) > p;
-    const int first = __ffs(__ballot_sync(0xffffffffu, gt)) - 1;  // lane 31 probes >= hi: always set
-    const int q = lo + (first + 1) * step;
-    if (first > 0) lo = q - step + 1;
-    hi = min(hi, q);
-  }
-  const int idx = lo + wlane;
-  const bool gt = idx >= hi || __ldg(indptr + idx) > p;  // lane hi - lo (< 32) has idx == hi
-  return lo + __ffs(__ballot_sync(0xffffffffu, gt)) - 1;
-}
-
+// first position together (row(p) = upper bound - 1, the search of
+// sparse_tir_lowered_buffer_scripts.py:530-549), and loads the column ids of the next batch before it
+// gathers for this one.  It asks for a row of A when it meets one: for matrices of 10 entries per row and
+// more (sddmm_run).
 // With PEERS the finished value of every position (the last feature tile's pass) is also stored
 // into the peers' copies of c: 128 contiguous bytes per warp and peer, over NVLink.
 template <int LPR, bool PEERS>
@@ -172,7 +155,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const float* a_lane = a + foff + lane * 8;
   const float* b_lane = b + foff + lane * 8;
 
-  int warp_row = max(0, min(m - 1, warp_row_search(indptr, m, static_cast<int>(e_begin), wlane) - 1));
+  int warp_row = max(0, min(m - 1, warp_upper_bound(indptr, 0, m + 1, static_cast<int>(e_begin), wlane) - 1));
   int warp_end = __ldg(indptr + warp_row + 1);  // first position past the warp's current row
   int cur_row = -1;
   Pack4 arow = pack4_zero();
