@@ -4,7 +4,7 @@
 // each), so a hub row of thousands of entries is spread over many sub-warps and a run of short
 // rows costs what its entries cost: one launch, whatever the row lengths.  It replaces a row-wise
 // kernel with two more launches for the rows of more than 32 entries (169 k-node power-law graph,
-// F = 32 / 512: 71 / 357 us against 25 / 220 us) and a row-wise kernel for the feature counts
+// F = 32 / 512: 74 / 358 us against 26.6 / 229 us) and a row-wise kernel for the feature counts
 // that are not whole tiles, where one sub-warp walked a hub row alone (100 k-node power-law
 // graph, F = 100: 2302 us against 33.5 us).
 //
