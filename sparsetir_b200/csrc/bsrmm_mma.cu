@@ -13,6 +13,7 @@
 #include <cuda_fp16.h>
 
 #include "common.h"
+#include "launch.cuh"
 #include "mma16.cuh"
 #include "vec.cuh"
 
@@ -31,6 +32,7 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
   const int slab = static_cast<int>(blockIdx.x) % slabs, rest = static_cast<int>(blockIdx.x) / slabs;
   const int part = rest % parts, i = rest / parts;
   const int f0 = slab * mma16::kSlab, row0 = part * 16 * MT;
+  chain_enter();
   const int p0 = __ldg(indptr + i), p1 = __ldg(indptr + i + 1);
   const int per_blk = blk >> 4;  // groups per stored block
   const long long total = static_cast<long long>(p1 - p0) * per_blk;
@@ -125,9 +127,9 @@ int bsrmm_mma_launch(const __half* a, const __half* b, float* c, const int32_t* 
   if (blocks > INT32_MAX) return 1;
   const int vec_out = aligned16(c) ? 1 : 0;
   if (mt == 2)
-    bsrmm_mma_kernel<2><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(a, b, c, indptr, indices, blk, feat, slabs, parts, vec_out);
+    launch_chained(bsrmm_mma_kernel<2>, static_cast<unsigned>(blocks), kThreads, 0, st, a, b, c, indptr, indices, blk, feat, slabs, parts, vec_out);
   else
-    bsrmm_mma_kernel<1><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(a, b, c, indptr, indices, blk, feat, slabs, parts, vec_out);
+    launch_chained(bsrmm_mma_kernel<1>, static_cast<unsigned>(blocks), kThreads, 0, st, a, b, c, indptr, indices, blk, feat, slabs, parts, vec_out);
   SPTIR_LAUNCH_OK("bsrmm_mma_kernel");
   return 0;
 }

@@ -29,6 +29,7 @@
 #include <cstring>
 
 #include "common.h"
+#include "launch.cuh"
 #include "tc05.cuh"
 #include "tmap.h"
 #include "vec.cuh"
@@ -212,6 +213,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const int i = blockIdx.x;
   const int f0 = blockIdx.y * kTileF;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  chain_enter();
   const int p0 = __ldg(indptr + i), nblk = __ldg(indptr + i + 1) - p0;
 
   float* crow = c + (static_cast<size_t>(i) * kBlk) * feat + f0 + warp * 32 + lane;
@@ -358,6 +360,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     tc05::prefetch_tensormap(&tm_b);
   }
   if (warp == 0) tc05::tmem_alloc(&s_tmem, 2 * kPAccCols);
+  chain_enter();
   tc05::fence_before_sync();
   __syncthreads();
   tc05::fence_after_sync();
@@ -504,8 +507,8 @@ int bsrmm_persist_launch(const __half* a, const __half* b, float* c, const int32
   const long long items = static_cast<long long>(nb) * items_per_row;
   if (items > INT32_MAX) return 1;
   const int grid = static_cast<int>(items < 2 * kNumSMs ? items : 2 * kNumSMs);  // two blocks per SM (shared memory)
-  bsrmm_persist_kernel<<<grid, kPThreads, kPSmem, stream>>>(tm_a, tm_b, c, indptr, indices, feat,
-                                                            static_cast<int>(items), items_per_row);
+  launch_chained(bsrmm_persist_kernel, grid, kPThreads, kPSmem, stream, tm_a, tm_b, c, indptr, indices, feat,
+                 static_cast<int>(items), items_per_row);
   SPTIR_LAUNCH_OK("bsrmm_persist_kernel");
   return 0;
 }
@@ -531,7 +534,7 @@ int bsrmm_tma_launch(const __half* a, const __half* b, float* c, const int32_t* 
     configured_device = dev;
   }
   dim3 grid(nb, feat / kTileF);
-  bsrmm_tma_kernel<<<grid, kThreads, kTmaSmem, stream>>>(tm_a, tm_b, c, indptr, indices, feat);
+  launch_chained(bsrmm_tma_kernel, grid, kThreads, kTmaSmem, stream, tm_a, tm_b, c, indptr, indices, feat);
   SPTIR_LAUNCH_OK("bsrmm_tma_kernel");
   return 0;
 }

@@ -9,6 +9,7 @@
 #include <cfloat>
 
 #include "common.h"
+#include "launch.cuh"
 #include "vec.cuh"
 
 namespace sptir {
@@ -54,6 +55,7 @@ sparse_softmax_kernel(const float* __restrict__ a, float* __restrict__ b,
   const int lane = threadIdx.x % LPR;
   const unsigned mask = group_mask<LPR>();
   const long long row = static_cast<long long>(blockIdx.x) * (kThreads / LPR) + threadIdx.x / LPR;
+  chain_enter();
   if (row >= n) return;
   const int p0 = __ldg(indptr + row), p1 = __ldg(indptr + row + 1);
   float v[CACHE];
@@ -176,9 +178,9 @@ extern "C" int sparsetir_sparse_softmax_raw(const float* a, float* b, const int3
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (validate_enabled() && validate_indptr("sparsetir_sparse_softmax", "indptr", indptr, n, nnz, st) != 0) return -1;
   if (static_cast<double>(nnz) / n >= 24.0) {
-    sparse_softmax_kernel<32, 16><<<ceil_div(n, kThreads / 32), kThreads, 0, st>>>(a, b, indptr, n);
+    launch_chained_if(nnz < kChainEntries, sparse_softmax_kernel<32, 16>, ceil_div(n, kThreads / 32), kThreads, 0, st, a, b, indptr, n);
   } else {
-    sparse_softmax_kernel<4, 4><<<ceil_div(n, kThreads / 4), kThreads, 0, st>>>(a, b, indptr, n);
+    launch_chained_if(nnz < kChainEntries, sparse_softmax_kernel<4, 4>, ceil_div(n, kThreads / 4), kThreads, 0, st, a, b, indptr, n);
   }
   SPTIR_LAUNCH_OK("sparse_softmax_kernel");
   return 0;

@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "row_walk.cuh"
 
 namespace sptir {
@@ -85,6 +86,7 @@ csr_split_kernel(const SplitArgs s) {
   const long long block_entries = static_cast<long long>(SUBS) * s.span;
   const unsigned row_bytes = static_cast<unsigned>(s.feat) * 4u;
   const long long warp_at = blockIdx.x * block_entries + static_cast<long long>((threadIdx.x / 32) * NW) * s.span;
+  chain_enter();
   // The stored entries are those between the first and the last row pointer: of a slice of a larger
   // matrix, or of arrays with room behind, not all nnz.  The two pointers are not waited for: ids and
   // row of the first entry are requested as if they were 0 and nnz, and once more where they are not.
@@ -386,7 +388,7 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
 
 template <int LPR, int W, int VPL>
 int launch_split(const SplitArgs& s, const SplitPlan& p, cudaStream_t st) {
-  csr_split_kernel<LPR, W, VPL><<<dim3(p.blocks, p.gy), kThreads, 0, st>>>(s);
+  launch_chained_if(s.nnz < kChainEntries, csr_split_kernel<LPR, W, VPL>, dim3(p.blocks, p.gy), kThreads, 0, st, s);
   SPTIR_LAUNCH_OK("csr_split_kernel");
   return 0;
 }

@@ -11,6 +11,7 @@
 #include <cstdlib>
 
 #include "common.h"
+#include "launch.cuh"
 #include "vec.cuh"
 
 namespace sptir {
@@ -131,6 +132,7 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const unsigned mask = group_mask<LPR>();
   const long long item = static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR;
   const long long r0l = item * rpi;
+  chain_enter();
   if (!HUBS && r0l >= m) return;
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m)));
   const int nr = min(rpi, m - r0);  // 0 past the last row
@@ -279,9 +281,9 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     dim3 grid(ceil_div(ceil_div(m, rpi), subs), feat / (w * lanes));
 #define SPTIR_CSR_LEAN(L, WW)                                                                                   \
   if (hub_rows)                                                                                                 \
-    csrmm_lean_kernel<L, WW, true><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi, long_row); \
+    launch_chained(csrmm_lean_kernel<L, WW, true>, grid, kThreads, 0, st, a, b, c, indptr, indices, m, feat, rpi, long_row); \
   else                                                                                                          \
-    csrmm_lean_kernel<L, WW, false><<<grid, kThreads, 0, st>>>(a, b, c, indptr, indices, m, feat, rpi, 0)
+    launch_chained(csrmm_lean_kernel<L, WW, false>, grid, kThreads, 0, st, a, b, c, indptr, indices, m, feat, rpi, 0)
     if (w == 8) {
       if (lanes == 4) { SPTIR_CSR_LEAN(4, 8); }
       else if (lanes == 8) { SPTIR_CSR_LEAN(8, 8); }

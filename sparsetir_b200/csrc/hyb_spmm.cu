@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "common.h"
+#include "launch.cuh"
 #include "spmm_core.cuh"
 
 namespace sptir {
@@ -506,6 +507,7 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   auto y_of = [&](int rid) -> char* {
     return cl + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * stride;
   };
+  chain_enter();
 
   if (spr == 1) {
     // ---- narrow bucket: a sub-warp owns rpi whole ELL rows
@@ -821,11 +823,11 @@ int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
   dim3 grid(static_cast<unsigned>(blocks), tiles);
   if (la.peers.n > 0) {
     if constexpr (W == 4 && WHOLE)
-      hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true><<<grid, kThreads, 0, stream>>>(tb, la);
+      launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true>, grid, kThreads, 0, stream, tb, la);
     else
       return fail("sparsetir_hyb_spmm_peers: whole tiles of 16-byte lanes only");  // the dispatcher picks them
   } else {
-    hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, false><<<grid, kThreads, 0, stream>>>(tb, la);
+    launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, false>, grid, kThreads, 0, stream, tb, la);
   }
   SPTIR_LAUNCH_OK("hyb_spmm_lean_kernel");
   return 0;

@@ -32,6 +32,7 @@
 #include <cstring>
 
 #include "common.h"
+#include "launch.cuh"
 #include "rgms_common.cuh"
 #include "tc05.cuh"
 #include "tmap.h"
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(kThreads)
 gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
                         const __half* __restrict__ x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
                         int32_t* __restrict__ ranges, int num_rels, int chunks) {
+  chain_enter();
   if (blockIdx.x == gridDim.x - 1) {
     write_ranges(tb, num_rels, ranges);
     return;
@@ -413,6 +415,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
                    const __half* __restrict__ gvals, const int32_t* __restrict__ run_if_set) {
   // run_if_set != nullptr: this launch is the fall-back of the reduction-free form and runs only
   // when that form found the input unsuitable (flag set on the device)
+  if (GATHER) chain_enter();
   if (run_if_set != nullptr && __ldg(run_if_set) == -1) return;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kStagesH];   // the stage's boxes have landed
@@ -426,10 +429,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
   const int nkc = (feat_in + kKC - 1) / kKC, nwb = (feat_out + 63) / 64;
 
   if (warp == 0) {
-    int rel, row0, row1;
-    const bool found = locate_tile_warp(ranges, num_ranges, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
     if (lane == 0) {
-      s_tile[0] = found ? 1 : 0; s_tile[1] = rel; s_tile[2] = row0; s_tile[3] = row1;
       for (int s = 0; s < kStagesH; ++s) {
         tc05::mbar_init(&bar_full[s], GATHER ? 1 + 128 : 1);  // the W boxes (+ the 128 gathering threads)
         tc05::mbar_init(&bar_empty[s], 1);
@@ -444,6 +444,14 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     }
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, tmem_cols);
+  }
+  if (!GATHER) chain_enter();
+  if (warp == 0) {
+    int rel, row0, row1;
+    const bool found = locate_tile_warp(ranges, num_ranges, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
+    if (lane == 0) {
+      s_tile[0] = found ? 1 : 0; s_tile[1] = rel; s_tile[2] = row0; s_tile[3] = row1;
+    }
   }
   tc05::fence_before_sync();
   __syncthreads();
@@ -895,9 +903,9 @@ int launch_tc(const __half* z, const __half* w, OutT* y, const int32_t* ranges, 
   const long long tiles = static_cast<long long>(total_rows) / kTM + num_ranges;  // upper bound
   const long long grid = tiles < kNumSMs ? tiles : kNumSMs;
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
-  rgms_f16_tc_kernel<OutT, GATHER><<<static_cast<unsigned>(grid), GATHER ? kTcThreadsG : kTcThreads, kSmemH, st>>>(
-      tm_z, tm_w, y, ranges, all_rows, num_ranges, num_rels, total_rows, tiles_per_cta, feat_in, feat_out,
-      tmem_cols, x, gcols, gvals, run_if_set);
+  launch_chained(rgms_f16_tc_kernel<OutT, GATHER>, static_cast<unsigned>(grid), GATHER ? kTcThreadsG : kTcThreads, kSmemH, st,
+                 tm_z, tm_w, y, ranges, all_rows, num_ranges, num_rels, total_rows, tiles_per_cta, feat_in, feat_out,
+                 tmem_cols, x, gcols, gvals, run_if_set);
   SPTIR_LAUNCH_OK("rgms_f16_tc_kernel");
   return 0;
 }
@@ -1016,8 +1024,8 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
       gt.first[b] = static_cast<int32_t>(tiles);
       tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
     }
-    gather_tiles_f16_kernel<<<static_cast<unsigned>(tiles + 1), kThreads, 0, st>>>(tb, gt, x, z, all_rows, ranges,
-                                                                                  num_rels, feat_in / 8);
+    launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(tiles + 1), kThreads, 0, st, tb, gt, x, z, all_rows, ranges,
+                   num_rels, feat_in / 8);
   } else if (vec)
     gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
   else

@@ -17,6 +17,7 @@
 // The one mbarrier wait (tensor core done) is bounded; a timeout is counted and the block gives
 // up cleanly.
 #include "common.h"
+#include "launch.cuh"
 #include "rgms_common.cuh"
 #include "spmm_core.cuh"
 #include <cstdlib>
@@ -278,10 +279,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
   unsigned char* base = smem_raw + ((1024u - (tc05::smem_u32(smem_raw) & 1023u)) & 1023u);
 
   if (warp == 0) {
-    int rel, row0, row1;
-    const bool found = locate_tile_warp(indptr_i, num_rels, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
     if (lane == 0) {
-      s_tile[0] = found ? 1 : 0; s_tile[1] = rel; s_tile[2] = row0; s_tile[3] = row1;
       for (int s = 0; s < kZStages; ++s) {
         tc05::mbar_init(&bar_full[s], 1);
         tc05::mbar_init(&bar_conv[s], 128);
@@ -296,6 +294,14 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
     }
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, 4 * kF);
+  }
+  chain_enter();
+  if (warp == 0) {
+    int rel, row0, row1;
+    const bool found = locate_tile_warp(indptr_i, num_rels, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
+    if (lane == 0) {
+      s_tile[0] = found ? 1 : 0; s_tile[1] = rel; s_tile[2] = row0; s_tile[3] = row1;
+    }
   }
   tc05::fence_before_sync();
   __syncthreads();
@@ -482,8 +488,8 @@ int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int
   const long long tiles = static_cast<long long>(nnz_i) / kTM + num_rels;  // upper bound
   const long long grid = tiles < kNumSMs ? tiles : kNumSMs;
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
-  rgms_tma_kernel<<<static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream>>>(
-      tm_z, w, y, indptr_i, indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
+  launch_chained(rgms_tma_kernel, static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream, tm_z, w, y, indptr_i, indices_i,
+                 num_rels, nnz_i, tiles_per_cta, rel_mod);
   SPTIR_LAUNCH_OK("rgms_tma_kernel");
   return 0;
 }

@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "rgms_common.cuh"
 
 namespace sptir {
@@ -34,6 +35,7 @@ rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32
   __shared__ __align__(16) float s_w[2][kK][kStride];
   const int tid = threadIdx.x, lane = tid & 31;
   TileWalk tw;
+  chain_enter();
   if (!locate_tile_warp(indptr_i, num_rels, static_cast<int>(blockIdx.x) * tiles_per_block, lane, &tw.rel, &tw.row0,
                         &tw.row1))
     return;  // the same in all warps
@@ -119,8 +121,8 @@ int rgms_wide_launch(const float* w, float* y, const int32_t* indptr_i, const in
   const long long want = std::max(1ll, 2ll * kNumSMs * 4 / ny);  // four runs of tiles per resident block: even ends
   const long long per = (tiles + want - 1) / want;
   const dim3 grid(static_cast<unsigned>((tiles + per - 1) / per), ny);
-  rgms_wide_kernel<<<grid, kThreads, 0, stream>>>(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat,
-                                                  static_cast<int>(per));
+  launch_chained(rgms_wide_kernel, grid, kThreads, 0, stream, w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat,
+                 static_cast<int>(per));
   SPTIR_LAUNCH_OK("rgms_wide_kernel");
   return 0;
 }

@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "row_walk.cuh"
 
 namespace sptir {
@@ -47,6 +48,7 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
   const int sub = wlane / LPR;
   const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
   const long long begin = warp * chunk;
+  chain_enter();
   if (begin >= nnz) return;
   const int e0 = static_cast<int>(begin);
   const int count = static_cast<int>(min(static_cast<long long>(chunk), nnz - begin));
@@ -150,6 +152,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const unsigned mask = group_mask<LPR>();
   const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
   const long long e_begin = warp * chunk;
+  chain_enter();
   if (e_begin >= nnz) return;
   const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + chunk));
   const float* a_lane = a + foff + lane * 8;
@@ -263,14 +266,14 @@ int launch(const float* a, const float* b, float* c, const int32_t* indptr, cons
   const float rows_per_entry = static_cast<float>(m) / static_cast<float>(nnz);
   if constexpr (W == 4) {
     if (po.n > 0) {
-      sddmm_kernel<LPR, W, VPL, true><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, feat, nnz,
-                                                                       chunk, rows_per_entry, po);
+      launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, true>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat,
+                     nnz, chunk, rows_per_entry, po);
       SPTIR_LAUNCH_OK("sddmm_kernel");
       return 0;
     }
   }
-  sddmm_kernel<LPR, W, VPL, false><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, feat, nnz,
-                                                                    chunk, rows_per_entry, po);
+  launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, false>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat, nnz,
+                 chunk, rows_per_entry, po);
   SPTIR_LAUNCH_OK("sddmm_kernel");
   return 0;
 }
@@ -305,11 +308,11 @@ int launch_lean_tile(const float* a, const float* b, float* c, const int32_t* in
   if (waves < 8) chunk = static_cast<int>((nnz + waves * resident - 1) / (waves * resident) + 31) & ~31;
   const int blocks = ceil_div(ceil_div(nnz, chunk), wpb);
   if (po.n > 0)
-    sddmm_lean_kernel<LPR, true><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, nnz, feat,
-                                                                  foff, foff != 0, chunk, last_tile, po);
+    launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, true>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, nnz, feat,
+                   foff, foff != 0, chunk, last_tile, po);
   else
-    sddmm_lean_kernel<LPR, false><<<blocks, kThreads, 0, stream>>>(a, b, c, indptr, indices, scale, m, nnz, feat,
-                                                                   foff, foff != 0, chunk, last_tile, po);
+    launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, false>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, nnz, feat,
+                   foff, foff != 0, chunk, last_tile, po);
   SPTIR_LAUNCH_OK("sddmm_lean_kernel");
   return 0;
 }

@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "tc05.cuh"
 #include "tmap.h"
 #include "vec.cuh"
@@ -155,6 +156,7 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, tmem_cols);
   }
+  chain_enter();
   tc05::fence_before_sync();
   __syncthreads();
   tc05::fence_after_sync();
@@ -351,8 +353,8 @@ int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const __half* w, c
   int tmem_cols = 32;
   while (tmem_cols < 2 * acc_cols) tmem_cols *= 2;
   const int grid = std::min(ceil_div(m, kTM), kNumSMs);
-  sparse_conv_kernel<OutT><<<grid, kThreads, smem, st>>>(tm_w, y, x, w, map, m, num_rels, feat_in, feat_out, tmem_cols,
-                                                        acc_cols, nstages, std::min(kGroups, nstages), add);
+  launch_chained(sparse_conv_kernel<OutT>, grid, kThreads, smem, st, tm_w, y, x, w, map, m, num_rels, feat_in, feat_out,
+                 tmem_cols, acc_cols, nstages, std::min(kGroups, nstages), add);
   SPTIR_LAUNCH_OK("sparse_conv_kernel");
   return 0;
 }

@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "mma16.cuh"
 #include "row_walk.cuh"
 #include "vec.cuh"
@@ -173,6 +174,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   const int q = lane & 3, r = lane >> 2;
   OutT* c = static_cast<OutT*>(s.c);
   float acc[MT][8][4];
+  chain_enter();
 
   if (unit >= s.windows) {  // ---- a short tile per warp
     const int io = (unit - s.windows) * 4 + warp;
@@ -348,7 +350,7 @@ int launch_mma(TcArgs s, int device_id, cudaStream_t st) {
   if (take_scratch(device_id, st, p.part_bytes, p.counter_bytes, &cs) != 0) return -1;
   s.part = reinterpret_cast<float*>(cs.scratch);
   s.counters = cs.counters;
-  tcspmm_mma_kernel<MT, OutT><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(s);
+  launch_chained(tcspmm_mma_kernel<MT, OutT>, static_cast<unsigned>(blocks), kThreads, 0, st, s);
   SPTIR_LAUNCH_OK("tcspmm_mma_kernel");
   return return_scratch(cs, st);
 }
