@@ -124,3 +124,23 @@ def test_long_windows_of_large_products(cuda_device):
         want = block @ b[up(ids[gp[io] * 16:gp[io + 1] * 16]).long()].double()
         # fp32 sums of exact products that are not negative
         assert bool(((c.view(-1, t, feat)[io].double() - want).abs() <= want * (g * 16 + 4) * 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("feat,shift", [(64, 8), (96, 8), (80, 0), (24, 0), (64, 0)])
+def test_outputs_with_and_without_whole_sectors(cuda_device, dtype, feat, shift):
+    """Results of 32-byte sectors are stored in one piece, others (a result 16 bytes off, rows of 48 bytes) in two."""
+    indptr, indices = matrix(700, {r: 1 + r % 30 for r in range(700)}, feat)
+    gp, tiles, mask = fmt.condense(indptr, indices, 16, 16)
+    mb = len(gp) - 1
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a).reshape(-1)).to(cuda_device)  # noqa: E731
+    a, gp_d, ids = up(mask.astype(np.float16)), up(gp), up(tiles)
+    b = (torch.randint(-8, 9, (44 * 16 * feat,), device=cuda_device) / 4).half()  # whole quarters: exact sums in any order
+    want = torch.zeros(mb * 16, feat, device=cuda_device)
+    rows = torch.repeat_interleave(torch.arange(700, device=cuda_device), torch.from_numpy(np.diff(indptr)).to(cuda_device))
+    want.index_add_(0, rows, b.view(-1, feat)[torch.from_numpy(indices).to(cuda_device).long()].float())
+    buf = torch.full((mb * 16 * feat + 64,), 3.0, dtype=dtype, device=cuda_device)
+    c = buf[shift:shift + mb * 16 * feat]
+    ops.tcspmm(a, b, c, gp_d, ids, mb, 44, len(tiles), feat, 16, 16)
+    assert torch.equal(c.view(-1, feat).float(), want.to(dtype).float())
+    assert bool((buf[:shift] == 3.0).all()) and bool((buf[shift + len(c):] == 3.0).all())
