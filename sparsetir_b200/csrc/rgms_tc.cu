@@ -225,11 +225,11 @@ rgms_tc_kernel(const float* __restrict__ a, const float* __restrict__ w,
 // tiles to each other through mbarriers, so loading, splitting, multiplying and scattering of
 // different tiles overlap:
 //   warp 0      producer: two TMA tile loads (128 rows x 128 bytes, 128-byte swizzle) bring the
-//               tile's z rows into one of two stages;
+//               tile's z rows into one of four stages;
 //   warps 8-11  converters: the tensor core reads only the upper 19 bits of an fp32 operand, so
-//               the raw tile serves as the "high" part as it is; the converters compute the
-//               remainder z - tf32(z) element by element into a second buffer at the same
-//               (swizzled) offsets, and stage W_r (raw and remainder) when the relation changes;
+//               the raw tile serves as the "high" part as it is; the converters (thread = tile row)
+//               compute the remainder z - tf32(z) element by element into TMEM, where the MMAs take
+//               it as their left operand, and stage W_r (raw and remainder) when the relation changes;
 //   warp 1      issues the 8 K-steps of the 3xTF32 product as two instructions each (W and its
 //               remainders stacked into one 128-row operand) into one of two TMEM accumulators
 //               of 128 columns, tcgen05.commit frees the stage and publishes the accumulator;
@@ -238,9 +238,14 @@ rgms_tc_kernel(const float* __restrict__ a, const float* __restrict__ w,
 //               into Y[I[t], :], four whole 128-byte lines per warp instruction.  (One bulk reduce-add per row, cp.reduce.async.bulk, was
 //               measured first: the block issues a bulk operation only every ~20 clocks, which
 //               made the epilogue the slowest role at 3,200 clocks per tile.)
+// With the remainders in shared memory there was room for two stages of raw tiles, and the MMAs read them from there a second
+// time (100 k nodes, 1.5 M edges: the call 128.1 us, with the remainders in TMEM 125.7; 20 k nodes, 90 relations, 200 k edges
+// 51.1 / 49.6).  What bounds it is the reductions into Y, which take 45 us in this launch and in the fp16 one.
 // Every mbarrier wait is bounded.
 constexpr int kPThreads = 512;
-constexpr int kZStages = 2;
+constexpr int kZStages = 4;
+constexpr uint32_t kPTmem = 512;         // two accumulators of 128 columns, two tiles of remainders of 64
+constexpr uint32_t kTmemLo = 4 * kF;     // column of the first remainders
 constexpr int kZBox = kTM * 128;     // one swizzled box: 128 rows x 32 floats
 constexpr int kZTile = 2 * kZBox;    // 32 KB
 // W_r as ONE operand of 128 rows: rows 0..63 = W (its upper 19 bits are what the tensor core
@@ -249,8 +254,7 @@ constexpr int kWBox = 2 * kF * 128;  // 16 KB
 constexpr int kWAll = 2 * kWBox;     // 32 KB
 constexpr int kOutStride = 128 + 16;  // padded half row: 16-byte stores of 32 rows spread over all banks
 constexpr int kOffZRaw = 0;
-constexpr int kOffZLo = kOffZRaw + kZStages * kZTile;
-constexpr int kOffW = kOffZLo + kZStages * kZTile;
+constexpr int kOffW = kOffZRaw + kZStages * kZTile;
 constexpr int kOffOut = kOffW + kWAll;
 constexpr int kPSmemBytes = kOffOut + 2 * kTM * kOutStride + 1024;  // two epilogue groups; + slack to align to 1024 bytes
 
@@ -269,7 +273,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
                 int rel_mod) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kZStages];   // z rows of the stage have landed
-  __shared__ __align__(8) uint64_t bar_conv[kZStages];   // remainders written (128 arrivals)
+  __shared__ __align__(8) uint64_t bar_conv[2];          // remainders written (128 arrivals)
   __shared__ __align__(8) uint64_t bar_empty[kZStages];  // tensor core has read the stage
   __shared__ __align__(8) uint64_t bar_acc_full[2];      // accumulator holds a finished tile
   __shared__ __align__(8) uint64_t bar_acc_empty[2];     // epilogue has read it (128 arrivals)
@@ -282,10 +286,10 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
     if (lane == 0) {
       for (int s = 0; s < kZStages; ++s) {
         tc05::mbar_init(&bar_full[s], 1);
-        tc05::mbar_init(&bar_conv[s], 128);
         tc05::mbar_init(&bar_empty[s], 1);
       }
       for (int b = 0; b < 2; ++b) {
+        tc05::mbar_init(&bar_conv[b], 128);
         tc05::mbar_init(&bar_acc_full[b], 1);
         tc05::mbar_init(&bar_acc_empty[b], 128);
       }
@@ -293,7 +297,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
       tc05::prefetch_tensormap(&tm_z);
     }
     __syncwarp();
-    tc05::tmem_alloc(&s_tmem, 4 * kF);
+    tc05::tmem_alloc(&s_tmem, kPTmem);
   }
   chain_enter();
   if (warp == 0) {
@@ -307,7 +311,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
   __syncthreads();
   tc05::fence_after_sync();
   if (s_tile[0] == 0) {  // no tile for this block (uniform)
-    if (warp == 0) tc05::tmem_dealloc(s_tmem, 4 * kF);
+    if (warp == 0) tc05::tmem_dealloc(s_tmem, kPTmem);
     return;
   }
   const uint32_t tmem = s_tmem;
@@ -342,21 +346,21 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
       // issues one dependent instruction every few clocks)
       const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base + kOffW), 0, 1024, tc05::kSwizzle128B);
       const uint64_t dzh0 = tc05::smem_desc_swizzled(tc05::smem_u32(base + kOffZRaw), 0, 1024, tc05::kSwizzle128B);
-      const uint64_t dzl0 = tc05::smem_desc_swizzled(tc05::smem_u32(base + kOffZLo), 0, 1024, tc05::kSwizzle128B);
       for (int k = 0; k < tiles_per_cta; ++k) {
         const int s = k % kZStages, use = k / kZStages, buf = k & 1, buse = k >> 1;
-        if (!tc05::mbar_wait(&bar_conv[s], use & 1)) { ok = false; break; }
+        if (!tc05::mbar_wait(&bar_full[s], use & 1)) { ok = false; break; }
+        if (!tc05::mbar_wait(&bar_conv[buf], buse & 1)) { ok = false; break; }
         if (buse > 0 && !tc05::mbar_wait(&bar_acc_empty[buf], (buse - 1) & 1)) { ok = false; break; }
         tc05::fence_after_sync();
         const uint64_t dzh_s = tc05::desc_advance(dzh0, s * kZTile);
-        const uint64_t dzl_s = tc05::desc_advance(dzl0, s * kZTile);
+        const uint32_t zlo = tmem + kTmemLo + buf * kF;
         const uint32_t acc = tmem + buf * 2 * kF;
 #pragma unroll
         for (int ks = 0; ks < kF / 8; ++ks) {  // K = 8 floats = 32 bytes inside the swizzled row
           const uint32_t zo = (ks >> 2) * kZBox + (ks & 3) * 32, wo = (ks >> 2) * kWBox + (ks & 3) * 32;
           const uint64_t dw = tc05::desc_advance(dw0, wo);
           tc05::mma_tf32(acc, tc05::desc_advance(dzh_s, zo), dw, idesc128, ks > 0 ? 1u : 0u);
-          tc05::mma_tf32(acc, tc05::desc_advance(dzl_s, zo), dw, idesc64, 1u);
+          tc05::mma_tf32_ts(acc, zlo + ks * 8, dw, idesc64, 1u);
         }
         tc05::mma_commit(&bar_empty[s]);
         tc05::mma_commit(&bar_acc_full[buf]);
@@ -385,17 +389,29 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
         }
       }
       if (!tc05::mbar_wait(&bar_full[s], use & 1)) { ok = false; break; }
+      // the remainders of the tile before the last one have been read
+      if (k > 1 && !tc05::mbar_wait(&bar_empty[(k - 2) % kZStages], ((k - 2) / kZStages) & 1)) { ok = false; break; }
+      tc05::fence_after_sync();
       const unsigned char* zr = base + kOffZRaw + s * kZTile;
-      unsigned char* zl = base + kOffZLo + s * kZTile;
-#pragma unroll 4
-      for (int j = 0; j < kZTile / 16 / 128; ++j) {
-        const int off = (j * 128 + ct) * 16;
-        const float4 v = *reinterpret_cast<const float4*>(zr + off);
-        *reinterpret_cast<float4*>(zl + off) =
-            make_float4(v.x - tf32_hi(v.x), v.y - tf32_hi(v.y), v.z - tf32_hi(v.z), v.w - tf32_hi(v.w));
+      const uint32_t zlo = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kTmemLo + (k & 1) * kF;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(zr + swz_off(ct, half * 8 + j, kZBox));
+          r[4 * j] = __float_as_uint(v.x - tf32_hi(v.x));
+          r[4 * j + 1] = __float_as_uint(v.y - tf32_hi(v.y));
+          r[4 * j + 2] = __float_as_uint(v.z - tf32_hi(v.z));
+          r[4 * j + 3] = __float_as_uint(v.w - tf32_hi(v.w));
+        }
+        __syncwarp();
+        tc05::tmem_st32(zlo + half * 32, r);
       }
-      tc05::fence_async_smem();
-      mbar_arrive(&bar_conv[s]);
+      tc05::tmem_st_wait();
+      tc05::fence_before_sync();
+      tc05::fence_async_smem();  // W, if it was staged for this tile
+      mbar_arrive(&bar_conv[k & 1]);
       if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
     }
   } else if (warp >= 4) {
@@ -464,7 +480,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
   }
   tc05::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc05::tmem_dealloc(tmem, 4 * kF);
+  if (warp == 0) tc05::tmem_dealloc(tmem, kPTmem);
 }
 
 // 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error
