@@ -21,9 +21,11 @@
 
 namespace sptir {
 
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  chain_wait();
+  chain_trigger();
 }
 
 // Where a call of many stored entries starts (0.3 ms and more), chaining is not worth what it can cost: blocks of the

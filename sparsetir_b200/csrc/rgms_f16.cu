@@ -42,6 +42,9 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBuckets = SPARSETIR_HYB_MAX_BUCKETS;
+// Fewest one-column rows that are transformed without a Z row: below, the two launches more cost what they save (64 -> 64,
+// a call that packs its tensors, 66 k such rows 30.3 us without, 33.3 with; 128 -> 64, 131 k 47.3 / 40.8).
+constexpr int kSingleRows = 96 << 10;
 
 __device__ unsigned int g_rgms_f16_timeouts = 0;
 
@@ -210,10 +213,16 @@ __device__ __forceinline__ void gather_few(const __half* __restrict__ a, const i
 __global__ void __launch_bounds__(kThreads)
 gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
                         const __half* __restrict__ x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
-                        int32_t* __restrict__ ranges, int num_rels, int chunks) {
-  chain_enter();
+                        int32_t* __restrict__ ranges, int num_rels, int chunks, int beside) {
+  // beside != 0: the launch before this one, the transform of the one-column rows, neither reads nor writes what
+  // this one writes, and its blocks have all passed their own wait when this one is scheduled, so that what lies ahead of
+  // both has ended: the gather runs beside it, in the registers that it leaves.  One block waits for it in the end,
+  // so that this launch has not ended before it.
+  if (beside == 0) chain_wait();
+  chain_trigger();
   if (blockIdx.x == gridDim.x - 1) {
     write_ranges(tb, num_rels, ranges);
+    if (beside != 0) chain_wait();
     return;
   }
   const int lanes = kThreads / chunks;  // rows side by side
@@ -869,6 +878,7 @@ namespace {
 // ranges[b * R + r] for every bucket (what the last block of the gather launches computes)
 __global__ void __launch_bounds__(kThreads)
 bucket_ranges_kernel(const __grid_constant__ BucketTable tb, int num_rels, int32_t* __restrict__ ranges) {
+  chain_enter();
   write_ranges(tb, num_rels, ranges);
 }
 
@@ -943,6 +953,99 @@ int launch_os(const __half* w, OutT* y, const __half* x, const int32_t* map, con
   return 0;
 }
 
+// Bytes of scratch for the two-launch form over these buckets: Z, the ranges, the row ids.
+size_t z_part(const BucketTable& tb, int feat_in) {
+  return (static_cast<size_t>(tb.z_base[tb.nb]) * feat_in * sizeof(__half) + 255) & ~static_cast<size_t>(255);
+}
+size_t range_part(const BucketTable& tb, int num_rels) {
+  return ((static_cast<size_t>(tb.nb) * num_rels + 1) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
+}
+size_t z_bytes(const BucketTable& tb, int num_rels, int feat_in) {
+  return z_part(tb, feat_in) + range_part(tb, num_rels) + static_cast<size_t>(tb.z_base[tb.nb]) * sizeof(int32_t);
+}
+
+void append_bucket(BucketTable& to, const BucketTable& from, int b) {
+  const int k = to.nb++;
+  to.a[k] = from.a[b]; to.cols[k] = from.cols[b]; to.rows[k] = from.rows[b]; to.mid[k] = from.mid[b];
+  to.num_groups[k] = from.num_groups[b];
+  to.rows_per_group[k] = from.rows_per_group[b];
+  to.width[k] = from.width[b];
+  to.z_base[k + 1] = to.z_base[k] + (from.z_base[b + 1] - from.z_base[b]);
+}
+BucketTable only_bucket(const BucketTable& tb, int b) {
+  BucketTable one{};
+  append_bucket(one, tb, b);
+  return one;
+}
+BucketTable without_bucket(const BucketTable& tb, int b) {
+  BucketTable rest{};
+  for (int k = 0; k < tb.nb; ++k)
+    if (k != b) append_bucket(rest, tb, k);
+  return rest;
+}
+// The largest bucket of one column, if there are others and it is worth launches of its own, or -1.
+int single_column_bucket(const BucketTable& tb) {
+  int best = -1, rows = kSingleRows - 1;
+  for (int b = 0; b < tb.nb; ++b)
+    if (tb.width[b] == 1 && tb.z_base[b + 1] - tb.z_base[b] > rows) {
+      best = b;
+      rows = tb.z_base[b + 1] - tb.z_base[b];
+    }
+  return tb.nb > 1 ? best : -1;
+}
+
+// The two launches over Z, ws: z_bytes() of scratch.  beside: the launch ahead is the transform of the one-column rows.
+template <typename OutT>
+int run_z(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int num_rels, int feat_in, int feat_out,
+          int path, char* ws, int beside, cudaStream_t st) {
+  const int total = tb.z_base[tb.nb];
+  const int num_ranges = tb.nb * num_rels;
+  const size_t zb = z_part(tb, feat_in), rb = range_part(tb, num_rels);
+  __half* z = reinterpret_cast<__half*>(ws);
+  int32_t* ranges = reinterpret_cast<int32_t*>(ws + zb);
+  int32_t* all_rows = reinterpret_cast<int32_t*>(ws + zb + rb);
+
+  const bool vec = feat_in % 8 == 0 && aligned16(x);
+  const int rows_per_tile = std::max(1, kThreads / (vec ? feat_in / 8 : feat_in));
+  const int blocks = static_cast<int>(std::min<long long>(ceil_div(total, rows_per_tile), 64ll * kNumSMs));
+  bool one_column = vec && feat_in / 8 <= kThreads;
+  for (int b = 0; b < tb.nb; ++b) one_column = one_column && tb.width[b] == 1;
+  if (one_column) {
+    const int rows_per_block = (kThreads / (feat_in / 8)) * kCopyR;
+    const int nblk = static_cast<int>(std::min<long long>(ceil_div(total, rows_per_block), 64ll * kNumSMs));
+    scale_rows_f16_kernel<<<nblk + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
+  } else if (vec && feat_in / 8 <= kThreads) {
+    GatherTiles gt{};
+    const int lanes = kThreads / (feat_in / 8);
+    long long tiles = 0;
+    for (int b = 0; b < tb.nb; ++b) {
+      gt.first[b] = static_cast<int32_t>(tiles);
+      tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
+    }
+    launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(tiles + 1), kThreads, 0, st, tb, gt, x, z, all_rows, ranges,
+                   num_rels, feat_in / 8, beside);
+  } else if (vec)
+    gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
+  else
+    gather_rows_f16_kernel<1><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
+  SPTIR_LAUNCH_OK("gather_rows_f16_kernel");
+
+  // Slices and boxes may reach past the last feature: what they bring from there is zeros, or the next
+  // relation's weights, and is not multiplied.  100 k nodes, 1.5 M edges, 46 relations, 32 -> 32: the
+  // CUDA-core transform 268 us in all, this 64 us.
+  if (path != 2 && feat_in % 16 == 0 && feat_out % 32 == 0 && feat_out <= kMaxOut && aligned16(w) && aligned16(y)) {
+    const int rc = launch_tc<OutT, false>(z, w, y, ranges, all_rows, num_ranges, num_rels, total,
+                                          feat_in, feat_out, st);
+    if (rc <= 0) return rc;
+  }
+  const size_t smem = static_cast<size_t>(kSimtRows) * feat_in * sizeof(float);
+  if (smem > 48 * 1024) return fail("sparsetir_rgms_ell3d_f16: feat_in %d is too large", feat_in);
+  transform_scatter_f16_kernel<OutT><<<ceil_div(total, kSimtRows), kThreads, smem, st>>>(
+      tb, z, w, y, all_rows, feat_in, feat_out);
+  SPTIR_LAUNCH_OK("transform_scatter_f16_kernel");
+  return 0;
+}
+
 template <typename OutT>
 int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m, int num_rels, int feat_in,
         int feat_out, int device_id, cudaStream_t st) {
@@ -983,7 +1086,7 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
     int32_t* ranges1 = reinterpret_cast<int32_t*>(ws1);
     int32_t* flag = reinterpret_cast<int32_t*>(ws1 + rb1);
     int32_t* map = reinterpret_cast<int32_t*>(ws1 + rb1 + 256);
-    bucket_ranges_kernel<<<1, kThreads, 0, st>>>(tb, num_rels, ranges1);
+    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, tb, num_rels, ranges1);
     SPTIR_LAUNCH_OK("bucket_ranges_kernel");
     int rc = 1;
     if (try_os) {
@@ -999,53 +1102,28 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
                                feat_in, feat_out, st, x, tb.cols[0], tb.a[0], rc == 0 ? flag : nullptr);
     if (rc <= 0) return rc;
   }
-  const size_t zb = (static_cast<size_t>(total) * feat_in * sizeof(__half) + 255) & ~static_cast<size_t>(255);
-  const size_t rb = (static_cast<size_t>(num_ranges + 1) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
-  char* ws = static_cast<char*>(workspace(device_id, st, zb + rb + static_cast<size_t>(total) * sizeof(int32_t)));
-  if (!ws) return -1;
-  __half* z = reinterpret_cast<__half*>(ws);
-  int32_t* ranges = reinterpret_cast<int32_t*>(ws + zb);
-  int32_t* all_rows = reinterpret_cast<int32_t*>(ws + zb + rb);
-
-  const bool vec = feat_in % 8 == 0 && aligned16(x);
-  const int rows_per_tile = std::max(1, kThreads / (vec ? feat_in / 8 : feat_in));
-  const int blocks = static_cast<int>(std::min<long long>(ceil_div(total, rows_per_tile), 64ll * kNumSMs));
-  bool one_column = vec && feat_in / 8 <= kThreads;
-  for (int b = 0; b < tb.nb; ++b) one_column = one_column && tb.width[b] == 1;
-  if (one_column) {
-    const int rows_per_block = (kThreads / (feat_in / 8)) * kCopyR;
-    const int nblk = static_cast<int>(std::min<long long>(ceil_div(total, rows_per_block), 64ll * kNumSMs));
-    scale_rows_f16_kernel<<<nblk + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
-  } else if (vec && feat_in / 8 <= kThreads) {
-    GatherTiles gt{};
-    const int lanes = kThreads / (feat_in / 8);
-    long long tiles = 0;
-    for (int b = 0; b < tb.nb; ++b) {
-      gt.first[b] = static_cast<int32_t>(tiles);
-      tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
-    }
-    launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(tiles + 1), kThreads, 0, st, tb, gt, x, z, all_rows, ranges,
-                   num_rels, feat_in / 8);
-  } else if (vec)
-    gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
-  else
-    gather_rows_f16_kernel<1><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
-  SPTIR_LAUNCH_OK("gather_rows_f16_kernel");
-
-  // Slices and boxes may reach past the last feature: what they bring from there is zeros, or the next
-  // relation's weights, and is not multiplied.  100 k nodes, 1.5 M edges, 46 relations, 32 -> 32: the
-  // CUDA-core transform 268 us in all, this 64 us.
-  if (path != 2 && feat_in % 16 == 0 && feat_out % 32 == 0 && feat_out <= kMaxOut && aligned16(w) && aligned16(y)) {
-    const int rc = launch_tc<OutT, false>(z, w, y, ranges, all_rows, static_cast<int>(num_ranges), num_rels, total,
-                                          feat_in, feat_out, st);
-    if (rc <= 0) return rc;
+  // The rows of one column need no Z either where there are buckets of wider rows beside them: they are transformed
+  // straight from X, and the launches over Z below see the other buckets, whose gather runs beside that transform: the
+  // one is bound by L2 reads, the other by the reductions into Y (3.9 TB/s).  In a relational graph most rows are
+  // such (100 k nodes, 46 relations, 1.5 M edges, 430 k rows of 690 k, us: 64 -> 64 one transform over Z 100, two 93, with the
+  // gather beside the first 84.6; 128 -> 128 180, 160, 150).
+  const int single = tc_shape && path == 0 && aligned16(x) ? single_column_bucket(tb) : -1;
+  if (single >= 0) {
+    const BucketTable one = only_bucket(tb, single), rest = without_bucket(tb, single);
+    const size_t rb1 = (static_cast<size_t>(num_rels + 1) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
+    char* ws1 = static_cast<char*>(workspace(device_id, st, rb1 + z_bytes(rest, num_rels, feat_in)));
+    if (!ws1) return -1;
+    int32_t* ranges1 = reinterpret_cast<int32_t*>(ws1);
+    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, one, num_rels, ranges1);
+    SPTIR_LAUNCH_OK("bucket_ranges_kernel");
+    const int rc = launch_tc<OutT, true>(nullptr, w, y, ranges1, one.rows[0], num_rels, num_rels, one.z_base[1], feat_in,
+                                         feat_out, st, x, one.cols[0], one.a[0]);
+    if (rc < 0) return rc;
+    if (rc == 0) return run_z<OutT>(rest, w, x, y, num_rels, feat_in, feat_out, path, ws1 + rb1, 1, st);
   }
-  const size_t smem = static_cast<size_t>(kSimtRows) * feat_in * sizeof(float);
-  if (smem > 48 * 1024) return fail("sparsetir_rgms_ell3d_f16: feat_in %d is too large", feat_in);
-  transform_scatter_f16_kernel<OutT><<<ceil_div(total, kSimtRows), kThreads, smem, st>>>(
-      tb, z, w, y, all_rows, feat_in, feat_out);
-  SPTIR_LAUNCH_OK("transform_scatter_f16_kernel");
-  return 0;
+  char* ws = static_cast<char*>(workspace(device_id, st, z_bytes(tb, num_rels, feat_in)));
+  if (!ws) return -1;
+  return run_z<OutT>(tb, w, x, y, num_rels, feat_in, feat_out, path, ws, 0, st);
 }
 
 }  // namespace
