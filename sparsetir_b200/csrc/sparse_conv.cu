@@ -6,19 +6,22 @@
 //
 // The product is one GEMM per tile with K = R * feat_in: row t of the left operand is the
 // concatenation of the X rows of its pairs (zeros where there is none), the right operand is W as
-// it lies in memory.  A persistent block per SM walks the tiles; per 64-wide slice of K
+// it lies in memory.  A persistent block per SM walks the tiles, one at a time or two side by side (TPS); per
+// 64-wide slice of K
 //  - six groups of four warps fetch the left operand with 16-byte asynchronous copies into the
 //    swizzled stage (a slice may straddle offsets, so channel counts that are not multiples of 64
 //    waste nothing; a missing pair is a copy of no bytes, which fills in zeros);
 //  - one thread brings the slice of W with TMA, one issues the MMAs into one of two accumulators;
 //  - four warps take finished tiles out of TMEM and write (or add to) Y, each row once.
 //
-// Bound by the instructions and round trips of the ring, not by a unit (100,000 points, 27 offsets,
-// 64 -> 128: tensor pipe 34 %, L1 data pipe 61 %, L2 22 %): the time goes with the steps and hardly
-// depends on the share of pairs or on feat_out.  What the steps cost is therefore what was cut: no
-// divisions in the loops and MMAs from an elected thread 97 -> 64 us, asynchronous copies instead of
-// loads and stores 64 -> 61 us.  Gathering by TMA (four rows per copy) took 215 us.  The map replaces one
-// built, checked and cleared on every call: together with the cleared Y that took 37 us of 122.
+// Bound by the issue slots of an SM and its L1 data pipe, not by memory or the tensor cores: at 100,000 points, 27
+// offsets, 64 -> 32 a layer with 2 % of the pairs takes as long as one with 95 % of them.  What was cut is therefore
+// instructions and what passes the data pipe: no divisions in the loops and MMAs from an elected thread 97 -> 64 us (64 ->
+// 128), asynchronous copies instead of loads and stores 64 -> 58; then (us, 64 -> 128 / 64 -> 32, 54.7 / 48.6 before) one
+// slice of W for two tiles and copies that arrive at the stage's barrier themselves, 51.5 / 44.2, the copies of a step
+// written out, 50.3 / 41.2, an epilogue of a third of the instructions, 47.2 / 39.7.  Rows loaded into registers and
+// stored took 54.9, gathering by TMA (four rows per copy) 215 us.  The map replaces one built, checked and cleared on
+// every call: together with the cleared Y that took 37 us of 122.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -43,6 +46,9 @@ constexpr int kFirstGather = 8;         // warp 0 loads W, 1 issues MMAs, 4-7 ep
 constexpr int kThreads = (kFirstGather + 4 * kGroups) * 32;
 constexpr int kOutStride = 128 + 16;    // padded row of 32 floats: rows spread over all banks
 constexpr int kOutBytes = kTM * kOutStride;
+// byte offset of 16-byte piece q of a row of 32 halves: unpadded rows, whose pieces are exchanged so that eight rows
+// written at once, or two read, touch every bank once
+__device__ __forceinline__ int half_piece(int row, int q) { return row * 64 + ((q ^ ((row >> 1) & 3)) << 4); }
 constexpr int kSmemLimit = 226 * 1024;  // dynamic part: the static barriers count against the 227 KB too
 
 __device__ unsigned int g_conv_timeouts = 0;
@@ -51,51 +57,102 @@ __device__ __forceinline__ void arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc05::smem_u32(bar)) : "memory");
 }
 
-// 32 columns of 32 rows of a finished tile, staged in shared memory, go to Y with whole 128-byte
-// (fp32) or 64-byte (fp16) row pieces; with `add` all old values are read before the first store
-__device__ __forceinline__ void write32(float* y, const unsigned char* wbase, int row_base, int nrows, int feat_out,
-                                        int c0, int lane, bool add) {
+// 32 columns of a lane's row of a finished tile go to the warp's part of the staging buffer, rounded to the result's type.
+// True if a value may be a NaN: 0 * v is one for every v that is not finite.  (A comparison per value is twice
+// the instructions, and the epilogue's instructions share the issue slots with those of the gathering warps.)
+__device__ __forceinline__ bool stage32(const float*, unsigned char* wbase, int lane, const uint32_t (&r)[32]) {
+  unsigned long long t[2] = {0ull, 0ull};
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    *reinterpret_cast<uint4*>(wbase + lane * kOutStride + q * 16) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const unsigned long long v = static_cast<unsigned long long>(r[4 * q + 2 * j + 1]) << 32 | r[4 * q + 2 * j];
+      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t[j]) : "l"(v), "l"(0ull));
+    }
+  }
+  float lo, hi, lo2, hi2;
+  unpack_pair(t[0], lo, hi);
+  unpack_pair(t[1], lo2, hi2);
+  const float any = (lo + hi) + (lo2 + hi2);
+  return any != any;
+}
+__device__ __forceinline__ bool stage32(const __half*, unsigned char* wbase, int lane, const uint32_t (&r)[32]) {
+  const __half2 zero = __floats2half2_rn(0.f, 0.f);
+  __half2 t[2] = {zero, zero};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 o;
+    __half2* h = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      h[j] = __floats2half2_rn(__uint_as_float(r[8 * q + 2 * j]), __uint_as_float(r[8 * q + 2 * j + 1]));
+      t[j & 1] = __hfma2(h[j], zero, t[j & 1]);
+    }
+    *reinterpret_cast<uint4*>(wbase + half_piece(lane, q)) = o;
+  }
+  const __half2 any = __hadd2(t[0], t[1]);
+  return __hisnan(__low2half(any)) || __hisnan(__high2half(any));
+}
+__device__ __forceinline__ void stage1(const float*, unsigned char* wbase, int row, int col, float v) {
+  *reinterpret_cast<float*>(wbase + row * kOutStride + col * 4) = v;
+}
+__device__ __forceinline__ void stage1(const __half*, unsigned char* wbase, int row, int col, float v) {
+  *reinterpret_cast<__half*>(wbase + half_piece(row, col >> 3) + (col & 7) * 2) = __float2half_rn(v);
+}
+
+// The warp's 32 staged rows go to Y with whole 128-byte (fp32) or 64-byte (fp16) row pieces; y points at the first of
+// the 32 columns in the warp's first row.  With `add` all old values are read before the first store.
+__device__ __forceinline__ void write32(float* y, const unsigned char* wbase, int nrows, int feat_out, int lane, bool add) {
+  const unsigned char* from = wbase + (lane >> 3) * kOutStride + (lane & 7) * 16;
+  float4* to = reinterpret_cast<float4*>(y + static_cast<size_t>(lane >> 3) * feat_out) + (lane & 7);
+  const size_t step = static_cast<size_t>(feat_out);  // four rows, in 16-byte pieces
+  if (!add) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (4 * i + (lane >> 3) < nrows) __stcs(to + i * step, *reinterpret_cast<const float4*>(from + 4 * i * kOutStride));
+    return;
+  }
   float4 old[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int lr = 4 * i + (lane >> 3);
     old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (add && lr < nrows)
-      old[i] = __ldcs(reinterpret_cast<const float4*>(y + static_cast<size_t>(row_base + lr) * feat_out + c0) + (lane & 7));
+    if (4 * i + (lane >> 3) < nrows) old[i] = __ldcs(to + i * step);
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int lr = 4 * i + (lane >> 3);
-    if (lr < nrows) {
-      const float4 v = *reinterpret_cast<const float4*>(wbase + lr * kOutStride + (lane & 7) * 16);
-      __stcs(reinterpret_cast<float4*>(y + static_cast<size_t>(row_base + lr) * feat_out + c0) + (lane & 7),
-             make_float4(old[i].x + v.x, old[i].y + v.y, old[i].z + v.z, old[i].w + v.w));
+    if (4 * i + (lane >> 3) < nrows) {
+      const float4 v = *reinterpret_cast<const float4*>(from + 4 * i * kOutStride);
+      __stcs(to + i * step, make_float4(old[i].x + v.x, old[i].y + v.y, old[i].z + v.z, old[i].w + v.w));
     }
   }
 }
-__device__ __forceinline__ void write32(__half* y, const unsigned char* wbase, int row_base, int nrows, int feat_out,
-                                        int c0, int lane, bool add) {
+__device__ __forceinline__ void write32(__half* y, const unsigned char* wbase, int nrows, int feat_out, int lane, bool add) {
+  const unsigned char* from = wbase + half_piece(lane >> 2, lane & 3);  // rows 8 apart have their pieces in the same order
+  uint4* to = reinterpret_cast<uint4*>(y + static_cast<size_t>(lane >> 2) * feat_out) + (lane & 3);
+  const size_t step = static_cast<size_t>(feat_out);  // eight rows, in 16-byte pieces
+  if (!add) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (8 * i + (lane >> 2) < nrows) __stcs(to + i * step, *reinterpret_cast<const uint4*>(from + 8 * i * 64));
+    return;
+  }
   uint4 old[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int lr = 8 * i + (lane >> 2);
     old[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (add && lr < nrows)
-      old[i] = __ldcs(reinterpret_cast<const uint4*>(y + static_cast<size_t>(row_base + lr) * feat_out + c0) + (lane & 3));
+    if (8 * i + (lane >> 2) < nrows) old[i] = __ldcs(to + i * step);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int lr = 8 * i + (lane >> 2);
-    if (lr < nrows) {
-      const float4 a = *reinterpret_cast<const float4*>(wbase + lr * kOutStride + (lane & 3) * 32);
-      const float4 b = *reinterpret_cast<const float4*>(wbase + lr * kOutStride + (lane & 3) * 32 + 16);
+    if (8 * i + (lane >> 2) < nrows) {
+      const uint4 v = *reinterpret_cast<const uint4*>(from + 8 * i * 64);
+      const __half2* vh = reinterpret_cast<const __half2*>(&v);
       uint4 o = old[i];
       __half2* h = reinterpret_cast<__half2*>(&o);
-      h[0] = __hadd2(h[0], __floats2half2_rn(a.x, a.y));
-      h[1] = __hadd2(h[1], __floats2half2_rn(a.z, a.w));
-      h[2] = __hadd2(h[2], __floats2half2_rn(b.x, b.y));
-      h[3] = __hadd2(h[3], __floats2half2_rn(b.z, b.w));
-      __stcs(reinterpret_cast<uint4*>(y + static_cast<size_t>(row_base + lr) * feat_out + c0) + (lane & 3), o);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = __hadd2(h[j], vh[j]);
+      __stcs(to + i * step, o);
     }
   }
 }
@@ -119,11 +176,35 @@ __device__ __noinline__ float row_by_pairs(const __half* __restrict__ x, const _
   return sum;
 }
 
-template <typename OutT>
+// Eight rows' pieces of 16 bytes into shared memory: row i from xb + from[i] * row_bytes to at0 (even i) or at1 (odd i)
+// + i / 2 * 1024; zeros where from[i] is negative, or everywhere with `skip`.  One statement, written out: what bounds the
+// kernel is the instructions of the gathering warps, and the selects and addresses that the compiler made of the
+// same loop were more: 16 instructions a step and warp are 4 us of 45 (100,000 points, 27 offsets, 64 -> 32).
+__device__ __forceinline__ void copy_rows(uint32_t at0, uint32_t at1, const int (&from)[8], uint32_t row_bytes, const char* xb, int skip) {
+#define SPTIR_COPY_ROW(E, AT, OFF)              \
+  "setp.lt.or.s32 p, " E ", 0, q;\n\t"          \
+  "max.s32 f, " E ", 0;\n\t"                    \
+  "mad.wide.u32 a, f, %10, %11;\n\t"            \
+  "cp.async.cg.shared.global [" AT "+" OFF "], [a], 16, p;\n\t"
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a;\n\t.reg .b32 f;\n\t"
+      "setp.ne.s32 q, %12, 0;\n\t"
+      SPTIR_COPY_ROW("%2", "%0", "0") SPTIR_COPY_ROW("%3", "%1", "0")
+      SPTIR_COPY_ROW("%4", "%0", "1024") SPTIR_COPY_ROW("%5", "%1", "1024")
+      SPTIR_COPY_ROW("%6", "%0", "2048") SPTIR_COPY_ROW("%7", "%1", "2048")
+      SPTIR_COPY_ROW("%8", "%0", "3072") SPTIR_COPY_ROW("%9", "%1", "3072")
+      "}"
+      ::"r"(at0), "r"(at1), "r"(from[0]), "r"(from[1]), "r"(from[2]), "r"(from[3]), "r"(from[4]), "r"(from[5]), "r"(from[6]),
+        "r"(from[7]), "r"(row_bytes), "l"(xb), "r"(skip)
+      : "memory");
+#undef SPTIR_COPY_ROW
+}
+
+template <typename OutT, int TPS>
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ y, const __half* __restrict__ x,
                    const __half* __restrict__ w, const int32_t* __restrict__ map, int m, int num_rels, int feat_in,
-                   int feat_out, int tmem_cols, int acc_cols, int nstages, int groups, int add) {
+                   int feat_out, int tmem_cols, int acc_cols, int nstages, int slots, int add) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];   // both operands of the stage are there
   __shared__ __align__(8) uint64_t bar_empty[kMaxStages];  // the tensor core has read the stage
@@ -133,17 +214,19 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* base = smem_raw + ((1024u - (tc05::smem_u32(smem_raw) & 1023u)) & 1023u);
   const int nwb = (feat_out + 63) / 64;
-  const int stride = kZBytes + nwb * kWBox;
+  const int stride = TPS * kZBytes + nwb * kWBox;
   const int ktotal = num_rels * feat_in;
-  const int steps = (ktotal + kKC - 1) / kKC;  // stages per tile
+  const int steps = (ktotal + kKC - 1) / kKC;  // stages per unit of TPS tiles
   const int ntiles = (m + kTM - 1) / kTM;
   // tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the grid never exceeds the number of tiles
   const int my_tiles = (ntiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
 
+  const int units = (my_tiles + TPS - 1) / TPS;  // the last one may be a tile short
+
   if (warp == 0) {
     if (lane == 0) {
       for (int s = 0; s < nstages; ++s) {
-        tc05::mbar_init(&bar_full[s], 1 + 4);  // W, and the four warps of a gather group
+        tc05::mbar_init(&bar_full[s], 1 + 128 * TPS);  // W, and the threads of a gather group per tile
         tc05::mbar_init(&bar_empty[s], 1);
       }
       for (int b = 0; b < 2; ++b) {
@@ -169,15 +252,15 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     if (tc05::elect_one()) {
       int s = 0;
       uint32_t phase = 0;
-      unsigned char* st = base + kZBytes;
-      for (int k = 0; k < my_tiles && ok; ++k) {
+      unsigned char* st = base + TPS * kZBytes;
+      for (int u = 0; u < units && ok; ++u) {
         for (int sidx = 0; sidx < steps; ++sidx) {
           if (!tc05::mbar_wait(&bar_empty[s], phase ^ 1u)) { ok = false; break; }
           tc05::mbar_arrive_expect_tx(&bar_full[s], nwb * kWBox);
           for (int j = 0; j < nwb; ++j) tc05::tma_load_2d(st + j * kWBox, &tm_w, j * 64, sidx * kKC, &bar_full[s]);
           ++armed;
           st += stride;
-          if (++s == nstages) { s = 0; phase ^= 1u; st = base + kZBytes; }
+          if (++s == nstages) { s = 0; phase ^= 1u; st = base + TPS * kZBytes; }
         }
       }
     }
@@ -186,17 +269,21 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     if (tc05::elect_one()) {
       const uint32_t idesc = tc05::instr_desc(tc05::kFmtF16, kTM, feat_out, /*a_mn=*/0, /*b_mn=*/1);
       const uint64_t dz0 = tc05::smem_desc_swizzled(tc05::smem_u32(base), 0, 1024, tc05::kSwizzle128B);
-      const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base) + kZBytes, kWBox, 1024, tc05::kSwizzle128B);
+      const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base) + TPS * kZBytes, kWBox, 1024, tc05::kSwizzle128B);
       const int last = (ktotal - (steps - 1) * kKC) / 16;  // instructions of the last slice
       int s = 0;
       uint32_t phase = 0;
       uint64_t dz = dz0, dw = dw0;
-      for (int k = 0; k < my_tiles && ok; ++k) {
-        const int buf = k & 1, buse = k >> 1;
+      for (int u = 0; u < units && ok; ++u) {
+        const int buf = u & 1, buse = u >> 1;
+        const bool both = TPS == 2 && u * TPS + 1 < my_tiles;
         if (!tc05::mbar_wait(&bar_acc_empty[buf], (buse & 1) ^ 1)) { ok = false; break; }
-        const uint32_t acc = tmem + buf * acc_cols;
+        const uint32_t acc = tmem + buf * (TPS * acc_cols);
         for (int sidx = 0; sidx < steps; ++sidx) {
           if (!tc05::mbar_wait(&bar_full[s], phase)) { ok = false; break; }
+          // the rows come by cp.async, whose writes the barrier has made visible to this thread: on to the
+          // proxy that the tensor core reads through
+          tc05::fence_async_smem();
           tc05::fence_after_sync();
           const int ksteps = sidx + 1 < steps ? kKC / 16 : last;
 #pragma unroll
@@ -204,6 +291,13 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
             if (ks < ksteps)
               tc05::mma_f16(acc, tc05::desc_advance(dz, ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
                             (sidx > 0 || ks > 0) ? 1u : 0u);
+          if (both) {
+#pragma unroll
+            for (int ks = 0; ks < kKC / 16; ++ks)
+              if (ks < ksteps)
+                tc05::mma_f16(acc + acc_cols, tc05::desc_advance(dz, kZBytes + ks * 32), tc05::desc_advance(dw, ks * 2048), idesc,
+                              (sidx > 0 || ks > 0) ? 1u : 0u);
+          }
           tc05::mma_commit(&bar_empty[s]);
           dz = tc05::desc_advance(dz, stride);
           dw = tc05::desc_advance(dw, stride);
@@ -214,112 +308,111 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
       }
     }
   } else if (warp >= kFirstGather) {
-    // ---- gather: group g fills the left operand of steps g, g + groups, ...; warp gw of it rows
-    // gw * 32 .. gw * 32 + 31, eight lanes per row.  No more groups than stages: a group that has
-    // written step n knows that the tensor core is past step n - nstages, and may wait for the stage
-    // of step n + groups only if that puts it at most one phase of the stage's barrier behind.  The map
-    // entries of a group's next step are requested before this step's rows are written.
+    // ---- gather: group g fills tile g % TPS of the steps g / TPS, g / TPS + slots, ...; warp gw of it rows
+    // gw * 32 .. gw * 32 + 31 of the tile, eight lanes per row.  Nobody waits for the copies: they arrive at the
+    // stage's barrier themselves.  No more slots than stages: the group that passes the wait of step n knows that the
+    // tensor core is past step n - nstages, and may wait for the stage of step n + slots only if that puts it at most
+    // one phase of the stage's barrier behind.  The map entries of a group's next step are requested before this
+    // step's rows are copied.
     //
     // (offset, piece) of the lane move by whole rows of the ring: quotients and remainders are formed once.
     const int g = (warp - kFirstGather) >> 2, gw = (warp - kFirstGather) & 3;
+    const int half = g % TPS, slot = g / TPS;
     const int cpr = feat_in / 8;  // 16-byte pieces per X row
+    const uint32_t row_bytes = static_cast<uint32_t>(feat_in) * 2u;
     const int chunk = lane & 7;
-    const int step_rel = groups * 8 / cpr, step_off = groups * 8 - step_rel * cpr;
-    const int tile_rel = steps * 8 / cpr, tile_off = steps * 8 - tile_rel * cpr;
-    int sidx = g, rel = (g * 8 + chunk) / cpr, off = g * 8 + chunk - rel * cpr;
-    int left = my_tiles;  // tiles from the one of this step on
+    const int step_rel = slots * 8 / cpr, step_off = slots * 8 - step_rel * cpr;
+    const int unit_rel = steps * 8 / cpr, unit_off = steps * 8 - unit_rel * cpr;
+    int sidx = slot, rel = (slot * 8 + chunk) / cpr, off = slot * 8 + chunk - rel * cpr;
+    int left = my_tiles;  // tiles from the unit of this step on
     const size_t tile_map = static_cast<size_t>(num_rels) * kTM;
-    const int32_t* mp = map + static_cast<size_t>(blockIdx.x) * tile_map + gw * 32 + (lane >> 3);
-    auto into_tile = [&]() {  // steps past the end of a tile belong to the block's next ones
+    const int32_t* mp = map + (blockIdx.x + static_cast<size_t>(half) * gridDim.x) * tile_map + gw * 32 + (lane >> 3);
+    auto into_unit = [&]() {  // steps past the end of a unit belong to the block's next ones
       while (left > 0 && sidx >= steps) {
         sidx -= steps;
-        --left;
-        mp += tile_map * gridDim.x;
-        rel -= tile_rel;
-        off -= tile_off;
+        left -= TPS;
+        mp += tile_map * (TPS * gridDim.x);
+        rel -= unit_rel;
+        off -= unit_off;
         if (off < 0) { off += cpr; --rel; }
       }
     };
-    int entry[8];
+    int entry[8];     // of the next step, as they come: looked at a step later, so that nobody waits for them here
+    int none = 0;     // not 0: the next step has none for this lane
     auto entries_of_step = [&]() {
-      const bool in = rel < num_rels;
-      const int32_t* e = mp + static_cast<size_t>(in ? rel : 0) * kTM;
+      const bool in = left > half && rel < num_rels;
+      none = in ? 0 : 1;
+      const int32_t* e = in ? mp + static_cast<size_t>(rel) * kTM : map;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int v = __ldg(e + 4 * i);
-        entry[i] = in ? v : -1;
-      }
+      for (int i = 0; i < 8; ++i) entry[i] = __ldg(e + 4 * i);
     };
-    int s = g;
-    uint32_t phase = 0;
-    if (g < groups) into_tile();
-    if (g < groups && left > 0) entries_of_step();
-    while (g < groups && left > 0) {
-      const int piece = off;
+    // the lane's rows of the tile are 4 apart: two places in an atom of 8 swizzled rows, atoms 1024 bytes apart
+    const int r4 = lane >> 3;
+    const uint32_t at0 = tc05::smem_u32(base) + half * kZBytes + gw * 4096 + r4 * 128 + ((chunk ^ r4) << 4);
+    const uint32_t at1 = tc05::smem_u32(base) + half * kZBytes + gw * 4096 + (4 + r4) * 128 + ((chunk ^ (4 + r4)) << 4);
+    int s = slot;
+    uint32_t phase = 0, stage = slot * stride;
+    if (slot < slots) into_unit();
+    if (slot < slots && left > 0) entries_of_step();
+    while (slot < slots && left > 0) {
+      const char* xb = reinterpret_cast<const char*>(x) + off * 16;
+      const bool tile_there = left > half;
+      const int skip = none;
       int from[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) from[i] = entry[i];
-      sidx += groups;
+      sidx += slots;
       rel += step_rel;
       off += step_off;
       if (off >= cpr) { off -= cpr; ++rel; }
-      into_tile();
+      into_unit();
       if (left > 0) entries_of_step();
       if (!tc05::mbar_wait(&bar_empty[s], phase ^ 1u)) { ok = false; break; }
-      const uint32_t st = tc05::smem_u32(base + s * stride);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int row = gw * 32 + 4 * i + (lane >> 3);
-        const uint32_t dst = st + (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
-        const __half* src = x + static_cast<size_t>(max(from[i], 0)) * feat_in + piece * 8;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(from[i] >= 0 ? 16u : 0u)
-                     : "memory");
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      tc05::fence_async_smem();
-      __syncwarp();
-      if (lane == 0) arrive(&bar_full[s]);
-      s += groups;
-      if (s >= nstages) { s -= nstages; phase ^= 1u; }
+      if (tile_there) copy_rows(at0 + stage, at1 + stage, from, row_bytes, xb, skip);
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc05::smem_u32(&bar_full[s])) : "memory");
+      s += slots;
+      stage += slots * stride;
+      if (s >= nstages) { s -= nstages; stage -= nstages * stride; phase ^= 1u; }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");  // also when giving up: nothing may land later
   } else if (warp >= 4) {
     // ---- epilogue: thread = tile row = TMEM lane, 32 columns at a time
-    unsigned char* buf0 = base + nstages * stride;
-    unsigned char* my_row = buf0 + ((warp & 3) * 32 + lane) * kOutStride;
-    const unsigned char* wbase = buf0 + (warp & 3) * 32 * kOutStride;
-    for (int k = 0; k < my_tiles; ++k) {
-      const int buf = k & 1, buse = k >> 1;
-      const int row_base = (static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x)) * kTM + (warp & 3) * 32;
-      const int nrows = min(32, m - row_base);  // live rows among the warp's 32 (may be <= 0)
+    unsigned char* wbase = base + nstages * stride + (warp & 3) * 32 * kOutStride;
+    for (int u = 0; u < units && ok; ++u) {
+      const int buf = u & 1, buse = u >> 1;
       if (!tc05::mbar_wait(&bar_acc_full[buf], buse & 1)) { ok = false; break; }
       tc05::fence_after_sync();
-      const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + buf * acc_cols;
-      for (int c0 = 0; c0 < feat_out; c0 += 32) {
-        uint32_t r[32];
-        tc05::tmem_ld32(taddr + c0, r);
-        if (c0 + 32 >= feat_out) {  // the accumulator is in registers: a later tile may overwrite it
-          tc05::fence_before_sync();
+#pragma unroll 1
+      for (int h = 0; h < TPS && u * TPS + h < my_tiles; ++h) {
+        const int tile = static_cast<int>(blockIdx.x) + (u * TPS + h) * static_cast<int>(gridDim.x);
+        const int row_base = tile * kTM + (warp & 3) * 32;
+        const int nrows = min(32, m - row_base);  // live rows among the warp's 32 (may be <= 0)
+        const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (buf * TPS + h) * acc_cols;
+        for (int c0 = 0; c0 < feat_out; c0 += 32) {
+          uint32_t r[32];
+          tc05::tmem_ld32(taddr + c0, r);
+          if (c0 + 32 >= feat_out && (h == TPS - 1 || u * TPS + h + 1 == my_tiles)) {
+            // the unit's results are in registers: a later one may overwrite its accumulators
+            tc05::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) arrive(&bar_acc_empty[buf]);
+          }
+          __syncwarp();  // the warp's reads of the previous 32 columns are over
+          bool nan = stage32(y, wbase, lane, r);
           __syncwarp();
-          if (lane == 0) arrive(&bar_acc_empty[buf]);
-        }
-        __syncwarp();  // the warp's reads of the previous 32 columns are over
+          if (nan) {
+            nan = false;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<uint4*>(my_row + q * 16) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-        __syncwarp();
-        bool nan = false;
-#pragma unroll
-        for (int q = 0; q < 32; ++q) nan |= __uint_as_float(r[q]) != __uint_as_float(r[q]);
-        for (unsigned todo = __ballot_sync(0xffffffffu, nan && lane < nrows); todo != 0u; todo &= todo - 1u) {
-          const int lr = __ffs(todo) - 1;
-          const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
-          const int32_t* entries = map + static_cast<size_t>(tile) * num_rels * kTM + (warp & 3) * 32 + lr;
-          *reinterpret_cast<float*>(buf0 + ((warp & 3) * 32 + lr) * kOutStride + lane * 4) =
-              row_by_pairs(x, w, entries, num_rels, feat_in, feat_out, c0 + lane);
-          __syncwarp();
+            for (int q = 0; q < 32; ++q) nan |= __uint_as_float(r[q]) != __uint_as_float(r[q]);
+          }
+          for (unsigned todo = __ballot_sync(0xffffffffu, nan && lane < nrows); todo != 0u; todo &= todo - 1u) {
+            const int lr = __ffs(todo) - 1;
+            const int32_t* entries = map + static_cast<size_t>(tile) * num_rels * kTM + (warp & 3) * 32 + lr;
+            stage1(y, wbase, lr, lane, row_by_pairs(x, w, entries, num_rels, feat_in, feat_out, c0 + lane));
+            __syncwarp();
+          }
+          write32(y + static_cast<size_t>(row_base) * feat_out + c0, wbase, nrows, feat_out, lane, add != 0);
         }
-        write32(y, wbase, row_base, nrows, feat_out, c0, lane, add != 0);
       }
     }
   }
@@ -336,27 +429,38 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
   if (warp == 0) tc05::tmem_dealloc(tmem, tmem_cols);
 }
 
-template <typename OutT>
-int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const __half* w, const int32_t* map, int m, int num_rels, int feat_in,
-           int feat_out, int add, cudaStream_t st) {
+template <typename OutT, int TPS>
+int launch_units(const CUtensorMap& tm_w, OutT* y, const __half* x, const __half* w, const int32_t* map, int m, int num_rels,
+                 int feat_in, int feat_out, int add, cudaStream_t st) {
   static thread_local int configured_device = -1;
   int dev = 0;
   SPTIR_CUDA_OK(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    SPTIR_CUDA_OK(cudaFuncSetAttribute(sparse_conv_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    SPTIR_CUDA_OK(cudaFuncSetAttribute(sparse_conv_kernel<OutT, TPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     configured_device = dev;
   }
-  const int stride = kZBytes + ceil_div(feat_out, 64) * kWBox;
+  const int stride = TPS * kZBytes + ceil_div(feat_out, 64) * kWBox;
   const int nstages = std::min(kMaxStages, (kSmemLimit - kOutBytes - 1024) / stride);
   const int smem = nstages * stride + kOutBytes + 1024;
   const int acc_cols = (feat_out + 31) & ~31;
   int tmem_cols = 32;
-  while (tmem_cols < 2 * acc_cols) tmem_cols *= 2;
+  while (tmem_cols < 2 * TPS * acc_cols) tmem_cols *= 2;
   const int grid = std::min(ceil_div(m, kTM), kNumSMs);
-  launch_chained(sparse_conv_kernel<OutT>, grid, kThreads, smem, st, tm_w, y, x, w, map, m, num_rels, feat_in, feat_out,
-                 tmem_cols, acc_cols, nstages, std::min(kGroups, nstages), add);
+  launch_chained(sparse_conv_kernel<OutT, TPS>, grid, kThreads, smem, st, tm_w, y, x, w, map, m, num_rels, feat_in, feat_out,
+                 tmem_cols, acc_cols, nstages, std::min(kGroups / TPS, nstages), add);
   SPTIR_LAUNCH_OK("sparse_conv_kernel");
   return 0;
+}
+
+template <typename OutT>
+int launch(const CUtensorMap& tm_w, OutT* y, const __half* x, const __half* w, const int32_t* map, int m, int num_rels, int feat_in,
+           int feat_out, int add, cudaStream_t st) {
+  // Two tiles side by side, where blocks have more than one and the accumulators fit twice: one slice of W and one round
+  // of the ring for 256 outputs (us, one / two, 27 offsets: 100,000 points 64 -> 32 43.7 / 37.9, 64 -> 128 50.4 / 47.0,
+  // 22,000 points 128 -> 64 31.0 / 28.3; 8 offsets, 40,000 points: 64 -> 64 11.6 / 11.7, 128 -> 128 18.5 / 18.2).
+  if (feat_out <= kMaxOut / 2 && m > kNumSMs * kTM)
+    return launch_units<OutT, 2>(tm_w, y, x, w, map, m, num_rels, feat_in, feat_out, add, st);
+  return launch_units<OutT, 1>(tm_w, y, x, w, map, m, num_rels, feat_in, feat_out, add, st);
 }
 
 }  // namespace

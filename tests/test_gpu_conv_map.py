@@ -46,6 +46,54 @@ def test_matches_a_float64_product(cuda_device, feat_in, feat_out, n_out, offset
     assert L.load().sparsetir_tc_timeouts(cuda_device.index or 0, L.ctypes.byref(count)) == 0 and count.value == 0
 
 
+@pytest.mark.parametrize("feat_in,feat_out", [(64, 128), (48, 96), (16, 32), (64, 160)])
+@pytest.mark.parametrize("n_out", [7, 8, 9, 1185, 18_943, 18_945, 37_889, 60_007])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_shares_of_blocks_and_maps_that_are_not_aligned(cuda_device, feat_in, feat_out, n_out, shift):
+    """Outputs shared among the blocks in octets, one or two tiles a stage; a map whose entries are not 16-byte aligned."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(n_out + feat_in)
+    offsets = 3
+    table = torch.full((-(-n_out // 128) * offsets * 128 + shift,), -1, dtype=torch.int32, device=cuda_device)[shift:]
+    x = torch.rand(500, feat_in, device=cuda_device, generator=g).half() - 0.5
+    w = torch.randn(offsets, feat_in, feat_out, device=cuda_device, generator=g).half() / 8
+    want = torch.zeros(n_out, feat_out, dtype=torch.float64, device=cuda_device)
+    mag = torch.zeros_like(want)
+    for k in range(offsets):
+        src = torch.randint(-300, 500, (n_out,), device=cuda_device, generator=g).clamp(min=-1)
+        at = torch.arange(n_out, device=cuda_device)
+        table[(at // 128 * offsets + k) * 128 + at % 128] = src.int()
+        rows = x.double()[src.clamp(min=0)] * (src >= 0)[:, None]
+        want += rows @ w[k].double()
+        mag += rows.abs() @ w[k].double().abs()
+    y = torch.full((n_out * feat_out + 32,), 3.0, device=cuda_device)
+    ops.sparse_conv_f16(w.view(-1), x.view(-1), y[:n_out * feat_out], table, n_out, offsets, feat_in, feat_out, 0)
+    bound = mag * (offsets * feat_in / 16 + 2) * 2.0 ** -22  # as above
+    assert bool(((y[:-32].view(n_out, feat_out).double() - want).abs() <= bound).all())
+    assert bool((y[-32:] == 3.0).all())
+
+
+@pytest.mark.parametrize("feat_in,feat_out", [(64, 128), (32, 64), (128, 256)])
+def test_the_same_bits_on_every_call(cuda_device, feat_in, feat_out):
+    """Copies of a stage arrive at its barrier by themselves: nothing of a stage may be read before it has landed."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(feat_in)
+    n, offsets = 50_000, 27
+    src = torch.randint(-n // 2, n, (-(-n // 128) * offsets * 128,), device=cuda_device, generator=g).clamp(min=-1).int()
+    x = (torch.randint(-2, 3, (n, feat_in), device=cuda_device, generator=g)).half()
+    w = (torch.randint(-2, 3, (offsets, feat_in, feat_out), device=cuda_device, generator=g)).half()
+    want = torch.zeros(n, feat_out, device=cuda_device)
+    table = src.view(-1, offsets, 128)
+    for k in range(offsets):  # whole numbers below 2^24: exact in any order
+        s = table[:, k].reshape(-1)[:n].long()
+        want += torch.where((s >= 0)[:, None], x[s.clamp(min=0)].float(), 0.0) @ w[k].float()
+    y = torch.empty(n * feat_out, device=cuda_device)
+    for _ in range(30):
+        y.fill_(7.0)
+        ops.sparse_conv_f16(w.view(-1), x.view(-1), y, src, n, offsets, feat_in, feat_out, 0)
+        assert torch.equal(y.view(n, feat_out), want)
+
+
 def test_weights_that_are_not_finite_reach_their_own_pairs_only(cuda_device):
     n, pairs = 300, torch.tensor([[5, 7], [9, 7], [2, 299]])
     x = torch.full((n, 32), 0.5, device=cuda_device).half()
