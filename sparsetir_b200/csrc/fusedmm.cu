@@ -166,16 +166,18 @@ namespace sptir {
 size_t csrmm_scratch(const float* b, const float* c, int m, int n, int feat, int nnz);
 int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices, int m, int n,
               int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats, void* pieces);
+bool softmax_by_blocks(int n, int nnz);  // defined in csr_misc.cu
 namespace {
-// scores and probabilities, and where the pieces of the SpMM may follow them
-size_t stage_bytes(int nnz) { return 2 * static_cast<size_t>(nnz) * sizeof(float); }
-size_t pieces_at(int nnz) { return (stage_bytes(nnz) + 255) & ~static_cast<size_t>(255); }
+// scores and probabilities, the second in place of the first where the softmax can, and where the pieces of the
+// SpMM may follow them
+size_t stage_bytes(int m, int nnz) { return (softmax_by_blocks(m, nnz) ? 1 : 2) * static_cast<size_t>(nnz) * sizeof(float); }
+size_t pieces_at(int m, int nnz) { return (stage_bytes(m, nnz) + 255) & ~static_cast<size_t>(255); }
 }  // namespace
 }  // namespace sptir
 
 extern "C" int sparsetir_fusedmm_workspace(int m, int n, int nnz, int feat, size_t* scratch_bytes, size_t* counter_bytes) {
   if (sparsetir_csrmm_workspace(m, n, feat, nnz, scratch_bytes, counter_bytes) != 0) return -1;
-  if (m > 0 && feat > 0 && nnz > 0) *scratch_bytes += sptir::pieces_at(nnz);
+  if (m > 0 && feat > 0 && nnz > 0) *scratch_bytes += sptir::pieces_at(m, nnz);
   return 0;
 }
 
@@ -221,12 +223,12 @@ extern "C" int sparsetir_fusedmm_raw(const float* q, const float* k, const float
   SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
   const bool eager = capture == cudaStreamCaptureStatusNone;
   const size_t piece_bytes = eager ? csrmm_scratch(v, o, m, n, feat, nnz) : 0;
-  char* ws = static_cast<char*>(workspace(device_id, st, piece_bytes > 0 ? pieces_at(nnz) + piece_bytes : stage_bytes(nnz)));
+  char* ws = static_cast<char*>(workspace(device_id, st, piece_bytes > 0 ? pieces_at(m, nnz) + piece_bytes : stage_bytes(m, nnz)));
   if (!ws) return -1;
   float* scores = reinterpret_cast<float*>(ws);
-  float* probs = scores + nnz;
+  float* probs = softmax_by_blocks(m, nnz) ? scores : scores + nnz;
   if (sparsetir_sddmm_raw(q, k, scores, indptr, indices, nullptr, m, n, feat, nnz, device_id, stream) != 0) return -1;
   if (sparsetir_sparse_softmax_raw(scores, probs, indptr, m, nnz, device_id, stream) != 0) return -1;
   return csrmm_run(probs, v, o, indptr, indices, m, n, feat, nnz, device_id, stream, /*hub_rows=*/true, 0,
-                   piece_bytes > 0 ? ws + pieces_at(nnz) : nullptr);
+                   piece_bytes > 0 ? ws + pieces_at(m, nnz) : nullptr);
 }
