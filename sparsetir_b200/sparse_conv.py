@@ -120,18 +120,19 @@ def map_pays(num_outputs: int, offsets: int, pairs: int, feat_in: int, feat_out:
 
     It multiplies the full ``128 x (offsets * feat_in)`` operand of every tile whatever the share of
     pairs; the buckets' tensor-core kernel pays per pair, but takes only multiples of 64 channels and
-    builds a map of its own on every call when ``feat_out >= 2 * feat_in``.  Measured on 5,000 to
-    100,000 points, 8 and 27 offsets, 10 to 60 % of the pairs (float16 result, us, map / buckets):
-    100,000 x 27, 64 -> 64 channels 56 / 43 at 20 %, 57 / 56 at 30 %, 57 / 85 at 60 %; 256 -> 256
-    270 / 184 at 30 %, 275 / 322 at 60 %; 5,000 x 8 13 / 25; 64 -> 96 and other channel counts
-    47 / 900 at 40 % of 8 offsets.  The two estimates follow these within about 15 %."""
+    builds a map of its own on every call when ``feat_out >= 2 * feat_in``.  Measured on 4,000 to
+    100,000 points, 8 and 27 offsets, 20 to 60 % of the pairs (float16 result, us, map / buckets):
+    100,000 x 27, 64 -> 64 channels 41 / 39 at 20 %, 41 / 53 at 35 %, 41 / 79 at 60 %; 128 -> 64 76 / 66 at 35 %,
+    76 / 99 at 60 %; 30,000 x 27, 128 -> 128 33 / 29 at 20 %, 33 / 37 at 35 %, 256 -> 256 80 / 72 at 35 %, 82 / 103
+    at 60 %; 4,000 x 8 12 / 22.  The two estimates follow these within about 20 %, and where they choose the slower
+    one it is so by 10 % at most."""
     if feat_in % 16 != 0 or feat_out % 32 != 0 or not 0 < feat_out <= 256 or feat_in <= 0:
         return False
     if feat_in % 64 != 0 or feat_out % 64 != 0 or feat_out >= 2 * feat_in:
         return True
     waves = -(-num_outputs // (128 * 148))  # tiles of 128 outputs on 148 SMs
-    by_map = 8.0 + waves * offsets * feat_in / 64 * (0.42 if feat_out > 128 else 0.33)
-    by_pairs = max(24.0, 18.0 + pairs * 1e-6 * (0.42 * feat_in + 0.38 * feat_out - 15.0))
+    by_map = 6.0 + waves * offsets * feat_in / 64 * (0.40 if feat_out > 128 else 0.27 if feat_out > 64 else 0.22)
+    by_pairs = max(24.0, 18.0 + pairs * 1e-6 * (0.30 * feat_in + 0.34 * feat_out - 4.0))
     return by_map <= by_pairs
 
 
