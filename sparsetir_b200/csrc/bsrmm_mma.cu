@@ -32,7 +32,7 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
   const int slab = static_cast<int>(blockIdx.x) % slabs, rest = static_cast<int>(blockIdx.x) / slabs;
   const int part = rest % parts, i = rest / parts;
   const int f0 = slab * mma16::kSlab, row0 = part * 16 * MT;
-  chain_enter();
+  chain_wait();
   const int p0 = __ldg(indptr + i), p1 = __ldg(indptr + i + 1);
   const int per_blk = blk >> 4;  // groups per stored block
   const long long total = static_cast<long long>(p1 - p0) * per_blk;

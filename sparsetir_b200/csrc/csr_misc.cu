@@ -55,7 +55,7 @@ sparse_softmax_kernel(const float* __restrict__ a, float* __restrict__ b,
   const int lane = threadIdx.x % LPR;
   const unsigned mask = group_mask<LPR>();
   const long long row = static_cast<long long>(blockIdx.x) * (kThreads / LPR) + threadIdx.x / LPR;
-  chain_enter();
+  chain_wait();
   if (row >= n) return;
   const int p0 = __ldg(indptr + row), p1 = __ldg(indptr + row + 1);
   float v[CACHE];

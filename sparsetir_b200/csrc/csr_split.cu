@@ -86,7 +86,7 @@ csr_split_kernel(const SplitArgs s) {
   const long long block_entries = static_cast<long long>(SUBS) * s.span;
   const unsigned row_bytes = static_cast<unsigned>(s.feat) * 4u;
   const long long warp_at = blockIdx.x * block_entries + static_cast<long long>((threadIdx.x / 32) * NW) * s.span;
-  chain_enter();
+  chain_wait();
   // The stored entries are those between the first and the last row pointer: of a slice of a larger
   // matrix, or of arrays with room behind, not all nnz.  The two pointers are not waited for: ids and
   // row of the first entry are requested as if they were 0 and nnz, and once more where they are not.

@@ -132,7 +132,7 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const unsigned mask = group_mask<LPR>();
   const long long item = static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR;
   const long long r0l = item * rpi;
-  chain_enter();
+  chain_wait();
   if (!HUBS && r0l >= m) return;
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m)));
   const int nr = min(rpi, m - r0);  // 0 past the last row

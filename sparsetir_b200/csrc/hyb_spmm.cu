@@ -507,7 +507,7 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   auto y_of = [&](int rid) -> char* {
     return cl + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * stride;
   };
-  chain_enter();
+  chain_wait();
 
   if (spr == 1) {
     // ---- narrow bucket: a sub-warp owns rpi whole ELL rows

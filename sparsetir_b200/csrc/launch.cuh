@@ -2,16 +2,19 @@
 //
 // Without it a kernel's blocks are scheduled only when the kernel before has ended and its writes are flushed,
 // one to two microseconds in which the GPU does nothing (calls in a row, us, without / with: CSR SpMM 3,000 rows of 5
-// entries, F = 32, 6.15 / 3.9; BSR 1,024^2, F = 128, 8.2 / 5.5; RGMS of 20,000 edges 19.5 / 14.4; hyb SpMM at F = 32 on
-// 169 k nodes 19.1 / 17.5).  A kernel launched by launch_chained() is scheduled as the blocks of the one before leave
-// their SMs, and calls chain_enter() before its first access to global memory:
-//  - the wait holds every thread until all launches before this one on the stream have ended and their writes are
-//    visible, whoever made them, so that the order of a stream is what it always was;
-//  - the trigger allows the next launch to be scheduled once every block of this one has got that far.  A
-//    block of the next launch that is resident early only waits; no block of this launch is still to be scheduled then,
-//    so it takes nobody's place.
-// Every block of such a kernel must call chain_enter(): a launch that ended without having waited would let the next
-// one pass its wait while the one before is still running.
+// entries, F = 32, 6.15 / 3.5; BSR 1,024^2, F = 128, 8.2 / 5.5; RGMS of 20,000 edges 19.5 / 14.4; hyb SpMM at F = 32 on
+// 169 k nodes 19.1 / 17.4).  A kernel launched by launch_chained() calls chain_wait() before its first access to global
+// memory: every thread waits until all launches before this one on the stream have ended and their writes are visible,
+// whoever made them, so that the order of a stream is what it always was.  It is scheduled when every block of the launch
+// before has ended or called chain_trigger().
+//  - Kernels of many small blocks do not trigger: their ends come close together, and the next launch then finds the SMs
+//    empty.  Scheduled earlier, its blocks fill the SMs that come free first, and a launch of less than a full
+//    wave lies unevenly over them (us, triggered at the start / not: SDDMM 20 k rows, F = 512, 34.8 / 29.0, CSR SpMM
+//    20 k rows, F = 512, 43.3 / 38.8, 4,096 rows 5.1 / 4.5).
+//  - Kernels whose blocks fill an SM each call chain_enter(), which triggers behind the wait, so that the next one's
+//    set-up overlaps: no block of this launch is still to be scheduled then, and a block of the next one only waits.
+// At least one block of every such kernel must have waited when the launch ends, or the next one could pass its wait
+// while the one before is still running; all of them do, but for the gather of rgms_f16.cu.
 #ifndef SPARSETIR_B200_LAUNCH_CUH_
 #define SPARSETIR_B200_LAUNCH_CUH_
 
@@ -28,9 +31,7 @@ __device__ __forceinline__ void chain_enter() {
   chain_trigger();
 }
 
-// Where a call of many stored entries starts (0.3 ms and more), chaining is not worth what it can cost: blocks of the
-// next kernel that become resident early are placed by what the leaving ones make room for, not evenly over the SMs
-// (attention over 20 M positions: 726 us without, 731 with; over 4.5 M: 102 without, 94 with).
+// A call of many stored entries (0.3 ms and more) is launched as usual: a microsecond is nothing to it.
 constexpr int kChainEntries = 8 << 20;
 
 // An error of the launch is the runtime's last error, which SPTIR_LAUNCH_OK reads, as behind <<<>>>.

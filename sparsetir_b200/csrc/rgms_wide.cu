@@ -35,7 +35,7 @@ rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32
   __shared__ __align__(16) float s_w[2][kK][kStride];
   const int tid = threadIdx.x, lane = tid & 31;
   TileWalk tw;
-  chain_enter();
+  chain_wait();
   if (!locate_tile_warp(indptr_i, num_rels, static_cast<int>(blockIdx.x) * tiles_per_block, lane, &tw.rel, &tw.row0,
                         &tw.row1))
     return;  // the same in all warps

@@ -48,7 +48,7 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
   const int sub = wlane / LPR;
   const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
   const long long begin = warp * chunk;
-  chain_enter();
+  chain_wait();
   if (begin >= nnz) return;
   const int e0 = static_cast<int>(begin);
   const int count = static_cast<int>(min(static_cast<long long>(chunk), nnz - begin));
@@ -152,7 +152,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const unsigned mask = group_mask<LPR>();
   const long long warp = static_cast<long long>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32;
   const long long e_begin = warp * chunk;
-  chain_enter();
+  chain_wait();
   if (e_begin >= nnz) return;
   const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + chunk));
   const float* a_lane = a + foff + lane * 8;

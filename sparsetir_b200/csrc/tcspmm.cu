@@ -200,7 +200,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   const int q = lane & 3, r = lane >> 2;
   OutT* c = static_cast<OutT*>(s.c);
   float acc[MT][8][4];
-  chain_enter();
+  chain_wait();
 
   if (unit >= s.windows) {  // ---- a short tile per warp
     const int io = (unit - s.windows) * 4 + warp;
