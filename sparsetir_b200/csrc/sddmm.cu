@@ -33,6 +33,11 @@ constexpr int kThreads = 256;
 // power-law graph, 5 entries per row, F = 64: 66 us when it did).  The feature tiles are walked
 // inside the kernel, the eight sums staying in registers; seven shuffles transpose and add them
 // over eight lanes, one more per doubling of the group adds the rest.
+//
+// What bounds it on short rows is instructions and latency per position (150 instructions of a warp for 8 positions with 16
+// lanes of 16 bytes a row, L1 data path 34 %).  Groups of 8 lanes of 32 bytes have as many bytes in flight and four
+// positions where those had two: power-law graphs, us, before / with them: 169 k rows, F = 64 43.1 / 31.9, 200 k rows
+// F = 192 131 / 102, F = 128 72 / 67, 20 k rows F = 128 10.1 / 8.6.  Groups of 16 such lanes gain nothing (F = 256 137 / 141).
 template <int LPR, int W, int VPL, bool PEERS>
 __global__ void __launch_bounds__(kThreads, 4)
 sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
@@ -42,7 +47,7 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
   using LT = LaneTile<LPR, W, VPL, false>;
   using V = typename LT::Piece;
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int U = VPL * W >= 4 ? 4 : 8;  // positions in flight
+  constexpr int U = W == 8 ? 2 : VPL * W >= 4 ? 4 : 8;  // positions in flight
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const int sub = wlane / LPR;
@@ -329,16 +334,18 @@ size_t l2_budget_bytes() {
 }
 
 // feat is a multiple of 32: the widest tile (32..256 features) that divides feat and whose
-// slice of B (n rows) fits the L2 budget; one launch per tile, in stream order.
+// slice of B (n rows) fits the L2 budget.
+int lean_tile(int n, int feat) {
+  for (int t = 256; t > 32; t /= 2)
+    if (feat % t == 0 && static_cast<size_t>(n) * t * 4 <= l2_budget_bytes()) return t;
+  return 32;
+}
+
+// One launch per tile, in stream order.
 int launch_lean(const float* a, const float* b, float* c, const int32_t* indptr,
                 const int32_t* indices, const float* scale, int m, int n, int feat, int nnz,
                 const PeerOut& po, cudaStream_t stream) {
-  int tile = 32;
-  for (int t = 256; t > 32; t /= 2)
-    if (feat % t == 0 && static_cast<size_t>(n) * t * 4 <= l2_budget_bytes()) {
-      tile = t;
-      break;
-    }
+  const int tile = lean_tile(n, feat);
   for (int foff = 0; foff < feat; foff += tile) {
     int rc;
     const int last = foff + tile >= feat;
@@ -377,9 +384,16 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(nnz) * sizeof(float), st));
     return 0;
   }
-  // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one
-  // (60 k rows, F = 64: 12 entries per row 25.5 against 27.9 us, 28 entries 49 against 54; the
-  // power-law graph of 5 entries per row 54 against 46 us).
+  // The general kernel with groups of 8 lanes of 32 bytes where rows are short, at 64 features whatever the rows, and in
+  // place of several launches of the lean one where B stays in L2 as a whole and rows are not so long that the rows of A
+  // are for nothing (us, lean / general: F = 64 100 k rows of 11 entries 33.6 / 26.2, of 40 95.7 / 77.2, 40 k of 500 375 / 341;
+  // F = 96 100 k of 20 85.6 / 74.9, 40 k of 80 89 / 99; F = 128 in one launch 40 k of 80 94 / 104, in two 100 k of 30
+  // 157 / 109; F = 192 40 k of 30 89 / 62, 150 k of 30 356 / 376; F = 32 40 k of 500 161 / 258).
+  const bool groups = lean && feat >= 64 && po.n == 0;
+  const bool several = feat > lean_tile(n, feat) && static_cast<size_t>(n) * feat * 4 <= (size_t{80} << 20) && nnz / m < 50;
+  if (groups && (nnz / m < 10 || feat == 64 || several))
+    return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one.
   if (lean && nnz / m >= 10) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
   if (feat % 4 == 0 && bits % 16 == 0) {

@@ -178,6 +178,7 @@ template <> struct LaneVec<8> {
   static __device__ __forceinline__ Pack4 ldg(const void* p) { return ldg256(p); }
   static __device__ __forceinline__ void stcs(void* p, const Pack4& v) { stcs256(p, v); }
   static __device__ __forceinline__ void fma(Pack4& acc, float w, const Pack4& x) { fma8(acc, w, x); }
+  static __device__ __forceinline__ float dot(const Pack4& a, const Pack4& b) { return dot8(a, b); }
   static __device__ __forceinline__ void atomic_add(void* p, const Pack4& v) {  // two 16-byte reductions
     float4 lo, hi;
     unpack_pair(v.q[0], lo.x, lo.y); unpack_pair(v.q[1], lo.z, lo.w);

@@ -40,3 +40,10 @@ def test_rows_and_alignments(cuda_device, shape, feat, offset, scaled):
     want, mag = prod.sum(1) * s, prod.abs().sum(1) * s
     # an fp32 sum of feat products in any order and one more product: feat + 1 half-ulps of the magnitudes
     assert bool(((out.double() - want).abs() <= mag * (feat + 2) * 2.0 ** -24).all())
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+@pytest.mark.parametrize("feat,offset", [(96, 0), (128, 0), (160, 0), (192, 0), (256, 0), (128, 8), (160, 8), (64, 8)])
+def test_groups_of_eight_lanes(cuda_device, shape, feat, offset):
+    """Whole and partly filled tiles of 64 features, rows on both sides of where the kernels change hands."""
+    test_rows_and_alignments(cuda_device, shape, feat, offset, True)
