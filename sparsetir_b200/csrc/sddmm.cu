@@ -269,7 +269,7 @@ int launch(const float* a, const float* b, float* c, const int32_t* indptr, cons
   chunk = (chunk + 31) & ~31;
   const int blocks = ceil_div(ceil_div(nnz, chunk), kThreads / 32);
   const float rows_per_entry = static_cast<float>(m) / static_cast<float>(nnz);
-  if constexpr (W == 4) {
+  if constexpr (W >= 4) {
     if (po.n > 0) {
       launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, true>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat,
                      nnz, chunk, rows_per_entry, po);
@@ -389,7 +389,7 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
   // are for nothing (us, lean / general: F = 64 100 k rows of 11 entries 33.6 / 26.2, of 40 95.7 / 77.2, 40 k of 500 375 / 341;
   // F = 96 100 k of 20 85.6 / 74.9, 40 k of 80 89 / 99; F = 128 in one launch 40 k of 80 94 / 104, in two 100 k of 30
   // 157 / 109; F = 192 40 k of 30 89 / 62, 150 k of 30 356 / 376; F = 32 40 k of 500 161 / 258).
-  const bool groups = lean && feat >= 64 && po.n == 0;
+  const bool groups = lean && feat >= 64;
   const bool several = feat > lean_tile(n, feat) && static_cast<size_t>(n) * feat * 4 <= (size_t{80} << 20) && nnz / m < 50;
   if (groups && (nnz / m < 10 || feat == 64 || several))
     return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
