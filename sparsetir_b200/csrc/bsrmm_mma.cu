@@ -24,8 +24,8 @@ constexpr int kThreads = 128;
 
 template <int MT>
 __global__ void __launch_bounds__(kThreads, MT == 1 ? 5 : 3)
-bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, float* __restrict__ c,
-                 const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int blk, int feat,
+bsrmm_mma_kernel(const __half* a, const __half* b, float* __restrict__ c,
+                 const int32_t* indptr, const int32_t* indices, int blk, int feat,
                  int slabs, int parts, int vec_out) {
   __shared__ float s_sum[4][MT][4][8][32];  // [warp][row tile][c][j][lane]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
@@ -33,7 +33,7 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
   const int part = rest % parts, i = rest / parts;
   const int f0 = slab * mma16::kSlab, row0 = part * 16 * MT;
   chain_wait();
-  const int p0 = __ldg(indptr + i), p1 = __ldg(indptr + i + 1);
+  const int p0 = ld_global(indptr + i), p1 = ld_global(indptr + i + 1);
   const int per_blk = blk >> 4;  // groups per stored block
   const long long total = static_cast<long long>(p1 - p0) * per_blk;
   const long long g0 = total * warp / 4, g1 = total * (warp + 1) / 4;
@@ -48,15 +48,15 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       v[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (in) v[k] = __ldg(reinterpret_cast<const uint4*>(p + static_cast<size_t>(k) * feat));
+      if (in) v[k] = ld_global(reinterpret_cast<const uint4*>(p + static_cast<size_t>(k) * feat));
     }
   };
   auto values_of = [&](int p, int kk, uint32_t (&av)[MT][4]) {
     const __half* at = al + static_cast<size_t>(p) * blk * blk + kk * 16;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-      const uint2 lo = __ldg(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16) * blk));
-      const uint2 hi = __ldg(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16 + 8) * blk));
+      const uint2 lo = ld_global(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16) * blk));
+      const uint2 hi = ld_global(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16 + 8) * blk));
       av[mt][0] = lo.x; av[mt][1] = hi.x; av[mt][2] = lo.y; av[mt][3] = hi.y;
     }
   };
@@ -67,7 +67,7 @@ bsrmm_mma_kernel(const __half* __restrict__ a, const __half* __restrict__ b, flo
   };
   int pb = pa, kb = ka;
   next(pb, kb);
-  auto id_of = [&](int p) { return __ldg(indices + min(p, p1 - 1)); };  // past the last block: not used
+  auto id_of = [&](int p) { return ld_global(indices + min(p, p1 - 1)); };  // past the last block: not used
   int ca = 0, cb = 0;
   if (p0 < p1) {
     ca = id_of(pa);

@@ -203,8 +203,8 @@ constexpr int kTmaSmem = kTStages * kStageBytes + 1024;  // + slack to align the
 
 __global__ void __launch_bounds__(kThreads)
 bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                 float* __restrict__ c, const int32_t* __restrict__ indptr,
-                 const int32_t* __restrict__ indices, int feat) {
+                 float* __restrict__ c, const int32_t* indptr,
+                 const int32_t* indices, int feat) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kTStages];   // operands of the stage have landed
   __shared__ __align__(8) uint64_t bar_empty[kTStages];  // the tensor core has read the stage
@@ -214,7 +214,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const int f0 = blockIdx.y * kTileF;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   chain_enter();
-  const int p0 = __ldg(indptr + i), nblk = __ldg(indptr + i + 1) - p0;
+  const int p0 = ld_global(indptr + i), nblk = ld_global(indptr + i + 1) - p0;
 
   float* crow = c + (static_cast<size_t>(i) * kBlk) * feat + f0 + warp * 32 + lane;
   if (nblk <= 0) {  // empty block-row: zeros, no tensor-core work
@@ -248,7 +248,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int cols = 0;
     for (int it = 0; it < nblk; ++it) {
       const int stage = it % kTStages, use = it / kTStages;
-      if ((it & 31) == 0) cols = (it + lane < nblk) ? __ldg(indices + p0 + it + lane) : 0;
+      if ((it & 31) == 0) cols = (it + lane < nblk) ? ld_global(indices + p0 + it + lane) : 0;
       const int col = __shfl_sync(0xffffffffu, cols, it & 31);
       if (use > 0) {
         if (lane == 0) ok = tc05::mbar_wait(&bar_empty[stage], (use - 1) & 1);
@@ -335,8 +335,8 @@ constexpr uint32_t kPAccCols = kPTiles * kBlk;          // 64 TMEM columns per a
 
 __global__ void __launch_bounds__(kPThreads, 2)
 bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                     float* __restrict__ c, const int32_t* __restrict__ indptr,
-                     const int32_t* __restrict__ indices, int feat, int num_items, int items_per_row) {
+                     float* __restrict__ c, const int32_t* indptr,
+                     const int32_t* indices, int feat, int num_items, int items_per_row) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kPStages];   // operands of the stage have landed
   __shared__ __align__(8) uint64_t bar_empty[kPStages];  // the tensor core has read the stage
@@ -373,11 +373,11 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     int bk = 0;  // stored blocks issued so far by this thread block
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       const int i = item / items_per_row, f0 = (item % items_per_row) * (kPTiles * kTileF);
-      const int p0 = __ldg(indptr + i), nblk = __ldg(indptr + i + 1) - p0;
+      const int p0 = ld_global(indptr + i), nblk = ld_global(indptr + i + 1) - p0;
       int cols = 0;
       for (int it = 0; it < nblk; ++it, ++bk) {
         const int stage = bk % kPStages, use = bk / kPStages;
-        if ((it & 31) == 0) cols = (it + lane < nblk) ? __ldg(indices + p0 + it + lane) : 0;
+        if ((it & 31) == 0) cols = (it + lane < nblk) ? ld_global(indices + p0 + it + lane) : 0;
         const int col = __shfl_sync(0xffffffffu, cols, it & 31);
         if (use > 0) {
           if (lane == 0) ok = tc05::mbar_wait(&bar_empty[stage], (use - 1) & 1);
@@ -407,7 +407,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     int bk = 0, acc_it = 0;  // stored blocks / non-empty items so far
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       const int i = item / items_per_row;
-      const int nblk = __ldg(indptr + i + 1) - __ldg(indptr + i);
+      const int nblk = ld_global(indptr + i + 1) - ld_global(indptr + i);
       if (nblk <= 0) continue;
       const int buf = acc_it & 1, buse = acc_it >> 1;
       if (buse > 0) {
@@ -444,7 +444,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     int acc_it = 0;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       const int i = item / items_per_row, f0 = (item % items_per_row) * (kPTiles * kTileF);
-      const int nblk = __ldg(indptr + i + 1) - __ldg(indptr + i);
+      const int nblk = ld_global(indptr + i + 1) - ld_global(indptr + i);
       float* crow = c + (static_cast<size_t>(i) * kBlk) * feat + f0 + q * 32 + lane;
       if (nblk <= 0) {  // empty block-row: zeros, no tensor-core work
 #pragma unroll

@@ -91,15 +91,15 @@ csr_split_kernel(const SplitArgs s) {
   // matrix, or of arrays with room behind, not all nnz.  The two pointers are not waited for: ids and
   // row of the first entry are requested as if they were 0 and nnz, and once more where they are not.
   int lo = 0, hi = s.nnz;
-  const int ptr_first = __ldg(s.indptr), ptr_last = __ldg(s.indptr + s.m);
+  const int ptr_first = ld_global(s.indptr), ptr_last = ld_global(s.indptr + s.m);
   int p0 = 0, count = 0, steps = 0, cid = 0;  // of the sub-warp: first entry, entries; entries of the warp's first sub-warp
   float av = 0.f;
   auto first_ids = [&]() {
     cid = 0;
     av = 0.f;
     if (lane < count) {
-      cid = __ldg(s.indices + p0 + lane);
-      av = __ldg(s.a + p0 + lane);
+      cid = ld_global(s.indices + p0 + lane);
+      av = ld_global(s.a + p0 + lane);
     }
   };
   int first_row = 0;
@@ -122,7 +122,7 @@ csr_split_kernel(const SplitArgs s) {
 #pragma unroll
       for (int i = 1; i < NW; ++i)
         if (wlane / LPR == i) first_row = row[i];
-      first_lead = count > 0 && __ldg(s.indptr + first_row) < p0;
+      first_lead = count > 0 && ld_global(s.indptr + first_row) < p0;
     }
     const int lo_now = max(0, min(ptr_first, s.nnz)), hi_now = max(lo_now, min(ptr_last, s.nnz));
     if (lo == lo_now && hi == hi_now) break;
@@ -164,16 +164,17 @@ csr_split_kernel(const SplitArgs s) {
 #pragma unroll
       for (int v = 0; v < VPL; ++v) acc[v] = LV::zero();
       for (int s0 = 0; s0 < steps; s0 += LPR) {
-        int cidn = 0;
-        float avn = 0.f;
-        if (s0 + LPR + lane < count) {  // ids and values of the next batch
-          cidn = __ldg(s.indices + p0 + s0 + LPR + lane);
-          avn = __ldg(s.a + p0 + s0 + LPR + lane);
-        }
+        int cidn;
+        float avn;
+        auto next_ids = [&]() {  // ids and values of the next batch; past the last one that of the last entry, not added
+          const int at_next = max(p0 + min(s0 + LPR + lane, count - 1), 0);
+          cidn = ld_global(s.indices + at_next);
+          avn = ld_global(s.a + at_next);
+        };
         const int cnt = max(0, min(LPR, count - s0));
         auto rows_of_b = [&](int k0, V (&x)[U][VPL]) {
 #pragma unroll
-          for (int u = 0; u < U; ++u) {  // entries past the end have column 0 and are not added
+          for (int u = 0; u < U; ++u) {  // entries past the end are not added
             const unsigned col = static_cast<unsigned>(__shfl_sync(0xffffffffu, cid, k0 + u, LPR));
             const char* src = bl + static_cast<unsigned long long>(col) * row_bytes;
 #pragma unroll
@@ -182,20 +183,32 @@ csr_split_kernel(const SplitArgs s) {
         };
         // Most batches of a matrix of long rows lie inside one row for every sub-warp of the warp: a loop of
         // their own without tests per entry (10 M entries in rows of 500 on average, F = 128: 322 -> 277 us).
-        if (__all_sync(0xffffffffu, lane != 0 || (cnt == LPR && wend - (p0 + s0) > LPR))) {
+        // Groups of 8 lanes, whose batch is one step, take all that are left of the row in it: one step at a time 9.3 M
+        // entries, F = 32, take 84 us, so 78.6.  Others gain nothing by it (F = 64 135, with the vote once per step 134).
+        const int batches = lane != 0 ? INT32_MAX : min(count - s0, wend - (p0 + s0) - 1) / LPR;  // inside the sub-warp's row
+        int inside_row = LPR == 8 ? __reduce_min_sync(0xffffffffu, batches) : __all_sync(0xffffffffu, batches > 0);
+        if (inside_row > 0) {
           pending = true;
+          while (true) {
 #pragma unroll
-          for (int k0 = 0; k0 < LPR; k0 += U) {
-            V x[U][VPL];
-            rows_of_b(k0, x);
+            for (int k0 = 0; k0 < LPR; k0 += U) {
+              V x[U][VPL];
+              rows_of_b(k0, x);
+              if (k0 == 0) next_ids();
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
+              for (int u = 0; u < U; ++u) {
+                const float ak = __shfl_sync(0xffffffffu, av, k0 + u, LPR);
 #pragma unroll
-              for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
+                for (int v = 0; v < VPL; ++v) LV::fma(acc[v], ak, x[u][v]);
+              }
             }
+            if (LPR != 8 || --inside_row == 0) break;
+            s0 += LPR;
+            cid = cidn;
+            av = avn;
           }
         } else {
+          next_ids();
           const int e = p0 + min(s0 + lane, count - 1);  // lanes past the last entry repeat it
           int row_end;
           const int row = row_in_window<LPR>(s.indptr, s.m, r, wend, e, row_end);
@@ -251,8 +264,8 @@ csr_split_kernel(const SplitArgs s) {
     // ---- rows that cross sub-warps
     auto finish = [&](V (&sum)[VPL], int row, bool from_before, bool goes_on) {
       if (from_before || goes_on) {
-        const int begin = __ldg(s.indptr + row) - s_bounds[0];
-        const int end = min(__ldg(s.indptr + row + 1), s_bounds[1]) - s_bounds[0];
+        const int begin = ld_global(s.indptr + row) - s_bounds[0];
+        const int end = min(ld_global(s.indptr + row + 1), s_bounds[1]) - s_bounds[0];
         const int b0 = static_cast<int>(begin / block_entries), b1 = static_cast<int>((end - 1) / block_entries);
         char* pl = reinterpret_cast<char*>(s.part);
         auto piece = [&](int b) -> char* {
@@ -324,7 +337,7 @@ csr_split_kernel(const SplitArgs s) {
     const long long rb = min(static_cast<long long>(s.m), ra + per);
     for (long long r0 = ra + threadIdx.x - wlane; r0 < rb; r0 += kThreads) {
       const long long rr = r0 + wlane;
-      const bool empty = rr < rb && __ldg(s.indptr + rr) == __ldg(s.indptr + rr + 1);
+      const bool empty = rr < rb && ld_global(s.indptr + rr) == ld_global(s.indptr + rr + 1);
       unsigned todo = __ballot_sync(0xffffffffu, empty);
       while (todo != 0u) {
         const int k = __ffs(todo) - 1;

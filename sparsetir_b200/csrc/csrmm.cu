@@ -41,15 +41,15 @@ constexpr int kLongRow = 64;
 
 // acc += the entries [p0, p1) of a row, taken LPR at a time, `stride` apart
 template <int LPR, int W>
-__device__ __forceinline__ void add_entries(const float* __restrict__ a, const int32_t* __restrict__ indices,
-                                            const char* __restrict__ bl, unsigned row_bytes, int p0, int p1, int stride,
+__device__ __forceinline__ void add_entries(const float* a, const int32_t* indices,
+                                            const char* bl, unsigned row_bytes, int p0, int p1, int stride,
                                             int lane, unsigned mask, typename LaneVec<W>::type& acc) {
   using LV = LaneVec<W>;
   constexpr int U = (32 / W) < LPR ? (32 / W) : LPR;
   for (int e0 = p0; e0 < p1; e0 += stride) {
     const bool live = lane < p1 - e0;
-    const int cid = live ? __ldg(indices + e0 + lane) : 0;
-    const float av = live ? __ldg(a + e0 + lane) : 0.f;
+    const int cid = live ? ld_global(indices + e0 + lane) : 0;
+    const float av = live ? ld_global(a + e0 + lane) : 0.f;
     const int cnt = min(LPR, p1 - e0);
 #pragma unroll
     for (int k0 = 0; k0 < LPR; k0 += U) {
@@ -91,7 +91,7 @@ __device__ __noinline__ void block_with_long_rows(const float* a, const float* b
   auto c_row = [&](int r) -> char* { return cl + static_cast<unsigned long long>(static_cast<unsigned>(r)) * row_bytes; };
   unsigned long_rows = 0;
   for (int j = 0; j < nr; ++j) {
-    const int begin = __ldg(indptr + r0 + j), end = __ldg(indptr + r0 + j + 1);
+    const int begin = ld_global(indptr + r0 + j), end = ld_global(indptr + r0 + j + 1);
     if (end - begin > long_row) {
       long_rows |= 1u << j;
       continue;
@@ -105,7 +105,7 @@ __device__ __noinline__ void block_with_long_rows(const float* a, const float* b
   for (int owner = 0; owner < SUBS; ++owner) {
     for (unsigned todo = s_long[owner]; todo != 0u; todo &= todo - 1u) {
       const int row = static_cast<int>((item0 + owner) * rpi) + __ffs(todo) - 1;
-      const int begin = __ldg(indptr + row), end = __ldg(indptr + row + 1);
+      const int begin = ld_global(indptr + row), end = ld_global(indptr + row + 1);
       typename LV::type acc = LV::zero();
       add_entries<LPR, W>(a, indices, bl, row_bytes, begin + sub * LPR, end, SUBS * LPR, lane, mask, acc);
       LV::sts(&s_part[sub][lane * W], acc);
@@ -121,8 +121,8 @@ __device__ __noinline__ void block_with_long_rows(const float* a, const float* b
 
 template <int LPR, int W, bool HUBS>  // W floats per lane: 4 (16-byte vectors) or 8 (32-byte vectors)
 __global__ void __launch_bounds__(kThreads, 4)
-csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
-                  const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int m,
+csrmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
+                  const int32_t* indptr, const int32_t* indices, int m,
                   int feat, int rpi, int long_row) {
   using LV = LaneVec<W>;
   using V = typename LV::type;
@@ -136,7 +136,7 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   if (!HUBS && r0l >= m) return;
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m)));
   const int nr = min(rpi, m - r0);  // 0 past the last row
-  const int ptr = __ldg(indptr + r0 + min(lane, nr));  // lane j: start of row r0+j (j <= nr)
+  const int ptr = ld_global(indptr + r0 + min(lane, nr));  // lane j: start of row r0+j (j <= nr)
   const unsigned row_bytes = static_cast<unsigned>(feat) * 4u;
   const unsigned off = (blockIdx.y * LPR + lane) * (W * 4u);
   const char* bl = reinterpret_cast<const char*>(b) + off;
@@ -174,15 +174,15 @@ csrmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
     int cid = 0, cidn = 0;
     float av = 0.f, avn = 0.f;
     if (lane < nslots_s) {
-      cid = __ldg(cols_s + lane);
-      av = __ldg(wts_s + lane);
+      cid = ld_global(cols_s + lane);
+      av = ld_global(wts_s + lane);
     }
     for (int s0 = 0; s0 < nslots_s; s0 += LPR) {
       cidn = 0;
       avn = 0.f;
       if (s0 + LPR + lane < nslots_s) {  // ids and values of the next batch
-        cidn = __ldg(cols_s + s0 + LPR + lane);
-        avn = __ldg(wts_s + s0 + LPR + lane);
+        cidn = ld_global(cols_s + s0 + LPR + lane);
+        avn = ld_global(wts_s + s0 + LPR + lane);
       }
       const int cnt = min(LPR, nslots_s - s0);
 #pragma unroll

@@ -76,19 +76,19 @@ __device__ __forceinline__ int find_bucket(const HybTable& tb, int block) {
 }
 
 // A bucket without a row-id array (`rows == nullptr`) writes ELL row r to output row base + r.
-__device__ __forceinline__ int row_id(const int32_t* __restrict__ rows, int r, int base) {
-  return rows != nullptr ? __ldg(rows + r) : base + r;
+__device__ __forceinline__ int row_id(const int32_t* rows, int r, int base) {
+  return rows != nullptr ? ld_global(rows + r) : base + r;
 }
 
-__device__ __forceinline__ bool is_split_row(const int32_t* __restrict__ rows, int r, int nrows,
+__device__ __forceinline__ bool is_split_row(const int32_t* rows, int r, int nrows,
                                              int row) {
   if (rows == nullptr) return false;
-  return (r > 0 && __ldg(rows + r - 1) == row) || (r + 1 < nrows && __ldg(rows + r + 1) == row);
+  return (r > 0 && ld_global(rows + r - 1) == row) || (r + 1 < nrows && ld_global(rows + r + 1) == row);
 }
 
 template <int LPR, int VPL, int VEC>
 __global__ void __launch_bounds__(kThreads, SPTIR_HYB_MIN_BLOCKS)
-hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* __restrict__ b,
+hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* b,
                 float* __restrict__ c, int feat, int all_atomic) {
   using V = typename Vec<VEC>::type;
   constexpr int SUBS = kThreads / LPR;
@@ -125,7 +125,7 @@ hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* __restrict__ b
     first = static_cast<size_t>(r0l) * width + s0;
   }
   const int r0 = static_cast<int>(r0l);
-  const int32_t* __restrict__ rows = tb.rows[q];
+  const int32_t* rows = tb.rows[q];
   for (int j = lane; j < nr + 2; j += LPR) {
     const int idx = r0 - 1 + j;
     s_rows[sub][j] = (idx >= 0 && idx < nrows) ? row_id(rows, idx, tb.row_base[q]) : -1;
@@ -201,9 +201,9 @@ constexpr int kFlagAtomic = static_cast<int>(0x80000000u);  // add atomically in
 // row_flag(g): flag word of ELL row g (called by the lane that will hold it)
 // row_end(acc, flag word): all lanes of the sub-warp, after the last slot of an ELL row
 template <int LPR, int WM, int W, int VPL, bool WHOLE, class RowFlag, class RowEnd>  // WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
-__device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
-                                          const float* __restrict__ wts, int r0, int nr, int nslots,
-                                          int per_row, const char* __restrict__ bl,
+__device__ __forceinline__ void lean_item(const int32_t* cols,
+                                          const float* wts, int r0, int nr, int nslots,
+                                          int per_row, const char* bl,
                                           unsigned row_bytes, const LaneTile<LPR, W, VPL, WHOLE>& lt, int lane,
                                           unsigned mask, RowFlag&& row_flag, RowEnd&& row_end) {
   using LT = LaneTile<LPR, W, VPL, WHOLE>;
@@ -221,8 +221,8 @@ __device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
   int c = 0, rf = 0;
   float a = 0.f;
   if (lane < nslots) {
-    c = __ldg(cols + lane);
-    a = __ldg(wts + lane);
+    c = ld_global(cols + lane);
+    a = ld_global(wts + lane);
   }
   if (WM < 8) {
     if (lane < RPB && lane < nr) rf = row_flag(r0 + lane);   // rows ending in batch 0
@@ -235,8 +235,8 @@ __device__ __forceinline__ void lean_item(const int32_t* __restrict__ cols,
     int cn = 0, rfn = 0;
     float an = 0.f;
     if (s0 + LPR + lane < nslots) {  // ids, weights (and row ids) of the next batch
-      cn = __ldg(cols + s0 + LPR + lane);
-      an = __ldg(wts + s0 + LPR + lane);
+      cn = ld_global(cols + s0 + LPR + lane);
+      an = ld_global(wts + s0 + LPR + lane);
     }
     if (WM < 8 && lane < RPB && (s0 + LPR) / WM + lane < nr) rfn = row_flag(r0 + (s0 + LPR) / WM + lane);
     const int cnt = nslots - s0;  // live slots of this batch if < LPR
@@ -334,7 +334,7 @@ __device__ __forceinline__ unsigned sub_ballot(unsigned mask, bool pred) {
 // ELL-row order; piece k keeps its partial sum in the scratch row of its first ELL row.
 template <int LPR, int W, int VPL, bool WHOLE>
 __device__ __noinline__ void finish_split_row(const LaneTile<LPR, W, VPL, WHOLE> lt, LanePiece<W, VPL> acc,
-                                              const int32_t* __restrict__ rows, int nrows, int g,
+                                              const int32_t* rows, int nrows, int g,
                                               int rpi, int rid, int part_base, char* part, char* c,
                                               unsigned* counters, unsigned row_bytes, int lane,
                                               unsigned mask, const PeerOut* po) {
@@ -343,14 +343,14 @@ __device__ __noinline__ void finish_split_row(const LaneTile<LPR, W, VPL, WHOLE>
   int first = g, last = g;
   while (true) {  // LPR ELL rows per step, backwards then forwards
     const int idx = first - 1 - lane;
-    const unsigned bits = sub_ballot<LPR>(mask, idx >= 0 && __ldg(rows + max(idx, 0)) == rid);
+    const unsigned bits = sub_ballot<LPR>(mask, idx >= 0 && ld_global(rows + max(idx, 0)) == rid);
     const int n = bits == kFull ? LPR : __ffs(~bits) - 1;
     first -= n;
     if (n < LPR) break;
   }
   while (true) {
     const int idx = last + 1 + lane;
-    const unsigned bits = sub_ballot<LPR>(mask, idx < nrows && __ldg(rows + min(idx, nrows - 1)) == rid);
+    const unsigned bits = sub_ballot<LPR>(mask, idx < nrows && ld_global(rows + min(idx, nrows - 1)) == rid);
     const int n = bits == kFull ? LPR : __ffs(~bits) - 1;
     last += n;
     if (n < LPR) break;
@@ -390,7 +390,7 @@ __device__ __noinline__ void finish_split_row(const LaneTile<LPR, W, VPL, WHOLE>
 // pieces of the largest row) were the last 8 us of a 21 us launch.
 template <int LPR, int W, int VPL, bool WHOLE>
 __device__ __noinline__ void finish_split_row_warp(const LaneTile<LPR, W, VPL, WHOLE> lt, LanePiece<W, VPL> acc,
-                                                   const int32_t* __restrict__ rows, int nrows, int g,
+                                                   const int32_t* rows, int nrows, int g,
                                                    int rid, int before, int behind, int part_base,
                                                    char* part, char* c, unsigned* counters,
                                                    unsigned row_bytes, const PeerOut* po) {
@@ -404,14 +404,14 @@ __device__ __noinline__ void finish_split_row_warp(const LaneTile<LPR, W, VPL, W
     const int n = bits == kAll ? 32 : __ffs(~bits) - 1;
     first -= n;
     if (n < 32) break;
-    before = __ldg(rows + max(first - 1 - wlane, 0));
+    before = ld_global(rows + max(first - 1 - wlane, 0));
   }
   while (true) {
     const unsigned bits = __ballot_sync(kAll, last + 1 + wlane < nrows && behind == rid);
     const int n = bits == kAll ? 32 : __ffs(~bits) - 1;
     last += n;
     if (n < 32) break;
-    behind = __ldg(rows + min(last + 1 + wlane, nrows - 1));
+    behind = ld_global(rows + min(last + 1 + wlane, nrows - 1));
   }
   char* dst = c + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes;
   if (first == last) {  // not split after all
@@ -453,10 +453,10 @@ __device__ __noinline__ void finish_split_row_warp(const LaneTile<LPR, W, VPL, W
 // whose last width is small put split rows into a narrow bucket).  Plain loop, one ELL row at a
 // time; consecutive ELL rows of the same output row inside the item are added up first.
 template <int LPR, int W, int VPL, bool WHOLE>
-__device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, const int32_t* __restrict__ cols,
-                                        const float* __restrict__ wts, const int32_t* __restrict__ rows,
+__device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, const int32_t* cols,
+                                        const float* wts, const int32_t* rows,
                                         int nrows, int r0, int nr, int width, int rpi, int part_base,
-                                        const char* __restrict__ b, char* part, char* c,
+                                        const char* b, char* part, char* c,
                                         unsigned* counters, unsigned row_bytes, int lane, unsigned mask,
                                         const PeerOut* po) {
   using LT = LaneTile<LPR, W, VPL, WHOLE>;
@@ -464,14 +464,14 @@ __device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, c
   for (int j = 0; j < nr; ++j) {
     const int g = r0 + j;
     for (int s = 0; s < width; ++s) {
-      const int col = __ldg(cols + j * width + s);
-      const float a = __ldg(wts + j * width + s);
+      const int col = ld_global(cols + j * width + s);
+      const float a = ld_global(wts + j * width + s);
       LT::fma(acc, a, lt.ldg(b + static_cast<unsigned long long>(static_cast<unsigned>(col)) * row_bytes));
     }
-    const int rid = __ldg(rows + g);
-    const bool next_same = g + 1 < nrows && __ldg(rows + g + 1) == rid;
+    const int rid = ld_global(rows + g);
+    const bool next_same = g + 1 < nrows && ld_global(rows + g + 1) == rid;
     if (next_same && j + 1 < nr) continue;  // the next ELL row of this item continues the row
-    if (next_same || (g > 0 && __ldg(rows + g - 1) == rid))
+    if (next_same || (g > 0 && ld_global(rows + g - 1) == rid))
       finish_split_row(lt, acc, rows, nrows, g, rpi, rid, part_base, part, c, counters, row_bytes, lane, mask, po);
     else
       store_out(lt, c + static_cast<unsigned long long>(static_cast<unsigned>(rid)) * row_bytes, acc, po);
@@ -520,7 +520,7 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
     if (!all_atomic && part_base >= 0) {
       // the widest bucket: an item that holds an ELL row of a split row takes the careful path
       bool any = false;
-      for (int j = lane; j < nr; j += LPR) any = any || is_split_row(rows, r0 + j, nrows, __ldg(rows + r0 + j));
+      for (int j = lane; j < nr; j += LPR) any = any || is_split_row(rows, r0 + j, nrows, ld_global(rows + r0 + j));
       if (sub_ballot<LPR>(mask, any) != 0u) {
         split_item(lt, tb.cols[q] + first, tb.w[q] + first, rows, nrows, r0, nr, width, rpi, part_base,
                    bl, pl, cl, la.counters, stride, lane, mask, po);
@@ -559,8 +559,8 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   if (live && part < NW) {
     rid = row_id(rows, r, 0);
     if (by_warp) {
-      before = __ldg(rows + max(r - 1 - static_cast<int>(threadIdx.x & 31), 0));
-      behind = __ldg(rows + min(r + 1 + static_cast<int>(threadIdx.x & 31), nrows - 1));
+      before = ld_global(rows + max(r - 1 - static_cast<int>(threadIdx.x & 31), 0));
+      behind = ld_global(rows + min(r + 1 + static_cast<int>(threadIdx.x & 31), nrows - 1));
     }
   }
   V total = LT::zero();
@@ -605,7 +605,7 @@ struct AsyncSmem {
 
 template <int LPR>
 __global__ void __launch_bounds__(kThreads, 3)
-hyb_spmm_async_kernel(const __grid_constant__ HybTable tb, const float* __restrict__ b,
+hyb_spmm_async_kernel(const __grid_constant__ HybTable tb, const float* b,
                       float* __restrict__ c, int feat, int all_atomic) {
   using S = AsyncSmem<LPR>;
   constexpr int SUBS = S::SUBS, ITEM = S::ITEM;
@@ -643,12 +643,12 @@ hyb_spmm_async_kernel(const __grid_constant__ HybTable tb, const float* __restri
   }
   const int r0 = static_cast<int>(r0l);
   {
-    const int32_t* __restrict__ cols = tb.cols[q] + first;
-    const float* __restrict__ wts = tb.w[q] + first;
-    const int32_t* __restrict__ rows = tb.rows[q];
+    const int32_t* cols = tb.cols[q] + first;
+    const float* wts = tb.w[q] + first;
+    const int32_t* rows = tb.rows[q];
     for (int s = lane; s < nslots; s += LPR) {
-      s_ids[s] = __ldg(cols + s);
-      s_wts[s] = __ldg(wts + s);
+      s_ids[s] = ld_global(cols + s);
+      s_wts[s] = ld_global(wts + s);
     }
     for (int j = lane; j < nr + 2; j += LPR) {
       const int idx = r0 - 1 + j;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(kThreads)
 hyb_rearm_kernel(const __grid_constant__ HybTable tb, float* __restrict__ c, int feat, bool all) {
   const int q = find_bucket(tb, blockIdx.x);
   const int nrows = tb.nrows[q];
-  const int32_t* __restrict__ rows = tb.rows[q];
+  const int32_t* rows = tb.rows[q];
   const long long r = static_cast<long long>(blockIdx.x - tb.block_start[q]) * kThreads + threadIdx.x;
   int row = -1;
   bool clear = false;
@@ -705,7 +705,7 @@ hyb_rearm_kernel(const __grid_constant__ HybTable tb, float* __restrict__ c, int
     row = row_id(rows, static_cast<int>(r), tb.row_base[q]);
     clear = all || tb.chunks_per_row[q] > 1 || is_split_row(rows, static_cast<int>(r), nrows, row);
     // of a run of equal ids only the first ELL row clears
-    if (clear && r > 0 && rows != nullptr && __ldg(rows + r - 1) == row) clear = false;
+    if (clear && r > 0 && rows != nullptr && ld_global(rows + r - 1) == row) clear = false;
   }
   unsigned todo = __ballot_sync(0xffffffffu, clear);
   const int lane = threadIdx.x & 31;

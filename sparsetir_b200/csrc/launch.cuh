@@ -13,6 +13,10 @@
 //    20 k rows, F = 512, 43.3 / 38.8, 4,096 rows 5.1 / 4.5).
 //  - Kernels whose blocks fill an SM each call chain_enter(), which triggers behind the wait, so that the next one's
 //    set-up overlaps: no block of this launch is still to be scheduled then, and a block of the next one only waits.
+// Such a kernel lives while the one before it still writes what it is going to read, so it reads its operands with
+// ld_global().  __ldg(), and what the compiler makes of a const __restrict__ pointer (ld.global.nc), promise that the
+// memory does not change as long as the kernel lives: the load may be moved ahead of the wait, or be answered by
+// what another block of the SM has brought before it.
 // At least one block of every such kernel must have waited when the launch ends, or the next one could pass its wait
 // while the one before is still running; all of them do, but for the gather of rgms_f16.cu.
 #ifndef SPARSETIR_B200_LAUNCH_CUH_
@@ -21,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 
 namespace sptir {
 
@@ -29,6 +34,25 @@ __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.l
 __device__ __forceinline__ void chain_enter() {
   chain_wait();
   chain_trigger();
+}
+
+// Loads of 2, 4, 8 or 16 bytes that stay behind chain_wait().
+template <class T>
+__device__ __forceinline__ T ld_global(const T* p) {
+  T v;
+  if constexpr (sizeof(T) == 16) {
+    uint4& r = reinterpret_cast<uint4&>(v);
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  } else if constexpr (sizeof(T) == 8) {
+    uint2& r = reinterpret_cast<uint2&>(v);
+    asm volatile("ld.global.v2.b32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  } else if constexpr (sizeof(T) == 4) {
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(reinterpret_cast<uint32_t&>(v)) : "l"(p));
+  } else {
+    static_assert(sizeof(T) == 2, "2, 4, 8 or 16 bytes");
+    asm volatile("ld.global.b16 %0, [%1];" : "=h"(reinterpret_cast<uint16_t&>(v)) : "l"(p));
+  }
+  return v;
 }
 
 // A call of many stored entries (0.3 ms and more) is launched as usual: a microsecond is nothing to it.

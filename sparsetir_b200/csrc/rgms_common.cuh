@@ -111,15 +111,15 @@ __device__ __forceinline__ void gather_tile_rows(const float* __restrict__ a,
 constexpr int kTileRows128 = 128;
 
 // Which relation and row range tile `tile_id` covers; called by the 32 lanes of one warp.
-__device__ inline bool locate_tile_warp(const int32_t* __restrict__ indptr_i, int num_rels,
+__device__ inline bool locate_tile_warp(const int32_t* indptr_i, int num_rels,
                                         int tile_id, int lane, int* rel, int* row0, int* row1) {
   int base = 0;
   for (int r0 = 0; r0 < num_rels; r0 += 32) {
     const int r = r0 + lane;
     int s = 0, e = 0, nt = 0;
     if (r < num_rels) {
-      s = __ldg(indptr_i + r);
-      e = __ldg(indptr_i + r + 1);
+      s = ld_global(indptr_i + r);
+      e = ld_global(indptr_i + r + 1);
       nt = (e - s + kTileRows128 - 1) / kTileRows128;
     }
     int incl = nt;
@@ -147,11 +147,11 @@ struct TileWalk {
   int rel, row0, row1, rel_end;  // rel_end: first row past the relation (cached indptr_i[rel + 1])
   // steps to the tile after this one; false when there is none.  Inside a relation this costs no
   // memory access; the row pointer is read again only when the relation changes.
-  __device__ __forceinline__ bool next(const int32_t* __restrict__ indptr_i, int num_rels) {
+  __device__ __forceinline__ bool next(const int32_t* indptr_i, int num_rels) {
     const int nrow0 = row1;
     while (nrow0 >= rel_end) {
       if (++rel >= num_rels) return false;
-      rel_end = __ldg(indptr_i + rel + 1);
+      rel_end = ld_global(indptr_i + rel + 1);
     }
     row0 = nrow0;
     row1 = min(rel_end, nrow0 + kTileRows128);

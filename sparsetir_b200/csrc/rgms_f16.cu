@@ -77,7 +77,7 @@ __device__ __forceinline__ void write_ranges(const BucketTable& tb, int num_rels
     int lo = 0, hi = tb.num_groups[b];  // first group of the bucket with mid >= r
     while (lo < hi) {
       const int m = lo + (hi - lo) / 2;
-      if (__ldg(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
+      if (ld_global(tb.mid[b] + m) < r) lo = m + 1; else hi = m;
     }
     ranges[e] = tb.z_base[b] + lo * tb.rows_per_group[b];
   }
@@ -178,8 +178,8 @@ __device__ __forceinline__ uint4 pack_piece(const float (&acc)[8]) {
 
 // R rows (step apart, from e on) of W >= width slots each; slots past the width are not read
 template <int W, int R>
-__device__ __forceinline__ void gather_few(const __half* __restrict__ a, const int32_t* __restrict__ cols,
-                                           const uint4* __restrict__ x, uint4* __restrict__ z, unsigned e, unsigned step,
+__device__ __forceinline__ void gather_few(const __half* a, const int32_t* cols,
+                                           const uint4* x, uint4* __restrict__ z, unsigned e, unsigned step,
                                            unsigned rows, int width, int chunks) {
   float av[R][W];
   int col[R][W];
@@ -190,14 +190,14 @@ __device__ __forceinline__ void gather_few(const __half* __restrict__ a, const i
       const unsigned row = e + r * step;
       const bool in = row < rows && j < width;
       const size_t at = in ? static_cast<size_t>(row) * width + j : 0;
-      av[r][j] = __half2float(__ldg(a + at));
-      col[r][j] = __ldg(cols + at);
+      av[r][j] = __half2float(ld_global(a + at));
+      col[r][j] = ld_global(cols + at);
     }
   uint4 raw[R][W];
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int j = 0; j < W; ++j) raw[r][j] = __ldg(x + static_cast<size_t>(col[r][j]) * chunks);
+    for (int j = 0; j < W; ++j) raw[r][j] = ld_global(x + static_cast<size_t>(col[r][j]) * chunks);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const unsigned row = e + r * step;
@@ -212,7 +212,7 @@ __device__ __forceinline__ void gather_few(const __half* __restrict__ a, const i
 
 __global__ void __launch_bounds__(kThreads)
 gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
-                        const __half* __restrict__ x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
+                        const __half* x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
                         int32_t* __restrict__ ranges, int num_rels, int chunks, int beside) {
   // beside != 0: the launch before this one, the transform of the one-column rows, neither reads nor writes what
   // this one writes, and its blocks have all passed their own wait when this one is scheduled, so that what lies ahead of
@@ -233,7 +233,7 @@ gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_con
   const int R = rows_in_flight(width);
   const int e0 = (static_cast<int>(blockIdx.x) - gt.first[b]) * (lanes * R);
   for (int i = threadIdx.x; i < lanes * R && i < rows - e0; i += kThreads)
-    all_rows[tb.z_base[b] + e0 + i] = __ldg(tb.rows[b] + e0 + i);
+    all_rows[tb.z_base[b] + e0 + i] = ld_global(tb.rows[b] + e0 + i);
   const unsigned e = static_cast<unsigned>(e0) + rl;
   if (rl >= lanes || e >= static_cast<unsigned>(rows)) return;
   const uint4* xv = reinterpret_cast<const uint4*>(x) + ch;
@@ -250,14 +250,14 @@ gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_con
     uint4 raw[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      av[u] = __half2float(__ldg(ap + j + u));
-      raw[u] = __ldg(xv + static_cast<size_t>(__ldg(cp + j + u)) * chunks);
+      av[u] = __half2float(ld_global(ap + j + u));
+      raw[u] = ld_global(xv + static_cast<size_t>(ld_global(cp + j + u)) * chunks);
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) add_piece(acc, av[u], raw[u]);
   }
   for (; j < width; ++j)
-    add_piece(acc, __half2float(__ldg(ap + j)), __ldg(xv + static_cast<size_t>(__ldg(cp + j)) * chunks));
+    add_piece(acc, __half2float(ld_global(ap + j)), ld_global(xv + static_cast<size_t>(ld_global(cp + j)) * chunks));
   zv[static_cast<size_t>(e) * chunks] = pack_piece(acc);
 }
 
@@ -417,15 +417,15 @@ __device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
 template <typename OutT, bool GATHER>
 __global__ void __launch_bounds__(GATHER ? kTcThreadsG : kTcThreads, 1)
 rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_w,
-                   OutT* __restrict__ y, const int32_t* __restrict__ ranges,
-                   const int32_t* __restrict__ all_rows, int num_ranges, int num_rels, int total_rows,
+                   OutT* __restrict__ y, const int32_t* ranges,
+                   const int32_t* all_rows, int num_ranges, int num_rels, int total_rows,
                    int tiles_per_cta, int feat_in, int feat_out, int tmem_cols,
-                   const __half* __restrict__ x, const int32_t* __restrict__ gcols,
-                   const __half* __restrict__ gvals, const int32_t* __restrict__ run_if_set) {
+                   const __half* x, const int32_t* gcols,
+                   const __half* gvals, const int32_t* run_if_set) {
   // run_if_set != nullptr: this launch is the fall-back of the reduction-free form and runs only
   // when that form found the input unsuitable (flag set on the device)
   if (GATHER) chain_enter();
-  if (run_if_set != nullptr && __ldg(run_if_set) == -1) return;
+  if (run_if_set != nullptr && ld_global(run_if_set) == -1) return;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kStagesH];   // the stage's boxes have landed
   __shared__ __align__(8) uint64_t bar_empty[kStagesH];  // the tensor core has read the stage
@@ -470,7 +470,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     return;
   }
   const uint32_t tmem = s_tmem;
-  TileWalk tw{s_tile[1], s_tile[2], s_tile[3], __ldg(ranges + s_tile[1] + 1)};
+  TileWalk tw{s_tile[1], s_tile[2], s_tile[3], ld_global(ranges + s_tile[1] + 1)};
   bool ok = true;
   int armed = 0;  // producer: stages whose loads have been issued
 
@@ -533,7 +533,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     const int gw = warp - 12;
     int it = 0, pending = -1;
     for (int k = 0; k < tiles_per_cta && ok; ++k) {
-      const int mycol = __ldg(gcols + min(tw.row0 + gw * 32 + lane, total_rows - 1));
+      const int mycol = ld_global(gcols + min(tw.row0 + gw * 32 + lane, total_rows - 1));
       for (int c = 0; c < nkc; ++c, ++it) {
         const int s = it % kStagesH, use = it / kStagesH;
         if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
@@ -577,8 +577,8 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     for (int k = grp; have && k < tiles_per_cta; k += 2) {
       const int buse = k >> 1;
       const int nrows = tw.row1 - tw.row0;
-      const int dst_row = __ldg(all_rows + min(tw.row0 + t, total_rows - 1));
-      const float a_t = GATHER ? __half2float(__ldg(gvals + min(tw.row0 + t, total_rows - 1))) : 1.f;
+      const int dst_row = ld_global(all_rows + min(tw.row0 + t, total_rows - 1));
+      const float a_t = GATHER ? __half2float(ld_global(gvals + min(tw.row0 + t, total_rows - 1))) : 1.f;
       if (!tc05::mbar_wait(&bar_acc_full[grp], buse & 1)) { ok = false; break; }
       tc05::fence_after_sync();
       const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + grp * feat_out;

@@ -267,9 +267,9 @@ __device__ __forceinline__ int swz_off(int row, int kc, int box_bytes) {
 }
 
 __global__ void __launch_bounds__(kPThreads, 1)
-rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restrict__ w,
-                float* __restrict__ y, const int32_t* __restrict__ indptr_i,
-                const int32_t* __restrict__ indices_i, int num_rels, int nnz_i, int tiles_per_cta,
+rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
+                float* __restrict__ y, const int32_t* indptr_i,
+                const int32_t* indices_i, int num_rels, int nnz_i, int tiles_per_cta,
                 int rel_mod) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kZStages];   // z rows of the stage have landed
@@ -315,7 +315,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
     return;
   }
   const uint32_t tmem = s_tmem;
-  TileWalk tw{s_tile[1], s_tile[2], s_tile[3], __ldg(indptr_i + s_tile[1] + 1)};
+  TileWalk tw{s_tile[1], s_tile[2], s_tile[3], ld_global(indptr_i + s_tile[1] + 1)};
   bool ok = true;
   int armed = 0;
 
@@ -382,7 +382,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
         const float4* wr = reinterpret_cast<const float4*>(w + static_cast<size_t>(wrel) * kF * kF);
         for (int ch = ct; ch < kF * kF / 4; ch += 128) {
           const int fo = ch >> 4, kc = ch & 15;
-          const float4 v = __ldg(wr + ch);
+          const float4 v = ld_global(wr + ch);
           const float4 l = make_float4(v.x - tf32_hi(v.x), v.y - tf32_hi(v.y), v.z - tf32_hi(v.z), v.w - tf32_hi(v.w));
           *reinterpret_cast<float4*>(base + kOffW + swz_off(fo, kc, kWBox)) = v;
           *reinterpret_cast<float4*>(base + kOffW + swz_off(kF + fo, kc, kWBox)) = l;
@@ -427,13 +427,13 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* __restric
     bool have = true;
     if (grp == 1) have = tiles_per_cta > 1 && tw.next(indptr_i, num_rels);
     int nrows = tw.row1 - tw.row0;
-    int dst_row = __ldg(indices_i + min(tw.row0 + t, nnz_i - 1));
+    int dst_row = ld_global(indices_i + min(tw.row0 + t, nnz_i - 1));
     for (int k = grp; have && k < tiles_per_cta; k += 2) {
       const int buse = k >> 1;
       // destination rows of this group's next tile (two tiles on): requested now, needed later
       bool has_next = (k + 2 < tiles_per_cta) && tw.next(indptr_i, num_rels);
       has_next = has_next && tw.next(indptr_i, num_rels);
-      const int dst_next = __ldg(indices_i + min(tw.row0 + t, nnz_i - 1));
+      const int dst_next = ld_global(indices_i + min(tw.row0 + t, nnz_i - 1));
       if (!tc05::mbar_wait(&bar_acc_full[grp], buse & 1)) { ok = false; break; }
       tc05::fence_after_sync();
       const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + grp * 2 * kF;

@@ -28,8 +28,8 @@ constexpr int kK = 16;
 constexpr int kStride = kTile + 4;  // padded: the transposed stores of a warp spread over the banks
 
 __global__ void __launch_bounds__(kThreads, 2)
-rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32_t* __restrict__ indptr_i,
-                 const int32_t* __restrict__ indices_i, const float* __restrict__ z, int num_rels, int nnz_i,
+rgms_wide_kernel(const float* w, float* __restrict__ y, const int32_t* indptr_i,
+                 const int32_t* indices_i, const float* z, int num_rels, int nnz_i,
                  int feat, int tiles_per_block) {
   __shared__ __align__(16) float s_z[2][kK][kStride];
   __shared__ __align__(16) float s_w[2][kK][kStride];
@@ -39,7 +39,7 @@ rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32
   if (!locate_tile_warp(indptr_i, num_rels, static_cast<int>(blockIdx.x) * tiles_per_block, lane, &tw.rel, &tw.row0,
                         &tw.row1))
     return;  // the same in all warps
-  tw.rel_end = __ldg(indptr_i + tw.rel + 1);
+  tw.rel_end = ld_global(indptr_i + tw.rel + 1);
   const int o0 = static_cast<int>(blockIdx.y) * kTile;
   const int lr = tid >> 1, lk = (tid & 1) * 8;  // row (and output) of the slice that this thread loads, 8 features
   const int ty = tid >> 4, tx = tid & 15;
@@ -49,8 +49,8 @@ rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32
   auto fetch = [&](const TileWalk& t, int s) {
     const float4* zp = reinterpret_cast<const float4*>(z + static_cast<size_t>(min(t.row0 + lr, nnz_i - 1)) * feat + s * kK + lk);
     const float4* wp = reinterpret_cast<const float4*>(w + (static_cast<size_t>(t.rel) * feat + o0 + lr) * feat + s * kK + lk);
-    nz[0] = __ldg(zp); nz[1] = __ldg(zp + 1);
-    nw[0] = __ldg(wp); nw[1] = __ldg(wp + 1);
+    nz[0] = ld_global(zp); nz[1] = ld_global(zp + 1);
+    nw[0] = ld_global(wp); nw[1] = ld_global(wp + 1);
   };
   auto put = [&](int buf) {
 #pragma unroll
@@ -100,7 +100,7 @@ rgms_wide_kernel(const float* __restrict__ w, float* __restrict__ y, const int32
     for (int i = 0; i < 8; ++i) {
       const int t = (i >> 2) * 64 + ty * 4 + (i & 3);
       if (t < nrows) {
-        float* dst = y + static_cast<size_t>(__ldg(indices_i + tw.row0 + t)) * feat + o0 + tx * 4;
+        float* dst = y + static_cast<size_t>(ld_global(indices_i + tw.row0 + t)) * feat + o0 + tx * 4;
         atomicAdd(reinterpret_cast<float4*>(dst), make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
         atomicAdd(reinterpret_cast<float4*>(dst + 64), make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]));
       }

@@ -9,24 +9,24 @@ namespace sptir {
 
 // row(p) = upper_bound(indptr[0..m], p) - 1, the search of
 // tests/python/sparsetir/sparse_tir_lowered_buffer_scripts.py:530-549 of the reference
-__device__ __forceinline__ int edge_row_search(const int32_t* __restrict__ indptr, int lo_row,
+__device__ __forceinline__ int edge_row_search(const int32_t* indptr, int lo_row,
                                                int m, int p) {
   int low = lo_row, high = m + 1;
   while (low < high) {
     int mid = low + (high - low) / 2;
-    if (__ldg(indptr + mid) > p) high = mid; else low = mid + 1;
+    if (ld_global(indptr + mid) > p) high = mid; else low = mid + 1;
   }
   return low - 1;
 }
 
 // First index of [lo, hi) whose pointer lies behind p, or hi, found by a whole warp: 32-ary steps, every
 // level is one load per lane (4 dependent reads instead of 18 at 2^18 rows).  Reads stay in [lo, hi).
-__device__ __forceinline__ int warp_upper_bound(const int32_t* __restrict__ indptr, int lo, int hi, int p, int wlane) {
+__device__ __forceinline__ int warp_upper_bound(const int32_t* indptr, int lo, int hi, int p, int wlane) {
   while (hi - lo >= 32) {
     const int step = (hi - lo + 31) / 32;
     const long long probe = static_cast<long long>(lo) + static_cast<long long>(wlane + 1) * step;
     const bool in = probe < hi;
-    const bool gt = !in || __ldg(indptr + (in ? probe : 0)) > p;
+    const bool gt = !in || ld_global(indptr + (in ? probe : 0)) > p;
     const int first = __ffs(__ballot_sync(0xffffffffu, gt)) - 1;  // lane 31 probes >= hi: always set
     const int q = lo + (first + 1) * step;
     if (first > 0) lo = q - step + 1;
@@ -34,7 +34,7 @@ __device__ __forceinline__ int warp_upper_bound(const int32_t* __restrict__ indp
   }
   const int idx = lo + wlane;
   const bool in = idx < hi;
-  const bool gt = !in || __ldg(indptr + (in ? idx : 0)) > p;  // lane hi - lo (< 32) has idx == hi
+  const bool gt = !in || ld_global(indptr + (in ? idx : 0)) > p;  // lane hi - lo (< 32) has idx == hi
   return lo + __ffs(__ballot_sync(0xffffffffu, gt)) - 1;
 }
 
@@ -43,7 +43,7 @@ __device__ __forceinline__ int warp_upper_bound(const int32_t* __restrict__ indp
 // bracket.  Two or three memory round trips where the rows are
 // roughly equally long in the large, four or five for any other matrix of 2^18 rows (a binary
 // search: 18).  Every read stays inside indptr whatever p says.
-__device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ indptr, int m, int p,
+__device__ __forceinline__ int warp_row_of(const int32_t* indptr, int m, int p,
                                            float rows_per_entry, int wlane) {
   int lo = 0, hi = m + 1;  // the answer + 1: first index whose pointer lies behind p
   if (m >= 64) {
@@ -51,7 +51,7 @@ __device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ indptr, i
     const long long at = wlane < 16 ? static_cast<long long>(guess) - (16ll << (15 - wlane))
                                     : static_cast<long long>(guess) + (16ll << (wlane - 16));
     const bool in = at >= 0 && at <= m;
-    const bool gt = at > m || (in && __ldg(indptr + (in ? at : 0)) > p);
+    const bool gt = at > m || (in && ld_global(indptr + (in ? at : 0)) > p);
     const unsigned bits = __ballot_sync(0xffffffffu, gt);
     const int first = bits != 0u ? __ffs(bits) - 1 : 32;
     const int idx = static_cast<int>(max(-1ll, min(at, static_cast<long long>(m) + 1)));
@@ -66,7 +66,7 @@ __device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ indptr, i
 // counting the row ends among the next 128 rows that lie at or before them (by a search each where
 // the rows are so short, or empty, that 128 of them end before the last position).
 template <int N>
-__device__ __forceinline__ void warp_rows_of(const int32_t* __restrict__ indptr, int m,
+__device__ __forceinline__ void warp_rows_of(const int32_t* indptr, int m,
                                              const int (&p)[N], float rows_per_entry, int wlane,
                                              int (&row)[N]) {
   row[0] = warp_row_of(indptr, m, p[0], rows_per_entry, wlane);
@@ -74,7 +74,7 @@ __device__ __forceinline__ void warp_rows_of(const int32_t* __restrict__ indptr,
     constexpr int kWin = 4;
     int end[kWin];
 #pragma unroll
-    for (int k = 0; k < kWin; ++k) end[k] = __ldg(indptr + min(row[0] + 1 + k * 32 + wlane, m));
+    for (int k = 0; k < kWin; ++k) end[k] = ld_global(indptr + min(row[0] + 1 + k * 32 + wlane, m));
     if (__shfl_sync(0xffffffffu, end[kWin - 1], 31) > p[N - 1]) {
 #pragma unroll
       for (int i = 1; i < N; ++i) {
@@ -96,11 +96,11 @@ __device__ __forceinline__ void warp_rows_of(const int32_t* __restrict__ indptr,
 // with log2(LPR) + 1 shuffles and no memory access as long as the row lies in the window (always,
 // unless rows are empty).  All 32 lanes of the warp take part, every group for itself.
 template <int LPR>
-__device__ __forceinline__ int row_window(const int32_t* __restrict__ indptr, int m, int r, int lane) {
-  return __ldg(indptr + min(r + 1 + lane, m));
+__device__ __forceinline__ int row_window(const int32_t* indptr, int m, int r, int lane) {
+  return ld_global(indptr + min(r + 1 + lane, m));
 }
 template <int LPR>
-__device__ __forceinline__ int row_in_window(const int32_t* __restrict__ indptr, int m, int r, int wend,
+__device__ __forceinline__ int row_in_window(const int32_t* indptr, int m, int r, int wend,
                                              int e, int& row_end) {
   int pos = 0;
 #pragma unroll
@@ -110,7 +110,7 @@ __device__ __forceinline__ int row_in_window(const int32_t* __restrict__ indptr,
   int row = r + pos;
   if (row_end <= e) {  // past the window (empty rows): search the rest
     row = min(m - 1, edge_row_search(indptr, min(row, m), m, e));
-    row_end = __ldg(indptr + row + 1);
+    row_end = ld_global(indptr + row + 1);
   }
   return row;
 }

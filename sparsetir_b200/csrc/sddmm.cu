@@ -40,14 +40,14 @@ constexpr int kThreads = 256;
 // F = 192 131 / 102, F = 128 72 / 67, 20 k rows F = 128 10.1 / 8.6.  Groups of 16 such lanes gain nothing (F = 256 137 / 141).
 template <int LPR, int W, int VPL, bool PEERS>
 __global__ void __launch_bounds__(kThreads, 4)
-sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
-             const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-             const float* __restrict__ scale, int m, int feat, int nnz, int chunk, float rows_per_entry,
+sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
+             const int32_t* indptr, const int32_t* indices,
+             const float* scale, int m, int feat, int nnz, int chunk, float rows_per_entry,
              const __grid_constant__ PeerOut po) {
   using LT = LaneTile<LPR, W, VPL, false>;
   using V = typename LT::Piece;
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int U = W == 8 ? 2 : VPL * W >= 4 ? 4 : 8;  // positions in flight
+  constexpr int U = W == 8 || VPL == 4 ? 2 : VPL * W >= 4 ? 4 : 8;  // positions in flight; four of four single floats spill
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const int sub = wlane / LPR;
@@ -62,15 +62,15 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
   const char* bb = reinterpret_cast<const char*>(b);
   const int tiles = (feat + LT::kFloats - 1) / LT::kFloats;
 
-  int col = wlane < count ? __ldg(indices + e0 + wlane) : 0;
+  int col = wlane < count ? ld_global(indices + e0 + wlane) : 0;
   int r = warp_row_of(indptr, m, e0, rows_per_entry, wlane);
   int wend = row_window<32>(indptr, m, r, wlane);
   for (int s0 = 0; s0 < count; s0 += 32) {
     const bool live = wlane < count - s0;
     const int e = e0 + min(s0 + wlane, count - 1);  // lanes past the last position repeat its row
     int col_next = 0;
-    if (s0 + 32 + wlane < count) col_next = __ldg(indices + e0 + s0 + 32 + wlane);
-    const float mul = live && scale != nullptr ? __ldg(scale + e) : 1.f;
+    if (s0 + 32 + wlane < count) col_next = ld_global(indices + e0 + s0 + 32 + wlane);
+    const float mul = live && scale != nullptr ? ld_global(scale + e) : 1.f;
     int row_end;
     const int row = row_in_window<32>(indptr, m, r, wend, e, row_end);
     r = __shfl_sync(kAll, row, 31);
@@ -147,9 +147,9 @@ sddmm_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __
 // into the peers' copies of c: 128 contiguous bytes per warp and peer, over NVLink.
 template <int LPR, bool PEERS>
 __global__ void __launch_bounds__(kThreads, LPR <= 8 ? 4 : 2)
-sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
-                  const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-                  const float* __restrict__ scale, int m, int nnz, int ld, int foff, int accumulate,
+sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
+                  const int32_t* indptr, const int32_t* indices,
+                  const float* scale, int m, int nnz, int ld, int foff, int accumulate,
                   int chunk, int last_tile, const __grid_constant__ PeerOut po) {
   constexpr int U = LPR < 4 ? LPR : 4;  // gathered rows in flight per lane (8 registers each)
   const int wlane = threadIdx.x & 31;
@@ -164,19 +164,19 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
   const float* b_lane = b + foff + lane * 8;
 
   int warp_row = max(0, min(m - 1, warp_upper_bound(indptr, 0, m + 1, static_cast<int>(e_begin), wlane) - 1));
-  int warp_end = __ldg(indptr + warp_row + 1);  // first position past the warp's current row
+  int warp_end = ld_global(indptr + warp_row + 1);  // first position past the warp's current row
   int cur_row = -1;
   Pack4 arow = pack4_zero();
 
-  int col_next = (static_cast<int>(e_begin) + wlane < e_end) ? __ldg(indices + e_begin + wlane) : 0;
+  int col_next = (static_cast<int>(e_begin) + wlane < e_end) ? ld_global(indices + e_begin + wlane) : 0;
   for (int base = static_cast<int>(e_begin); base < e_end; base += 32) {
     const int e = base + wlane;
     const bool live = e < e_end;
     const int col = col_next;
-    if (e + 32 < e_end) col_next = __ldg(indices + e + 32);
+    if (e + 32 < e_end) col_next = ld_global(indices + e + 32);
     float mul = 1.f, old = 0.f;
     if (live) {
-      if (scale != nullptr) mul = __ldg(scale + e);
+      if (scale != nullptr) mul = ld_global(scale + e);
       if (accumulate) old = c[e];
     }
     float part[LPR];
@@ -200,7 +200,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
       if (live) {
         int steps = 0;
         // row < m - 1 keeps every read inside indptr even if nnz disagrees with indptr[m]
-        while (row < m - 1 && __ldg(indptr + row + 1) <= e) {
+        while (row < m - 1 && ld_global(indptr + row + 1) <= e) {
           ++row;
           if (++steps == 8) {  // long run of empty rows: finish with a search
             row = min(m - 1, edge_row_search(indptr, row, m, e));
@@ -210,7 +210,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
       }
       // the next batch starts from the row of this batch's last live position
       warp_row = __shfl_sync(0xffffffffu, row, min(31, e_end - 1 - base));
-      warp_end = __ldg(indptr + warp_row + 1);
+      warp_end = ld_global(indptr + warp_row + 1);
 #pragma unroll
       for (int k0 = 0; k0 < LPR; k0 += U) {
         Pack4 x[U];
@@ -254,7 +254,7 @@ sddmm_lean_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
 }
 
 __global__ void __launch_bounds__(kThreads)
-edge_to_row_kernel(const int32_t* __restrict__ indptr, int32_t* __restrict__ mid, int m, int nnz) {
+edge_to_row_kernel(const int32_t* indptr, int32_t* __restrict__ mid, int m, int nnz) {
   const long long p = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
   if (p < nnz) mid[p] = edge_row_search(indptr, 0, m, static_cast<int>(p));
 }

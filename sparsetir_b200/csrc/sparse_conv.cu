@@ -160,18 +160,18 @@ __device__ __forceinline__ void write32(__half* y, const unsigned char* wbase, i
 // One row's 32 outputs from its pairs alone, lane = output.  A row without a pair of some offset takes
 // part in that offset's product with zeros, and 0 * W is NaN where W is not finite: rows that came
 // out with a NaN are formed again here, from the terms of the sum and no others.
-__device__ __noinline__ float row_by_pairs(const __half* __restrict__ x, const __half* __restrict__ w,
-                                           const int32_t* __restrict__ entries, int num_rels, int feat_in,
+__device__ __noinline__ float row_by_pairs(const __half* x, const __half* w,
+                                           const int32_t* entries, int num_rels, int feat_in,
                                            int feat_out, int col) {
   float sum = 0.f;
   for (int rel = 0; rel < num_rels; ++rel) {
-    const int e = __ldg(entries + static_cast<size_t>(rel) * kTM);
+    const int e = ld_global(entries + static_cast<size_t>(rel) * kTM);
     if (e < 0) continue;
     const __half* xr = x + static_cast<size_t>(e) * feat_in;
     const __half* wr = w + static_cast<size_t>(rel) * feat_in * feat_out + col;
 #pragma unroll 8
     for (int fi = 0; fi < feat_in; ++fi)
-      sum = fmaf(__half2float(__ldg(xr + fi)), __half2float(__ldg(wr + static_cast<size_t>(fi) * feat_out)), sum);
+      sum = fmaf(__half2float(ld_global(xr + fi)), __half2float(ld_global(wr + static_cast<size_t>(fi) * feat_out)), sum);
   }
   return sum;
 }
@@ -202,8 +202,8 @@ __device__ __forceinline__ void copy_rows(uint32_t at0, uint32_t at1, const int 
 
 template <typename OutT, int TPS>
 __global__ void __launch_bounds__(kThreads, 1)
-sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ y, const __half* __restrict__ x,
-                   const __half* __restrict__ w, const int32_t* __restrict__ map, int m, int num_rels, int feat_in,
+sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ y, const __half* x,
+                   const __half* w, const int32_t* map, int m, int num_rels, int feat_in,
                    int feat_out, int tmem_cols, int acc_cols, int nstages, int slots, int add) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];   // both operands of the stage are there
@@ -344,7 +344,7 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
       none = in ? 0 : 1;
       const int32_t* e = in ? mp + static_cast<size_t>(rel) * kTM : map;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) entry[i] = __ldg(e + 4 * i);
+      for (int i = 0; i < 8; ++i) entry[i] = ld_global(e + 4 * i);
     };
     // the lane's rows of the tile are 4 apart: two places in an atom of 8 swizzled rows, atoms 1024 bytes apart
     const int r4 = lane >> 3;

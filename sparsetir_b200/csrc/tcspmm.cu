@@ -142,24 +142,24 @@ __device__ __forceinline__ bool accumulate(const TcArgs& s, int g0, int g1, int 
   const __half* bl = s.b + (in ? f0 + r * 8 : 0);
   auto ids_of = [&](int g) {
     const int32_t* p = s.indices + static_cast<size_t>(g) * kG + q * 4;
-    if (s.vec_indices) return __ldg(reinterpret_cast<const int4*>(p));
-    return make_int4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+    if (s.vec_indices) return ld_global(reinterpret_cast<const int4*>(p));
+    return make_int4(ld_global(p), ld_global(p + 1), ld_global(p + 2), ld_global(p + 3));
   };
   auto rows_of = [&](const int4& id, uint4 (&v)[4]) {
     const int row[4] = {id.x, id.y, id.z, id.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       v[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (in) v[k] = __ldg(reinterpret_cast<const uint4*>(bl + static_cast<size_t>(row[k]) * s.feat));
+      if (in) v[k] = ld_global(reinterpret_cast<const uint4*>(bl + static_cast<size_t>(row[k]) * s.feat));
     }
   };
   auto values_of = [&](int g, uint32_t (&av)[MT][4]) {
     const __half* p = s.a + (static_cast<size_t>(g) * s.t + r) * kG + q * 4;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-      const uint2 lo = __ldg(reinterpret_cast<const uint2*>(p + mt * 16 * kG));
+      const uint2 lo = ld_global(reinterpret_cast<const uint2*>(p + mt * 16 * kG));
       uint2 hi = make_uint2(0u, 0u);
-      if (s.t >= 16) hi = __ldg(reinterpret_cast<const uint2*>(p + (mt * 16 + 8) * kG));
+      if (s.t >= 16) hi = ld_global(reinterpret_cast<const uint2*>(p + (mt * 16 + 8) * kG));
       av[mt][0] = lo.x; av[mt][1] = hi.x; av[mt][2] = lo.y; av[mt][3] = hi.y;
     }
   };
@@ -205,7 +205,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   if (unit >= s.windows) {  // ---- a short tile per warp
     const int io = (unit - s.windows) * 4 + warp;
     if (io >= s.mb) return;
-    const int g0 = __ldg(s.indptr + io), g1 = __ldg(s.indptr + io + 1);
+    const int g0 = ld_global(s.indptr + io), g1 = ld_global(s.indptr + io + 1);
     if (g1 - g0 > kLight) return;
     const bool nan = accumulate<MT>(s, g0, g1, f0, lane, acc);
 #pragma unroll
@@ -241,7 +241,7 @@ tcspmm_mma_kernel(const __grid_constant__ TcArgs s) {
   const int w0 = unit << s.window_log, w1 = w0 + min(1 << s.window_log, s.nnzb - w0);
   int cur = warp_row_of(s.indptr, s.mb, w0, s.tiles_per_group, lane);
   while (cur < s.mb) {
-    const int start = __ldg(s.indptr + min(cur + lane, s.mb)), end = __ldg(s.indptr + min(cur + lane + 1, s.mb));
+    const int start = ld_global(s.indptr + min(cur + lane, s.mb)), end = ld_global(s.indptr + min(cur + lane + 1, s.mb));
     unsigned todo = __ballot_sync(0xffffffffu, end - start > kLight && start < w1 && end > w0);
     while (todo != 0u) {  // the same in all four warps
       const int k = __ffs(todo) - 1;

@@ -1,4 +1,4 @@
-// Small helpers shared by the SIMT kernels: 1- or 4-wide feature vectors, read-only loads,
+// Small helpers shared by the SIMT kernels: 1- or 4-wide feature vectors, loads of operands,
 // sub-warp shuffles with the sub-warp's own participation mask.
 #ifndef SPARSETIR_B200_VEC_CUH_
 #define SPARSETIR_B200_VEC_CUH_
@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdlib>
+
+#include "launch.cuh"
 
 namespace sptir {
 
@@ -56,10 +58,10 @@ __device__ __forceinline__ Pack4 pack4_zero() {
   r.q[0] = r.q[1] = r.q[2] = r.q[3] = 0ull;
   return r;
 }
-// read-only 32-byte load; the address must be 32-byte aligned
+// 32-byte load of an operand (ld_global); the address must be 32-byte aligned
 __device__ __forceinline__ Pack4 ldg256(const void* p) {
   Pack4 r;
-  asm volatile("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];"
                : "=l"(r.q[0]), "=l"(r.q[1]), "=l"(r.q[2]), "=l"(r.q[3])
                : "l"(p));
   return r;
@@ -103,7 +105,7 @@ template <int W> struct LaneVec;
 template <> struct LaneVec<1> {
   using type = float;
   static __device__ __forceinline__ float zero() { return 0.f; }
-  static __device__ __forceinline__ float ldg(const void* p) { return __ldg(reinterpret_cast<const float*>(p)); }
+  static __device__ __forceinline__ float ldg(const void* p) { return ld_global(reinterpret_cast<const float*>(p)); }
   static __device__ __forceinline__ void stcs(void* p, float v) { __stcs(reinterpret_cast<float*>(p), v); }
   static __device__ __forceinline__ void fma(float& acc, float w, float x) { acc = fmaf(w, x, acc); }
   static __device__ __forceinline__ void atomic_add(void* p, float v) { atomicAdd(reinterpret_cast<float*>(p), v); }
@@ -125,7 +127,7 @@ template <> struct LaneVec<1> {
 template <> struct LaneVec<2> {
   using type = float2;
   static __device__ __forceinline__ float2 zero() { return make_float2(0.f, 0.f); }
-  static __device__ __forceinline__ float2 ldg(const void* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+  static __device__ __forceinline__ float2 ldg(const void* p) { return ld_global(reinterpret_cast<const float2*>(p)); }
   static __device__ __forceinline__ void stcs(void* p, const float2& v) { __stcs(reinterpret_cast<float2*>(p), v); }
   static __device__ __forceinline__ void fma(float2& acc, float w, const float2& x) {
     acc.x = fmaf(w, x.x, acc.x); acc.y = fmaf(w, x.y, acc.y);
@@ -149,7 +151,7 @@ template <> struct LaneVec<2> {
 template <> struct LaneVec<4> {
   using type = float4;
   static __device__ __forceinline__ float4 zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-  static __device__ __forceinline__ float4 ldg(const void* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+  static __device__ __forceinline__ float4 ldg(const void* p) { return ld_global(reinterpret_cast<const float4*>(p)); }
   static __device__ __forceinline__ void stcs(void* p, const float4& v) { __stcs(reinterpret_cast<float4*>(p), v); }
   static __device__ __forceinline__ void fma(float4& acc, float w, const float4& x) { Vec<4>::fma(acc, w, x); }
   static __device__ __forceinline__ void atomic_add(void* p, const float4& v) { atomicAdd(reinterpret_cast<float4*>(p), v); }
