@@ -213,7 +213,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const int i = blockIdx.x;
   const int f0 = blockIdx.y * kTileF;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  chain_enter();
+  chain_wait();
   const int p0 = ld_global(indptr + i), nblk = ld_global(indptr + i + 1) - p0;
 
   float* crow = c + (static_cast<size_t>(i) * kBlk) * feat + f0 + warp * 32 + lane;
@@ -360,9 +360,10 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     tc05::prefetch_tensormap(&tm_b);
   }
   if (warp == 0) tc05::tmem_alloc(&s_tmem, 2 * kPAccCols);
-  chain_enter();
+  chain_wait();
   tc05::fence_before_sync();
   __syncthreads();
+  chain_trigger();
   tc05::fence_after_sync();
   const uint32_t tmem = s_tmem;
   bool ok = true;

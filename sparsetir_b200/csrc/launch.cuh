@@ -11,8 +11,11 @@
 //    empty.  Scheduled earlier, its blocks fill the SMs that come free first, and a launch of less than a full
 //    wave lies unevenly over them (us, triggered at the start / not: SDDMM 20 k rows, F = 512, 34.8 / 29.0, CSR SpMM
 //    20 k rows, F = 512, 43.3 / 38.8, 4,096 rows 5.1 / 4.5).
-//  - Kernels whose blocks fill an SM each call chain_enter(), which triggers behind the wait, so that the next one's
-//    set-up overlaps: no block of this launch is still to be scheduled then, and a block of the next one only waits.
+//  - Kernels of one wave of blocks, one or two to an SM, trigger behind the wait, so that the next one's set-up overlaps:
+//    no block of this launch is still to be scheduled then, and a block of the next one only waits.
+//  - A kernel that takes tensor memory triggers when its block has it (behind the barrier that publishes the address).
+//    The next launch may take some before it waits, and would keep it until this one has ended: a block of this one that
+//    had yet to take its own on the same SM would wait for it for good.
 // Such a kernel lives while the one before it still writes what it is going to read, so it reads its operands with
 // ld_global().  __ldg(), and what the compiler makes of a const __restrict__ pointer (ld.global.nc), promise that the
 // memory does not change as long as the kernel lives: the load may be moved ahead of the wait, or be answered by

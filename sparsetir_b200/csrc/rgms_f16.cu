@@ -424,8 +424,10 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
                    const __half* gvals, const int32_t* run_if_set) {
   // run_if_set != nullptr: this launch is the fall-back of the reduction-free form and runs only
   // when that form found the input unsuitable (flag set on the device)
-  if (GATHER) chain_enter();
-  if (run_if_set != nullptr && ld_global(run_if_set) == -1) return;
+  if (run_if_set != nullptr) {
+    chain_wait();
+    if (ld_global(run_if_set) == -1) return;
+  }
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kStagesH];   // the stage's boxes have landed
   __shared__ __align__(8) uint64_t bar_empty[kStagesH];  // the tensor core has read the stage
@@ -454,7 +456,9 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, tmem_cols);
   }
-  if (!GATHER) chain_enter();
+  __syncthreads();  // the block has its tensor memory
+  chain_wait();
+  chain_trigger();
   if (warp == 0) {
     int rel, row0, row1;
     const bool found = locate_tile_warp(ranges, num_ranges, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);

@@ -299,7 +299,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, kPTmem);
   }
-  chain_enter();
+  chain_wait();
   if (warp == 0) {
     int rel, row0, row1;
     const bool found = locate_tile_warp(indptr_i, num_rels, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
@@ -309,6 +309,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
   }
   tc05::fence_before_sync();
   __syncthreads();
+  chain_trigger();
   tc05::fence_after_sync();
   if (s_tile[0] == 0) {  // no tile for this block (uniform)
     if (warp == 0) tc05::tmem_dealloc(s_tmem, kPTmem);

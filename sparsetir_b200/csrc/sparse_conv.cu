@@ -239,9 +239,10 @@ sparse_conv_kernel(const __grid_constant__ CUtensorMap tm_w, OutT* __restrict__ 
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, tmem_cols);
   }
-  chain_enter();
+  chain_wait();
   tc05::fence_before_sync();
   __syncthreads();
+  chain_trigger();
   tc05::fence_after_sync();
   const uint32_t tmem = s_tmem;
   bool ok = true;

@@ -74,3 +74,15 @@ def test_operands_are_read_behind_the_wait(kernel):
     for file, name, params, body in reached:
         for what in (r"__ldg\w*\(", r"ld\.global\.nc", r"const [\w:<>\s]+\*\s*__restrict__"):
             assert not re.search(what, params + body), f"{file}: {name}, which {kernel} calls, has {what}"
+
+
+def test_tensor_memory_is_taken_before_the_next_launch_may_take_it():
+    """A block of the next launch takes its tensor memory and then waits for this launch to end: every block of this one
+    has to have its own by then."""
+    with_tmem = [k for k in LAUNCHED if "tmem_alloc(" in _kernel(k)[3]]
+    assert len(with_tmem) >= 5
+    for kernel in with_tmem:
+        body = _kernel(kernel)[3]
+        taken = body.index("__syncthreads()", body.index("tmem_alloc("))  # the block has it behind this barrier
+        early = body.find("chain_enter("), body.find("chain_trigger(")
+        assert all(at < 0 or at > taken for at in early), kernel
