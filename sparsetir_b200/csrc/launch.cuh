@@ -21,7 +21,9 @@
 // memory does not change as long as the kernel lives: the load may be moved ahead of the wait, or be answered by
 // what another block of the SM has brought before it.
 // At least one block of every such kernel must have waited when the launch ends, or the next one could pass its wait
-// while the one before is still running; all of them do, but for the gather of rgms_f16.cu.
+// while the one before is still running.  All blocks of all of them do, but for the gather of rgms_f16.cu, which runs
+// beside the launch before it: there a flag, set by that launch behind its own wait (st_release) and read by this one
+// (ld_acquire), stands for the wait, and one block waits in the end.
 #ifndef SPARSETIR_B200_LAUNCH_CUH_
 #define SPARSETIR_B200_LAUNCH_CUH_
 
@@ -55,6 +57,16 @@ __device__ __forceinline__ T ld_global(const T* p) {
     static_assert(sizeof(T) == 2, "2, 4, 8 or 16 bytes");
     asm volatile("ld.global.b16 %0, [%1];" : "=h"(reinterpret_cast<uint16_t&>(v)) : "l"(p));
   }
+  return v;
+}
+
+// A flag between launches that run side by side: what happened before it was set is visible to who has read it.
+__device__ __forceinline__ void st_release(int32_t* p, int32_t v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int32_t ld_acquire(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 

@@ -213,16 +213,17 @@ __device__ __forceinline__ void gather_few(const __half* a, const int32_t* cols,
 __global__ void __launch_bounds__(kThreads)
 gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
                         const __half* x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
-                        int32_t* __restrict__ ranges, int num_rels, int chunks, int beside) {
-  // beside != 0: the launch before this one, the transform of the one-column rows, neither reads nor writes what
-  // this one writes, and its blocks have all passed their own wait when this one is scheduled, so that what lies ahead of
-  // both has ended: the gather runs beside it, in the registers that it leaves.  One block waits for it in the end,
-  // so that this launch has not ended before it.
-  if (beside == 0) chain_wait();
+                        int32_t* __restrict__ ranges, int num_rels, int chunks, const int32_t* passed) {
+  // passed != nullptr: the launch before this one, the transform of the one-column rows, neither reads nor writes what
+  // this one writes, and the gather runs beside it, in the registers that it leaves.  The transform sets *passed behind
+  // its own wait, so that a block which finds it set sees all that lies ahead of both as one that has waited; a block
+  // which does not find it set waits.  One block waits for the transform in the end, so that this launch has not
+  // ended before it.
+  if (passed == nullptr || ld_acquire(passed) == 0) chain_wait();
   chain_trigger();
   if (blockIdx.x == gridDim.x - 1) {
     write_ranges(tb, num_rels, ranges);
-    if (beside != 0) chain_wait();
+    chain_wait();
     return;
   }
   const int lanes = kThreads / chunks;  // rows side by side
@@ -421,7 +422,8 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
                    const int32_t* all_rows, int num_ranges, int num_rels, int total_rows,
                    int tiles_per_cta, int feat_in, int feat_out, int tmem_cols,
                    const __half* x, const int32_t* gcols,
-                   const __half* gvals, const int32_t* run_if_set) {
+                   const __half* gvals, const int32_t* run_if_set, int32_t* passed) {
+  // passed != nullptr: set to 1 as soon as what lies ahead of this launch has ended, for the launch that runs beside it.
   // run_if_set != nullptr: this launch is the fall-back of the reduction-free form and runs only
   // when that form found the input unsuitable (flag set on the device)
   if (run_if_set != nullptr) {
@@ -456,8 +458,9 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, tmem_cols);
   }
-  __syncthreads();  // the block has its tensor memory
   chain_wait();
+  if (passed != nullptr && blockIdx.x == 0 && tid == 0) st_release(passed, 1);
+  __syncthreads();  // the block has its tensor memory, and the flag is set
   chain_trigger();
   if (warp == 0) {
     int rel, row0, row1;
@@ -879,10 +882,11 @@ int rgms_f16_timeouts(unsigned int* count) {
 
 namespace {
 
-// ranges[b * R + r] for every bucket (what the last block of the gather launches computes)
+// ranges[b * R + r] for every bucket (what the last block of the gather launches computes); *passed is cleared
 __global__ void __launch_bounds__(kThreads)
-bucket_ranges_kernel(const __grid_constant__ BucketTable tb, int num_rels, int32_t* __restrict__ ranges) {
+bucket_ranges_kernel(const __grid_constant__ BucketTable tb, int num_rels, int32_t* __restrict__ ranges, int32_t* passed) {
   chain_enter();
+  if (passed != nullptr && threadIdx.x == 0) *passed = 0;
   write_ranges(tb, num_rels, ranges);
 }
 
@@ -892,7 +896,7 @@ template <typename OutT, bool GATHER>
 int launch_tc(const __half* z, const __half* w, OutT* y, const int32_t* ranges, const int32_t* all_rows,
               int num_ranges, int num_rels, int total_rows, int feat_in, int feat_out, cudaStream_t st,
               const __half* x = nullptr, const int32_t* gcols = nullptr, const __half* gvals = nullptr,
-              const int32_t* run_if_set = nullptr) {
+              const int32_t* run_if_set = nullptr, int32_t* passed = nullptr) {
   CUtensorMap tm_z, tm_w;
   if (make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w, static_cast<uint64_t>(feat_out),
                    static_cast<uint64_t>(num_rels) * feat_in, static_cast<uint64_t>(feat_out) * 2, 64, kKC,
@@ -919,7 +923,7 @@ int launch_tc(const __half* z, const __half* w, OutT* y, const int32_t* ranges, 
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
   launch_chained(rgms_f16_tc_kernel<OutT, GATHER>, static_cast<unsigned>(grid), GATHER ? kTcThreadsG : kTcThreads, kSmemH, st,
                  tm_z, tm_w, y, ranges, all_rows, num_ranges, num_rels, total_rows, tiles_per_cta, feat_in, feat_out,
-                 tmem_cols, x, gcols, gvals, run_if_set);
+                 tmem_cols, x, gcols, gvals, run_if_set, passed);
   SPTIR_LAUNCH_OK("rgms_f16_tc_kernel");
   return 0;
 }
@@ -998,10 +1002,11 @@ int single_column_bucket(const BucketTable& tb) {
   return tb.nb > 1 ? best : -1;
 }
 
-// The two launches over Z, ws: z_bytes() of scratch.  beside: the launch ahead is the transform of the one-column rows.
+// The two launches over Z, ws: z_bytes() of scratch.  passed: set by the launch ahead, the transform of the one-column rows,
+// beside which the gather may run; nullptr: there is none.
 template <typename OutT>
 int run_z(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int num_rels, int feat_in, int feat_out,
-          int path, char* ws, int beside, cudaStream_t st) {
+          int path, char* ws, const int32_t* passed, cudaStream_t st) {
   const int total = tb.z_base[tb.nb];
   const int num_ranges = tb.nb * num_rels;
   const size_t zb = z_part(tb, feat_in), rb = range_part(tb, num_rels);
@@ -1027,7 +1032,7 @@ int run_z(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int 
       tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
     }
     launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(tiles + 1), kThreads, 0, st, tb, gt, x, z, all_rows, ranges,
-                   num_rels, feat_in / 8, beside);
+                   num_rels, feat_in / 8, passed);
   } else if (vec)
     gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
   else
@@ -1090,7 +1095,7 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
     int32_t* ranges1 = reinterpret_cast<int32_t*>(ws1);
     int32_t* flag = reinterpret_cast<int32_t*>(ws1 + rb1);
     int32_t* map = reinterpret_cast<int32_t*>(ws1 + rb1 + 256);
-    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, tb, num_rels, ranges1);
+    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, tb, num_rels, ranges1, nullptr);
     SPTIR_LAUNCH_OK("bucket_ranges_kernel");
     int rc = 1;
     if (try_os) {
@@ -1114,20 +1119,21 @@ int run(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int m,
   const int single = tc_shape && path == 0 && aligned16(x) ? single_column_bucket(tb) : -1;
   if (single >= 0) {
     const BucketTable one = only_bucket(tb, single), rest = without_bucket(tb, single);
-    const size_t rb1 = (static_cast<size_t>(num_rels + 1) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
+    const size_t rb1 = (static_cast<size_t>(num_rels + 2) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
     char* ws1 = static_cast<char*>(workspace(device_id, st, rb1 + z_bytes(rest, num_rels, feat_in)));
     if (!ws1) return -1;
     int32_t* ranges1 = reinterpret_cast<int32_t*>(ws1);
-    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, one, num_rels, ranges1);
+    int32_t* passed = ranges1 + num_rels + 1;
+    launch_chained(bucket_ranges_kernel, 1, kThreads, 0, st, one, num_rels, ranges1, passed);
     SPTIR_LAUNCH_OK("bucket_ranges_kernel");
     const int rc = launch_tc<OutT, true>(nullptr, w, y, ranges1, one.rows[0], num_rels, num_rels, one.z_base[1], feat_in,
-                                         feat_out, st, x, one.cols[0], one.a[0]);
+                                         feat_out, st, x, one.cols[0], one.a[0], nullptr, passed);
     if (rc < 0) return rc;
-    if (rc == 0) return run_z<OutT>(rest, w, x, y, num_rels, feat_in, feat_out, path, ws1 + rb1, 1, st);
+    if (rc == 0) return run_z<OutT>(rest, w, x, y, num_rels, feat_in, feat_out, path, ws1 + rb1, passed, st);
   }
   char* ws = static_cast<char*>(workspace(device_id, st, z_bytes(tb, num_rels, feat_in)));
   if (!ws) return -1;
-  return run_z<OutT>(tb, w, x, y, num_rels, feat_in, feat_out, path, ws, 0, st);
+  return run_z<OutT>(tb, w, x, y, num_rels, feat_in, feat_out, path, ws, nullptr, st);
 }
 
 }  // namespace

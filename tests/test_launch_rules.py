@@ -86,3 +86,19 @@ def test_tensor_memory_is_taken_before_the_next_launch_may_take_it():
         taken = body.index("__syncthreads()", body.index("tmem_alloc("))  # the block has it behind this barrier
         early = body.find("chain_enter("), body.find("chain_trigger(")
         assert all(at < 0 or at > taken for at in early), kernel
+
+
+@pytest.mark.parametrize("kernel", LAUNCHED)
+def test_every_block_waits_or_has_seen_a_flag(kernel):
+    """The first thing that touches memory is the wait, or the flag of a launch that has waited."""
+    body = _kernel(kernel)[3]
+    waits = [m.start() for m in re.finditer(r"\bchain_(?:wait|enter)\(", body)]
+    read = body.find("ld_global(")
+    assert read < 0 or waits[0] < read, f"{kernel} reads before it waits"
+    depth = lambda at: body.count("{", 0, at) - body.count("}", 0, at)  # noqa: E731
+    statement = lambda at: body[max(body.rfind(c, 0, at) for c in ";{}") + 1:at].strip()  # noqa: E731
+    plain = [at for at in waits if depth(at) == 1 and statement(at) == ""]
+    flagged = [at for at in waits if depth(at) == 1 and re.fullmatch(r"if \(\w+ == nullptr \|\| ld_acquire\(\w+\) == 0\)", statement(at))]
+    assert plain or flagged, f"{kernel} waits only under a condition"
+    if not plain:  # then one block has to wait before the launch ends
+        assert any(depth(at) > 1 and statement(at) == "" for at in waits), kernel
