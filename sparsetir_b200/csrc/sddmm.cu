@@ -341,6 +341,27 @@ int lean_tile(int n, int feat) {
   return 32;
 }
 
+// Whether a call of whole 32-feature tiles takes the general kernel in groups of 8 lanes of 32 bytes.  It reads the
+// whole row of B and of A at every position, so it wants B in L2 as a whole, where the lean kernel needs a slice of it
+// and keeps the row of A.  All figures: us, lean / groups, of 60 matrices of equal and of log-normal rows.
+//  - Rows of less than 10 entries: always (power-law graphs, the header of sddmm_kernel).
+//  - 64 features in one launch of the lean one: 100 k rows of 20 entries 52 / 44, of 100 191 / 181, of 200 358 / 358,
+//    40 k of 500 336 / 348.
+//  - In place of several launches: rows of up to 50 entries (F = 96: 40 k of 30 46 / 38, of 80 86 / 96; F = 64: 233 k of 50
+//    248 / 235, of 80 349 / 363, of 500 1734 / 2241), and B up to a share of the L2 budget that grows with the launches
+//    saved: F = 512, two, 20 k of 30 87 / 77, 30 k 136 / 141; F = 256, two, 50 k of 30 109 / 103, 80 k 182 / 225; F = 96,
+//    three narrow ones, 100 k of 30 108 / 99, 150 k 162 / 167, 200 k 219 / 270; F = 64, two, 200 k of 30 147 / 121, 300 k
+//    of 45 at 0.91; F = 128, two, 150 k of 30 226 / 203, 200 k 291 / 318; F = 192, three, 80 k of 30 178 / 137.  At 192
+//    features and a B of 31 MB the groups are the faster ones at any length (40 k rows of 80 185 / 148, of 500 1097 / 895): not taken.
+bool in_groups(int m, int n, int feat, int nnz) {
+  const int per_row = nnz / m, tile = lean_tile(n, feat);
+  if (feat < 64) return false;
+  if (per_row < 10) return true;
+  if (feat == tile) return feat == 64 && per_row < 200;
+  const int eighths = tile == 256 || feat == 96 ? 8 : tile == 128 ? 9 : feat == 64 ? 11 : 13;
+  return per_row < (feat == 64 ? 64 : 50) && static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes() / 8 * eighths;
+}
+
 // One launch per tile, in stream order.
 int launch_lean(const float* a, const float* b, float* c, const int32_t* indptr,
                 const int32_t* indices, const float* scale, int m, int n, int feat, int nnz,
@@ -384,15 +405,7 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(nnz) * sizeof(float), st));
     return 0;
   }
-  // The general kernel with groups of 8 lanes of 32 bytes where rows are short, at 64 features whatever the rows, and in
-  // place of several launches of the lean one where B stays in L2 as a whole and rows are not so long that the rows of A
-  // are for nothing (us, lean / general: F = 64 100 k rows of 11 entries 33.6 / 26.2, of 40 95.7 / 77.2, 40 k of 500 375 / 341;
-  // F = 96 100 k of 20 85.6 / 74.9, 40 k of 80 89 / 99; F = 128 in one launch 40 k of 80 94 / 104, in two 100 k of 30
-  // 157 / 109; F = 192 40 k of 30 89 / 62, 150 k of 30 356 / 376; F = 32 40 k of 500 161 / 258).
-  const bool groups = lean && feat >= 64;
-  const bool several = feat > lean_tile(n, feat) && static_cast<size_t>(n) * feat * 4 <= (size_t{80} << 20) && nnz / m < 50;
-  if (groups && (nnz / m < 10 || feat == 64 || several))
-    return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  if (lean && in_groups(m, n, feat, nnz)) return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one.
   if (lean && nnz / m >= 10) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);

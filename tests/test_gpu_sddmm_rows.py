@@ -47,3 +47,25 @@ def test_rows_and_alignments(cuda_device, shape, feat, offset, scaled):
 def test_groups_of_eight_lanes(cuda_device, shape, feat, offset):
     """Whole and partly filled tiles of 64 features, rows on both sides of where the kernels change hands."""
     test_rows_and_alignments(cuda_device, shape, feat, offset, True)
+
+
+@pytest.mark.parametrize("n,feat,per_row", [(300_000, 64, 100), (150_000, 96, 20), (80_000, 256, 20), (40_000, 512, 20)])
+def test_operands_beyond_l2_are_taken_in_slices(cuda_device, n, feat, per_row):
+    """Where the rows of B do not stay in L2 as a whole, a call is a launch per slice of them.  It shows in the
+    rounding: the products of the first slice sum to 1 and those of a later one to half an ulp of it in 4 lanes' parts, which are
+    added up before they meet the 1; a kernel that walks whole rows adds them to the 1 part by part, and loses them."""
+    rows = 300
+    tile = 32
+    while tile < 256 and feat % (2 * tile) == 0 and n * 2 * tile * 4 <= 48 << 20:
+        tile *= 2
+    assert tile < feat
+    b = torch.zeros(n, feat, device=cuda_device)
+    b[:, 0] = 1.0
+    parts = tile // 8  # 8 features to a lane
+    b[:, tile:2 * tile:8] = 2.0 ** -23 / parts
+    a = torch.ones(rows * feat, device=cuda_device)
+    ptr = torch.arange(0, rows * per_row + 1, per_row, dtype=torch.int32, device=cuda_device)
+    cols = torch.randint(0, n, (rows * per_row,), device=cuda_device, dtype=torch.int32)
+    out = torch.empty(rows * per_row, device=cuda_device)
+    ops.sddmm(a, b.view(-1), out, ptr, cols)
+    assert bool((out == 1.0 + 2.0 ** -23).all())
