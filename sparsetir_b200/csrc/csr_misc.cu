@@ -108,13 +108,17 @@ sparse_softmax_kernel(const float* a, float* b,
   beyond([&](int e, float x) { to[e] = expf(x - mx) * scale; });
 }
 
-// Rows of any length, a block per 8 of them.  A warp takes a row of up to 32 * kCache entries, which stay in its
-// registers between the three passes; longer rows wait until the block's short ones are done and are then shared by its
+// Rows of any length, a block per 8 of them.  A warp takes a row of up to kWarpRow entries, 32 * kCache of which stay in
+// its registers between the three passes; longer rows wait until the block's other ones are done and are then shared by its
 // eight warps, 256 * kCache entries in registers.  Bound: instructions, about 20 per 32 entries.  So addresses are a
 // pointer and a constant, and the entries are taken kBatch to a thread, of which those behind the row's end are skipped
-// by all.  20 M entries in 40 k rows of 245 in the median and 10,000 at most: 62 us; a warp that walks its row alone, with
-// the launch as long as the longest row: 78.  Smaller matrices keep that form (softmax_by_blocks).
+// by all.  20 M entries in 40 k rows of 245 in the median and 10,000 at most: 64 us; a warp that walks its row alone, with
+// the launch as long as the longest row: 79.  Smaller matrices keep that form (softmax_by_blocks).
+// Eight rows that are all shared are taken one after the other, two barriers each, so a row is shared only where a warp
+// alone would be the launch's tail (us, a warp per row at any length / shared from 512 / 2048 / 4096 entries on: 13 M entries in rows
+// of 600 29 / 58 / 27 / 27, of 1,000 27 / 45 / 25 / 25, of 2,000 28 / 39 / 34 / 29; 20 M as above 79 / 66 / 64 / 76).
 // b may be a: an entry is read for the last time by the thread that then writes it.
+constexpr int kWarpRow = 2048;
 constexpr int kCache = 16, kBatch = 4;
 
 // Maximum, sum and store over the entries a[0], a[STRIDE], ... of which the thread has those below `left` (the
@@ -206,7 +210,7 @@ sparse_softmax_rows_kernel(const float* a, float* b, const int32_t* indptr, int 
     p0 = ld_global(indptr + row);
     len = ld_global(indptr + row + 1) - p0;
   }
-  const bool is_long = len > 32 * kCache;
+  const bool is_long = len > kWarpRow;
   if (!is_long && len > 0)
     softmax_row<32>(a + p0 + lane, b + p0 + lane, len - lane, len, [](float v) { return group_max<32>(v, 0xffffffffu); },
                     [](float v) { return group_sum<32>(v, 0xffffffffu); });

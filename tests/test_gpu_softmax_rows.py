@@ -83,3 +83,23 @@ def test_attention_with_the_scores_in_place(cuda_device):
     ops.sparse_softmax(s, p, ptr.int(), cols)
     ops.csrmm(p, v, want, ptr.int(), cols)
     assert torch.equal(o, want)
+
+
+@pytest.mark.parametrize("length", [600, 1000, 2000])
+def test_rows_of_some_hundred_entries_are_not_shared(cuda_device, length):
+    """Rows that a warp takes in a few steps: shared by a block, a matrix of them took twice as long.  It shows in the
+    rounding: behind the row's largest value, whose exponential is 1, a thread adds values of just less than half an ulp of 1,
+    and loses them; a thread of a warp has eight times as many of the row's values as one of a block."""
+    n = (12 << 20) // length + 1
+    ptr = torch.arange(0, (n + 1) * length, length, dtype=torch.int32, device=cuda_device)
+    small = -16.66  # exp: 0.98 * 2^-24
+    a = torch.full((n, length), small, device=cuda_device)
+    a[:, 0] = 0.0
+    got = torch.empty(n * length, device=cuda_device)
+    ops.sparse_softmax(a.view(-1), got, ptr, torch.zeros(n * length, dtype=torch.int32, device=cuda_device))
+    lost = -(-length // 32) - 1  # the others of the first thread
+    term = torch.exp(torch.tensor(small, dtype=torch.float32).double())
+    want = 1.0 / (1.0 + (length - 1 - lost) * term)
+    # the other sums and the division round by 2^-24 of 1 a few times; of a block's threads the first would lose an
+    # eighth of this, and the result be lower by the rest, 0.8 * lost * 2^-24 and more
+    assert float((got.view(n, length)[:, 0].double() - want).abs().max()) < 0.3 * lost * 2.0 ** -24
