@@ -50,7 +50,8 @@ def test_matches_a_float64_product(cuda_device, feat_in, feat_out, n_out, offset
 @pytest.mark.parametrize("n_out", [7, 8, 9, 1185, 18_943, 18_945, 37_889, 60_007])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_shares_of_blocks_and_maps_that_are_not_aligned(cuda_device, feat_in, feat_out, n_out, shift):
-    """Outputs shared among the blocks in octets, one or two tiles a stage; a map whose entries are not 16-byte aligned."""
+    """Tiles of a few rows, blocks with one tile and with two side by side, an odd one left over; a map whose entries are not
+    16-byte aligned."""
     g = torch.Generator(device=cuda_device)
     g.manual_seed(n_out + feat_in)
     offsets = 3
@@ -92,6 +93,29 @@ def test_the_same_bits_on_every_call(cuda_device, feat_in, feat_out):
         y.fill_(7.0)
         ops.sparse_conv_f16(w.view(-1), x.view(-1), y, src, n, offsets, feat_in, feat_out, 0)
         assert torch.equal(y.view(n, feat_out), want)
+
+
+@pytest.mark.parametrize("feat_in,feat_out", [(64, 128), (48, 96), (16, 32), (64, 160)])
+@pytest.mark.parametrize("n_out", [5, 18_943, 18_945, 37_889, 60_007])
+@pytest.mark.parametrize("dtype,add", [(torch.float16, 0), (torch.float16, 1), (torch.float32, 1)])
+def test_two_tiles_a_stage_in_both_types_and_added(cuda_device, feat_in, feat_out, n_out, dtype, add):
+    """The forms of the test above with a float16 result and with addition into the output: whole numbers, exact in both."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(n_out + feat_in)
+    offsets = 3
+    table = torch.full((-(-n_out // 128) * offsets * 128,), -1, dtype=torch.int32, device=cuda_device)
+    x = torch.randint(-1, 2, (500, feat_in), device=cuda_device, generator=g).half()
+    w = torch.randint(-1, 2, (offsets, feat_in, feat_out), device=cuda_device, generator=g).half()
+    y = torch.randint(-5, 6, (n_out * feat_out + 32,), device=cuda_device, generator=g).to(dtype)
+    want = y[:-32].view(n_out, feat_out).double() * add
+    for k in range(offsets):
+        src = torch.randint(-300, 500, (n_out,), device=cuda_device, generator=g).clamp(min=-1)
+        at = torch.arange(n_out, device=cuda_device)
+        table[(at // 128 * offsets + k) * 128 + at % 128] = src.int()
+        want += (x.double()[src.clamp(min=0)] * (src >= 0)[:, None]) @ w[k].double()
+    behind = y[-32:].clone()
+    ops.sparse_conv_f16(w.view(-1), x.view(-1), y[:n_out * feat_out], table, n_out, offsets, feat_in, feat_out, add)
+    assert torch.equal(y[:-32].view(n_out, feat_out).double(), want) and torch.equal(y[-32:], behind)
 
 
 def test_weights_that_are_not_finite_reach_their_own_pairs_only(cuda_device):

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 SINGLE = 96 << 10  # rows from which the one-column bucket gets launches of its own
 
 
-def _layer(device, widths, rows, group, rels, n, m, fi, fo, seed):
+def _layer(device, widths, rows, group, rels, n, m, fi, fo, seed, top=2):
     g = torch.Generator(device=device)
     g.manual_seed(seed)
     pick = lambda lo, hi, *shape: torch.randint(lo, hi, shape, device=device, generator=g)  # noqa: E731
@@ -23,8 +23,8 @@ def _layer(device, widths, rows, group, rels, n, m, fi, fo, seed):
         vals = (pick(0, 4, groups * group, width).float() / 2).half()  # zeros among them
         mid = torch.sort(pick(0, rels, groups))[0].int()
         buckets.append((vals.view(-1), pick(0, m, groups * group).int(), pick(0, n, groups * group * width).int(), mid))
-    x = pick(-2, 3, n, fi).half()
-    w = pick(-2, 3, rels, fi, fo).half()
+    x = pick(-top, top + 1, n, fi).half()
+    w = pick(-top, top + 1, rels, fi, fo).half()
     want = torch.zeros(m, fo, dtype=torch.float64, device=device)
     for width, (vals, to, cols, mid) in zip(widths, buckets):
         z = (vals.view(-1, width, 1).double() * x[cols.long()].view(-1, width, fi).double()).sum(1)
@@ -48,6 +48,18 @@ def test_exact_sums(cuda_device, widths, rows, group, fi, fo):
     assert torch.equal(y.double(), want + 2.0)
     count = ctypes.c_uint(0)
     assert L.load().sparsetir_tc_timeouts(cuda_device.index or 0, ctypes.byref(count)) == 0 and count.value == 0
+
+
+@pytest.mark.parametrize("widths,rows,group", [((1, 2), (SINGLE, 500), 32), ((4, 1, 2), (1000, SINGLE + 37, 3000), 1), ((1, 1), (SINGLE, SINGLE + 128), 128)])
+@pytest.mark.parametrize("fi,fo", [(64, 64), (128, 64), (64, 192), (64, 32)])
+def test_exact_sums_in_float16(cuda_device, widths, rows, group, fi, fo):
+    """The result in half precision: multiples of a half below 1024, which every order of addition keeps."""
+    n, m, rels = 700, 40_000, 7
+    buckets, x, w, want = _layer(cuda_device, widths, rows, group, rels, n, m, fi, fo, len(widths) + fi + fo, top=1)
+    assert float(want.abs().max()) < 500
+    y = torch.full((m, fo), 2.0, device=cuda_device, dtype=torch.float16)
+    ops.rgms_ell3d_f16(*ops.rgms_ell3d_f16_args(w.view(-1), x.view(-1), y.view(-1), buckets, fi, fo))
+    assert torch.equal(y.double(), want + 2.0)
 
 
 def test_calls_in_a_row_and_in_a_graph(cuda_device):
