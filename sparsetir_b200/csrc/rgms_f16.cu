@@ -155,8 +155,12 @@ gather_rows_f16_kernel(const __grid_constant__ BucketTable tb, const __half* __r
 // after the other the chain ids -> X row was waited for once per row (1.5 M edges, 1.2 M rows of 64
 // features: the call 122 -> 105 us).  Bound: the L2 gather of X and the write of Z.
 struct GatherTiles {
-  int32_t first[kMaxBuckets + 1];  // first tile of every bucket
+  int32_t first[kMaxBuckets + 1];  // first tile of every bucket; [nb] = all tiles
 };
+// Tiles from which a block that runs beside the transform takes two: the flag is read once for both.  Below, the last
+// wave of blocks weighs more (us, one / two, tiles: 46 relations, 1.5 M edges 64 -> 64, 4,600, 87.4 / 83.2; 128 -> 128, 9,200,
+// 152 / 146; 30 relations, 600 k edges 128 -> 128, 3,750, 74.3 / 71.6; 64 -> 64, 1,880, 41.5 / 43.1).
+constexpr int kTwoTiles = 20 * kNumSMs;
 __host__ __device__ __forceinline__ int rows_in_flight(int width) { return width == 1 || width == 2 ? 4 : (width <= 4 ? 2 : 1); }
 
 __device__ __forceinline__ void add_piece(float (&acc)[8], float av, const uint4& raw) {
@@ -213,7 +217,7 @@ __device__ __forceinline__ void gather_few(const __half* a, const int32_t* cols,
 __global__ void __launch_bounds__(kThreads)
 gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_constant__ GatherTiles gt,
                         const __half* x, __half* __restrict__ z, int32_t* __restrict__ all_rows,
-                        int32_t* __restrict__ ranges, int num_rels, int chunks, const int32_t* passed) {
+                        int32_t* __restrict__ ranges, int num_rels, int chunks, const int32_t* passed, int per_block) {
   // passed != nullptr: the launch before this one, the transform of the one-column rows, neither reads nor writes what
   // this one writes, and the gather runs beside it, in the registers that it leaves.  The transform sets *passed behind
   // its own wait, so that a block which finds it set sees all that lies ahead of both as one that has waited; a block
@@ -228,38 +232,42 @@ gather_tiles_f16_kernel(const __grid_constant__ BucketTable tb, const __grid_con
   }
   const int lanes = kThreads / chunks;  // rows side by side
   const int rl = static_cast<int>(threadIdx.x) / chunks, ch = static_cast<int>(threadIdx.x) % chunks;
-  int b = 0;
-  while (b + 1 < tb.nb && static_cast<int>(blockIdx.x) >= gt.first[b + 1]) ++b;
-  const int width = tb.width[b], rows = tb.z_base[b + 1] - tb.z_base[b];
-  const int R = rows_in_flight(width);
-  const int e0 = (static_cast<int>(blockIdx.x) - gt.first[b]) * (lanes * R);
-  for (int i = threadIdx.x; i < lanes * R && i < rows - e0; i += kThreads)
-    all_rows[tb.z_base[b] + e0 + i] = ld_global(tb.rows[b] + e0 + i);
-  const unsigned e = static_cast<unsigned>(e0) + rl;
-  if (rl >= lanes || e >= static_cast<unsigned>(rows)) return;
-  const uint4* xv = reinterpret_cast<const uint4*>(x) + ch;
-  uint4* zv = reinterpret_cast<uint4*>(z) + static_cast<size_t>(tb.z_base[b]) * chunks + ch;
-  if (width == 1) return gather_few<1, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
-  if (width == 2) return gather_few<2, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
-  if (width <= 4) return gather_few<4, 2>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
-  const __half* ap = tb.a[b] + static_cast<size_t>(e) * width;
-  const int32_t* cp = tb.cols[b] + static_cast<size_t>(e) * width;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  int j = 0;
-  for (; j + 8 <= width; j += 8) {
-    float av[8];
-    uint4 raw[8];
+  auto one_tile = [&](int tile) {
+    int b = 0;
+    while (b + 1 < tb.nb && tile >= gt.first[b + 1]) ++b;
+    const int width = tb.width[b], rows = tb.z_base[b + 1] - tb.z_base[b];
+    const int R = rows_in_flight(width);
+    const int e0 = (tile - gt.first[b]) * (lanes * R);
+    for (int i = threadIdx.x; i < lanes * R && i < rows - e0; i += kThreads)
+      all_rows[tb.z_base[b] + e0 + i] = ld_global(tb.rows[b] + e0 + i);
+    const unsigned e = static_cast<unsigned>(e0) + rl;
+    if (rl >= lanes || e >= static_cast<unsigned>(rows)) return;
+    const uint4* xv = reinterpret_cast<const uint4*>(x) + ch;
+    uint4* zv = reinterpret_cast<uint4*>(z) + static_cast<size_t>(tb.z_base[b]) * chunks + ch;
+    if (width == 1) return gather_few<1, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+    if (width == 2) return gather_few<2, 4>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+    if (width <= 4) return gather_few<4, 2>(tb.a[b], tb.cols[b], xv, zv, e, lanes, rows, width, chunks);
+    const __half* ap = tb.a[b] + static_cast<size_t>(e) * width;
+    const int32_t* cp = tb.cols[b] + static_cast<size_t>(e) * width;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int j = 0;
+    for (; j + 8 <= width; j += 8) {
+      float av[8];
+      uint4 raw[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      av[u] = __half2float(ld_global(ap + j + u));
-      raw[u] = ld_global(xv + static_cast<size_t>(ld_global(cp + j + u)) * chunks);
+      for (int u = 0; u < 8; ++u) {
+        av[u] = __half2float(ld_global(ap + j + u));
+        raw[u] = ld_global(xv + static_cast<size_t>(ld_global(cp + j + u)) * chunks);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) add_piece(acc, av[u], raw[u]);
     }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) add_piece(acc, av[u], raw[u]);
-  }
-  for (; j < width; ++j)
-    add_piece(acc, __half2float(ld_global(ap + j)), ld_global(xv + static_cast<size_t>(ld_global(cp + j)) * chunks));
-  zv[static_cast<size_t>(e) * chunks] = pack_piece(acc);
+    for (; j < width; ++j)
+      add_piece(acc, __half2float(ld_global(ap + j)), ld_global(xv + static_cast<size_t>(ld_global(cp + j)) * chunks));
+    zv[static_cast<size_t>(e) * chunks] = pack_piece(acc);
+  };
+  const int first = static_cast<int>(blockIdx.x) * per_block, last = min(first + per_block, gt.first[tb.nb]);
+  for (int tile = first; tile < last; ++tile) one_tile(tile);
 }
 
 // ---- launch (1) when every bucket has one column per row (the sparse-convolution shape): the Z
@@ -1031,8 +1039,10 @@ int run_z(const BucketTable& tb, const __half* w, const __half* x, OutT* y, int 
       gt.first[b] = static_cast<int32_t>(tiles);
       tiles += ceil_div(tb.z_base[b + 1] - tb.z_base[b], lanes * rows_in_flight(tb.width[b]));
     }
-    launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(tiles + 1), kThreads, 0, st, tb, gt, x, z, all_rows, ranges,
-                   num_rels, feat_in / 8, passed);
+    gt.first[tb.nb] = static_cast<int32_t>(tiles);
+    const int per_block = passed != nullptr && tiles >= kTwoTiles ? 2 : 1;
+    launch_chained(gather_tiles_f16_kernel, static_cast<unsigned>(ceil_div(tiles, per_block) + 1), kThreads, 0, st, tb, gt, x, z, all_rows,
+                   ranges, num_rels, feat_in / 8, passed, per_block);
   } else if (vec)
     gather_rows_f16_kernel<8><<<blocks + 1, kThreads, 0, st>>>(tb, x, z, all_rows, ranges, num_rels, feat_in);
   else

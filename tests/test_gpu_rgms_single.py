@@ -50,7 +50,8 @@ def test_exact_sums(cuda_device, widths, rows, group, fi, fo):
     assert L.load().sparsetir_tc_timeouts(cuda_device.index or 0, ctypes.byref(count)) == 0 and count.value == 0
 
 
-@pytest.mark.parametrize("widths,rows,group", [((1, 2), (SINGLE, 500), 32), ((4, 1, 2), (1000, SINGLE + 37, 3000), 1), ((1, 1), (SINGLE, SINGLE + 128), 128)])
+@pytest.mark.parametrize("widths,rows,group", [((1, 2), (SINGLE, 500), 32), ((4, 1, 2), (1000, SINGLE + 37, 3000), 1), ((1, 1), (SINGLE, SINGLE + 128), 128),
+                                               ((8, 1, 4), (47_500, SINGLE + 1, 500), 1)])  # at 128 features two tiles of the gather per block
 @pytest.mark.parametrize("fi,fo", [(64, 64), (128, 64), (64, 192), (64, 32)])
 def test_exact_sums_in_float16(cuda_device, widths, rows, group, fi, fo):
     """The result in half precision: multiples of a half below 1024, which every order of addition keeps."""
