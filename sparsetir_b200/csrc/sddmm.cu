@@ -34,9 +34,9 @@ constexpr int kThreads = 256;
 // inside the kernel, the eight sums staying in registers; seven shuffles transpose and add them
 // over eight lanes, one more per doubling of the group adds the rest.
 //
-// What bounds it on short rows is instructions and latency per position (150 instructions of a warp for 8 positions with 16
-// lanes of 16 bytes a row, L1 data path 34 %).  Groups of 8 lanes of 32 bytes have as many bytes in flight and four
-// positions where those had two: power-law graphs, us, before / with them: 169 k rows, F = 64 43.1 / 31.9, 200 k rows
+// What bounds it on short rows is the latency of the gathers (169 k rows of 5 entries, F = 64, counters of one launch: 17 of
+// the 23 warps per issued instruction wait for memory, L1 data path 35 %, L2 32 %, issue slots 22 %, DRAM 30 %).  Groups of
+// 8 lanes of 32 bytes have as many bytes in flight as 16 lanes of 16 bytes and four positions where those had two: power-law graphs, us, before / with them: 169 k rows, F = 64 43.1 / 31.9, 200 k rows
 // F = 192 131 / 102, F = 128 72 / 67, 20 k rows F = 128 10.1 / 8.6.  Groups of 16 such lanes gain nothing (F = 256 137 / 141).
 template <int LPR, int W, int VPL, bool PEERS>
 __global__ void __launch_bounds__(kThreads, 4)

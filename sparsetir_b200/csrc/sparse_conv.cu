@@ -14,9 +14,10 @@
 //  - one thread brings the slice of W with TMA, one issues the MMAs into one of two accumulators;
 //  - four warps take finished tiles out of TMEM and write (or add to) Y, each row once.
 //
-// Bound by the issue slots of an SM and its L1 data pipe, not by memory or the tensor cores: at 100,000 points, 27
-// offsets, 64 -> 32 a layer with 2 % of the pairs takes as long as one with 95 % of them.  What was cut is therefore
-// instructions and what passes the data pipe: no divisions in the loops and MMAs from an elected thread 97 -> 64 us (64 ->
+// No unit is at its limit (100,000 points, 27 offsets, 64 -> 128, counters of one launch: tensor pipe 39 %, L1 data pipe
+// 47 %, issue slots 35 %, L2 25 %, DRAM 5 % of the elapsed time): a step of the ring costs the gathering warps'
+// instructions and their waits for map entries and stages, whatever the share of pairs (64 -> 32: a layer with 2 % of
+// them takes as long as one with 95 %).  What was cut is therefore instructions and what passes the data pipe: no divisions in the loops and MMAs from an elected thread 97 -> 64 us (64 ->
 // 128), asynchronous copies instead of loads and stores 64 -> 58; then (us, 64 -> 128 / 64 -> 32, 54.7 / 48.6 before) one
 // slice of W for two tiles and copies that arrive at the stage's barrier themselves, 51.5 / 44.2, the copies of a step
 // written out, 50.3 / 41.2, an epilogue of a third of the instructions, 47.2 / 39.7.  Rows loaded into registers and
@@ -177,9 +178,9 @@ __device__ __noinline__ float row_by_pairs(const __half* x, const __half* w,
 }
 
 // Eight rows' pieces of 16 bytes into shared memory: row i from xb + from[i] * row_bytes to at0 (even i) or at1 (odd i)
-// + i / 2 * 1024; zeros where from[i] is negative, or everywhere with `skip`.  One statement, written out: what bounds the
-// kernel is the instructions of the gathering warps, and the selects and addresses that the compiler made of the
-// same loop were more: 16 instructions a step and warp are 4 us of 45 (100,000 points, 27 offsets, 64 -> 32).
+// + i / 2 * 1024; zeros where from[i] is negative, or everywhere with `skip`.  One statement, written out: what a
+// step costs is the instructions of the gathering warps, and the selects and addresses that the compiler made of the
+// same loop were more: 16 instructions a step and warp were 4 us of 45 (100,000 points, 27 offsets, 64 -> 32).
 __device__ __forceinline__ void copy_rows(uint32_t at0, uint32_t at1, const int (&from)[8], uint32_t row_bytes, const char* xb, int skip) {
 #define SPTIR_COPY_ROW(E, AT, OFF)              \
   "setp.lt.or.s32 p, " E ", 0, q;\n\t"          \
