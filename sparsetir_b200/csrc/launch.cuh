@@ -11,6 +11,8 @@
 //    empty.  Scheduled earlier, its blocks fill the SMs that come free first, and a launch of less than a full
 //    wave lies unevenly over them (us, triggered at the start / not: SDDMM 20 k rows, F = 512, 34.8 / 29.0, CSR SpMM
 //    20 k rows, F = 512, 43.3 / 38.8, 4,096 rows 5.1 / 4.5).
+//    The gather of rgms_f16.cu does so all the same: behind it comes one block per SM that sets up barriers and waits (20.7 /
+//    21.3 at 64 -> 64 on 22 k nodes, 16.8 / 17.9 at 32 -> 32).
 //  - Kernels of one wave of blocks, one or two to an SM, trigger behind the wait, so that the next one's set-up overlaps:
 //    no block of this launch is still to be scheduled then, and a block of the next one only waits.
 //  - A kernel that takes tensor memory triggers when its block has it (behind the barrier that publishes the address).
