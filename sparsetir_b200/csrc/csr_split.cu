@@ -57,7 +57,9 @@ __device__ __forceinline__ unsigned group_ballot(unsigned mask, bool pred) {
 // Resident blocks.  The widest pieces per lane spill at 64 registers: three blocks of 80 hold them (50 k-node
 // power-law graph, F = 299: 80 against 77.6 us; 100 k nodes, F = 222: 76 against 70; 30 k rows of 38 entries,
 // F = 151: 104 against 99; two single floats per lane: F = 41, 49 against 53).
-__host__ __device__ constexpr int blocks_per_sm(int w, int vpl) { return vpl > 1 && vpl * w > 2 ? 3 : 4; }
+// Two 16-byte vectors per lane hold eight rows each in flight: two blocks of 128 (40 k rows of 20 entries, F = 64, four rows
+// in flight at 80 registers 21.7 us, eight 19.0).
+__host__ __device__ constexpr int blocks_per_sm(int w, int vpl) { return vpl == 1 || vpl * w <= 2 ? 4 : w == 4 ? 2 : 3; }
 
 // A lane owns VPL vectors of W floats of the feature tile (VPL * LPR * W floats), LPR * W apart: one
 // 16-byte vector where rows allow it, several 4- or 8-byte ones where their length or alignment
@@ -354,7 +356,22 @@ struct SplitShape {
   int lanes, w, vpl;
 };
 
-SplitShape split_shape(uintptr_t bits, int n, int feat, int nnz) {
+// Two vectors per lane on half the lanes, us, one vector / two (rows of about equal length unless said otherwise):
+//  - up to 64 features: 30 k rows of 12 15.3 / 12.1, 9 k of 60 15.9 / 13.8, 200 k of 30 117 / 109, power-law graphs (4.5 per row)
+//    70 k 18.1 / 15.8, 200 k 34.7 / 34.7; 36 features, 300 per row, 40 k 209 / 184.
+//  - more: 30 k of 12 F = 128 21.7 / 17.7, F = 256 39.9 / 32.6, 60 k of 8 F = 100 28.9 / 24.0; where a slice of B is more than L2 keeps
+//    they bring nothing (200 k of 16 F = 128 148 / 161), nor on power-law graphs (100 k F = 128 28.4 / 29.5).
+//  - whole tiles on long rows are at the L2-to-SM rate with either (200 per row and more, F = 64 and 128: within the 15 % by which
+//    one kernel's time moves there with the share of a sub-warp): not taken.
+//  - less than a batch for each of the resident blocks, half as many here: not taken (3 k of 30 F = 128 9.4 / 10.0).
+bool two_vectors(int m, int n, int feat, int nnz, bool whole) {
+  const int per_row = nnz / m;
+  if (whole && per_row >= 100) return false;
+  if (feat <= 64) return nnz >= 80000;
+  return nnz >= 100000 && per_row >= 6 && static_cast<size_t>(n) * std::min(feat * 4, 512) <= (size_t{48} << 20);
+}
+
+SplitShape split_shape(uintptr_t bits, int m, int n, int feat, int nnz) {
   if (feat % 4 == 0 && bits % 16 == 0) {
     // The narrowest group that covers a row, a warp at most: several sub-warps per warp keep more
     // rows in flight (4.5 M entries, F = 64: 16 lanes 93, 32 lanes 160, 8 lanes 107 us), a second
@@ -365,6 +382,8 @@ SplitShape split_shape(uintptr_t bits, int n, int feat, int nnz) {
     while (lanes > 8 && n > 0 && nnz / n >= 64 &&
            static_cast<size_t>(n) * std::min(lanes * 16, feat * 4) > (size_t{48} << 20))
       lanes /= 2;
+    // Half the lanes with two vectors each: half the shuffles per entry.
+    if (lanes > 8 && two_vectors(m, n, feat, nnz, feat % (lanes * 4) == 0)) return {lanes / 2, 4, 2};
     return {lanes, 4, 1};
   }
   if (feat % 2 == 0 && bits % 8 == 0) return {feat <= 16 ? 8 : (feat <= 32 ? 16 : 32), 2, feat <= 64 ? 1 : 2};
@@ -408,6 +427,7 @@ int launch_split(const SplitArgs& s, const SplitPlan& p, cudaStream_t st) {
 
 int dispatch_split(const SplitArgs& s, const SplitShape& sh, const SplitPlan& p, cudaStream_t st) {
   if (sh.w == 4) {
+    if (sh.vpl == 2) return sh.lanes == 8 ? launch_split<8, 4, 2>(s, p, st) : launch_split<16, 4, 2>(s, p, st);
     if (sh.lanes == 8) return launch_split<8, 4, 1>(s, p, st);
     if (sh.lanes == 16) return launch_split<16, 4, 1>(s, p, st);
     return launch_split<32, 4, 1>(s, p, st);
@@ -435,7 +455,7 @@ inline uintptr_t low_bits(const float* b, const float* c) {
 // Bytes of scratch that the pieces of this call need.
 size_t csr_split_scratch(const float* b, const float* c, int m, int n, int feat, int nnz) {
   if (nnz == 0) return 0;
-  return split_plan(split_shape(low_bits(b, c), n, feat, nnz), m, feat, nnz).part_bytes;
+  return split_plan(split_shape(low_bits(b, c), m, n, feat, nnz), m, feat, nnz).part_bytes;
 }
 
 // The most that a call of these sizes needs, whatever its operands' alignment.
@@ -443,7 +463,7 @@ void csr_split_scratch_bound(int m, int n, int feat, int nnz, size_t* part_bytes
   *part_bytes = *counter_bytes = 0;
   if (m == 0 || feat == 0 || nnz == 0) return;
   for (const uintptr_t bits : {16, 8, 4}) {
-    const SplitPlan p = split_plan(split_shape(bits, n, feat, nnz), m, feat, nnz);
+    const SplitPlan p = split_plan(split_shape(bits, m, n, feat, nnz), m, feat, nnz);
     *part_bytes = std::max(*part_bytes, p.part_bytes);
     *counter_bytes = std::max(*counter_bytes, p.counter_bytes);
   }
@@ -457,7 +477,7 @@ int csr_split_run(const float* a, const float* b, float* c, const int32_t* indpt
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(m) * feat * sizeof(float), st));
     return 0;
   }
-  const SplitShape sh = split_shape(low_bits(b, c), n, feat, nnz);
+  const SplitShape sh = split_shape(low_bits(b, c), m, n, feat, nnz);
   const SplitPlan p = split_plan(sh, m, feat, nnz);
   CallScratch cs;
   if (pieces != nullptr) {

@@ -52,6 +52,30 @@ def test_rows_meet_across_sub_warps_and_blocks(cuda_device, shape, feat, offset)
     assert torch.equal(again, y)  # one writer and one order: the same bits
 
 
+@pytest.mark.parametrize("feat", [36, 64, 68, 128, 132, 256])
+@pytest.mark.parametrize("deg", [[0, 1, 2, 30, 7, 0, 0, 13, 32, 11] * 1100, [3000, 8, 0] * 10 + [8] * 10_000, [99] * 1200,
+                                 [12, 0, 4] * 5000, [12, 0, 4] * 4999 + [12, 0, 3]], ids=["mixed", "hubs", "long", "least", "less"])
+def test_two_vectors_per_lane(cuda_device, deg, feat):
+    # more and less than 80,000 and 100,000 entries, and rows of 100 where whole tiles go back to one vector
+    deg = torch.tensor(deg, device=cuda_device)
+    m, n, nnz = len(deg), 2003, int(deg.sum())
+    g = torch.Generator(device=cuda_device).manual_seed(feat)
+    ptr = torch.zeros(m + 1, dtype=torch.int32, device=cuda_device)
+    ptr[1:] = deg.cumsum(0)
+    cols = torch.randint(0, n, (nnz,), generator=g, device=cuda_device, dtype=torch.int32)
+    vals = torch.rand(nnz, generator=g, device=cuda_device) - 0.5
+    x = torch.rand(n, feat, generator=g, device=cuda_device) - 0.5
+    y = torch.full((m * feat,), float("nan"), device=cuda_device)
+    ops.csrmm(vals, x.view(-1), y, ptr, cols)
+    a = torch.sparse_csr_tensor(ptr, cols, vals.double(), (m, n))
+    mag = torch.sparse_csr_tensor(ptr, cols, vals.abs().double(), (m, n)) @ x.abs().double()
+    # a sum of d fp32 products in any order: at most d half-ulps of the sum of magnitudes
+    assert bool(((y.view(m, feat).double() - a @ x.double()).abs() <= mag * (deg[:, None] + 1) * 2.0 ** -24).all())
+    again = y.clone()
+    ops.csrmm(vals, x.view(-1), y, ptr, cols)
+    assert torch.equal(again, y)
+
+
 def test_first_call_on_a_stream_can_be_captured(cuda_device):
     m, feat = 9000, 41
     ptr = torch.arange(0, 8 * m + 1, 8, dtype=torch.int32, device=cuda_device)
