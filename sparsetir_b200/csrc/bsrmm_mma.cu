@@ -2,14 +2,15 @@
 // operands, fp32 sums: the shapes that the tcgen05 kernels of bsrmm_tc.cu (block size 32, features in
 // steps of 128) do not take.  They ran on CUDA cores at 11 TFLOP/s.
 //
-// A thread block owns 16 MT rows of a block row and 64 features; its four warps share the stored blocks,
-// 16 columns ("a group") at a time, two groups in flight per warp, operands straight into the registers
-// of the matrix instruction (mma16.cuh).  The warps' sums meet in shared memory in a fixed order and every
-// result is written once.  MT = 2 halves the reads of B per result where the block size allows it.
+// A thread block owns 16 MT rows of a block row and 64 features; its four warps share the stored blocks, 16 columns ("a group")
+// at a time.  The rows of B and the values of A of a warp's next three or four groups are on their way into shared memory
+// by asynchronous copies (mma16.cuh).  The warps' sums meet there in a fixed order and every result is written once.
+// MT = 2 halves the reads of B per result where the block size allows it.
 //
-// Bound: the L2-to-SM gather of B (each block reads the 16 rows of its groups once per 16 MT rows of C).
-// 10 % of the blocks stored, us, before / now: 8192 x 8192, block 16, F = 512 626 / 84; block 64 645 / 66; block
-// 32, F = 496 630 / 57; 4096 x 4096, block 16, F = 64 68 / 11; 1024 x 1024, block 64, F = 64 31 / 7.
+// Bound: the L2-to-SM gather of B (each block reads the 16 rows of its groups once per 16 MT rows of C) and the copies' latency on
+// small matrices.  10 % of the blocks stored, us, CUDA cores / operands straight into registers, where four rows per
+// load met in the same banks of L1 / now: 8192 x 8192, block 16, F = 512 626 / 79 / 53; block 64 645 / 62 / 53; block 32, F = 496
+// 630 / 54 / 49; 4096 x 4096, block 16, 5 %, F = 208 - / 11.1 / 9.4; 2048 x 2048, block 16, F = 64 - / 4.4 / 3.4.
 #include <cuda_fp16.h>
 
 #include "common.h"
@@ -22,12 +23,20 @@ namespace {
 
 constexpr int kThreads = 128;
 
+__host__ __device__ constexpr int stages(int mt) { return mt == 1 ? 4 : 3; }
 template <int MT>
-__global__ void __launch_bounds__(kThreads, MT == 1 ? 5 : 3)
+struct __align__(128) WarpRing {
+  unsigned char rows[stages(MT)][mma16::kGroupBytes];
+  unsigned char values[stages(MT)][MT * 512];
+};
+
+template <int MT>
+__global__ void __launch_bounds__(kThreads, MT == 1 ? 5 : 4)
 bsrmm_mma_kernel(const __half* a, const __half* b, float* __restrict__ c,
                  const int32_t* indptr, const int32_t* indices, int blk, int feat,
                  int slabs, int parts, int vec_out) {
-  __shared__ float s_sum[4][MT][4][8][32];  // [warp][row tile][c][j][lane]
+  constexpr int S = stages(MT);
+  __shared__ WarpRing<MT> s_ring[4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2;
   const int slab = static_cast<int>(blockIdx.x) % slabs, rest = static_cast<int>(blockIdx.x) / slabs;
   const int part = rest % parts, i = rest / parts;
@@ -36,82 +45,94 @@ bsrmm_mma_kernel(const __half* a, const __half* b, float* __restrict__ c,
   const int p0 = ld_global(indptr + i), p1 = ld_global(indptr + i + 1);
   const int per_blk = blk >> 4;  // groups per stored block
   const long long total = static_cast<long long>(p1 - p0) * per_blk;
-  const long long g0 = total * warp / 4, g1 = total * (warp + 1) / 4;
+  const long long g0 = total * warp / 4;
+  const int groups = static_cast<int>(total * (warp + 1) / 4 - g0);
 
   float acc[MT][8][4];
   mma16::clear(acc);
-  const bool in = f0 + r * 8 < feat;
-  const __half* bl = b + static_cast<size_t>(4 * q) * feat + (in ? f0 + r * 8 : 0);
-  const __half* al = a + static_cast<size_t>(row0 + r) * blk + 4 * q;
-  auto rows_of = [&](int col, int kk, uint4 (&v)[4]) {
-    const __half* p = bl + (static_cast<size_t>(col) * blk + kk * 16) * feat;
+  const int piece = lane & 7, first = (lane >> 3) * 4;  // of the rows of B that this lane copies
+  const bool in = f0 + piece * 8 < feat;
+  const __half* bl = b + static_cast<size_t>(first) * feat + (in ? f0 + piece * 8 : 0);
+  const __half* al = a + static_cast<size_t>(row0 + (lane >> 1)) * blk + (lane & 1) * 8;
+  WarpRing<MT>& ring = s_ring[warp];
+  const uint32_t rows0 = static_cast<uint32_t>(__cvta_generic_to_shared(&ring.rows[0][0]));
+  const uint32_t values0 = static_cast<uint32_t>(__cvta_generic_to_shared(&ring.values[0][0]));
+  // the next group to copy: stored block, group inside it; lane k holds the column of block id0 + k
+  int pc = p0 + static_cast<int>(g0 / per_blk), kc = static_cast<int>(g0 % per_blk);
+  int id0 = pc, ids = 0;
+  if (groups > 0) ids = ld_global(indices + min(id0 + lane, p1 - 1));
+  auto copy_group = [&](int n) {
+    if (n < groups) {
+      if (pc - id0 == 32) {
+        id0 = pc;
+        ids = ld_global(indices + min(id0 + lane, p1 - 1));
+      }
+      const int col = __shfl_sync(0xffffffffu, ids, pc - id0), stage = n % S;
+      const __half* p = bl + (static_cast<size_t>(col) * blk + kc * 16) * feat;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (in) v[k] = ld_global(reinterpret_cast<const uint4*>(p + static_cast<size_t>(k) * feat));
+      for (int k = 0; k < 4; ++k)
+        mma16::copy16(rows0 + stage * mma16::kGroupBytes + mma16::piece_at(mma16::row_slot(first + k), piece),
+                      p + static_cast<size_t>(k) * feat, in);
+      const __half* at = al + static_cast<size_t>(pc) * blk * blk + kc * 16;
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+        mma16::copy16(values0 + stage * (MT * 512) + (m * 32 + lane) * 16, at + static_cast<size_t>(m * 16) * blk, true);
+      if (++kc == per_blk) {
+        kc = 0;
+        ++pc;
+      }
     }
   };
-  auto values_of = [&](int p, int kk, uint32_t (&av)[MT][4]) {
-    const __half* at = al + static_cast<size_t>(p) * blk * blk + kk * 16;
+#pragma unroll
+  for (int n = 0; n < S; ++n) {
+    copy_group(n);
+    cp_async_commit();
+  }
+  for (int n = 0; n < groups; ++n) {
+    cp_async_wait<S - 1>();
+    __syncwarp();
+    const unsigned char* v = ring.values[n % S];
+    uint32_t av[MT][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-      const uint2 lo = ld_global(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16) * blk));
-      const uint2 hi = ld_global(reinterpret_cast<const uint2*>(at + static_cast<size_t>(mt * 16 + 8) * blk));
+      const uint2 lo = *reinterpret_cast<const uint2*>(v + (mt * 16 + r) * 32 + q * 8);
+      const uint2 hi = *reinterpret_cast<const uint2*>(v + (mt * 16 + 8 + r) * 32 + q * 8);
       av[mt][0] = lo.x; av[mt][1] = hi.x; av[mt][2] = lo.y; av[mt][3] = hi.y;
     }
-  };
-  // (block, group inside it) of the next two groups; their column ids are requested one pair ahead
-  int pa = p0 + static_cast<int>(g0 / per_blk), ka = static_cast<int>(g0 % per_blk);
-  auto next = [&](int& p, int& k) {
-    if (++k == per_blk) { k = 0; ++p; }
-  };
-  int pb = pa, kb = ka;
-  next(pb, kb);
-  auto id_of = [&](int p) { return ld_global(indices + min(p, p1 - 1)); };  // past the last block: not used
-  int ca = 0, cb = 0;
-  if (p0 < p1) {
-    ca = id_of(pa);
-    cb = id_of(pb);
+    mma16::multiply(acc, rows0 + n % S * mma16::kGroupBytes, lane, av);
+    __syncwarp();
+    copy_group(n + S);
+    cp_async_commit();
   }
-  for (long long g = g0; g < g1; g += 2) {
-    const bool two = g + 1 < g1;
-    uint4 va[4], vb[4];
-    uint32_t aa[MT][4], ab[MT][4];
-    rows_of(ca, ka, va);
-    if (two) rows_of(cb, kb, vb);
-    values_of(pa, ka, aa);
-    if (two) values_of(pb, kb, ab);
-    next(pa, ka); next(pa, ka);
-    next(pb, kb); next(pb, kb);
-    ca = id_of(pa);
-    cb = id_of(pb);
-    mma16::multiply(acc, va, aa);
-    if (two) mma16::multiply(acc, vb, ab);
-  }
+  cp_async_wait<0>();
+  __syncwarp();
+  // the warps' sums meet, row by row, in place of their rings
+  constexpr int kRow = mma16::kSlab + 8;  // floats; rows of four neighbours lie in all banks
+  static_assert(MT * 16 * kRow * 4 <= sizeof(WarpRing<MT>), "fits the ring");
+  float* mine = reinterpret_cast<float*>(&ring) + r * kRow + 2 * q;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s_sum[warp][mt][k][j][lane] = acc[mt][j][k];
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float2*>(mine + (mt * 16 + h * 8) * kRow + j * 8) = make_float2(acc[mt][j][2 * h], acc[mt][j][2 * h + 1]);
   __syncthreads();
-  // warp w finishes the pieces c = w
-  const int f = f0 + (2 * q + (warp & 1)) * 8;
-  if (f >= feat) return;
+  // a warp finishes every fourth row, 16 bytes per lane: whole lines
+  const int f = (lane & 15) * 4;
+  if (f0 + f >= feat) return;
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      v[j] = (s_sum[0][mt][warp][j][lane] + s_sum[1][mt][warp][j][lane]) +
-             (s_sum[2][mt][warp][j][lane] + s_sum[3][mt][warp][j][lane]);
-    float* dst = c + (static_cast<size_t>(i) * blk + row0 + mt * 16 + r + (warp >> 1) * 8) * feat + f;
+  for (int k = 0; k < 2 * MT; ++k) {
+    const int row = (k * 4 + warp) * 2 + (lane >> 4);  // of 16 MT
+    const auto of = [&](int w) { return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(&s_ring[w]) + row * kRow + f); };
+    const float4 s0 = of(0), s1 = of(1), s2 = of(2), s3 = of(3);
+    const float4 v = make_float4((s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y), (s0.z + s1.z) + (s2.z + s3.z),
+                                 (s0.w + s1.w) + (s2.w + s3.w));
+    float* dst = c + (static_cast<size_t>(i) * blk + row0 + row) * feat + f0 + f;
     if (vec_out) {
-      __stcs(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
-      __stcs(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
+      __stcs(reinterpret_cast<float4*>(dst), v);
     } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dst[j] = v[j];
+      dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
     }
   }
 }
