@@ -6,8 +6,10 @@
 //
 // This file holds the CUDA-core kernel that works for every block size; bsrmm_tc.cu (block size 32,
 // features in steps of 128) and bsrmm_mma.cu (block sizes in steps of 16, features in steps of 8) hold
-// the tensor-core kernels and are tried first, in this order.
+// the tensor-core kernels and are tried first.
 #include <cuda_fp16.h>
+
+#include <cstdlib>
 
 #include "common.h"
 
@@ -83,7 +85,22 @@ extern "C" int sparsetir_bsrmm_raw(const void* a_f16, const void* b_f16, float* 
   if (validate_enabled() && validate_csr("sparsetir_bsrmm", indptr, nb, indices, nnzb, mb, st) != 0) return -1;
   const __half* a = static_cast<const __half*>(a_f16);
   const __half* b = static_cast<const __half*>(b_f16);
-  int rc = bsrmm_tc_launch(a, b, c, indptr, indices, nb, mb, nnzb, blk, feat, st);
+  // Blocks of 32 and features in steps of 128 could take either tensor-core kernel.  bsrmm_mma.cu has the shorter chain in front of
+  // the first product and is the faster one as long as all its thread blocks, 64 features of a block row each, are resident at
+  // once (10 % stored, us, tcgen05 / mma: 4096^2, F = 128 10.5 / 6.9, F = 256 9.8 / 9.4, 2720^2, F = 384 10.0 / 7.8; in more than one wave
+  // 4096^2, F = 384 12.4 / 13.6, 8192^2, F = 256 18.2 / 24.5); where whole pairs of feature tiles share the loads of A, less than that
+  // (1536^2, F = 512 6.7 / 5.7, 2048^2 6.7 / 7.2).
+  const long long units = static_cast<long long>(nb) * ceil_div(feat, 64);
+  static const bool chosen = [] {  // a comparison switch of bsrmm_tc.cu
+    const char* e = std::getenv("SPARSETIR_BSR_PATH");
+    return e != nullptr && e[0] != '\0';
+  }();
+  int rc = 1;
+  if (!chosen && blk == 32 && units <= (feat > 256 && feat % 256 == 0 ? 400 : 4 * kNumSMs)) {
+    rc = bsrmm_mma_launch(a, b, c, indptr, indices, nb, blk, feat, st);
+    if (rc <= 0) return rc;
+  }
+  rc = bsrmm_tc_launch(a, b, c, indptr, indices, nb, mb, nnzb, blk, feat, st);
   if (rc <= 0) return rc;
   rc = bsrmm_mma_launch(a, b, c, indptr, indices, nb, blk, feat, st);
   if (rc <= 0) return rc;

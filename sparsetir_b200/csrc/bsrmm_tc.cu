@@ -258,8 +258,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (lane == 0) {
         unsigned char* st = tiles + stage * kStageBytes;
         tc05::mbar_arrive_expect_tx(&bar_full[stage], kStageBytes);
-        tc05::tma_load_2d(st, &tm_b, f0, col * kBlk, &bar_full[stage]);
-        tc05::tma_load_2d(st + kBBytes / 2, &tm_b, f0 + 64, col * kBlk, &bar_full[stage]);
+        tc05::tma_load_3d(st, &tm_b, 0, col * kBlk, f0 / 64, &bar_full[stage]);  // two parts of 64 features
         tc05::tma_load_2d(st + kBBytes, &tm_a, 0, (p0 + it) * kBlk, &bar_full[stage]);
       }
       armed = it + 1;
@@ -312,7 +311,7 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------
-// Persistent variant (the default when feat is a multiple of 256): at 128 x 128 blocks and 512
+// Persistent variant (the default for whole pairs of feature tiles): at 128 x 128 blocks and 512
 // features the kernel above is 512 short-lived thread blocks, and what a call costs is mostly what
 // every one of them pays before and after its dozen tile loads: barrier set-up, TMEM allocation,
 // the first load's latency with nothing to overlap it, an epilogue nothing overlaps either.  Here
@@ -322,7 +321,9 @@ bsrmm_tma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 //     item, the tiles of the next are already landing (8 stages of 18 KB),
 //   - two TMEM accumulators alternate, so the epilogue of an item (TMEM -> registers -> 32
 //     coalesced row stores per warp) overlaps the loads and MMAs of the next,
-//   - the A block of a stored block is loaded once for two feature tiles.
+//   - the A block of a stored block is loaded once for two feature tiles;
+//   - one load brings all four 64-feature parts of a tile of B: with a load for each, the loads' own cost bounded the steps
+//     (4096 x 4096, 10 %, F = 512 12.0 / 10.3 us, 8192 x 8192, F = 1024 56.5 / 45.1, 12 TB/s of tiles).
 // Roles: warp 0 producer (TMA), warp 1 MMA issuer, warps 2-5 epilogue (a warp reads the TMEM lanes
 // 32 * (warp % 4) .. + 31: lane = feature inside the tile, column = row inside the block row).
 // Every mbarrier wait is bounded.
@@ -388,11 +389,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (lane == 0) {
           unsigned char* st = tiles + stage * kPStageBytes;
           tc05::mbar_arrive_expect_tx(&bar_full[stage], kPStageBytes);
-#pragma unroll
-          for (int tt = 0; tt < kPTiles; ++tt) {
-            tc05::tma_load_2d(st + tt * kBBytes, &tm_b, f0 + tt * kTileF, col * kBlk, &bar_full[stage]);
-            tc05::tma_load_2d(st + tt * kBBytes + kBBytes / 2, &tm_b, f0 + tt * kTileF + 64, col * kBlk, &bar_full[stage]);
-          }
+          tc05::tma_load_3d(st, &tm_b, 0, col * kBlk, f0 / 64, &bar_full[stage]);  // four parts of 64 features
           tc05::tma_load_2d(st + kPTiles * kBBytes, &tm_a, 0, (p0 + it) * kBlk, &bar_full[stage]);
         }
         armed = bk + 1;
@@ -448,8 +445,7 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const int nblk = ld_global(indptr + i + 1) - ld_global(indptr + i);
       float* crow = c + (static_cast<size_t>(i) * kBlk) * feat + f0 + q * 32 + lane;
       if (nblk <= 0) {  // empty block-row: zeros, no tensor-core work
-#pragma unroll
-        for (int tt = 0; tt < kPTiles; ++tt)
+        for (int tt = 0; tt < kPTiles && f0 + tt * kTileF < feat; ++tt)
 #pragma unroll 4
           for (int bi = 0; bi < kBlk; ++bi) crow[static_cast<size_t>(bi) * feat + tt * kTileF] = 0.f;
         continue;
@@ -465,9 +461,11 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           tc05::fence_before_sync();
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc05::smem_u32(&bar_acc_empty[buf])) : "memory");
         }
+        if (tt == 0 || f0 + tt * kTileF < feat) {
 #pragma unroll
-        for (int bi = 0; bi < kBlk; ++bi)
-          __stcs(crow + static_cast<size_t>(bi) * feat + tt * kTileF, __uint_as_float(r[bi]));
+          for (int bi = 0; bi < kBlk; ++bi)
+            __stcs(crow + static_cast<size_t>(bi) * feat + tt * kTileF, __uint_as_float(r[bi]));
+        }
       }
       ++acc_it;
     }
@@ -488,14 +486,18 @@ bsrmm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 // 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error
 int bsrmm_persist_launch(const __half* a, const __half* b, float* c, const int32_t* indptr,
                          const int32_t* indices, int nb, int mb, int nnzb, int feat, cudaStream_t stream) {
-  if (nnzb <= 0 || mb <= 0 || feat % (kPTiles * kTileF) != 0) return 1;
+  if (nnzb <= 0 || mb <= 0) return 1;
+  // An item of one feature tile costs what one of two does: taken while every item has a block of its own (10 % stored, us, one
+  // block per tile / here: 4096^2, F = 384 12.4 / 10.2, F = 640, 384 items, 14.4 / 17.3).
+  const long long all = static_cast<long long>(nb) * ceil_div(feat, kPTiles * kTileF);
+  if (feat % (kPTiles * kTileF) != 0 && (feat <= kTileF || all > 2 * kNumSMs)) return 1;
   CUtensorMap tm_a, tm_b;
   if (make_tmap_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a, kBlk, static_cast<uint64_t>(nnzb) * kBlk,
                    kBlk * 2, kBlk, kBlk, CU_TENSOR_MAP_SWIZZLE_64B) != 0)
     return 1;
-  if (make_tmap_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, static_cast<uint64_t>(feat),
-                   static_cast<uint64_t>(mb) * kBlk, static_cast<uint64_t>(feat) * 2, 64, kBlk,
-                   CU_TENSOR_MAP_SWIZZLE_128B) != 0)
+  if (make_tmap_parts(&tm_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, static_cast<uint64_t>(feat),
+                      static_cast<uint64_t>(mb) * kBlk, static_cast<uint64_t>(feat) * 2, 64, 128, kBlk,
+                      kPTiles * kTileF / 64, CU_TENSOR_MAP_SWIZZLE_128B) != 0)
     return 1;
   static thread_local int configured_device = -1;
   int dev = 0;
@@ -504,8 +506,8 @@ int bsrmm_persist_launch(const __half* a, const __half* b, float* c, const int32
     SPTIR_CUDA_OK(cudaFuncSetAttribute(bsrmm_persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmem));
     configured_device = dev;
   }
-  const int items_per_row = feat / (kPTiles * kTileF);
-  const long long items = static_cast<long long>(nb) * items_per_row;
+  const int items_per_row = ceil_div(feat, kPTiles * kTileF);  // the parts of the last one that are past the row load as zeros
+  const long long items = all;
   if (items > INT32_MAX) return 1;
   const int grid = static_cast<int>(items < 2 * kNumSMs ? items : 2 * kNumSMs);  // two blocks per SM (shared memory)
   launch_chained(bsrmm_persist_kernel, grid, kPThreads, kPSmem, stream, tm_a, tm_b, c, indptr, indices, feat,
@@ -522,9 +524,9 @@ int bsrmm_tma_launch(const __half* a, const __half* b, float* c, const int32_t* 
   if (make_tmap_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a, kBlk, static_cast<uint64_t>(nnzb) * kBlk,
                    kBlk * 2, kBlk, kBlk, CU_TENSOR_MAP_SWIZZLE_64B) != 0)
     return 1;
-  if (make_tmap_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, static_cast<uint64_t>(feat),
-                   static_cast<uint64_t>(mb) * kBlk, static_cast<uint64_t>(feat) * 2, 64, kBlk,
-                   CU_TENSOR_MAP_SWIZZLE_128B) != 0)
+  if (make_tmap_parts(&tm_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, static_cast<uint64_t>(feat),
+                      static_cast<uint64_t>(mb) * kBlk, static_cast<uint64_t>(feat) * 2, 64, 128, kBlk, kTileF / 64,
+                      CU_TENSOR_MAP_SWIZZLE_128B) != 0)
     return 1;
   static thread_local int configured_device = -1;
   int dev = 0;
