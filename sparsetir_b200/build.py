@@ -26,7 +26,7 @@ PYCALL_PATH = os.path.join(PKG_DIR, "_pycall.so")
 
 SOURCES = [
     "runtime.cc", "abi.cc", "format.cc", "validate.cu",
-    "csrmm.cu", "csr_split.cu", "hyb_spmm.cu", "sddmm.cu", "bsrmm.cu", "bsrmm_tc.cu", "bsrmm_mma.cu", "rgms.cu", "rgms_tc.cu", "rgms_fused.cu", "rgms_wide.cu", "rgms_noalloc.cu", "rgms_ell3d.cu", "rgms_f16.cu", "sparse_conv.cu", "tcspmm.cu", "csr_misc.cu", "fusedmm.cu", "peer_scatter.cu",
+    "csrmm.cu", "csr_split.cu", "hyb_spmm.cu", "sddmm.cu", "bsrmm.cu", "bsrmm_tc.cu", "bsrmm_mma.cu", "rgms.cu", "rgms_tc.cu", "rgms_pairs.cu", "rgms_fused.cu", "rgms_wide.cu", "rgms_noalloc.cu", "rgms_ell3d.cu", "rgms_f16.cu", "sparse_conv.cu", "tcspmm.cu", "csr_misc.cu", "fusedmm.cu", "peer_scatter.cu",
 ]
 
 NVCC_FLAGS = [

@@ -41,6 +41,10 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
                    const int32_t* indptr_i, const int32_t* indices_i, const int32_t* indptr_j,
                    const int32_t* indices_j, int num_rels, int feat, int nnz_i,
                    const float* z, cudaStream_t stream);
+int rgms_pairs_launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m,
+                      cudaStream_t st);
+int rgms_tma_launch_pairs(const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i, int num_rels,
+                          int nnz_i, const float* z, const int2* from, cudaStream_t stream);
 int rgms_wide_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i, const float* z,
                      int num_rels, int nnz_i, int feat, cudaStream_t stream);
 
@@ -186,13 +190,22 @@ size_t wide_scratch(int feat, int nnz_i) {
   return bytes <= (size_t{1} << 30) ? bytes : 0;
 }
 
+bool single_rows() {
+  static const bool chosen = [] {  // a comparison switch
+    const char* e = std::getenv("SPARSETIR_RGMS_PATH");
+    return e != nullptr && e[0] != '\0';
+  }();
+  return !chosen;
+}
+
 }  // namespace
 }  // namespace sptir
 
 extern "C" int sparsetir_rgms_workspace(int feat, int nnz_i, size_t* scratch_bytes) {
   if (!scratch_bytes || feat < 0 || nnz_i < 0) return sptir::fail("sparsetir_rgms_workspace: bad argument");
   // the two-launch form keeps one aggregated feature row per (relation, destination) pair
-  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : sptir::wide_scratch(feat, nnz_i);
+  // and where its row comes from
+  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * (feat * sizeof(float) + sizeof(int2)) : sptir::wide_scratch(feat, nnz_i);
   return 0;
 }
 
@@ -240,8 +253,22 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
         if (rc1 <= 0) return rc1;
       }
       float* z = nullptr;
-      if (!fused)
-        z = static_cast<float*>(workspace(device_id, st, static_cast<size_t>(nnz_i) * 64 * sizeof(float)));
+      if (!fused) {
+        const size_t z_bytes = static_cast<size_t>(nnz_i) * 64 * sizeof(float), all = z_bytes + static_cast<size_t>(nnz_i) * sizeof(int2);
+        if (single_rows()) {
+          // a captured call keeps to what has been reserved
+          cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+          SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+          if (capture == cudaStreamCaptureStatusNone || workspace_fits(device_id, st, all, 0)) z = static_cast<float*>(workspace(device_id, st, all));
+          if (z != nullptr) {
+            int2* from = reinterpret_cast<int2*>(z + static_cast<size_t>(nnz_i) * 64);
+            if (rgms_pairs_launch(a, x, z, from, indptr_j, indices_j, nnz_i, st) != 0) return -1;
+            const int rc2 = rgms_tma_launch_pairs(w, x, y, indptr_i, indices_i, num_rels, nnz_i, z, from, st);
+            if (rc2 <= 0) return rc2;
+          }
+        }
+        z = static_cast<float*>(workspace(device_id, st, z_bytes));
+      }
       if (z != nullptr) {
         if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, 64, nnz_j, device_id, stream) != 0)
           return -1;

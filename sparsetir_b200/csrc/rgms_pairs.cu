@@ -1,0 +1,131 @@
+// The first launch of RGMS at 64 features where many (relation, destination) pairs have one edge: those need no sum, and the
+// transform (rgms_tc.cu) can take their row straight from X.
+//   Z[t,:] = sum_{p in CSF row t} A[p] * X[J[p],:]   for rows of two entries and more (and zeros for rows without);
+//   from[t] = (J[p], A[p])                           for rows of one;  (-1, 1) for the others: the row lies in Z.
+//
+// 100 k nodes, 46 relations, 1.5 M edges: 530 k of the 690 k pairs have one edge.  With a row of Z for each of them the SpMM kernel
+// gathered 401 MB and wrote 177 in 57 us; 248 and 41 MB are left.
+//
+// A group of LPR lanes takes LPR consecutive rows: lane j looks at row j, and the entries of the rows of two and more are one
+// stream, LPR at a time (the row of an entry by a search in the running sum of the lengths, in registers), with the ids of
+// the next batch on their way and 8 (16-byte lanes) or 4 (32-byte lanes) rows of X in flight.
+#include "common.h"
+#include "launch.cuh"
+#include "vec.cuh"
+
+namespace sptir {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kF = 64;
+
+template <int LPR, int W>
+__global__ void __launch_bounds__(kThreads, 4)
+rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z, int2* __restrict__ from,
+                  const int32_t* indptr, const int32_t* indices, int m, int rpi) {
+  static_assert(LPR * W == kF, "a group covers a row");
+  using LV = LaneVec<W>;
+  constexpr int SUBS = kThreads / LPR;
+  constexpr int U = 32 / W;
+  const int lane = threadIdx.x % LPR, shift = (threadIdx.x & 31) / LPR * LPR;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr unsigned kGroup = LPR == 32 ? kAll : (1u << LPR) - 1u;
+  const long long r0l = (static_cast<long long>(blockIdx.x) * SUBS + threadIdx.x / LPR) * rpi;
+  chain_wait();
+  const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m))), row = r0 + lane;
+  const bool there = lane < rpi && row < m;
+  const int begin = ld_global(indptr + min(row, m)), len = there ? ld_global(indptr + min(row + 1, m)) - begin : -1;
+  int src = -1;
+  float scale = 1.f;
+  if (len == 1) {
+    src = ld_global(indices + begin);
+    scale = ld_global(a + begin);
+  }
+  const int own = len >= 2 ? len : 0;
+  int upto = own;  // entries of the rows up to this lane's
+#pragma unroll
+  for (int o = 1; o < LPR; o <<= 1) {
+    const int v = __shfl_up_sync(kAll, upto, o, LPR);
+    if (lane >= o) upto += v;
+  }
+  const int total = __shfl_sync(kAll, upto, LPR - 1, LPR);
+  const int steps = __reduce_max_sync(kAll, total);  // the groups of a warp run in step
+  const int base = begin - (upto - own);  // position of entry e of the stream, if it is in this lane's row: base + e
+  char* zl = reinterpret_cast<char*>(z) + static_cast<size_t>(r0) * (kF * 4) + lane * (W * 4);
+  const char* xl = reinterpret_cast<const char*>(x) + lane * (W * 4);
+
+  for (unsigned empty = (__ballot_sync(kAll, len == 0) >> shift) & kGroup; empty != 0u; empty &= empty - 1u)
+    LV::stcg(zl + (__ffs(empty) - 1) * (kF * 4), LV::zero());
+
+  int cid = 0, at = 0;   // of the batch to come: column, row inside the group
+  float av = 0.f;
+  unsigned ends = 0;     // bit k: the row of entry k ends with it
+  auto request = [&](int e0) {  // lanes past the group's last entry repeat it: it is added to a sum that nobody stores
+    const int e = min(e0 + lane, total - 1);
+    int pos = 0;
+#pragma unroll
+    for (int step = LPR / 2; step >= 1; step >>= 1)
+      if (__shfl_sync(kAll, upto, pos + step - 1, LPR) <= e) pos += step;
+    const int p = __shfl_sync(kAll, base, pos, LPR) + e;
+    const bool last = __shfl_sync(kAll, upto, pos, LPR) == e + 1 && e0 + lane < total;
+    at = pos * (kF * 4);
+    ends = (__ballot_sync(kAll, last) >> shift) & kGroup;
+    if (total > 0) {
+      cid = ld_global(indices + p);
+      av = ld_global(a + p);
+    }
+  };
+  if (steps > 0) request(0);
+  typename LV::type acc = LV::zero();
+  for (int e0 = 0; e0 < steps; e0 += LPR) {
+    const int cid_now = cid, at_now = at, left = total - e0;
+    const float av_now = av;
+    const unsigned ends_now = ends, any_ends = __reduce_or_sync(kAll, ends);
+    if (e0 + LPR < steps) request(e0 + LPR);
+#pragma unroll
+    for (int k0 = 0; k0 < LPR; k0 += U) {
+      if (k0 < steps - e0) {
+        typename LV::type v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned col = static_cast<unsigned>(__shfl_sync(kAll, cid_now, k0 + u, LPR));
+          v[u] = LV::zero();
+          if (k0 + u < left) v[u] = LV::ldg(xl + static_cast<unsigned long long>(col) * (kF * 4));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          LV::fma(acc, __shfl_sync(kAll, av_now, k0 + u, LPR), v[u]);
+          if ((any_ends >> (k0 + u)) & 1u) {  // a row ends here in some group of the warp
+            const int to = __shfl_sync(kAll, at_now, k0 + u, LPR);
+            const bool end = (ends_now >> (k0 + u)) & 1u;
+            if (end) LV::stcg(zl + to, acc);
+            LV::zero_if(acc, end);
+          }
+        }
+      }
+    }
+  }
+  if (there) from[row] = make_int2(src, __float_as_int(scale));
+}
+
+template <int LPR, int W>
+int launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st) {
+  // fewer rows per group where the groups would not fill the SMs
+  constexpr int kGroups = kThreads / LPR;
+  int rpi = LPR;
+  while (rpi > 1 && ceil_div(m, rpi) < kNumSMs * 4 * kGroups) rpi /= 2;
+  launch_chained(rgms_pairs_kernel<LPR, W>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, from, indptr, indices, m, rpi);
+  SPTIR_LAUNCH_OK("rgms_pairs_kernel");
+  return 0;
+}
+
+}  // namespace
+
+int rgms_pairs_launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m,
+                      cudaStream_t st) {
+  // 32-byte lanes lose where there are too few rows for the groups (3 k nodes, 12 k edges, the call 12.3 us with 16 bytes, 13.9 with 32)
+  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8>(a, x, z, from, indptr, indices, m, st);
+  return launch<16, 4>(a, x, z, from, indptr, indices, m, st);
+}
+
+}  // namespace sptir

@@ -245,8 +245,8 @@ rgms_tc_kernel(const float* __restrict__ a, const float* __restrict__ w,
 // Every mbarrier wait is bounded.
 constexpr int kPThreads = 512;
 constexpr int kZStages = 4;
-constexpr uint32_t kPTmem = 512;         // two accumulators of 128 columns, two tiles of remainders of 64
-constexpr uint32_t kTmemLo = 4 * kF;     // column of the first remainders
+constexpr uint32_t kPTmem = 512;         // two accumulators of 128 columns, two tiles of rows and their remainders of 64 each
+constexpr uint32_t kTmemZ = 4 * kF;      // column of the first rows
 constexpr int kZBox = kTM * 128;     // one swizzled box: 128 rows x 32 floats
 constexpr int kZTile = 2 * kZBox;    // 32 KB
 // W_r as ONE operand of 128 rows: rows 0..63 = W (its upper 19 bits are what the tensor core
@@ -267,15 +267,17 @@ __device__ __forceinline__ int swz_off(int row, int kc, int box_bytes) {
   return (kc >> 3) * box_bytes + (row >> 3) * 1024 + (row & 7) * 128 + (((kc & 7) ^ (row & 7)) << 4);
 }
 
-__global__ void __launch_bounds__(kPThreads, 1)
-rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
+template <bool GATHER>
+__global__ void __launch_bounds__(kPThreads + (GATHER ? 128 : 0), 1)
+rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const float* x, const int2* from, const float* w,
                 float* __restrict__ y, const int32_t* indptr_i,
                 const int32_t* indices_i, int num_rels, int nnz_i, int tiles_per_cta,
                 int rel_mod) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kZStages];   // z rows of the stage have landed
-  __shared__ __align__(8) uint64_t bar_conv[2];          // remainders written (128 arrivals)
-  __shared__ __align__(8) uint64_t bar_empty[kZStages];  // tensor core has read the stage
+  __shared__ __align__(8) uint64_t bar_empty[kZStages];  // the converters have read the stage (128 arrivals)
+  __shared__ __align__(8) uint64_t bar_conv[2];          // rows and remainders in tensor memory (128 arrivals)
+  __shared__ __align__(8) uint64_t bar_used[2];          // the tensor core has read them
   __shared__ __align__(8) uint64_t bar_acc_full[2];      // accumulator holds a finished tile
   __shared__ __align__(8) uint64_t bar_acc_empty[2];     // epilogue has read it (128 arrivals)
   __shared__ uint32_t s_tmem;
@@ -286,16 +288,17 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
   if (warp == 0) {
     if (lane == 0) {
       for (int s = 0; s < kZStages; ++s) {
-        tc05::mbar_init(&bar_full[s], 1);
-        tc05::mbar_init(&bar_empty[s], 1);
+        tc05::mbar_init(&bar_full[s], GATHER ? 128 : 1);
+        tc05::mbar_init(&bar_empty[s], 128);
       }
       for (int b = 0; b < 2; ++b) {
         tc05::mbar_init(&bar_conv[b], 128);
+        tc05::mbar_init(&bar_used[b], 1);
         tc05::mbar_init(&bar_acc_full[b], 1);
         tc05::mbar_init(&bar_acc_empty[b], 128);
       }
       tc05::fence_mbar_init();
-      tc05::prefetch_tensormap(&tm_z);
+      if (!GATHER) tc05::prefetch_tensormap(&tm_z);
     }
     __syncwarp();
     tc05::tmem_alloc(&s_tmem, kPTmem);
@@ -321,9 +324,34 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
   bool ok = true;
   int armed = 0;
 
-  if (warp == 0) {
+  if (GATHER && warp >= 16) {
+    // ---- gather: lane = tile row, whose source it holds; two rows per copy, 16 bytes per lane
+    const int t0 = (warp & 3) * 32, piece = lane & 15, half = lane >> 4;
+    uint32_t put[4];  // of the lane's piece of rows 2i + half, which repeat every eight rows
+#pragma unroll
+    for (int i = 0; i < 4; ++i) put[i] = tc05::smem_u32(base + kOffZRaw) + swz_off(t0 + 2 * i + half, piece, kZBox);
+    auto source = [&]() { return ld_global(&from[min(tw.row0 + t0 + lane, nnz_i - 1)].x); };
+    int src = source();
+    for (int k = 0; k < tiles_per_cta; ++k) {
+      const int s = k % kZStages, use = k / kZStages;
+      const int row0 = tw.row0, nrows = tw.row1 - tw.row0, src_now = src;
+      const bool more = k + 1 < tiles_per_cta && tw.next(indptr_i, num_rels);
+      if (more) src = source();
+      if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int t = t0 + 2 * i + half, col = __shfl_sync(0xffffffffu, src_now, 2 * i + half);
+        const float* row = col >= 0 ? x + static_cast<size_t>(col) * kF : z + static_cast<size_t>(min(row0 + t, nnz_i - 1)) * kF;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(put[i & 3] + s * kZTile + (i >> 2) * 1024), "l"(row + piece * 4),
+                     "r"(t < nrows ? 16 : 0) : "memory");  // zeros past the last row
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc05::smem_u32(&bar_full[s])) : "memory");
+      if (!more) break;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");  // also when giving up: nothing may land later
+  } else if (warp == 0) {
     // ---- producer
-    if (lane == 0) {
+    if (!GATHER && lane == 0) {
       for (int k = 0; k < tiles_per_cta; ++k) {
         const int s = k % kZStages, use = k / kZStages;
         if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
@@ -347,24 +375,21 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
       // descriptors are built once; the loop only advances their address fields (a lone thread
       // issues one dependent instruction every few clocks)
       const uint64_t dw0 = tc05::smem_desc_swizzled(tc05::smem_u32(base + kOffW), 0, 1024, tc05::kSwizzle128B);
-      const uint64_t dzh0 = tc05::smem_desc_swizzled(tc05::smem_u32(base + kOffZRaw), 0, 1024, tc05::kSwizzle128B);
       for (int k = 0; k < tiles_per_cta; ++k) {
-        const int s = k % kZStages, use = k / kZStages, buf = k & 1, buse = k >> 1;
-        if (!tc05::mbar_wait(&bar_full[s], use & 1)) { ok = false; break; }
+        const int buf = k & 1, buse = k >> 1;
         if (!tc05::mbar_wait(&bar_conv[buf], buse & 1)) { ok = false; break; }
         if (buse > 0 && !tc05::mbar_wait(&bar_acc_empty[buf], (buse - 1) & 1)) { ok = false; break; }
         tc05::fence_after_sync();
-        const uint64_t dzh_s = tc05::desc_advance(dzh0, s * kZTile);
-        const uint32_t zlo = tmem + kTmemLo + buf * kF;
+        const uint32_t zrow = tmem + kTmemZ + buf * 2 * kF, zlo = zrow + kF;
         const uint32_t acc = tmem + buf * 2 * kF;
 #pragma unroll
         for (int ks = 0; ks < kF / 8; ++ks) {  // K = 8 floats = 32 bytes inside the swizzled row
-          const uint32_t zo = (ks >> 2) * kZBox + (ks & 3) * 32, wo = (ks >> 2) * kWBox + (ks & 3) * 32;
+          const uint32_t wo = (ks >> 2) * kWBox + (ks & 3) * 32;
           const uint64_t dw = tc05::desc_advance(dw0, wo);
-          tc05::mma_tf32(acc, tc05::desc_advance(dzh_s, zo), dw, idesc128, ks > 0 ? 1u : 0u);
+          tc05::mma_tf32_ts(acc, zrow + ks * 8, dw, idesc128, ks > 0 ? 1u : 0u);
           tc05::mma_tf32_ts(acc, zlo + ks * 8, dw, idesc64, 1u);
         }
-        tc05::mma_commit(&bar_empty[s]);
+        tc05::mma_commit(&bar_used[buf]);
         tc05::mma_commit(&bar_acc_full[buf]);
         if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
       }
@@ -373,13 +398,16 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
     // ---- converters
     const int ct = tid - 256;
     int staged_rel = -1;
+    auto scale_of = [&]() { return GATHER ? __int_as_float(ld_global(&from[min(tw.row0 + ct, nnz_i - 1)].y)) : 1.f; };
+    float scale_next = scale_of();
     for (int k = 0; k < tiles_per_cta; ++k) {
       const int s = k % kZStages, use = k / kZStages;
+      const float scale = scale_next;  // of a row that came from X
       // rel_mod > 0: the row ranges are (bucket, relation) pairs, W is indexed by the relation
       const int wrel = rel_mod > 0 ? tw.rel % rel_mod : tw.rel;
       if (wrel != staged_rel) {
         // the MMAs of the previous tile are the last readers of the staged W
-        if (k > 0 && !tc05::mbar_wait(&bar_empty[(k - 1) % kZStages], ((k - 1) / kZStages) & 1)) { ok = false; break; }
+        if (k > 0 && !tc05::mbar_wait(&bar_used[(k - 1) & 1], ((k - 1) >> 1) & 1)) { ok = false; break; }
         staged_rel = wrel;
         const float4* wr = reinterpret_cast<const float4*>(w + static_cast<size_t>(wrel) * kF * kF);
         for (int ch = ct; ch < kF * kF / 4; ch += 128) {
@@ -391,32 +419,37 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
         }
       }
       if (!tc05::mbar_wait(&bar_full[s], use & 1)) { ok = false; break; }
-      // the remainders of the tile before the last one have been read
-      if (k > 1 && !tc05::mbar_wait(&bar_empty[(k - 2) % kZStages], ((k - 2) / kZStages) & 1)) { ok = false; break; }
+      // the rows of the tile before the last one have been read
+      if (k > 1 && !tc05::mbar_wait(&bar_used[k & 1], ((k - 2) >> 1) & 1)) { ok = false; break; }
       tc05::fence_after_sync();
       const unsigned char* zr = base + kOffZRaw + s * kZTile;
-      const uint32_t zlo = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kTmemLo + (k & 1) * kF;
+      const uint32_t zrow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kTmemZ + (k & 1) * 2 * kF;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t r[32];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float4 v = *reinterpret_cast<const float4*>(zr + swz_off(ct, half * 8 + j, kZBox));
-          r[4 * j] = __float_as_uint(v.x - tf32_hi(v.x));
-          r[4 * j + 1] = __float_as_uint(v.y - tf32_hi(v.y));
-          r[4 * j + 2] = __float_as_uint(v.z - tf32_hi(v.z));
-          r[4 * j + 3] = __float_as_uint(v.w - tf32_hi(v.w));
+          r[4 * j] = __float_as_uint(GATHER ? v.x * scale : v.x);
+          r[4 * j + 1] = __float_as_uint(GATHER ? v.y * scale : v.y);
+          r[4 * j + 2] = __float_as_uint(GATHER ? v.z * scale : v.z);
+          r[4 * j + 3] = __float_as_uint(GATHER ? v.w * scale : v.w);
         }
+        if (half == 1) mbar_arrive(&bar_empty[s]);
         __syncwarp();
-        tc05::tmem_st32(zlo + half * 32, r);
+        tc05::tmem_st32(zrow + half * 32, r);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(__uint_as_float(r[q]) - tf32_hi(__uint_as_float(r[q])));
+        tc05::tmem_st32(zrow + kF + half * 32, r);
       }
       tc05::tmem_st_wait();
       tc05::fence_before_sync();
       tc05::fence_async_smem();  // W, if it was staged for this tile
       mbar_arrive(&bar_conv[k & 1]);
       if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
+      scale_next = scale_of();
     }
-  } else if (warp >= 4) {
+  } else if (warp >= 4 && warp < 16) {
     // ---- epilogue, two groups of four warps: group 0 (warps 4-7) takes the even tiles and
     // accumulator 0, group 1 (warps 12-15) the odd tiles and accumulator 1, so that one group
     // reads TMEM and transposes while the other is busy issuing its atomics.
@@ -485,9 +518,10 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* w,
   if (warp == 0) tc05::tmem_dealloc(tmem, kPTmem);
 }
 
-// 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error
+// 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error.  x, from: as rgms_pairs.cu leaves
+// them, or null: every row lies in z.
 int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i,
-                    int num_rels, int nnz_i, const float* z, cudaStream_t stream, int rel_mod = 0) {
+                    int num_rels, int nnz_i, const float* z, const float* x, const int2* from, cudaStream_t stream, int rel_mod = 0) {
   if (nnz_i <= 0 || num_rels <= 0) return 1;
   if ((reinterpret_cast<uintptr_t>(z) & 15u) || (reinterpret_cast<uintptr_t>(y) & 15u) ||
       (reinterpret_cast<uintptr_t>(w) & 15u))
@@ -500,14 +534,19 @@ int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int
   int dev = 0;
   SPTIR_CUDA_OK(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    SPTIR_CUDA_OK(cudaFuncSetAttribute(rgms_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmemBytes));
+    SPTIR_CUDA_OK(cudaFuncSetAttribute(rgms_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmemBytes));
+    SPTIR_CUDA_OK(cudaFuncSetAttribute(rgms_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmemBytes));
     configured_device = dev;
   }
   const long long tiles = static_cast<long long>(nnz_i) / kTM + num_rels;  // upper bound
   const long long grid = tiles < kNumSMs ? tiles : kNumSMs;
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
-  launch_chained(rgms_tma_kernel, static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream, tm_z, w, y, indptr_i, indices_i,
-                 num_rels, nnz_i, tiles_per_cta, rel_mod);
+  if (from != nullptr)
+    launch_chained(rgms_tma_kernel<true>, static_cast<unsigned>(grid), kPThreads + 128, kPSmemBytes, stream, tm_z, z, x, from, w, y, indptr_i,
+                   indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
+  else
+    launch_chained(rgms_tma_kernel<false>, static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream, tm_z, z, x, from, w, y, indptr_i,
+                   indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
   SPTIR_LAUNCH_OK("rgms_tma_kernel");
   return 0;
 }
@@ -524,7 +563,14 @@ int rgms_tma_launch_ranges(const float* w, float* y, const int32_t* indptr_i, co
     return !(e && std::strcmp(e, "regs") == 0);
   }();
   if (!use_tma) return 1;
-  return rgms_tma_launch(w, y, indptr_i, indices_i, num_ranges, nnz_i, z, stream, rel_mod);
+  return rgms_tma_launch(w, y, indptr_i, indices_i, num_ranges, nnz_i, z, nullptr, nullptr, stream, rel_mod);
+}
+
+// The second launch behind rgms_pairs_launch(): rows of one entry straight from X.  0 when launched, 1 when this path cannot take the
+// call, -1 on error.
+int rgms_tma_launch_pairs(const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i, int num_rels,
+                          int nnz_i, const float* z, const int2* from, cudaStream_t stream) {
+  return rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, x, from, stream);
 }
 
 // Returns 0 when launched, 1 when the shape is not handled here, -1 on error.
@@ -540,7 +586,7 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
     return !(e && std::strcmp(e, "regs") == 0);
   }();
   if (z != nullptr && use_tma) {
-    const int rc = rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, stream);
+    const int rc = rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, nullptr, nullptr, stream);
     if (rc <= 0) return rc;
   }
   static thread_local int configured_device = -1;
