@@ -41,10 +41,10 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
                    const int32_t* indptr_i, const int32_t* indices_i, const int32_t* indptr_j,
                    const int32_t* indices_j, int num_rels, int feat, int nnz_i,
                    const float* z, cudaStream_t stream);
-int rgms_pairs_launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m,
-                      cudaStream_t st);
-int rgms_tma_launch_pairs(const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i, int num_rels,
-                          int nnz_i, const float* z, const int2* from, cudaStream_t stream);
+int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st);
+int rgms_tma_launch_pairs(const float* a, const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i,
+                          const int32_t* indptr_j, const int32_t* indices_j, int num_rels, int nnz_i, const float* z,
+                          cudaStream_t stream);
 int rgms_wide_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i, const float* z,
                      int num_rels, int nnz_i, int feat, cudaStream_t stream);
 
@@ -190,6 +190,7 @@ size_t wide_scratch(int feat, int nnz_i) {
   return bytes <= (size_t{1} << 30) ? bytes : 0;
 }
 
+// Whether the rows of one edge are taken from X.
 bool single_rows() {
   static const bool chosen = [] {  // a comparison switch
     const char* e = std::getenv("SPARSETIR_RGMS_PATH");
@@ -204,8 +205,7 @@ bool single_rows() {
 extern "C" int sparsetir_rgms_workspace(int feat, int nnz_i, size_t* scratch_bytes) {
   if (!scratch_bytes || feat < 0 || nnz_i < 0) return sptir::fail("sparsetir_rgms_workspace: bad argument");
   // the two-launch form keeps one aggregated feature row per (relation, destination) pair
-  // and where its row comes from
-  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * (feat * sizeof(float) + sizeof(int2)) : sptir::wide_scratch(feat, nnz_i);
+  *scratch_bytes = feat == 64 ? static_cast<size_t>(nnz_i) * feat * sizeof(float) : sptir::wide_scratch(feat, nnz_i);
   return 0;
 }
 
@@ -230,10 +230,11 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
   const bool al = aligned16(x) && aligned16(y) && aligned16(w);
   if (al) {
     if (feat == 64) {
-      // Two launches: (1) Z = A_csf * X, one row per (relation, destination) pair, with the CSR
-      // SpMM kernel — thousands of independent short rows in flight instead of one latency chain
-      // per tile; (2) the tensor-core tile product and scatter, reading Z tiles with coalesced
-      // loads.  Z (nnz_i x 64 floats) lives in the library's per-stream scratch buffer.
+      // Two launches: (1) Z = A_csf * X, one row per (relation, destination) pair of two edges and more: thousands of
+      // independent short rows in flight instead of one latency chain per tile; (2) the tensor-core tile product and scatter,
+      // which takes the rows of one edge from X (rgms_pairs.cu).  Z (nnz_i x 64 floats) lies in the library's per-stream scratch
+      // buffer.  With every row through Z 100 k nodes, 1.5 M edges, 46 relations took 126 us instead of 99, and layers without
+      // rows of one edge lose nothing (one relation of 64 edges per row 176 / 153).
       // SPARSETIR_RGMS_FUSED=1 selects the single fused kernel instead (no scratch).
       static const bool fused = [] {
         const char* e = std::getenv("SPARSETIR_RGMS_FUSED");
@@ -242,7 +243,7 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
       // SPARSETIR_RGMS_PATH=fused selects the one-launch form of rgms_fused.cu instead: it gathers,
       // multiplies and scatters tile by tile and needs no scratch memory, but its sixteen gather
       // warps per SM keep fewer loads in flight than a whole launch of the SpMM kernel does
-      // (measured at 100 k nodes / 1.5 M edges: 183 us against 139 us for the two launches).
+      // (measured at 100 k nodes / 1.5 M edges: 183 us against 99 us for the two launches).
       static const bool one_launch = [] {
         const char* e = std::getenv("SPARSETIR_RGMS_PATH");
         return e != nullptr && std::strcmp(e, "fused") == 0;
@@ -253,21 +254,12 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
         if (rc1 <= 0) return rc1;
       }
       float* z = nullptr;
-      if (!fused) {
-        const size_t z_bytes = static_cast<size_t>(nnz_i) * 64 * sizeof(float), all = z_bytes + static_cast<size_t>(nnz_i) * sizeof(int2);
-        if (single_rows()) {
-          // a captured call keeps to what has been reserved
-          cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-          SPTIR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
-          if (capture == cudaStreamCaptureStatusNone || workspace_fits(device_id, st, all, 0)) z = static_cast<float*>(workspace(device_id, st, all));
-          if (z != nullptr) {
-            int2* from = reinterpret_cast<int2*>(z + static_cast<size_t>(nnz_i) * 64);
-            if (rgms_pairs_launch(a, x, z, from, indptr_j, indices_j, nnz_i, st) != 0) return -1;
-            const int rc2 = rgms_tma_launch_pairs(w, x, y, indptr_i, indices_i, num_rels, nnz_i, z, from, st);
-            if (rc2 <= 0) return rc2;
-          }
-        }
-        z = static_cast<float*>(workspace(device_id, st, z_bytes));
+      if (!fused)
+        z = static_cast<float*>(workspace(device_id, st, static_cast<size_t>(nnz_i) * 64 * sizeof(float)));
+      if (z != nullptr && single_rows()) {
+        if (rgms_pairs_launch(a, x, z, indptr_j, indices_j, nnz_i, st) != 0) return -1;
+        const int rc2 = rgms_tma_launch_pairs(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, z, st);
+        if (rc2 <= 0) return rc2;
       }
       if (z != nullptr) {
         if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, 64, nnz_j, device_id, stream) != 0)

@@ -1,14 +1,17 @@
 // The first launch of RGMS at 64 features where many (relation, destination) pairs have one edge: those need no sum, and the
 // transform (rgms_tc.cu) can take their row straight from X.
-//   Z[t,:] = sum_{p in CSF row t} A[p] * X[J[p],:]   for rows of two entries and more (and zeros for rows without);
-//   from[t] = (J[p], A[p])                           for rows of one;  (-1, 1) for the others: the row lies in Z.
+//   Z[t,:] = sum_{p in CSF row t} A[p] * X[J[p],:]   for rows of two entries and more, and zeros for rows without;
+// rows of one are left out.
 //
 // 100 k nodes, 46 relations, 1.5 M edges: 530 k of the 690 k pairs have one edge.  With a row of Z for each of them the SpMM kernel
-// gathered 401 MB and wrote 177 in 57 us; 248 and 41 MB are left.
+// gathered 401 MB and wrote 177 in 57 us; 248 and 41 MB are left, 34 us.
 //
 // A group of LPR lanes takes LPR consecutive rows: lane j looks at row j, and the entries of the rows of two and more are one
 // stream, LPR at a time (the row of an entry by a search in the running sum of the lengths, in registers), with the ids of
-// the next batch on their way and 8 (16-byte lanes) or 4 (32-byte lanes) rows of X in flight.
+// the next batch on their way and 8 (16-byte lanes) or 4 (32-byte lanes) rows of X in flight.  The groups of a warp run in step:
+// with branches of their own they executed 20.2 M instructions and took 47 us instead of 14.5 M and 37 (counters of one launch).
+// What bounds it is the latency of the gathers (10 of 16 waiting warps; L1 data path 49 %, issue slots 34 %, L2 35 %); twice the rows
+// in flight on half the warps is slower (the call 112 us against 99).
 #include "common.h"
 #include "launch.cuh"
 #include "vec.cuh"
@@ -21,7 +24,7 @@ constexpr int kF = 64;
 
 template <int LPR, int W>
 __global__ void __launch_bounds__(kThreads, 4)
-rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z, int2* __restrict__ from,
+rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
                   const int32_t* indptr, const int32_t* indices, int m, int rpi) {
   static_assert(LPR * W == kF, "a group covers a row");
   using LV = LaneVec<W>;
@@ -35,12 +38,6 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z, int2* _
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m))), row = r0 + lane;
   const bool there = lane < rpi && row < m;
   const int begin = ld_global(indptr + min(row, m)), len = there ? ld_global(indptr + min(row + 1, m)) - begin : -1;
-  int src = -1;
-  float scale = 1.f;
-  if (len == 1) {
-    src = ld_global(indices + begin);
-    scale = ld_global(a + begin);
-  }
   const int own = len >= 2 ? len : 0;
   int upto = own;  // entries of the rows up to this lane's
 #pragma unroll
@@ -105,27 +102,26 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z, int2* _
       }
     }
   }
-  if (there) from[row] = make_int2(src, __float_as_int(scale));
 }
 
 template <int LPR, int W>
-int launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st) {
+int launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st) {
   // fewer rows per group where the groups would not fill the SMs
   constexpr int kGroups = kThreads / LPR;
   int rpi = LPR;
   while (rpi > 1 && ceil_div(m, rpi) < kNumSMs * 4 * kGroups) rpi /= 2;
-  launch_chained(rgms_pairs_kernel<LPR, W>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, from, indptr, indices, m, rpi);
+  launch_chained(rgms_pairs_kernel<LPR, W>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, indptr, indices, m, rpi);
   SPTIR_LAUNCH_OK("rgms_pairs_kernel");
   return 0;
 }
 
 }  // namespace
 
-int rgms_pairs_launch(const float* a, const float* x, float* z, int2* from, const int32_t* indptr, const int32_t* indices, int m,
+int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m,
                       cudaStream_t st) {
   // 32-byte lanes lose where there are too few rows for the groups (3 k nodes, 12 k edges, the call 12.3 us with 16 bytes, 13.9 with 32)
-  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8>(a, x, z, from, indptr, indices, m, st);
-  return launch<16, 4>(a, x, z, from, indptr, indices, m, st);
+  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8>(a, x, z, indptr, indices, m, st);
+  return launch<16, 4>(a, x, z, indptr, indices, m, st);
 }
 
 }  // namespace sptir

@@ -225,11 +225,12 @@ rgms_tc_kernel(const float* __restrict__ a, const float* __restrict__ w,
 // tiles to each other through mbarriers, so loading, splitting, multiplying and scattering of
 // different tiles overlap:
 //   warp 0      producer: two TMA tile loads (128 rows x 128 bytes, 128-byte swizzle) bring the
-//               tile's z rows into one of four stages;
-//   warps 8-11  converters: the tensor core reads only the upper 19 bits of an fp32 operand, so
-//               the raw tile serves as the "high" part as it is; the converters (thread = tile row)
-//               compute the remainder z - tf32(z) element by element into TMEM, where the MMAs take
-//               it as their left operand, and stage W_r (raw and remainder) when the relation changes;
+//               tile's z rows into one of four stages; with rows of one edge left in X (GATHER), four more warps copy the
+//               rows from X or Z instead, 16 bytes per lane, and the copies arrive at the stage's barrier themselves;
+//   warps 8-11  converters (thread = tile row): the row, times its value if it came from X, and the remainders
+//               z - tf32(z) go into tensor memory, where the MMAs take them as their left operand (the tensor core reads only
+//               the upper 19 bits of an fp32 operand, so the row serves as the "high" part as it is); they stage W_r (raw and
+//               remainder) when the relation changes;
 //   warp 1      issues the 8 K-steps of the 3xTF32 product as two instructions each (W and its
 //               remainders stacked into one 128-row operand) into one of two TMEM accumulators
 //               of 128 columns, tcgen05.commit frees the stage and publishes the accumulator;
@@ -238,10 +239,9 @@ rgms_tc_kernel(const float* __restrict__ a, const float* __restrict__ w,
 //               into Y[I[t], :], four whole 128-byte lines per warp instruction.  (One bulk reduce-add per row, cp.reduce.async.bulk, was
 //               measured first: the block issues a bulk operation only every ~20 clocks, which
 //               made the epilogue the slowest role at 3,200 clocks per tile.)
-// With the remainders in shared memory there was room for two stages of raw tiles, and the MMAs read them from there a second
-// time (100 k nodes, 1.5 M edges: the call 128.1 us, with the remainders in TMEM 125.7; 20 k nodes, 90 relations, 200 k edges
-// 51.1 / 49.6).  What bounds it is the reductions into Y, which take 45 us in this launch and in the fp16 one
-// (counters of one launch: L1 data path 53 % of the elapsed time, DRAM 43 %, L2 36 %, tensor pipe 26 %, issue slots 24 %).
+// What bounds it: no role alone.  Of its 59 us at 100 k nodes and 1.5 M edges (148 blocks of 37 tiles) 35 are left without converters,
+// MMAs and epilogue, 47 without the epilogue, 56 without the converters, 53 without the reductions into Y (which take 31
+// by themselves); a third accumulator, three or four epilogue groups and twice the gathering warps changed nothing.
 // Every mbarrier wait is bounded.
 constexpr int kPThreads = 512;
 constexpr int kZStages = 4;
@@ -267,9 +267,66 @@ __device__ __forceinline__ int swz_off(int row, int kc, int box_bytes) {
   return (kc >> 3) * box_bytes + (row >> 3) * 1024 + (row & 7) * 128 + (((kc & 7) ^ (row & 7)) << 4);
 }
 
+// Where the rows of one entry lie: the CSF's second level and X (null: every row lies in z).
+struct PairRows {
+  const float* x;
+  const float* a;
+  const int32_t* indptr;
+  const int32_t* indices;
+};
+
+// What a thread needs of row `t` of every tile of its block in turn: from[p] (a column or a value) if the row has one entry p, `none` if
+// not.  The row pointers are read two tiles ahead and the entry one.
+template <class T>
+struct LookAhead {
+  TileWalk& tw;
+  const int32_t* indptr_i;
+  int num_rels, tiles;
+  const PairRows& pairs;
+  const T* from;
+  int t, nnz_i;
+  T none, value, value_next;
+  int row0, nrows, row0_next, nrows_next, begin, len;
+  bool more;
+  __device__ __forceinline__ LookAhead(TileWalk& walk, const int32_t* ptr_i, int rels, int num_tiles, const PairRows& p, const T* f,
+                                       int row, int rows, T other)
+      : tw(walk), indptr_i(ptr_i), num_rels(rels), tiles(num_tiles), pairs(p), from(f), t(row), nnz_i(rows), none(other), value(other) {
+    row0 = tw.row0;
+    nrows = tw.row1 - tw.row0;
+    more = false;
+    if (tiles == 0) return;
+    pointers(row0);
+    value = entry();
+    advance(0);
+  }
+  __device__ __forceinline__ void pointers(int tile_row0) {
+    const int r = min(tile_row0 + t, nnz_i - 1);
+    begin = ld_global(pairs.indptr + r);
+    len = ld_global(pairs.indptr + r + 1) - begin;
+  }
+  __device__ __forceinline__ T entry() const { return len == 1 ? ld_global(from + begin) : none; }
+  __device__ __forceinline__ void advance(int k) {  // the tile behind tile k: its rows and pointers
+    more = k + 1 < tiles && tw.next(indptr_i, num_rels);
+    if (more) {
+      row0_next = tw.row0;
+      nrows_next = tw.row1 - tw.row0;
+      pointers(row0_next);
+    }
+  }
+  // to the tile behind tile k; false when there is none
+  __device__ __forceinline__ bool next(int k) {
+    if (!more) return false;
+    value = entry();
+    row0 = row0_next;
+    nrows = nrows_next;
+    advance(k + 1);
+    return true;
+  }
+};
+
 template <bool GATHER>
 __global__ void __launch_bounds__(kPThreads + (GATHER ? 128 : 0), 1)
-rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const float* x, const int2* from, const float* w,
+rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const PairRows pairs, const float* w,
                 float* __restrict__ y, const int32_t* indptr_i,
                 const int32_t* indices_i, int num_rels, int nnz_i, int tiles_per_cta,
                 int rel_mod) {
@@ -330,18 +387,16 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     uint32_t put[4];  // of the lane's piece of rows 2i + half, which repeat every eight rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) put[i] = tc05::smem_u32(base + kOffZRaw) + swz_off(t0 + 2 * i + half, piece, kZBox);
-    auto source = [&]() { return ld_global(&from[min(tw.row0 + t0 + lane, nnz_i - 1)].x); };
-    int src = source();
+    LookAhead<int> ahead(tw, indptr_i, num_rels, tiles_per_cta, pairs, pairs.indices, t0 + lane, nnz_i, -1);
     for (int k = 0; k < tiles_per_cta; ++k) {
       const int s = k % kZStages, use = k / kZStages;
-      const int row0 = tw.row0, nrows = tw.row1 - tw.row0, src_now = src;
-      const bool more = k + 1 < tiles_per_cta && tw.next(indptr_i, num_rels);
-      if (more) src = source();
+      const int row0 = ahead.row0, nrows = ahead.nrows, src = ahead.value;
+      const bool more = ahead.next(k);
       if (use > 0 && !tc05::mbar_wait(&bar_empty[s], (use - 1) & 1)) { ok = false; break; }
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const int t = t0 + 2 * i + half, col = __shfl_sync(0xffffffffu, src_now, 2 * i + half);
-        const float* row = col >= 0 ? x + static_cast<size_t>(col) * kF : z + static_cast<size_t>(min(row0 + t, nnz_i - 1)) * kF;
+        const int t = t0 + 2 * i + half, col = __shfl_sync(0xffffffffu, src, 2 * i + half);
+        const float* row = col >= 0 ? pairs.x + static_cast<size_t>(col) * kF : z + static_cast<size_t>(min(row0 + t, nnz_i - 1)) * kF;
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(put[i & 3] + s * kZTile + (i >> 2) * 1024), "l"(row + piece * 4),
                      "r"(t < nrows ? 16 : 0) : "memory");  // zeros past the last row
       }
@@ -398,11 +453,12 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     // ---- converters
     const int ct = tid - 256;
     int staged_rel = -1;
-    auto scale_of = [&]() { return GATHER ? __int_as_float(ld_global(&from[min(tw.row0 + ct, nnz_i - 1)].y)) : 1.f; };
-    float scale_next = scale_of();
+    TileWalk twa = tw;
+    LookAhead<float> ahead(twa, indptr_i, num_rels, GATHER ? tiles_per_cta : 0, pairs, pairs.a, ct, nnz_i, 1.f);
     for (int k = 0; k < tiles_per_cta; ++k) {
       const int s = k % kZStages, use = k / kZStages;
-      const float scale = scale_next;  // of a row that came from X
+      const float scale = ahead.value;  // of a row that came from X
+      if (GATHER) ahead.next(k);
       // rel_mod > 0: the row ranges are (bucket, relation) pairs, W is indexed by the relation
       const int wrel = rel_mod > 0 ? tw.rel % rel_mod : tw.rel;
       if (wrel != staged_rel) {
@@ -447,7 +503,6 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
       tc05::fence_async_smem();  // W, if it was staged for this tile
       mbar_arrive(&bar_conv[k & 1]);
       if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
-      scale_next = scale_of();
     }
   } else if (warp >= 4 && warp < 16) {
     // ---- epilogue, two groups of four warps: group 0 (warps 4-7) takes the even tiles and
@@ -518,10 +573,9 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
   if (warp == 0) tc05::tmem_dealloc(tmem, kPTmem);
 }
 
-// 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error.  x, from: as rgms_pairs.cu leaves
-// them, or null: every row lies in z.
+// 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error
 int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i,
-                    int num_rels, int nnz_i, const float* z, const float* x, const int2* from, cudaStream_t stream, int rel_mod = 0) {
+                    int num_rels, int nnz_i, const float* z, const PairRows& pairs, cudaStream_t stream, int rel_mod = 0) {
   if (nnz_i <= 0 || num_rels <= 0) return 1;
   if ((reinterpret_cast<uintptr_t>(z) & 15u) || (reinterpret_cast<uintptr_t>(y) & 15u) ||
       (reinterpret_cast<uintptr_t>(w) & 15u))
@@ -541,11 +595,11 @@ int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int
   const long long tiles = static_cast<long long>(nnz_i) / kTM + num_rels;  // upper bound
   const long long grid = tiles < kNumSMs ? tiles : kNumSMs;
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
-  if (from != nullptr)
-    launch_chained(rgms_tma_kernel<true>, static_cast<unsigned>(grid), kPThreads + 128, kPSmemBytes, stream, tm_z, z, x, from, w, y, indptr_i,
+  if (pairs.x != nullptr)
+    launch_chained(rgms_tma_kernel<true>, static_cast<unsigned>(grid), kPThreads + 128, kPSmemBytes, stream, tm_z, z, pairs, w, y, indptr_i,
                    indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
   else
-    launch_chained(rgms_tma_kernel<false>, static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream, tm_z, z, x, from, w, y, indptr_i,
+    launch_chained(rgms_tma_kernel<false>, static_cast<unsigned>(grid), kPThreads, kPSmemBytes, stream, tm_z, z, pairs, w, y, indptr_i,
                    indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
   SPTIR_LAUNCH_OK("rgms_tma_kernel");
   return 0;
@@ -563,14 +617,15 @@ int rgms_tma_launch_ranges(const float* w, float* y, const int32_t* indptr_i, co
     return !(e && std::strcmp(e, "regs") == 0);
   }();
   if (!use_tma) return 1;
-  return rgms_tma_launch(w, y, indptr_i, indices_i, num_ranges, nnz_i, z, nullptr, nullptr, stream, rel_mod);
+  return rgms_tma_launch(w, y, indptr_i, indices_i, num_ranges, nnz_i, z, PairRows{}, stream, rel_mod);
 }
 
 // The second launch behind rgms_pairs_launch(): rows of one entry straight from X.  0 when launched, 1 when this path cannot take the
 // call, -1 on error.
-int rgms_tma_launch_pairs(const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i, int num_rels,
-                          int nnz_i, const float* z, const int2* from, cudaStream_t stream) {
-  return rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, x, from, stream);
+int rgms_tma_launch_pairs(const float* a, const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i,
+                          const int32_t* indptr_j, const int32_t* indices_j, int num_rels, int nnz_i, const float* z,
+                          cudaStream_t stream) {
+  return rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, PairRows{x, a, indptr_j, indices_j}, stream);
 }
 
 // Returns 0 when launched, 1 when the shape is not handled here, -1 on error.
@@ -586,7 +641,7 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
     return !(e && std::strcmp(e, "regs") == 0);
   }();
   if (z != nullptr && use_tma) {
-    const int rc = rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, nullptr, nullptr, stream);
+    const int rc = rgms_tma_launch(w, y, indptr_i, indices_i, num_rels, nnz_i, z, PairRows{}, stream);
     if (rc <= 0) return rc;
   }
   static thread_local int configured_device = -1;
