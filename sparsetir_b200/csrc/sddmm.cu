@@ -132,7 +132,7 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
 }
 
 // ---------------------------------------------------------------------------------------------
-// Lean variant for feature counts that are multiples of 32 with 32-byte aligned operands.
+// Lean variant for feature counts that are multiples of 32, or of 8 and 256 at most (PART), with 32-byte aligned operands.
 //
 // One launch covers a tile of 8*LPR consecutive features [foff, foff + 8*LPR) of every stored
 // position; the host walks the tiles with one launch each, the first storing C and the others
@@ -145,13 +145,24 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
 // more (sddmm_run).
 // With PEERS the finished value of every position (the last feature tile's pass) is also stored
 // into the peers' copies of c: 128 contiguous bytes per warp and peer, over NVLink.
-template <int LPR, bool PEERS>
-__global__ void __launch_bounds__(kThreads, LPR <= 8 ? 4 : 2)
+// A product that came out as a NaN, feature by feature.
+__device__ __noinline__ float plain_dot(const float* a, const float* b, int feat) {
+  float s = 0.f;
+  for (int f = 0; f < feat; ++f) s = fmaf(ld_global(a + f), ld_global(b + f), s);
+  return s;
+}
+
+template <int LPR, bool PEERS, bool PART>
+__global__ void __launch_bounds__(kThreads, LPR == 4 ? 4 : 2)
 sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
                   const int32_t* indptr, const int32_t* indices,
                   const float* scale, int m, int nnz, int ld, int foff, int accumulate,
                   int chunk, int last_tile, const __grid_constant__ PeerOut po) {
-  constexpr int U = LPR < 4 ? LPR : 4;  // gathered rows in flight per lane (8 registers each)
+  // Gathered rows in flight per lane (8 registers each).  Tiles of 64 features keep the eight of a batch in flight on half the blocks
+  // (us, four on four blocks per SM / eight on two: 20 M positions in 40 k rows F = 64 366 / 317, 10 M in 100 k rows F = 128,
+  // two tiles, 413 / 353, F = 256 827 / 704); tiles of 32 with two batches at once lose (117 M, F = 128 3720 / 4150), and so do wider
+  // ones with eight (F = 128 558 / 721).
+  constexpr int U = LPR == 8 ? 8 : 4;
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const unsigned mask = group_mask<LPR>();
@@ -160,8 +171,19 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
   chain_wait();
   if (e_begin >= nnz) return;
   const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + chunk));
-  const float* a_lane = a + foff + lane * 8;
-  const float* b_lane = b + foff + lane * 8;
+  // PART: lanes past the row load its first piece once more.  Groups of 8 and 16 multiply it by zeros, and what that makes a NaN is
+  // formed again; the others, which have no registers for that, mask their products (20 M positions, F = 72, a select that
+  // became a branch around each product 910 us, a mask, which spills, 800, zeros 595; F = 24 a mask 166, zeros 242).
+  constexpr bool kMask = PART && LPR != 8 && LPR != 16, kAgain = PART && !kMask;
+  const bool in = !PART || lane * 8 < ld - foff;
+  const unsigned keep_bits = in ? 0xffffffffu : 0u;
+  const float* a_lane = a + foff + (in ? lane * 8 : 0);
+  const float* b_lane = b + foff + (in ? lane * 8 : 0);
+  auto product = [&](const Pack4& p, const Pack4& q) {
+    const float d = dot8(p, q);
+    return kMask ? __uint_as_float(__float_as_uint(d) & keep_bits) : d;
+  };
+  auto row_of_a = [&](int r) { return in || kMask ? ldg256(a_lane + static_cast<size_t>(r) * ld) : pack4_zero(); };
 
   int warp_row = max(0, min(m - 1, warp_upper_bound(indptr, 0, m + 1, static_cast<int>(e_begin), wlane) - 1));
   int warp_end = ld_global(indptr + warp_row + 1);  // first position past the warp's current row
@@ -180,11 +202,12 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
       if (accumulate) old = c[e];
     }
     float part[LPR];
+    int row = warp_row;
     if (base + 32 <= min(warp_end, e_end)) {
       // every position of the batch lies in the warp's current row
       if (cur_row != warp_row) {
         cur_row = warp_row;
-        arow = ldg256(a_lane + static_cast<size_t>(cur_row) * ld);
+        arow = row_of_a(cur_row);
       }
 #pragma unroll
       for (int k0 = 0; k0 < LPR; k0 += U) {
@@ -193,10 +216,9 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
         for (int u = 0; u < U; ++u)
           x[u] = ldg256(b_lane + static_cast<size_t>(__shfl_sync(mask, col, k0 + u, LPR)) * ld);
 #pragma unroll
-        for (int u = 0; u < U; ++u) part[k0 + u] = dot8(arow, x[u]);
+        for (int u = 0; u < U; ++u) part[k0 + u] = product(arow, x[u]);
       }
     } else {
-      int row = warp_row;
       if (live) {
         int steps = 0;
         // row < m - 1 keeps every read inside indptr even if nnz disagrees with indptr[m]
@@ -224,9 +246,9 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
         for (int u = 0; u < U; ++u) {
           if (rk[u] != cur_row) {  // uniform inside the sub-warp
             cur_row = rk[u];
-            arow = ldg256(a_lane + static_cast<size_t>(cur_row) * ld);
+            arow = row_of_a(cur_row);
           }
-          part[k0 + u] = dot8(arow, x[u]);
+          part[k0 + u] = product(arow, x[u]);
         }
       }
     }
@@ -242,6 +264,9 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
       }
     }
     if (live) {
+      if constexpr (kAgain) {
+        if (part[0] != part[0]) part[0] = plain_dot(a + static_cast<size_t>(row) * ld, b + static_cast<size_t>(col) * ld, ld);
+      }
       const float v = fmaf(part[0], mul, old);
       c[e] = v;
       if constexpr (PEERS) {
@@ -284,14 +309,14 @@ int launch(const float* a, const float* b, float* c, const int32_t* indptr, cons
 }
 
 // Blocks of sddmm_lean_kernel<LPR> that fit one SM at a time (asked of the runtime once per device).
-template <int LPR>
+template <int LPR, bool PART>
 int lean_blocks_per_sm() {
   static thread_local int cached_device = -1, cached = 0;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 4;
   if (dev != cached_device) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sddmm_lean_kernel<LPR, false>, kThreads, 0) != cudaSuccess || n < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sddmm_lean_kernel<LPR, false, PART>, kThreads, 0) != cudaSuccess || n < 1)
       n = 4;
     cached = n;
     cached_device = dev;
@@ -299,7 +324,7 @@ int lean_blocks_per_sm() {
   return cached;
 }
 
-template <int LPR>
+template <int LPR, bool PART>
 int launch_lean_tile(const float* a, const float* b, float* c, const int32_t* indptr,
                      const int32_t* indices, const float* scale, int m, int feat, int nnz, int foff,
                      int last_tile, const PeerOut& po, cudaStream_t stream) {
@@ -307,16 +332,20 @@ int launch_lean_tile(const float* a, const float* b, float* c, const int32_t* in
   // launch of a few waves ends with a partly filled one otherwise (3.02 waves cost as much as 4;
   // 1.7 M positions, F = 64: 59 us in 1.4 waves of 256 positions per warp).
   const int wpb = kThreads / 32;
-  const long long resident = static_cast<long long>(kNumSMs) * lean_blocks_per_sm<LPR>() * wpb;
+  const long long resident = static_cast<long long>(kNumSMs) * lean_blocks_per_sm<LPR, PART>() * wpb;
   const long long waves = std::max<long long>(1, (nnz / 1024 + resident / 2) / resident);
   int chunk = 1024;
   if (waves < 8) chunk = static_cast<int>((nnz + waves * resident - 1) / (waves * resident) + 31) & ~31;
   const int blocks = ceil_div(ceil_div(nnz, chunk), wpb);
-  if (po.n > 0)
-    launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, true>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, nnz, feat,
-                   foff, foff != 0, chunk, last_tile, po);
-  else
-    launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, false>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, nnz, feat,
+  if constexpr (!PART) {
+    if (po.n > 0) {
+      launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, true, false>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m,
+                        nnz, feat, foff, foff != 0, chunk, last_tile, po);
+      SPTIR_LAUNCH_OK("sddmm_lean_kernel");
+      return 0;
+    }
+  }
+  launch_chained_if(nnz < kChainEntries, sddmm_lean_kernel<LPR, false, PART>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, nnz, feat,
                    foff, foff != 0, chunk, last_tile, po);
   SPTIR_LAUNCH_OK("sddmm_lean_kernel");
   return 0;
@@ -345,21 +374,31 @@ int lean_tile(int n, int feat) {
 // whole row of B and of A at every position, so it wants B in L2 as a whole, where the lean kernel needs a slice of it
 // and keeps the row of A.  All figures: us, lean / groups, of 60 matrices of equal and of log-normal rows.
 //  - Rows of less than 10 entries: always (power-law graphs, the header of sddmm_kernel).
-//  - 64 features in one launch of the lean one: 100 k rows of 20 entries 52 / 44, of 100 191 / 181, of 200 358 / 358,
-//    40 k of 500 336 / 348.
-//  - In place of several launches: rows of up to 50 entries (F = 96: 40 k of 30 46 / 38, of 80 86 / 96; F = 64: 233 k of 50
+//  - 64 features in one launch of the lean one: rows of up to 64 entries, 100 for a B of more than 32 MB (20 k of 24 12.7 / 12.4, of 40 17.1 / 17.4, of 80 26.8 /
+//    30.1, 60 k of 40 44.1 / 43.3, of 80 84 / 86, 150 k of 40 128 / 112, 140 k of 70 186 / 177).
+//  - In place of several launches: rows of up to 50 entries (F = 96: 60 k of 24 56 / 49, 20 k of 80 49.4 / 49.5; F = 64: 233 k of 50
 //    248 / 235, of 80 349 / 363, of 500 1734 / 2241), and B up to a share of the L2 budget that grows with the launches
 //    saved: F = 512, two, 20 k of 30 87 / 77, 30 k 136 / 141; F = 256, two, 50 k of 30 109 / 103, 80 k 182 / 225; F = 96,
 //    three narrow ones, 100 k of 30 108 / 99, 150 k 162 / 167, 200 k 219 / 270; F = 64, two, 200 k of 30 147 / 121, 300 k
-//    of 45 at 0.91; F = 128, two, 150 k of 30 226 / 203, 200 k 291 / 318; F = 192, three, 80 k of 30 178 / 137.  At 192
-//    features and a B of 31 MB the groups are the faster ones at any length (40 k rows of 80 185 / 148, of 500 1097 / 895): not taken.
+//    of 45 at 0.91; F = 128, two, 150 k of 24 186 / 171, of 40 267 / 266; F = 192, three, 60 k of 24 108 / 78, 150 k 277 / 308.
+//  - 192 features: rows of any length while B fits (20 k of 80 81 / 73, of 480 465 / 425, 60 k of 80 268 / 226).
 bool in_groups(int m, int n, int feat, int nnz) {
   const int per_row = nnz / m, tile = lean_tile(n, feat);
   if (feat < 64) return false;
   if (per_row < 10) return true;
-  if (feat == tile) return feat == 64 && per_row < 200;
+  const size_t b_bytes = static_cast<size_t>(n) * feat * 4;
+  if (feat == tile) return feat == 64 && per_row < (b_bytes > (size_t{32} << 20) ? 100 : 64);
+  if (feat == 192 && b_bytes <= l2_budget_bytes()) return true;
   const int eighths = tile == 256 || feat == 96 ? 8 : tile == 128 ? 9 : feat == 64 ? 11 : 13;
-  return per_row < (feat == 64 ? 64 : 50) && static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes() / 8 * eighths;
+  return per_row < (feat == 64 ? 64 : 50) && b_bytes <= l2_budget_bytes() / 8 * eighths;
+}
+
+// Feature counts in steps of 8, of rows long enough for the lean kernel, whose B stays in L2 (us, general kernel / lean: 20 k rows of 11
+// F = 24 5.4 / 5.6, F = 72 13.9 / 11.3; 60 k of 30 F = 40 48.7 / 42, F = 104 88 / 69, F = 136 145 / 130; 40 k of 500 F = 24 265 / 166, F = 120
+// 936 / 619, F = 200 1584 / 1179).
+bool lean_part(int m, int n, int feat, int nnz) {
+  return feat % 8 == 0 && feat % 32 != 0 && feat <= 256 && nnz / m >= (feat < 32 ? 16 : 10) &&
+         static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes();
 }
 
 // One launch per tile, in stream order.
@@ -371,14 +410,24 @@ int launch_lean(const float* a, const float* b, float* c, const int32_t* indptr,
     int rc;
     const int last = foff + tile >= feat;
     switch (tile) {
-      case 256: rc = launch_lean_tile<32>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
-      case 128: rc = launch_lean_tile<16>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
-      case 64: rc = launch_lean_tile<8>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
-      default: rc = launch_lean_tile<4>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
+      case 256: rc = launch_lean_tile<32, false>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
+      case 128: rc = launch_lean_tile<16, false>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
+      case 64: rc = launch_lean_tile<8, false>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
+      default: rc = launch_lean_tile<4, false>(a, b, c, indptr, indices, scale, m, feat, nnz, foff, last, po, stream); break;
     }
     if (rc != 0) return rc;
   }
   return 0;
+}
+
+// Other feature counts in steps of 8, in one launch whose last lanes are idle.
+int launch_lean_part(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices, const float* scale,
+                     int m, int feat, int nnz, cudaStream_t stream) {
+  const PeerOut none{};
+  if (feat > 128) return launch_lean_tile<32, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
+  if (feat > 64) return launch_lean_tile<16, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
+  if (feat > 32) return launch_lean_tile<8, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
+  return launch_lean_tile<4, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
 }
 
 }  // namespace
@@ -408,6 +457,7 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
   if (lean && in_groups(m, n, feat, nnz)) return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one.
   if (lean && nnz / m >= 10) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
+  if (lean_part(m, n, feat, nnz) && aligned32(a) && aligned32(b)) return launch_lean_part(a, b, c, indptr, indices, scale, m, feat, nnz, st);
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
   if (feat % 4 == 0 && bits % 16 == 0) {
     if (feat <= 32) return launch<8, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);

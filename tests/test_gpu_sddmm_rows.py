@@ -69,3 +69,31 @@ def test_operands_beyond_l2_are_taken_in_slices(cuda_device, n, feat, per_row):
     out = torch.empty(rows * per_row, device=cuda_device)
     ops.sddmm(a, b.view(-1), out, ptr, cols)
     assert bool((out == 1.0 + 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("feat", [8, 24, 40, 56, 64, 72, 120, 128, 136, 192, 200, 248, 264])
+@pytest.mark.parametrize("per_row", [9, 10, 16, 33, 64, 200])
+def test_tiles_that_rows_do_not_fill(cuda_device, feat, per_row):
+    # around the row lengths at which the kernels change, with a row of infinities in B
+    m, n = 3001, 801
+    g = torch.Generator(device=cuda_device).manual_seed(feat)
+    deg = torch.full((m,), per_row, device=cuda_device)
+    deg[::7] = 0
+    deg[1::7] = 2 * per_row
+    ptr = torch.zeros(m + 1, dtype=torch.int32, device=cuda_device)
+    ptr[1:] = deg.cumsum(0)
+    nnz = int(ptr[-1])
+    cols = torch.randint(0, n, (nnz,), generator=g, device=cuda_device, dtype=torch.int32)
+    a, b = (torch.rand(k, feat, generator=g, device=cuda_device) - 0.5 for k in (m, n))
+    b[5] = float("inf")
+    a[:, 0] = 1.0
+    a[:, 1:4] = 0.25  # sums of infinities of one sign where only the first piece counts
+    a[:, 4:] = a[:, 4:].abs()
+    out = torch.full((nnz,), 7.0, device=cuda_device)
+    ops.sddmm(a.view(-1), b.view(-1), out, ptr, cols)
+    rows = torch.repeat_interleave(torch.arange(m, device=cuda_device), deg)
+    prod = a[rows].double() * b[cols.long()].double()
+    want, mag = prod.sum(1), prod.abs().sum(1)
+    inf = cols == 5
+    assert bool((out[inf] == float("inf")).all())
+    assert bool(((out.double() - want).abs() <= mag * (feat + 8) * 2.0 ** -24)[~inf].all())
