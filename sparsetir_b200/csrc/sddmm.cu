@@ -38,8 +38,15 @@ constexpr int kThreads = 256;
 // the 23 warps per issued instruction wait for memory, L1 data path 35 %, L2 32 %, issue slots 22 %, DRAM 30 %).  Groups of
 // 8 lanes of 32 bytes have as many bytes in flight as 16 lanes of 16 bytes and four positions where those had two: power-law graphs, us, before / with them: 169 k rows, F = 64 43.1 / 31.9, 200 k rows
 // F = 192 131 / 102, F = 128 72 / 67, 20 k rows F = 128 10.1 / 8.6.  Groups of 16 such lanes gain nothing (F = 256 137 / 141).
-template <int LPR, int W, int VPL, bool PEERS>
-__global__ void __launch_bounds__(kThreads, 4)
+//
+// Five blocks per SM with one position in flight per group, where four had two (BLOCKS): B in L2 far from the SMs is waited for longer, and
+// a fifth more warps bring more than the second position (us, two on four blocks / one on five: 169 k power-law rows, F = 64 31 / 28.6,
+// 80 k F = 128 27 / 20.3, F = 64 10.0 / 9.8, 200 k F = 192 101 / 93, 150 k rows of 20 F = 64 61.7 / 56.5; below 24 MB of B 60 k of 20 F = 96
+// 39.2 / 40.2, 20 k of 11 F = 64 6.7 / 7.2).  Four positions on three or two blocks: 42.7, 52.2 on the first of these; two on five and
+// one on six blocks spill (35.9, 31.4).
+constexpr size_t kFarBytes = size_t{24} << 20;
+template <int LPR, int W, int VPL, bool PEERS, int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
 sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
              const int32_t* indptr, const int32_t* indices,
              const float* scale, int m, int feat, int nnz, int chunk, float rows_per_entry,
@@ -47,7 +54,7 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
   using LT = LaneTile<LPR, W, VPL, false>;
   using V = typename LT::Piece;
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int U = W == 8 || VPL == 4 ? 2 : VPL * W >= 4 ? 4 : 8;  // positions in flight; four of four single floats spill
+  constexpr int U = BLOCKS == 5 ? 1 : W == 8 || VPL == 4 ? 2 : VPL * W >= 4 ? 4 : 8;  // positions in flight; four of four single floats spill
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const int sub = wlane / LPR;
@@ -132,7 +139,7 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
 }
 
 // ---------------------------------------------------------------------------------------------
-// Lean variant for feature counts that are multiples of 32, or of 8 and 256 at most (PART), with 32-byte aligned operands.
+// Lean variant for feature counts that are multiples of 32, or of 8 and below 128 (PART), with 32-byte aligned operands.
 //
 // One launch covers a tile of 8*LPR consecutive features [foff, foff + 8*LPR) of every stored
 // position; the host walks the tiles with one launch each, the first storing C and the others
@@ -172,9 +179,9 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
   if (e_begin >= nnz) return;
   const int e_end = static_cast<int>(min(static_cast<long long>(nnz), e_begin + chunk));
   // PART: lanes past the row load its first piece once more.  Groups of 8 and 16 multiply it by zeros, and what that makes a NaN is
-  // formed again; the others, which have no registers for that, mask their products (20 M positions, F = 72, a select that
+  // formed again; those of 4, which have no registers for that, mask their products (20 M positions, F = 72, a select that
   // became a branch around each product 910 us, a mask, which spills, 800, zeros 595; F = 24 a mask 166, zeros 242).
-  constexpr bool kMask = PART && LPR != 8 && LPR != 16, kAgain = PART && !kMask;
+  constexpr bool kMask = PART && LPR == 4, kAgain = PART && !kMask;
   const bool in = !PART || lane * 8 < ld - foff;
   const unsigned keep_bits = in ? 0xffffffffu : 0u;
   const float* a_lane = a + foff + (in ? lane * 8 : 0);
@@ -284,26 +291,26 @@ edge_to_row_kernel(const int32_t* indptr, int32_t* __restrict__ mid, int m, int 
   if (p < nnz) mid[p] = edge_row_search(indptr, 0, m, static_cast<int>(p));
 }
 
-template <int LPR, int W, int VPL>
+template <int LPR, int W, int VPL, int BLOCKS = 4>
 int launch(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
            const float* scale, int m, int feat, int nnz, const PeerOut& po, cudaStream_t stream) {
   // one wave of resident blocks; two for the narrow vectors, whose positions take longer (50 k-node
   // power-law graph, F = 299: 88 against 97 us)
-  const long long warps = static_cast<long long>(kNumSMs) * 4 * (kThreads / 32) * (W < 4 ? 2 : 1);
+  const long long warps = static_cast<long long>(kNumSMs) * BLOCKS * (kThreads / 32) * (W < 4 ? 2 : 1);
   int chunk = static_cast<int>((nnz + warps - 1) / warps);
   chunk = (chunk + 31) & ~31;
   const int blocks = ceil_div(ceil_div(nnz, chunk), kThreads / 32);
   const float rows_per_entry = static_cast<float>(m) / static_cast<float>(nnz);
-  if constexpr (W >= 4) {
+  if constexpr (W >= 4 && BLOCKS == 4) {
     if (po.n > 0) {
-      launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, true>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat,
-                     nnz, chunk, rows_per_entry, po);
+      launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, true, BLOCKS>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m,
+                        feat, nnz, chunk, rows_per_entry, po);
       SPTIR_LAUNCH_OK("sddmm_kernel");
       return 0;
     }
   }
-  launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, false>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat, nnz,
-                 chunk, rows_per_entry, po);
+  launch_chained_if(nnz < kChainEntries, sddmm_kernel<LPR, W, VPL, false, BLOCKS>, blocks, kThreads, 0, stream, a, b, c, indptr, indices, scale, m, feat,
+                    nnz, chunk, rows_per_entry, po);
   SPTIR_LAUNCH_OK("sddmm_kernel");
   return 0;
 }
@@ -393,12 +400,22 @@ bool in_groups(int m, int n, int feat, int nnz) {
   return per_row < (feat == 64 ? 64 : 50) && b_bytes <= l2_budget_bytes() / 8 * eighths;
 }
 
-// Feature counts in steps of 8, of rows long enough for the lean kernel, whose B stays in L2 (us, general kernel / lean: 20 k rows of 11
-// F = 24 5.4 / 5.6, F = 72 13.9 / 11.3; 60 k of 30 F = 40 48.7 / 42, F = 104 88 / 69, F = 136 145 / 130; 40 k of 500 F = 24 265 / 166, F = 120
-// 936 / 619, F = 200 1584 / 1179).
+// Whether groups of 32-byte lanes run on five blocks per SM: far B, or where the positions make fewer rounds of 32 per warp of them (160 k
+// positions, F = 64 6.5 / 5.8, F = 256 17.4 / 14.2).
+bool five_blocks(int n, int feat, int nnz) {
+  if (static_cast<size_t>(n) * feat * 4 >= kFarBytes) return true;
+  const int round = kNumSMs * (kThreads / 32) * 32;
+  const int four = ceil_div(nnz, 4 * round), five = ceil_div(nnz, 5 * round);
+  return five < four && four <= 3;
+}
+
+// Feature counts in steps of 8 below 128 whose lanes the lean kernel fills better than the groups fill their tiles of 64, on rows long
+// enough for it and with a B that stays in L2 (us, groups / lean: 40 k rows of 500 F = 40 461 / 397, F = 104 711 / 611, F = 72 572 / 605,
+// F = 136 815 / 1146; 60 k of 20 F = 40 30.9 / 30.1, F = 104 48.1 / 49.2, 20 k of 40 34.9 / 30.8; F = 24, a group of 8 / lean, 20 k of 11 5.4 /
+// 5.6, 60 k of 30 26.2 / 21.3).
 bool lean_part(int m, int n, int feat, int nnz) {
-  return feat % 8 == 0 && feat % 32 != 0 && feat <= 256 && nnz / m >= (feat < 32 ? 16 : 10) &&
-         static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes();
+  if (feat % 8 != 0 || feat % 32 == 0 || feat >= 128 || (feat > 64 && feat <= 80)) return false;
+  return nnz / m >= (feat < 32 ? 16 : feat < 64 ? 10 : 24) && static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes();
 }
 
 // One launch per tile, in stream order.
@@ -424,7 +441,6 @@ int launch_lean(const float* a, const float* b, float* c, const int32_t* indptr,
 int launch_lean_part(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices, const float* scale,
                      int m, int feat, int nnz, cudaStream_t stream) {
   const PeerOut none{};
-  if (feat > 128) return launch_lean_tile<32, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
   if (feat > 64) return launch_lean_tile<16, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
   if (feat > 32) return launch_lean_tile<8, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
   return launch_lean_tile<4, true>(a, b, c, indptr, indices, scale, m, feat, nnz, 0, 1, none, stream);
@@ -454,27 +470,34 @@ int sddmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
     SPTIR_CUDA_OK(cudaMemsetAsync(c, 0, static_cast<size_t>(nnz) * sizeof(float), st));
     return 0;
   }
-  if (lean && in_groups(m, n, feat, nnz)) return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  if (lean && in_groups(m, n, feat, nnz)) {
+    if (po.n == 0 && five_blocks(n, feat, nnz)) return launch<8, 8, 1, 5>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  }
   // The lean kernel where rows are long enough for it: it asks for a row of A when it meets one.
   if (lean && nnz / m >= 10) return launch_lean(a, b, c, indptr, indices, scale, m, n, feat, nnz, po, st);
   if (lean_part(m, n, feat, nnz) && aligned32(a) && aligned32(b)) return launch_lean_part(a, b, c, indptr, indices, scale, m, feat, nnz, st);
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
+  // Groups of 8 lanes with 64 features between them, of 16 where a lane holds single floats.  With a warp to a row of more than 64
+  // features, and two positions of more than 32 (us, power-law graphs of 80 k rows, that / now: F = 72 21.1 / 15.6, F = 136 44 / 27, F = 100
+  // 29.2 / 18.7, F = 260 75 / 55, F = 46 21.5 / 17.9, F = 190 71 / 47, F = 41 27.7 / 21.4, F = 189 96 / 83).
+  if (feat % 8 == 0 && feat > 32 && bits % 32 == 0) {
+    if (five_blocks(n, feat, nnz)) return launch<8, 8, 1, 5>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<8, 8, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  }
   if (feat % 4 == 0 && bits % 16 == 0) {
     if (feat <= 32) return launch<8, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-    if (feat <= 64) return launch<16, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-    return launch<32, 4, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<8, 4, 2, 5>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   }
   if (feat % 2 == 0 && bits % 8 == 0) {
     if (feat <= 16) return launch<8, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
     if (feat <= 32) return launch<16, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-    if (feat <= 64) return launch<32, 2, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-    return launch<32, 2, 2>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+    return launch<8, 2, 4, 5>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   }
   if (feat <= 8) return launch<8, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   if (feat <= 16) return launch<16, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
   if (feat <= 32) return launch<32, 1, 1>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-  if (feat <= 64) return launch<32, 1, 2>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
-  return launch<32, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
+  return launch<16, 1, 4>(a, b, c, indptr, indices, scale, m, feat, nnz, po, st);
 }
 }  // namespace
 }  // namespace sptir
