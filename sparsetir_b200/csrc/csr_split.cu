@@ -407,8 +407,13 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
   const long long resident = static_cast<long long>(blocks_per_sm(sh.w, sh.vpl)) * kNumSMs, batch = static_cast<long long>(subs) * sh.lanes;
   const long long fewest = (nnz + batch - 1) / batch;
   SplitPlan p;
-  p.gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident / fewest)));
-  const long long want = resident / p.gy * subs;
+  // Up to twice as many blocks as fit at once where that spares them a round of tiles, with no more of them than the rounds need (us, as
+  // many as fit / so: 20 k-node power-law graph F = 256 19.8 / 16.9, F = 384 28.0 / 22.7, 9 k rows of 9 F = 384 24.3 / 17.8, 14 k power-law
+  // F = 130 18.9 / 13.5; with 2.25 times as many 30 k rows of 5, F = 256 20.9 / 21.5).
+  const long long side_by_side = std::min<long long>(tiles, std::max<long long>(1, resident * 15 / 8 / fewest));
+  const long long rounds = (tiles + side_by_side - 1) / side_by_side;
+  p.gy = static_cast<int>((tiles + rounds - 1) / rounds);
+  const long long want = std::max(resident / p.gy, std::min(fewest, resident)) * subs;
   p.span = static_cast<int>((nnz + want - 1) / want + sh.lanes - 1) / sh.lanes * sh.lanes;
   const long long per_block = static_cast<long long>(subs) * p.span;
   const long long with_entries = (nnz + per_block - 1) / per_block;  // the first blocks; the others clear rows
