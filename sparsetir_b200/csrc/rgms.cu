@@ -42,6 +42,8 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
                    const int32_t* indices_j, int num_rels, int feat, int nnz_i,
                    const float* z, cudaStream_t stream);
 int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st);
+int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int feat,
+                     cudaStream_t st);
 int rgms_tma_launch_pairs(const float* a, const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i,
                           const int32_t* indptr_j, const int32_t* indices_j, int num_rels, int nnz_i, const float* z,
                           cudaStream_t stream);
@@ -279,8 +281,10 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
       const int rc = take_scratch(device_id, st, wide_scratch(feat, nnz_i), 0, &cs);
       if (rc == 0) {
         float* z = reinterpret_cast<float*>(cs.scratch);
-        if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, feat, nnz_j, device_id, stream) != 0)
-          return -1;
+        const int sums = aligned32(x) && aligned32(z)
+                             ? rgms_rows_launch(a, x, z, indptr_j, indices_j, nnz_i, feat, st)
+                             : csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, feat, nnz_j, device_id, stream);
+        if (sums != 0) return -1;
         if (rgms_wide_launch(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat, st) != 0) return -1;
         return return_scratch(cs, st);
       }

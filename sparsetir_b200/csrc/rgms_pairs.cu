@@ -20,13 +20,12 @@ namespace sptir {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kF = 64;
-
-template <int LPR, int W>
+// ALL: rows of one entry as well.
+template <int LPR, int W, bool ALL>
 __global__ void __launch_bounds__(kThreads, 4)
 rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
                   const int32_t* indptr, const int32_t* indices, int m, int rpi) {
-  static_assert(LPR * W == kF, "a group covers a row");
+  constexpr int kF = LPR * W;
   using LV = LaneVec<W>;
   constexpr int SUBS = kThreads / LPR;
   constexpr int U = 32 / W;
@@ -38,7 +37,7 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m))), row = r0 + lane;
   const bool there = lane < rpi && row < m;
   const int begin = ld_global(indptr + min(row, m)), len = there ? ld_global(indptr + min(row + 1, m)) - begin : -1;
-  const int own = len >= 2 ? len : 0;
+  const int own = len >= (ALL ? 1 : 2) ? len : 0;
   int upto = own;  // entries of the rows up to this lane's
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) {
@@ -104,13 +103,13 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
   }
 }
 
-template <int LPR, int W>
+template <int LPR, int W, bool ALL>
 int launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st) {
   // fewer rows per group where the groups would not fill the SMs
   constexpr int kGroups = kThreads / LPR;
   int rpi = LPR;
   while (rpi > 1 && ceil_div(m, rpi) < kNumSMs * 4 * kGroups) rpi /= 2;
-  launch_chained(rgms_pairs_kernel<LPR, W>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, indptr, indices, m, rpi);
+  launch_chained(rgms_pairs_kernel<LPR, W, ALL>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, indptr, indices, m, rpi);
   SPTIR_LAUNCH_OK("rgms_pairs_kernel");
   return 0;
 }
@@ -120,8 +119,15 @@ int launch(const float* a, const float* x, float* z, const int32_t* indptr, cons
 int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m,
                       cudaStream_t st) {
   // 32-byte lanes lose where there are too few rows for the groups (3 k nodes, 12 k edges, the call 12.3 us with 16 bytes, 13.9 with 32)
-  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8>(a, x, z, indptr, indices, m, st);
-  return launch<16, 4>(a, x, z, indptr, indices, m, st);
+  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8, false>(a, x, z, indptr, indices, m, st);
+  return launch<16, 4, false>(a, x, z, indptr, indices, m, st);
+}
+
+// All rows, 128 or 256 features, x and z 32-byte aligned.
+int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int feat,
+                     cudaStream_t st) {
+  if (feat == 128) return launch<16, 8, true>(a, x, z, indptr, indices, m, st);
+  return launch<32, 8, true>(a, x, z, indptr, indices, m, st);
 }
 
 }  // namespace sptir

@@ -69,26 +69,31 @@ rgms_wide_kernel(const float* w, float* __restrict__ y, const int32_t* indptr_i,
   for (int k = 0; k < tiles_per_block; ++k) {
     TileWalk ahead = tw;
     const bool more = k + 1 < tiles_per_block && ahead.next(indptr_i, num_rels);
-    float acc[8][8];
+    unsigned long long acc[8][4];  // results (i, 2j) and (i, 2j + 1)
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
     for (int s = 0; s < slices; ++s) {
       const bool last = s + 1 == slices;
       if (!last) fetch(tw, s + 1);
       else if (more) fetch(ahead, 0);
 #pragma unroll
       for (int f = 0; f < kK; ++f) {
-        float zr[8], wr[8];
+        float zr[8];
+        ulonglong2 wr[2];
         *reinterpret_cast<float4*>(zr) = *reinterpret_cast<const float4*>(&s_z[buf][f][ty * 4]);
         *reinterpret_cast<float4*>(zr + 4) = *reinterpret_cast<const float4*>(&s_z[buf][f][64 + ty * 4]);
-        *reinterpret_cast<float4*>(wr) = *reinterpret_cast<const float4*>(&s_w[buf][f][tx * 4]);
-        *reinterpret_cast<float4*>(wr + 4) = *reinterpret_cast<const float4*>(&s_w[buf][f][64 + tx * 4]);
+        wr[0] = *reinterpret_cast<const ulonglong2*>(&s_w[buf][f][tx * 4]);
+        wr[1] = *reinterpret_cast<const ulonglong2*>(&s_w[buf][f][64 + tx * 4]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(zr[i], wr[j], acc[i][j]);
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long zz = pack_pair(zr[i], zr[i]);
+          fma_pair(acc[i][0], zz, wr[0].x);
+          fma_pair(acc[i][1], zz, wr[0].y);
+          fma_pair(acc[i][2], zz, wr[1].x);
+          fma_pair(acc[i][3], zz, wr[1].y);
+        }
       }
       // the other buffer was last read before the previous barrier
       if (!last || more) put(buf ^ 1);
@@ -101,8 +106,13 @@ rgms_wide_kernel(const float* w, float* __restrict__ y, const int32_t* indptr_i,
       const int t = (i >> 2) * 64 + ty * 4 + (i & 3);
       if (t < nrows) {
         float* dst = y + static_cast<size_t>(ld_global(indices_i + tw.row0 + t)) * feat + o0 + tx * 4;
-        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
-        atomicAdd(reinterpret_cast<float4*>(dst + 64), make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float4 v;
+          unpack_pair(acc[i][2 * h], v.x, v.y);
+          unpack_pair(acc[i][2 * h + 1], v.z, v.w);
+          atomicAdd(reinterpret_cast<float4*>(dst + h * 64), v);
+        }
       }
     }
     if (!more) break;

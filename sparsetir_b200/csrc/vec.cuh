@@ -80,6 +80,10 @@ __device__ __forceinline__ unsigned long long pack_pair(float lo, float hi) {
 __device__ __forceinline__ void unpack_pair(unsigned long long v, float& lo, float& hi) {
   asm("mov.b64 {%0,%1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
+// both halves: acc += x * y
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long x, unsigned long long y) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
+}
 // acc[i] += w * x[i] for the 8 floats
 __device__ __forceinline__ void fma8(Pack4& acc, float w, const Pack4& x) {
   const unsigned long long ww = pack_pair(w, w);
