@@ -6,13 +6,15 @@
 //
 // A block walks consecutive tiles of 128 rows of one relation x 128 outputs.  Slices of 16 features of
 // both operands are stored transposed in shared memory (two buffers, the next slice - of the next tile
-// too - in registers meanwhile); a thread owns 8 x 8 results as 2 x 2 pieces of 4 x 4, so that its
-// operands are four 16-byte reads per 64 FMAs.  Sums run over ascending fi.  Two blocks per SM.
+// too - in registers meanwhile), four lanes to the 64 bytes of a row; a thread owns 8 x 8 results as 2 x 2 pieces of 4 x 4, so
+// that its operands are four 16-byte reads per 64 FMAs, and these 32 two-wide instructions.  Sums run over ascending fi.  Two
+// blocks per SM.  100 k nodes, 46 relations, 1 M edges, F = 128 / 256, the call: single FMAs and two lanes to a row 527 / 1830 us, two-wide
+// ones, and the sums of rgms_pairs.cu in front, 490 / 1727, four lanes 471 / 1647 (a lane to a row, without conflicts in
+// the transposed stores, 561 / 2025).
 //
 // It replaces a kernel that gathered, multiplied and scattered tile by tile with one block of 256
 // threads per SM (131 KB of shared memory) at F = 128, and one warp per row at other sizes.  With the
-// aggregation, 100 k nodes, 46 relations, 1 M edges: F = 128 1602 / 531 us, F = 256 125 / 1.8 ms; 3 k
-// nodes, 30 k edges 105 / 45 and 4159 / 123 us.
+// aggregation, 100 k nodes, 46 relations, 1 M edges: F = 128 1602 / 471 us, F = 256 125 / 1.65 ms.
 #include <algorithm>
 
 #include "common.h"
@@ -41,24 +43,24 @@ rgms_wide_kernel(const float* w, float* __restrict__ y, const int32_t* indptr_i,
     return;  // the same in all warps
   tw.rel_end = ld_global(indptr_i + tw.rel + 1);
   const int o0 = static_cast<int>(blockIdx.y) * kTile;
-  const int lr = tid >> 1, lk = (tid & 1) * 8;  // row (and output) of the slice that this thread loads, 8 features
+  const int lr = tid >> 2, lk = (tid & 3) * 4;  // rows (and outputs) lr and lr + 64 of the slice: 4 features of each
   const int ty = tid >> 4, tx = tid & 15;
   const int slices = feat / kK;
 
   float4 nz[2], nw[2];
   auto fetch = [&](const TileWalk& t, int s) {
-    const float4* zp = reinterpret_cast<const float4*>(z + static_cast<size_t>(min(t.row0 + lr, nnz_i - 1)) * feat + s * kK + lk);
-    const float4* wp = reinterpret_cast<const float4*>(w + (static_cast<size_t>(t.rel) * feat + o0 + lr) * feat + s * kK + lk);
-    nz[0] = ld_global(zp); nz[1] = ld_global(zp + 1);
-    nw[0] = ld_global(wp); nw[1] = ld_global(wp + 1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      nz[h] = ld_global(reinterpret_cast<const float4*>(z + static_cast<size_t>(min(t.row0 + lr + h * 64, nnz_i - 1)) * feat + s * kK + lk));
+      nw[h] = ld_global(reinterpret_cast<const float4*>(w + (static_cast<size_t>(t.rel) * feat + o0 + lr + h * 64) * feat + s * kK + lk));
+    }
   };
   auto put = [&](int buf) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      s_z[buf][lk + 4 * h + 0][lr] = nz[h].x; s_z[buf][lk + 4 * h + 1][lr] = nz[h].y;
-      s_z[buf][lk + 4 * h + 2][lr] = nz[h].z; s_z[buf][lk + 4 * h + 3][lr] = nz[h].w;
-      s_w[buf][lk + 4 * h + 0][lr] = nw[h].x; s_w[buf][lk + 4 * h + 1][lr] = nw[h].y;
-      s_w[buf][lk + 4 * h + 2][lr] = nw[h].z; s_w[buf][lk + 4 * h + 3][lr] = nw[h].w;
+      const int r = lr + h * 64;
+      s_z[buf][lk + 0][r] = nz[h].x; s_z[buf][lk + 1][r] = nz[h].y; s_z[buf][lk + 2][r] = nz[h].z; s_z[buf][lk + 3][r] = nz[h].w;
+      s_w[buf][lk + 0][r] = nw[h].x; s_w[buf][lk + 1][r] = nw[h].y; s_w[buf][lk + 2][r] = nw[h].z; s_w[buf][lk + 3][r] = nw[h].w;
     }
   };
 
