@@ -143,15 +143,33 @@ __device__ inline bool locate_tile_warp(const int32_t* indptr_i, int num_rels,
   return false;
 }
 
+// The row ranges of a walk, in shared memory where there are not too many: every role of a kernel steps through them for itself, and
+// over the ranges without rows one by one, a round trip to L2 each otherwise.
+constexpr int kStagedRanges = 1024;
+struct StagedRanges {
+  const int32_t* shared;  // null: too many
+  const int32_t* global;
+};
+__device__ __forceinline__ int32_t range_at(const int32_t* ranges, int i) { return ld_global(ranges + i); }
+__device__ __forceinline__ int32_t range_at(const StagedRanges& r, int i) { return r.shared != nullptr ? r.shared[i] : ld_global(r.global + i); }
+// Called by the whole block, in front of a barrier; the first warp, which goes on to look for the block's tile, leaves it to the others.
+__device__ __forceinline__ StagedRanges stage_ranges(const int32_t* ranges, int num_ranges, int32_t* shared) {
+  if (num_ranges > kStagedRanges) return {nullptr, ranges};
+  if (threadIdx.x >= 32)
+    for (int i = threadIdx.x - 32; i <= num_ranges; i += blockDim.x - 32) shared[i] = ld_global(ranges + i);
+  return {shared, ranges};
+}
+
 struct TileWalk {
   int rel, row0, row1, rel_end;  // rel_end: first row past the relation (cached indptr_i[rel + 1])
   // steps to the tile after this one; false when there is none.  Inside a relation this costs no
   // memory access; the row pointer is read again only when the relation changes.
-  __device__ __forceinline__ bool next(const int32_t* indptr_i, int num_rels) {
+  template <class Ranges>
+  __device__ __forceinline__ bool next(const Ranges& indptr_i, int num_rels) {
     const int nrow0 = row1;
     while (nrow0 >= rel_end) {
       if (++rel >= num_rels) return false;
-      rel_end = ld_global(indptr_i + rel + 1);
+      rel_end = range_at(indptr_i, rel + 1);
     }
     row0 = nrow0;
     row1 = min(rel_end, nrow0 + kTileRows128);

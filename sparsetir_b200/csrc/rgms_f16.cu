@@ -445,6 +445,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
   __shared__ __align__(8) uint64_t bar_acc_empty[2];     // epilogue has read it (128 arrivals)
   __shared__ uint32_t s_tmem;
   __shared__ int s_tile[4];
+  __shared__ int32_t s_ranges[kStagedRanges + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* base = smem_raw + ((1024u - (tc05::smem_u32(smem_raw) & 1023u)) & 1023u);
   const int nkc = (feat_in + kKC - 1) / kKC, nwb = (feat_out + 63) / 64;
@@ -470,6 +471,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
   if (passed != nullptr && blockIdx.x == 0 && tid == 0) st_release(passed, 1);
   __syncthreads();  // the block has its tensor memory, and the flag is set
   chain_trigger();
+  const StagedRanges walk = stage_ranges(ranges, num_ranges, s_ranges);
   if (warp == 0) {
     int rel, row0, row1;
     const bool found = locate_tile_warp(ranges, num_ranges, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
@@ -506,7 +508,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
             tc05::tma_load_2d(st + kZBoxB + j * kWBoxB, &tm_w, j * 64, wrow + c * kKC, &bar_full[s]);
           armed = it + 1;
         }
-        if (k + 1 == tiles_per_cta || !tw.next(ranges, num_ranges)) break;
+        if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
       }
     }
   } else if (warp == 1) {
@@ -538,7 +540,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         }
         if (!ok) break;
         tc05::mma_commit(&bar_acc_full[buf]);
-        if (k + 1 == tiles_per_cta || !tw.next(ranges, num_ranges)) break;
+        if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
       }
     }
   } else if (GATHER && warp >= 12) {
@@ -570,7 +572,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         }
         pending = s;
       }
-      if (k + 1 == tiles_per_cta || !tw.next(ranges, num_ranges)) break;
+      if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");  // also when giving up: nothing may land later
     if (ok && pending >= 0) {
@@ -588,7 +590,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     unsigned char* my_row = gbuf + t * kOutStride;
     const unsigned char* wbase = gbuf + (warp & 3) * 32 * kOutStride;
     bool have = true;
-    if (grp == 1) have = tiles_per_cta > 1 && tw.next(ranges, num_ranges);
+    if (grp == 1) have = tiles_per_cta > 1 && tw.next(walk, num_ranges);
     for (int k = grp; have && k < tiles_per_cta; k += 2) {
       const int buse = k >> 1;
       const int nrows = tw.row1 - tw.row0;
@@ -615,8 +617,8 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         __syncwarp();
         scatter32(y, wbase, kOutStride, dst_row, (warp & 3) * 32, nrows, feat_out, c0, lane);
       }
-      bool has_next = (k + 2 < tiles_per_cta) && tw.next(ranges, num_ranges);
-      has_next = has_next && tw.next(ranges, num_ranges);
+      bool has_next = (k + 2 < tiles_per_cta) && tw.next(walk, num_ranges);
+      has_next = has_next && tw.next(walk, num_ranges);
       if (!has_next) break;
     }
   }

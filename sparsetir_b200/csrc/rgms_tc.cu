@@ -280,7 +280,7 @@ struct PairRows {
 template <class T>
 struct LookAhead {
   TileWalk& tw;
-  const int32_t* indptr_i;
+  const StagedRanges& indptr_i;
   int num_rels, tiles;
   const PairRows& pairs;
   const T* from;
@@ -288,7 +288,7 @@ struct LookAhead {
   T none, value, value_next;
   int row0, nrows, row0_next, nrows_next, begin, len;
   bool more;
-  __device__ __forceinline__ LookAhead(TileWalk& walk, const int32_t* ptr_i, int rels, int num_tiles, const PairRows& p, const T* f,
+  __device__ __forceinline__ LookAhead(TileWalk& walk, const StagedRanges& ptr_i, int rels, int num_tiles, const PairRows& p, const T* f,
                                        int row, int rows, T other)
       : tw(walk), indptr_i(ptr_i), num_rels(rels), tiles(num_tiles), pairs(p), from(f), t(row), nnz_i(rows), none(other), value(other) {
     row0 = tw.row0;
@@ -339,6 +339,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
   __shared__ __align__(8) uint64_t bar_acc_empty[2];     // epilogue has read it (128 arrivals)
   __shared__ uint32_t s_tmem;
   __shared__ int s_tile[4];
+  __shared__ int32_t s_ranges[kStagedRanges + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* base = smem_raw + ((1024u - (tc05::smem_u32(smem_raw) & 1023u)) & 1023u);
 
@@ -361,6 +362,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     tc05::tmem_alloc(&s_tmem, kPTmem);
   }
   chain_wait();
+  const StagedRanges walk = stage_ranges(indptr_i, num_rels, s_ranges);
   if (warp == 0) {
     int rel, row0, row1;
     const bool found = locate_tile_warp(indptr_i, num_rels, blockIdx.x * tiles_per_cta, lane, &rel, &row0, &row1);
@@ -387,7 +389,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     uint32_t put[4];  // of the lane's piece of rows 2i + half, which repeat every eight rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) put[i] = tc05::smem_u32(base + kOffZRaw) + swz_off(t0 + 2 * i + half, piece, kZBox);
-    LookAhead<int> ahead(tw, indptr_i, num_rels, tiles_per_cta, pairs, pairs.indices, t0 + lane, nnz_i, -1);
+    LookAhead<int> ahead(tw, walk, num_rels, tiles_per_cta, pairs, pairs.indices, t0 + lane, nnz_i, -1);
     for (int k = 0; k < tiles_per_cta; ++k) {
       const int s = k % kZStages, use = k / kZStages;
       const int row0 = ahead.row0, nrows = ahead.nrows, src = ahead.value;
@@ -415,7 +417,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
         tc05::tma_load_2d(dst, &tm_z, 0, tw.row0, &bar_full[s]);
         tc05::tma_load_2d(dst + kZBox, &tm_z, 32, tw.row0, &bar_full[s]);
         armed = k + 1;
-        if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
+        if (k + 1 == tiles_per_cta || !tw.next(walk, num_rels)) break;
       }
     }
   } else if (warp == 1) {
@@ -446,7 +448,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
         }
         tc05::mma_commit(&bar_used[buf]);
         tc05::mma_commit(&bar_acc_full[buf]);
-        if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
+        if (k + 1 == tiles_per_cta || !tw.next(walk, num_rels)) break;
       }
     }
   } else if (warp >= 8 && warp < 12) {
@@ -454,7 +456,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     const int ct = tid - 256;
     int staged_rel = -1;
     TileWalk twa = tw;
-    LookAhead<float> ahead(twa, indptr_i, num_rels, GATHER ? tiles_per_cta : 0, pairs, pairs.a, ct, nnz_i, 1.f);
+    LookAhead<float> ahead(twa, walk, num_rels, GATHER ? tiles_per_cta : 0, pairs, pairs.a, ct, nnz_i, 1.f);
     for (int k = 0; k < tiles_per_cta; ++k) {
       const int s = k % kZStages, use = k / kZStages;
       const float scale = ahead.value;  // of a row that came from X
@@ -502,7 +504,7 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
       tc05::fence_before_sync();
       tc05::fence_async_smem();  // W, if it was staged for this tile
       mbar_arrive(&bar_conv[k & 1]);
-      if (k + 1 == tiles_per_cta || !tw.next(indptr_i, num_rels)) break;
+      if (k + 1 == tiles_per_cta || !tw.next(walk, num_rels)) break;
     }
   } else if (warp >= 4 && warp < 16) {
     // ---- epilogue, two groups of four warps: group 0 (warps 4-7) takes the even tiles and
@@ -515,14 +517,14 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
     unsigned char* my_row = gbuf + t * kOutStride;
     const unsigned char* wbase = gbuf + (warp & 3) * 32 * kOutStride;
     bool have = true;
-    if (grp == 1) have = tiles_per_cta > 1 && tw.next(indptr_i, num_rels);
+    if (grp == 1) have = tiles_per_cta > 1 && tw.next(walk, num_rels);
     int nrows = tw.row1 - tw.row0;
     int dst_row = ld_global(indices_i + min(tw.row0 + t, nnz_i - 1));
     for (int k = grp; have && k < tiles_per_cta; k += 2) {
       const int buse = k >> 1;
       // destination rows of this group's next tile (two tiles on): requested now, needed later
-      bool has_next = (k + 2 < tiles_per_cta) && tw.next(indptr_i, num_rels);
-      has_next = has_next && tw.next(indptr_i, num_rels);
+      bool has_next = (k + 2 < tiles_per_cta) && tw.next(walk, num_rels);
+      has_next = has_next && tw.next(walk, num_rels);
       const int dst_next = ld_global(indices_i + min(tw.row0 + t, nnz_i - 1));
       if (!tc05::mbar_wait(&bar_acc_full[grp], buse & 1)) { ok = false; break; }
       tc05::fence_after_sync();

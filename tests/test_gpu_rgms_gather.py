@@ -41,3 +41,28 @@ def test_matches_a_float64_product(cuda_device, widths, feat_in, feat_out, group
     # z is rounded to float16 once (its own magnitude, subnormal steps below 2^-14), the rest is fp32
     bound = mag * (2.0 ** -11 + (feat_in + adds[:, None] + 40) * 2.0 ** -23) + adds[:, None] * feat_in * 2.0 ** -25
     assert bool(((y.view(m, feat_out).double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rels", [511, 512, 513])
+def test_more_ranges_than_a_block_keeps(cuda_device, rels):
+    # (bucket, relation) ranges of two buckets lie in shared memory up to 1,024 of them; most have no rows
+    g = torch.Generator(device=cuda_device).manual_seed(rels)
+    m, n, feat, groups, rows_per_group = 200, 150, 64, 90, 7
+    x = (torch.rand(n, feat, generator=g, device=cuda_device) - 0.5).half()
+    w = (torch.randn(rels, feat, feat, generator=g, device=cuda_device) / 8).half()
+    want = torch.zeros(m, feat, dtype=torch.float64, device=cuda_device)
+    mag, buckets = torch.zeros_like(want), []
+    for width in (2, 4):
+        a = torch.rand(groups, rows_per_group, width, generator=g, device=cuda_device).half()
+        cols = torch.randint(0, n, (groups, rows_per_group, width), generator=g, device=cuda_device)
+        ids = torch.randint(0, m, (groups, rows_per_group), generator=g, device=cuda_device)
+        mid = torch.randint(0, rels, (groups,), generator=g, device=cuda_device).sort()[0]
+        z = (a.double()[..., None] * x.double()[cols]).sum(2)
+        zmag = (a.double()[..., None] * x.double().abs()[cols]).sum(2)
+        want.index_add_(0, ids.view(-1), torch.bmm(z, w.double()[mid]).view(-1, feat))
+        mag.index_add_(0, ids.view(-1), torch.bmm(zmag, w.double().abs()[mid]).view(-1, feat))
+        buckets.append((a, ids.int(), cols.int(), mid.int()))
+    y = torch.zeros(m * feat, device=cuda_device)
+    ops.rgms_ell3d_f16(*ops.rgms_ell3d_f16_args(w.view(-1), x.view(-1), y, buckets, feat, feat))
+    bound = mag * (2.0 ** -11 + 150 * 2.0 ** -23) + feat * 2.0 ** -21  # as above
+    assert bool(((y.view(m, feat).double() - want).abs() <= bound).all())

@@ -61,6 +61,19 @@ def test_rows_of_one_edge(cuda_device, lens, relations, shift):
     assert L.load().sparsetir_tc_timeouts(0, L.ctypes.byref(count)) == 0 and count.value == 0
 
 
+@pytest.mark.parametrize("rels", [1023, 1024, 1025, 3000])
+def test_more_relations_than_a_block_keeps(cuda_device, rels):
+    # the row ranges lie in shared memory up to 1,024 relations; two of three have no row
+    relations = [(r % 3 == 0) * (1 + 130 * (r % 100 == 0)) for r in range(rels)]
+    lens = [1, 2, 0, 5] * (sum(relations) // 4 + 1)
+    n = 500
+    parts = layer(cuda_device, lens[:sum(relations)], relations, n, 0, rels)
+    y = torch.zeros(n * F, device=cuda_device)
+    ops.rgms(parts[0], parts[1], parts[2], y, *parts[3:])
+    want, mag = exact(*parts, n)
+    assert bool(((y.view(n, F).double() - want).abs() <= mag * ((5 + 64 + 2 * rels) * 2.0 ** -24 + 2.0 ** -20)).all())
+
+
 def test_an_infinite_row_reaches_its_destinations_only(cuda_device):
     n, lens = 400, [1, 2, 0, 1] * 75
     a, w, x, ptr_i, rows, ptr_j, cols = layer(cuda_device, lens, [300], n, 0, 3)
