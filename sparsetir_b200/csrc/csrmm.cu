@@ -4,8 +4,8 @@
 // without entries are written as zeros.
 //
 // Two kernels.  Matrices of a few thousand rows, and callers that promise short rows (the
-// aggregation launch of RGMS), take the row-wise kernel below: row pointer -> ids -> rows of B is
-// the shortest chain of memory round trips there is.  All others take the kernel that splits the
+// sums of RGMS in the forms that rgms_pairs.cu does not take), take the row-wise kernel below: row
+// pointer -> ids -> rows of B is the shortest chain of memory round trips there is.  All others take the kernel that splits the
 // matrix by stored entries (csr_split.cu).
 #include <algorithm>
 #include <cstdlib>
