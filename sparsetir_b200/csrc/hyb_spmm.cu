@@ -23,6 +23,7 @@
 //    kernels cannot see; the caller says so with SPARSETIR_HYB_ALL_ATOMIC.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "common.h"
@@ -66,6 +67,7 @@ struct HybTable {
   int32_t block_start[kMaxB + 1];
   int32_t row_base[kMaxB];         // buckets without a row-id array: ELL row r -> output row base + r
   int32_t part_base[kMaxB];        // lean kernel: scratch row of ELL row 0, or -1 (bucket has no split rows)
+  int32_t long_rows;               // lean kernel: at least 8 slots per ELL row on average
   int32_t nb;
 };
 
@@ -179,8 +181,8 @@ hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* b,
 // on a 100 k-node power-law graph 58 -> 35 us, F = 41 on 60 k nodes 50 -> 16 us, F = 184 on 194 k
 // nodes with 36 entries per row in two column partitions 1065 -> 566 us).  Written for instruction
 // economy — the gathers come from L2 at well over 10 TB/s if, and only if, the warp spends its
-// issue slots on loads: per stored slot the loop executes one shuffle + one address + one
-// 16-byte load, then one shuffle + four FMAs; row ends sit at compile-time positions of the
+// issue slots on loads: per stored slot the loop executes one address + one 16-byte load and four
+// FMAs, and between them two shuffles or half a read of shared memory (enum Hand below); row ends sit at compile-time positions of the
 // unrolled batch (narrow rows) or are tested once per 8 slots (wide rows); row ids travel in
 // registers with two flag bits, so a row end costs one shuffle and a store.
 //
@@ -198,14 +200,41 @@ hyb_spmm_kernel(const __grid_constant__ HybTable tb, const float* b,
 // W = floats per lane: 4 (16-byte vectors) or 8 (32-byte vectors, two-wide FMAs)
 constexpr int kFlagAtomic = static_cast<int>(0x80000000u);  // add atomically instead of storing
 
+// Ids and weights of two batches of a sub-warp, written by its lanes and read by all of them four at a time.
+template <int LPR>
+struct __align__(16) SlotBuffer {
+  static constexpr int kWords = 2 * LPR + 4;  // the sub-warps of a warp read from different banks
+  int32_t cols[kWords];
+  float wts[kWords];
+};
+// Volatile, so that the weights are not read, and held in registers, long before they are used.
+__device__ __forceinline__ int4 lds4(const int32_t* from) {
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(from))) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 lds4(const float* from) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(from))) : "memory");
+  return v;
+}
+
 // row_flag(g): flag word of ELL row g (called by the lane that will hold it)
 // row_end(acc, flag word): all lanes of the sub-warp, after the last slot of an ELL row
-template <int LPR, int WM, int W, int VPL, bool WHOLE, class RowFlag, class RowEnd>  // WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
+// How ids and weights come to all lanes of a sub-warp: by shuffles, or four at a time by way of shared memory, which spares the data
+// path of L1, the busiest unit, three of four of these steps.  us, shuffles / shared: 20 k rows of 30 F = 128 28.7 / 27.3, F = 256 46.1 /
+// 40.5, F = 512 89.7 / 77.3; rows of 500 F = 300 420 / 387, F = 512 558 / 528; the 169 k-node power-law graph F = 256 100.6 / 98.4, F = 512
+// 187 / 182.  kChunks: shuffles in the loop that kShared has.
+enum Hand : int { kShuffles, kChunks, kShared };
+// WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
+template <int LPR, int WM, int W, int VPL, bool WHOLE, Hand HAND, class RowFlag, class RowEnd>
 __device__ __forceinline__ void lean_item(const int32_t* cols,
                                           const float* wts, int r0, int nr, int nslots,
                                           int per_row, const char* bl,
                                           unsigned row_bytes, const LaneTile<LPR, W, VPL, WHOLE>& lt, int lane,
-                                          unsigned mask, RowFlag&& row_flag, RowEnd&& row_end) {
+                                          unsigned mask, SlotBuffer<LPR>& sb, RowFlag&& row_flag, RowEnd&& row_end) {
   using LT = LaneTile<LPR, W, VPL, WHOLE>;
   using V = typename LT::Piece;
   constexpr int kU = W == 8 ? 4 : W == 4 ? 8 : VPL == 1 ? 16 : VPL == 2 ? 8 : 4;  // gathered rows in flight
@@ -215,6 +244,7 @@ __device__ __forceinline__ void lean_item(const int32_t* cols,
     return base + static_cast<unsigned long long>(static_cast<unsigned>(col)) * row_bytes;
   };
   static_assert(LPR % U == 0, "a batch is a whole number of chunks");
+  static_assert(HAND == kShuffles || (WM == 8 && U % 4 == 0), "read four at a time");
   constexpr int RPB = WM < 8 ? LPR / WM : 0;  // ELL rows that end inside one batch (narrow rows)
 
   V acc = LT::zero();
@@ -240,7 +270,57 @@ __device__ __forceinline__ void lean_item(const int32_t* cols,
     }
     if (WM < 8 && lane < RPB && (s0 + LPR) / WM + lane < nr) rfn = row_flag(r0 + (s0 + LPR) / WM + lane);
     const int cnt = nslots - s0;  // live slots of this batch if < LPR
-    if (cnt >= LPR) {
+    if constexpr (HAND != kShuffles) {
+      const int at = s0 / LPR % 2 * LPR;
+      if constexpr (HAND == kShared) {
+        sb.cols[at + lane] = c;
+        sb.wts[at + lane] = a;
+        __syncwarp(mask);  // and every lane is done with the batch before, which lies where the next one will
+      }
+      auto chunk = [&](int k0) {  // U live slots: nslots and per_row are multiples of 8
+        V x[U];
+#pragma unroll
+        for (int u = 0; u < U; u += 4) {
+          if constexpr (HAND == kShared) {
+            const int4 id = lds4(sb.cols + at + k0 + u);
+            x[u] = lt.ldg(vec_of(bl, id.x));
+            x[u + 1] = lt.ldg(vec_of(bl, id.y));
+            x[u + 2] = lt.ldg(vec_of(bl, id.z));
+            x[u + 3] = lt.ldg(vec_of(bl, id.w));
+          } else {
+#pragma unroll
+            for (int k = u; k < u + 4; ++k) x[k] = lt.ldg(vec_of(bl, __shfl_sync(mask, c, k0 + k, LPR)));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u += 4) {
+          if constexpr (HAND == kShared) {
+            const float4 ak = lds4(sb.wts + at + k0 + u);
+            LT::fma(acc, ak.x, x[u]);
+            LT::fma(acc, ak.y, x[u + 1]);
+            LT::fma(acc, ak.z, x[u + 2]);
+            LT::fma(acc, ak.w, x[u + 3]);
+          } else {
+#pragma unroll
+            for (int k = u; k < u + 4; ++k) LT::fma(acc, __shfl_sync(mask, a, k0 + k, LPR), x[k]);
+          }
+        }
+        left -= U;
+        if (left == 0) {
+          row_end(acc, __shfl_sync(mask, rf, jrow, LPR));
+          ++jrow;
+          left = per_row;
+        }
+      };
+      if (cnt >= LPR) {
+#pragma unroll
+        for (int k0 = 0; k0 < LPR; k0 += U) chunk(k0);
+      } else {
+#pragma unroll
+        for (int k0 = 0; k0 < LPR; k0 += U)
+          if (k0 < cnt) chunk(k0);
+      }
+    } else if (cnt >= LPR) {
 #pragma unroll
       for (int k0 = 0; k0 < LPR; k0 += U) {
         V x[U];
@@ -480,7 +560,7 @@ __device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, c
 }
 
 // blockIdx.y = feature tile of LPR * W * VPL floats; the last one may be partly filled
-template <int LPR, int W, int VPL, bool WHOLE, bool PEERS>
+template <int LPR, int W, int VPL, bool WHOLE, bool PEERS, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 8)
 hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant__ LeanArgs la) {
   using LT = LaneTile<LPR, W, VPL, WHOLE>;
@@ -488,7 +568,10 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
   const PeerOut* po = PEERS ? &la.peers : nullptr;
   constexpr int SUBS = kThreads / LPR;
   constexpr int NW = 32 / LPR;
-  __shared__ __align__(32) float s_part[SUBS][LT::kFloats];  // wide rows: partial sums of the spans
+  __shared__ union __align__(32) {  // of a sub-warp: its batches, then, in wide rows, the partial sum of its span
+    SlotBuffer<LPR> slots;
+    float part[LT::kFloats];
+  } s_sub[SUBS];
   const int lane = threadIdx.x % LPR;
   const int sub = threadIdx.x / LPR;
   const unsigned mask = group_mask<LPR>();
@@ -539,10 +622,14 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
     const int32_t* cols = tb.cols[q] + first;
     const float* wts = tb.w[q] + first;
     const int nslots = nr * width;
-    if (width == 1) lean_item<LPR, 1, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
-    else if (width == 2) lean_item<LPR, 2, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
-    else if (width == 4) lean_item<LPR, 4, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
-    else lean_item<LPR, 8, W, VPL, WHOLE>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, row_flag, row_end);
+    if (width == 1) lean_item<LPR, 1, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    else if (width == 2) lean_item<LPR, 2, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    else if (width == 4) lean_item<LPR, 4, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    else if (!SHARED) lean_item<LPR, 8, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    // Not in one tile of 8 lanes (20 k rows of 30, F = 32, by shuffles / shared 10.1 / 10.6), nor on short rows in tiles that rows do not fill
+    // (169 k-node power-law graph, F = 300, 160.3 / 161.5).
+    else if (LPR == 8 ? gridDim.y > 1 : LPR > 16 || WHOLE || tb.long_rows != 0) lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kShared : kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    else lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kChunks : kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
     return;
   }
 
@@ -570,14 +657,15 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
     const size_t first = static_cast<size_t>(r) * width + s0;
     auto no_flag = [](int) -> int { return 0; };
     auto keep = [&](V& acc, int) { total = acc; };
-    lean_item<LPR, 8, W, VPL, WHOLE>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lt, lane, mask,
-                              no_flag, keep);
+    lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kShared : kShuffles>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lt, lane, mask,
+                                              s_sub[sub].slots, no_flag, keep);
   }
-  if (part != 0) LT::sts(s_part[sub], lane, total);
+  __syncwarp(mask);  // every lane is done with the batches
+  if (part != 0) LT::sts(s_sub[sub].part, lane, total);
   __syncthreads();
   if (!live || part >= NW || (part != 0 && !by_warp)) return;
   if (part == 0)
-    for (int k = 1; k < spr; ++k) LT::add(total, LT::lds(s_part[sub + k], lane));
+    for (int k = 1; k < spr; ++k) LT::add(total, LT::lds(s_sub[sub + k].part, lane));
   if (by_warp) {
     finish_split_row_warp(lt, total, rows, nrows, r, rid, before, behind, part_base, pl, cl, la.counters, stride, po);
   } else if (all_atomic) {
@@ -815,19 +903,37 @@ long long plan_blocks(HybTable& tb, int subs) {
 template <int LPR, int W, int VPL, bool WHOLE>
 int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
   const int tiles = ceil_div(la.feat, W * LPR * VPL);
-  long long slots = 0;
-  for (int q = 0; q < tb.nb; ++q) slots += static_cast<long long>(tb.nrows[q]) * tb.width[q];
+  long long slots = 0, rows = 0;
+  for (int q = 0; q < tb.nb; ++q) {
+    rows += tb.nrows[q];
+    slots += static_cast<long long>(tb.nrows[q]) * tb.width[q];
+  }
+  tb.long_rows = slots >= 8 * rows ? 1 : 0;
   plan_items_lean(tb, lean_item_slots(LPR, W, tiles, slots), kThreads / LPR);
   const long long blocks = plan_blocks_lean(tb, kThreads / LPR);
   if (blocks < 0) return fail("sparsetir_hyb_spmm: too many thread blocks");
   dim3 grid(static_cast<unsigned>(blocks), tiles);
-  if (la.peers.n > 0) {
-    if constexpr (W == 4 && WHOLE)
-      launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true>, grid, kThreads, 0, stream, tb, la);
-    else
-      return fail("sparsetir_hyb_spmm_peers: whole tiles of 16-byte lanes only");  // the dispatcher picks them
+  // 32-byte lanes and rows of 34, 38, 42... features, one pair to a lane, lose by it (20 k-node power-law graph, F = 34 8.9 / 10.7 us).
+  constexpr bool kMay = W <= 4 && !(W == 2 && VPL == 1);
+  // Tiles of 8 lanes: not on short rows, where they wait for chains of loads and not for L1 (169 k-node power-law graph, F = 100 59.8 / 61.1,
+  // F = 128 53.9 / 54.5; F = 32 among other work 19.3 / 19.6), nor where one tile adds all results atomically (F = 32, two partitions 24.6 / 25.3).
+  const bool shared = kMay && (LPR > 8 || (tb.long_rows != 0 && (tiles > 1 || la.all_atomic == 0)));
+  auto go = [&](auto in_shared) -> int {
+    constexpr bool S = decltype(in_shared)::value;
+    if (la.peers.n > 0) {
+      if constexpr (W == 4 && WHOLE)
+        launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true, S>, grid, kThreads, 0, stream, tb, la);
+      else
+        return fail("sparsetir_hyb_spmm_peers: whole tiles of 16-byte lanes only");  // the dispatcher picks them
+    } else {
+      launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, false, S>, grid, kThreads, 0, stream, tb, la);
+    }
+    return 0;
+  };
+  if constexpr (LPR > 8 || !kMay) {
+    if (go(std::bool_constant<kMay>{}) != 0) return -1;
   } else {
-    launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, false>, grid, kThreads, 0, stream, tb, la);
+    if ((shared ? go(std::true_type{}) : go(std::false_type{})) != 0) return -1;
   }
   SPTIR_LAUNCH_OK("hyb_spmm_lean_kernel");
   return 0;

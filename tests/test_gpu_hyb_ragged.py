@@ -47,6 +47,34 @@ def test_ragged_features_and_alignments(cuda_device, buckets, parts, feat, offse
     assert bool(((y.view(m, feat).double() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("low,high", [(0, 9), (9, 80)])
+@pytest.mark.parametrize("parts", [1, 2])
+@pytest.mark.parametrize("n,feat", [(3000, 32), (3000, 64), (3000, 100), (3000, 128), (3000, 256), (3000, 260), (110000, 300), (110000, 320)])
+def test_ids_by_shuffles_and_through_shared_memory(cuda_device, n, feat, parts, low, high):
+    """Short and long rows, on tiles of 8, 16 and 32 lanes (16 where a slice of b is more than L2 keeps), one tile and several, whole and
+    partly filled, with rows of 8 slots to rows that a block shares, and partly filled batches in all of them."""
+    rng = np.random.default_rng(feat + high)
+    deg = np.concatenate([[2900, 1300, 520, 257, 8, 9, 0], rng.integers(low, high, 800)]).astype(np.int64)
+    m, nnz, buckets = len(deg), int(deg.sum()), [8, 24, 64, 512]
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(n, d, replace=False)) for d in deg]).astype(np.int32)
+    vals = rng.uniform(-1, 1, nnz).astype(np.float32)
+    if low == 0:
+        buckets = [1, 2, 4] + buckets
+    r, c, _, v, _ = fmt.column_part_hyb(m, n, indptr, cols, parts, buckets, data=vals)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)  # noqa: E731
+    bk = [(dev(v[p][b]), dev(r[p][b]), dev(c[p][b])) for p in range(parts) for b in range(len(buckets)) if len(r[p][b])]
+    x = torch.rand(n, feat, generator=torch.Generator(cuda_device).manual_seed(feat), device=cuda_device) * 2 - 1
+    y = torch.zeros(m, feat, device=cuda_device)
+    for _ in range(2):
+        ops.hyb_spmm(*ops.hyb_args(x.view(-1), y.view(-1), bk, feat, L.HYB_ALL_ATOMIC | L.HYB_ZERO_C if parts > 1 else 0))
+    a = torch.sparse_csr_tensor(dev(indptr).long(), dev(cols).long(), dev(vals).double(), (m, n))
+    want = a @ x.double()
+    mag = torch.sparse_csr_tensor(dev(indptr).long(), dev(cols).long(), dev(vals).double().abs(), (m, n)) @ x.double().abs()
+    # an fp32 sum of d products in any order: at most d half-ulps of the sum of magnitudes
+    assert bool(((y.double() - want).abs() <= mag * (dev(deg)[:, None].double() + 1) * 2.0 ** -24).all())
+
+
 BEYOND_THE_LIMIT = """
 import numpy as np, torch
 from sparsetir_b200 import format as fmt, ops
