@@ -138,6 +138,13 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
   }
 }
 
+// A product that came out as a NaN, feature by feature.
+__device__ __noinline__ float plain_dot(const float* a, const float* b, int feat) {
+  float s = 0.f;
+  for (int f = 0; f < feat; ++f) s = fmaf(ld_global(a + f), ld_global(b + f), s);
+  return s;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Lean variant for feature counts that are multiples of 32, or of 8 and below 128 (PART), with 32-byte aligned operands.
 //
@@ -148,17 +155,18 @@ sddmm_kernel(const float* a, const float* b, float* __restrict__ c,
 // packed two-wide fp32 FMAs.  A warp owns `chunk` consecutive positions, finds the row of its
 // first position together (row(p) = upper bound - 1, the search of
 // sparse_tir_lowered_buffer_scripts.py:530-549), and loads the column ids of the next batch before it
-// gathers for this one.  It asks for a row of A when it meets one: for matrices of 10 entries per row and
-// more (sddmm_run).
+// gathers for this one.  It keeps the row of A that it is in: for matrices of 10 entries per row and more (sddmm_run).
+//
+// Batches in which rows end.  Rows that are short beside the average make most batches such ones, and a matrix whose rows vary has
+// many of them whatever its average is.  Tiles of 64 features, and PART, find the rows of a batch in a register window of row ends
+// (kWindow; up to four ends are counted, more are searched), and tiles of 64 ask for up to four rows of A together with those of B
+// (kTogether).  A walk along the row pointers, lane by lane, and a row of A when it is met took, us, log-normal rows of sigma 2 and their mean,
+// walk / so (groups of sddmm_kernel): 100 k rows of 30, F = 256 409 / 280, 20 k of 80, F = 64 29.1 / 25.8, 20 k of 30, F = 24 12.1 / 9.0
+// (10.5), F = 40 21.5 / 18.3; rows of one length within 2 %.  Tiles of 32, 128 and 256 keep the walk (the window on 60 k rows of 15 to 70
+// entries: F = 96 102 to 105 %, F = 128 97 to 101 %, F = 256 from 40 k rows 102 to 105 %, 60 k rows of log-normal lengths F = 32 and rows of A
+// together 250 / 239), PART and tiles of 32 ask for rows of A one by one (together: 20 k of 30, F = 40 16.2 / 21.9, F = 24 9.1 / 10.3).
 // With PEERS the finished value of every position (the last feature tile's pass) is also stored
 // into the peers' copies of c: 128 contiguous bytes per warp and peer, over NVLink.
-// A product that came out as a NaN, feature by feature.
-__device__ __noinline__ float plain_dot(const float* a, const float* b, int feat) {
-  float s = 0.f;
-  for (int f = 0; f < feat; ++f) s = fmaf(ld_global(a + f), ld_global(b + f), s);
-  return s;
-}
-
 template <int LPR, bool PEERS, bool PART>
 __global__ void __launch_bounds__(kThreads, LPR == 4 ? 4 : 2)
 sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
@@ -170,6 +178,7 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
   // two tiles, 413 / 353, F = 256 827 / 704); tiles of 32 with two batches at once lose (117 M, F = 128 3720 / 4150), and so do wider
   // ones with eight (F = 128 558 / 721).
   constexpr int U = LPR == 8 ? 8 : 4;
+  constexpr bool kWindow = LPR == 8 || PART, kTogether = LPR == 8 && !PART;
   const int wlane = threadIdx.x & 31;
   const int lane = wlane % LPR;
   const unsigned mask = group_mask<LPR>();
@@ -193,7 +202,8 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
   auto row_of_a = [&](int r) { return in || kMask ? ldg256(a_lane + static_cast<size_t>(r) * ld) : pack4_zero(); };
 
   int warp_row = max(0, min(m - 1, warp_upper_bound(indptr, 0, m + 1, static_cast<int>(e_begin), wlane) - 1));
-  int warp_end = ld_global(indptr + warp_row + 1);  // first position past the warp's current row
+  // end of the warp's current row; kWindow: in lane j that of the row j behind it
+  int wend = kWindow ? row_window<32>(indptr, m, warp_row, wlane) : ld_global(indptr + warp_row + 1);
   int cur_row = -1;
   Pack4 arow = pack4_zero();
 
@@ -210,7 +220,7 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
     }
     float part[LPR];
     int row = warp_row;
-    if (base + 32 <= min(warp_end, e_end)) {
+    if (base + 32 <= min(kWindow ? __shfl_sync(0xffffffffu, wend, 0) : wend, e_end)) {
       // every position of the batch lies in the warp's current row
       if (cur_row != warp_row) {
         cur_row = warp_row;
@@ -226,36 +236,73 @@ sddmm_lean_kernel(const float* a, const float* b, float* __restrict__ c,
         for (int u = 0; u < U; ++u) part[k0 + u] = product(arow, x[u]);
       }
     } else {
-      if (live) {
-        int steps = 0;
-        // row < m - 1 keeps every read inside indptr even if nnz disagrees with indptr[m]
-        while (row < m - 1 && ld_global(indptr + row + 1) <= e) {
-          ++row;
-          if (++steps == 8) {  // long run of empty rows: finish with a search
-            row = min(m - 1, edge_row_search(indptr, row, m, e));
-            break;
+      if constexpr (kWindow) {
+        const int last = min(e, e_end - 1);  // dead positions: the last live one's row
+        const int over = __popc(__ballot_sync(0xffffffffu, wend <= min(base + 31, e_end - 1)));  // rows that end before the batch does
+        if (over <= 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) row += __shfl_sync(0xffffffffu, wend, k) <= last ? 1 : 0;
+          row = min(row, m - 1);
+        } else {
+          int row_end;
+          row = row_in_window<32>(indptr, m, warp_row, wend, last, row_end);
+        }
+        warp_row = __shfl_sync(0xffffffffu, row, 31);
+        wend = row_window<32>(indptr, m, warp_row, wlane);
+      } else {
+        if (live) {
+          int steps = 0;
+          // row < m - 1 keeps every read inside indptr even if nnz disagrees with indptr[m]
+          while (row < m - 1 && ld_global(indptr + row + 1) <= e) {
+            ++row;
+            if (++steps == 8) {  // long run of empty rows: finish with a search
+              row = min(m - 1, edge_row_search(indptr, row, m, e));
+              break;
+            }
           }
         }
+        // the next batch starts from the row of this batch's last live position
+        warp_row = __shfl_sync(0xffffffffu, row, min(31, e_end - 1 - base));
+        wend = ld_global(indptr + warp_row + 1);
       }
-      // the next batch starts from the row of this batch's last live position
-      warp_row = __shfl_sync(0xffffffffu, row, min(31, e_end - 1 - base));
-      warp_end = ld_global(indptr + warp_row + 1);
+      if constexpr (kTogether) {
+        constexpr int UM = 4;  // rows of B in flight beside as many of A
 #pragma unroll
-      for (int k0 = 0; k0 < LPR; k0 += U) {
-        Pack4 x[U];
-        int rk[U];
+        for (int k0 = 0; k0 < LPR; k0 += UM) {
+          Pack4 x[UM], ar[UM];
+          bool other[UM];  // uniform inside the sub-warp
 #pragma unroll
-        for (int u = 0; u < U; ++u) {  // dead positions carry column 0 and the warp's row
-          rk[u] = __shfl_sync(mask, row, k0 + u, LPR);
-          x[u] = ldg256(b_lane + static_cast<size_t>(__shfl_sync(mask, col, k0 + u, LPR)) * ld);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (rk[u] != cur_row) {  // uniform inside the sub-warp
-            cur_row = rk[u];
-            arow = row_of_a(cur_row);
+          for (int u = 0; u < UM; ++u) {  // dead positions carry column 0
+            const int rk = __shfl_sync(mask, row, k0 + u, LPR);
+            x[u] = ldg256(b_lane + static_cast<size_t>(__shfl_sync(mask, col, k0 + u, LPR)) * ld);
+            other[u] = rk != cur_row;
+            if (other[u]) ar[u] = ldg256(a_lane + static_cast<size_t>(rk) * ld);
+            cur_row = rk;
           }
-          part[k0 + u] = product(arow, x[u]);
+#pragma unroll
+          for (int u = 0; u < UM; ++u) {
+            if (other[u]) arow = ar[u];
+            part[k0 + u] = product(arow, x[u]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int k0 = 0; k0 < LPR; k0 += U) {
+          Pack4 x[U];
+          int rk[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {  // dead positions carry column 0 and the warp's row
+            rk[u] = __shfl_sync(mask, row, k0 + u, LPR);
+            x[u] = ldg256(b_lane + static_cast<size_t>(__shfl_sync(mask, col, k0 + u, LPR)) * ld);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (rk[u] != cur_row) {  // uniform inside the sub-warp
+              cur_row = rk[u];
+              arow = row_of_a(cur_row);
+            }
+            part[k0 + u] = product(arow, x[u]);
+          }
         }
       }
     }

@@ -97,3 +97,25 @@ def test_tiles_that_rows_do_not_fill(cuda_device, feat, per_row):
     inf = cols == 5
     assert bool((out[inf] == float("inf")).all())
     assert bool(((out.double() - want).abs() <= mag * (feat + 8) * 2.0 ** -24)[~inf].all())
+
+
+@pytest.mark.parametrize("feat", [24, 40, 64, 104])
+@pytest.mark.parametrize("tail", [0, 40])
+def test_rows_that_end_inside_a_batch(cuda_device, feat, tail):
+    """Batches of 32 positions in which no row, one to six rows and more than 32 rows end, rows without positions among and
+    behind them, and a last batch of every length; rows are long enough on average for the kernel that keeps the row of A."""
+    rng = np.random.default_rng(feat)
+    ends = [[32], [31, 1], [5, 27], [8] * 4, [7, 6, 6, 6, 7], [6, 5, 5, 5, 5, 6], [1] * 32, [0, 0, 32], [16] + [0] * 40 + [16], [3] * 10 + [2]]
+    deg = np.array(sum((ends[i] for i in rng.integers(0, len(ends), 900)), []) + [500] * (1800 if feat == 64 else 450) + [13] + [0] * tail)
+    deg = np.concatenate([deg[rng.permutation(len(deg) - tail)], deg[len(deg) - tail:]])
+    m, nnz, n = len(deg), int(deg.sum()), 4001
+    assert nnz >= 120_000 and nnz // m >= (64 if feat == 64 else 24)
+    ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(feat)
+    cols = torch.randint(0, n, (nnz,), generator=g, device=cuda_device, dtype=torch.int32)
+    a, b = (torch.rand(k, feat, generator=g, device=cuda_device) - 0.5 for k in (m, n))
+    out = torch.full((nnz,), 7.0, device=cuda_device)
+    ops.sddmm(a.view(-1), b.view(-1), out, ptr, cols)
+    rows = torch.repeat_interleave(torch.arange(m, device=cuda_device), torch.from_numpy(deg).to(cuda_device))
+    prod = a[rows].double() * b[cols.long()].double()
+    assert bool(((out.double() - prod.sum(1)).abs() <= prod.abs().sum(1) * (feat + 2) * 2.0 ** -24).all())

@@ -1,0 +1,68 @@
+"""Calls whose time must follow the work in them: rows of very different lengths beside rows of one length, fewer features beside
+more.  A ratio of two times, taken in turn on the same GPU; every limit lies well above what is measured."""
+import numpy as np
+import pytest
+import torch
+
+from sparsetir_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def times(calls, rounds=7):
+    """us of each call among others like it: the median of rounds that take the calls in turn."""
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    reps = []
+    for call in calls:
+        for _ in range(3):
+            call()
+        begin.record()
+        call()
+        end.record()
+        end.synchronize()
+        reps.append(int(min(200, max(5, 2.0 / max(begin.elapsed_time(end), 1e-3)))))
+    out = [[] for _ in calls]
+    for _ in range(rounds):
+        for i, call in enumerate(calls):
+            call()
+            begin.record()
+            for _ in range(reps[i]):
+                call()
+            end.record()
+            end.synchronize()
+            out[i].append(begin.elapsed_time(end) / reps[i] * 1e3)
+    return [sorted(t)[rounds // 2] for t in out]
+
+
+def check_ratio(call, other, limit):
+    """call takes at most `limit` times as long as other; a GPU that was busy gets two more chances."""
+    seen = []
+    for _ in range(3):
+        t, u = times([call, other])
+        seen.append(t / u)
+        if seen[-1] <= limit:
+            return
+    pytest.fail(f"{seen} against {limit}")
+
+
+def lengths(kind, n, mean):
+    if kind == "equal":
+        return np.full(n, mean, np.int64)
+    rng = np.random.default_rng(n)  # log-normal of sigma 2: half of the rows have less than a seventh of the mean
+    return np.clip(np.rint(rng.lognormal(np.log(mean) - 2.0, 2.0, n)), 1, n // 4).astype(np.int64)
+
+
+def sddmm_call(device, deg, feat):
+    n, nnz = len(deg), int(deg.sum())
+    g = torch.Generator(device=device).manual_seed(feat)
+    ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(device)
+    cols = torch.randint(0, n, (nnz,), generator=g, device=device, dtype=torch.int32)
+    a, b = (torch.rand(n * feat, generator=g, device=device) for _ in range(2))
+    return ops.sddmm.prepare(a, b, torch.empty(nnz, device=device), ptr, cols)
+
+
+@pytest.mark.parametrize("n,mean,feat,limit", [(100_000, 30, 256, 1.2), (20_000, 30, 24, 1.18)])
+def test_sddmm_on_uneven_rows(cuda_device, n, mean, feat, limit):
+    uneven = lengths("uneven", n, mean)
+    even = lengths("equal", n, int(round(uneven.sum() / n)))
+    check_ratio(sddmm_call(cuda_device, uneven, feat), sddmm_call(cuda_device, even, feat), limit)
