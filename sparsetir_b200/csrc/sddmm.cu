@@ -430,21 +430,23 @@ int lean_tile(int n, int feat) {
 // whole row of B and of A at every position, so it wants B in L2 as a whole, where the lean kernel needs a slice of it
 // and keeps the row of A.  All figures: us, lean / groups, of 60 matrices of equal and of log-normal rows.
 //  - Rows of less than 10 entries: always (power-law graphs, the header of sddmm_kernel).
-//  - 64 features in one launch of the lean one: rows of up to 64 entries, 100 for a B of more than 32 MB (20 k of 24 12.7 / 12.4, of 40 17.1 / 17.4, of 80 26.8 /
-//    30.1, 60 k of 40 44.1 / 43.3, of 80 84 / 86, 150 k of 40 128 / 112, 140 k of 70 186 / 177).
+//  - 64 features in one launch of the lean one: rows of up to 64 entries, 100 where B is far (20 k of 24 12.7 / 12.4, of 40 17.1 / 17.4, of 80 26.8 /
+//    30.1, 60 k of 40 44.1 / 43.3, of 80 84 / 86, 150 k of 40 128 / 112, 100 k of 80, log-normal of sigma 1 149 / 138, 140 k of 70 186 / 177).
 //  - In place of several launches: rows of up to 50 entries (F = 96: 60 k of 24 56 / 49, 20 k of 80 49.4 / 49.5; F = 64: 233 k of 50
 //    248 / 235, of 80 349 / 363, of 500 1734 / 2241), and B up to a share of the L2 budget that grows with the launches
 //    saved: F = 512, two, 20 k of 30 87 / 77, 30 k 136 / 141; F = 256, two, 50 k of 30 109 / 103, 80 k 182 / 225; F = 96,
 //    three narrow ones, 100 k of 30 108 / 99, 150 k 162 / 167, 200 k 219 / 270; F = 64, two, 200 k of 30 147 / 121, 300 k
 //    of 45 at 0.91; F = 128, two, 150 k of 24 186 / 171, of 40 267 / 266; F = 192, three, 60 k of 24 108 / 78, 150 k 277 / 308.
-//  - 192 features: rows of any length while B fits (20 k of 80 81 / 73, of 480 465 / 425, 60 k of 80 268 / 226).
+//  - In place of three launches and more over tiles of 32 or 64, which read and add to C once for each, if the groups fill seven eighths of
+//    their tiles of 64: rows of any length while B fits (20 k rows of 200 F = 192 179 / 177, F = 224 231 / 222, F = 288 299 / 275, F = 320 306 / 288,
+//    F = 448 431 / 400; 60 k of 200 F = 192 610 / 549; F = 160, five sixths, 165 / 168, and F = 96 99 / 117 do not).
 bool in_groups(int m, int n, int feat, int nnz) {
   const int per_row = nnz / m, tile = lean_tile(n, feat);
   if (feat < 64) return false;
   if (per_row < 10) return true;
   const size_t b_bytes = static_cast<size_t>(n) * feat * 4;
-  if (feat == tile) return feat == 64 && per_row < (b_bytes > (size_t{32} << 20) ? 100 : 64);
-  if (feat == 192 && b_bytes <= l2_budget_bytes()) return true;
+  if (feat == tile) return feat == 64 && per_row < (b_bytes >= kFarBytes ? 100 : 64);
+  if (tile <= 64 && feat / tile >= 3 && feat * 8 >= ceil_div(feat, 64) * 64 * 7 && b_bytes <= l2_budget_bytes()) return true;
   const int eighths = tile == 256 || feat == 96 ? 8 : tile == 128 ? 9 : feat == 64 ? 11 : 13;
   return per_row < (feat == 64 ? 64 : 50) && b_bytes <= l2_budget_bytes() / 8 * eighths;
 }
