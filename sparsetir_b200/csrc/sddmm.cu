@@ -464,11 +464,13 @@ bool five_blocks(int n, int feat, int nnz) {
 
 // Feature counts in steps of 8 below 128 whose lanes the lean kernel fills better than the groups fill their tiles of 64, on rows long
 // enough for it and with a B that stays in L2 (us, groups / lean: 40 k rows of 500 F = 40 461 / 397, F = 104 711 / 611, F = 72 572 / 605,
-// F = 136 815 / 1146; 60 k of 20 F = 40 30.9 / 30.1, F = 104 48.1 / 49.2, 20 k of 40 34.9 / 30.8; F = 24, a group of 8 / lean, 20 k of 11 5.4 /
-// 5.6, 60 k of 30 26.2 / 21.3).
+// F = 136 815 / 1146; 60 k of 60 F = 88 126 / 138; 20 k of 11 F = 40 7.9 / 8.7, of 30 16.6 / 16.2, F = 104 24.5 / 23.9; F = 24, a group of 8 / lean, 20 k
+// of 11 5.4 / 5.6, 60 k of 30 26.2 / 21.6).  The lean kernel has half the blocks: not where the positions make one round of the groups
+// (10 k of 11 F = 40 4.9 / 6.5, 3 k of 30 4.7 / 5.9).
 bool lean_part(int m, int n, int feat, int nnz) {
-  if (feat % 8 != 0 || feat % 32 == 0 || feat >= 128 || (feat > 64 && feat <= 80)) return false;
-  return nnz / m >= (feat < 32 ? 16 : feat < 64 ? 10 : 24) && static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes();
+  if (feat % 8 != 0 || feat % 32 == 0 || feat >= 128 || (feat > 64 && feat < 96)) return false;
+  if (feat > 32 && nnz < 120000) return false;
+  return nnz / m >= (feat < 64 ? 16 : 24) && static_cast<size_t>(n) * feat * 4 <= l2_budget_bytes();
 }
 
 // One launch per tile, in stream order.
