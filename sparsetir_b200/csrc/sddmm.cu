@@ -344,10 +344,16 @@ template <int LPR, int W, int VPL, int BLOCKS = 4>
 int launch(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
            const float* scale, int m, int feat, int nnz, const PeerOut& po, cudaStream_t stream) {
   // one wave of resident blocks; two for the narrow vectors, whose positions take longer (50 k-node
-  // power-law graph, F = 299: 88 against 97 us)
-  const long long warps = static_cast<long long>(kNumSMs) * BLOCKS * (kThreads / 32) * (W < 4 ? 2 : 1);
-  int chunk = static_cast<int>((nnz + warps - 1) / warps);
-  chunk = (chunk + 31) & ~31;
+  // power-law graph, F = 299: 88 against 97 us), but one of them, with more positions per warp, where the second would be filled to less than 0.6
+  // (pairs, two waves / one, 1.06 of them, 80 k rows of 5, F = 298 131 / 105 us, 1.16, 20 k of 11, F = 190 26.3 / 22.7; 1.69, 80 k of 8,
+  // F = 46 25.6 / 26.9)
+  const long long wave = static_cast<long long>(kNumSMs) * BLOCKS * (kThreads / 32);
+  auto chunk_of = [&](long long warps) { return (static_cast<int>((nnz + warps - 1) / warps) + 31) & ~31; };
+  int chunk = chunk_of(W < 4 ? 2 * wave : wave);
+  if (W < 4 && BLOCKS == 5) {
+    const long long last = ceil_div(nnz, chunk) - wave;  // warps of the second
+    if (last > 0 && last * 10 < wave * 6) chunk = chunk_of(wave);
+  }
   const int blocks = ceil_div(ceil_div(nnz, chunk), kThreads / 32);
   const float rows_per_entry = static_cast<float>(m) / static_cast<float>(nnz);
   if constexpr (W >= 4 && BLOCKS == 4) {

@@ -68,7 +68,7 @@ def test_sddmm_on_uneven_rows(cuda_device, n, mean, feat, limit):
     check_ratio(sddmm_call(cuda_device, uneven, feat), sddmm_call(cuda_device, even, feat), limit)
 
 
-@pytest.mark.parametrize("n,mean,feat,other,limit", [(20_000, 10, 512, 128, 3.85), (20_000, 100, 224, 256, 1.08), (10_000, 11, 40, 64, 1.3)])
+@pytest.mark.parametrize("n,mean,feat,other,limit", [(20_000, 10, 512, 128, 3.85), (20_000, 100, 224, 256, 1.08), (10_000, 11, 40, 64, 1.3), (80_000, 5, 298, 300, 1.4)])
 def test_sddmm_of_more_and_fewer_features(cuda_device, n, mean, feat, other, limit):
     """Beside a neighbour that is known to be served well: what is fixed in a call weighs less where there are more features."""
     deg = lengths("equal", n, mean)
