@@ -403,18 +403,21 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
   // meeting of the pieces) is paid once, 4.5 M entries, F = 64: 94 us against 109 with four waves.
   // A block walks the feature tiles one after the other, all blocks roughly in step, which keeps
   // the slice of B that they gather from in L2; matrices too small to give every resident block
-  // a batch of entries deal the tiles to more blocks (60 k entries, F = 512: 25 against 37 us).
+  // three batches of entries for each of its sub-warps deal the tiles to more blocks, equal shares of them.
+  //
+  // Shares of a few batches are made up to a multiple of 8 entries and not to whole batches: of 32 entries, 40 k of them, F = 512, took 628
+  // blocks, 1.06 waves, or a third of the blocks for four tiles (us, four tiles side by side in 1.06 waves / three in one / four in one with
+  // shares of 40 entries: 10 k rows of 4 16.5 / 17.8 / 13.9, 10 k power-law rows 16.4 / 19.0 / 14.8; other calls of up to two waves, two waves / one
+  // with such shares: 20 k power-law rows F = 256 16.8 / 15.0, 9 k rows of 9 F = 384 18.0 / 15.3, 30 k of 5, F = 299 32.4 / 29.5; one tile, 40 k
+  // power-law rows, F = 100 16.9 / 15.4).  Two tiles on one block and one on the next: 14 k rows of 7, F = 384 20.2 / 23.5, three side by side 17.0.
   const long long resident = static_cast<long long>(blocks_per_sm(sh.w, sh.vpl)) * kNumSMs, batch = static_cast<long long>(subs) * sh.lanes;
   const long long fewest = (nnz + batch - 1) / batch;
   SplitPlan p;
-  // Up to twice as many blocks as fit at once where that spares them a round of tiles, with no more of them than the rounds need (us, as
-  // many as fit / so: 20 k-node power-law graph F = 256 19.8 / 16.9, F = 384 28.0 / 22.7, 9 k rows of 9 F = 384 24.3 / 17.8, 14 k power-law
-  // F = 130 18.9 / 13.5; with 2.25 times as many 30 k rows of 5, F = 256 20.9 / 21.5).
-  const long long side_by_side = std::min<long long>(tiles, std::max<long long>(1, resident * 15 / 8 / fewest));
-  const long long rounds = (tiles + side_by_side - 1) / side_by_side;
-  p.gy = static_cast<int>((tiles + rounds - 1) / rounds);
-  const long long want = std::max(resident / p.gy, std::min(fewest, resident)) * subs;
-  p.span = static_cast<int>((nnz + want - 1) / want + sh.lanes - 1) / sh.lanes * sh.lanes;
+  p.gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident * 3 / fewest)));
+  while (tiles % p.gy != 0) ++p.gy;
+  const long long want = std::max<long long>(1, resident / p.gy) * subs, share = (nnz + want - 1) / want;
+  const long long step = share < 4 * sh.lanes ? 8 : sh.lanes;
+  p.span = static_cast<int>(std::max<long long>(sh.lanes, (share + step - 1) / step * step));
   const long long per_block = static_cast<long long>(subs) * p.span;
   const long long with_entries = (nnz + per_block - 1) / per_block;  // the first blocks; the others clear rows
   p.blocks = static_cast<int>(std::max(with_entries, (static_cast<long long>(m) + 8 * kThreads - 1) / (8 * kThreads)));

@@ -18,12 +18,15 @@ SHAPES = {
     "empty_runs": ([0] * 5000 + [1] * 40) * 5 + [0] * 3000,
     "single_entries": [1] * 70_003,
     "mixed": [0, 1, 2, 300, 7, 0, 0, 33, 32, 31] * 1700,
+    # shares of a sub-warp that are more than one batch of entries and not a whole number of them
+    "shares_of_40_entries": [4, 0, 9, 1, 3, 11, 2, 5, 0, 6] * 1000,
+    "shares_of_24_to_80_entries": [9, 0, 20, 1, 13, 2, 45, 0] * 1000,
 }
 
 
 @pytest.mark.parametrize("shape", sorted(SHAPES))
 @pytest.mark.parametrize("feat,offset", [(32, 0), (64, 0), (100, 0), (300, 0), (41, 0), (46, 0), (299, 0), (130, 0), (1, 0),
-                                         (64, 1), (128, 2)])
+                                         (64, 1), (128, 2), (384, 0), (512, 0), (640, 0)])
 def test_rows_meet_across_sub_warps_and_blocks(cuda_device, shape, feat, offset):
     deg = np.asarray(SHAPES[shape], np.int64)
     m, n, nnz = len(deg), 4001, int(deg.sum())

@@ -52,24 +52,27 @@ def lengths(kind, n, mean):
     return np.clip(np.rint(rng.lognormal(np.log(mean) - 2.0, 2.0, n)), 1, n // 4).astype(np.int64)
 
 
-def sddmm_call(device, deg, feat):
+def csr_call(f, device, deg, feat):
+    """A kept call of sddmm or csrmm on a matrix of uniformly drawn columns."""
     n, nnz = len(deg), int(deg.sum())
     g = torch.Generator(device=device).manual_seed(feat)
     ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(device)
     cols = torch.randint(0, n, (nnz,), generator=g, device=device, dtype=torch.int32)
-    a, b = (torch.rand(n * feat, generator=g, device=device) for _ in range(2))
-    return ops.sddmm.prepare(a, b, torch.empty(nnz, device=device), ptr, cols)
+    a, b, e = (torch.rand(k, generator=g, device=device) for k in (n * feat, n * feat, nnz))
+    return f.prepare(a, b, e, ptr, cols) if f is ops.sddmm else f.prepare(e, a, b, ptr, cols)
 
 
 @pytest.mark.parametrize("n,mean,feat,limit", [(100_000, 30, 256, 1.2), (20_000, 30, 24, 1.18)])
 def test_sddmm_on_uneven_rows(cuda_device, n, mean, feat, limit):
     uneven = lengths("uneven", n, mean)
     even = lengths("equal", n, int(round(uneven.sum() / n)))
-    check_ratio(sddmm_call(cuda_device, uneven, feat), sddmm_call(cuda_device, even, feat), limit)
+    check_ratio(csr_call(ops.sddmm, cuda_device, uneven, feat), csr_call(ops.sddmm, cuda_device, even, feat), limit)
 
 
-@pytest.mark.parametrize("n,mean,feat,other,limit", [(20_000, 10, 512, 128, 3.85), (20_000, 100, 224, 256, 1.08), (10_000, 11, 40, 64, 1.3), (80_000, 5, 298, 300, 1.4)])
-def test_sddmm_of_more_and_fewer_features(cuda_device, n, mean, feat, other, limit):
+@pytest.mark.parametrize("op,n,mean,feat,other,limit", [
+    ("sddmm", 20_000, 10, 512, 128, 3.85), ("sddmm", 20_000, 100, 224, 256, 1.08), ("sddmm", 10_000, 11, 40, 64, 1.3), ("sddmm", 80_000, 5, 298, 300, 1.4),
+    ("csrmm", 10_000, 4, 512, 256, 1.62), ("csrmm", 20_000, 3, 384, 256, 1.4)])
+def test_more_and_fewer_features(cuda_device, op, n, mean, feat, other, limit):
     """Beside a neighbour that is known to be served well: what is fixed in a call weighs less where there are more features."""
-    deg = lengths("equal", n, mean)
-    check_ratio(sddmm_call(cuda_device, deg, feat), sddmm_call(cuda_device, deg, other), limit)
+    deg, f = lengths("equal", n, mean), getattr(ops, op)
+    check_ratio(csr_call(f, cuda_device, deg, feat), csr_call(f, cuda_device, deg, other), limit)
