@@ -41,8 +41,9 @@ int rgms_tc_launch(const float* a, const float* w, const float* x, float* y,
                    const int32_t* indptr_i, const int32_t* indices_i, const int32_t* indptr_j,
                    const int32_t* indices_j, int num_rels, int feat, int nnz_i,
                    const float* z, cudaStream_t stream);
-int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st);
-int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int feat,
+int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int nnz,
+                      cudaStream_t st);
+int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int nnz, int feat,
                      cudaStream_t st);
 int rgms_tma_launch_pairs(const float* a, const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i,
                           const int32_t* indptr_j, const int32_t* indices_j, int num_rels, int nnz_i, const float* z,
@@ -259,7 +260,7 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
       if (!fused)
         z = static_cast<float*>(workspace(device_id, st, static_cast<size_t>(nnz_i) * 64 * sizeof(float)));
       if (z != nullptr && single_rows()) {
-        if (rgms_pairs_launch(a, x, z, indptr_j, indices_j, nnz_i, st) != 0) return -1;
+        if (rgms_pairs_launch(a, x, z, indptr_j, indices_j, nnz_i, nnz_j, st) != 0) return -1;
         const int rc2 = rgms_tma_launch_pairs(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, z, st);
         if (rc2 <= 0) return rc2;
       }
@@ -282,7 +283,7 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
       if (rc == 0) {
         float* z = reinterpret_cast<float*>(cs.scratch);
         const int sums = aligned32(x) && aligned32(z)
-                             ? rgms_rows_launch(a, x, z, indptr_j, indices_j, nnz_i, feat, st)
+                             ? rgms_rows_launch(a, x, z, indptr_j, indices_j, nnz_i, nnz_j, feat, st)
                              : csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, feat, nnz_j, device_id, stream);
         if (sums != 0) return -1;
         if (rgms_wide_launch(w, y, indptr_i, indices_i, z, num_rels, nnz_i, feat, st) != 0) return -1;

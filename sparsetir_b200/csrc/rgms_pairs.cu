@@ -12,19 +12,56 @@
 // with branches of their own they executed 20.2 M instructions and took 47 us instead of 14.5 M and 37 (counters of one launch).
 // What bounds it is the latency of the gathers (10 of 16 waiting warps; L1 data path 49 %, issue slots 34 %, L2 35 %); twice the rows
 // in flight on half the warps is slower (the call 112 us against 99).
+#include <algorithm>
+
 #include "common.h"
 #include "launch.cuh"
-#include "vec.cuh"
+#include "row_walk.cuh"
 
 namespace sptir {
 namespace {
 
 constexpr int kThreads = 256;
+
+// The rows of a block that one group would walk alone while the rest of the call waits (more than 64 entries, or four times the average: a
+// destination with 1,000 edges of one relation): all groups share each of them, and their sums are added in a fixed order.  s_long: a bit for each
+// such row of a group.  us, alone / so, 1.5 M edges on 100 k nodes, destinations drawn as the square, the fourth and the eighth power of a uniform number:
+// 46 relations F = 64 360 / 107, 4361 / 253, 16054 / 739; 80 k edges on 10 k nodes, F = 128 86 / 57, 386 / 57, 1064 / 97; uniform ones 98.4 / 98.6
+// and 51 / 51.  The sums of the groups of a warp meet by shuffles: with 8 KB of shared memory for all of them, off L1, uniform ones took 99.6.
+template <int LPR, int W>
+__device__ __noinline__ void long_rows(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int rpi,
+                                       const unsigned* s_long) {
+  using LV = LaneVec<W>;
+  constexpr int SUBS = kThreads / LPR;
+  constexpr unsigned kRowBytes = LPR * W * 4;
+  constexpr int WARPS = kThreads / 32;
+  __shared__ __align__(32) float s_part[WARPS][LPR * W];
+  const int lane = threadIdx.x % LPR, sub = threadIdx.x / LPR;
+  const char* xl = reinterpret_cast<const char*>(x) + lane * (W * 4);
+  for (int owner = 0; owner < SUBS; ++owner) {
+    for (unsigned todo = s_long[owner]; todo != 0u; todo &= todo - 1u) {
+      const long long row = (static_cast<long long>(blockIdx.x) * SUBS + owner) * rpi + __ffs(todo) - 1;
+      const int begin = ld_global(indptr + row), end = ld_global(indptr + row + 1);
+      typename LV::type acc = LV::zero();
+      add_entries<LPR, W>(a, indices, xl, kRowBytes, begin + sub * LPR, end, SUBS * LPR, lane, group_mask<LPR>(), acc);
+#pragma unroll
+      for (int o = LPR; o < 32; o <<= 1) LV::add_xor(acc, o);
+      if (threadIdx.x % 32 < LPR) LV::sts(&s_part[threadIdx.x / 32][lane * W], acc);
+      __syncthreads();
+      if (sub == 0) {
+        for (int j = 1; j < WARPS; ++j) LV::add(acc, LV::lds(&s_part[j][lane * W]));
+        LV::stcg(reinterpret_cast<char*>(z) + row * kRowBytes + lane * (W * 4), acc);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // ALL: rows of one entry as well.
 template <int LPR, int W, bool ALL>
 __global__ void __launch_bounds__(kThreads, 4)
 rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
-                  const int32_t* indptr, const int32_t* indices, int m, int rpi) {
+                  const int32_t* indptr, const int32_t* indices, int m, int rpi, int long_row) {
   constexpr int kF = LPR * W;
   using LV = LaneVec<W>;
   constexpr int SUBS = kThreads / LPR;
@@ -37,7 +74,11 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
   const int r0 = static_cast<int>(min(r0l, static_cast<long long>(m))), row = r0 + lane;
   const bool there = lane < rpi && row < m;
   const int begin = ld_global(indptr + min(row, m)), len = there ? ld_global(indptr + min(row + 1, m)) - begin : -1;
-  const int own = len >= (ALL ? 1 : 2) ? len : 0;
+  __shared__ unsigned s_long[SUBS];
+  const unsigned own_long = (__ballot_sync(kAll, len > long_row) >> shift) & kGroup;
+  if (lane == 0) s_long[threadIdx.x / LPR] = own_long;
+  const bool any_long = __syncthreads_or(own_long != 0u);
+  const int own = len >= (ALL ? 1 : 2) && len <= long_row ? len : 0;
   int upto = own;  // entries of the rows up to this lane's
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) {
@@ -101,15 +142,16 @@ rgms_pairs_kernel(const float* a, const float* x, float* __restrict__ z,
       }
     }
   }
+  if (any_long) long_rows<LPR, W>(a, x, z, indptr, indices, rpi, s_long);
 }
 
 template <int LPR, int W, bool ALL>
-int launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, cudaStream_t st) {
+int launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int nnz, cudaStream_t st) {
   // fewer rows per group where the groups would not fill the SMs
   constexpr int kGroups = kThreads / LPR;
   int rpi = LPR;
   while (rpi > 1 && ceil_div(m, rpi) < kNumSMs * 4 * kGroups) rpi /= 2;
-  launch_chained(rgms_pairs_kernel<LPR, W, ALL>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, indptr, indices, m, rpi);
+  launch_chained(rgms_pairs_kernel<LPR, W, ALL>, ceil_div(ceil_div(m, rpi), kGroups), kThreads, 0, st, a, x, z, indptr, indices, m, rpi, std::max(64, 4 * (nnz / m)));
   SPTIR_LAUNCH_OK("rgms_pairs_kernel");
   return 0;
 }
@@ -117,17 +159,17 @@ int launch(const float* a, const float* x, float* z, const int32_t* indptr, cons
 }  // namespace
 
 int rgms_pairs_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m,
-                      cudaStream_t st) {
+                      int nnz, cudaStream_t st) {
   // 32-byte lanes lose where there are too few rows for the groups (3 k nodes, 12 k edges, the call 12.3 us with 16 bytes, 13.9 with 32)
-  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8, false>(a, x, z, indptr, indices, m, st);
-  return launch<16, 4, false>(a, x, z, indptr, indices, m, st);
+  if (m >= (1 << 15) && aligned32(x) && aligned32(z)) return launch<8, 8, false>(a, x, z, indptr, indices, m, nnz, st);
+  return launch<16, 4, false>(a, x, z, indptr, indices, m, nnz, st);
 }
 
 // All rows, 128 or 256 features, x and z 32-byte aligned.
-int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int feat,
-                     cudaStream_t st) {
-  if (feat == 128) return launch<16, 8, true>(a, x, z, indptr, indices, m, st);
-  return launch<32, 8, true>(a, x, z, indptr, indices, m, st);
+int rgms_rows_launch(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int m, int nnz,
+                     int feat, cudaStream_t st) {
+  if (feat == 128) return launch<16, 8, true>(a, x, z, indptr, indices, m, nnz, st);
+  return launch<32, 8, true>(a, x, z, indptr, indices, m, nnz, st);
 }
 
 }  // namespace sptir

@@ -115,5 +115,36 @@ __device__ __forceinline__ int row_in_window(const int32_t* indptr, int m, int r
   return row;
 }
 
+// acc += the entries [p0, p1) of a row, taken LPR at a time, `stride` apart
+template <int LPR, int W>
+__device__ __forceinline__ void add_entries(const float* a, const int32_t* indices,
+                                            const char* bl, unsigned row_bytes, int p0, int p1, int stride,
+                                            int lane, unsigned mask, typename LaneVec<W>::type& acc) {
+  using LV = LaneVec<W>;
+  constexpr int U = (32 / W) < LPR ? (32 / W) : LPR;
+  for (int e0 = p0; e0 < p1; e0 += stride) {
+    const bool live = lane < p1 - e0;
+    const int cid = live ? ld_global(indices + e0 + lane) : 0;
+    const float av = live ? ld_global(a + e0 + lane) : 0.f;
+    const int cnt = min(LPR, p1 - e0);
+#pragma unroll
+    for (int k0 = 0; k0 < LPR; k0 += U) {
+      if (k0 < cnt) {
+        typename LV::type x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned col = static_cast<unsigned>(__shfl_sync(mask, cid, k0 + u, LPR));
+          x[u] = LV::ldg(bl + static_cast<unsigned long long>(col) * row_bytes);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const float ak = __shfl_sync(mask, av, k0 + u, LPR);
+          if (k0 + u < cnt) LV::fma(acc, ak, x[u]);
+        }
+      }
+    }
+  }
+}
+
 }  // namespace sptir
 #endif  // SPARSETIR_B200_ROW_WALK_CUH_

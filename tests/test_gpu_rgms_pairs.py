@@ -45,8 +45,10 @@ def exact(a, w, x, ptr_i, rows, ptr_j, cols, n):
 
 @pytest.mark.parametrize("lens,relations", [
     ([1], [1]), ([0], [1]), ([0, 1, 2, 0, 3] * 51 + [1], [127, 129]), ([1] * 385, [128, 129, 0, 128]), ([1, 2] * 4097, [8000, 194]),
-    ([700, 1, 0, 1, 2, 33] * 40, [239, 1]), ([2, 0, 0, 1, 1, 1, 9, 1] * 10_000, [30_000, 50_000])],
-    ids=["one", "none", "mixed", "ones", "pairs", "hubs", "many"])
+    ([700, 1, 0, 1, 2, 33] * 40, [239, 1]), ([2, 0, 0, 1, 1, 1, 9, 1] * 10_000, [30_000, 50_000]),
+    # rows that all groups of a block share, from 65 entries on, alone and next to each other, in both forms of the first launch
+    ([64, 65, 66, 1, 0, 2] + [1, 2] * 400 + [5_000, 300], [807, 1]), (([1, 0, 2, 1, 1, 1, 1, 2] * 99 + [65, 0, 900, 257, 1, 64, 66, 511]) * 50, [40_000])],
+    ids=["one", "none", "mixed", "ones", "pairs", "hubs", "many", "shared", "shared_many"])
 @pytest.mark.parametrize("shift", [0, 4])
 def test_rows_of_one_edge(cuda_device, lens, relations, shift):
     n = 50_000

@@ -73,3 +73,25 @@ def test_inside_a_capture(cuda_device, warm):
     graph.replay()
     torch.cuda.synchronize()
     torch.testing.assert_close(y, want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("feat", [128, 256])
+def test_rows_that_a_block_shares(cuda_device, feat):
+    """(relation, destination) pairs of 63 to 66 edges and of thousands, beside rows of one and two edges and of none."""
+    lens = torch.tensor(([1, 2, 0, 1, 63, 1, 64, 0, 65, 66] + [1, 0, 2] * 40) * 6 + [3000, 0, 700], device=cuda_device)
+    n, rels, pairs = 1500, 2, len(lens)
+    g = torch.Generator(device=cuda_device).manual_seed(feat)
+    ptr_j = torch.cat([torch.zeros(1, dtype=torch.long, device=cuda_device), lens.cumsum(0)])
+    edges = int(ptr_j[-1])
+    ptr_i = torch.tensor([0, 500, pairs], device=cuda_device).int()
+    at = torch.arange(pairs, device=cuda_device)
+    pair = at + (at >= 500) * (n - 500)  # rows 0, 1, ... of each relation
+    a, x = torch.rand(edges, device=cuda_device, generator=g), torch.rand(n, feat, device=cuda_device, generator=g) * 2 - 1
+    w = torch.randn(rels, feat, feat, device=cuda_device, generator=g) / feat ** 0.5
+    src = torch.randint(0, n, (edges,), device=cuda_device, generator=g)
+    args = a, w, x, ptr_i, pair, ptr_j, src
+    d = [t.double() if t.is_floating_point() else t for t in args]
+    want, mag = product(*d), product(d[0], d[1].abs(), d[2].abs(), *d[3:])
+    y = torch.full((n, feat), 2.0, device=cuda_device)
+    ops.rgms(*arguments(*args, y))
+    assert bool(((y.double() - 2.0 - want).abs() <= (mag + 2.0) * (int(lens.max()) + feat + rels + 1) * 2.0 ** -24).all())

@@ -76,3 +76,20 @@ def test_more_and_fewer_features(cuda_device, op, n, mean, feat, other, limit):
     """Beside a neighbour that is known to be served well: what is fixed in a call weighs less where there are more features."""
     deg, f = lengths("equal", n, mean), getattr(ops, op)
     check_ratio(csr_call(f, cuda_device, deg, feat), csr_call(f, cuda_device, deg, other), limit)
+
+
+@pytest.mark.parametrize("feat", [64, 128])
+def test_rgms_with_hub_destinations(cuda_device, feat):
+    """20 of 10,000 destinations with 2,000 edges each, beside as many edges evenly."""
+    def layer(deg):
+        n, nnz = len(deg), int(deg.sum())
+        g = torch.Generator(device=cuda_device).manual_seed(feat)
+        ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(cuda_device)
+        cols = torch.randint(0, n, (nnz,), generator=g, device=cuda_device, dtype=torch.int32)
+        a, w, x = (torch.rand(k, generator=g, device=cuda_device) for k in (nnz, feat * feat, n * feat))
+        rows = torch.arange(n, device=cuda_device, dtype=torch.int32)
+        return ops.rgms.prepare(a, w, x, torch.zeros(n * feat, device=cuda_device), torch.tensor([0, n], device=cuda_device, dtype=torch.int32), rows,
+                                ptr, cols)
+    hubs = np.full(10_000, 4, np.int64)
+    hubs[250::500] = 2_000
+    check_ratio(layer(hubs), layer(np.full(10_000, 8, np.int64)), 2.0)
