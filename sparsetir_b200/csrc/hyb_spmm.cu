@@ -67,7 +67,6 @@ struct HybTable {
   int32_t block_start[kMaxB + 1];
   int32_t row_base[kMaxB];         // buckets without a row-id array: ELL row r -> output row base + r
   int32_t part_base[kMaxB];        // lean kernel: scratch row of ELL row 0, or -1 (bucket has no split rows)
-  int32_t long_rows;               // lean kernel: at least 8 slots per ELL row on average
   int32_t nb;
 };
 
@@ -221,14 +220,16 @@ __device__ __forceinline__ float4 lds4(const float* from) {
   return v;
 }
 
-// row_flag(g): flag word of ELL row g (called by the lane that will hold it)
-// row_end(acc, flag word): all lanes of the sub-warp, after the last slot of an ELL row
 // How ids and weights come to all lanes of a sub-warp: by shuffles, or four at a time by way of shared memory, which spares the data
 // path of L1, the busiest unit, three of four of these steps.  us, shuffles / shared: 20 k rows of 30 F = 128 28.7 / 27.3, F = 256 46.1 /
 // 40.5, F = 512 89.7 / 77.3; rows of 500 F = 300 420 / 387, F = 512 558 / 528; the 169 k-node power-law graph F = 256 100.6 / 98.4, F = 512
-// 187 / 182.  kChunks: shuffles in the loop that kShared has.
+// 187 / 182.  kChunks: shuffles in the loop that kShared has, for long rows in one tile of 8 lanes (3 k rows of 30, F = 32 4.4, so 4.0, shared 4.2; 60 k
+// of them 20.3, 19.1, 19.8), but not for the spans of wide rows (log-normal rows, 60 k of 60, F = 32 so 51.7, shared 47.6).
 enum Hand : int { kShuffles, kChunks, kShared };
-// WM = 1, 2, 4: the ELL width itself; 8: a multiple of 8
+
+// Walks the slots of an item's ELL rows.  WM = 1, 2, 4: their width itself; 8: a multiple of 8.
+// row_flag(g): flag word of ELL row g (called by the lane that will hold it)
+// row_end(acc, flag word): all lanes of the sub-warp, after the last slot of an ELL row
 template <int LPR, int WM, int W, int VPL, bool WHOLE, Hand HAND, class RowFlag, class RowEnd>
 __device__ __forceinline__ void lean_item(const int32_t* cols,
                                           const float* wts, int r0, int nr, int nslots,
@@ -560,7 +561,8 @@ __device__ __noinline__ void split_item(const LaneTile<LPR, W, VPL, WHOLE> lt, c
 }
 
 // blockIdx.y = feature tile of LPR * W * VPL floats; the last one may be partly filled
-template <int LPR, int W, int VPL, bool WHOLE, bool PEERS, bool SHARED>
+// HAND: of rows of 8 slots and more
+template <int LPR, int W, int VPL, bool WHOLE, bool PEERS, Hand HAND>
 __global__ void __launch_bounds__(kThreads, 8)
 hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant__ LeanArgs la) {
   using LT = LaneTile<LPR, W, VPL, WHOLE>;
@@ -625,11 +627,7 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
     if (width == 1) lean_item<LPR, 1, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
     else if (width == 2) lean_item<LPR, 2, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
     else if (width == 4) lean_item<LPR, 4, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
-    else if (!SHARED) lean_item<LPR, 8, W, VPL, WHOLE, kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
-    // Not in one tile of 8 lanes (20 k rows of 30, F = 32, by shuffles / shared 10.1 / 10.6), nor on short rows in tiles that rows do not fill
-    // (169 k-node power-law graph, F = 300, 160.3 / 161.5).
-    else if (LPR == 8 ? gridDim.y > 1 : LPR > 16 || WHOLE || tb.long_rows != 0) lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kShared : kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
-    else lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kChunks : kShuffles>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
+    else lean_item<LPR, 8, W, VPL, WHOLE, HAND>(cols, wts, r0, nr, nslots, width, bl, stride, lt, lane, mask, s_sub[sub].slots, row_flag, row_end);
     return;
   }
 
@@ -657,8 +655,8 @@ hyb_spmm_lean_kernel(const __grid_constant__ HybTable tb, const __grid_constant_
     const size_t first = static_cast<size_t>(r) * width + s0;
     auto no_flag = [](int) -> int { return 0; };
     auto keep = [&](V& acc, int) { total = acc; };
-    lean_item<LPR, 8, W, VPL, WHOLE, SHARED ? kShared : kShuffles>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lt, lane, mask,
-                                              s_sub[sub].slots, no_flag, keep);
+    lean_item<LPR, 8, W, VPL, WHOLE, HAND == kShuffles ? kShuffles : kShared>(tb.cols[q] + first, tb.w[q] + first, r, 1, nslots, nslots, bl, stride, lt, lane, mask,
+                                             s_sub[sub].slots, no_flag, keep);
   }
   __syncwarp(mask);  // every lane is done with the batches
   if (part != 0) LT::sts(s_sub[sub].part, lane, total);
@@ -903,23 +901,28 @@ long long plan_blocks(HybTable& tb, int subs) {
 template <int LPR, int W, int VPL, bool WHOLE>
 int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
   const int tiles = ceil_div(la.feat, W * LPR * VPL);
-  long long slots = 0, rows = 0;
+  long long slots = 0, rows = 0, wide = 0;  // wide: slots of rows of 8 and more
   for (int q = 0; q < tb.nb; ++q) {
+    const long long of = static_cast<long long>(tb.nrows[q]) * tb.width[q];
     rows += tb.nrows[q];
-    slots += static_cast<long long>(tb.nrows[q]) * tb.width[q];
+    slots += of;
+    if (tb.width[q] >= 8) wide += of;
   }
-  tb.long_rows = slots >= 8 * rows ? 1 : 0;
   plan_items_lean(tb, lean_item_slots(LPR, W, tiles, slots), kThreads / LPR);
   const long long blocks = plan_blocks_lean(tb, kThreads / LPR);
   if (blocks < 0) return fail("sparsetir_hyb_spmm: too many thread blocks");
   dim3 grid(static_cast<unsigned>(blocks), tiles);
   // 32-byte lanes and rows of 34, 38, 42... features, one pair to a lane, lose by it (20 k-node power-law graph, F = 34 8.9 / 10.7 us).
   constexpr bool kMay = W <= 4 && !(W == 2 && VPL == 1);
-  // Tiles of 8 lanes: not on short rows, where they wait for chains of loads and not for L1 (169 k-node power-law graph, F = 100 59.8 / 61.1,
-  // F = 128 53.9 / 54.5; F = 32 among other work 19.3 / 19.6), nor where one tile adds all results atomically (F = 32, two partitions 24.6 / 25.3).
-  const bool shared = kMay && (LPR > 8 || (tb.long_rows != 0 && (tiles > 1 || la.all_atomic == 0)));
-  auto go = [&](auto in_shared) -> int {
-    constexpr bool S = decltype(in_shared)::value;
+  // Shared memory is written and waited for once per batch, whatever its rows: where most slots are in rows of 1, 2 and 4, which keep the shuffles, the
+  // kernel with both loops only has fewer registers for theirs (20 k rows of 3, F = 299 13.3 / 14.5, F = 256 10.8 / 11.3).  Tiles of 8 lanes: not on
+  // short rows either, where they wait for chains of loads and not for L1 (169 k-node power-law graph, F = 100 59.8 / 61.1, F = 128 53.9 / 54.5; F = 32 among
+  // other work 19.3 / 19.6; tiles that rows do not fill, 40 k rows of 8, F = 100 16.5 / 17.6; one tile, 40 k rows of 9, F = 32 8.3 / 8.6), nor where one tile adds all
+  // results atomically (F = 32, two partitions 24.6 / 25.3).
+  const bool long_rows = slots >= (tiles == 1 ? 16 * rows : WHOLE ? 8 * rows : 8 * rows + 1);
+  const bool shared = kMay && (LPR > 8 ? 4 * wide >= slots : long_rows && (tiles > 1 || la.all_atomic == 0));
+  auto go = [&](auto hand) -> int {
+    constexpr Hand S = decltype(hand)::value;
     if (la.peers.n > 0) {
       if constexpr (W == 4 && WHOLE)
         launch_chained(hyb_spmm_lean_kernel<LPR, W, VPL, WHOLE, true, S>, grid, kThreads, 0, stream, tb, la);
@@ -930,11 +933,15 @@ int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
     }
     return 0;
   };
-  if constexpr (LPR > 8 || !kMay) {
-    if (go(std::bool_constant<kMay>{}) != 0) return -1;
+  using Shuffles = std::integral_constant<Hand, kShuffles>;
+  int rc;
+  if constexpr (!kMay) {
+    rc = go(Shuffles{});
   } else {
-    if ((shared ? go(std::true_type{}) : go(std::false_type{})) != 0) return -1;
+    using InChunks = std::integral_constant<Hand, LPR == 8 ? kChunks : kShared>;
+    rc = !shared ? go(Shuffles{}) : LPR == 8 && tiles == 1 ? go(InChunks{}) : go(std::integral_constant<Hand, kShared>{});
   }
+  if (rc != 0) return -1;
   SPTIR_LAUNCH_OK("hyb_spmm_lean_kernel");
   return 0;
 }

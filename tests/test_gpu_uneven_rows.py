@@ -93,3 +93,15 @@ def test_rgms_with_hub_destinations(cuda_device, feat):
     hubs = np.full(10_000, 4, np.int64)
     hubs[250::500] = 2_000
     check_ratio(layer(hubs), layer(np.full(10_000, 8, np.int64)), 2.0)
+
+
+@pytest.mark.parametrize("n,width,feat,other,limit", [(20_000, 4, 299, 300, 1.13)])
+def test_hyb_of_more_and_fewer_features(cuda_device, n, width, feat, other, limit):
+    """ELL rows of one width."""
+    def call(f):
+        g = torch.Generator(device=cuda_device).manual_seed(f)
+        x = torch.rand(n, f, generator=g, device=cuda_device)
+        bucket = (torch.rand(n * width, generator=g, device=cuda_device), torch.arange(n, device=cuda_device, dtype=torch.int32),
+                  torch.randint(0, n, (n * width,), generator=g, device=cuda_device, dtype=torch.int32))
+        return ops.hyb_spmm.prepare(*ops.hyb_args(x, torch.zeros(n, f, device=cuda_device), [bucket], f, 0))
+    check_ratio(call(feat), call(other), limit)
