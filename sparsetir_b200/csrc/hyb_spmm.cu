@@ -823,8 +823,9 @@ void plan_items(HybTable& tb, int item) {
 }
 
 // Lean kernel: a bucket wider than an item gives each ELL row a power-of-two number of sub-warps of
-// one block (all of them from SUBS * item slots on; a sub-warp then walks a longer span).
-void plan_items_lean(HybTable& tb, int item, int subs) {
+// one block (all of them from SUBS * item slots on; a sub-warp then walks a longer span).  Returns the number of blocks or -1.
+long long plan_lean(HybTable& tb, int item, int subs) {
+  long long blocks = 0;
   for (int q = 0; q < tb.nb; ++q) {
     tb.rows_per_item[q] = std::max(1, item / tb.width[q]);
     // rows of 8 slots or more: the row ids of an item travel in one register per lane
@@ -833,14 +834,7 @@ void plan_items_lean(HybTable& tb, int item, int subs) {
     while (spr < subs && spr * item < tb.width[q]) spr *= 2;
     tb.chunks_per_row[q] = spr;
     if (spr > 1) tb.rows_per_item[q] = 1;
-  }
-}
-
-long long plan_blocks_lean(HybTable& tb, int subs) {
-  long long blocks = 0;
-  for (int q = 0; q < tb.nb; ++q) {
     tb.block_start[q] = static_cast<int32_t>(blocks);
-    const int spr = tb.chunks_per_row[q];
     const long long per_block = spr > 1 ? subs / spr : static_cast<long long>(subs) * tb.rows_per_item[q];
     blocks += (tb.nrows[q] + per_block - 1) / per_block;
     if (blocks > INT32_MAX) return -1;
@@ -908,9 +902,18 @@ int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
     slots += of;
     if (tb.width[q] >= 8) wide += of;
   }
-  plan_items_lean(tb, lean_item_slots(LPR, W, tiles, slots), kThreads / LPR);
-  const long long blocks = plan_blocks_lean(tb, kThreads / LPR);
+  const int item = lean_item_slots(LPR, W, tiles, slots);
+  long long blocks = plan_lean(tb, item, kThreads / LPR);
   if (blocks < 0) return fail("sparsetir_hyb_spmm: too many thread blocks");
+  // A second wave of a few blocks costs as much as a full one: items long enough to make one of both, up to a quarter longer, a third where rows are
+  // long and all alike in cost (us, 1.06 waves / one: 10 k rows of 12, F = 512 25.5 / 17.7, 20 k of 8, F = 128 10.3 / 7.7; 1.32 waves, 10 k of 10,
+  // F = 300 19.1 / 14.3, but power-law rows, 20 k, F = 200 14.8 / 16.1).  Single floats per lane lose by it (14 k power-law rows, F = 299 19.4 / 21.5).
+  constexpr long long kResident = 8ll * kNumSMs;
+  if (W > 1 && blocks * tiles > kResident && blocks * tiles * 100 <= kResident * (slots >= 8 * rows ? 135 : 125)) {
+    long long fit = blocks;
+    for (int more = item + 8; fit * tiles > kResident && more <= 2 * item; more += 8) fit = plan_lean(tb, more, kThreads / LPR);
+    blocks = fit * tiles > kResident ? plan_lean(tb, item, kThreads / LPR) : fit;
+  }
   dim3 grid(static_cast<unsigned>(blocks), tiles);
   // 32-byte lanes and rows of 34, 38, 42... features, one pair to a lane, lose by it (20 k-node power-law graph, F = 34 8.9 / 10.7 us).
   constexpr bool kMay = W <= 4 && !(W == 2 && VPL == 1);

@@ -75,6 +75,42 @@ def test_ids_by_shuffles_and_through_shared_memory(cuda_device, n, feat, parts, 
     assert bool(((y.double() - want).abs() <= mag * (dev(deg)[:, None].double() + 1) * 2.0 ** -24).all())
 
 
+@pytest.mark.parametrize("feat,lanes,floats", [(512, 32, 4), (64, 8, 4), (130, 32, 2), (256, 32, 4)])
+@pytest.mark.parametrize("buckets", [[1, 2, 4, 8], [4, 8, 24]])
+def test_items_that_fill_one_wave(cuda_device, feat, lanes, floats, buckets):
+    """Calls of a little more than one wave of blocks, whose items are made longer: numbers of rows per item that are no power of two, in
+    every bucket, with rows split over items of the widest one."""
+    rng = np.random.default_rng(feat)
+    n, rows, top = 3000, 60_000, buckets[-1]
+    deg = np.minimum(rng.integers(1, 14, rows), top)
+    if top == 24:
+        deg[::5] = rng.integers(9, 25, rows // 5)
+    tiles, per_block = -(-feat // (lanes * floats * (2 if floats == 2 else 1))), 128 // lanes
+
+    def blocks(deg, item=lanes * floats):
+        width = np.array(buckets)[np.searchsorted(buckets, np.minimum(deg, top))]
+        ell = np.where(deg > top, -(-deg // top), 1)
+        return sum(-(-int(ell[width == w].sum()) // (per_block * max(1, item // w))) for w in buckets) * tiles / (8 * 148)
+
+    deg = np.concatenate([[2900, 100, 30, 1300], deg[:next(k for k in range(1000, rows, 250) if blocks(deg[:k]) > 1.1)], [60, 2000]])
+    deg = deg[rng.permutation(len(deg))]
+    assert 1.0 < blocks(deg) < 1.25
+    m = len(deg)
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    cols = np.concatenate([np.sort((k + np.arange(d) * (n // d)) % n) for k, d in zip(rng.integers(0, n, m), deg)]).astype(np.int32)
+    vals = rng.uniform(-1, 1, len(cols)).astype(np.float32)
+    r, c, _, v, _ = fmt.column_part_hyb(m, n, indptr, cols, 1, buckets, data=vals)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)  # noqa: E731
+    bk = [(dev(v[0][b]), dev(r[0][b]), dev(c[0][b])) for b in range(len(buckets)) if len(r[0][b])]
+    x = torch.rand(n, feat, generator=torch.Generator(cuda_device).manual_seed(feat), device=cuda_device) * 2 - 1
+    y = torch.full((m, feat), float("nan"), device=cuda_device)
+    for _ in range(2):
+        ops.hyb_spmm(*ops.hyb_args(x.view(-1), y.view(-1), bk, feat, 0))
+    a = torch.sparse_csr_tensor(dev(indptr).long(), dev(cols).long(), dev(vals).double(), (m, n))
+    mag = torch.sparse_csr_tensor(dev(indptr).long(), dev(cols).long(), dev(vals).double().abs(), (m, n)) @ x.double().abs()
+    assert bool(((y.double() - a @ x.double()).abs() <= mag * (dev(deg)[:, None].double() + 1) * 2.0 ** -24).all())
+
+
 BEYOND_THE_LIMIT = """
 import numpy as np, torch
 from sparsetir_b200 import format as fmt, ops

@@ -95,7 +95,7 @@ def test_rgms_with_hub_destinations(cuda_device, feat):
     check_ratio(layer(hubs), layer(np.full(10_000, 8, np.int64)), 2.0)
 
 
-@pytest.mark.parametrize("n,width,feat,other,limit", [(20_000, 4, 299, 300, 1.13)])
+@pytest.mark.parametrize("n,width,feat,other,limit", [(20_000, 4, 299, 300, 1.13), (20_000, 8, 512, 256, 2.2)])
 def test_hyb_of_more_and_fewer_features(cuda_device, n, width, feat, other, limit):
     """ELL rows of one width."""
     def call(f):
