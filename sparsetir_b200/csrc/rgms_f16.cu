@@ -508,7 +508,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
             tc05::tma_load_2d(st + kZBoxB + j * kWBoxB, &tm_w, j * 64, wrow + c * kKC, &bar_full[s]);
           armed = it + 1;
         }
-        if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
+        if (k + 1 == tiles_per_cta || !tw.next_apart(walk, num_ranges)) break;
       }
     }
   } else if (warp == 1) {
@@ -540,7 +540,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         }
         if (!ok) break;
         tc05::mma_commit(&bar_acc_full[buf]);
-        if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
+        if (k + 1 == tiles_per_cta || !tw.next_apart(walk, num_ranges)) break;
       }
     }
   } else if (GATHER && warp >= 12) {
@@ -572,7 +572,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         }
         pending = s;
       }
-      if (k + 1 == tiles_per_cta || !tw.next(walk, num_ranges)) break;
+      if (k + 1 == tiles_per_cta || !tw.next_apart(walk, num_ranges)) break;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");  // also when giving up: nothing may land later
     if (ok && pending >= 0) {
@@ -590,7 +590,7 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
     unsigned char* my_row = gbuf + t * kOutStride;
     const unsigned char* wbase = gbuf + (warp & 3) * 32 * kOutStride;
     bool have = true;
-    if (grp == 1) have = tiles_per_cta > 1 && tw.next(walk, num_ranges);
+    if (grp == 1) have = tiles_per_cta > 1 && tw.next_apart(walk, num_ranges);
     for (int k = grp; have && k < tiles_per_cta; k += 2) {
       const int buse = k >> 1;
       const int nrows = tw.row1 - tw.row0;
@@ -617,8 +617,8 @@ rgms_f16_tc_kernel(const __grid_constant__ CUtensorMap tm_z, const __grid_consta
         __syncwarp();
         scatter32(y, wbase, kOutStride, dst_row, (warp & 3) * 32, nrows, feat_out, c0, lane);
       }
-      bool has_next = (k + 2 < tiles_per_cta) && tw.next(walk, num_ranges);
-      has_next = has_next && tw.next(walk, num_ranges);
+      bool has_next = (k + 2 < tiles_per_cta) && tw.next_apart(walk, num_ranges);
+      has_next = has_next && tw.next_apart(walk, num_ranges);
       if (!has_next) break;
     }
   }

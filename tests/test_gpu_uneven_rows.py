@@ -105,3 +105,19 @@ def test_hyb_of_more_and_fewer_features(cuda_device, n, width, feat, other, limi
                   torch.randint(0, n, (n * width,), generator=g, device=cuda_device, dtype=torch.int32))
         return ops.hyb_spmm.prepare(*ops.hyb_args(x, torch.zeros(n, f, device=cuda_device), [bucket], f, 0))
     check_ratio(call(feat), call(other), limit)
+
+
+def test_rgms_f16_with_more_ranges_than_a_block_keeps(cuda_device):
+    """1,800 (bucket, relation) ranges, most of them empty, beside 900."""
+    def layer(rels, n=2000, feat=32):
+        g = torch.Generator(device=cuda_device).manual_seed(rels)
+        buckets = []
+        for width in (1, 2, 4, 8, 16, 32):
+            k = rels if width == 1 else 2
+            shape = (k, 32 // width, width)
+            buckets.append((torch.rand(shape, generator=g, device=cuda_device).half(),
+                            torch.randint(0, n, shape[:2], generator=g, device=cuda_device).int(),
+                            torch.randint(0, n, shape, generator=g, device=cuda_device).int(), torch.arange(k, device=cuda_device).int()))
+        x, w = (torch.rand(k, generator=g, device=cuda_device).half() for k in (n * feat, rels * feat * feat))
+        return ops.rgms_ell3d_f16.prepare(*ops.rgms_ell3d_f16_args(w, x, torch.zeros(n * feat, device=cuda_device), buckets, feat, feat))
+    check_ratio(layer(300), layer(150), 3.45)
