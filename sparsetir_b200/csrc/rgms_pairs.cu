@@ -29,7 +29,7 @@ constexpr int kThreads = 256;
 // 46 relations F = 64 360 / 107, 4361 / 253, 16054 / 739; 80 k edges on 10 k nodes, F = 128 86 / 57, 386 / 57, 1064 / 97; uniform ones 98.4 / 98.6
 // and 51 / 51.  The sums of the groups of a warp meet by shuffles: with 8 KB of shared memory for all of them, off L1, uniform ones took 99.6.
 template <int LPR, int W>
-__device__ __noinline__ void long_rows(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int rpi,
+__device__ __forceinline__ void long_rows(const float* a, const float* x, float* z, const int32_t* indptr, const int32_t* indices, int rpi,
                                        const unsigned* s_long) {
   using LV = LaneVec<W>;
   constexpr int SUBS = kThreads / LPR;
