@@ -261,8 +261,7 @@ extern "C" int sparsetir_rgms_raw(const float* a, const float* w, const float* x
         z = static_cast<float*>(workspace(device_id, st, static_cast<size_t>(nnz_i) * 64 * sizeof(float)));
       if (z != nullptr && single_rows()) {
         if (rgms_pairs_launch(a, x, z, indptr_j, indices_j, nnz_i, nnz_j, st) != 0) return -1;
-        const int rc2 = rgms_tma_launch_pairs(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, z, st);
-        if (rc2 <= 0) return rc2;
+        return rgms_tma_launch_pairs(a, w, x, y, indptr_i, indices_i, indptr_j, indices_j, num_rels, nnz_i, z, st);
       }
       if (z != nullptr) {
         if (csrmm_short_rows_impl(a, x, z, indptr_j, indices_j, nnz_i, n, 64, nnz_j, device_id, stream) != 0)

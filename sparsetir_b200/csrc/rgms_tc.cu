@@ -285,7 +285,7 @@ struct LookAhead {
   const PairRows& pairs;
   const T* from;
   int t, nnz_i;
-  T none, value, value_next;
+  T none, value;
   int row0, nrows, row0_next, nrows_next, begin, len;
   bool more;
   __device__ __forceinline__ LookAhead(TileWalk& walk, const StagedRanges& ptr_i, int rels, int num_tiles, const PairRows& p, const T* f,
@@ -575,15 +575,15 @@ rgms_tma_kernel(const __grid_constant__ CUtensorMap tm_z, const float* z, const 
   if (warp == 0) tc05::tmem_dealloc(tmem, kPTmem);
 }
 
-// 0 when launched, 1 when this path cannot take the call (caller falls back), -1 on error
+// 0 when launched, 1 when this path cannot take the call (caller falls back; never with pairs, whose rows need no tensor map), -1 on error.
+// With pairs z, x, y and w are 16-byte aligned and there are rows.
 int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int32_t* indices_i,
                     int num_rels, int nnz_i, const float* z, const PairRows& pairs, cudaStream_t stream, int rel_mod = 0) {
-  if (nnz_i <= 0 || num_rels <= 0) return 1;
-  if ((reinterpret_cast<uintptr_t>(z) & 15u) || (reinterpret_cast<uintptr_t>(y) & 15u) ||
-      (reinterpret_cast<uintptr_t>(w) & 15u))
-    return 1;
-  CUtensorMap tm_z;
-  if (make_tmap_2d(&tm_z, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z, kF, static_cast<uint64_t>(nnz_i), kF * 4, 32,
+  const bool gather = pairs.x != nullptr;
+  if (!gather && (nnz_i <= 0 || num_rels <= 0 || !aligned16(z) || !aligned16(y) || !aligned16(w))) return 1;
+  CUtensorMap tm_z{};
+  if (!gather &&
+      make_tmap_2d(&tm_z, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z, kF, static_cast<uint64_t>(nnz_i), kF * 4, 32,
                    kTM, CU_TENSOR_MAP_SWIZZLE_128B) != 0)
     return 1;
   static thread_local int configured_device = -1;
@@ -597,7 +597,7 @@ int rgms_tma_launch(const float* w, float* y, const int32_t* indptr_i, const int
   const long long tiles = static_cast<long long>(nnz_i) / kTM + num_rels;  // upper bound
   const long long grid = tiles < kNumSMs ? tiles : kNumSMs;
   const int tiles_per_cta = static_cast<int>((tiles + grid - 1) / grid);
-  if (pairs.x != nullptr)
+  if (gather)
     launch_chained(rgms_tma_kernel<true>, static_cast<unsigned>(grid), kPThreads + 128, kPSmemBytes, stream, tm_z, z, pairs, w, y, indptr_i,
                    indices_i, num_rels, nnz_i, tiles_per_cta, rel_mod);
   else
@@ -622,8 +622,8 @@ int rgms_tma_launch_ranges(const float* w, float* y, const int32_t* indptr_i, co
   return rgms_tma_launch(w, y, indptr_i, indices_i, num_ranges, nnz_i, z, PairRows{}, stream, rel_mod);
 }
 
-// The second launch behind rgms_pairs_launch(): rows of one entry straight from X.  0 when launched, 1 when this path cannot take the
-// call, -1 on error.
+// The second launch behind rgms_pairs_launch(): rows of one entry straight from X.  There are rows, and w, x, y and z are 16-byte aligned.
+// 0 when launched, -1 on error.
 int rgms_tma_launch_pairs(const float* a, const float* w, const float* x, float* y, const int32_t* indptr_i, const int32_t* indices_i,
                           const int32_t* indptr_j, const int32_t* indices_j, int num_rels, int nnz_i, const float* z,
                           cudaStream_t stream) {
