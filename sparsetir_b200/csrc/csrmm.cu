@@ -191,8 +191,7 @@ void csr_split_scratch_bound(int m, int n, int feat, int nnz, size_t* part_bytes
 
 namespace {
 // Whether a call takes the row-wise kernel, and with which lanes.
-bool row_wise(const float* b, const float* c, int m, int n, int feat, int nnz, bool hub_rows, int lane_floats,
-              int* lane_w, int* lanes_per_row) {
+bool row_wise(const float* b, const float* c, int m, int n, int feat, int nnz, bool hub_rows, int* lane_w, int* lanes_per_row) {
   const bool vec4 = (feat % 4 == 0) && aligned16(b) && aligned16(c);
   // The row-wise kernel needs whole feature tiles.  Its share ends where the split by entries is
   // the faster one although it has to search for its rows: 4,096 rows of 10 entries, F = 64, 4.8
@@ -203,7 +202,7 @@ bool row_wise(const float* b, const float* c, int m, int n, int feat, int nnz, b
   // lanes per row: one per 32-byte vector when the operands allow it, else one per 16-byte
   // vector; narrowed until the n x tile slice of B that a pass over the rows gathers from fits
   // the resident part of L2 (see hyb_spmm.cu)
-  const int w = (feat % 32 == 0 && aligned32(b) && aligned32(c)) ? (lane_floats == 8 ? 8 : max_lane_floats()) : 4;
+  const int w = (feat % 32 == 0 && aligned32(b) && aligned32(c)) ? max_lane_floats() : 4;
   const int nv = feat / w;
   int lanes = nv <= 4 ? 4 : (nv <= 8 ? 8 : (nv <= 16 ? 16 : 32));
   if (w == 4 && lanes < 8) lanes = 8;
@@ -219,17 +218,15 @@ bool row_wise(const float* b, const float* c, int m, int n, int feat, int nnz, b
 // Scratch that a csrmm call over these operands needs (0: none), for callers that hold the stream's buffer.
 size_t csrmm_scratch(const float* b, const float* c, int m, int n, int feat, int nnz) {
   int w = 0, lanes = 0;
-  return row_wise(b, c, m, n, feat, nnz, true, 0, &w, &lanes) ? 0 : csr_split_scratch(b, c, m, n, feat, nnz);
+  return row_wise(b, c, m, n, feat, nnz, true, &w, &lanes) ? 0 : csr_split_scratch(b, c, m, n, feat, nnz);
 }
 
 // The launcher behind sparsetir_csrmm_raw.  hub_rows = false: the caller knows that its rows are
 // short, and that b and c are 16-byte aligned with feat a multiple of 64 that makes whole tiles; such a
 // call never touches the per-stream workspace (the caller may hold it).
-// lane_floats: 0 = the library's default lane width, 8 = 32-byte lanes where the operands allow.
 // pieces: csrmm_scratch() bytes from a caller that holds the stream's scratch buffer, null from others.
 int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
-              int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats,
-              void* pieces) {
+              int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows, void* pieces) {
   if (m < 0 || feat < 0 || nnz < 0) return fail("sparsetir_csrmm: negative size");
   if (m == 0 || feat == 0) return 0;
   if (!b || !c || !indptr || (nnz > 0 && (!a || !indices)))
@@ -238,7 +235,7 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (validate_enabled() && validate_csr("sparsetir_csrmm", indptr, m, indices, nnz, n, st) != 0) return -1;
   int w = 0, lanes = 0;
-  if (row_wise(b, c, m, n, feat, nnz, hub_rows, lane_floats, &w, &lanes)) {
+  if (row_wise(b, c, m, n, feat, nnz, hub_rows, &w, &lanes)) {
     const int subs = kThreads / lanes;
     // about four id batches per item, but never so few items that SMs sit idle
     const double avg = m > 0 ? static_cast<double>(nnz) / m : 0.0;
@@ -273,19 +270,15 @@ int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, c
 
 int csrmm_impl(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices,
                int m, int n, int feat, int nnz, int device_id, void* stream, bool hub_rows) {
-  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, hub_rows, 0, nullptr);
+  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, hub_rows, nullptr);
 }
 
-// For matrices of very short rows (the aggregation launch of RGMS: 2.2 entries per row), where the
-// kernel is bound by instruction issue: 32-byte lanes halve the instructions per gathered byte
-// (60 -> 56.5 us at 690,812 rows x 64 features), although they lose on long rows and on launches
-// too small to fill the SMs with the halved number of lanes (a quarter of those rows: 64 against
-// 58 us for the whole operator), so they are taken from half a million rows up.
+// For matrices of very short rows: the sums of RGMS where rgms_pairs.cu does not take them, which is under its comparison switch at 64
+// features, and at 128 and 256 where X is not 32-byte aligned.
 int csrmm_short_rows_impl(const float* a, const float* b, float* c, const int32_t* indptr,
                           const int32_t* indices, int m, int n, int feat, int nnz, int device_id,
                           void* stream) {
-  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, false, m >= (1 << 19) ? 8 : 0,
-                   nullptr);
+  return csrmm_run(a, b, c, indptr, indices, m, n, feat, nnz, device_id, stream, false, nullptr);
 }
 }  // namespace sptir
 

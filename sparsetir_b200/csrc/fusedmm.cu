@@ -165,7 +165,7 @@ namespace sptir {
 // defined in csrmm.cu
 size_t csrmm_scratch(const float* b, const float* c, int m, int n, int feat, int nnz);
 int csrmm_run(const float* a, const float* b, float* c, const int32_t* indptr, const int32_t* indices, int m, int n,
-              int feat, int nnz, int device_id, void* stream, bool hub_rows, int lane_floats, void* pieces);
+              int feat, int nnz, int device_id, void* stream, bool hub_rows, void* pieces);
 bool softmax_by_blocks(int n, int nnz);  // defined in csr_misc.cu
 namespace {
 // scores and probabilities, the second in place of the first where the softmax can, and where the pieces of the
@@ -229,6 +229,6 @@ extern "C" int sparsetir_fusedmm_raw(const float* q, const float* k, const float
   float* probs = softmax_by_blocks(m, nnz) ? scores : scores + nnz;
   if (sparsetir_sddmm_raw(q, k, scores, indptr, indices, nullptr, m, n, feat, nnz, device_id, stream) != 0) return -1;
   if (sparsetir_sparse_softmax_raw(scores, probs, indptr, m, nnz, device_id, stream) != 0) return -1;
-  return csrmm_run(probs, v, o, indptr, indices, m, n, feat, nnz, device_id, stream, /*hub_rows=*/true, 0,
+  return csrmm_run(probs, v, o, indptr, indices, m, n, feat, nnz, device_id, stream, /*hub_rows=*/true,
                    piece_bytes > 0 ? ws + pieces_at(m, nnz) : nullptr);
 }
