@@ -14,6 +14,8 @@ SHAPES = {
     "empty_runs": ([0] * 400 + [1, 2, 3] + [0] * 33 + [5]) * 20,
     "hubs_among_short_rows": [3, 0, 1, 900, 2, 2, 31, 32, 33, 0, 1] * 30,
     "long_rows": [700, 0, 1500, 64, 65],
+    # 159,000 positions: groups of 32-byte lanes take five blocks per SM
+    "one_round_of_five_blocks": [3, 0, 1, 9, 2, 31, 0, 7] * 3000,
 }
 
 
