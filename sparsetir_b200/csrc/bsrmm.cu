@@ -87,9 +87,11 @@ extern "C" int sparsetir_bsrmm_raw(const void* a_f16, const void* b_f16, float* 
   const __half* b = static_cast<const __half*>(b_f16);
   // Blocks of 32 and features in steps of 128 could take either tensor-core kernel.  bsrmm_mma.cu has the shorter chain in front of
   // the first product and is the faster one as long as all its thread blocks, 64 features of a block row each, are resident at
-  // once (10 % stored, us, tcgen05 / mma: 4096^2, F = 128 10.5 / 6.9, F = 256 9.8 / 9.4, 2720^2, F = 384 10.0 / 7.8; in more than one wave
-  // 4096^2, F = 384 12.4 / 13.6, 8192^2, F = 256 18.2 / 24.5); where whole pairs of feature tiles share the loads of A, less than that
-  // (1536^2, F = 512 6.7 / 5.7, 2048^2 6.7 / 7.2).
+  // once; where whole pairs of feature tiles share the loads of A, less than that.  How many blocks are stored moves both alike.
+  // us, tcgen05 / mma, at 2, 10, 50 and 100 % stored: 1024^2, F = 256 4.0 / 3.0, 5.3 / 3.2, 9.9 / 5.7, 13.0 / 7.3; 4096^2, F = 128 5.3 / 4.1, 10.5 / 7.0,
+  // 32.6 / 18.9, 48.8 / 30.6; F = 256 5.4 / 5.2, 9.8 / 9.4, 31.3 / 27.6, 47.3 / 47.5; in more than one wave F = 384 5.8 / 7.3, 10.2 / 13.6, 31.5 / 39.9,
+  // 47.9 / 70.7; pairs of tiles, 1536^2, F = 512 4.5 / 4.1, 6.7 / 5.8, 13.7 / 11.5, 19.0 / 15.9, 2048^2 4.5 / 4.6, 6.8 / 7.2, 16.6 / 15.9, 25.1 / 25.5.
+  // One row of 2,000 blocks among rows of 10, F = 256, 64 block rows 873 / 312.
   const long long units = static_cast<long long>(nb) * ceil_div(feat, 64);
   static const bool chosen = [] {  // a comparison switch of bsrmm_tc.cu
     const char* e = std::getenv("SPARSETIR_BSR_PATH");

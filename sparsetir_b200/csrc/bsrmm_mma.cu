@@ -1,6 +1,6 @@
 // BSR SpMM for block sizes that are multiples of 16 and feature counts that are multiples of 8, fp16
-// operands, fp32 sums: the shapes that the tcgen05 kernels of bsrmm_tc.cu (block size 32, features in
-// steps of 128) do not take.  They ran on CUDA cores at 11 TFLOP/s.
+// operands, fp32 sums: calls of one wave on blocks of 32 (bsrmm.cu has the rule), and all shapes that the tcgen05 kernels of
+// bsrmm_tc.cu (block size 32, features in steps of 128) do not take.  Those ran on CUDA cores at 11 TFLOP/s.
 //
 // A thread block owns 16 MT rows of a block row and 64 features; its four warps share the stored blocks, 16 columns ("a group")
 // at a time.  The rows of B and the values of A of a warp's next three or four groups are on their way into shared memory

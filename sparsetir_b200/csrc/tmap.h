@@ -1,4 +1,4 @@
-// Host-side construction of TMA tensor maps (CUtensorMap) for 2-D row-major arrays.
+// Host-side construction of TMA tensor maps (CUtensorMap) for row-major arrays: 2-D, and 3-D as column parts.
 // cuTensorMapEncodeTiled lives in the driver library; it is looked up through the runtime
 // (cudaGetDriverEntryPoint), so the shared library keeps no link-time dependency on libcuda.
 #ifndef SPARSETIR_B200_TMAP_H_
