@@ -414,7 +414,9 @@ SplitPlan split_plan(const SplitShape& sh, int m, int feat, int nnz) {
   const long long fewest = (nnz + batch - 1) / batch;
   SplitPlan p;
   p.gy = static_cast<int>(std::min<long long>(tiles, std::max<long long>(1, resident * 3 / fewest)));
-  while (tiles % p.gy != 0) ++p.gy;
+  int even = p.gy;
+  while (tiles % even != 0) ++even;
+  if (even <= resident) p.gy = even;  // a prime number of tiles is not a number of blocks that a grid can have
   const long long want = std::max<long long>(1, resident / p.gy) * subs, share = (nnz + want - 1) / want;
   const long long step = share < 4 * sh.lanes ? 8 : sh.lanes;
   p.span = static_cast<int>(std::max<long long>(sh.lanes, (share + step - 1) / step * step));

@@ -81,6 +81,22 @@ def test_two_vectors_per_lane(cuda_device, deg, feat):
     assert torch.equal(again, y)
 
 
+def test_a_prime_number_of_feature_tiles(cuda_device):
+    # 65,537 tiles of 160 features: more blocks than a grid can have if every tile had its own
+    feat, n, deg = 65_537 * 160 - 1, 2, [2, 0, 1]
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    ptr = torch.tensor([0, 2, 2, 3], dtype=torch.int32, device=cuda_device)
+    cols = torch.tensor([1, 0, 1], dtype=torch.int32, device=cuda_device)
+    vals = torch.rand(3, generator=g, device=cuda_device) - 0.5
+    x = torch.rand(n, feat, generator=g, device=cuda_device) - 0.5
+    y = torch.full((len(deg), feat), float("nan"), device=cuda_device)
+    ops.csrmm(vals, x.view(-1), y.view(-1), ptr, cols)
+    want = torch.stack([vals[0].double() * x[1] + vals[1].double() * x[0], torch.zeros_like(x[0]).double(), vals[2].double() * x[1]])
+    mag = torch.stack([(vals[0] * x[1]).abs() + (vals[1] * x[0]).abs(), torch.zeros_like(x[0]), (vals[2] * x[1]).abs()]).double()
+    # two products and their sum, or one product: at most three half-ulps of the sum of magnitudes
+    assert bool(((y.double() - want).abs() <= mag * 3 * 2.0 ** -24).all())
+
+
 def test_first_call_on_a_stream_can_be_captured(cuda_device):
     m, feat = 9000, 41
     ptr = torch.arange(0, 8 * m + 1, 8, dtype=torch.int32, device=cuda_device)
