@@ -920,10 +920,10 @@ int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
   // Shared memory is written and waited for once per batch, whatever its rows: where most slots are in rows of 1, 2 and 4, which keep the shuffles, the
   // kernel with both loops only has fewer registers for theirs (20 k rows of 3, F = 299 13.3 / 14.5, F = 256 10.8 / 11.3).  Tiles of 8 lanes: not on
   // short rows either, where they wait for chains of loads and not for L1 (169 k-node power-law graph, F = 100 59.8 / 61.1, F = 128 53.9 / 54.5; F = 32 among
-  // other work 19.3 / 19.6; tiles that rows do not fill, 40 k rows of 8, F = 100 16.5 / 17.6; one tile, 40 k rows of 9, F = 32 8.3 / 8.6), nor where one tile adds all
-  // results atomically (F = 32, two partitions 24.6 / 25.3).
+  // other work 19.3 / 19.6; tiles that rows do not fill, 40 k rows of 8, F = 100 16.5 / 17.6; one tile, 40 k rows of 9, F = 32 8.3 / 8.6).  One tile that adds its
+  // results atomically, F = 32, two partitions, shuffles / chunks: 105 k rows of 37 61.6 / 57.5, 40 k of 100 57.6 / 55.5, of 20 19.6 / 19.4.
   const bool long_rows = slots >= (tiles == 1 ? 16 * rows : WHOLE ? 8 * rows : 8 * rows + 1);
-  const bool shared = kMay && (LPR > 8 ? 4 * wide >= slots : long_rows && (tiles > 1 || la.all_atomic == 0));
+  const bool shared = kMay && (LPR > 8 ? 4 * wide >= slots : long_rows);
   auto go = [&](auto hand) -> int {
     constexpr Hand S = decltype(hand)::value;
     if (la.peers.n > 0) {
