@@ -41,9 +41,8 @@ constexpr int kThreads = 256;
 //
 // Five blocks per SM with one position in flight per group, where four had two (BLOCKS): B in L2 far from the SMs is waited for longer, and
 // a fifth more warps bring more than the second position (us, two on four blocks / one on five: 169 k power-law rows, F = 64 31 / 28.6,
-// 110 k rows of 12 F = 64 28.9 / 26.3, F = 256 164 / 149, 130 k of 20 F = 64 55.4 / 49.5, 80 k of 11 F = 512 219 / 205).  What is far is told by the
-// rows of B and not by its bytes (20 k of 11, F = 512 and 41 MB, 41.1 / 45.1, 50 k of 12 125 / 137, 40 k of 11 92 / 102).  Nearer ones
-// only where five_blocks() says so.  Four positions on three or two blocks: 42.7, 52.2 on the first of these; two on five and
+// 110 k rows of 12 F = 64 28.9 / 26.3, F = 256 164 / 149, 130 k of 20 F = 64 55.4 / 49.5, 80 k of 11 F = 512 219 / 205).  Only where that spares a round
+// of positions (five_blocks(); 20 k of 11, F = 512, 41.1 / 45.1, 50 k of 12 125 / 137, 40 k of 11 92 / 102 spare none).  Four positions on three or two blocks: 42.7, 52.2 on the first of these; two on five and
 // one on six blocks spill (35.9, 31.4).  16-byte lanes spill on four, 36 features and 100, 20 k rows of 11, a warp or half of one to a row / four
 // blocks / five 8.7 / 13.2 / 7.3 and 14.1 / 21.3 / 11.7, 3 k of 11 4.3 / 5.1 / 4.0 and 6.0 / 7.7 / 5.9.
 constexpr size_t kFarBytes = size_t{24} << 20;
@@ -457,12 +456,11 @@ bool in_groups(int m, int n, int feat, int nnz) {
   return per_row < (feat == 64 ? 64 : 50) && b_bytes <= l2_budget_bytes() / 8 * eighths;
 }
 
-// Whether groups of 32-byte lanes run on five blocks per SM: rows of B over 24 MB and more, 64 features of each; or where the positions
-// make fewer rounds of 32 per warp of them (us, four / five, 160 k positions, F = 64 6.1 / 5.2, F = 256 15.6 / 12.3; as many rounds, 200 k, 6.4 / 6.7 and
-// 16.3 / 17.8), of few rounds, where one counts, or with a large B (40 k rows of 20, F = 256 59 / 57, 50 k of 30, F = 512 295 / 262, but 20 k of
-// 30, F = 64 12.3 / 12.7).
+// Whether groups of 32-byte lanes run on five blocks per SM: where the positions make fewer rounds of 32 per warp of them (us, four / five, 160 k
+// positions, F = 64 6.1 / 5.2, F = 256 15.6 / 12.3, 80 k power-law rows F = 128 33.1 / 25.8, 120 k 44.5 / 37.4, 200 k 67.5 / 61.1; as many rounds, 200 k
+// positions 6.4 / 6.7 and 16.3 / 17.8, power-law rows 101 k F = 128 34.8 / 35.4, F = 256 65.9 / 67.3, 60 k F = 512 82.6 / 84.5), of few rounds, where
+// one counts, or with a large B (40 k rows of 20, F = 256 59 / 57, 50 k of 30, F = 512 295 / 262, but 20 k of 30, F = 64 12.3 / 12.7).
 bool five_blocks(int n, int feat, int nnz) {
-  if (static_cast<size_t>(n) * std::min(feat, 64) * 4 >= kFarBytes) return true;
   const int round = kNumSMs * (kThreads / 32) * 32;
   const int four = ceil_div(nnz, 4 * round), five = ceil_div(nnz, 5 * round);
   return five < four && (four <= 3 || static_cast<size_t>(n) * feat * 4 >= kFarBytes);
