@@ -358,7 +358,12 @@ struct SplitShape {
 
 // Two vectors per lane on half the lanes, us, one vector / two (rows of about equal length unless said otherwise):
 //  - up to 64 features: 30 k rows of 12 15.3 / 12.1, 9 k of 60 15.9 / 13.8, 200 k of 30 117 / 109, power-law graphs (4.5 per row)
-//    70 k 18.1 / 15.8, 200 k 34.7 / 34.7; 36 features, 300 per row, 40 k 209 / 184.
+//    70 k 18.1 / 15.8, 200 k 34.7 / 34.7; 36 features, 20 k of 40 24.2 / 19.5, 40 k of 200 161 / 146.
+//  - up to 64, no whole tile, long rows: equal ones lose by it and uneven ones gain, more by the fewer of the lanes' second vectors are in use:
+//    20 k rows of 500 / 20 k log-normal ones of that mean, F = 36 180 / 192 and 173 / 153, F = 48 180 / 186 and 170 / 147, F = 52 181 / 200 and
+//    172 / 162, F = 60 183 / 205 and 176 / 167; 40 k of 300 F = 36 213 / 223, F = 60 213 / 239; 40 k of 200 F = 52 153 / 153, F = 60 154 / 157, 20 k of 200 F = 60
+//    77 / 72.  Sizes do not tell the two apart; uneven rows, which graphs of that density have, decide (attention over 40 k of
+//    them, F = 56, one vector from 250 entries per row on 806, two 789).
 //  - more: 30 k of 12 F = 128 21.7 / 17.7, F = 256 39.9 / 32.6, 60 k of 8 F = 100 28.9 / 24.0; where a slice of B is more than L2 keeps
 //    they bring nothing (200 k of 16 F = 128 148 / 161), nor on power-law graphs (100 k F = 128 28.4 / 29.5).
 //  - whole tiles on long rows are at the L2-to-SM rate with either (200 per row and more, F = 64 and 128: within the 15 % by which
