@@ -905,13 +905,16 @@ int launch_lean_as(HybTable& tb, const LeanArgs& la, cudaStream_t stream) {
   const int item = lean_item_slots(LPR, W, tiles, slots);
   long long blocks = plan_lean(tb, item, kThreads / LPR);
   if (blocks < 0) return fail("sparsetir_hyb_spmm: too many thread blocks");
-  // A second wave of a few blocks costs as much as a full one: items long enough to make one of both, up to a quarter longer, a third where rows are
-  // long and all alike in cost (us, 1.06 waves / one: 10 k rows of 12, F = 512 25.5 / 17.7, 20 k of 8, F = 128 10.3 / 7.7; 1.32 waves, 10 k of 10,
-  // F = 300 19.1 / 14.3, but power-law rows, 20 k, F = 200 14.8 / 16.1).  Single floats per lane lose by it (14 k power-law rows, F = 299 19.4 / 21.5).
+  // A second wave of a few blocks costs as much as a full one: items up to half longer where that makes one of both (us, 1.06 waves / one: 10 k rows of
+  // 12, F = 512 25.5 / 17.7, 20 k of 8, F = 128 10.3 / 7.7; 1.34 waves, 19 k of 8, F = 512 32.4 / 29.5).  Up to 1.1 waves where rows of 1 and 2 slots are many,
+  // which end the more often the longer the item is: power-law rows, 1.05 waves, 59 k, F = 64 14.0 / 11.7, but 1.2, 62 k, F = 64 15.2 / 16.2, 31 k, F = 512 38.9 / 44.0.
+  // Twice the item takes half the blocks away that wider rows would have (rows of 1 and 20 slots, 18 k, F = 100 12.2 / 14.3).  Single floats per lane lose by it (14 k
+  // power-law rows, F = 299 19.4 / 21.5).  Over 313 matrices of 1 to 1.35 waves, among them rows of 1 and 10 and power-law rows in pieces of 32, 179 take it:
+  // the mean of these gains 11 %, seven lose 2 to 6.
   constexpr long long kResident = 8ll * kNumSMs;
-  if (W > 1 && blocks * tiles > kResident && blocks * tiles * 100 <= kResident * (slots >= 8 * rows ? 135 : 125)) {
+  if (W > 1 && blocks * tiles > kResident && blocks * tiles * 100 <= kResident * (slots >= 7 * rows ? 135 : 110)) {
     long long fit = blocks;
-    for (int more = item + 8; fit * tiles > kResident && more <= 2 * item; more += 8) fit = plan_lean(tb, more, kThreads / LPR);
+    for (int more = item + 8; fit * tiles > kResident && more <= item + item / 2; more += 8) fit = plan_lean(tb, more, kThreads / LPR);
     blocks = fit * tiles > kResident ? plan_lean(tb, item, kThreads / LPR) : fit;
   }
   dim3 grid(static_cast<unsigned>(blocks), tiles);
