@@ -9,8 +9,8 @@
 //
 // Bound: the L2-to-SM gather of B (each block reads the 16 rows of its groups once per 16 MT rows of C) and the copies' latency on
 // small matrices.  10 % of the blocks stored, us, CUDA cores / operands straight into registers, where four rows per
-// load met in the same banks of L1 / now: 8192 x 8192, block 16, F = 512 626 / 79 / 53; block 64 645 / 62 / 53; block 32, F = 496
-// 630 / 54 / 49; 4096 x 4096, block 16, 5 %, F = 208 - / 11.1 / 9.4; 2048 x 2048, block 16, F = 64 - / 4.4 / 3.4.
+// load met in the same banks of L1 / now: 8192 x 8192, block 16, F = 512 626 / 81 / 49; block 64 645 / 64 / 48; block 32, F = 496
+// 630 / 56 / 45; 4096 x 4096, block 16, 5 %, F = 208 - / 11.2 / 8.1.
 #include <cuda_fp16.h>
 
 #include "common.h"
