@@ -1,5 +1,6 @@
 """Calls whose time must follow the work in them: rows of very different lengths beside rows of one length, fewer features beside
-more.  A ratio of two times, taken in turn on the same GPU; every limit lies well above what is measured."""
+more.  A ratio of two times, taken in turn on the same GPU.  The same ratio differs by up to 7 % from one GPU to another, so only
+faults that are a factor have a test: a limit lies about midway, in factors, between what the call takes and what it took with the fault."""
 import numpy as np
 import pytest
 import torch
@@ -52,30 +53,21 @@ def lengths(kind, n, mean):
     return np.clip(np.rint(rng.lognormal(np.log(mean) - 2.0, 2.0, n)), 1, n // 4).astype(np.int64)
 
 
-def csr_call(f, device, deg, feat):
-    """A kept call of sddmm or csrmm on a matrix of uniformly drawn columns."""
+def sddmm_call(device, deg, feat):
+    """A kept call on a matrix of uniformly drawn columns."""
     n, nnz = len(deg), int(deg.sum())
     g = torch.Generator(device=device).manual_seed(feat)
     ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(device)
     cols = torch.randint(0, n, (nnz,), generator=g, device=device, dtype=torch.int32)
     a, b, e = (torch.rand(k, generator=g, device=device) for k in (n * feat, n * feat, nnz))
-    return f.prepare(a, b, e, ptr, cols) if f is ops.sddmm else f.prepare(e, a, b, ptr, cols)
+    return ops.sddmm.prepare(a, b, e, ptr, cols)
 
 
-@pytest.mark.parametrize("n,mean,feat,limit", [(100_000, 30, 256, 1.2), (20_000, 30, 24, 1.18)])
+@pytest.mark.parametrize("n,mean,feat,limit", [(100_000, 30, 256, 1.2), (20_000, 30, 24, 1.22)])
 def test_sddmm_on_uneven_rows(cuda_device, n, mean, feat, limit):
     uneven = lengths("uneven", n, mean)
     even = lengths("equal", n, int(round(uneven.sum() / n)))
-    check_ratio(csr_call(ops.sddmm, cuda_device, uneven, feat), csr_call(ops.sddmm, cuda_device, even, feat), limit)
-
-
-@pytest.mark.parametrize("op,n,mean,feat,other,limit", [
-    ("sddmm", 20_000, 10, 512, 128, 3.85), ("sddmm", 20_000, 100, 224, 256, 1.08), ("sddmm", 10_000, 11, 40, 64, 1.3), ("sddmm", 80_000, 5, 298, 300, 1.4),
-    ("csrmm", 10_000, 4, 512, 256, 1.62), ("csrmm", 20_000, 3, 384, 256, 1.4)])
-def test_more_and_fewer_features(cuda_device, op, n, mean, feat, other, limit):
-    """Beside a neighbour that is known to be served well: what is fixed in a call weighs less where there are more features."""
-    deg, f = lengths("equal", n, mean), getattr(ops, op)
-    check_ratio(csr_call(f, cuda_device, deg, feat), csr_call(f, cuda_device, deg, other), limit)
+    check_ratio(sddmm_call(cuda_device, uneven, feat), sddmm_call(cuda_device, even, feat), limit)
 
 
 @pytest.mark.parametrize("feat", [64, 128])
@@ -92,11 +84,10 @@ def test_rgms_with_hub_destinations(cuda_device, feat):
                                 ptr, cols)
     hubs = np.full(10_000, 4, np.int64)
     hubs[250::500] = 2_000
-    check_ratio(layer(hubs), layer(np.full(10_000, 8, np.int64)), 2.0)
+    check_ratio(layer(hubs), layer(np.full(10_000, 8, np.int64)), 4.4)
 
 
-@pytest.mark.parametrize("n,width,feat,other,limit", [(20_000, 4, 299, 300, 1.13), (20_000, 8, 512, 256, 2.2)])
-def test_hyb_of_more_and_fewer_features(cuda_device, n, width, feat, other, limit):
+def test_hyb_of_more_features(cuda_device, n=20_000, width=8, feat=512, other=256, limit=2.0):
     """ELL rows of one width."""
     def call(f):
         g = torch.Generator(device=cuda_device).manual_seed(f)
@@ -105,19 +96,3 @@ def test_hyb_of_more_and_fewer_features(cuda_device, n, width, feat, other, limi
                   torch.randint(0, n, (n * width,), generator=g, device=cuda_device, dtype=torch.int32))
         return ops.hyb_spmm.prepare(*ops.hyb_args(x, torch.zeros(n, f, device=cuda_device), [bucket], f, 0))
     check_ratio(call(feat), call(other), limit)
-
-
-def test_rgms_f16_with_more_ranges_than_a_block_keeps(cuda_device):
-    """1,800 (bucket, relation) ranges, most of them empty, beside 900."""
-    def layer(rels, n=2000, feat=32):
-        g = torch.Generator(device=cuda_device).manual_seed(rels)
-        buckets = []
-        for width in (1, 2, 4, 8, 16, 32):
-            k = rels if width == 1 else 2
-            shape = (k, 32 // width, width)
-            buckets.append((torch.rand(shape, generator=g, device=cuda_device).half(),
-                            torch.randint(0, n, shape[:2], generator=g, device=cuda_device).int(),
-                            torch.randint(0, n, shape, generator=g, device=cuda_device).int(), torch.arange(k, device=cuda_device).int()))
-        x, w = (torch.rand(k, generator=g, device=cuda_device).half() for k in (n * feat, rels * feat * feat))
-        return ops.rgms_ell3d_f16.prepare(*ops.rgms_ell3d_f16_args(w, x, torch.zeros(n * feat, device=cuda_device), buckets, feat, feat))
-    check_ratio(layer(300), layer(150), 3.45)
