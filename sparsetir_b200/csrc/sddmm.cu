@@ -42,9 +42,10 @@ constexpr int kThreads = 256;
 // Five blocks per SM with one position in flight per group, where four had two (BLOCKS): B in L2 far from the SMs is waited for longer, and
 // a fifth more warps bring more than the second position (us, two on four blocks / one on five: 169 k power-law rows, F = 64 31 / 28.6,
 // 110 k rows of 12 F = 64 28.9 / 26.3, F = 256 164 / 149, 130 k of 20 F = 64 55.4 / 49.5, 80 k of 11 F = 512 219 / 205).  Only where that spares a round
-// of positions (five_blocks(); 20 k of 11, F = 512, 41.1 / 45.1, 50 k of 12 125 / 137, 40 k of 11 92 / 102 spare none).  Four positions on three or two blocks: 42.7, 52.2 on the first of these; two on five and
-// one on six blocks spill (35.9, 31.4).  16-byte lanes spill on four, 36 features and 100, 20 k rows of 11, a warp or half of one to a row / four
-// blocks / five 8.7 / 13.2 / 7.3 and 14.1 / 21.3 / 11.7, 3 k of 11 4.3 / 5.1 / 4.0 and 6.0 / 7.7 / 5.9.
+// of positions (five_blocks(); 20 k of 11, F = 512, 41.1 / 45.1, 50 k of 12 125 / 137, 40 k of 11 92 / 102 spare none).  Four positions on three or two
+// blocks: 42.7, 52.2 on the first of these; two on five and one on six blocks spill (35.9, 31.4).  16-byte lanes spill on four, 36 features and
+// 100, 20 k rows of 11, a warp or half of one to a row / four blocks / five 8.7 / 13.2 / 7.3 and 14.1 / 21.3 / 11.7, 3 k of 11 4.3 / 5.1 / 4.0
+// and 6.0 / 7.7 / 5.9.
 constexpr size_t kFarBytes = size_t{24} << 20;
 template <int LPR, int W, int VPL, bool PEERS, int BLOCKS>
 __global__ void __launch_bounds__(kThreads, BLOCKS)
