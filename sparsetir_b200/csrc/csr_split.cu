@@ -364,8 +364,10 @@ struct SplitShape {
 //    172 / 162, F = 60 183 / 205 and 176 / 167; 40 k of 300 F = 36 213 / 223, F = 60 213 / 239; 40 k of 200 F = 52 153 / 153, F = 60 154 / 157, 20 k of 200 F = 60
 //    77 / 72.  Sizes do not tell the two apart; uneven rows, which graphs of that density have, decide (attention over 40 k of
 //    them, F = 56, one vector from 250 entries per row on 806, two 789).
-//  - more: 30 k of 12 F = 128 21.7 / 17.7, F = 256 39.9 / 32.6, 60 k of 8 F = 100 28.9 / 24.0; where a slice of B is more than L2 keeps
-//    they bring nothing (200 k of 16 F = 128 148 / 161), nor on power-law graphs (100 k F = 128 28.4 / 29.5).
+//  - more: 30 k of 8 F = 128 18.1 / 17.5, of 12 21.8 / 21.1, F = 512 70.8 / 68.1, 20 k of 10 F = 68 14.7 / 13.1; where a slice of B is more than a share of L2, from 10
+//    entries per row on (60 k of 10 F = 128 31.5 / 31.1, 75 k of 12 42.9 / 42.1, 60 k of 20 F = 512 186 / 176; 60 k of 8 F = 100 28.1 / 29.6, F = 512 97 / 103, 90 k of 6
+//    F = 256 62.9 / 66.9); where it is more than L2 keeps they bring nothing (200 k of 16 F = 128 148 / 161), nor on power-law graphs (100 k
+//    F = 128 28.4 / 29.5).
 //  - whole tiles on long rows are at the L2-to-SM rate with either (200 per row and more, F = 64 and 128: within the 15 % by which
 //    one kernel's time moves there with the share of a sub-warp): not taken.
 //  - less than a batch for each of the resident blocks, half as many here: not taken (3 k of 30 F = 128 9.4 / 10.0).
@@ -373,7 +375,8 @@ bool two_vectors(int m, int n, int feat, int nnz, bool whole) {
   const int per_row = nnz / m;
   if (whole && per_row >= 100) return false;
   if (feat <= 64) return nnz >= 80000;
-  return nnz >= 100000 && per_row >= 6 && static_cast<size_t>(n) * std::min(feat * 4, 512) <= (size_t{48} << 20);
+  const size_t slice = static_cast<size_t>(n) * std::min(feat * 4, 512);
+  return nnz >= 100000 && per_row >= (slice <= (size_t{22} << 20) ? 6 : 10) && slice <= (size_t{48} << 20);
 }
 
 SplitShape split_shape(uintptr_t bits, int m, int n, int feat, int nnz) {

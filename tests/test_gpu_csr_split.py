@@ -57,10 +57,11 @@ def test_rows_meet_across_sub_warps_and_blocks(cuda_device, shape, feat, offset)
 
 @pytest.mark.parametrize("feat", [36, 64, 68, 128, 132, 256])
 @pytest.mark.parametrize("deg", [[0, 1, 2, 30, 7, 0, 0, 13, 32, 11] * 1100, [3000, 8, 0] * 10 + [8] * 10_000, [99] * 1200, [100] * 1200, [101] * 1200,
-                                 [12, 0, 4] * 5000, [12, 0, 4] * 4999 + [12, 0, 3]],
-                         ids=["mixed", "hubs", "below", "long", "longer", "least", "less"])
+                                 [12, 0, 4] * 5000, [12, 0, 4] * 4999 + [12, 0, 3],
+                                 [0, 1, 2, 60, 7, 0, 0, 43, 32, 15] * 900, [2000, 11, 0] * 10 + [11] * 8000],
+                         ids=["mixed", "hubs", "below", "long", "longer", "least", "less", "mixed_16", "hubs_13"])
 def test_two_vectors_per_lane(cuda_device, deg, feat):
-    # more and less than 80,000 and 100,000 entries, and rows of 99, 100 and 101: from 100 on whole tiles (64, 128 and 256 features) go
+    # more and less than 80,000 and 100,000 entries, rows of 5 to 13 on average, and rows of 99, 100 and 101: from 100 on whole tiles (64, 128 and 256 features) go
     # back to one vector
     deg = torch.tensor(deg, device=cuda_device)
     m, n, nnz = len(deg), 2003, int(deg.sum())
